@@ -70,13 +70,14 @@ class Context:
         if rc != 0:
             raise MetalTileError(rc, (self._lib.mtc_last_error(None) or b"").decode())
         self._h = h
+        self._handle = h.value             # the same as an integer, for the native binding of the typed ops
         self.device = int(device)
 
     # ---- lifecycle ------------------------------------------------------------
     def close(self):
         if getattr(self, "_h", None):
             self._lib.mtc_destroy(self._h)
-            self._h = None
+            self._h = self._handle = None
 
     def __del__(self):
         try:
