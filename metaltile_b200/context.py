@@ -60,6 +60,20 @@ def _dt(dtype) -> int:
                   .replace("float32", "f32")]
 
 
+_native = None
+
+
+def _binding():
+    """The native binding (it needs torch in the process, which nothing else of this module does: loaded on first use)."""
+    global _native
+    if _native is None:
+        import torch  # noqa: F401
+
+        from . import _native as mod
+        _native = mod
+    return _native
+
+
 class Context:
     """One per device; not thread-safe (the caller serialises, as the reference's tests do)."""
 
@@ -126,25 +140,8 @@ class Context:
         items = dict(buffers)
         for k, v in (fn_consts or {}).items():
             items[k] = int(v).to_bytes(4, "little")
-        keep = []
-        arr = (NamedBuf * len(items))()
-        for i, (name, data) in enumerate(items.items()):
-            raw = ctypes.create_string_buffer(bytes(data), len(data))
-            keep.append(raw)
-            arr[i].name = name.encode()
-            arr[i].data = ctypes.cast(raw, ctypes.c_void_p)
-            arr[i].bytes = len(data)
-            arr[i].is_output = 1 if name in outputs else 0
-        g = (ctypes.c_uint32 * 3)(*[int(v) for v in grid_groups])
-        t = (ctypes.c_uint32 * 3)(*[int(v) for v in threads_per_group])
-        us = ctypes.c_float(0.0)
-        self._check(self._lib.mtc_dispatch(self._h, kernel.encode(), _dt(dtype), arr, len(items), g, t,
-                                           ctypes.byref(us)))
-        res = DispatchResult(elapsed_us=float(us.value))
-        for i, name in enumerate(items):
-            if arr[i].is_output:
-                res.outputs[name] = keep[i].raw
-        return res
+        outs, us = _binding().dispatch(self, kernel, _dt(dtype), items, outputs, grid_groups, threads_per_group)
+        return DispatchResult(outputs=outs, elapsed_us=us)
 
     def bench(self, kernel: str, buffers: Mapping[str, bytes], fn_consts: Optional[Mapping[str, int]] = None,
               dtype="f32", outputs: Sequence[str] = ("out",), warmup: int = 15, iters: int = 10, cold_l2: bool = True):

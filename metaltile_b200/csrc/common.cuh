@@ -23,6 +23,8 @@ struct Ctx {
     uint32_t *d_status = nullptr;  // device status word (bounded waits / rejected indices)
     void *d_scratch = nullptr;     // grow-only scratch owned by the context
     size_t scratch_bytes = 0;
+    char *h_stage = nullptr;       // page-locked block of mtc_dispatch (1 MiB, made on the first call)
+    cudaEvent_t timing[2] = {};    // mtc_dispatch: events around the kernel
     int qmm_force_tn = 0;          // option "qmm_tile_tokens": 0 = choose per shape
     int qmv_max_occ = 0;           // option "qmv_max_ctas_per_sm": > 0 caps the CTAs per SM of the qmv kernel's grid
     int qmv_small_m_mma = 1;       // option "qmv_small_m_mma": 0 keeps 2 <= M <= 16 on the CUDA-core kernel

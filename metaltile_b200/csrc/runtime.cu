@@ -208,6 +208,17 @@ int ensure_scratch(Ctx *ctx, size_t bytes) {
     return MTC_OK;
 }
 
+// Page-locked block of mtc_dispatch: small inputs on their way up, outputs and the status word on their way down.
+constexpr size_t kHostStageBytes = 1u << 20;
+constexpr size_t kSmallUpload = 64u << 10;
+int ensure_host_stage(Ctx *ctx) {
+    if (ctx->h_stage) return MTC_OK;
+    void *p = nullptr;
+    MTC_CUDA(ctx, cudaMallocHost(&p, kHostStageBytes), MTC_ERR_BUFFER);
+    ctx->h_stage = static_cast<char *>(p);
+    return MTC_OK;
+}
+
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 int ensure_worklist(Ctx *ctx, size_t bytes, cudaStream_t st) {
@@ -290,6 +301,9 @@ int mtc_destroy(mtc_ctx *ctx) {
     if (ctx->d_ksplit) cudaFree(ctx->d_ksplit);
     if (ctx->d_tc_scratch) cudaFree(ctx->d_tc_scratch);
     if (ctx->d_tc_counters) cudaFree(ctx->d_tc_counters);
+    if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
+    for (cudaEvent_t ev : ctx->timing)
+        if (ev) cudaEventDestroy(ev);
     for (void *p : ctx->retired) cudaFree(p);
     delete ctx;
     return MTC_OK;
@@ -358,9 +372,7 @@ int mtc_memset(mtc_ctx *ctx, void *stream, void *d_ptr, int value, size_t bytes)
 
 // A kernel that gave up on a bounded wait (or rejected an index) leaves a code in the status word and returns; the
 // host learns of it at the next synchronising call.
-static int check_status(mtc_ctx *ctx, const char *who) {
-    uint32_t word = 0;
-    MTC_CUDA(ctx, cudaMemcpy(&word, ctx->d_status, sizeof(uint32_t), cudaMemcpyDeviceToHost), MTC_ERR_DISPATCH);
+static int status_error(mtc_ctx *ctx, const char *who, uint32_t word) {
     if (word != 0) {
         char buf[160];
         std::snprintf(buf, sizeof(buf), "%s: a kernel reported status 0x%x (a bounded device-side wait expired or an index was rejected); "
@@ -368,6 +380,11 @@ static int check_status(mtc_ctx *ctx, const char *who) {
         return fail(ctx, MTC_ERR_TIMEOUT, buf);
     }
     return MTC_OK;
+}
+static int check_status(mtc_ctx *ctx, const char *who) {
+    uint32_t word = 0;
+    MTC_CUDA(ctx, cudaMemcpy(&word, ctx->d_status, sizeof(uint32_t), cudaMemcpyDeviceToHost), MTC_ERR_DISPATCH);
+    return status_error(ctx, who, word);
 }
 
 int mtc_sync(mtc_ctx *ctx, void *stream) {
@@ -1499,8 +1516,31 @@ int dispatch_pass(mtc_ctx *ctx, const char *kernel_name, int dtype, mtc_named_bu
     const size_t base_off = cc ? cc->offset : 0;
     if (cc) cc->offset += total;
     cudaStream_t st = nullptr;
+    if (!cc) {
+        rc = ensure_host_stage(ctx);
+        if (rc != MTC_OK) return rc;
+    }
+    // Buffers of a few KB that lie side by side in the scratch block travel as one copy out of the page-locked block: a
+    // pageable copy costs ~8 us of host time each, whatever its size.  Larger ones go as they are - the driver's own
+    // staging of pageable memory (17-20 GB/s) is as fast as one host thread can read them.
+    size_t run_begin = 0, run_end = 0;
+    auto flush_run = [&]() -> cudaError_t {
+        const cudaError_t e = run_end > run_begin ? cudaMemcpyAsync(static_cast<char *>(ctx->d_scratch) + run_begin, ctx->h_stage + run_begin,
+                                                                    run_end - run_begin, cudaMemcpyHostToDevice, st)
+                                                  : cudaSuccess;
+        run_begin = run_end = 0;
+        return e;
+    };
     for (Staged &sb : st_bufs) {
         sb.dev = static_cast<char *>(ctx->d_scratch) + base_off + sb.offset;
+        if (!cc && sb.need && sb.need <= kSmallUpload && sb.offset + sb.need <= kHostStageBytes) {
+            // h_stage mirrors the scratch block's offsets; the previous call's copies out of it ended with that call
+            if (run_end == 0) run_begin = sb.offset;
+            std::memcpy(ctx->h_stage + sb.offset, sb.buf->data, sb.need);
+            run_end = sb.offset + sb.need;
+            continue;
+        }
+        if (!cc) MTC_CUDA(ctx, flush_run(), MTC_ERR_BUFFER);
         Produced *from = nullptr;
         if (cc && !sb.buf->is_output)
             for (Produced &pr : cc->produced)
@@ -1515,6 +1555,7 @@ int dispatch_pass(mtc_ctx *ctx, const char *kernel_name, int dtype, mtc_named_bu
             MTC_CUDA(ctx, cudaMemcpyAsync(sb.dev, sb.buf->data, sb.need, cudaMemcpyHostToDevice, st), MTC_ERR_BUFFER);
         }
     }
+    if (!cc) MTC_CUDA(ctx, flush_run(), MTC_ERR_BUFFER);
     auto dev = [&](const char *name) -> char * {
         for (Staged &sb : st_bufs)
             if (std::strcmp(sb.buf->name, name) == 0) return sb.dev;
@@ -1522,8 +1563,10 @@ int dispatch_pass(mtc_ctx *ctx, const char *kernel_name, int dtype, mtc_named_bu
     };
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     if (elapsed_us) {
-        MTC_CUDA(ctx, cudaEventCreate(&e0), MTC_ERR_DISPATCH);
-        MTC_CUDA(ctx, cudaEventCreate(&e1), MTC_ERR_DISPATCH);
+        for (cudaEvent_t &ev : ctx->timing)
+            if (!ev) MTC_CUDA(ctx, cudaEventCreate(&ev), MTC_ERR_DISPATCH);
+        e0 = ctx->timing[0];
+        e1 = ctx->timing[1];
         cudaEventRecord(e0, st);
     }
     switch (row->family) {
@@ -1624,25 +1667,35 @@ int dispatch_pass(mtc_ctx *ctx, const char *kernel_name, int dtype, mtc_named_bu
         if (rc == MTC_OK)
             for (Staged &sb : st_bufs)
                 if (sb.buf->is_output) cc->produced.push_back(Produced{sb.buf->name, sb.dev, sb.need, sb.buf, false});
-        if (elapsed_us) {
-            cudaEventDestroy(e0);
-            cudaEventDestroy(e1);
-        }
         return rc;
     }
     if (rc == MTC_OK) {
-        // every is_output parameter is read back (crates/metaltile-runtime/src/dispatch/single_dispatch.rs:100-117)
-        for (Staged &sb : st_bufs)
-            if (sb.buf->is_output && sb.need) cudaMemcpyAsync(sb.buf->data, sb.dev, sb.need, cudaMemcpyDeviceToHost, st);
+        // every is_output parameter is read back (crates/metaltile-runtime/src/dispatch/single_dispatch.rs:100-117): outputs
+        // that fit land in the page-locked block with the status word, so that one synchronisation ends the call (a
+        // copy to pageable memory waits by itself: ~10 us each, and 12 us for the status word on its own)
+        size_t at = 256;
+        for (Staged &sb : st_bufs) {
+            if (!sb.buf->is_output || !sb.need) continue;
+            const bool fits = at + sb.need <= kHostStageBytes;
+            cudaMemcpyAsync(fits ? static_cast<void *>(ctx->h_stage + at) : sb.buf->data, sb.dev, sb.need, cudaMemcpyDeviceToHost, st);
+            sb.offset = fits ? at : 0;
+            if (fits) at += align_up(sb.need, 256);
+        }
+        cudaMemcpyAsync(ctx->h_stage, ctx->d_status, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
         cudaError_t e = cudaStreamSynchronize(st);
-        if (e != cudaSuccess) rc = fail(ctx, MTC_ERR_DISPATCH, std::string("dispatch: ") + cudaGetErrorString(e));
-        else rc = check_status(ctx, "dispatch");
+        if (e != cudaSuccess) {
+            rc = fail(ctx, MTC_ERR_DISPATCH, std::string("dispatch: ") + cudaGetErrorString(e));
+        } else {
+            for (Staged &sb : st_bufs)
+                if (sb.buf->is_output && sb.need && sb.offset) std::memcpy(sb.buf->data, ctx->h_stage + sb.offset, sb.need);
+            uint32_t word = 0;
+            std::memcpy(&word, ctx->h_stage, sizeof(word));
+            rc = status_error(ctx, "dispatch", word);
+        }
     }
     if (elapsed_us) {
         float ms = 0.f;
         if (rc == MTC_OK && cudaEventElapsedTime(&ms, e0, e1) == cudaSuccess) *elapsed_us = ms * 1000.0f;
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
     }
     return rc;
 }
