@@ -96,8 +96,9 @@ int mtc_qmv(mtc_ctx *ctx, void *stream, const void *w, const void *scales, const
  * Ragged M needs no padding (the reference pads to 32: quantized_mma_dynamic_m.rs:46-112). */
 int mtc_qmm(mtc_ctx *ctx, void *stream, const void *w, const void *scales, const void *biases,
             const void *x, void *out, int M, int N, int K, int bits, int group_size, int dtype);
-/* Name of the kernel family mtc_qmm would run for these arguments with aligned pointers and default options
- * ("qmv_stream", "qmv_cuda_core", "qmv_mma_sync", "qmm_tcgen05"); the analogue of asserting on
+/* Name of the kernel family mtc_qmm's selector names for these arguments with aligned pointers and default options
+ * ("qmv_stream", "qmv_cuda_core", "qmv_mma_sync", "qmm_tcgen05"; option "qmv_frag" lets the fragment kernel stand in for the
+ * first three and, below 32 Mi codes, for the last at M <= 16); the analogue of asserting on
  * mt_qmm_for's routing (quantized.rs:5127-5199). */
 const char *mtc_qmm_route(int M, int N, int K, int bits, int group_size, int dtype);
 
@@ -108,8 +109,9 @@ const char *mtc_qmm_route(int M, int N, int K, int bits, int group_size, int dty
  * mtc_qmv_batched: 1 to 4 projections that read the SAME activations (same x, M, K, dtype) in one launch, each
  * writing its own output.  With the outputs laid out one after the other this is ffai_batched_qkv_qgemv(_fast)
  * (crates/metaltile-std/src/ffai/batched_qkv_qgemv.rs:1-35: q, k, v in one dispatch, one concatenated result) and
- * ffai_batched_4_qgemv (crates/metaltile-std/src/ffai/batched_4_qgemv.rs:1-45).  Shapes outside the streaming
- * kernel's contract (4-bit, f16 / bf16, M <= 8, K % 256 == 0, group 64 or 128) run as separate mtc_qmv launches.
+ * ffai_batched_4_qgemv (crates/metaltile-std/src/ffai/batched_4_qgemv.rs:1-45).  The streaming kernel (M = 1), the ring
+ * kernel (2 <= M <= 16) and the fragment kernel take several projections in one launch; what none of them takes runs as
+ * separate mtc_qmv launches.
  *
  * mtc_chain_*: a prepared list of projections walked by ONE persistent grid, the counterpart of
  * Context::dispatch_chain (crates/metaltile-runtime/src/context.rs:363-395: several passes, one commit, ordering
@@ -258,6 +260,11 @@ int mtc_peer_barrier(mtc_ctx *ctx, void *stream, void *const *peer_flags, int n_
  *                      CUDA-core kernel is faster), fused projections at any size; 2 takes every M <= 8 at any size
  *                      (slower than the register-ring kernel at M >= 2); 0 never.  mtc_qmv_batched fuses its projections into one launch where this kernel
  *                      takes them and launches them one by one otherwise
+ *   "qmv_frag"         the fragment kernel (warp-level tensor cores, every width, weights straight from global memory): 1
+ *                      (default) where it is faster than the other small-M kernels (widths other than 4-bit from M = 2 on, f32
+ *                      activations from M = 5 on, 4-bit shapes the ring kernel does not take, M = 1 up to 24 Mi codes) unless
+ *                      "qmv_stream", "qmv_small_m_mma" or "qmv_small_m_tc" selects another kernel; 2 whenever it supports
+ *                      the shape (M <= 16, K % 32 == 0, power-of-two group >= 32, 16-byte aligned w and x); 0 never
  *   "qmv_tc"           1: those shapes run on the tensor-memory decode kernel instead (slower today; default 0)
  *   "gather_stream"    0: grouped products never take the weight-streaming kernel (default 1: the CSR form with
  *                      4-bit codes, f16 / bf16, k_in % 256 == 0, group 64 or 128 and m_total <= 64 n_experts does)

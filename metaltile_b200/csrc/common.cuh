@@ -39,6 +39,7 @@ struct Ctx {
     size_t tc_scratch_bytes = 0;
     uint32_t *d_tc_counters = nullptr;   // its arrival counters, zero between launches
     std::vector<void *> retired;   // outgrown scratch blocks: freed by mtc_destroy, so that captured graphs never see freed memory
+    int qmv_frag = 1;              // option "qmv_frag": 0 = never use the fragment kernel (qmv_frag.cuh), 2 = whenever it supports the shape
     int qmv_stream = 1;            // option "qmv_stream": 0 = never use the streaming decode kernel (qmv_stream.cu)
     int pdl_early_weights = 1;     // option "pdl_early_weights": 0 = no load of w / scales / biases before the previous kernel of the stream is complete
     void *d_worklist = nullptr;    // gather_qmm work list (grow-only, owned by the context)
@@ -166,6 +167,9 @@ struct StreamChain;
 cudaError_t stream_chain_create(Ctx *ctx, const mtc_qmv_desc *descs, int n, StreamChain **out, std::string *why);
 cudaError_t stream_chain_run(Ctx *ctx, cudaStream_t st, StreamChain *c);
 void stream_chain_destroy(StreamChain *c);
+bool qmv_frag_supported(int M, int N, int K, int bits, int group_size, int dt, const void *w, const void *scales, const void *biases,
+                        const void *x);
+cudaError_t launch_qmv_frag(Ctx *ctx, cudaStream_t st, const mtc_qmv_desc *d, int n);
 bool qmv_mma_supported(int M, int N, int K, int bits, int group_size, int dt, const void *w, const void *x);
 cudaError_t launch_qmv_mma(Ctx *ctx, cudaStream_t st, const void *w, const void *scales, const void *biases, const void *x,
                            void *out, int M, int N, int K, int group_size, int dt);

@@ -182,6 +182,31 @@ inline bool stream_takes_single(const Ctx *ctx, int M, int N, int K) {
     return stream_takes(ctx, M) && (ctx->qmv_stream == 2 || static_cast<long long>(N) * K >= kStreamMinCodes);
 }
 
+// The fragment kernel (qmv_frag.cuh) against the other small-M kernels, measured with cold weights (us, other kernel -> it).
+//   widths other than 4-bit, 16-bit activations, 2 <= M: 8-bit 4096 x 4096 M = 4 13.7 -> 7.2, M = 8 19.9 -> 8.6; 3-bit group 32
+//     8192 x 8192 M = 4 32.5 -> 21.5 (CUDA cores spend one FFMA per code and token).  From M = 9 on the tcgen05 kernel with K
+//     slices is the other one: 4096 x 4096 19 -> 12-17, but 8192 x 8192 49 -> 60, hence the limit on codes; groups of 32
+//     need twice the tiles of columns there (19 -> 25).
+//   f32 activations: three pieces per value, so the FFMA kernel wins below M = 5 (M = 4: 14.0 against 16.8), not above (M = 16
+//     39.3 -> 27).
+//   4-bit, 16-bit: where the ring kernel of qmv_mma.cu does not go (K % 512 != 0 or group 32; 2880 x 2880 M = 4 7.7 -> 5.0), and at
+//     M = 1 up to 24 Mi codes (4096 x 4096 5.3 -> 4.7; 14336 x 4096 stays with the streaming kernel: 10.3 against 10.9).
+inline bool frag_rule(int M, int N, int K, int bits, int group_size, int dt) {
+    const long long codes = static_cast<long long>(N) * K;
+    if (dt == MTC_F32) return M >= 5;
+    if (M >= 9 && (codes >= (32ll << 20) || group_size % 64 != 0)) return false;
+    if (bits != 4) return M >= 2;
+    if (M == 1) return group_size % 64 == 0 && (K % 512 != 0 || codes <= (24ll << 20));
+    return K % 512 != 0 || group_size < 64 || group_size > 256;
+}
+inline bool frag_takes(const Ctx *ctx, int M, int N, int K, int bits, int group_size, int dt, const void *w, const void *scales,
+                       const void *biases, const void *x) {
+    // an option that selects another kernel for these shapes wins over the rule
+    const bool by_rule = ctx->qmv_frag == 1 && ctx->qmv_stream == 1 && ctx->qmv_small_m_mma == 1 && ctx->qmv_small_m_tc == 1 &&
+                         frag_rule(M, N, K, bits, group_size, dt);
+    return (ctx->qmv_frag == 2 || by_rule) && mtc::qmv_frag_supported(M, N, K, bits, group_size, dt, w, scales, biases, x);
+}
+
 int ensure_tc_scratch(Ctx *ctx, size_t bytes, cudaStream_t st) {
     if (bytes <= ctx->tc_scratch_bytes) return MTC_OK;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -478,6 +503,15 @@ int mtc_qmv(mtc_ctx *ctx, void *stream, const void *w, const void *scales, const
         const int t = try_qmv_tc(ctx, stream, w, scales, biases, x, outs1, 1, M, N, K, bits, group_size, dtype);
         if (t <= 0) return t;
     }
+    if (frag_takes(ctx, M, N, K, bits, group_size, dtype, w, scales, biases, x)) {
+        mtc_qmv_desc d{};
+        d.w = w; d.scales = scales; d.biases = biases; d.x = x;
+        d.outs[0] = out; d.n_outs = 1;
+        d.M = M; d.N = N; d.K = K; d.bits = bits; d.group_size = group_size; d.dtype = dtype;
+        cudaError_t e0 = mtc::launch_qmv_frag(ctx, static_cast<cudaStream_t>(stream), &d, 1);
+        if (e0 == cudaSuccess) return MTC_OK;
+        if (e0 != cudaErrorNotSupported) return fail(ctx, MTC_ERR_DISPATCH, std::string("qmv (fragments) launch: ") + cudaGetErrorString(e0));
+    }
     if (stream_takes_single(ctx, M, N, K) && mtc::qmv_stream_supported(M, N, K, bits, group_size, dtype, w, scales, biases, x)) {
         mtc_qmv_desc d{};
         d.w = w; d.scales = scales; d.biases = biases; d.x = x;
@@ -557,7 +591,7 @@ int mtc_qmv_batched(mtc_ctx *ctx, void *stream, const mtc_qmv_desc *descs, int n
     if (!ctx) return MTC_ERR_INVALID;
     MTC_ENTER(ctx);
     if (!descs || n < 1 || n > 4) return fail(ctx, MTC_ERR_INVALID, "qmv_batched: 1 to 4 projections");
-    bool fused = stream_takes(ctx, descs[0].M);
+    bool fused = stream_takes(ctx, descs[0].M), frag = true;
     for (int i = 0; i < n; ++i) {
         int rc = check_desc(ctx, descs[i], "qmv_batched");
         if (rc != MTC_OK) return rc;
@@ -565,8 +599,15 @@ int mtc_qmv_batched(mtc_ctx *ctx, void *stream, const mtc_qmv_desc *descs, int n
         if (d.x != descs[0].x || d.M != descs[0].M || d.K != descs[0].K || d.dtype != descs[0].dtype)
             return fail(ctx, MTC_ERR_INVALID, "qmv_batched: the projections must share x, M, K and dtype");
         fused = fused && d.group_size == descs[0].group_size;
+        frag = frag && d.n_outs == 1 && d.bits == descs[0].bits && d.group_size == descs[0].group_size && d.M > 0 && d.N > 0 &&
+               frag_takes(ctx, d.M, d.N, d.K, d.bits, d.group_size, d.dtype, d.w, d.scales, d.biases, d.x);
         fused = fused && d.M > 0 && d.N > 0 &&
                 mtc::qmv_stream_supported(d.M, d.N, d.K, d.bits, d.group_size, d.dtype, d.w, d.scales, d.biases, d.x);
+    }
+    if (frag) {
+        cudaError_t e = mtc::launch_qmv_frag(ctx, static_cast<cudaStream_t>(stream), descs, n);
+        if (e == cudaSuccess) return MTC_OK;
+        if (e != cudaErrorNotSupported) return fail(ctx, MTC_ERR_DISPATCH, std::string("qmv_batched (fragments) launch: ") + cudaGetErrorString(e));
     }
     if (fused) {
         cudaError_t e = mtc::launch_qmv_stream(ctx, static_cast<cudaStream_t>(stream), descs, n);
@@ -976,6 +1017,10 @@ int mtc_set_option(mtc_ctx *ctx, const char *name, int value) {
     }
     if (std::strcmp(name, "qmv_tc") == 0) {
         ctx->qmv_tc = value ? 1 : 0;
+        return MTC_OK;
+    }
+    if (std::strcmp(name, "qmv_frag") == 0) {
+        ctx->qmv_frag = value < 0 ? 0 : (value > 2 ? 2 : value);
         return MTC_OK;
     }
     if (std::strcmp(name, "qmv_stream") == 0) {
