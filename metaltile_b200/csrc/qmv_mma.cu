@@ -30,6 +30,14 @@ constexpr int kMmaWarps = 8;
 constexpr int kStageBytes = 64 * 1024;   // activations staged at a time: 64 segments (4096 k) for M <= 8, 32 for M <= 16
 constexpr int kMmaPF = 8;                // 64-code segments of packed words in flight per lane
 
+// One of the projections of a ring launch (they share x): its rows are the 16-row tiles from tile0 on.
+struct RingProj {
+    const uint32_t *w;
+    const void *scales, *biases;
+    void *out;
+    int N, tile0;
+};
+
 struct MmaArgs {
     const uint32_t *w;
     const void *scales, *biases, *x;
@@ -38,7 +46,17 @@ struct MmaArgs {
     int wpr, gpr, nseg;      // words / groups per weight row, 64-code segments per row
     int tiles, ksplit_shift, iters;
     int block_segs;          // ring kernel: segments of x staged at a time (a multiple of 8 << ksplit_shift)
+    RingProj proj[4];        // ring kernel
+    int n_proj;
 };
+
+__device__ __forceinline__ const RingProj &ring_proj(const MmaArgs &a, int tile) {
+    int i = 0;
+#pragma unroll
+    for (int j = 1; j < 4; ++j)
+        if (j < a.n_proj && tile >= a.proj[j].tile0) i = j;
+    return a.proj[i];
+}
 
 // d = a * b + (kZero ? 0 : d): m16n8k16, 16-bit operands, f32 accumulators
 template <bool BF16, bool kZero>
@@ -410,21 +428,21 @@ __global__ void __launch_bounds__(kRingWarps * 32, 1) qmv_mma_ring_kernel(const 
     // ---- copy side: lane l moves chunk (l & 15) of rows 2i + (l >> 4), i = 0..7, and 16 bytes of scales
     //      (even lanes) or biases (odd lanes) of row l >> 1.  Chunk c of row r lands at c ^ ((r & 3) << 1). ----
     const int c_row = lane >> 4, c_chunk = lane & 15, c_srow = lane >> 1;
-    const char *c_sb = static_cast<const char *>((lane & 1) ? a.biases : a.scales);
     const size_t w_pitch = static_cast<size_t>(a.wpr) * 4, sb_pitch = static_cast<size_t>(a.gpr) * 2;
     auto issue = [&](int tile, int s_run, int buf) {
         const uint32_t dst = ring + buf * kRunBytes;
-        const int row0 = tile * 16;
-        const char *src0 = reinterpret_cast<const char *>(a.w) + static_cast<size_t>(s_run) * 32 + c_chunk * 16;
+        const RingProj &pr = ring_proj(a, tile);
+        const int row0 = (tile - pr.tile0) * 16;
+        const char *src0 = reinterpret_cast<const char *>(pr.w) + static_cast<size_t>(s_run) * 32 + c_chunk * 16;
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const int row = 2 * i + c_row;
-            const int gr = min(row0 + row, a.N - 1);                    // rows past N re-read the last row
+            const int gr = min(row0 + row, pr.N - 1);                   // rows past N re-read the last row
             cp_async16(dst + row * 256 + ((c_chunk ^ ((row & 3) << 1)) << 4), src0 + gr * w_pitch);
         }
-        const int gr = min(row0 + c_srow, a.N - 1);
+        const int gr = min(row0 + c_srow, pr.N - 1);
         const uint32_t sdst = dst + kRunWBytes + (lane & 1) * 256 + c_srow * 16;
-        const char *ssrc = c_sb + gr * sb_pitch + static_cast<size_t>(s_run >> GSH) * 2;
+        const char *ssrc = static_cast<const char *>((lane & 1) ? pr.biases : pr.scales) + gr * sb_pitch + static_cast<size_t>(s_run >> GSH) * 2;
         if (GSH == 0) cp_async16(sdst, ssrc);
         else if (GSH == 1) cp_async_small<8>(sdst, ssrc);
         else cp_async_small<4>(sdst, ssrc);
@@ -595,14 +613,15 @@ __global__ void __launch_bounds__(kRingWarps * 32, 1) qmv_mma_ring_kernel(const 
             __syncthreads();   // the partial sums are rewritten by the next tile
         }
         if (active && ks == 0) {
-            const int n_lo = tile * 16 + g, n_hi = n_lo + 8;
+            const RingProj &pr = ring_proj(a, tile);
+            const int n_lo = (tile - pr.tile0) * 16 + g, n_hi = n_lo + 8;
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt) {
                 const int m0 = nt * 8 + 2 * t;
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     const int m = m0 + (q & 1), n = (q & 2) ? n_hi : n_lo;
-                    if (m < a.M && n < a.N) st_from_f32(a.out, static_cast<size_t>(m) * a.N + n, acc[nt][q], BF16 ? MTC_BF16 : MTC_F16);
+                    if (m < a.M && n < pr.N) st_from_f32(pr.out, static_cast<size_t>(m) * pr.N + n, acc[nt][q], BF16 ? MTC_BF16 : MTC_F16);
                 }
             }
         }
@@ -619,7 +638,6 @@ constexpr size_t ring_smem_bytes() {
 template <int NT, bool BF16, int GSH>
 cudaError_t launch_ring(Ctx *ctx, cudaStream_t st, MmaArgs a) {
     const int sms = ctx->sm_count;
-    a.tiles = (a.N + 15) / 16;
     int grid = a.tiles < sms ? a.tiles : sms;
     const int max_tiles = (a.tiles + grid - 1) / grid;
     // K split over the warps of a CTA: the split with the fewest runs on the busiest warp (then the fewest
@@ -714,30 +732,56 @@ bool qmv_mma_supported(int M, int N, int K, int bits, int group_size, int dt, co
            group_size >= 64 && (group_size & (group_size - 1)) == 0 && K % group_size == 0 && al(w, 16) && al(x, 16);
 }
 
-cudaError_t launch_qmv_mma(Ctx *ctx, cudaStream_t st, const void *w, const void *scales, const void *biases, const void *x,
-                           void *out, int M, int N, int K, int group_size, int dt) {
-    MmaArgs a{};
-    a.w = static_cast<const uint32_t *>(w);
-    a.scales = scales;
-    a.biases = biases;
-    a.x = x;
-    a.out = out;
-    a.M = M; a.N = N; a.K = K; a.dt = dt;
-    a.gs_shift = 0;
-    while ((1 << a.gs_shift) < group_size) ++a.gs_shift;
-    a.wpr = K / 8;
-    a.gpr = K / group_size;
-    a.nseg = K / 64;
+// ... and on the ring kernel, which several projections can share
+bool qmv_ring_supported(int M, int N, int K, int bits, int group_size, int dt, const void *w, const void *scales, const void *biases,
+                        const void *x) {
     const auto al16 = [](const void *p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
-    if (group_size <= 256 && K % 512 == 0 && al16(scales) && al16(biases)) {
+    return qmv_mma_supported(M, N, K, bits, group_size, dt, w, x) && group_size <= 256 && K % 512 == 0 && al16(scales) && al16(biases);
+}
+
+static MmaArgs mma_args(const mtc_qmv_desc &d) {
+    MmaArgs a{};
+    a.w = static_cast<const uint32_t *>(d.w);
+    a.scales = d.scales;
+    a.biases = d.biases;
+    a.x = d.x;
+    a.out = d.outs[0];
+    a.M = d.M; a.N = d.N; a.K = d.K; a.dt = d.dtype;
+    a.gs_shift = 0;
+    while ((1 << a.gs_shift) < d.group_size) ++a.gs_shift;
+    a.wpr = d.K / 8;
+    a.gpr = d.K / d.group_size;
+    a.nseg = d.K / 64;
+    return a;
+}
+
+// 1 to 4 projections that read the same activations, one launch of the ring kernel
+cudaError_t launch_qmv_ring(Ctx *ctx, cudaStream_t st, const mtc_qmv_desc *d, int n) {
+    if (n < 1 || n > 4) return cudaErrorInvalidValue;
+    MmaArgs a = mma_args(d[0]);
+    a.n_proj = n;
+    for (int i = 0; i < n; ++i) {
+        a.proj[i] = RingProj{static_cast<const uint32_t *>(d[i].w), d[i].scales, d[i].biases, d[i].outs[0], d[i].N, a.tiles};
+        a.tiles += (d[i].N + 15) / 16;
+    }
+    const int M = a.M, dt = a.dt;
 #define MTC_RING(GSH_)                                                                                              \
     if (dt == MTC_BF16) return M <= 8 ? launch_ring<1, true, GSH_>(ctx, st, a) : launch_ring<2, true, GSH_>(ctx, st, a); \
     return M <= 8 ? launch_ring<1, false, GSH_>(ctx, st, a) : launch_ring<2, false, GSH_>(ctx, st, a);
-        if (group_size == 64) { MTC_RING(0) }
-        if (group_size == 128) { MTC_RING(1) }
-        { MTC_RING(2) }
+    if (d[0].group_size == 64) { MTC_RING(0) }
+    if (d[0].group_size == 128) { MTC_RING(1) }
+    { MTC_RING(2) }
 #undef MTC_RING
-    }
+}
+
+cudaError_t launch_qmv_mma(Ctx *ctx, cudaStream_t st, const void *w, const void *scales, const void *biases, const void *x,
+                           void *out, int M, int N, int K, int group_size, int dt) {
+    mtc_qmv_desc d{};
+    d.w = w; d.scales = scales; d.biases = biases; d.x = x;
+    d.outs[0] = out; d.n_outs = 1;
+    d.M = M; d.N = N; d.K = K; d.bits = 4; d.group_size = group_size; d.dtype = dt;
+    if (qmv_ring_supported(M, N, K, 4, group_size, dt, w, scales, biases, x)) return launch_qmv_ring(ctx, st, &d, 1);
+    const MmaArgs a = mma_args(d);
     if (dt == MTC_BF16) return M <= 8 ? launch_mma<1, true>(ctx, st, a) : launch_mma<2, true>(ctx, st, a);
     return M <= 8 ? launch_mma<1, false>(ctx, st, a) : launch_mma<2, false>(ctx, st, a);
 }

@@ -591,7 +591,7 @@ int mtc_qmv_batched(mtc_ctx *ctx, void *stream, const mtc_qmv_desc *descs, int n
     if (!ctx) return MTC_ERR_INVALID;
     MTC_ENTER(ctx);
     if (!descs || n < 1 || n > 4) return fail(ctx, MTC_ERR_INVALID, "qmv_batched: 1 to 4 projections");
-    bool fused = stream_takes(ctx, descs[0].M), frag = true;
+    bool fused = stream_takes(ctx, descs[0].M), frag = true, ring = ctx->qmv_small_m_mma != 0;
     for (int i = 0; i < n; ++i) {
         int rc = check_desc(ctx, descs[i], "qmv_batched");
         if (rc != MTC_OK) return rc;
@@ -601,6 +601,8 @@ int mtc_qmv_batched(mtc_ctx *ctx, void *stream, const mtc_qmv_desc *descs, int n
         fused = fused && d.group_size == descs[0].group_size;
         frag = frag && d.n_outs == 1 && d.bits == descs[0].bits && d.group_size == descs[0].group_size && d.M > 0 && d.N > 0 &&
                frag_takes(ctx, d.M, d.N, d.K, d.bits, d.group_size, d.dtype, d.w, d.scales, d.biases, d.x);
+        ring = ring && d.n_outs == 1 && d.group_size == descs[0].group_size &&
+               mtc::qmv_ring_supported(d.M, d.N, d.K, d.bits, d.group_size, d.dtype, d.w, d.scales, d.biases, d.x);
         fused = fused && d.M > 0 && d.N > 0 &&
                 mtc::qmv_stream_supported(d.M, d.N, d.K, d.bits, d.group_size, d.dtype, d.w, d.scales, d.biases, d.x);
     }
@@ -612,6 +614,11 @@ int mtc_qmv_batched(mtc_ctx *ctx, void *stream, const mtc_qmv_desc *descs, int n
     if (fused) {
         cudaError_t e = mtc::launch_qmv_stream(ctx, static_cast<cudaStream_t>(stream), descs, n);
         if (e != cudaSuccess) return fail(ctx, MTC_ERR_DISPATCH, std::string("qmv_batched launch: ") + cudaGetErrorString(e));
+        return MTC_OK;
+    }
+    if (ring) {
+        cudaError_t e = mtc::launch_qmv_ring(ctx, static_cast<cudaStream_t>(stream), descs, n);
+        if (e != cudaSuccess) return fail(ctx, MTC_ERR_DISPATCH, std::string("qmv_batched (ring) launch: ") + cudaGetErrorString(e));
         return MTC_OK;
     }
     for (int i = 0; i < n; ++i) {

@@ -1,0 +1,78 @@
+"""The fragment kernel (option "qmv_frag" = 2) and the fused launches of the small-M kernels against the oracle.
+
+Sizes where the kernel can go wrong: rows short of and past a 16-row tile, K of one chunk (32), of a partial step (128
+codes) and of a partial run (512), slices of K shorter than the eight warps, more tiles than the grid takes in one round,
+every token count at which the layout of the columns changes, activations too large for one staged block."""
+import numpy as np
+import pytest
+
+import oracle
+from helpers import dense_case, rel_err, to_dev
+
+pytestmark = pytest.mark.gpu
+
+# |got - oracle| / max(|oracle|, 1).  Rounding a value to a significand of p bits moves it by at most half a unit in the last
+# place, 2^-p of the value (bf16: p = 8, f16: p = 11); the f32 sums on both sides add less than 2^-14 at these lengths
+# (K <= 14336 products of magnitude ~1 and random sign: sqrt(K) * 2^-24 each way, and the bias term's cancellation)
+BOUND = {"bf16": 2.0 ** -8 + 2.0 ** -14, "f16": 2.0 ** -11 + 2.0 ** -14, "f32": 2.0 ** -14}
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    from metaltile_b200 import ops
+    return ops.context(0)
+
+
+def _check(ctx, m, n, k, bits, gs, dt, seed=11):
+    import torch
+    from metaltile_b200 import ops
+    w, s, b, x = dense_case(m, n, k, bits, gs, dt, seed=seed)
+    ref = oracle.qmm(w, s, b, x, m, n, k, bits, gs)
+    ctx.set_option("qmv_frag", 2)
+    try:
+        got = ops.qmv(to_dev(w), to_dev(s, dt), to_dev(b, dt), to_dev(x, dt), bits, gs, ctx=ctx)
+    finally:
+        ctx.set_option("qmv_frag", 1)
+    torch.cuda.synchronize()
+    assert rel_err(got.float().cpu().numpy(), ref) <= BOUND[dt]
+
+
+@pytest.mark.parametrize("dt", ["bf16", "f16", "f32"])
+@pytest.mark.parametrize("bits", [2, 3, 4, 5, 6, 8])
+@pytest.mark.parametrize("n,k,gs", [(1, 32, 32), (15, 96, 32), (17, 320, 64), (33, 640, 128), (40, 1536, 64)])
+def test_edges_of_tiles_and_runs(ctx, n, k, gs, bits, dt):
+    for m in (1, 2, 3, 5):
+        _check(ctx, m, n, k, bits, gs, dt)
+
+
+@pytest.mark.parametrize("m", [1, 2, 3, 4, 5, 7, 8, 9, 16])
+@pytest.mark.parametrize("bits,gs,dt", [(4, 64, "bf16"), (4, 128, "f16"), (4, 32, "bf16"), (8, 64, "f32"), (3, 64, "bf16"), (6, 32, "f16")])
+def test_every_column_layout(ctx, bits, gs, dt, m):
+    _check(ctx, m, 50, 1024, bits, gs, dt)
+
+
+@pytest.mark.parametrize("m,n,k,bits,gs,dt", [(1, 9600, 512, 4, 64, "bf16"),       # three rounds of tiles
+                                              (8, 48, 14336, 4, 64, "bf16"),       # activations staged block by block
+                                              (16, 32, 8192, 8, 64, "bf16"), (8, 32, 4096, 8, 64, "f32")])
+def test_rounds_and_blocks(ctx, m, n, k, bits, gs, dt):
+    _check(ctx, m, n, k, bits, gs, dt)
+
+
+@pytest.mark.parametrize("m,k,bits,gs", [(1, 1024, 4, 64), (3, 1024, 4, 64), (8, 1024, 4, 128), (16, 512, 4, 64), (4, 1088, 4, 64), (5, 640, 8, 32)])
+def test_projections_in_one_launch_equal_separate_ones(ctx, m, k, bits, gs):
+    """Rows that end inside a tile in the middle of the launch: every projection has its own tiles, so the results are the
+    separate launches' bit for bit on one kernel (M = 2 to 16 on the ring kernel, else the fragment kernel)."""
+    import torch
+    from metaltile_b200 import ops
+    mats = []
+    for i, n in enumerate((100, 17, 48)):
+        w, s, b, x = dense_case(m, n, k, bits, gs, "bf16", seed=21, salt=i)
+        mats.append((to_dev(w), to_dev(s, "bf16"), to_dev(b, "bf16"), oracle.qmm(w, s, b, dense_case(m, n, k, bits, gs, "bf16", seed=21)[3], m, n, k, bits, gs)))
+    xd = to_dev(dense_case(m, 100, k, bits, gs, "bf16", seed=21)[3], "bf16")
+    got = ops.qmv_batched([t[:3] for t in mats], xd, bits, gs, ctx=ctx)
+    torch.cuda.synchronize()
+    if m == 1:
+        got = [g for g in torch.split(got, [100, 17, 48], dim=1)]
+    for g, t in zip(got, mats):
+        assert rel_err(g.float().cpu().numpy().reshape(m, -1), t[3]) <= BOUND["bf16"]
+        assert torch.equal(g.reshape(m, -1), ops.qmv(*t[:3], xd, bits, gs, ctx=ctx).reshape(m, -1))
