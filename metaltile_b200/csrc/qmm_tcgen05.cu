@@ -45,12 +45,14 @@ constexpr int TN_MAX = 256;      // token rows per tile (TMEM columns of one acc
 constexpr int MAX_STAGES = 8;    // ring depth: as many stages as fit in RING_BYTES, at most this
 constexpr int RING_BYTES = 224 * 1024;      // stages of the ring, then the raw staging buffers; SmemCtrl follows
 constexpr int SB_PER_RAW = 4;               // k blocks per raw super-block: 256 codes = 32*BITS bytes per weight row
-constexpr int RAW_SB_BYTES = 2 * BMW * 16;  // scales then biases of a super-block: 16 bytes per row each
+constexpr int RAW_SB_PITCH = 24;            // scales (and biases) of a super-block: up to 20 bytes per row
+constexpr int RAW_SB_BYTES = 2 * BMW * RAW_SB_PITCH;
+constexpr int MAX_RAW = 3;
 constexpr int A_BYTES = BMW * BK * 2;       // 16 KB, dequantised weights
-constexpr int B_BYTES = TN_MAX * BK * 2;    // 32 KB, activations
 constexpr int NUM_THREADS = 512;
 constexpr int DEQ_WARP0 = 8, DEQ_THREADS = 256;
 constexpr int EPI_WARP0 = 4;
+constexpr int COPY_WARP0 = 2, COPY_THREADS = 64;
 constexpr uint32_t kSpinLimit = 1u << 22;   // bounded waits: ~seconds, then give up
 struct QmmParams {
     const uint32_t *w;
@@ -75,13 +77,16 @@ struct QmmParams {
     int nst;                     // ring depth
     uint32_t hint_ns;            // base suspend-time hint of the waits (0: plain polling)
     int raw;                     // 1: packed words reach the dequant warps through shared memory (cp.async, whole lines)
-    uint32_t raw_off, raw_tile;  // byte offset of the raw buffers in shared memory; bytes of one tile of one buffer
+    uint32_t raw_off, raw_tile;  // byte offset of the raw buffers in shared memory; bytes of one buffer
+    int nraw;                    // raw: number of buffers (2 or 3): super-blocks are requested nraw - 1 ahead
+    int raw8;                    // raw: 1 = rows of packed words start on 8-byte boundaries only (3 / 5 bits, K an odd multiple of 64)
+    int sb_words;                // raw: 0 = a row's scales of a super-block are one aligned copy; else 4-byte words copied per row
+    long long sb_total;          // elements of the scale (and bias) array
     int wide_items;              // wide: items [0, wide_items) cover two token chunks, each later pair of items one such unit
     int wide;                    // 1: a dense item covers up to 2 TN token rows: one dequantised W stage meets two X chunks, both
                                  //    accumulators belong to the item (the dequant work per flop halves; no epilogue overlap)
     int n_tiles;                 // dense: weight-row tiles
-    int ksplit;                  // dense, one token chunk: K slices per weight-row tile (each an item of its own); 1 = none
-    int kb_per;                  // k blocks per item (K / BK / ksplit)
+    int ksplit;                  // dense, one token item per weight-row tile: K slices (each an item of its own); 1 = none
     float *partial;              // ksplit > 1: f32 partial sums [ksplit][M][N], added by ksplit_sum_kernel
     int pdl_roles;               // programmatic dependent launch: 1 = only the roles that touch what an earlier kernel of the
                                  //    stream may have written (producer: x; epilogue: token factors, out) wait for it, the
@@ -94,7 +99,8 @@ struct __align__(8) SmemCtrl {
     uint64_t empty[MAX_STAGES];  // MMAs that read the stage have completed
     uint64_t acc_full[2];        // accumulator buffer complete
     uint64_t acc_empty[2];       // epilogue drained the accumulator buffer
-    uint64_t raw_full[2];        // every dequant warp's copies of a raw super-block have landed
+    uint64_t raw_full[MAX_RAW];  // the copies of a raw super-block have landed
+    uint64_t raw_empty[MAX_RAW]; // every dequant warp has read it
     uint32_t tmem_base;
     volatile uint32_t abort;
 };
@@ -145,19 +151,24 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, SmemCt
     atomicCAS(status, 0u, code);
     return false;
 }
-// Whole-warp wait: lane 0 polls, the result is broadcast.
+// Whole-warp wait.  All lanes poll together, one instruction for the warp: with lane 0 polling and broadcasting, the other
+// lanes' yields and the reconvergence after every poll were on the path of every hand-off.
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t parity, SmemCtrl *ctl, uint32_t *status, uint32_t code,
                                                uint32_t sleep_ns) {
-    uint32_t ok = 1;
-    if ((threadIdx.x & 31) == 0) ok = mbar_wait(bar, parity, ctl, status, code, sleep_ns) ? 1u : 0u;
-    ok = __shfl_sync(0xffffffffu, ok, 0);
-    return ok != 0;
+    const bool ok = mbar_wait(bar, parity, ctl, status, code, sleep_ns);
+    return __all_sync(0xffffffffu, ok);
 }
 
 __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, int c0, int c1, uint64_t *bar) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
         ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(smem_u32(bar)) : "memory");
+}
+
+__device__ __forceinline__ void tma_load_2d_at(uint32_t dst, const CUtensorMap *map, int c0, int c1, uint64_t *bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+        ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(smem_u32(bar)) : "memory");
 }
 
 // Shared-memory matrix descriptor: K-major operand, 128-byte swizzle, 8-row atoms 1024 B apart.
@@ -358,17 +369,56 @@ __device__ __forceinline__ uint32_t sb_half(const uint4 &v, int j, int h, int gs
     return (w[0] >> (16 * ((j >> 1) & 1))) & 0xFFFFu;
 }
 
+// One super-block of a weight tile as it lies in a raw buffer: the packed words of 128 rows, then the scales, then the biases.
+// 4 and 8 bits: TMA boxes of 128 bytes x 128 rows with the 128-byte swizzle; other widths: rows padded by 16 bytes.
+template <int BITS>
+struct RawTile {
+    static constexpr bool TMA = BITS == 4 || BITS == 8;
+    static constexpr int ROW_BYTES = 32 * BITS, PITCH = ROW_BYTES + 16;
+    static constexpr int SB_OFF = TMA ? BMW * ROW_BYTES : BMW * PITCH;
+    static constexpr int BYTES = SB_OFF + RAW_SB_BYTES;
+    // the 32 codes of k block j, half h of row r
+    static __device__ __forceinline__ void read(uint32_t base, int r, int j, int h, uint32_t (&w)[BITS]) {
+        if constexpr (TMA) {
+#pragma unroll
+            for (int q = 0; q < BITS / 4; ++q) {
+                const int c = (2 * j + h) * (BITS / 4) + q;          // 16-byte chunk of the row
+                const uint32_t a = base + (c >> 3) * (BMW * 128) + r * 128 + (((c & 7) ^ (r & 7)) << 4);
+                asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(w[4 * q]), "=r"(w[4 * q + 1]), "=r"(w[4 * q + 2]), "=r"(w[4 * q + 3]) : "r"(a));
+            }
+        } else {
+            lds_words<BITS>(base + r * PITCH + (2 * j + h) * (4 * BITS), w);
+        }
+    }
+};
+int raw_bytes(int bits) { return (bits == 4 || bits == 8 ? BMW * 32 * bits : BMW * (32 * bits + 16)) + RAW_SB_BYTES; }
+
 struct Item {
     int n_tile, expert, row0, rows;
     int nc;                                 // token chunks of TN rows covered (1 or 2): one accumulator each
-    int kb0, ks;                            // first k block and index of the K slice (0, 0 unless the launch splits K)
+    int kb0, nkb, ks;                       // first k block, k blocks and index of the K slice (0, all, 0 unless the launch splits K)
 };
 
 template <bool KSPLIT>
 __device__ __forceinline__ Item get_item(const QmmParams &p, int i) {
     Item it;
     it.kb0 = 0;
+    it.nkb = p.K / BK;
     it.ks = 0;
+    if (KSPLIT) {
+        // K slices of a tile are adjacent items: whole super-blocks, as even as they come, against all token rows
+        it.n_tile = i / p.ksplit;
+        it.ks = i - it.n_tile * p.ksplit;
+        const int nsb = (it.nkb + SB_PER_RAW - 1) / SB_PER_RAW;
+        const int sb0 = it.ks * nsb / p.ksplit, sb1 = (it.ks + 1) * nsb / p.ksplit;
+        it.kb0 = sb0 * SB_PER_RAW;
+        it.nkb = min(sb1 * SB_PER_RAW, it.nkb) - it.kb0;
+        it.expert = 0;
+        it.row0 = 0;
+        it.rows = p.M;
+        it.nc = p.M > p.TN ? 2 : 1;
+        return it;
+    }
     if (p.items) {
         const int4 v = __ldg(p.items + i);
         it.n_tile = v.x; it.expert = v.y & 0xFFFFFF; it.row0 = v.z; it.rows = v.w;
@@ -389,13 +439,7 @@ __device__ __forceinline__ Item get_item(const QmmParams &p, int i) {
     } else {
         // dense: the token chunks of one weight-row tile are adjacent, so CTAs running at the same time share its
         // packed words in L2
-        // K slices of one tile are adjacent items too
-        const int b = KSPLIT ? i / p.ksplit : i;
-        if (KSPLIT) {
-            it.ks = i - b * p.ksplit;
-            it.kb0 = it.ks * p.kb_per;
-        }
-        const int unit = b / p.m_chunks, chunk = b - unit * p.m_chunks;
+        const int unit = i / p.m_chunks, chunk = i - unit * p.m_chunks;
         it.nc = 1;
         it.expert = 0;
         it.n_tile = unit;
@@ -409,7 +453,7 @@ __device__ __forceinline__ Item get_item(const QmmParams &p, int i) {
 // separate instantiation, so that the code of every other launch is what it was without the feature.
 template <int BITS, bool KSPLIT>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
-qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const QmmParams p) {
+qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w, const QmmParams p) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
     const int nst = p.nst;
@@ -421,7 +465,6 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const QmmParams p
     SmemCtrl *ctl = reinterpret_cast<SmemCtrl *>(smem + RING_BYTES);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int num_kb = KSPLIT ? p.kb_per : p.K / BK;       // k blocks per item
     const int num_items = p.items ? __ldg(p.item_count) : p.dense_items;
     const uint32_t x_bytes = static_cast<uint32_t>(p.TN) * BK * 2;
 
@@ -433,7 +476,10 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const QmmParams p
         for (int b = 0; b < 2; ++b) {
             mbar_init(&ctl->acc_full[b], 1);
             mbar_init(&ctl->acc_empty[b], 4);
-            mbar_init(&ctl->raw_full[b], DEQ_THREADS / 32);
+        }
+        for (int b = 0; b < MAX_RAW; ++b) {
+            mbar_init(&ctl->raw_full[b], COPY_THREADS + 1);
+            mbar_init(&ctl->raw_empty[b], DEQ_THREADS / 32);
         }
         ctl->abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -458,7 +504,7 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const QmmParams p
             if (p.pdl_roles) asm volatile("griddepcontrol.wait;" ::: "memory");      // x may come from the previous kernel
             for (int i = blockIdx.x; i < num_items && ok; i += gridDim.x) {
                 const Item item = get_item<KSPLIT>(p, i);
-                for (int kb = 0; kb < num_kb; ++kb) {
+                for (int kb = 0; kb < item.nkb; ++kb) {
                     if (!(ok = mbar_wait(&ctl->empty[s], ph ^ 1, ctl, p.status, 0x101, p.hint_ns))) break;
                     mbar_expect_tx(&ctl->full[s], x_bytes * item.nc);
                     for (int c = 0; c < item.nc; ++c)
@@ -499,7 +545,7 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const QmmParams p
                 if (!(ok = mbar_wait_warp(&ctl->acc_empty[buf], acc_ph ^ 1, ctl, p.status, 0x201, 0))) break;
                 tc_fence_after();
                 const uint32_t tmem_d = tmem_base + buf * TN_MAX;
-                for (int kb = 0; kb < num_kb; ++kb) {
+                for (int kb = 0; kb < item.nkb; ++kb) {
                     if (!(ok = mbar_wait_warp(&ctl->full[s], ph, ctl, p.status, 0x202, 0))) break;
                     tc_fence_after();
                     if (leader) {
@@ -521,6 +567,101 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const QmmParams p
                 }
                 if (ok && leader) umma_commit(&ctl->acc_full[buf]);
                 __syncwarp();
+            }
+        }
+    } else if (warp >= COPY_WARP0 && warp < COPY_WARP0 + COPY_THREADS / 32) {
+        // ---------------- copies: packed words and scales -> raw buffers ----------------
+        // A super-block of 4 k blocks of the tile at a time, up to nraw ahead of the dequant warps and across items.  4- and
+        // 8-bit words are one or two TMA boxes (128 bytes x 128 rows, swizzled so that the rows' reads do not conflict);
+        // other widths and all scales are cp.async copies of these two warps.  Issued by the dequant warps themselves the
+        // copies cost them 380 of ~1050 cycles a k block, and 150 more behind the queue they filled.
+        if (p.raw) {
+            using R = RawTile<BITS>;
+            const int t = threadIdx.x - COPY_WARP0 * 32;
+            const uint32_t raw0 = smem_u32(smem) + p.raw_off;
+            const int sb_bytes = (2 * SB_PER_RAW * BK) >> p.gs_shift;       // scale bytes of a row per super-block: 16, 8 or 4
+            int buf = 0;
+            uint32_t ph = 0;
+            bool ok = true;
+            for (int i = blockIdx.x; i < num_items && ok; i += gridDim.x) {
+                const Item im = get_item<KSPLIT>(p, i);
+                const int n0 = im.n_tile * BMW;
+                const size_t erow = static_cast<size_t>(im.expert) * p.N;
+                const int sb0 = (KSPLIT ? im.kb0 : 0) / SB_PER_RAW, sb1 = sb0 + (im.nkb + SB_PER_RAW - 1) / SB_PER_RAW;
+                for (int sbk = sb0; sbk < sb1; ++sbk) {
+                    if (!(ok = mbar_wait_warp(&ctl->raw_empty[buf], ph ^ 1, ctl, p.status, 0x501, p.hint_ns))) break;
+                    const uint32_t dstt = raw0 + buf * p.raw_tile;
+                    if constexpr (R::TMA) {
+                        if (t == 0) {
+                            mbar_expect_tx(&ctl->raw_full[buf], R::SB_OFF);
+                            // rows past the array and words past the row arrive as zeros; rows past N are never stored
+#pragma unroll
+                            for (int q = 0; q < BITS / 4; ++q)
+                                tma_load_2d_at(dstt + q * (BMW * 128), &tmap_w, sbk * (8 * BITS) + q * 32, static_cast<int>(erow) + n0, &ctl->raw_full[buf]);
+                        }
+                    } else {
+                        if (t == 0) mbar_arrive(&ctl->raw_full[buf]);
+                        const int bytes = min(SB_PER_RAW, p.K / BK - sbk * SB_PER_RAW) * (8 * BITS);   // the last one of a row may be short
+                        const char *src = reinterpret_cast<const char *>(p.w) + static_cast<size_t>(sbk) * R::ROW_BYTES;
+                        if (!p.raw8) {
+                            constexpr int CPR = 2 * BITS;
+#pragma unroll 4
+                            for (int ch = t; ch < BMW * CPR; ch += COPY_THREADS) {
+                                const int row = ch / CPR, col = ch - row * CPR;
+                                const size_t grow = erow + min(n0 + row, p.N - 1);          // rows past N copy the last row; never stored
+                                if (col * 16 < bytes) cp_async_16(dstt + row * R::PITCH + col * 16, src + grow * (p.wpr * 4) + col * 16);
+                            }
+                        } else {
+                            constexpr int CPR = 4 * BITS;
+#pragma unroll 4
+                            for (int ch = t; ch < BMW * CPR; ch += COPY_THREADS) {
+                                const int row = ch / CPR, col = ch - row * CPR;
+                                const size_t grow = erow + min(n0 + row, p.N - 1);
+                                if (col * 8 < bytes) cp_async_small<8>(dstt + row * R::PITCH + col * 8, src + grow * (p.wpr * 4) + col * 8);
+                            }
+                        }
+                    }
+                    const uint32_t d = dstt + R::SB_OFF;
+                    if (p.sb_words == 0) {
+#pragma unroll
+                        for (int e = 0; e < 2 * BMW / COPY_THREADS; ++e) {
+                            const int row = (e * COPY_THREADS + t) & (BMW - 1), arr = e >> 1;
+                            const size_t grow = erow + min(n0 + row, p.N - 1);
+                            const char *src = static_cast<const char *>(arr ? p.biases : p.scales) + (grow * p.gpr) * 2 + static_cast<size_t>(sbk) * sb_bytes;
+                            const uint32_t dd = d + arr * (BMW * 16) + row * 16;            // 16-byte pitch: one aligned copy
+                            if (sb_bytes == 16) cp_async_16(dd, src);
+                            else if (sb_bytes == 8) cp_async_small<8>(dd, src);
+                            else cp_async_small<4>(dd, src);
+                        }
+                    } else {
+                        // rows of scales start anywhere: the 4-byte words that cover the super-block's, neighbouring lanes on
+                        // neighbouring words; the element that ends the array alone in its word is copied by itself
+                        const int nw = p.sb_words;
+                        for (int e = t; e < 2 * BMW * nw; e += COPY_THREADS) {
+                            const int rowa = e / nw, wd = e - rowa * nw, arr = rowa >> 7, row = rowa & (BMW - 1);
+                            const size_t grow = erow + min(n0 + row, p.N - 1);
+                            const long long el = static_cast<long long>(((grow * p.gpr + static_cast<size_t>(sbk) * (sb_bytes / 2)) & ~static_cast<size_t>(1)) + 2 * wd);
+                            const unsigned short *base = static_cast<const unsigned short *>(arr ? p.biases : p.scales);
+                            const uint32_t dd = d + rowa * RAW_SB_PITCH + wd * 4;
+                            if (el + 1 < p.sb_total) {
+                                cp_async_small<4>(dd, base + el);
+                            } else if (el < p.sb_total) {
+                                asm volatile("st.shared.u16 [%0], %1;" ::"r"(dd), "h"(__ldg(base + el)) : "memory");
+                                __threadfence_block();
+                            }
+                        }
+                    }
+                    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&ctl->raw_full[buf])) : "memory");
+                    if (++buf == p.nraw) {
+                        buf = 0;
+                        ph ^= 1;
+                    }
+                }
+            }
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            if (!ok && R::TMA) {   // let copies already in flight land before the CTA tears down
+                for (int b = 0; b < p.nraw; ++b)
+                    for (uint32_t j = 0; j < 4096 && !mbar_try(&ctl->raw_full[b], 0) && !mbar_try(&ctl->raw_full[b], 1); ++j) {}
             }
         }
     } else if (warp >= EPI_WARP0 && warp < EPI_WARP0 + 4) {
@@ -591,79 +732,49 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const QmmParams p
         uint32_t ph = 0;                                  // stage and ring-pass parity, advanced without a division
         bool ok = true;
         if (p.raw) {
-            // Packed words through shared memory.  A thread that loads its own row's 16 bytes per k block makes
-            // every warp-load touch 32 cache lines (plus 64 for the scale and the bias): measured, the L1 tag stage,
-            // not the arithmetic, set the pace of a k block (0.8 us whatever the tile width or the ring depth).  Here
-            // the 256 dequant threads copy a super-block of 4 k blocks of the tile - 32*BITS contiguous bytes per
-            // row, 16 bytes per thread and copy, two rows per warp-copy - with cp.async into one of two raw
-            // buffers, one super-block ahead and across items, and read their pieces back from shared memory.
-            constexpr int ROW_BYTES = 32 * BITS, PITCH = ROW_BYTES + 16, CPR = 2 * BITS;   // padded rows: conflict-free reads
+            // packed words and scales through the raw buffers that the copy warps fill
+            using R = RawTile<BITS>;
             const uint32_t raw0 = smem_u32(smem) + p.raw_off;
-            const uint32_t buf_bytes = p.raw_tile;
-            const int num_sb = num_kb / SB_PER_RAW;
-            const int sb_bytes = (2 * SB_PER_RAW * BK) >> p.gs_shift;       // scale bytes of a row per super-block: 16, 8 or 4
-            const int srow = t & (BMW - 1), sarr = t >> 7;                  // this thread copies scales (0) or biases (1) of a row
-            auto issue = [&](const Item &im, int sb_rel, int buf) {
-                const int sbk = (KSPLIT ? im.kb0 / SB_PER_RAW : 0) + sb_rel;      // super-block of the row
-                const uint32_t dstt = raw0 + buf * buf_bytes;
-                const int n0 = im.n_tile * BMW;
-                const size_t erow = static_cast<size_t>(im.expert) * p.N;
-#pragma unroll
-                for (int c = 0; c < BITS; ++c) {
-                    const int ch = c * DEQ_THREADS + t, row = ch / CPR, col = ch - row * CPR;
-                    const size_t grow = erow + min(n0 + row, p.N - 1);          // rows past N copy the last row; never stored
-                    cp_async_16(dstt + row * PITCH + col * 16,
-                                reinterpret_cast<const char *>(p.w + grow * p.wpr) + static_cast<size_t>(sbk) * ROW_BYTES + col * 16);
-                }
-                const size_t grow = erow + min(n0 + srow, p.N - 1);
-                const char *src = static_cast<const char *>(sarr ? p.biases : p.scales) + (grow * p.gpr) * 2 +
-                                  static_cast<size_t>(sbk) * sb_bytes;
-                const uint32_t d = dstt + BMW * PITCH + sarr * (BMW * 16) + srow * 16;
-                if (sb_bytes == 16) cp_async_16(d, src);
-                else if (sb_bytes == 8) cp_async_small<8>(d, src);
-                else cp_async_small<4>(d, src);
-            };
-            // request stream: (item, super-block) pairs in processing order
-            int i_n = blockIdx.x, sb_n = 0;
-            Item item_n{};
-            if (i_n < num_items) {
-                item_n = get_item<KSPLIT>(p, i_n);
-                issue(item_n, 0, 0);
-            }
-            asm volatile("cp.async.commit_group;" ::: "memory");
-            uint32_t q = 0;
+            const int nraw = p.nraw;
+            const int sb_elems = (SB_PER_RAW * BK) >> p.gs_shift;           // scales of a row per super-block: 8, 4 or 2
+            int buf = 0;
+            uint32_t buf_ph = 0;
             for (int i = blockIdx.x; i < num_items && ok; i += gridDim.x) {
                 const Item item = get_item<KSPLIT>(p, i);
-                for (int sbk = 0; sbk < num_sb && ok; ++sbk, ++q) {
-                    const int buf = q & 1;
-                    // this super-block has landed: my copies, then every warp's (which also says that every warp is
-                    // done reading the other buffer)
-                    asm volatile("cp.async.wait_group 0;" ::: "memory");
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&ctl->raw_full[buf]);
-                    if (!(ok = mbar_wait_warp(&ctl->raw_full[buf], (q >> 1) & 1, ctl, p.status, 0x402, 0))) break;
-                    // the next one, into the other buffer
-                    if (++sb_n == num_sb) {
-                        sb_n = 0;
-                        i_n += gridDim.x;
-                        if (i_n < num_items) item_n = get_item<KSPLIT>(p, i_n);
-                    }
-                    if (i_n < num_items) issue(item_n, sb_n, buf ^ 1);
-                    asm volatile("cp.async.commit_group;" ::: "memory");
-                    // the row's scales and biases of the whole super-block: one 16-byte load each (4, 8 or 16 bytes are in use)
+                for (int kb0 = 0; kb0 < item.nkb && ok; kb0 += SB_PER_RAW) {
+                    if (!(ok = mbar_wait_warp(&ctl->raw_full[buf], buf_ph, ctl, p.status, 0x402, 0))) break;
+                    const uint32_t base = raw0 + buf * p.raw_tile;
+                    // the row's scales and biases of the whole super-block (4, 8 or 16 bytes are in use)
                     uint4 sline, bline;
-                    {
-                        const uint32_t sb_addr = raw0 + buf * buf_bytes + BMW * PITCH + r * 16;
+                    if (p.sb_words == 0) {
+                        const uint32_t sb_addr = base + R::SB_OFF + r * 16;
                         asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(sline.x), "=r"(sline.y), "=r"(sline.z), "=r"(sline.w) : "r"(sb_addr));
                         asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(bline.x), "=r"(bline.y), "=r"(bline.z), "=r"(bline.w) : "r"(sb_addr + BMW * 16));
+                    } else {
+                        const size_t grow = static_cast<size_t>(item.expert) * p.N + min(item.n_tile * BMW + r, p.N - 1);
+                        const int sbk = ((KSPLIT ? item.kb0 : 0) + kb0) / SB_PER_RAW;
+                        const int sh = static_cast<int>((grow * p.gpr + static_cast<size_t>(sbk) * sb_elems) & 1) * 16;
+                        uint32_t v[2][5];
+#pragma unroll
+                        for (int arr = 0; arr < 2; ++arr)
+#pragma unroll
+                            for (int j = 0; j < 5; ++j) {
+                                v[arr][j] = 0u;
+                                if (j < p.sb_words)
+                                    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v[arr][j]) : "r"(base + R::SB_OFF + (arr * BMW + r) * RAW_SB_PITCH + j * 4));
+                            }
+                        sline = make_uint4(__funnelshift_r(v[0][0], v[0][1], sh), __funnelshift_r(v[0][1], v[0][2], sh),
+                                           __funnelshift_r(v[0][2], v[0][3], sh), __funnelshift_r(v[0][3], v[0][4], sh));
+                        bline = make_uint4(__funnelshift_r(v[1][0], v[1][1], sh), __funnelshift_r(v[1][1], v[1][2], sh),
+                                           __funnelshift_r(v[1][2], v[1][3], sh), __funnelshift_r(v[1][3], v[1][4], sh));
                     }
 #pragma unroll
                     for (int j = 0; j < SB_PER_RAW; ++j) {
+                        if (kb0 + j >= item.nkb) break;
+                        uint32_t wv[BITS];                   // read before the wait for the stage
+                        R::read(base, r, j, h, wv);
                         if (!(ok = mbar_wait_warp(&ctl->empty[s], ph ^ 1, ctl, p.status, 0x401, 0))) break;
                         {
-                            const uint32_t base = raw0 + buf * buf_bytes;
-                            uint32_t wv[BITS];
-                            lds_words<BITS>(base + r * PITCH + (2 * j + h) * (4 * BITS), wv);
                             const unsigned short sr = static_cast<unsigned short>(sb_half(sline, j, h, p.gs_shift));
                             const unsigned short br = static_cast<unsigned short>(sb_half(bline, j, h, p.gs_shift));
                             float sc, bi;
@@ -684,9 +795,14 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const QmmParams p
                             ph ^= 1;
                         }
                     }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&ctl->raw_empty[buf]);
+                    if (++buf == nraw) {
+                        buf = 0;
+                        buf_ph ^= 1;
+                    }
                 }
             }
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
         } else
         for (int i = blockIdx.x; i < num_items && ok; i += gridDim.x) {
             const Item item = get_item<KSPLIT>(p, i);
@@ -708,12 +824,12 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const QmmParams p
             };
             const int kb0 = KSPLIT ? item.kb0 : 0;
             request(kb0);
-            for (int kb = 0; kb < num_kb; ++kb) {
+            for (int kb = 0; kb < item.nkb; ++kb) {
                 uint32_t wcur[BITS];
 #pragma unroll
                 for (int j = 0; j < BITS; ++j) wcur[j] = wnext[j];
                 const uint32_t sr = sn, br = bn;
-                if (kb + 1 < num_kb) request(kb0 + kb + 1);      // the next k block is requested before this one is converted
+                if (kb + 1 < item.nkb) request(kb0 + kb + 1);      // the next k block is requested before this one is converted
                 // the stage is free once empty[s] has completed (the producer waits on the same barrier)
                 if (!(ok = mbar_wait_warp(&ctl->empty[s], ph ^ 1, ctl, p.status, 0x401, 0))) break;
                 float sc, bi;
@@ -857,7 +973,7 @@ constexpr size_t qmm_smem_bytes() {
 }
 
 template <int BITS>
-cudaError_t launch_bits(cudaStream_t st, const CUtensorMap &tmap, const QmmParams &p, int grid) {
+cudaError_t launch_bits(cudaStream_t st, const CUtensorMap &tmap, const CUtensorMap &wmap, const QmmParams &p, int grid) {
     constexpr size_t smem = qmm_smem_bytes<BITS>();
     static_assert(smem <= 227 * 1024, "shared memory per CTA");
     cudaLaunchConfig_t cfg{};
@@ -875,24 +991,13 @@ cudaError_t launch_bits(cudaStream_t st, const CUtensorMap &tmap, const QmmParam
         static PerDeviceAttr attr;
         cudaError_t e = attr.set(kern, smem);
         if (e != cudaSuccess) return e;
-        return cudaLaunchKernelEx(&cfg, kern, tmap, p);
+        return cudaLaunchKernelEx(&cfg, kern, tmap, wmap, p);
     }
     auto kern = qmm_tcgen05_kernel<BITS, false>;
     static PerDeviceAttr attr;
     cudaError_t e = attr.set(kern, smem);
     if (e != cudaSuccess) return e;
-    return cudaLaunchKernelEx(&cfg, kern, tmap, p);
-}
-
-cudaError_t launch_any(int bits, cudaStream_t st, const CUtensorMap &tmap, const QmmParams &p, int grid) {
-    switch (bits) {
-        case 2: return launch_bits<2>(st, tmap, p, grid);
-        case 3: return launch_bits<3>(st, tmap, p, grid);
-        case 4: return launch_bits<4>(st, tmap, p, grid);
-        case 5: return launch_bits<5>(st, tmap, p, grid);
-        case 6: return launch_bits<6>(st, tmap, p, grid);
-        default: return launch_bits<8>(st, tmap, p, grid);
-    }
+    return cudaLaunchKernelEx(&cfg, kern, tmap, wmap, p);
 }
 
 // X as a 2-D tensor [rows, K] of 16-bit elements, box 64 x TN, 128-byte swizzle; rows past the end read as zero.
@@ -916,17 +1021,52 @@ cudaError_t make_x_map(CUtensorMap *tmap, const void *x, int rows, int K, int TN
     return cudaSuccess;
 }
 
-// Ring depth and raw staging buffers for p.TN / p.wide.  The raw path needs whole super-blocks (K % 256 == 0), 4 to 16
-// bytes of scales per row and super-block (group 32, 64 or 128) and 16-byte aligned scale / bias arrays; it takes
-// two buffers per weight tile out of the ring, which costs nothing: measured, a ring deeper than 2 stages does not
-// change the time of any shape.
+// Packed words as a 2-D tensor [rows, words], box 128 bytes x 128 rows, 128-byte swizzle
+cudaError_t make_w_map(CUtensorMap *tmap, const QmmParams &p, long long rows, std::string *why) {
+    EncodeTiledFn encode = get_encode_fn();
+    if (!encode) return cudaErrorNotSupported;          // make_x_map has said why
+    const cuuint64_t dims[2] = {static_cast<cuuint64_t>(p.wpr), static_cast<cuuint64_t>(rows)};
+    const cuuint64_t strides[1] = {static_cast<cuuint64_t>(p.wpr) * 4};
+    const cuuint32_t box[2] = {32, BMW};
+    const cuuint32_t estr[2] = {1, 1};
+    CUresult r = encode(tmap, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<uint32_t *>(p.w), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) {
+        if (why) *why = "cuTensorMapEncodeTiled failed with code " + std::to_string(static_cast<int>(r));
+        return cudaErrorInvalidValue;
+    }
+    return cudaSuccess;
+}
+
+cudaError_t launch_any(int bits, cudaStream_t st, const CUtensorMap &tmap, const QmmParams &p, int grid, long long w_rows, std::string *why) {
+    CUtensorMap wmap = tmap;                            // not read where the words do not travel by TMA
+    if (p.raw && (bits == 4 || bits == 8)) {
+        cudaError_t e = make_w_map(&wmap, p, w_rows, why);
+        if (e != cudaSuccess) return e;
+    }
+    switch (bits) {
+        case 2: return launch_bits<2>(st, tmap, wmap, p, grid);
+        case 3: return launch_bits<3>(st, tmap, wmap, p, grid);
+        case 4: return launch_bits<4>(st, tmap, wmap, p, grid);
+        case 5: return launch_bits<5>(st, tmap, wmap, p, grid);
+        case 6: return launch_bits<6>(st, tmap, wmap, p, grid);
+        default: return launch_bits<8>(st, tmap, wmap, p, grid);
+    }
+}
+
+// Ring depth and raw staging buffers for p.TN / p.wide.  The raw path needs groups of 32, 64 or 128 (4 to 16 bytes of scales per
+// row and super-block) and 4-byte aligned scale / bias arrays.  Rows of scales that are whole super-blocks arrive as one
+// copy per row, others (K % 256 != 0) word by word.  A third raw buffer is taken where three ring stages remain.
 void plan_smem(QmmParams &p, Ctx *ctx, int bits) {
     const int stage = A_BYTES + (p.wide ? 2 : 1) * p.TN * BK * 2;
-    const auto al16 = [](const void *ptr) { return reinterpret_cast<uintptr_t>(ptr) % 16 == 0; };
-    p.raw_tile = static_cast<uint32_t>(BMW * (32 * bits + 16) + RAW_SB_BYTES);
-    const int raw_total = 2 * static_cast<int>(p.raw_tile);
-    p.raw = ctx->qmm_raw != 0 && p.K % (SB_PER_RAW * BK) == 0 && p.gs_shift >= 5 && p.gs_shift <= 7 && al16(p.scales) &&
-            al16(p.biases) && (RING_BYTES - raw_total) / stage >= 2;
+    const auto al = [](const void *ptr, size_t n) { return reinterpret_cast<uintptr_t>(ptr) % n == 0; };
+    p.raw_tile = static_cast<uint32_t>(raw_bytes(bits));
+    p.nraw = RING_BYTES - 3 * static_cast<int>(p.raw_tile) >= 3 * stage ? 3 : 2;
+    const int raw_total = p.nraw * static_cast<int>(p.raw_tile);
+    p.raw = ctx->qmm_raw != 0 && p.gs_shift >= 5 && p.gs_shift <= 7 && al(p.scales, 4) && al(p.biases, 4) &&
+            (RING_BYTES - raw_total) / stage >= 2;
+    p.raw8 = (p.wpr * 4) % 16 != 0;
+    p.sb_words = p.K % (SB_PER_RAW * BK) == 0 && al(p.scales, 16) && al(p.biases, 16) ? 0 : ((2 * SB_PER_RAW * BK) >> p.gs_shift) / 4 + (p.gpr & 1);
     p.nst = (RING_BYTES - (p.raw ? raw_total : 0)) / stage;
     if (p.nst > MAX_STAGES) p.nst = MAX_STAGES;
     if (ctx->qmm_max_stages > 0 && p.nst > ctx->qmm_max_stages) p.nst = ctx->qmm_max_stages;
@@ -954,7 +1094,7 @@ void fill_common(QmmParams &p, Ctx *ctx, const void *w, const void *scales, cons
     p.TN = TN;
     p.wide = 0;
     p.ksplit = 1;
-    p.kb_per = K / BK;
+    p.sb_total = static_cast<long long>(N) * p.gpr;          // a gather launch multiplies by its experts
     p.partial = nullptr;
     p.pdl_roles = 0;               // the dense launcher turns it on: a gather launch reads a work list the previous kernel built
     plan_smem(p, ctx, bits);
@@ -981,6 +1121,54 @@ cudaError_t stage_x(Ctx *ctx, cudaStream_t st, const void *x, int rows, int K, i
     *x_op = y;
     *tok_scale = scale;
     return cudaSuccess;
+}
+
+// Time of a k block of an item on one SM by its token rows, us (measured): the dequantisation sets the pace of narrow items.
+constexpr double kKbBase = 0.40, kKbPerToken = 0.0010;
+constexpr double kItemUs = 0.4;         // a further item on the same SM: its accumulators drain before the next pair starts
+
+// How a dense launch covers its M token rows: items of one chunk (TN rows, one accumulator) or of two (the dequantised W stage
+// is built once for both), chunks of equal width (333 rows are 2 x 176, not 256 + 77), and K slices where the items alone
+// would leave SMs idle.  Every form is priced by the rounds of the grid it takes.
+struct DensePlan {
+    int TN, items_m, ksplit, halves;      // halves: wide items of an incomplete last round that run as two single-chunk items each
+    bool wide;
+};
+DensePlan plan_dense(const Ctx *ctx, int M, int N, int K, int bits, bool may_split) {
+    const int n_tiles = (N + BMW - 1) / BMW, nkb = K / BK, nsb = (nkb + SB_PER_RAW - 1) / SB_PER_RAW, sms = ctx->sm_count;
+    const auto up16 = [](int v) { return (v + 15) / 16 * 16; };
+    if (ctx->qmm_force_tn > 0) return DensePlan{ctx->qmm_force_tn, (M + ctx->qmm_force_tn - 1) / ctx->qmm_force_tn, 1, 0, false};
+    // two ring stages of one W and two X chunks beside two raw buffers
+    const int raw_total = 2 * raw_bytes(bits);
+    int tn_wide = ((RING_BYTES - raw_total) / 2 - A_BYTES) / (2 * BK * 2) / 16 * 16;
+    if (tn_wide > TN_MAX) tn_wide = TN_MAX;
+    DensePlan best{};
+    double best_us = 1e30;
+    for (int form = 0; form < 2; ++form) {                     // 0: one chunk per item, 1: two
+        if (form == 1 && (!ctx->qmm_wide || M <= TN_MAX)) continue;
+        if (form == 0 && ctx->qmm_wide == 2 && M > TN_MAX) continue;                 // 2: whenever the shape allows (tests)
+        const int most = form == 1 ? 2 * tn_wide : TN_MAX;
+        const int items_m = (M + most - 1) / most;
+        const int TN = form == 1 ? up16((M + 2 * items_m - 1) / (2 * items_m)) : up16((M + items_m - 1) / items_m);
+        const double one = kKbBase + kKbPerToken * TN, kb_us = form == 1 ? kKbBase + kKbPerToken * 2 * TN : one;
+        const long long units = static_cast<long long>(n_tiles) * items_m;
+        // the last round of wide items on twice as many SMs, a chunk each, where that still is one round and every unit has two
+        const int left = static_cast<int>(units % sms), last_rows = M - (items_m - 1) * 2 * TN;
+        const bool tail = form == 1 && units > sms && left > 0 && 2 * left <= sms && last_rows > TN;
+        for (int S = 1; S <= 16; ++S) {
+            if (S > 1 && (!ctx->qmm_ksplit || !may_split || items_m > 1 || S > nsb || (form == 1 && ctx->qmm_wide == 2))) break;
+            const int kb = S == 1 ? nkb : (nsb + S - 1) / S * SB_PER_RAW;
+            const long long full = units * S / sms, rest = units * S % sms;
+            double us = full * (kb * kb_us + kItemUs);
+            if (rest > 0) us += (S == 1 && tail ? kb * one : kb * kb_us) + kItemUs;
+            if (S > 1) us += 2.0 + static_cast<double>(S) * M * N * 8 / 6e6;
+            if (us < best_us - 1e-9) {
+                best_us = us;
+                best = DensePlan{TN, items_m, S, S == 1 && tail ? left : 0, form == 1};
+            }
+        }
+    }
+    return best;
 }
 
 // out[i] = sum over the K slices of partial[s][i], in slice order
@@ -1011,7 +1199,9 @@ bool qmm_tcgen05_supported(int M, int N, int K, int bits, int group_size, int dt
 cudaError_t launch_qmm_tcgen05(Ctx *ctx, cudaStream_t st, const void *w, const void *scales, const void *biases,
                                const void *x, void *out, int M, int N, int K, int bits, int group_size, int dt,
                                std::string *why, void *const *outs, int n_outs, long long out_ld) {
-    int TN = ctx->qmm_force_tn > 0 ? ctx->qmm_force_tn : (M >= TN_MAX ? TN_MAX : ((M + 15) / 16) * 16);
+    const int sms = ctx->sm_count;
+    const DensePlan plan = plan_dense(ctx, M, N, K, bits, outs == nullptr);
+    const int TN = plan.TN;
     const void *x_op = nullptr;
     const float *tok_scale = nullptr;
     cudaError_t e = stage_x(ctx, st, x, M, K, dt, &x_op, &tok_scale, why);
@@ -1032,64 +1222,22 @@ cudaError_t launch_qmm_tcgen05(Ctx *ctx, cudaStream_t st, const void *w, const v
     p.m_chunks = (M + TN - 1) / TN;
     p.n_tiles = (N + BMW - 1) / BMW;
     p.pdl_roles = ctx->pdl_early_weights ? 1 : 0;
-    const int sms = ctx->sm_count;
-    {
-        // Two token chunks per item: the dequantised W stage, which sets the pace of a k block, is built once per
-        // 2 TN token rows instead of once per TN.
-        // Worth it when it saves rounds of the grid: a k block of a wide item costs ~1.55 x one of a single-chunk item
-        // (measured), so 7 rounds of single chunks against 3 wide rounds + a short one is a win, one round against one
-        // wide round on half the SMs is not.
-        bool wide_pays = false;
-        if (ctx->qmm_wide && TN == TN_MAX && M > TN_MAX) {
-            const int single = p.n_tiles * p.m_chunks, units = p.n_tiles * ((M + 2 * TN - 1) / (2 * TN));
-            const double cost_single = static_cast<double>((single + sms - 1) / sms);
-            const int left = units % sms;
-            const bool two_halves = M % (2 * TN) == 0 || M % (2 * TN) > TN;
-            const bool split_tail = units > sms && left > 0 && 2 * left <= sms && two_halves;
-            const double cost_wide = 1.55 * (units / sms) + (left == 0 ? 0.0 : (split_tail ? 1.0 : 1.55));
-            wide_pays = cost_wide < cost_single || ctx->qmm_wide == 2;      // 2: whenever the shape allows (tests)
-        }
-        if (wide_pays) {
-            p.wide = 1;
-            plan_smem(p, ctx, bits);
-            if (p.nst < 2) {
-                p.wide = 0;
-                plan_smem(p, ctx, bits);
-            } else {
-                p.m_chunks = (M + 2 * TN - 1) / (2 * TN);
-            }
-        }
-        p.dense_items = p.n_tiles * p.m_chunks;
-        if (p.wide) {
-            // a k block costs the same whatever the token count, so the leftover of the last round is cheaper as
-            // single-chunk items on twice as many SMs - when those still fit in one round and every unit has two halves
-            const int units = p.n_tiles * p.m_chunks, left = units % sms;
-            const bool two_halves = M % (2 * TN) == 0 || M % (2 * TN) > TN;
-            p.wide_items = units;
-            if (units > sms && left > 0 && 2 * left <= sms && two_halves) {
-                p.wide_items = units - left;
-                p.dense_items = p.wide_items + 2 * left;
-            }
-        }
-    }
-    // Few weight-row tiles and one token chunk: the tiles alone would leave most SMs idle, so K is cut into slices that
-    // run as items of their own (f32 partial sums, added in slice order by a second small kernel).
-    if (ctx->qmm_ksplit && !p.wide && p.m_chunks == 1 && !outs && 2 * p.n_tiles <= sms) {
-        const int nkb = K / BK, unit = p.raw ? SB_PER_RAW : 1;
-        int S = sms / p.n_tiles;
-        if (S > 16) S = 16;
-        while (S > 1 && (nkb % (S * unit) != 0 || nkb / S < 4)) --S;
-        if (S > 1) {
-            cudaError_t ge = grow_block(ctx, st, &ctx->d_ksplit, &ctx->ksplit_bytes, static_cast<size_t>(S) * M * N * sizeof(float), why);
-            if (ge != cudaSuccess) return ge;
-            p.ksplit = S;
-            p.kb_per = nkb / S;
-            p.partial = static_cast<float *>(ctx->d_ksplit);
-            p.dense_items *= S;
-        }
+    p.wide = plan.wide ? 1 : 0;
+    plan_smem(p, ctx, bits);
+    p.m_chunks = plan.items_m;
+    p.wide_items = p.n_tiles * p.m_chunks - plan.halves;      // the last units run as two single-chunk items each
+    p.dense_items = p.wide_items + 2 * plan.halves;
+    // Few weight-row tiles: they alone would leave most SMs idle, so K is cut into slices that run as items of their own (f32
+    // partial sums, added in slice order by a second small kernel).
+    if (plan.ksplit > 1) {
+        cudaError_t ge = grow_block(ctx, st, &ctx->d_ksplit, &ctx->ksplit_bytes, static_cast<size_t>(plan.ksplit) * M * N * sizeof(float), why);
+        if (ge != cudaSuccess) return ge;
+        p.ksplit = plan.ksplit;
+        p.partial = static_cast<float *>(ctx->d_ksplit);
+        p.dense_items = p.n_tiles * plan.ksplit;
     }
     const int grid = p.dense_items < sms ? p.dense_items : sms;
-    e = launch_any(bits, st, tmap, p, grid);
+    e = launch_any(bits, st, tmap, p, grid, N, why);
     if (e != cudaSuccess || p.ksplit == 1) return e;
     const size_t mn = static_cast<size_t>(M) * N;
     size_t sgrid = (mn + 255) / 256;
@@ -1148,10 +1296,11 @@ cudaError_t launch_gather_qmm_tcgen05(Ctx *ctx, cudaStream_t st, const void *x, 
     QmmParams p{};
     fill_common(p, ctx, w, scales, biases, out, N, K, bits, group_size, dt, TN);
     p.tok_scale = tok_scale;
+    p.sb_total *= n_experts;
     p.M = total_rows;
     p.items = items;
     p.item_count = count;
-    return launch_any(bits, st, tmap, p, ctx->sm_count);
+    return launch_any(bits, st, tmap, p, ctx->sm_count, static_cast<long long>(n_experts) * N, why);
 }
 
 // ---- gather_qmm for callers that cannot allocate ---------------------------------------------------
@@ -1235,10 +1384,11 @@ cudaError_t launch_gather_qmm_static(Ctx *ctx, cudaStream_t st, const void *x, c
     QmmParams p{};
     fill_common(p, ctx, w, scales, biases, out, N, K, bits, group_size, dt, TN);
     p.tok_scale = tok_scale;
+    p.sb_total *= n_experts;
     p.M = total_rows;
     p.items = items;
     p.item_count = count;
-    return launch_any(bits, st, tmap, p, ctx->sm_count);
+    return launch_any(bits, st, tmap, p, ctx->sm_count, static_cast<long long>(n_experts) * N, why);
 }
 
 }  // namespace mtc
