@@ -156,7 +156,8 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, SmemCt
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t parity, SmemCtrl *ctl, uint32_t *status, uint32_t code,
                                                uint32_t sleep_ns) {
     const bool ok = mbar_wait(bar, parity, ctl, status, code, sleep_ns);
-    return __all_sync(0xffffffffu, ok);
+    __syncwarp();
+    return ok;
 }
 
 __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, int c0, int c1, uint64_t *bar) {
@@ -206,6 +207,19 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
         "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
         : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
           "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
+          "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
+          "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
         : "r"(taddr));
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
@@ -683,6 +697,21 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                 const int c = hh;
                 const int row_base = item.row0 + c * p.TN;
                 const int rows_h = item.nc == 2 ? min(p.TN, item.rows - c * p.TN) : item.rows;
+                if constexpr (KSPLIT) {
+                    // a K slice: f32 partial sums, 32 token rows at a time in 128-byte segments per warp and row
+                    for (int c0 = 0; c0 < rows_h; c0 += 32) {
+                        uint32_t v[32];
+                        tmem_ld32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + (buf + hh) * TN_MAX + c0, v);
+                        if (!n_ok) continue;
+                        float *o = p.partial + (static_cast<size_t>(item.ks) * p.M + row_base + c0) * p.N + n;
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) {
+                            if (c0 + j < rows_h) *o = __uint_as_float(v[j]);       // the sum kernel applies the token factors
+                            o += p.N;
+                        }
+                    }
+                    continue;
+                }
                 const int cols = (rows_h + 15) & ~15;
                 for (int c0 = 0; c0 < cols; c0 += 16) {
                     float ts[16];                  // per-token factors first, so their latency hides behind the TMEM load
@@ -691,13 +720,7 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                         ts[j] = (p.tok_scale && c0 + j < rows_h) ? __ldg(p.tok_scale + row_base + c0 + j) : 1.0f;
                     uint32_t v[16];
                     tmem_ld16(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + (buf + hh) * TN_MAX + c0, v);
-                    if (KSPLIT && n_ok) {
-                        // a K slice: f32 partial sums, 128-byte segments per warp and token row
-                        float *o = p.partial + (static_cast<size_t>(item.ks) * p.M + row_base + c0) * p.N + n;
-#pragma unroll
-                        for (int j = 0; j < 16; ++j)
-                            if (c0 + j < rows_h) o[static_cast<size_t>(j) * p.N] = __uint_as_float(v[j]) * ts[j];
-                    } else if (n_ok) {
+                    if (n_ok) {
                         // lanes of a warp hold 32 consecutive columns of the same output row: 64-byte segments
                         unsigned short hv[16];
 #pragma unroll
@@ -1171,8 +1194,8 @@ DensePlan plan_dense(const Ctx *ctx, int M, int N, int K, int bits, bool may_spl
     return best;
 }
 
-// out[i] = sum over the K slices of partial[s][i], in slice order
-__global__ void __launch_bounds__(256) ksplit_sum_kernel(const float *partial, void *out, size_t mn, int S, int dt) {
+// out[i] = sum over the K slices of partial[s][i], in slice order, times the factor of its token row
+__global__ void __launch_bounds__(256) ksplit_sum_kernel(const float *partial, const float *tok_scale, void *out, size_t mn, int N, int S, int dt) {
     asm volatile("griddepcontrol.wait;" ::: "memory");       // launched while the product kernel runs
     for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < mn; i += static_cast<size_t>(gridDim.x) * blockDim.x) {
         float pv[16];
@@ -1181,6 +1204,7 @@ __global__ void __launch_bounds__(256) ksplit_sum_kernel(const float *partial, v
         float v = pv[0];
 #pragma unroll
         for (int q = 1; q < 16; ++q) v += pv[q];
+        if (tok_scale) v *= __ldg(tok_scale + static_cast<uint32_t>(i) / static_cast<uint32_t>(N));
         st_from_f32(out, i, v, dt);
     }
 }
@@ -1251,7 +1275,7 @@ cudaError_t launch_qmm_tcgen05(Ctx *ctx, cudaStream_t st, const void *w, const v
     la[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = la;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, ksplit_sum_kernel, static_cast<const float *>(p.partial), out, mn, p.ksplit, dt);
+    return cudaLaunchKernelEx(&cfg, ksplit_sum_kernel, static_cast<const float *>(p.partial), p.tok_scale, out, mn, N, p.ksplit, dt);
 }
 
 // scratch bytes the gather work list needs for these sizes
