@@ -43,7 +43,10 @@ constexpr int BMW = 128;         // weight rows per tile (TMEM lanes, MMA M)
 constexpr int BK = 64;           // k per stage: 64 x 16-bit = one 128B swizzle row
 constexpr int TN_MAX = 256;      // token rows per tile (TMEM columns of one accumulator, MMA N)
 constexpr int MAX_STAGES = 8;    // ring depth: as many stages as fit in RING_BYTES, at most this
-constexpr int RING_BYTES = 224 * 1024;      // stages of the ring, then the raw staging buffers; SmemCtrl follows
+constexpr int RING_BYTES = 216 * 1024;      // stages of the ring, then the raw staging buffers
+constexpr int EPI_TOK = 16;                 // token rows of one epilogue block: 128 outputs each, two buffers; SmemCtrl follows
+constexpr int EPI_PITCH = BMW * 2 + 16;     // bytes of a row: eight consecutive rows start on different banks
+constexpr int EPI_BYTES = 2 * EPI_TOK * EPI_PITCH;
 constexpr int SB_PER_RAW = 4;               // k blocks per raw super-block: 256 codes = 32*BITS bytes per weight row
 constexpr int RAW_SB_PITCH = 24;            // scales (and biases) of a super-block: up to 20 bytes per row
 constexpr int RAW_SB_BYTES = 2 * BMW * RAW_SB_PITCH;
@@ -71,6 +74,7 @@ struct QmmParams {
     int op_f16;                  // MMA operand format: 1 = f16, 0 = bf16 (dequantised W and the X tensor map)
     int sb_dt;                   // element type of scales / biases (MTC_F16 or MTC_BF16)
     int out_dt;                  // element type of out
+    int out_vec;                 // 1: eight outputs of a row are one aligned 16-byte store (N, out_ld and the pointers allow it)
     const float *tok_scale;      // per-token power-of-two factor applied in the epilogue, or nullptr
     int wpr, gpr;                // words / groups per weight row
     int TN;                      // token rows per item (TMA box rows, MMA N)
@@ -201,14 +205,25 @@ __device__ __forceinline__ void umma_commit(uint64_t *bar) {
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-        : "r"(taddr));
+// 32 TMEM lanes x 16 columns in the layout of an MMA accumulator: thread t holds, for the 8 lanes of block k (0..3) and the 8
+// columns of half g, lane t / 4 and columns 2 (t % 4), 2 (t % 4) + 1: v[k >> 1][4 g + 2 (k & 1)], + 1.
+__device__ __forceinline__ void tmem_ld_frag(uint32_t taddr, uint32_t (&v)[2][8]) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+        asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=r"(v[i][0]), "=r"(v[i][1]), "=r"(v[i][2]), "=r"(v[i][3]), "=r"(v[i][4]), "=r"(v[i][5]), "=r"(v[i][6]), "=r"(v[i][7])
+                     : "r"(taddr + (static_cast<uint32_t>(16 * i) << 16)));
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t pack_out(float lo, float hi, bool f16) {
+    uint32_t r;
+    if (f16) asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    else asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
+}
+// four 8 x 8 blocks, each stored transposed: lane i gives the address of row i % 8 of block i / 8
+__device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
 
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
@@ -407,6 +422,14 @@ struct RawTile {
 };
 int raw_bytes(int bits) { return (bits == 4 || bits == 8 ? BMW * 32 * bits : BMW * (32 * bits + 16)) + RAW_SB_BYTES; }
 
+// up to eight 16-bit outputs one by one
+__device__ __noinline__ void store_row8(char *o, uint4 v, int n) {
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+        if (e < n) reinterpret_cast<unsigned short *>(o)[e] = static_cast<unsigned short>(w[e >> 1] >> (16 * (e & 1)));
+}
+
 struct Item {
     int n_tile, expert, row0, rows;
     int nc;                                 // token chunks of TN rows covered (1 or 2): one accumulator each
@@ -476,7 +499,7 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
     const uint32_t x_slot = (p.wide ? 2 : 1) * x_stage;                 // one or two X chunks per stage
     uint8_t *sW = smem;                                  // nst x w_stage: dequantised weights (A operand)
     uint8_t *sX = smem + nst * w_stage;                  // nst x x_slot: activations (B operand)
-    SmemCtrl *ctl = reinterpret_cast<SmemCtrl *>(smem + RING_BYTES);
+    SmemCtrl *ctl = reinterpret_cast<SmemCtrl *>(smem + RING_BYTES + EPI_BYTES);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int num_items = p.items ? __ldg(p.item_count) : p.dense_items;
@@ -681,6 +704,16 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
     } else if (warp >= EPI_WARP0 && warp < EPI_WARP0 + 4) {
         // ---------------- epilogue: TMEM -> registers -> out (transposed) ----------------
         const int q = warp - EPI_WARP0;          // == warp % 4: the TMEM lane quarter this warp may read
+        uint32_t epi_buf = 0;
+        // what the loop below reads of the parameters, kept in registers: read again for every row the constant bank costs
+        // ~200 cycles each time
+        uint64_t out0 = reinterpret_cast<uint64_t>(p.outs[0]), ld2 = static_cast<uint64_t>(p.out_ld) * 2, tokp = reinterpret_cast<uint64_t>(p.tok_scale);
+        uint32_t more_outs = p.n_outs - 1, out_f16 = p.out_dt == MTC_F16, out_vec = p.out_vec;
+        int pN = p.N;
+        asm volatile("" : "+l"(out0), "+l"(ld2), "+l"(tokp), "+r"(more_outs), "+r"(out_f16), "+r"(out_vec), "+r"(pN));
+        const float *tok_scale = reinterpret_cast<const float *>(tokp);
+        const int tok_last = p.M - 1;
+        const uint32_t epi0 = smem_u32(smem + RING_BYTES);
         uint32_t tile_i = 0;
         bool ok = true;
         if (p.pdl_roles) asm volatile("griddepcontrol.wait;" ::: "memory");          // token factors; nothing is stored before this
@@ -712,28 +745,49 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                     }
                     continue;
                 }
-                const int cols = (rows_h + 15) & ~15;
-                for (int c0 = 0; c0 < cols; c0 += 16) {
-                    float ts[16];                  // per-token factors first, so their latency hides behind the TMEM load
+                // 16 token rows at a time through shared memory, transposed on the way ([row][128 outputs]), then whole rows of
+                // 256 bytes.  Kept to ~45 instructions a block: the four warps have nobody to hide instruction fetches
+                // behind, and a block of 16 conversions and 16 stores a thread took 600 cycles.
+                const int n8 = item.n_tile * BMW + (lane & 15) * 8;
+                char *row_out = reinterpret_cast<char *>(out0) + static_cast<uint64_t>(row_base + 2 * q + (lane >> 4)) * ld2 + static_cast<uint64_t>(n8) * 2;
+                for (int c0 = 0; c0 < rows_h; c0 += EPI_TOK) {
+                    float2 ts[2] = {{1.0f, 1.0f}, {1.0f, 1.0f}};       // this lane's token factors
+                    if (tok_scale) {
 #pragma unroll
-                    for (int j = 0; j < 16; ++j)
-                        ts[j] = (p.tok_scale && c0 + j < rows_h) ? __ldg(p.tok_scale + row_base + c0 + j) : 1.0f;
-                    uint32_t v[16];
-                    tmem_ld16(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + (buf + hh) * TN_MAX + c0, v);
-                    if (n_ok) {
-                        // lanes of a warp hold 32 consecutive columns of the same output row: 64-byte segments
-                        unsigned short hv[16];
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) {
-                            const float f = __uint_as_float(v[j]) * ts[j];
-                            hv[j] = p.out_dt == MTC_F16 ? __half_as_ushort(__float2half_rn(f)) : __bfloat16_as_ushort(__float2bfloat16_rn(f));
+                        for (int g = 0; g < 2; ++g) {
+                            const int j = row_base + c0 + 8 * g + 2 * (lane & 3);
+                            ts[g].x = __ldg(tok_scale + min(j, tok_last));
+                            ts[g].y = __ldg(tok_scale + min(j + 1, tok_last));
                         }
-                        for (int d = 0; d < p.n_outs; ++d) {
-                            unsigned short *o = static_cast<unsigned short *>(p.outs[d]) + static_cast<size_t>(row_base + c0) * p.out_ld + n;
+                    }
+                    uint32_t v[2][8];
+                    tmem_ld_frag(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + (buf + hh) * TN_MAX + c0, v);
+                    const uint32_t sb = epi0 + (epi_buf & 1) * (EPI_TOK * EPI_PITCH);
+                    ++epi_buf;
 #pragma unroll
-                            for (int j = 0; j < 16; ++j)
-                                if (c0 + j < rows_h) o[static_cast<size_t>(j) * p.out_ld] = hv[j];
+                    for (int g = 0; g < 2; ++g) {
+                        uint32_t o[4];
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+                            o[k] = pack_out(__uint_as_float(v[k >> 1][4 * g + 2 * (k & 1)]) * ts[g].x, __uint_as_float(v[k >> 1][4 * g + 2 * (k & 1) + 1]) * ts[g].y, out_f16);
+                        stmatrix_x4_trans(sb + (8 * g + (lane & 7)) * EPI_PITCH + q * 64 + (lane >> 3) * 16, o[0], o[1], o[2], o[3]);
+                    }
+                    asm volatile("bar.sync 1, 128;" ::: "memory");     // the four epilogue warps; two buffers: one barrier a block
+#pragma unroll
+                    for (int rr = 0; rr < EPI_TOK / 8; ++rr) {          // two rows per warp and step, 16 lanes each
+                        const int j = rr * 8 + 2 * q + (lane >> 4);
+                        if (c0 + j < rows_h && n8 < pN) {
+                            uint4 o4;
+                            asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(o4.x), "=r"(o4.y), "=r"(o4.z), "=r"(o4.w) : "r"(sb + j * EPI_PITCH + (lane & 15) * 16));
+                            if (out_vec) *reinterpret_cast<uint4 *>(row_out) = o4;
+                            else store_row8(row_out, o4, pN - n8);
+                            for (uint32_t d = 0; d < more_outs; ++d) {  // the peers' copies of a column block
+                                char *o = static_cast<char *>(p.outs[d + 1]) + static_cast<uint64_t>(row_base + c0 + j) * ld2 + static_cast<uint64_t>(n8) * 2;
+                                if (out_vec) *reinterpret_cast<uint4 *>(o) = o4;
+                                else store_row8(o, o4, pN - n8);
+                            }
                         }
+                        row_out += 8 * ld2;
                     }
                 }
             }
@@ -888,33 +942,48 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
 // 2^38 below the row maximum lose bits, which changes nothing measurable.  The MMA then runs on f16
 // operands, whose 3 extra mantissa bits keep the dequantised weights 8x closer to the f32 oracle than
 // bf16 weights would be; the epilogue multiplies the accumulator by 2^e again.
+// W warps share a row and hold it in registers between the maximum and the conversion (one read of x instead of two), eight
+// 16-byte loads a lane in flight: 2048 x 4096 10.1 -> 5 us, which every bf16 product waits for.  Longer rows are read twice.
+template <int W>
 __global__ void __launch_bounds__(256) rows_to_f16_kernel(const __nv_bfloat16 *x, __half *y, float *row_scale, int rows, int K) {
     asm volatile("griddepcontrol.launch_dependents;");      // the product kernel may start on the weights meanwhile
-    const int lane = threadIdx.x & 31;
-    const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (row >= rows) return;
-    const uint4 *src = reinterpret_cast<const uint4 *>(x + static_cast<size_t>(row) * K);
-    uint4 *dst = reinterpret_cast<uint4 *>(y + static_cast<size_t>(row) * K);
-    const int nvec = K / 8;
+    constexpr int ROWS = 8 / W, HELD = 8, STEP = 32 * W;
+    __shared__ uint32_t part[8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int row = blockIdx.x * ROWS + warp / W, i0 = (warp % W) * 32 + lane;
+    const bool on = row < rows;
+    const int nvec = on ? K / 8 : 0;
+    const uint4 *src = reinterpret_cast<const uint4 *>(x + static_cast<size_t>(on ? row : 0) * K);
+    uint4 *dst = reinterpret_cast<uint4 *>(y + static_cast<size_t>(on ? row : 0) * K);
+    uint4 held[HELD];
+#pragma unroll
+    for (int q = 0; q < HELD; ++q) held[q] = i0 + q * STEP < nvec ? __ldg(src + i0 + q * STEP) : make_uint4(0u, 0u, 0u, 0u);
     uint32_t amax = 0;                       // max of |x| as bf16 bit patterns (monotone for finite values)
-    for (int i = lane; i < nvec; i += 32) {
-        const uint4 v = __ldg(src + i);
+    auto fold = [&](const uint4 &v) {
         const uint32_t u[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             amax = max(amax, u[j] & 0x7FFFu);
             amax = max(amax, (u[j] >> 16) & 0x7FFFu);
         }
-    }
+    };
+#pragma unroll
+    for (int q = 0; q < HELD; ++q) fold(held[q]);
+    for (int i = i0 + HELD * STEP; i < nvec; i += STEP) fold(__ldg(src + i));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) amax = max(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    if constexpr (W > 1) {
+        if (lane == 0) part[warp] = amax;
+        __syncthreads();
+#pragma unroll
+        for (int w = 0; w < W; ++w) amax = max(amax, part[warp / W * W + w]);
+    }
     const int ex = static_cast<int>(amax >> 7);                    // biased exponent of the row maximum
     int e = (ex == 0 || ex == 0xFF) ? 0 : ex - 127 - 14;           // zero rows and inf/nan rows stay unscaled
     e = max(e, -126);                                              // 2^-e and 2^e must both be normal f32 numbers
     const float down = __uint_as_float(static_cast<uint32_t>(127 - e) << 23);
-    if (lane == 0) row_scale[row] = __uint_as_float(static_cast<uint32_t>(127 + e) << 23);
-    for (int i = lane; i < nvec; i += 32) {
-        const uint4 v = __ldg(src + i);
+    if (on && i0 == 0) row_scale[row] = __uint_as_float(static_cast<uint32_t>(127 + e) << 23);
+    auto convert = [&](const uint4 &v) {
         const uint32_t u[4] = {v.x, v.y, v.z, v.w};
         uint32_t o[4];
 #pragma unroll
@@ -922,8 +991,22 @@ __global__ void __launch_bounds__(256) rows_to_f16_kernel(const __nv_bfloat16 *x
             const __half2 h = __floats2half2_rn(__uint_as_float(u[j] << 16) * down, __uint_as_float(u[j] & 0xFFFF0000u) * down);
             o[j] = *reinterpret_cast<const uint32_t *>(&h);
         }
-        dst[i] = make_uint4(o[0], o[1], o[2], o[3]);
-    }
+        return make_uint4(o[0], o[1], o[2], o[3]);
+    };
+#pragma unroll
+    for (int q = 0; q < HELD; ++q)
+        if (i0 + q * STEP < nvec) dst[i0 + q * STEP] = convert(held[q]);
+    for (int i = i0 + HELD * STEP; i < nvec; i += STEP) dst[i] = convert(__ldg(src + i));
+}
+cudaError_t launch_rows_to_f16(cudaStream_t st, const void *x, __half *y, float *row_scale, int rows, int K) {
+    const __nv_bfloat16 *xb = static_cast<const __nv_bfloat16 *>(x);
+    const int per = K <= 2048 ? 1 : K <= 4096 ? 2 : K <= 8192 ? 4 : 8;                 // warps per row: eight vectors a lane
+    const int grid = (rows + 8 / per - 1) / (8 / per);
+    if (per == 1) rows_to_f16_kernel<1><<<grid, 256, 0, st>>>(xb, y, row_scale, rows, K);
+    else if (per == 2) rows_to_f16_kernel<2><<<grid, 256, 0, st>>>(xb, y, row_scale, rows, K);
+    else if (per == 4) rows_to_f16_kernel<4><<<grid, 256, 0, st>>>(xb, y, row_scale, rows, K);
+    else rows_to_f16_kernel<8><<<grid, 256, 0, st>>>(xb, y, row_scale, rows, K);
+    return cudaGetLastError();
 }
 
 // Work list of the gather case, built on the device from the CSR expert_offsets (or, when only the
@@ -992,7 +1075,7 @@ EncodeTiledFn get_encode_fn() {
 
 template <int BITS>
 constexpr size_t qmm_smem_bytes() {
-    return RING_BYTES + sizeof(SmemCtrl) + 1024;
+    return RING_BYTES + EPI_BYTES + sizeof(SmemCtrl) + 1024;
 }
 
 template <int BITS>
@@ -1127,6 +1210,11 @@ void fill_common(QmmParams &p, Ctx *ctx, const void *w, const void *scales, cons
               (static_cast<uint32_t>(BMW >> 4) << 24);
 }
 
+void set_out_vec(QmmParams &p) {
+    p.out_vec = p.N % 8 == 0 && p.out_ld % 8 == 0;
+    for (int d = 0; d < p.n_outs; ++d) p.out_vec = p.out_vec && reinterpret_cast<uintptr_t>(p.outs[d]) % 16 == 0;
+}
+
 // bf16 activations: stage a scaled f16 copy of x in the context's conversion buffer.
 cudaError_t stage_x(Ctx *ctx, cudaStream_t st, const void *x, int rows, int K, int dt, const void **x_op,
                     const float **tok_scale, std::string *why) {
@@ -1138,8 +1226,7 @@ cudaError_t stage_x(Ctx *ctx, cudaStream_t st, const void *x, int rows, int K, i
     if (ge != cudaSuccess) return ge;
     __half *y = static_cast<__half *>(ctx->d_xconv);
     float *scale = reinterpret_cast<float *>(static_cast<char *>(ctx->d_xconv) + ((static_cast<size_t>(rows) * K * 2 + 255) & ~static_cast<size_t>(255)));
-    rows_to_f16_kernel<<<(rows + 7) / 8, 256, 0, st>>>(static_cast<const __nv_bfloat16 *>(x), y, scale, rows, K);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = launch_rows_to_f16(st, x, y, scale, rows, K);
     if (e != cudaSuccess) return e;
     *x_op = y;
     *tok_scale = scale;
@@ -1260,6 +1347,7 @@ cudaError_t launch_qmm_tcgen05(Ctx *ctx, cudaStream_t st, const void *w, const v
         p.partial = static_cast<float *>(ctx->d_ksplit);
         p.dense_items = p.n_tiles * plan.ksplit;
     }
+    set_out_vec(p);
     const int grid = p.dense_items < sms ? p.dense_items : sms;
     e = launch_any(bits, st, tmap, p, grid, N, why);
     if (e != cudaSuccess || p.ksplit == 1) return e;
@@ -1324,6 +1412,7 @@ cudaError_t launch_gather_qmm_tcgen05(Ctx *ctx, cudaStream_t st, const void *x, 
     p.M = total_rows;
     p.items = items;
     p.item_count = count;
+    set_out_vec(p);
     return launch_any(bits, st, tmap, p, ctx->sm_count, static_cast<long long>(n_experts) * N, why);
 }
 
@@ -1397,8 +1486,7 @@ cudaError_t launch_gather_qmm_static(Ctx *ctx, cudaStream_t st, const void *x, c
     if (dt == MTC_BF16) {
         __half *y = reinterpret_cast<__half *>(base + kStaticXOff);
         float *scale = reinterpret_cast<float *>(base + kStaticScaleOff);
-        rows_to_f16_kernel<<<(total_rows + 7) / 8, 256, 0, st>>>(static_cast<const __nv_bfloat16 *>(x), y, scale, total_rows, K);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        if ((e = launch_rows_to_f16(st, x, y, scale, total_rows, K)) != cudaSuccess) return e;
         x_op = y;
         tok_scale = scale;
     }
@@ -1412,6 +1500,7 @@ cudaError_t launch_gather_qmm_static(Ctx *ctx, cudaStream_t st, const void *x, c
     p.M = total_rows;
     p.items = items;
     p.item_count = count;
+    set_out_vec(p);
     return launch_any(bits, st, tmap, p, ctx->sm_count, static_cast<long long>(n_experts) * N, why);
 }
 
