@@ -90,7 +90,7 @@ struct QmmParams {
     int wide;                    // 1: a dense item covers up to 2 TN token rows: one dequantised W stage meets two X chunks, both
                                  //    accumulators belong to the item (the dequant work per flop halves; no epilogue overlap)
     int n_tiles;                 // dense: weight-row tiles
-    int ksplit;                  // dense, one token item per weight-row tile: K slices (each an item of its own); 1 = none
+    int ksplit;                  // dense: K slices per (weight-row tile, token rows) unit, each an item of its own; 1 = none
     float *partial;              // ksplit > 1: f32 partial sums [ksplit][M][N], added by ksplit_sum_kernel
     int pdl_roles;               // programmatic dependent launch: 1 = only the roles that touch what an earlier kernel of the
                                  //    stream may have written (producer: x; epilogue: token factors, out) wait for it, the
@@ -443,17 +443,18 @@ __device__ __forceinline__ Item get_item(const QmmParams &p, int i) {
     it.nkb = p.K / BK;
     it.ks = 0;
     if (KSPLIT) {
-        // K slices of a tile are adjacent items: whole super-blocks, as even as they come, against all token rows
-        it.n_tile = i / p.ksplit;
-        it.ks = i - it.n_tile * p.ksplit;
+        // K slices of a (tile, token rows) unit are adjacent items: whole super-blocks, as even as they come
+        const int u = i / p.ksplit, unit = u / p.m_chunks, span = p.wide ? 2 * p.TN : p.TN;
+        it.n_tile = unit;
+        it.ks = i - u * p.ksplit;
         const int nsb = (it.nkb + SB_PER_RAW - 1) / SB_PER_RAW;
         const int sb0 = it.ks * nsb / p.ksplit, sb1 = (it.ks + 1) * nsb / p.ksplit;
         it.kb0 = sb0 * SB_PER_RAW;
         it.nkb = min(sb1 * SB_PER_RAW, it.nkb) - it.kb0;
         it.expert = 0;
-        it.row0 = 0;
-        it.rows = p.M;
-        it.nc = p.M > p.TN ? 2 : 1;
+        it.row0 = (u - unit * p.m_chunks) * span;
+        it.rows = min(span, p.M - it.row0);
+        it.nc = it.rows > p.TN ? 2 : 1;
         return it;
     }
     if (p.items) {
@@ -947,6 +948,7 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
 template <int W>
 __global__ void __launch_bounds__(256) rows_to_f16_kernel(const __nv_bfloat16 *x, __half *y, float *row_scale, int rows, int K) {
     asm volatile("griddepcontrol.launch_dependents;");      // the product kernel may start on the weights meanwhile
+    asm volatile("griddepcontrol.wait;" ::: "memory");       // x may come from the previous kernel, which may read the last y
     constexpr int ROWS = 8 / W, HELD = 8, STEP = 32 * W;
     __shared__ uint32_t part[8];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1002,11 +1004,17 @@ cudaError_t launch_rows_to_f16(cudaStream_t st, const void *x, __half *y, float 
     const __nv_bfloat16 *xb = static_cast<const __nv_bfloat16 *>(x);
     const int per = K <= 2048 ? 1 : K <= 4096 ? 2 : K <= 8192 ? 4 : 8;                 // warps per row: eight vectors a lane
     const int grid = (rows + 8 / per - 1) / (8 / per);
-    if (per == 1) rows_to_f16_kernel<1><<<grid, 256, 0, st>>>(xb, y, row_scale, rows, K);
-    else if (per == 2) rows_to_f16_kernel<2><<<grid, 256, 0, st>>>(xb, y, row_scale, rows, K);
-    else if (per == 4) rows_to_f16_kernel<4><<<grid, 256, 0, st>>>(xb, y, row_scale, rows, K);
-    else rows_to_f16_kernel<8><<<grid, 256, 0, st>>>(xb, y, row_scale, rows, K);
-    return cudaGetLastError();
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(256);
+    cfg.stream = st;
+    cudaLaunchAttribute la[1];
+    la[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    la[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = la;
+    cfg.numAttrs = 1;
+    const auto kern = per == 1 ? rows_to_f16_kernel<1> : per == 2 ? rows_to_f16_kernel<2> : per == 4 ? rows_to_f16_kernel<4> : rows_to_f16_kernel<8>;
+    return cudaLaunchKernelEx(&cfg, kern, xb, y, row_scale, rows, K);
 }
 
 // Work list of the gather case, built on the device from the CSR expert_offsets (or, when only the
@@ -1234,7 +1242,9 @@ cudaError_t stage_x(Ctx *ctx, cudaStream_t st, const void *x, int rows, int K, i
 }
 
 // Time of a k block of an item on one SM by its token rows, us (measured): the dequantisation sets the pace of narrow items.
-constexpr double kKbBase = 0.40, kKbPerToken = 0.0010;
+constexpr double kKbBase = 0.47, kKbPerToken = 0.0006;
+constexpr double kWideBase = 0.45, kWidePerToken = 0.00075;      // an item of two chunks
+constexpr double kSliceUs = 2e-6;       // an f32 partial sum: written at ~3 TB/s, read at ~6
 constexpr double kItemUs = 0.4;         // a further item on the same SM: its accumulators drain before the next pair starts
 
 // How a dense launch covers its M token rows: items of one chunk (TN rows, one accumulator) or of two (the dequantised W stage
@@ -1260,18 +1270,18 @@ DensePlan plan_dense(const Ctx *ctx, int M, int N, int K, int bits, bool may_spl
         const int most = form == 1 ? 2 * tn_wide : TN_MAX;
         const int items_m = (M + most - 1) / most;
         const int TN = form == 1 ? up16((M + 2 * items_m - 1) / (2 * items_m)) : up16((M + items_m - 1) / items_m);
-        const double one = kKbBase + kKbPerToken * TN, kb_us = form == 1 ? kKbBase + kKbPerToken * 2 * TN : one;
+        const double one = kKbBase + kKbPerToken * TN, kb_us = form == 1 ? kWideBase + kWidePerToken * 2 * TN : one;
         const long long units = static_cast<long long>(n_tiles) * items_m;
         // the last round of wide items on twice as many SMs, a chunk each, where that still is one round and every unit has two
         const int left = static_cast<int>(units % sms), last_rows = M - (items_m - 1) * 2 * TN;
         const bool tail = form == 1 && units > sms && left > 0 && 2 * left <= sms && last_rows > TN;
         for (int S = 1; S <= 16; ++S) {
-            if (S > 1 && (!ctx->qmm_ksplit || !may_split || items_m > 1 || S > nsb || (form == 1 && ctx->qmm_wide == 2))) break;
+            if (S > 1 && (!ctx->qmm_ksplit || !may_split || S > nsb || (form == 1 && ctx->qmm_wide == 2))) break;
             const int kb = S == 1 ? nkb : (nsb + S - 1) / S * SB_PER_RAW;
             const long long full = units * S / sms, rest = units * S % sms;
             double us = full * (kb * kb_us + kItemUs);
             if (rest > 0) us += (S == 1 && tail ? kb * one : kb * kb_us) + kItemUs;
-            if (S > 1) us += 2.0 + static_cast<double>(S) * M * N * 8 / 6e6;
+            if (S > 1) us += 2.0 + static_cast<double>(S) * M * N * kSliceUs;
             if (us < best_us - 1e-9) {
                 best_us = us;
                 best = DensePlan{TN, items_m, S, S == 1 && tail ? left : 0, form == 1};
@@ -1345,7 +1355,7 @@ cudaError_t launch_qmm_tcgen05(Ctx *ctx, cudaStream_t st, const void *w, const v
         if (ge != cudaSuccess) return ge;
         p.ksplit = plan.ksplit;
         p.partial = static_cast<float *>(ctx->d_ksplit);
-        p.dense_items = p.n_tiles * plan.ksplit;
+        p.dense_items = p.n_tiles * p.m_chunks * plan.ksplit;
     }
     set_out_vec(p);
     const int grid = p.dense_items < sms ? p.dense_items : sms;
