@@ -109,6 +109,27 @@ struct PerDeviceAttr {
     }
 };
 
+// Programmatic dependent launch for a kernel that reads what the previous kernel of its stream wrote: it is scheduled while that
+// kernel drains (the launch latency overlaps) and waits on the device before it touches anything.
+__device__ __forceinline__ void pdl_enter() {
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <typename... P, typename... A>
+cudaError_t launch_pdl(void (*kern)(P...), int grid, int block, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute la[1];
+    la[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    la[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = la;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
 // ---- dtype-generic element access (dtype is a launch-time constant) ----------
 __device__ __forceinline__ float ld_as_f32(const void *p, size_t i, int dt) {
     if (dt == MTC_F32) return __ldg(reinterpret_cast<const float *>(p) + i);

@@ -35,7 +35,7 @@ constexpr int kGMaxPasses = 4096;
 constexpr uint32_t kGOffX = 128;
 
 struct GPass {
-    int expert, tok0, ntok;
+    int expert, tok0, ntok;           // rows tok0 .. tok0 + ntok - 1 of the product
     int cost0;            // weight of the passes before this one (a pass weighs 2 + its token tiles, per row tile)
 };
 struct GTable {
@@ -52,6 +52,8 @@ struct GArgs {
     int tpe1;                        // row tiles of the first matrix: tile indices from tpe1 on belong to the second
     const unsigned char *xfrag;      // [m_total][K / 64][4][2] units of 16 bytes
     const float *xsum;               // [m_total][K / 64]
+    const uint32_t *row_src;         // row m of the product is row row_src[m] of xfrag / xsum (null: row m)
+    int n_src_rows;
     const GTable *table;
     void *out;
     uint32_t *status;
@@ -111,13 +113,15 @@ __device__ __forceinline__ float g_f32_of_half(uint32_t word, int hi) {
 // past m_total are clamped (the rows they would have named are left out) and reported in the status word (0x901).
 // Every block converts rows: the four lanes of a quad share (row, segment); lane t reads x[16t .. 16t+15] of the
 // segment and writes two 16-byte units: fragments 0,1 (nibbles 0,4 and 1,5) and 2,3 (nibbles 2,6 and 3,7).
-// MODE 0: row m of x.  MODE 1: row row_src[m] of x (the permutation of mt_moe_permute, moe.rs:222-281, without the copy).
+// n_rows rows are converted: m_total, or the n_src_rows source rows themselves when the gather kernel follows row_src (MODE 0
+// then: a token that eight experts see is converted once).  MODE 0: row m of x.  MODE 1: row row_src[m] of x (the permutation of mt_moe_permute, moe.rs:222-281, without the copy).
 // MODE 2: silu(x[m]) * x2[m] rounded to the activation type first (mt_swiglu, crates/metaltile-std/src/mlx/swiglu.rs:45-57,
 // with the arithmetic of the stand-alone kernel: g / (1 + expf(-g)) * u in f32).
 template <bool BF16, int MODE>
 __global__ void __launch_bounds__(256) gather_prep_kernel(const void *x, const void *x2, const uint32_t *row_src, int n_src_rows,
-                                                          const uint32_t *offsets, int n_experts, int m_total, int K, int TB,
+                                                          const uint32_t *offsets, int n_experts, int m_total, int n_rows, int K, int TB,
                                                           unsigned char *xfrag, float *xsum, GTable *table, uint32_t *status) {
+    pdl_enter();
     if (blockIdx.x == 0 && threadIdx.x < 32) {
         const int lane = threadIdx.x;
         int n_pass = 0, cost = 0;
@@ -165,7 +169,7 @@ __global__ void __launch_bounds__(256) gather_prep_kernel(const void *x, const v
     }
     const int nseg = K >> 6;
     const int t = threadIdx.x & 3;
-    const long long quads = static_cast<long long>(m_total) * nseg;
+    const long long quads = static_cast<long long>(n_rows) * nseg;
     for (long long q = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 2; q < ((quads + 7) & ~7ll);
          q += (static_cast<long long>(gridDim.x) * blockDim.x) >> 2) {
         const bool on = q < quads;                     // whole warps stay in the loop: the sums use shuffles
@@ -175,18 +179,18 @@ __global__ void __launch_bounds__(256) gather_prep_kernel(const void *x, const v
         if (on) {
             size_t src = static_cast<size_t>(m);
             if (MODE == 1) {
-                const uint32_t r = __ldg(row_src + m);
+                const uint32_t r = row_src[m];
                 if (r >= static_cast<uint32_t>(n_src_rows)) atomicCAS(status, 0u, 0x903u);     // not a row of x: row 0 is read instead
                 src = r < static_cast<uint32_t>(n_src_rows) ? r : 0;
             }
             const uint4 *p = reinterpret_cast<const uint4 *>(static_cast<const uint16_t *>(x) + src * K + s * 64 + 16 * t);
-            v0 = __ldg(p);
-            v1 = __ldg(p + 1);
+            v0 = p[0];
+            v1 = p[1];
         }
         uint32_t u[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
         if (MODE == 2 && on) {
             const uint4 *p2 = reinterpret_cast<const uint4 *>(static_cast<const uint16_t *>(x2) + static_cast<size_t>(m) * K + s * 64 + 16 * t);
-            const uint4 w0 = __ldg(p2), w1 = __ldg(p2 + 1);
+            const uint4 w0 = p2[0], w1 = p2[1];
             const uint32_t uu[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
@@ -242,16 +246,17 @@ __global__ void __launch_bounds__(256) gather_prep_kernel(const void *x, const v
 
 // ---- the gather kernel ------------------------------------------------------------------------------------------
 
-// Row tiles [ta, tb) of pass `ps` that belong to the cost range [lo, hi).  Work is dealt in UNITS of kGW tiles (one per
-// warp), so that no warp idles at the end of a pass while the others finish: unit i sits at cost0 * UPE + i * c.
-__device__ __forceinline__ void g_tile_range(const GPass &ps, long long lo, long long hi, int TPE, int &ta, int &tb) {
+// Row tiles [ta, tb) of pass `ps` that belong to the cost range [lo, hi).  Work is dealt in UNITS of ut tiles - one per warp where
+// there is plenty, so that no warp idles at the end of a pass while the others finish; single tiles where a CTA gets a
+// handful, so that every SM reads its share: unit i sits at cost0 * UPE + i * c.
+__device__ __forceinline__ void g_tile_range(const GPass &ps, long long lo, long long hi, int TPE, int ut, int &ta, int &tb) {
     const int c = 2 + ((ps.ntok + 7) >> 3);
-    const int UPE = (TPE + kGW - 1) / kGW;
+    const int UPE = (TPE + ut - 1) / ut;
     const long long base = static_cast<long long>(ps.cost0) * UPE;
     const int ua = lo <= base ? 0 : static_cast<int>(min(static_cast<long long>(UPE), (lo - base + c - 1) / c));
     const int ub = hi <= base ? 0 : static_cast<int>(min(static_cast<long long>(UPE), (hi - base + c - 1) / c));
-    ta = min(ua * kGW, TPE);
-    tb = min(ub * kGW, TPE);
+    ta = min(ua * ut, TPE);
+    tb = min(ub * ut, TPE);
 }
 
 // The integer codes of one 64-code segment of 16 rows as the four A fragments of its MMAs.
@@ -337,12 +342,15 @@ struct GCopy {
 template <bool BF16, int GSH, int DEPTH>
 __global__ void __launch_bounds__(kGThreads, 1) gather_stream_kernel(const __grid_constant__ GArgs a) {
     extern __shared__ __align__(128) unsigned char gsm[];
+    pdl_enter();                                        // the table, the fragments
     int *ctl = reinterpret_cast<int *>(gsm);            // [0] first pass, [1] last pass of this CTA
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
     const GTable *tb_ = a.table;
     const int n_pass = tb_->n_pass, TPE = a.tiles_per_expert;
-    const long long total = static_cast<long long>(tb_->total_cost) * ((TPE + kGW - 1) / kGW);
+    const int share = static_cast<int>(static_cast<long long>(n_pass) * TPE / gridDim.x);          // tiles per CTA
+    const int ut = share >= 4 * kGW ? kGW : share >= 2 * kGW ? kGW / 2 : share >= kGW ? kGW / 4 : 1;
+    const long long total = static_cast<long long>(tb_->total_cost) * ((TPE + ut - 1) / ut);
     const long long lo = total * blockIdx.x / gridDim.x, hi = total * (blockIdx.x + 1) / gridDim.x;
     const int runs = a.K >> 8;
     if (threadIdx.x == 0) {
@@ -352,7 +360,7 @@ __global__ void __launch_bounds__(kGThreads, 1) gather_stream_kernel(const __gri
     __syncthreads();
     for (int p = threadIdx.x; p < n_pass; p += kGThreads) {
         int ta, tb;
-        g_tile_range(tb_->pass[p], lo, hi, TPE, ta, tb);
+        g_tile_range(tb_->pass[p], lo, hi, TPE, ut, ta, tb);
         if (tb > ta) {
             atomicMin(&ctl[0], p);
             atomicMax(&ctl[1], p);
@@ -376,7 +384,7 @@ __global__ void __launch_bounds__(kGThreads, 1) gather_stream_kernel(const __gri
         for (; cit.pp <= p_last; ++cit.pp) {
             const GPass ps = tb_->pass[cit.pp];
             int ta, tb;
-            g_tile_range(ps, lo, hi, TPE, ta, tb);
+            g_tile_range(ps, lo, hi, TPE, ut, ta, tb);
             if (ta + warp < tb) {
                 cit.tile = ta + warp;
                 cit.tb = tb;
@@ -498,16 +506,21 @@ __global__ void __launch_bounds__(kGThreads, 1) gather_stream_kernel(const __gri
     for (int pp = p_first; pp <= p_last; ++pp) {
         const GPass ps = tb_->pass[pp];
         int ta, tb;
-        g_tile_range(ps, lo, hi, TPE, ta, tb);
+        g_tile_range(ps, lo, hi, TPE, ut, ta, tb);
         if (pp != p_first) __syncthreads();                      // every warp is done with the previous pass's activations
-        for (int idx = threadIdx.x; idx < ps.ntok * upr; idx += kGThreads) {
-            const int m = idx / upr, r = idx - m * upr;
-            const int s = r >> 3, tt = (r >> 1) & 3, h = r & 1;
-            g_cp16(xdst + ((((s * TB + m) * 4 + tt) * 2 + (h ^ (m & 1))) << 4), a.xfrag + (static_cast<size_t>(ps.tok0 + m) * upr + r) * 16);
-        }
-        for (int idx = threadIdx.x; idx < ps.ntok * nseg; idx += kGThreads) {
-            const int m = idx / nseg, s = idx - m * nseg;
-            g_cp4(sdst0 + ((s * TB + m) << 2), a.xsum + static_cast<size_t>(ps.tok0 + m) * nseg + s);
+        // a warp stages whole rows: the row it follows is looked up once, no division per copy
+        for (int m = warp; m < ps.ntok; m += kGW) {
+            size_t row = static_cast<size_t>(ps.tok0 + m);
+            if (a.row_src) {
+                const uint32_t r = a.row_src[row];
+                if (r >= static_cast<uint32_t>(a.n_src_rows)) atomicCAS(a.status, 0u, 0x903u);   // not a row of x: row 0 is read instead
+                row = r < static_cast<uint32_t>(a.n_src_rows) ? r : 0;
+            }
+            const unsigned char *src = a.xfrag + row * upr * 16;
+            for (int r = lane; r < upr; r += 32)
+                g_cp16(xdst + (((((r >> 3) * TB + m) * 4 + ((r >> 1) & 3)) * 2 + ((r & 1) ^ (m & 1))) << 4), src + r * 16);
+            const float *sums = a.xsum + row * nseg;
+            for (int s = lane; s < nseg; s += 32) g_cp4(sdst0 + ((s * TB + m) << 2), sums + s);
         }
         g_commit();
         asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -529,9 +542,12 @@ struct GPlan {
     uint32_t off_xsum = 0, off_ring = 0;
 };
 
-GPlan g_plan(int K) {
+// rows: mean rows per expert.  A pass for up to 8 rows where an expert sees one or two leaves the ring the shared memory.
+GPlan g_plan(int K, int rows) {
     GPlan p;
     p.TB = K <= 2048 ? 32 : K <= 4096 ? 16 : 8;
+    if (rows <= 2) p.TB = 8;
+    else if (rows <= 8 && p.TB > 16) p.TB = 16;
     const size_t xfrag = static_cast<size_t>(p.TB) * K * 2, xsum = static_cast<size_t>(p.TB) * (K / 64) * 4;
     p.off_xsum = static_cast<uint32_t>(kGOffX + xfrag);
     p.off_ring = static_cast<uint32_t>((p.off_xsum + xsum + 127) / 128 * 128);
@@ -551,8 +567,7 @@ cudaError_t g_launch(const GArgs &a, int grid, size_t smem, cudaStream_t st) {
     static PerDeviceAttr attr;
     cudaError_t e = attr.set(gather_stream_kernel<BF16, GSH, DEPTH>, 227 * 1024);
     if (e != cudaSuccess) return e;
-    gather_stream_kernel<BF16, GSH, DEPTH><<<grid, kGThreads, smem, st>>>(a);
-    return cudaGetLastError();
+    return launch_pdl(gather_stream_kernel<BF16, GSH, DEPTH>, grid, kGThreads, smem, st, a);
 }
 
 template <bool BF16, int GSH>
@@ -568,7 +583,7 @@ bool gather_stream_supported(int m_total, int n_out, int K, int n_experts, int b
                              const void *scales, const void *biases, const void *x) {
     if (bits != 4 || (dtype != MTC_F16 && dtype != MTC_BF16) || (group_size != 64 && group_size != 128)) return false;
     if (m_total <= 0 || n_out <= 0 || K <= 0 || K % 256 != 0 || K > 8192 || n_experts <= 0) return false;
-    const GPlan p = g_plan(K);
+    const GPlan p = g_plan(K, m_total / n_experts);
     if (p.depth == 0) return false;
     if (static_cast<long long>(n_experts) + m_total / p.TB > kGMaxPasses) return false;
     auto al = [](const void *q, uintptr_t n) { return q == nullptr || reinterpret_cast<uintptr_t>(q) % n == 0; };
@@ -586,26 +601,26 @@ size_t gather_stream_scratch_bytes(int m_total, int K) {
 cudaError_t launch_gather_stream(Ctx *ctx, cudaStream_t st, const void *x, const void *x2, const uint32_t *row_src, int n_src_rows,
                                  const GatherMats *mats, int n_mats, const uint32_t *expert_offsets, int m_total, int n_out, int K,
                                  int n_experts, int group_size, int dtype, void *scratch) {
-    const GPlan p = g_plan(K);
+    const GPlan p = g_plan(K, m_total / n_experts);
     if (p.depth == 0 || n_mats < 1 || n_mats > 2 || (x2 && row_src)) return cudaErrorInvalidValue;
     unsigned char *xfrag = static_cast<unsigned char *>(scratch);
     float *xsum = reinterpret_cast<float *>(xfrag + g_up256(static_cast<size_t>(m_total) * K * 2));
     GTable *table = reinterpret_cast<GTable *>(reinterpret_cast<unsigned char *>(xsum) + g_up256(static_cast<size_t>(m_total) * (K / 64) * 4));
     const bool bf16 = dtype == MTC_BF16;
-    const long long threads = static_cast<long long>(m_total) * (K / 64) * 4;
+    // A permuted product reads every source row top-k times: convert the source rows and let the gather kernel follow row_src
+    const bool follow = row_src != nullptr && n_src_rows <= m_total;
+    const int n_rows = follow ? n_src_rows : m_total;
+    const long long threads = static_cast<long long>(n_rows) * (K / 64) * 4;
     int pgrid = static_cast<int>(std::min<long long>((threads + 255) / 256, 8ll * ctx->sm_count));
     if (pgrid < 1) pgrid = 1;
     auto prep = [&](auto kern) {
-        kern<<<pgrid, 256, 0, st>>>(x, x2, row_src, n_src_rows, expert_offsets, n_experts, m_total, K, p.TB, xfrag, xsum, table, ctx->d_status);
+        return launch_pdl(kern, pgrid, 256, 0, st, x, x2, row_src, n_src_rows, expert_offsets, n_experts, m_total, n_rows, K, p.TB, xfrag, xsum, table,
+                          ctx->d_status);
     };
-    if (x2) {
-        if (bf16) prep(gather_prep_kernel<true, 2>); else prep(gather_prep_kernel<false, 2>);
-    } else if (row_src) {
-        if (bf16) prep(gather_prep_kernel<true, 1>); else prep(gather_prep_kernel<false, 1>);
-    } else {
-        if (bf16) prep(gather_prep_kernel<true, 0>); else prep(gather_prep_kernel<false, 0>);
-    }
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e;
+    if (x2) e = bf16 ? prep(gather_prep_kernel<true, 2>) : prep(gather_prep_kernel<false, 2>);
+    else if (row_src && !follow) e = bf16 ? prep(gather_prep_kernel<true, 1>) : prep(gather_prep_kernel<false, 1>);
+    else e = bf16 ? prep(gather_prep_kernel<true, 0>) : prep(gather_prep_kernel<false, 0>);
     if (e != cudaSuccess) return e;
     GArgs a{};
     a.w = static_cast<const uint32_t *>(mats[0].w);
@@ -627,6 +642,8 @@ cudaError_t launch_gather_stream(Ctx *ctx, cudaStream_t st, const void *x, const
     }
     a.xfrag = xfrag;
     a.xsum = xsum;
+    a.row_src = follow ? row_src : nullptr;
+    a.n_src_rows = n_src_rows;
     a.table = table;
     a.status = ctx->d_status;
     a.n_out = n_out;

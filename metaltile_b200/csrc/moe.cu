@@ -12,10 +12,12 @@ namespace {
 // its lowest index among equals), then the warp takes the maximum value and, among the lanes holding
 // it, the minimum index: ties go to the lower expert index.  Weights: exp(z - max_all) divided by the
 // sum over the chosen k (norm_topk_prob = 1) or over all experts (= 0).
-constexpr int kMaxPerLane = 32;   // n_experts <= 1024
-
+// kMaxPerLane: experts a lane holds; the instance that just fits is launched (with 32 for 128 experts, seven eighths of
+// the unrolled code was predicated off: 10 us instead of 4 for 512 rows).
+template <int kMaxPerLane>
 __global__ void __launch_bounds__(128) router_topk_kernel(const void *logits, uint32_t *indices_out, void *weights_out,
                                                           int n_rows, int n_experts, int k, int norm_topk_prob, int dt) {
+    pdl_enter();
     const int lane = threadIdx.x & 31;
     const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= n_rows) return;
@@ -87,34 +89,44 @@ __global__ void __launch_bounds__(128) router_topk_kernel(const void *logits, ui
 // atomics: a warp only writes its own row), (2) per expert a prefix over the 32 warps and the expert
 // totals, scanned into expert_offsets, (3) the same walk again, now placing: position = first row of the
 // expert + slots of earlier warps + slots of earlier sub-chunks of this warp + rank inside the sub-chunk.
-constexpr int kSortThreads = 1024;
+constexpr int kSortThreads = 1024, kSortHeld = 4;
 
 __global__ void __launch_bounds__(kSortThreads) moe_sort_kernel(const uint32_t *topk_idx, int total, int k, int n_experts,
                                                                 uint32_t *sort_token_idx, uint32_t *inv_perm,
                                                                 uint32_t *expert_offsets, uint32_t *row_expert,
                                                                 uint32_t *status) {
+    pdl_enter();
     extern __shared__ uint32_t sm[];
     uint32_t *cursor = sm;                         // [n_experts + 1] first row of every expert
     uint32_t *wcnt = sm + n_experts + 1;           // [32][n_experts] per-warp counts, then running positions
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int per = ((total + 32 * 32 - 1) / (32 * 32)) * 32;          // slots per warp, whole sub-chunks
     const int f0 = warp * per, f1 = min(f0 + per, total);
+    // the first sub-chunks' ids are read once, all of them in flight, and kept for the second walk
+    uint32_t held[kSortHeld];
+#pragma unroll
+    for (int q = 0; q < kSortHeld; ++q) held[q] = f0 + 32 * q + lane < f1 ? topk_idx[f0 + 32 * q + lane] : 0xFFFFFFFFu;
     for (int i = tid; i < 32 * n_experts; i += kSortThreads) wcnt[i] = 0;
     __syncthreads();
     uint32_t *mine = wcnt + warp * n_experts;
-    for (int c = f0; c < f1; c += 32) {
+    auto count = [&](int c, uint32_t id) {
         const int f = c + lane;
         const bool have = f < f1;
-        const uint32_t e = have ? topk_idx[f] : 0xFFFFFFFFu;
+        const uint32_t e = have ? id : 0xFFFFFFFFu;
         const bool ok = have && e < static_cast<uint32_t>(n_experts);
         if (have && !ok) atomicCAS(status, 0u, 0x501u);        // expert id out of range: recorded, slot skipped
         const uint32_t peers = __match_any_sync(0xffffffffu, ok ? e : 0xFFFFFFFFu);
         if (ok && __popc(peers & ((1u << lane) - 1u)) == 0) mine[e] += __popc(peers);
         __syncwarp();
-    }
+    };
+#pragma unroll
+    for (int q = 0; q < kSortHeld; ++q)
+        if (f0 + 32 * q < f1) count(f0 + 32 * q, held[q]);
+    for (int c = f0 + 32 * kSortHeld; c < f1; c += 32) count(c, c + lane < f1 ? topk_idx[c + lane] : 0xFFFFFFFFu);
     __syncthreads();
     for (int ee = tid; ee < n_experts; ee += kSortThreads) {   // per expert: exclusive prefix over the warps, total
         uint32_t run = 0;
+#pragma unroll 8
         for (int w = 0; w < 32; ++w) {
             const uint32_t c = wcnt[w * n_experts + ee];
             wcnt[w * n_experts + ee] = run;
@@ -140,10 +152,10 @@ __global__ void __launch_bounds__(kSortThreads) moe_sort_kernel(const uint32_t *
     }
     __syncthreads();
     for (int e = tid; e <= n_experts; e += kSortThreads) expert_offsets[e] = cursor[e];
-    for (int c = f0; c < f1; c += 32) {
+    auto place = [&](int c, uint32_t id) {
         const int f = c + lane;
         const bool have = f < f1;
-        const uint32_t e = have ? topk_idx[f] : 0xFFFFFFFFu;
+        const uint32_t e = have ? id : 0xFFFFFFFFu;
         const bool ok = have && e < static_cast<uint32_t>(n_experts);
         const uint32_t peers = __match_any_sync(0xffffffffu, ok ? e : 0xFFFFFFFFu);
         const uint32_t rank = __popc(peers & ((1u << lane) - 1u));
@@ -158,7 +170,11 @@ __global__ void __launch_bounds__(kSortThreads) moe_sort_kernel(const uint32_t *
             inv_perm[f] = pos;
             if (row_expert) row_expert[pos] = e;
         }
-    }
+    };
+#pragma unroll
+    for (int q = 0; q < kSortHeld; ++q)
+        if (f0 + 32 * q < f1) place(f0 + 32 * q, held[q]);
+    for (int c = f0 + 32 * kSortHeld; c < f1; c += 32) place(c, c + lane < f1 ? topk_idx[c + lane] : 0xFFFFFFFFu);
 }
 
 // ---- mt_moe_permute (moe.rs:283-302): permuted[p, :] = tokens[sort_token_idx[p], :] ----------------
@@ -197,14 +213,28 @@ __global__ void __launch_bounds__(256) unpermute_kernel(const void *expert_out, 
 // 16-bit activations, hidden % 8 == 0, 16-byte aligned rows: 8 columns per thread, one 128-bit load per expert row
 __global__ void __launch_bounds__(256) unpermute16_kernel(const uint4 *expert_out, const uint32_t *inv_perm, const void *weights,
                                                           uint4 *out, int n_tokens, int hidden8, int k, int dt) {
+    pdl_enter();
     const int t = blockIdx.x;
     if (t >= n_tokens) return;
     for (int h8 = threadIdx.x; h8 < hidden8; h8 += blockDim.x) {
         float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        for (int j = 0; j < k; ++j) {
-            const uint32_t pos = __ldg(inv_perm + static_cast<size_t>(t) * k + j);
-            const float w = ld_as_f32(weights, static_cast<size_t>(t) * k + j, dt);
-            const uint4 v = __ldg(expert_out + static_cast<size_t>(pos) * hidden8 + h8);
+        // eight expert rows in flight at a time
+        for (int j0 = 0; j0 < k; j0 += 8) {
+          uint4 rows[8];
+          float wts[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            if (j0 + i < k) {
+                const uint32_t pos = inv_perm[static_cast<size_t>(t) * k + j0 + i];
+                wts[i] = ld_as_f32(weights, static_cast<size_t>(t) * k + j0 + i, dt);
+                rows[i] = expert_out[static_cast<size_t>(pos) * hidden8 + h8];
+            }
+          }
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            if (j0 + i >= k) break;
+            const float w = wts[i];
+            const uint4 v = rows[i];
             const uint32_t u[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
@@ -219,6 +249,7 @@ __global__ void __launch_bounds__(256) unpermute16_kernel(const uint4 *expert_ou
                 acc[2 * q] = acc[2 * q] + w * lo;
                 acc[2 * q + 1] = acc[2 * q + 1] + w * hi;
             }
+          }
         }
         uint32_t o[4];
 #pragma unroll
@@ -247,9 +278,10 @@ __global__ void __launch_bounds__(256) swiglu_kernel(const void *gate, const voi
 
 // 16-bit activations, n % 8 == 0, 16-byte aligned: 8 elements per thread
 __global__ void __launch_bounds__(256) swiglu16_kernel(const uint4 *gate, const uint4 *up, uint4 *out, size_t n8, int dt) {
+    pdl_enter();
     for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n8;
          i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-        const uint4 gv = __ldg(gate + i), uv = __ldg(up + i);
+        const uint4 gv = gate[i], uv = up[i];
         const uint32_t g4[4] = {gv.x, gv.y, gv.z, gv.w}, u4[4] = {uv.x, uv.y, uv.z, uv.w};
         uint32_t o[4];
 #pragma unroll
@@ -315,8 +347,10 @@ gather_generic_kernel(const void *x, const uint32_t *w, const void *scales, cons
 cudaError_t launch_router_topk(cudaStream_t st, const void *logits, uint32_t *idx, void *wts, int n_rows, int n_experts,
                                int k, int norm, int dt) {
     if (n_rows <= 0) return cudaSuccess;
-    router_topk_kernel<<<(n_rows + 3) / 4, 128, 0, st>>>(logits, idx, wts, n_rows, n_experts, k, norm, dt);
-    return cudaGetLastError();
+    const int per = (n_experts + 31) / 32;                     // n_experts <= 1024
+    auto *kern = per <= 1 ? router_topk_kernel<1> : per <= 2 ? router_topk_kernel<2> : per <= 4 ? router_topk_kernel<4>
+               : per <= 8 ? router_topk_kernel<8> : router_topk_kernel<32>;
+    return launch_pdl(kern, (n_rows + 3) / 4, 128, 0, st, logits, idx, wts, n_rows, n_experts, k, norm, dt);
 }
 
 cudaError_t launch_moe_sort(cudaStream_t st, const uint32_t *topk_idx, int n_tokens, int k, int n_experts, uint32_t *sti,
@@ -325,8 +359,7 @@ cudaError_t launch_moe_sort(cudaStream_t st, const uint32_t *topk_idx, int n_tok
     static PerDeviceAttr attr;
     cudaError_t e = attr.set(moe_sort_kernel, 200 * 1024);
     if (e != cudaSuccess) return e;
-    moe_sort_kernel<<<1, kSortThreads, smem, st>>>(topk_idx, n_tokens * k, k, n_experts, sti, inv, offsets, row_expert, status);
-    return cudaGetLastError();
+    return launch_pdl(moe_sort_kernel, 1, kSortThreads, smem, st, topk_idx, n_tokens * k, k, n_experts, sti, inv, offsets, row_expert, status);
 }
 
 cudaError_t launch_permute(cudaStream_t st, const void *tokens, const uint32_t *sti, void *permuted, int n_rows, int hidden,
@@ -347,8 +380,8 @@ cudaError_t launch_unpermute(cudaStream_t st, const void *eo, const uint32_t *in
     if (n_tokens <= 0) return cudaSuccess;
     const auto al16 = [](const void *p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
     if (dt != MTC_F32 && hidden % 8 == 0 && al16(eo) && al16(out))
-        unpermute16_kernel<<<n_tokens, 256, 0, st>>>(static_cast<const uint4 *>(eo), inv, wts, static_cast<uint4 *>(out), n_tokens,
-                                                     hidden / 8, k, dt);
+        return launch_pdl(unpermute16_kernel, n_tokens, hidden / 8 >= 256 ? 256 : 128, 0, st, static_cast<const uint4 *>(eo), inv, wts,
+                          static_cast<uint4 *>(out), n_tokens, hidden / 8, k, dt);
     else
         unpermute_kernel<<<n_tokens, 256, 0, st>>>(eo, inv, wts, out, n_tokens, hidden, k, dt);
     return cudaGetLastError();
@@ -362,8 +395,8 @@ cudaError_t launch_swiglu(cudaStream_t st, const void *gate, const void *up, voi
     size_t grid = (work + 255) / 256;
     if (grid > static_cast<size_t>(kNumSMsB200) * 16) grid = static_cast<size_t>(kNumSMsB200) * 16;
     if (vec)
-        swiglu16_kernel<<<static_cast<int>(grid), 256, 0, st>>>(static_cast<const uint4 *>(gate), static_cast<const uint4 *>(up),
-                                                               static_cast<uint4 *>(out), n / 8, dt);
+        return launch_pdl(swiglu16_kernel, static_cast<int>(grid), 256, 0, st, static_cast<const uint4 *>(gate), static_cast<const uint4 *>(up),
+                          static_cast<uint4 *>(out), n / 8, dt);
     else
         swiglu_kernel<<<static_cast<int>(grid), 256, 0, st>>>(gate, up, out, n, dt);
     return cudaGetLastError();

@@ -79,6 +79,7 @@ struct QmmParams {
     int wpr, gpr;                // words / groups per weight row
     int TN;                      // token rows per item (TMA box rows, MMA N)
     int nst;                     // ring depth
+    int kps;                     // k blocks per stage: 1 or 2 (one chunk of few token rows)
     uint32_t hint_ns;            // base suspend-time hint of the waits (0: plain polling)
     int raw;                     // 1: packed words reach the dequant warps through shared memory (cp.async, whole lines)
     uint32_t raw_off, raw_tile;  // byte offset of the raw buffers in shared memory; bytes of one buffer
@@ -489,15 +490,15 @@ __device__ __forceinline__ Item get_item(const QmmParams &p, int i) {
 
 // KSPLIT: the launch cuts K into slices (items carry a first k block, the epilogue writes f32 partial sums); a
 // separate instantiation, so that the code of every other launch is what it was without the feature.
-template <int BITS, bool KSPLIT>
+template <int BITS, bool KSPLIT, int KPS>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w, const QmmParams p) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
     const int nst = p.nst;
-    const uint32_t w_stage = A_BYTES;                                   // one dequantised W tile per stage
+    const uint32_t w_stage = KPS * A_BYTES;                             // KPS dequantised W blocks per stage
     const uint32_t x_stage = static_cast<uint32_t>(p.TN) * BK * 2;      // one X chunk; multiple of 2 KB
-    const uint32_t x_slot = (p.wide ? 2 : 1) * x_stage;                 // one or two X chunks per stage
+    const uint32_t x_slot = KPS == 2 || p.wide ? 2 * x_stage : x_stage;  // two X chunks, or one per k block, per stage (KPS is 1 when wide)
     uint8_t *sW = smem;                                  // nst x w_stage: dequantised weights (A operand)
     uint8_t *sX = smem + nst * w_stage;                  // nst x x_slot: activations (B operand)
     SmemCtrl *ctl = reinterpret_cast<SmemCtrl *>(smem + RING_BYTES + EPI_BYTES);
@@ -542,11 +543,17 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
             if (p.pdl_roles) asm volatile("griddepcontrol.wait;" ::: "memory");      // x may come from the previous kernel
             for (int i = blockIdx.x; i < num_items && ok; i += gridDim.x) {
                 const Item item = get_item<KSPLIT>(p, i);
-                for (int kb = 0; kb < item.nkb; ++kb) {
+                for (int kb = 0; kb < item.nkb; kb += KPS) {
                     if (!(ok = mbar_wait(&ctl->empty[s], ph ^ 1, ctl, p.status, 0x101, p.hint_ns))) break;
-                    mbar_expect_tx(&ctl->full[s], x_bytes * item.nc);
-                    for (int c = 0; c < item.nc; ++c)
-                        tma_load_2d(sX + s * x_slot + c * x_stage, &tmap_x, ((KSPLIT ? item.kb0 : 0) + kb) * BK, item.row0 + c * p.TN, &ctl->full[s]);
+                    const int k0 = ((KSPLIT ? item.kb0 : 0) + kb) * BK;
+                    if constexpr (KPS == 2) {
+                        const int nb = min(2, item.nkb - kb);                 // k blocks of this stage
+                        mbar_expect_tx(&ctl->full[s], x_bytes * nb);
+                        for (int c = 0; c < nb; ++c) tma_load_2d(sX + s * x_slot + c * x_stage, &tmap_x, k0 + c * BK, item.row0, &ctl->full[s]);
+                    } else {
+                        mbar_expect_tx(&ctl->full[s], x_bytes * item.nc);
+                        for (int c = 0; c < item.nc; ++c) tma_load_2d(sX + s * x_slot + c * x_stage, &tmap_x, k0, item.row0 + c * p.TN, &ctl->full[s]);
+                    }
                     if (++s == nst) {
                         s = 0;
                         ph ^= 1;
@@ -583,17 +590,27 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                 if (!(ok = mbar_wait_warp(&ctl->acc_empty[buf], acc_ph ^ 1, ctl, p.status, 0x201, 0))) break;
                 tc_fence_after();
                 const uint32_t tmem_d = tmem_base + buf * TN_MAX;
-                for (int kb = 0; kb < item.nkb; ++kb) {
+                for (int kb = 0; kb < item.nkb; kb += KPS) {
                     if (!(ok = mbar_wait_warp(&ctl->full[s], ph, ctl, p.status, 0x202, 0))) break;
                     tc_fence_after();
                     if (leader) {
                         const uint64_t bdesc = bdesc0 + static_cast<uint64_t>(s * b_step);
                         const uint64_t adesc = adesc0 + static_cast<uint64_t>(s * a_step);
-                        for (int c = 0; c < item.nc; ++c) {          // token chunk c accumulates in TMEM half c
-                            const uint64_t bd = bdesc + static_cast<uint64_t>(c * (x_stage >> 4));
+                        if constexpr (KPS == 2) {                    // two k blocks, one accumulator
+                            const int nb = min(2, item.nkb - kb);
+                            for (int c = 0; c < nb; ++c) {
+                                const uint64_t ad = adesc + static_cast<uint64_t>(c * (A_BYTES >> 4)), bd = bdesc + static_cast<uint64_t>(c * (x_stage >> 4));
 #pragma unroll
-                            for (int k = 0; k < BK / 16; ++k)       // 16 elements = 32 bytes further along the swizzled row
-                                umma_f16(tmem_d + c * TN_MAX, adesc + 2 * k, bd + 2 * k, p.idesc, (kb | k) ? 1u : 0u);
+                                for (int k = 0; k < BK / 16; ++k)
+                                    umma_f16(tmem_d, ad + 2 * k, bd + 2 * k, p.idesc, (kb | c | k) ? 1u : 0u);
+                            }
+                        } else {
+                            for (int c = 0; c < item.nc; ++c) {      // token chunk c accumulates in TMEM half c
+                                const uint64_t bd = bdesc + static_cast<uint64_t>(c * (x_stage >> 4));
+#pragma unroll
+                                for (int k = 0; k < BK / 16; ++k)   // 16 elements = 32 bytes further along the swizzled row
+                                    umma_f16(tmem_d + c * TN_MAX, adesc + 2 * k, bd + 2 * k, p.idesc, (kb | k) ? 1u : 0u);
+                            }
                         }
                         umma_commit(&ctl->empty[s]);         // frees the stage when these MMAs have read it
                     }
@@ -851,7 +868,8 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                         if (kb0 + j >= item.nkb) break;
                         uint32_t wv[BITS];                   // read before the wait for the stage
                         R::read(base, r, j, h, wv);
-                        if (!(ok = mbar_wait_warp(&ctl->empty[s], ph ^ 1, ctl, p.status, 0x401, 0))) break;
+                        const uint32_t sub = KPS == 2 ? j & 1 : 0;              // k block of the stage
+                        if (sub == 0 && !(ok = mbar_wait_warp(&ctl->empty[s], ph ^ 1, ctl, p.status, 0x401, 0))) break;
                         {
                             const unsigned short sr = static_cast<unsigned short>(sb_half(sline, j, h, p.gs_shift));
                             const unsigned short br = static_cast<unsigned short>(sb_half(bline, j, h, p.gs_shift));
@@ -863,8 +881,9 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                                 sc = __uint_as_float(static_cast<uint32_t>(sr) << 16);
                                 bi = __uint_as_float(static_cast<uint32_t>(br) << 16);
                             }
-                            dequant_half<BITS>(wv, sc, bi, dst, s * w_stage);
+                            dequant_half<BITS>(wv, sc, bi, dst, s * w_stage + sub * A_BYTES);
                         }
+                        if (KPS == 2 && sub == 0 && kb0 + j + 1 < item.nkb) continue;
                         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic-proxy stores -> async proxy (MMA)
                         __syncwarp();
                         if (lane == 0) mbar_arrive(&ctl->full[s]);
@@ -1100,18 +1119,13 @@ cudaError_t launch_bits(cudaStream_t st, const CUtensorMap &tmap, const CUtensor
     la[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = la;
     cfg.numAttrs = 1;
-    if (p.ksplit > 1) {
-        auto kern = qmm_tcgen05_kernel<BITS, true>;
-        static PerDeviceAttr attr;
+    auto go = [&](auto kern, PerDeviceAttr &attr) {
         cudaError_t e = attr.set(kern, smem);
-        if (e != cudaSuccess) return e;
-        return cudaLaunchKernelEx(&cfg, kern, tmap, wmap, p);
-    }
-    auto kern = qmm_tcgen05_kernel<BITS, false>;
-    static PerDeviceAttr attr;
-    cudaError_t e = attr.set(kern, smem);
-    if (e != cudaSuccess) return e;
-    return cudaLaunchKernelEx(&cfg, kern, tmap, wmap, p);
+        return e != cudaSuccess ? e : cudaLaunchKernelEx(&cfg, kern, tmap, wmap, p);
+    };
+    static PerDeviceAttr attr[4];
+    if (p.kps == 2) return p.ksplit > 1 ? go(qmm_tcgen05_kernel<BITS, true, 2>, attr[0]) : go(qmm_tcgen05_kernel<BITS, false, 2>, attr[1]);
+    return p.ksplit > 1 ? go(qmm_tcgen05_kernel<BITS, true, 1>, attr[2]) : go(qmm_tcgen05_kernel<BITS, false, 1>, attr[3]);
 }
 
 // X as a 2-D tensor [rows, K] of 16-bit elements, box 64 x TN, 128-byte swizzle; rows past the end read as zero.
@@ -1181,10 +1195,13 @@ void plan_smem(QmmParams &p, Ctx *ctx, int bits) {
             (RING_BYTES - raw_total) / stage >= 2;
     p.raw8 = (p.wpr * 4) % 16 != 0;
     p.sb_words = p.K % (SB_PER_RAW * BK) == 0 && al(p.scales, 16) && al(p.biases, 16) ? 0 : ((2 * SB_PER_RAW * BK) >> p.gs_shift) / 4 + (p.gpr & 1);
-    p.nst = (RING_BYTES - (p.raw ? raw_total : 0)) / stage;
+    // Two k blocks per hand-off where two such stages fit: waits, fence and arrival are paid half as often (64 token rows 0.51 ->
+    // 0.42 us a k block, 128 rows 0.54 -> 0.46); from ~200 rows on the deeper ring is worth more.
+    p.kps = p.raw && !p.wide && (RING_BYTES - raw_total) / (2 * stage) >= 2 ? 2 : 1;
+    p.nst = (RING_BYTES - (p.raw ? raw_total : 0)) / (p.kps * stage);
     if (p.nst > MAX_STAGES) p.nst = MAX_STAGES;
     if (ctx->qmm_max_stages > 0 && p.nst > ctx->qmm_max_stages) p.nst = ctx->qmm_max_stages;
-    p.raw_off = static_cast<uint32_t>(p.nst * stage);
+    p.raw_off = static_cast<uint32_t>(p.nst * p.kps * stage);
 }
 
 void fill_common(QmmParams &p, Ctx *ctx, const void *w, const void *scales, const void *biases, void *out, int N, int K,
@@ -1276,7 +1293,7 @@ DensePlan plan_dense(const Ctx *ctx, int M, int N, int K, int bits, bool may_spl
         const int left = static_cast<int>(units % sms), last_rows = M - (items_m - 1) * 2 * TN;
         const bool tail = form == 1 && units > sms && left > 0 && 2 * left <= sms && last_rows > TN;
         for (int S = 1; S <= 16; ++S) {
-            if (S > 1 && (!ctx->qmm_ksplit || !may_split || S > nsb || (form == 1 && ctx->qmm_wide == 2))) break;
+            if (S > 1 && (!ctx->qmm_ksplit || !may_split || S > nsb || (ctx->qmm_wide != 1 && M > TN_MAX))) break;
             const int kb = S == 1 ? nkb : (nsb + S - 1) / S * SB_PER_RAW;
             const long long full = units * S / sms, rest = units * S % sms;
             double us = full * (kb * kb_us + kItemUs);

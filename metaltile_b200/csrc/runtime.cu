@@ -191,19 +191,20 @@ inline bool stream_takes_single(const Ctx *ctx, int M, int N, int K) {
 //     39.3 -> 27).
 //   4-bit, 16-bit: where the ring kernel of qmv_mma.cu does not go (K % 512 != 0 or group 32; 2880 x 2880 M = 4 7.7 -> 5.0), and at
 //     M = 1 up to 24 Mi codes (4096 x 4096 5.3 -> 4.7; 14336 x 4096 stays with the streaming kernel: 10.3 against 10.9).
-inline bool frag_rule(int M, int N, int K, int bits, int group_size, int dt) {
+inline bool frag_rule(int M, long long N, int K, int bits, int group_size, int dt) {
     const long long codes = static_cast<long long>(N) * K;
     if (dt == MTC_F32) return M >= 5;
     if (M >= 9 && (codes >= (32ll << 20) || group_size % 64 != 0)) return false;
     if (bits != 4) return M >= 2;
-    if (M == 1) return group_size % 64 == 0 && (K % 512 != 0 || codes <= (24ll << 20));
+    if (M == 1) return true;
     return K % 512 != 0 || group_size < 64 || group_size > 256;
 }
-inline bool frag_takes(const Ctx *ctx, int M, int N, int K, int bits, int group_size, int dt, const void *w, const void *scales,
+// rows: weight rows of the launch (N, or those of all fused projections)
+inline bool frag_takes(const Ctx *ctx, int M, long long rows, int N, int K, int bits, int group_size, int dt, const void *w, const void *scales,
                        const void *biases, const void *x) {
     // an option that selects another kernel for these shapes wins over the rule
     const bool by_rule = ctx->qmv_frag == 1 && ctx->qmv_stream == 1 && ctx->qmv_small_m_mma == 1 && ctx->qmv_small_m_tc == 1 &&
-                         frag_rule(M, N, K, bits, group_size, dt);
+                         frag_rule(M, rows, K, bits, group_size, dt);
     return (ctx->qmv_frag == 2 || by_rule) && mtc::qmv_frag_supported(M, N, K, bits, group_size, dt, w, scales, biases, x);
 }
 
@@ -503,7 +504,7 @@ int mtc_qmv(mtc_ctx *ctx, void *stream, const void *w, const void *scales, const
         const int t = try_qmv_tc(ctx, stream, w, scales, biases, x, outs1, 1, M, N, K, bits, group_size, dtype);
         if (t <= 0) return t;
     }
-    if (frag_takes(ctx, M, N, K, bits, group_size, dtype, w, scales, biases, x)) {
+    if (frag_takes(ctx, M, N, N, K, bits, group_size, dtype, w, scales, biases, x)) {
         mtc_qmv_desc d{};
         d.w = w; d.scales = scales; d.biases = biases; d.x = x;
         d.outs[0] = out; d.n_outs = 1;
@@ -591,6 +592,8 @@ int mtc_qmv_batched(mtc_ctx *ctx, void *stream, const mtc_qmv_desc *descs, int n
     if (!ctx) return MTC_ERR_INVALID;
     MTC_ENTER(ctx);
     if (!descs || n < 1 || n > 4) return fail(ctx, MTC_ERR_INVALID, "qmv_batched: 1 to 4 projections");
+    int rows = 0;                       // of all projections: they are one launch
+    for (int i = 0; i < n; ++i) rows += descs[i].N > 0 && descs[i].N < (1 << 28) ? descs[i].N : 0;
     bool fused = stream_takes(ctx, descs[0].M), frag = true, ring = ctx->qmv_small_m_mma != 0;
     for (int i = 0; i < n; ++i) {
         int rc = check_desc(ctx, descs[i], "qmv_batched");
@@ -600,7 +603,7 @@ int mtc_qmv_batched(mtc_ctx *ctx, void *stream, const mtc_qmv_desc *descs, int n
             return fail(ctx, MTC_ERR_INVALID, "qmv_batched: the projections must share x, M, K and dtype");
         fused = fused && d.group_size == descs[0].group_size;
         frag = frag && d.n_outs == 1 && d.bits == descs[0].bits && d.group_size == descs[0].group_size && d.M > 0 && d.N > 0 &&
-               frag_takes(ctx, d.M, d.N, d.K, d.bits, d.group_size, d.dtype, d.w, d.scales, d.biases, d.x);
+               frag_takes(ctx, d.M, rows, d.N, d.K, d.bits, d.group_size, d.dtype, d.w, d.scales, d.biases, d.x);
         ring = ring && d.n_outs == 1 && d.group_size == descs[0].group_size &&
                mtc::qmv_ring_supported(d.M, d.N, d.K, d.bits, d.group_size, d.dtype, d.w, d.scales, d.biases, d.x);
         fused = fused && d.M > 0 && d.N > 0 &&
