@@ -1271,7 +1271,7 @@ struct DensePlan {
     int TN, items_m, ksplit, halves;      // halves: wide items of an incomplete last round that run as two single-chunk items each
     bool wide;
 };
-DensePlan plan_dense(const Ctx *ctx, int M, int N, int K, int bits, bool may_split) {
+DensePlan plan_dense(const Ctx *ctx, int M, int N, int K, int bits) {
     const int n_tiles = (N + BMW - 1) / BMW, nkb = K / BK, nsb = (nkb + SB_PER_RAW - 1) / SB_PER_RAW, sms = ctx->sm_count;
     const auto up16 = [](int v) { return (v + 15) / 16 * 16; };
     if (ctx->qmm_force_tn > 0) return DensePlan{ctx->qmm_force_tn, (M + ctx->qmm_force_tn - 1) / ctx->qmm_force_tn, 1, 0, false};
@@ -1293,7 +1293,7 @@ DensePlan plan_dense(const Ctx *ctx, int M, int N, int K, int bits, bool may_spl
         const int left = static_cast<int>(units % sms), last_rows = M - (items_m - 1) * 2 * TN;
         const bool tail = form == 1 && units > sms && left > 0 && 2 * left <= sms && last_rows > TN;
         for (int S = 1; S <= 16; ++S) {
-            if (S > 1 && (!ctx->qmm_ksplit || !may_split || S > nsb || (ctx->qmm_wide != 1 && M > TN_MAX))) break;
+            if (S > 1 && (!ctx->qmm_ksplit || S > nsb || (ctx->qmm_wide != 1 && M > TN_MAX))) break;
             const int kb = S == 1 ? nkb : (nsb + S - 1) / S * SB_PER_RAW;
             const long long full = units * S / sms, rest = units * S % sms;
             double us = full * (kb * kb_us + kItemUs);
@@ -1308,18 +1308,57 @@ DensePlan plan_dense(const Ctx *ctx, int M, int N, int K, int bits, bool may_spl
     return best;
 }
 
-// out[i] = sum over the K slices of partial[s][i], in slice order, times the factor of its token row
-__global__ void __launch_bounds__(256) ksplit_sum_kernel(const float *partial, const float *tok_scale, void *out, size_t mn, int N, int S, int dt) {
+// out[m, n] = sum over the K slices of partial[s][m, n], in slice order, times the factor of token row m; V outputs of a row per
+// thread (16-byte loads of every slice in flight for V = 4)
+struct SumOuts {
+    void *outs[8];
+    int n_outs;
+    long long ld;
+};
+template <int V>
+__global__ void __launch_bounds__(256) ksplit_sum_kernel(const float *partial, const float *tok_scale, const SumOuts o, int M, int N, int S, int dt) {
+    asm volatile("griddepcontrol.launch_dependents;");
     asm volatile("griddepcontrol.wait;" ::: "memory");       // launched while the product kernel runs
-    for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < mn; i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-        float pv[16];
+    const size_t mn = static_cast<size_t>(M) * N;
+    const uint32_t per_row = N / V;
+    for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < mn / V; i += static_cast<size_t>(gridDim.x) * blockDim.x) {
+        // 32-bit division: more outputs than that never take K slices (their partial sums would not fit the device)
+        const uint32_t m = static_cast<uint32_t>(i) / per_row, n = (static_cast<uint32_t>(i) - m * per_row) * V;
+        float v[V];
+        if constexpr (V == 4) {
+            float4 pv[16];
 #pragma unroll
-        for (int q = 0; q < 16; ++q) pv[q] = q < S ? partial[static_cast<size_t>(q) * mn + i] : 0.0f;
-        float v = pv[0];
+            for (int q = 0; q < 16; ++q)
+                if (q < S) pv[q] = *reinterpret_cast<const float4 *>(partial + static_cast<size_t>(q) * mn + i * 4);
+            v[0] = pv[0].x; v[1] = pv[0].y; v[2] = pv[0].z; v[3] = pv[0].w;
 #pragma unroll
-        for (int q = 1; q < 16; ++q) v += pv[q];
-        if (tok_scale) v *= __ldg(tok_scale + static_cast<uint32_t>(i) / static_cast<uint32_t>(N));
-        st_from_f32(out, i, v, dt);
+            for (int q = 1; q < 16; ++q)
+                if (q < S) { v[0] += pv[q].x; v[1] += pv[q].y; v[2] += pv[q].z; v[3] += pv[q].w; }
+        } else {
+            float pv[16];
+#pragma unroll
+            for (int q = 0; q < 16; ++q)
+                if (q < S) pv[q] = partial[static_cast<size_t>(q) * mn + i];
+            v[0] = pv[0];
+#pragma unroll
+            for (int q = 1; q < 16; ++q)
+                if (q < S) v[0] += pv[q];
+        }
+        if (tok_scale) {
+            const float f = tok_scale[m];
+#pragma unroll
+            for (int e = 0; e < V; ++e) v[e] *= f;
+        }
+        for (int d = 0; d < o.n_outs; ++d) {
+            const size_t at = static_cast<size_t>(m) * o.ld + n;
+            if (V == 4 && o.ld % 4 == 0 && reinterpret_cast<uintptr_t>(o.outs[d]) % 8 == 0) {
+                *reinterpret_cast<uint2 *>(static_cast<unsigned short *>(o.outs[d]) + at) =
+                    make_uint2(pack_out(v[0], v[V > 1 ? 1 : 0], dt == MTC_F16), pack_out(v[V > 2 ? 2 : 0], v[V > 3 ? 3 : 0], dt == MTC_F16));
+            } else {
+#pragma unroll
+                for (int e = 0; e < V; ++e) st_from_f32(o.outs[d], at + e, v[e], dt);
+            }
+        }
     }
 }
 
@@ -1338,7 +1377,7 @@ cudaError_t launch_qmm_tcgen05(Ctx *ctx, cudaStream_t st, const void *w, const v
                                const void *x, void *out, int M, int N, int K, int bits, int group_size, int dt,
                                std::string *why, void *const *outs, int n_outs, long long out_ld) {
     const int sms = ctx->sm_count;
-    const DensePlan plan = plan_dense(ctx, M, N, K, bits, outs == nullptr);
+    const DensePlan plan = plan_dense(ctx, M, N, K, bits);
     const int TN = plan.TN;
     const void *x_op = nullptr;
     const float *tok_scale = nullptr;
@@ -1378,19 +1417,15 @@ cudaError_t launch_qmm_tcgen05(Ctx *ctx, cudaStream_t st, const void *w, const v
     const int grid = p.dense_items < sms ? p.dense_items : sms;
     e = launch_any(bits, st, tmap, p, grid, N, why);
     if (e != cudaSuccess || p.ksplit == 1) return e;
-    const size_t mn = static_cast<size_t>(M) * N;
-    size_t sgrid = (mn + 255) / 256;
+    const bool vec = N % 4 == 0;
+    size_t sgrid = (static_cast<size_t>(M) * N / (vec ? 4 : 1) + 255) / 256;
     if (sgrid > static_cast<size_t>(sms) * 8) sgrid = static_cast<size_t>(sms) * 8;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(static_cast<unsigned>(sgrid));
-    cfg.blockDim = dim3(256);
-    cfg.stream = st;
-    cudaLaunchAttribute la[1];
-    la[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    la[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = la;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, ksplit_sum_kernel, static_cast<const float *>(p.partial), p.tok_scale, out, mn, N, p.ksplit, dt);
+    SumOuts so{};
+    for (int i = 0; i < p.n_outs; ++i) so.outs[i] = p.outs[i];
+    so.n_outs = p.n_outs;
+    so.ld = p.out_ld;
+    return launch_pdl(vec ? ksplit_sum_kernel<4> : ksplit_sum_kernel<1>, static_cast<int>(sgrid), 256, 0, st, static_cast<const float *>(p.partial),
+                      p.tok_scale, so, M, N, p.ksplit, dt);
 }
 
 // scratch bytes the gather work list needs for these sizes
