@@ -54,7 +54,7 @@ struct FragArgs {
 
 namespace frag {
 
-constexpr int kWarps = 8, kThreads = 32 * kWarps;
+constexpr int kMaxWarps = 16;                  // 8 warps a CTA and two CTAs an SM, or 16 warps where there are few tiles
 enum { S1 = 0, S2 = 1, S4 = 2, G8 = 3 };
 
 template <int BITS>
@@ -159,6 +159,39 @@ __device__ __forceinline__ void ldg2(const void *p, uint32_t *v, bool on) {
                  : "+r"(v[0]) : "l"(p), "r"(static_cast<uint32_t>(on)));
 }
 
+// ... and the plain ones, where the whole run lies inside the row
+__device__ __forceinline__ void ldg16(const void *p, uint32_t *v) {
+    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "l"(p));
+}
+__device__ __forceinline__ void ldg8(const void *p, uint32_t *v) {
+    asm volatile("ld.global.nc.v2.u32 {%0,%1}, [%2];" : "=r"(v[0]), "=r"(v[1]) : "l"(p));
+}
+__device__ __forceinline__ void ldg4(const void *p, uint32_t *v) { asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v[0]) : "l"(p)); }
+__device__ __forceinline__ void ldg2(const void *p, uint32_t *v) {
+    unsigned short h;
+    asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(h) : "l"(p));
+    v[0] = h;
+}
+template <int BITS, int MODE>
+__device__ __forceinline__ void load_words(const char *p, uint32_t (&w)[BITS]) {
+    if constexpr (MODE == G8 && BITS == 4) {
+        ldg8(p, w);
+        ldg8(p + 32, w + 2);
+    } else if constexpr (MODE == G8) {
+        ldg16(p, w);
+        ldg16(p + 64, w + 4);
+    } else if constexpr (BITS % 4 == 0) {
+#pragma unroll
+        for (int i = 0; i < BITS; i += 4) ldg16(p + 4 * i, w + i);
+    } else if constexpr (BITS % 2 == 0) {
+#pragma unroll
+        for (int i = 0; i < BITS; i += 2) ldg8(p + 4 * i, w + i);
+    } else {
+#pragma unroll
+        for (int i = 0; i < BITS; ++i) ldg4(p + 4 * i, w + i);
+    }
+}
+
 // One row's packed words of one step for this lane.  p: the lane's words of the step in the row (S modes: chunk t; G8: its 16
 // codes of the first half, the second half is HALF bytes further on); on0, on1: whether they lie inside the row.
 template <int BITS, int MODE>
@@ -196,6 +229,11 @@ template <int XT>
 __device__ __forceinline__ void ld_scale(const char *p, uint32_t *v, bool on) {
     if (XT == MTC_F32) ldg4(p, v, on);
     else ldg2(p, v, on);
+}
+template <int XT>
+__device__ __forceinline__ void ld_scale(const char *p, uint32_t *v) {
+    if (XT == MTC_F32) ldg4(p, v);
+    else ldg2(p, v);
 }
 
 // The 32 activations of (step, token, quad lane t) as 16 B registers per piece: block (s*Mp + m)*4 + t of kPitch bytes (Mp = columns for tokens), 64
@@ -351,7 +389,7 @@ struct Affine {
 
 // ---- kernel ----------------------------------------------------------------------------------------------------------
 template <int BITS, int XT, int MODE, int NT, int VEC>
-__global__ void __launch_bounds__(kThreads, 2) qmv_frag_kernel(const __grid_constant__ FragArgs a) {
+__global__ void __launch_bounds__(32 * kMaxWarps, 1) qmv_frag_kernel(const __grid_constant__ FragArgs a) {
     constexpr int RUN = (MODE == G8 && !VEC) ? 2 : kRun<BITS>;
     constexpr int H = MODE == G8 ? 2 : 1;
     constexpr int CAP = kCap<MODE>, MP = CAP * NT;
@@ -360,7 +398,7 @@ __global__ void __launch_bounds__(kThreads, 2) qmv_frag_kernel(const __grid_cons
     constexpr int ESZ = XT == MTC_F32 ? 4 : 2;
     extern __shared__ __align__(128) char smem[];
     const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const int slots = kWarps / a.ks, slot = warp / a.ks, slice = warp - slot * a.ks;
+    const int nwarps = blockDim.x >> 5, slots = nwarps / a.ks, slot = warp / a.ks, slice = warp - slot * a.ks;
     const int total_runs = (a.steps + RUN - 1) / RUN;
     const int r0 = slice * total_runs / a.ks, r1 = (slice + 1) * total_runs / a.ks;
     char *part = smem + warp * a.warp_bytes;
@@ -399,38 +437,48 @@ __global__ void __launch_bounds__(kThreads, 2) qmv_frag_kernel(const __grid_cons
     };
     const int n_units = MODE == G8 ? a.K >> 6 : a.K >> 5;                          // halves (G8) or chunks of a row
     const char *pl = nullptr, *ph = nullptr, *ps[2] = {nullptr, nullptr}, *pb[2] = {nullptr, nullptr};    // of the run being requested
+    bool whole = true;                        // the run being requested lies inside the row (VEC: all do)
     auto request_words = [&](int i, int limit) {
-        bool on0 = limit > 0, on1 = on0;
-        if constexpr (VEC == 0) {             // the last run of a row may be partial
+        if (limit == 0) return;               // nothing left for this warp (uniform)
+        if (VEC != 0 || whole) {
+            load_words<BITS, MODE>(pl + i * (16 * BITS), wl[i]);
+            load_words<BITS, MODE>(ph + i * (16 * BITS), wh[i]);
+        } else {
             const int s = l_run * RUN + i;
-            on0 = (MODE == G8 ? 2 * s : 4 * s + t) < limit;
-            on1 = 2 * s + 1 < limit;
+            const bool on0 = (MODE == G8 ? 2 * s : 4 * s + t) < limit, on1 = 2 * s + 1 < limit;
+            load_words<BITS, MODE>(pl + i * (16 * BITS), wl[i], on0, on1);
+            load_words<BITS, MODE>(ph + i * (16 * BITS), wh[i], on0, on1);
         }
-        load_words<BITS, MODE>(pl + i * (16 * BITS), wl[i], on0, on1);
-        load_words<BITS, MODE>(ph + i * (16 * BITS), wh[i], on0, on1);
     };
     auto request_affine = [&](const char *const (&p)[2], Affine<XT, MODE, RUN, VEC> &f, int i, int limit) {   // VEC: the whole run, i unused
+        if (limit == 0) return;
         if constexpr (VEC != 0) {
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
-                if constexpr (VEC == 6) ldg16(p[j], f.r[j], limit > 0);
-                else ldg8(p[j], f.r[j], limit > 0);
+                if constexpr (VEC == 6) ldg16(p[j], f.r[j]);
+                else ldg8(p[j], f.r[j]);
             }
         } else {
 #pragma unroll
             for (int h = 0; h < H; ++h) {
                 const int s = l_run * RUN + i;
                 const int k = MODE == G8 ? 128 * s + 64 * h : MODE == S4 ? 128 * s + 64 * (t >> 1) : 128 * s + 32 * t;
-                const bool in = (MODE == G8 ? 2 * s + h : MODE == S4 ? 4 * s + 2 * (t >> 1) : 4 * s + t) < limit;
                 const uint32_t off = static_cast<uint32_t>(k >> a.gs_shift) * ESZ;
+                if (whole) {
 #pragma unroll
-                for (int j = 0; j < 2; ++j) ld_scale<XT>(p[j] + off, &f.r[j][i * H + h], in);
+                    for (int j = 0; j < 2; ++j) ld_scale<XT>(p[j] + off, &f.r[j][i * H + h]);
+                } else {
+                    const bool in = (MODE == G8 ? 2 * s + h : MODE == S4 ? 4 * s + 2 * (t >> 1) : 4 * s + t) < limit;
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) ld_scale<XT>(p[j] + off, &f.r[j][i * H + h], in);
+                }
             }
         }
     };
     auto open_run = [&]() {
         const uint32_t run_w = static_cast<uint32_t>(l_run) * (RUN * 16 * BITS);
         const uint32_t run_a = VEC ? static_cast<uint32_t>(l_run) * (VEC == 6 ? 16 : 8) : 0u;
+        whole = (l_run + 1) * (RUN * 128) <= a.K;
         pl = wbase + (wo[0] + run_w);
         ph = wbase + (wo[1] + run_w);
 #pragma unroll
@@ -567,7 +615,7 @@ __global__ void __launch_bounds__(kThreads, 2) qmv_frag_kernel(const __grid_cons
                 if constexpr (VEC != 0) sc = sc_next;
             }
             // this warp's partial tile: [token][16 rows]
-            float *mine = red + (buf * kWarps + warp) * (MP * 16);
+            float *mine = red + (buf * nwarps + warp) * (MP * 16);
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
@@ -586,11 +634,11 @@ __global__ void __launch_bounds__(kThreads, 2) qmv_frag_kernel(const __grid_cons
         if (++buf == a.nred || it + 1 == a.iters) {
             __syncthreads();
             const int round0 = it + 1 - buf, n = buf * slots * MP * 16;
-            for (int e = threadIdx.x; e < n; e += kThreads) {
+            for (int e = threadIdx.x; e < n; e += blockDim.x) {
                 const int row = e & 15, tok = (e >> 4) % MP, ts = (e >> 4) / MP, rs = ts / slots, sl = ts - rs * slots;
                 const int tl = ((round0 + rs) * static_cast<int>(gridDim.x) + static_cast<int>(blockIdx.x)) * slots + sl;
                 if (tl >= a.tiles || tok >= a.M) continue;
-                const float *base = red + (rs * kWarps + sl * a.ks) * (MP * 16) + tok * 16 + row;
+                const float *base = red + (rs * nwarps + sl * a.ks) * (MP * 16) + tok * 16 + row;
                 float v = base[0];
                 for (int q = 1; q < a.ks; ++q) v += base[q * (MP * 16)];
                 int pi = 0;
@@ -626,20 +674,22 @@ cudaError_t launch_one(cudaStream_t st, FragArgs a, int sms) {
     int best_grid = 0;
     size_t best_smem = 0;
     FragArgs pick = a;
-    for (int per_sm = 2; per_sm >= 1; --per_sm) {
-        for (int ks = kWarps; ks >= 1; ks >>= 1) {
-            const int slots = kWarps / ks;
+    int best_warps = 8;
+    for (int form = 0; form < 3; ++form) {                     // 8 warps and two CTAs an SM, 16 warps, 8 warps and one CTA
+        const int nw = form == 1 ? 16 : 8, per_sm = form == 0 ? 2 : 1;
+        for (int ks = nw; ks >= 1; ks >>= 1) {
+            const int slots = nw / ks;
             const int want = (a.tiles + slots - 1) / slots;
             const int grid = want < sms * per_sm ? want : sms * per_sm;
             const int iters = (a.tiles + grid * slots - 1) / (grid * slots);
             const int runs = (total_runs + ks - 1) / ks;
-            constexpr size_t kTileRed = static_cast<size_t>(kWarps) * kCap<MODE> * NT * 64;      // partial sums of one round
-            int nred = static_cast<int>(24 * 1024 / kTileRed);
+            const size_t tile_red = static_cast<size_t>(nw) * kCap<MODE> * NT * 64;              // partial sums of one round
+            int nred = static_cast<int>(24 * 1024 / tile_red);
             nred = nred < 1 ? 1 : nred > iters ? iters : nred;
-            const size_t red = nred * kTileRed;
+            const size_t red = nred * tile_red;
             const size_t limit = per_sm == 2 ? kSmemTwo : kSmemMax;
             if (red >= limit) continue;
-            int blk = static_cast<int>((limit - red) / kWarps / 128 * 128 / (RUN * step_bytes));
+            int blk = static_cast<int>((limit - red) / nw / 128 * 128 / (RUN * step_bytes));
             if (blk < 1) continue;
             if (blk > runs) blk = runs;
             const bool resident = blk >= runs;
@@ -648,11 +698,12 @@ cudaError_t launch_one(cudaStream_t st, FragArgs a, int sms) {
             const int on_sm = (grid + sms - 1) / sms;
             const double staging = (4.0 * a.M * (P == 3 ? 260 : 45) / 32 + 20) / 65 * runs * RUN;
             const double warp_cost = iters * (runs * RUN + 1.0) + staging * (resident ? 1 : iters);
-            // a CTA alone on its SM has half the warps to hide latency with
-            const double cost = kWarps * warp_cost * on_sm * (on_sm > 1 ? 1.0 : 1.5);
+            // fewer than 16 warps on an SM have half as many to hide latency with
+            const double cost = nw * warp_cost * on_sm * (nw * on_sm >= 16 ? 1.0 : 1.5);
             if (cost < best - 1e-9) {
                 best = cost;
                 best_grid = grid;
+                best_warps = nw;
                 pick.ks = ks;
                 pick.iters = iters;
                 pick.blk_runs = blk;
@@ -660,8 +711,8 @@ cudaError_t launch_one(cudaStream_t st, FragArgs a, int sms) {
                 const size_t part = (blk * RUN * step_bytes + 127) / 128 * 128;
                 pick.warp_bytes = static_cast<uint32_t>(part);
                 pick.off_sum = static_cast<uint32_t>(blk * RUN * kFrags);
-                pick.off_red = static_cast<uint32_t>(kWarps * part);
-                best_smem = kWarps * part + red;
+                pick.off_red = static_cast<uint32_t>(nw * part);
+                best_smem = nw * part + red;
             }
         }
     }
@@ -672,7 +723,7 @@ cudaError_t launch_one(cudaStream_t st, FragArgs a, int sms) {
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(best_grid);
-    cfg.blockDim = dim3(kThreads);
+    cfg.blockDim = dim3(32 * best_warps);
     cfg.dynamicSmemBytes = best_smem;
     cfg.stream = st;
     cudaLaunchAttribute la[1];

@@ -183,28 +183,33 @@ inline bool stream_takes_single(const Ctx *ctx, int M, int N, int K) {
 }
 
 // The fragment kernel (qmv_frag.cuh) against the other small-M kernels, measured with cold weights (us, other kernel -> it).
-//   widths other than 4-bit, 16-bit activations, 2 <= M: 8-bit 4096 x 4096 M = 4 13.7 -> 7.2, M = 8 19.9 -> 8.6; 3-bit group 32
-//     8192 x 8192 M = 4 32.5 -> 21.5 (CUDA cores spend one FFMA per code and token).  From M = 9 on the tcgen05 kernel with K
-//     slices is the other one: 4096 x 4096 19 -> 12-17, but 8192 x 8192 49 -> 60, hence the limit on codes; groups of 32
-//     need twice the tiles of columns there (19 -> 25).
+//   M = 1: a decode step that stays on one kernel overlaps its launches best (32 layers, 4-bit: streaming kernel 1.40 ms,
+//     fragment kernel 1.27, a mixture of the two 1.67; 8-bit 6 layers 382 -> 317).  By itself the CUDA-core kernel is faster
+//     on large matrices of 2, 3 and 6 bits (3-bit 16384 x 16384 46 against 60) and on every 5-bit one.
+//   2 <= M <= 4, widths other than 4-bit: 8-bit 16384 x 16384 M = 4 182 -> 70; 3-bit group 32 8192 x 8192 M = 4 32.5 -> 21.5 (CUDA
+//     cores spend one FFMA per code and token).
+//   5 <= M <= 8: 8-bit 4096 x 4096 19.9 -> 8.6, until the activations of a row no longer fit an SM (K > 8192), where the tcgen05
+//     kernel takes matrices of 32 Mi codes on.
+//   M >= 9: the tcgen05 kernel's time does not grow with M; this one keeps the small matrices (8-bit 4096 x 4096 14.4 -> 10.6) and,
+//     as one launch instead of three a projection, fused ones whose activations fit an SM (8-bit, 6 layers 823 -> 690).
 //   f32 activations: three pieces per value, so the FFMA kernel wins below M = 5 (M = 4: 14.0 against 16.8), not above (M = 16
-//     39.3 -> 27).
-//   4-bit, 16-bit: where the ring kernel of qmv_mma.cu does not go (K % 512 != 0 or group 32; 2880 x 2880 M = 4 7.7 -> 5.0), and at
-//     M = 1 up to 24 Mi codes (4096 x 4096 5.3 -> 4.7; 14336 x 4096 stays with the streaming kernel: 10.3 against 10.9).
-inline bool frag_rule(int M, long long N, int K, int bits, int group_size, int dt) {
-    const long long codes = static_cast<long long>(N) * K;
+//     39.3 -> 25).
+//   4-bit, 2 <= M: where the ring kernel of qmv_mma.cu does not go (K % 512 != 0 or group 32; 2880 x 2880 M = 4 7.7 -> 5.0).
+inline bool frag_rule(int M, long long N, int K, int bits, int group_size, int dt, bool fused) {
+    const long long codes = N * K;
     if (dt == MTC_F32) return M >= 5;
-    if (M >= 9 && (codes >= (32ll << 20) || group_size % 64 != 0)) return false;
-    if (bits != 4) return M >= 2;
-    if (M == 1) return true;
-    return K % 512 != 0 || group_size < 64 || group_size > 256;
+    if (M == 1) return bits == 4 || bits == 8 || (bits != 5 && (fused || codes <= (64ll << 20)));
+    if (bits == 4 && K % 512 == 0 && group_size >= 64 && group_size <= 256) return false;
+    if (M <= 4) return true;
+    if (M <= 8) return K <= 8192 || codes < (32ll << 20);
+    return group_size % 64 == 0 && K <= 5120 && codes <= (fused ? 128ll << 20 : 20ll << 20);
 }
 // rows: weight rows of the launch (N, or those of all fused projections)
-inline bool frag_takes(const Ctx *ctx, int M, long long rows, int N, int K, int bits, int group_size, int dt, const void *w, const void *scales,
+inline bool frag_takes(const Ctx *ctx, int M, long long rows, bool fused, int N, int K, int bits, int group_size, int dt, const void *w, const void *scales,
                        const void *biases, const void *x) {
     // an option that selects another kernel for these shapes wins over the rule
     const bool by_rule = ctx->qmv_frag == 1 && ctx->qmv_stream == 1 && ctx->qmv_small_m_mma == 1 && ctx->qmv_small_m_tc == 1 &&
-                         frag_rule(M, rows, K, bits, group_size, dt);
+                         frag_rule(M, rows, K, bits, group_size, dt, fused);
     return (ctx->qmv_frag == 2 || by_rule) && mtc::qmv_frag_supported(M, N, K, bits, group_size, dt, w, scales, biases, x);
 }
 
@@ -504,7 +509,7 @@ int mtc_qmv(mtc_ctx *ctx, void *stream, const void *w, const void *scales, const
         const int t = try_qmv_tc(ctx, stream, w, scales, biases, x, outs1, 1, M, N, K, bits, group_size, dtype);
         if (t <= 0) return t;
     }
-    if (frag_takes(ctx, M, N, N, K, bits, group_size, dtype, w, scales, biases, x)) {
+    if (frag_takes(ctx, M, N, false, N, K, bits, group_size, dtype, w, scales, biases, x)) {
         mtc_qmv_desc d{};
         d.w = w; d.scales = scales; d.biases = biases; d.x = x;
         d.outs[0] = out; d.n_outs = 1;
@@ -603,7 +608,7 @@ int mtc_qmv_batched(mtc_ctx *ctx, void *stream, const mtc_qmv_desc *descs, int n
             return fail(ctx, MTC_ERR_INVALID, "qmv_batched: the projections must share x, M, K and dtype");
         fused = fused && d.group_size == descs[0].group_size;
         frag = frag && d.n_outs == 1 && d.bits == descs[0].bits && d.group_size == descs[0].group_size && d.M > 0 && d.N > 0 &&
-               frag_takes(ctx, d.M, rows, d.N, d.K, d.bits, d.group_size, d.dtype, d.w, d.scales, d.biases, d.x);
+               frag_takes(ctx, d.M, rows, n > 1, d.N, d.K, d.bits, d.group_size, d.dtype, d.w, d.scales, d.biases, d.x);
         ring = ring && d.n_outs == 1 && d.group_size == descs[0].group_size &&
                mtc::qmv_ring_supported(d.M, d.N, d.K, d.bits, d.group_size, d.dtype, d.w, d.scales, d.biases, d.x);
         fused = fused && d.M > 0 && d.N > 0 &&
