@@ -116,9 +116,9 @@ __device__ __forceinline__ void pdl_enter() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 template <typename... P, typename... A>
-cudaError_t launch_pdl(void (*kern)(P...), int grid, int block, size_t smem, cudaStream_t st, A... args) {
+cudaError_t launch_pdl(void (*kern)(P...), dim3 grid, int block, size_t smem, cudaStream_t st, A... args) {
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
+    cfg.gridDim = grid;
     cfg.blockDim = dim3(block);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
@@ -236,7 +236,7 @@ size_t moe_decode_smem_bytes(int n_slots, int in_dim);
 cudaError_t launch_moe_decode(Ctx *ctx, cudaStream_t st, const void *const *gate, const void *const *up, const void *experts,
                               const void *slot_w, const void *w, const void *scales, const void *biases, void *out, int n_slots, int in_dim,
                               int out_dim, int n_experts, int group_size, int dt, int fused, float *staged);
-int qvm_k_chunks(int sms, int N, int K, int bits, int group_size);
+int qvm_k_chunks(int sms, int M, int N, int K, int bits, int group_size, int dt);
 bool qvm_fast_supported(int N, int K, int bits, int group_size);
 cudaError_t launch_qvm(Ctx *ctx, cudaStream_t st, const void *w, const void *scales, const void *biases, const void *x, void *out,
                        int M, int N, int K, int bits, int group_size, int dt, void *scratch, int KC);

@@ -1,0 +1,35 @@
+"""The codec kernels that give a lane 8 consecutive values, four times: every group size that a warp reduces in its own
+way (4 to 32 lanes of a unit, two and four units), a tail that ends inside a warp's 1024 values, and a group size that
+is not a power of two.  Codes, scales, biases and values are compared for equality."""
+import numpy as np
+import pytest
+
+import oracle
+from helpers import ODT, to_dev
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dt", ["f32", "f16", "bf16"])
+@pytest.mark.parametrize("bits", [2, 3, 4, 5, 6, 8])
+@pytest.mark.parametrize("gs", [32, 64, 96, 128, 256, 512, 1024])
+def test_codec_is_exact(bits, gs, dt):
+    import torch
+    from metaltile_b200 import ops
+    rng = np.random.default_rng(gs * 10 + bits)
+    n = 1024 // gs * 3 + 1 if gs <= 512 else 3            # groups: one row each, total not a multiple of 1024 values
+    wf = rng.standard_normal((n, gs)) * np.exp2(rng.integers(-12, 8, size=(n, 1)))
+    wf[0] = 0.25                                          # a constant group: the scale is 1
+    if n > 1:
+        wf[1, :] = np.linspace(-1.0, 1.0, gs)             # values that fall on code boundaries
+    wf = oracle.round_through(wf.astype(np.float32), ODT[dt])
+    q, s, b = ops.affine_quantize(to_dev(wf, dt), bits, gs)
+    back = ops.affine_dequantize(q, s, b, bits, gs)
+    torch.cuda.synchronize()
+    oq, osc, obi = oracle.affine_quantize(wf, bits, gs)
+    assert np.array_equal(q.cpu().numpy().view(np.uint32).reshape(-1), oq)
+    s_h, b_h = s.float().cpu().numpy().reshape(-1), b.float().cpu().numpy().reshape(-1)
+    assert np.array_equal(s_h, oracle.round_through(osc, ODT[dt]))
+    assert np.array_equal(b_h, oracle.round_through(obi, ODT[dt]))
+    ref = oracle.round_through(oracle.affine_dequantize(oq, s_h, b_h, n * gs, bits, gs), ODT[dt])
+    assert np.array_equal(back.float().cpu().numpy().reshape(-1), ref)
