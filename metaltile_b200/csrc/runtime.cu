@@ -935,7 +935,7 @@ int mtc_qvm(mtc_ctx *ctx, void *stream, const void *w, const void *scales, const
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     int kc = 1;
     if (mtc::qvm_fast_supported(N, K, bits, group_size)) {
-        kc = mtc::qvm_k_chunks(ctx->sm_count, N, K, bits, group_size);
+        kc = mtc::qvm_k_chunks(ctx->sm_count, M, N, K, bits, group_size, dtype);
         if (kc > 1) {
             std::string why;
             void *before = ctx->d_qvm;
