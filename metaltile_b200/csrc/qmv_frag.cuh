@@ -22,8 +22,9 @@
 //       S4  chunks 0, 1 meet columns 0-3, chunks 2, 3 columns 4-7: four tokens a tile, groups that are multiples of 64;
 //       G   (4- and 8-bit) lane t takes 16 codes of each 64-code half instead of 32 codes of the step: eight tokens a
 //           tile, two accumulators a step, groups that are multiples of 64.
-//   * every warp stages the activations of its own slice (fragment order, 256 bytes per step and token) and their sums,
-//     which come out of the same MMA against codes that are all one: no CTA barrier before the products.
+//   * every warp stages the activations of its own slice (fragment order, 256 bytes per step and token) and their sums, which
+//     a lane adds up from the activations it stages (through MMAs against codes that are all one they were 0.6-1.1 us of a
+//     decode launch: 4096 x 4096, M = 1, 4.46 -> 3.79 us; 4096 x 14336 10.7 -> 9.5 us): no CTA barrier before the products.
 //   * the KS partial tiles are added in shared memory in warp order, once per launch where they fit: deterministic.
 #pragma once
 
@@ -242,8 +243,9 @@ __device__ __forceinline__ void ld_scale(const char *p, uint32_t *v) {
 template <int XT>
 constexpr int kPitch = 64 * kPieces<XT> + 16;
 
+// Returns the sum of the 32 activations (not for G8, whose two halves have sums of their own).
 template <int BITS, int XT, int MODE>
-__device__ __forceinline__ void stage_chunk(const FragArgs &a, int m, int k_lo, int k_hi, char *dst) {
+__device__ __forceinline__ float stage_chunk(const FragArgs &a, int m, int k_lo, int k_hi, char *dst) {
     // k_lo: first activation of registers 0-7, k_hi: of registers 8-15 (16 values each; both inside or outside the row)
     constexpr bool BF = XT != MTC_F16;
     if constexpr (XT == MTC_F32) {
@@ -254,6 +256,11 @@ __device__ __forceinline__ void stage_chunk(const FragArgs &a, int m, int k_lo, 
             const int k = (q < 4 ? k_lo : k_hi - 16) + 4 * q;
             const float4 f = k < a.K && m < a.M ? *reinterpret_cast<const float4 *>(x + k) : make_float4(0.f, 0.f, 0.f, 0.f);
             v[4 * q] = f.x; v[4 * q + 1] = f.y; v[4 * q + 2] = f.z; v[4 * q + 3] = f.w;
+        }
+        float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        if (MODE != G8) {
+#pragma unroll
+            for (int q = 0; q < 32; ++q) sum[q & 3] += v[q];
         }
         uint32_t o[3][4];
 #pragma unroll
@@ -273,6 +280,7 @@ __device__ __forceinline__ void stage_chunk(const FragArgs &a, int m, int k_lo, 
                     *reinterpret_cast<uint4 *>(dst + p * 64 + ((r >> 2) << 4)) = make_uint4(o[p][0], o[p][1], o[p][2], o[p][3]);
             }
         }
+        return (sum[0] + sum[1]) + (sum[2] + sum[3]);
     } else {
         uint32_t u[16];
         const uint16_t *x = static_cast<const uint16_t *>(a.x) + static_cast<size_t>(m) * a.K;
@@ -281,6 +289,16 @@ __device__ __forceinline__ void stage_chunk(const FragArgs &a, int m, int k_lo, 
             const int k = (q < 2 ? k_lo : k_hi - 16) + 8 * q;
             const uint4 f = k < a.K && m < a.M ? *reinterpret_cast<const uint4 *>(x + k) : make_uint4(0u, 0u, 0u, 0u);
             u[4 * q] = f.x; u[4 * q + 1] = f.y; u[4 * q + 2] = f.z; u[4 * q + 3] = f.w;
+        }
+        float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        if (MODE != G8) {
+#pragma unroll
+            for (int q = 0; q < 16; ++q) {
+                const float2 f = BF ? make_float2(__uint_as_float(u[q] << 16), __uint_as_float(u[q] & 0xFFFF0000u))
+                                    : __half22float2(*reinterpret_cast<const __half2 *>(&u[q]));
+                sum[2 * (q & 1)] += f.x;
+                sum[2 * (q & 1) + 1] += f.y;
+            }
         }
         uint32_t o[4];
 #pragma unroll
@@ -294,6 +312,7 @@ __device__ __forceinline__ void stage_chunk(const FragArgs &a, int m, int k_lo, 
             o[r & 3] = b;
             if ((r & 3) == 3) *reinterpret_cast<uint4 *>(dst + ((r >> 2) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
         }
+        return (sum[0] + sum[1]) + (sum[2] + sum[3]);
     }
 }
 
@@ -521,14 +540,26 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1) qmv_frag_kernel(const __gri
     auto stage = [&](int from, int to) {
         __syncwarp();
         const int n = (to - from) * RUN * 4 * MP;
-        for (int e = lane; e < n; e += 32) {
-            const int et = e & 3, em = (e >> 2) % MP, es = (e >> 2) / MP;
+        for (int e0 = 0; e0 < n; e0 += 32) {
+            const int e = e0 + lane, et = e & 3, em = (e >> 2) % MP, es = (e >> 2) / MP;
             const int k = (from * RUN + es) * 128;
-            stage_chunk<BITS, XT, MODE>(a, em, MODE == G8 ? k + 16 * et : k + 32 * et, MODE == G8 ? k + 64 + 16 * et : k + 32 * et + 16,
-                                        part + static_cast<size_t>(e) * kPitch<XT>);
+            float sum = 0.0f;
+            if (e < n)
+                sum = stage_chunk<BITS, XT, MODE>(a, em, MODE == G8 ? k + 16 * et : k + 32 * et, MODE == G8 ? k + 64 + 16 * et : k + 32 * et + 16,
+                                                  part + static_cast<size_t>(e) * kPitch<XT>);
+            if (MODE != G8) {
+                // in the units of the products: x times 2^64 against codes times 2^-133, f16: codes times 2^-24
+                constexpr uint32_t unit = (XT == MTC_F16 ? 127u - 24u : 127u - 69u) << 23;
+                if (MODE == S4) sum += __shfl_xor_sync(0xffffffffu, sum, 1);             // chunks 0 and 1, 2 and 3
+                // as the products leave the MMA: chunk t (S4: pair t >> 1) and token at the columns they meet
+                const uint32_t at = MODE == S1 ? et * 4 : (em / CAP) * 32 + (MODE == S2 ? et * 8 : (et >> 1) * 16) + (em % CAP) * 4;
+                if (e < n && (MODE != S4 || !(et & 1))) *reinterpret_cast<float *>(sums + es * SUM + at) = sum * __uint_as_float(unit);
+            }
         }
         __syncwarp();
-        for (int s = 0; s < (to - from) * RUN; ++s) {
+        // G8 adds over the quad and keeps its halves apart: the same MMAs against codes that are all one
+#pragma unroll 2
+        for (int s = 0; s < (MODE == G8 ? (to - from) * RUN : 0); ++s) {
             const uint32_t none[BITS] = {};
             float d[NT][H][4];
             step_mma<BITS, XT, MODE, NT, true>(none, none, frag0 + s * STEP, on, br, d);
@@ -537,9 +568,8 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1) qmv_frag_kernel(const __gri
                 for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
                     for (int h = 0; h < H; ++h) {
-                        char *q = sums + s * SUM + (nt * H + h) * (MODE == S1 ? 16 : 32);
-                        if (MODE == S1) reinterpret_cast<float *>(q)[t] = d[nt][h][0];
-                        else reinterpret_cast<float2 *>(q)[t] = make_float2(d[nt][h][0], d[nt][h][1]);
+                        char *q = sums + s * SUM + (nt * H + h) * 32;
+                        reinterpret_cast<float2 *>(q)[t] = make_float2(d[nt][h][0], d[nt][h][1]);
                     }
             }
         }

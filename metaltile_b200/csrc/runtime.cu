@@ -194,12 +194,14 @@ inline bool stream_takes_single(const Ctx *ctx, int M, int N, int K) {
 //     as one launch instead of three a projection, fused ones whose activations fit an SM (8-bit, 6 layers 823 -> 690).
 //   f32 activations: three pieces per value, so the FFMA kernel wins below M = 5 (M = 4: 14.0 against 16.8), not above (M = 16
 //     39.3 -> 25).
-//   4-bit, 2 <= M: where the ring kernel of qmv_mma.cu does not go (K % 512 != 0 or group 32; 2880 x 2880 M = 4 7.7 -> 5.0).
+//   4-bit, 2 <= M: up to M = 4 (4096 x 4096 / 28672 x 4096 / 4096 x 14336, ring kernel of qmv_mma.cu -> here, M = 2 5.0 / 20.0 /
+//     12.2 -> 4.0 / 14.5 / 10.2, M = 4 5.4 / 20.4 / 14.2 -> 5.0 / 16.2 / 12.3, M = 5 5.9 / 21.3 / 16.6 -> 6.0 / 27.9 / 20.4), and where the ring
+//     kernel does not go (K % 512 != 0 or group 32; 2880 x 2880 M = 4 7.7 -> 5.0).
 inline bool frag_rule(int M, long long N, int K, int bits, int group_size, int dt, bool fused) {
     const long long codes = N * K;
     if (dt == MTC_F32) return M >= 5;
     if (M == 1) return bits == 4 || bits == 8 || (bits != 5 && (fused || codes <= (64ll << 20)));
-    if (bits == 4 && K % 512 == 0 && group_size >= 64 && group_size <= 256) return false;
+    if (bits == 4 && K % 512 == 0 && group_size >= 64 && group_size <= 256) return M <= 4 && group_size <= 128;
     if (M <= 4) return true;
     if (M <= 8) return K <= 8192 || codes < (32ll << 20);
     return group_size % 64 == 0 && K <= 5120 && codes <= (fused ? 128ll << 20 : 20ll << 20);
