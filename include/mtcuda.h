@@ -247,22 +247,23 @@ int mtc_peer_barrier(mtc_ctx *ctx, void *stream, void *const *peer_flags, int n_
  *   "qmm_wide"         a dense work item of the tensor-core kernel covers two 256-row token chunks (one dequantised
  *                      weight stage meets two activation chunks; same results): 0 never, 1 (default) when that saves
  *                      rounds of the grid (M > 256), 2 whenever M > 256
- *   "qmm_ksplit"       0: a dense launch of the tensor-core kernel never cuts K into slices (default 1: with one token
- *                      chunk (M <= 256) and weight-row tiles for less than half of the SMs, K is cut into up to 16
- *                      slices that run as work items of their own; f32 partial sums in a context scratch block are
+ *   "qmm_ksplit"       0: a dense launch of the tensor-core kernel never cuts K into slices (default 1: where whole tiles
+ *                      would leave SMs idle in the last round, K is cut into up to 16 slices that run as work items of
+ *                      their own, as the plan with the shortest estimated time says; f32 partial sums in a context scratch block are
  *                      added in slice order by a second kernel - deterministic, same products)
  *   "qmv_small_m_tc"   2 <= M <= 16 on shapes the warp-level kernels do not take (other widths than 4-bit, group 32):
  *                      1 (default) 9 <= M <= 16, and 5 <= M <= 8 on matrices of 32 Mi codes or more, run on the
  *                      tensor-core kernel (f16 / bf16, K % 64 == 0, power-of-two group >= 32) instead of one FFMA per
  *                      (code, token) on CUDA cores; 0 never; 2 whenever that kernel takes the shape
  *   "qmv_stream"       the streaming decode kernel (4-bit, f16 / bf16, K % 512 == 0, group 64 or 128, 16-byte aligned
- *                      pointers): 1 (default) takes M = 1 - a single projection from 8 Mi codes on (below that the
- *                      CUDA-core kernel is faster), fused projections at any size; 2 takes every M <= 8 at any size
- *                      (slower than the register-ring kernel at M >= 2); 0 never.  mtc_qmv_batched fuses its projections into one launch where this kernel
- *                      takes them and launches them one by one otherwise
+ *                      pointers): 1 (default) takes M = 1 where "qmv_frag" leaves it (0 there) - a single projection
+ *                      from 8 Mi codes on, fused projections at any size; 2 takes every M <= 8 at any size
+ *                      (slower than the register-ring kernel at M >= 2); 0 never.  mtc_qmv_batched fuses its projections into one launch where this kernel,
+ *                      the fragment kernel or the ring kernel takes them and launches them one by one otherwise
  *   "qmv_frag"         the fragment kernel (warp-level tensor cores, every width, weights straight from global memory): 1
  *                      (default) where it is faster than the other small-M kernels (widths other than 4-bit from M = 2 on, f32
- *                      activations from M = 5 on, 4-bit shapes the ring kernel does not take, M = 1 up to 24 Mi codes) unless
+ *                      activations from M = 5 on, 4-bit up to M = 4 and where the ring kernel does not go, M = 1 except
+ *                      5-bit codes and large single 2 / 3 / 6-bit matrices) unless
  *                      "qmv_stream", "qmv_small_m_mma" or "qmv_small_m_tc" selects another kernel; 2 whenever it supports
  *                      the shape (M <= 16, K % 32 == 0, power-of-two group >= 32, 16-byte aligned w and x); 0 never
  *   "qmv_tc"           1: those shapes run on the tensor-memory decode kernel instead (slower today; default 0)

@@ -15,16 +15,16 @@
 //
 // One persistent CTA per SM, 512 threads, warp-specialised:
 //   warp 0      producer   one lane issues TMA (cp.async.bulk.tensor, 128B swizzle) loads of the X
-//                          chunk [TN x 64] into a 4-stage shared-memory ring
+//                          chunk [TN x 64] into a shared-memory ring (one or two k blocks a stage)
 //   warp 1      MMA        one lane issues tcgen05.mma (M=128, N=TN, K=16, kind::f16), accumulators in
 //                          TMEM, double buffered (2 x 256 columns)
-//   warp 2      TMEM allocation / deallocation
-//   warps 4-7   epilogue   tcgen05.ld of the finished accumulator, f32 -> T, transposed stores to out
-//   warps 8-15  dequant    256 threads = 128 weight rows x 2 halves of a 64-wide k block: packed words
-//                          come straight from global memory into registers one k block ahead, every
-//                          code is extracted with one LOP3 ((win & mask<<p) | 1.0f, minus 1.0f =
-//                          q * 2^(p-23)), w = q*scale + bias in f32, rounded to f16, written as the
-//                          K-major 128B-swizzled A operand tile the MMA reads
+//   warps 2-3   copies     packed words, scales and biases into the raw staging buffers, super-blocks ahead (4 and 8
+//                          bits: one TMA box of words); warp 2 also allocates and frees the TMEM
+//   warps 4-7   epilogue   tcgen05.ld of the finished accumulator, f32 -> T, transposed through shared memory, 256-byte
+//                          rows to out (K slices: f32 partial sums)
+//   warps 8-15  dequant    256 threads = 128 weight rows x 2 halves of a 64-wide k block: codes out of the raw
+//                          buffers (registers, one k block ahead, where a shape has no raw form), w = q*scale + bias
+//                          rounded to the operand type, written as the K-major 128B-swizzled A tile the MMA reads
 // Stage hand-off uses mbarriers; tcgen05.commit releases a stage when its MMAs have read it.  Every
 // wait is bounded: on expiry the kernel records a code in the context's status word, all roles leave
 // their loops, TMEM is released and the kernel returns.

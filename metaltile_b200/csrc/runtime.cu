@@ -171,8 +171,8 @@ constexpr size_t kTcCounterBytes = 1u << 20;       // (tile, quarter) counters o
 
 // Partial-sum planes of the tcgen05 decode kernel.  Grow-only; an outgrown block is kept until mtc_destroy, so a CUDA
 // graph captured earlier never reads freed memory.  Growing allocates: not during stream capture.
-// Option "qmv_stream": 1 (default) = the streaming decode kernel takes M = 1, where it is the fastest kernel of the
-// library; 2 = every M <= 8 it supports (at 2 <= M <= 8 the register-ring kernel of qmv_mma.cu is faster: measured
+// Option "qmv_stream": 1 (default) = the streaming decode kernel takes M = 1 where the fragment kernel (frag_rule below) does
+// not; 2 = every M <= 8 it supports (at 2 <= M <= 8 the register-ring kernel of qmv_mma.cu is faster: measured
 // 13.3 against 21.7 us on 14336 x 4096 at M = 8); 0 = never.
 inline bool stream_takes(const Ctx *ctx, int M) { return ctx->qmv_stream == 2 ? M <= 8 : (ctx->qmv_stream == 1 && M == 1); }
 // A single projection on its own launch: below 8 Mi codes the CUDA-core kernel is the faster one (measured at M = 1:
