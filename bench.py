@@ -200,8 +200,8 @@ def p2p_trial(ctx, dev, rank, world, stream_opt=1):
 
 
 # dram__bytes_read.sum + dram__bytes_write.sum over algorithmic bytes for one launch of the step's kernel
-# (qmv_stream_kernel on the 14336 x 4096 projection, ncu --set full, cold L2: 33.69 MB read, 0.8 KB written, 33.07 MB algorithmic)
-NCU_TRAFFIC_RATIO = 1.019
+# (qmv_frag_kernel on the fused 28672 x 4096 projections, ncu, cold L2: 66.09 MB read, 0.59 MB written, 66.13 MB algorithmic)
+NCU_TRAFFIC_RATIO = 1.008
 
 
 def main():
@@ -563,8 +563,8 @@ def main():
     us_per_launch = ms * 1e3 / launches_per_step
     roofline = {"bound": "hbm", "achieved": value / world, "peak": hbm_peak, "unit": "GB/s",
                 "frac": value / world / hbm_peak, "traffic": per_launch_bytes * NCU_TRAFFIC_RATIO, "peak_kind": peak_kind,
-                "traffic_source": f"ncu dram bytes / algorithmic bytes = {NCU_TRAFFIC_RATIO} on the 14336x4096 launch of the streaming kernel, scaled to the average launch",
-                "kernel": "qmv_stream_kernel<bf16, g64, M1>", "alg_bytes_per_launch": per_launch_bytes,
+                "traffic_source": f"ncu dram bytes / algorithmic bytes = {NCU_TRAFFIC_RATIO} on the 28672x4096 launch of the fragment kernel, scaled to the average launch",
+                "kernel": "qmv_frag_kernel<4-bit, bf16, M1>", "alg_bytes_per_launch": per_launch_bytes,
                 "avg_us_per_launch": us_per_launch,
                 "note": "per-GPU; launch-averaged over the 4 matrix shapes of the step (graph replay, events)"}
     line = {"metric": METRIC, "value": value, "unit": "GB/s", "n_gpus": world, "steps": args.steps,

@@ -61,12 +61,10 @@ __global__ void __launch_bounds__(128) router_topk_kernel(const void *logits, ui
                 }
             }
         }
-        float gbest = best;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) gbest = fmaxf(gbest, __shfl_xor_sync(0xffffffffu, gbest, o));
-        uint32_t cand_idx = (best == gbest) ? best_idx : 0xFFFFFFFFu;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) cand_idx = min(cand_idx, __shfl_xor_sync(0xffffffffu, cand_idx, o));
+        // one warp reduction each (ten dependent shuffles before: the k passes are the whole chain of this kernel)
+        float gbest;
+        asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(gbest) : "f"(best));
+        const uint32_t cand_idx = __reduce_min_sync(0xffffffffu, (best == gbest) ? best_idx : 0xFFFFFFFFu);
         if ((cand_idx & 31u) == static_cast<uint32_t>(lane) && cand_idx != 0xFFFFFFFFu) taken |= 1u << (cand_idx >> 5);
         if (lane == it) { my_val = gbest; my_idx = cand_idx; }
     }
@@ -106,7 +104,8 @@ __global__ void __launch_bounds__(kSortThreads) moe_sort_kernel(const uint32_t *
     uint32_t held[kSortHeld];
 #pragma unroll
     for (int q = 0; q < kSortHeld; ++q) held[q] = f0 + 32 * q + lane < f1 ? topk_idx[f0 + 32 * q + lane] : 0xFFFFFFFFu;
-    for (int i = tid; i < 32 * n_experts; i += kSortThreads) wcnt[i] = 0;
+    const int used = min(32, (total + per - 1) / max(per, 1));          // warps that have slots
+    for (int i = tid; i < used * n_experts; i += kSortThreads) wcnt[i] = 0;
     __syncthreads();
     uint32_t *mine = wcnt + warp * n_experts;
     auto count = [&](int c, uint32_t id) {
@@ -127,7 +126,7 @@ __global__ void __launch_bounds__(kSortThreads) moe_sort_kernel(const uint32_t *
     for (int ee = tid; ee < n_experts; ee += kSortThreads) {   // per expert: exclusive prefix over the warps, total
         uint32_t run = 0;
 #pragma unroll 8
-        for (int w = 0; w < 32; ++w) {
+        for (int w = 0; w < used; ++w) {
             const uint32_t c = wcnt[w * n_experts + ee];
             wcnt[w * n_experts + ee] = run;
             run += c;
