@@ -61,10 +61,12 @@ enum { S1 = 0, S2 = 1, S4 = 2, G8 = 3 };
 template <int BITS>
 constexpr int kRun = BITS <= 4 ? 4 : 2;       // steps requested at once (registers: 2 * BITS words a step)
 
-// Planar widths in S1 and S2, where every chunk has its own columns: lane t takes RUN consecutive chunks of a run, one a step
-// (else chunk t of every step), so that its words of the run are whole 16-byte loads: 3-bit, 6 loads a run and two rows instead of 24.
+// 3-bit codes in S1 and S2, where every chunk has its own columns: where rows start on 16 bytes, lane t takes RUN consecutive chunks
+// of a run, one a step (else chunk t of every step), so that its words of the run are whole 16-byte loads, 6 a run and two
+// rows instead of 24 (8192 x 8192, groups of 32, 4 tokens 18.3 -> 16.9 us, groups of 64, one token 14.7 -> 12.5).  Not for 6 bits,
+// whose 8-byte loads are enough (18.7 -> 19.4), nor 5, whose runs of two are 40 bytes a lane.
 template <int BITS, int MODE>
-constexpr bool kLong = (BITS == 3 || BITS == 6) && (MODE == S1 || MODE == S2);           // 5-bit runs of two are 40 bytes a lane
+constexpr bool kLong = BITS == 3 && (MODE == S1 || MODE == S2);
 
 template <int MODE>
 constexpr int kCap = MODE == S1 ? 1 : MODE == S2 ? 2 : MODE == S4 ? 4 : 8;      // tokens of one tile of columns
@@ -421,7 +423,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1) qmv_frag_kernel(const __gri
     constexpr int RUN = (MODE == G8 && !VEC) ? 2 : kRun<BITS>;
     constexpr int H = MODE == G8 ? 2 : 1;
     constexpr int CAP = kCap<MODE>, MP = CAP * NT;
-    constexpr bool LONG = kLong<BITS, MODE>;
+    const bool lng = kLong<BITS, MODE> && a.wpr % 4 == 0;
     constexpr uint32_t STEP = MP * 4 * kPitch<XT>;                                 // fragments of one step
     constexpr uint32_t SUM = NT * H * 4 * (MODE == S1 ? 4 : 8);                    // activation sums of one step
     constexpr int ESZ = XT == MTC_F32 ? 4 : 2;
@@ -460,7 +462,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1) qmv_frag_kernel(const __gri
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
             const uint32_t row = min(n + 8 * j, pr.N - 1);
-            wo[j] = row * static_cast<uint32_t>(a.wpr * 4) + (MODE == G8 ? t * (BITS * 2) : t * (BITS * 4) * (LONG ? RUN : 1));
+            wo[j] = row * static_cast<uint32_t>(a.wpr * 4) + (MODE == G8 ? t * (BITS * 2) : t * (BITS * 4) * (lng ? RUN : 1));
             ao[j] = row * static_cast<uint32_t>(a.gpr * ESZ);
         }
     };
@@ -469,24 +471,26 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1) qmv_frag_kernel(const __gri
     bool whole = true;                        // the run being requested lies inside the row (VEC: all do)
     auto request_words = [&](int i, int limit) {
         if (limit == 0) return;               // nothing left for this warp (uniform)
-        constexpr int STEP_W = LONG ? 4 * BITS : 16 * BITS;                        // bytes from a lane's words of a step to those of the next
-        if (LONG && whole && a.wpr % 4 == 0) {                                     // rows, runs and lanes start on 16 bytes
-            static_assert(!LONG || (RUN * BITS) % 4 == 0, "whole 16-byte loads");
-            // a load goes out with the last step whose words it replaces
+        if (lng && whole) {
+            if constexpr (kLong<BITS, MODE>) {
+                static_assert((RUN * BITS) % 4 == 0, "whole 16-byte loads");
+                // a load goes out with the last step whose words it replaces
 #pragma unroll
-            for (int v = 0; v < RUN * BITS / 4; ++v)
-                if ((4 * v + 3) / BITS == i) {
-                    ldg16_l1(pl + 16 * v, &wl[0][0] + 4 * v);
-                    ldg16_l1(ph + 16 * v, &wh[0][0] + 4 * v);
-                }
+                for (int v = 0; v < RUN * BITS / 4; ++v)
+                    if ((4 * v + 3) / BITS == i) {
+                        ldg16_l1(pl + 16 * v, &wl[0][0] + 4 * v);
+                        ldg16_l1(ph + 16 * v, &wh[0][0] + 4 * v);
+                    }
+            }
         } else if (VEC != 0 || whole) {
-            load_words<BITS, MODE>(pl + i * STEP_W, wl[i]);
-            load_words<BITS, MODE>(ph + i * STEP_W, wh[i]);
+            load_words<BITS, MODE>(pl + i * (16 * BITS), wl[i]);
+            load_words<BITS, MODE>(ph + i * (16 * BITS), wh[i]);
         } else {
             const int s = l_run * RUN + i;
-            const bool on0 = (MODE == G8 ? 2 * s : LONG ? (4 * l_run + t) * RUN + i : 4 * s + t) < limit, on1 = 2 * s + 1 < limit;
-            load_words<BITS, MODE>(pl + i * STEP_W, wl[i], on0, on1);
-            load_words<BITS, MODE>(ph + i * STEP_W, wh[i], on0, on1);
+            const bool on0 = (MODE == G8 ? 2 * s : lng ? (4 * l_run + t) * RUN + i : 4 * s + t) < limit, on1 = 2 * s + 1 < limit;
+            const int step_w = lng ? 4 * BITS : 16 * BITS;                         // bytes from a lane's words of a step to those of the next
+            load_words<BITS, MODE>(pl + i * step_w, wl[i], on0, on1);
+            load_words<BITS, MODE>(ph + i * step_w, wh[i], on0, on1);
         }
     };
     auto request_affine = [&](const char *const (&p)[2], Affine<XT, MODE, RUN, VEC> &f, int i, int limit) {   // VEC: the whole run, i unused
@@ -501,13 +505,13 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1) qmv_frag_kernel(const __gri
 #pragma unroll
             for (int h = 0; h < H; ++h) {
                 const int s = l_run * RUN + i;
-                const int k = MODE == G8 ? 128 * s + 64 * h : MODE == S4 ? 128 * s + 64 * (t >> 1) : LONG ? ((4 * l_run + t) * RUN + i) * 32 : 128 * s + 32 * t;
+                const int k = MODE == G8 ? 128 * s + 64 * h : MODE == S4 ? 128 * s + 64 * (t >> 1) : lng ? ((4 * l_run + t) * RUN + i) * 32 : 128 * s + 32 * t;
                 const uint32_t off = static_cast<uint32_t>(k >> a.gs_shift) * ESZ;
                 if (whole) {
 #pragma unroll
                     for (int j = 0; j < 2; ++j) ld_scale<XT>(p[j] + off, &f.r[j][i * H + h]);
                 } else {
-                    const bool in = (MODE == G8 ? 2 * s + h : MODE == S4 ? 4 * s + 2 * (t >> 1) : LONG ? (4 * l_run + t) * RUN + i : 4 * s + t) < limit;
+                    const bool in = (MODE == G8 ? 2 * s + h : MODE == S4 ? 4 * s + 2 * (t >> 1) : lng ? (4 * l_run + t) * RUN + i : 4 * s + t) < limit;
 #pragma unroll
                     for (int j = 0; j < 2; ++j) ld_scale<XT>(p[j] + off, &f.r[j][i * H + h], in);
                 }
@@ -562,7 +566,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1) qmv_frag_kernel(const __gri
         const int n = (to - from) * RUN * 4 * MP;
         for (int e0 = 0; e0 < n; e0 += 32) {
             const int e = e0 + lane, et = e & 3, em = (e >> 2) % MP, es = (e >> 2) / MP;
-            const int k = LONG ? ((from + es / RUN) * 4 * RUN + es % RUN) * 32 + et * (32 * RUN - 32) : (from * RUN + es) * 128;
+            const int k = lng ? ((from + es / RUN) * 4 * RUN + es % RUN) * 32 + et * (32 * RUN - 32) : (from * RUN + es) * 128;
             float sum = 0.0f;
             if (e < n)
                 sum = stage_chunk<BITS, XT, MODE>(a, em, MODE == G8 ? k + 16 * et : k + 32 * et, MODE == G8 ? k + 64 + 16 * et : k + 32 * et + 16,
