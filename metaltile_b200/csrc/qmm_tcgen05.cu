@@ -459,7 +459,7 @@ __device__ __forceinline__ Item get_item(const QmmParams &p, int i) {
         return it;
     }
     if (p.items) {
-        const int4 v = __ldg(p.items + i);
+        const int4 v = p.items[i];               // written by the kernel before this one: no read-only load
         it.n_tile = v.x; it.expert = v.y & 0xFFFFFF; it.row0 = v.z; it.rows = v.w;
         it.nc = 1;
     } else if (p.wide) {
@@ -504,7 +504,6 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
     SmemCtrl *ctl = reinterpret_cast<SmemCtrl *>(smem + RING_BYTES + EPI_BYTES);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int num_items = p.items ? __ldg(p.item_count) : p.dense_items;
     const uint32_t x_bytes = static_cast<uint32_t>(p.TN) * BK * 2;
 
     if (threadIdx.x == 0) {
@@ -533,6 +532,8 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
     const uint32_t tmem_base = ctl->tmem_base;
     asm volatile("griddepcontrol.launch_dependents;");
     if (!p.pdl_roles) asm volatile("griddepcontrol.wait;" ::: "memory");
+    // a list of work items comes from an earlier kernel of the stream (pdl_roles is 0 then): its length after the wait
+    const int num_items = p.items ? *p.item_count : p.dense_items;
 
     if (warp == 0) {
         // ---------------- producer: TMA loads of the X chunk ----------------
