@@ -39,12 +39,12 @@ constexpr uint32_t kTwo23 = 0x4B000000u;               // 2^23 as f32
 // (the second word only where the unit reaches it, so nothing past the last unit is read).
 template <int BITS>
 __device__ __forceinline__ uint64_t ld_codes(const uint32_t *w, uint32_t i) {
-    if (BITS == 8) return __ldg(w + 2 * i) | static_cast<uint64_t>(__ldg(w + 2 * i + 1)) << 32;
-    if (BITS == 4) return __ldg(w + i);
-    if (BITS == 2) return __ldg(reinterpret_cast<const uint16_t *>(w) + i);
+    if (BITS == 8) return w[2 * i] | static_cast<uint64_t>(w[2 * i + 1]) << 32;
+    if (BITS == 4) return w[i];
+    if (BITS == 2) return reinterpret_cast<const uint16_t *>(w)[i];
     const uint32_t at = i * BITS, sh = (at & 3) * 8;       // byte, bit of its word
     const uint32_t *p = w + (at >> 2);
-    return (__ldg(p) | static_cast<uint64_t>(__ldg(p + (sh + 8 * BITS > 32 ? 1 : 0))) << 32) >> sh;
+    return (p[0] | static_cast<uint64_t>(p[sh + 8 * BITS > 32 ? 1 : 0]) << 32) >> sh;
 }
 // Eight codes of a unit in two words of four (lo, hi: code k at bit (k & 3) * BITS) to the b bytes of unit i.  Every lane of a
 // warp calls it (3 / 5 / 6-bit: the four lanes of a quad hold b whole words, and a lane that stores one gets the other half of it from a neighbour);
@@ -123,8 +123,8 @@ __global__ void __launch_bounds__(256) affine_dequantize_kernel(const uint32_t *
             // power of two: the tile starts on a group, or lies inside one
             const size_t g = upg_log2 >= 0 ? g0 + (at >> upg_log2) : (base + at) / units_per_group;
             codes[u] = ld_codes<BITS>(wt, at);
-            s[u] = ld_as_f32(scales, g, DT);
-            b[u] = ld_as_f32(biases, g, DT);
+            s[u] = ld_written_as_f32(scales, g, DT);
+            b[u] = ld_written_as_f32(biases, g, DT);
         }
 #pragma unroll
         for (int u = 0; u < kUnits; ++u) {
@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(256) affine_quantize8_kernel(const void *w, ui
             const uint32_t off = u * 32 + lane, at = off < rem ? off : 0;
 #pragma unroll
             for (int q = 0; q < RW / 4; ++q) {
-                const uint4 t = __ldg(wt + at * (RW / 4) + q);
+                const uint4 t = wt[at * (RW / 4) + q];
                 raw[u][4 * q] = t.x; raw[u][4 * q + 1] = t.y; raw[u][4 * q + 2] = t.z; raw[u][4 * q + 3] = t.w;
             }
         }

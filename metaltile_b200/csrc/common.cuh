@@ -110,7 +110,10 @@ struct PerDeviceAttr {
 };
 
 // Programmatic dependent launch for a kernel that reads what the previous kernel of its stream wrote: it is scheduled while that
-// kernel drains (the launch latency overlaps) and waits on the device before it touches anything.
+// kernel drains (the launch latency overlaps) and waits on the device before it touches anything.  Such a kernel is alive
+// while that data is being written, so it must not read it through the read-only path (__ldg, ld.global.nc, ld_as_f32): that path
+// is for data that nothing writes during the kernel's life, and the compiler may move such a load above the wait.
+// Weights, scales and biases of a product are constants by contract and stay on it; everything else takes plain loads.
 __device__ __forceinline__ void pdl_enter() {
     asm volatile("griddepcontrol.launch_dependents;");
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -131,6 +134,13 @@ cudaError_t launch_pdl(void (*kern)(P...), dim3 grid, int block, size_t smem, cu
 }
 
 // ---- dtype-generic element access (dtype is a launch-time constant) ----------
+// plain load: for what an earlier kernel of the stream may have written (see pdl_enter); ld_as_f32: read-only path
+__device__ __forceinline__ float ld_written_as_f32(const void *p, size_t i, int dt) {
+    if (dt == MTC_F32) return reinterpret_cast<const float *>(p)[i];
+    const unsigned short h = reinterpret_cast<const unsigned short *>(p)[i];
+    if (dt == MTC_BF16) return __uint_as_float(static_cast<uint32_t>(h) << 16);
+    return __half2float(__ushort_as_half(h));
+}
 __device__ __forceinline__ float ld_as_f32(const void *p, size_t i, int dt) {
     if (dt == MTC_F32) return __ldg(reinterpret_cast<const float *>(p) + i);
     unsigned short h = __ldg(reinterpret_cast<const unsigned short *>(p) + i);

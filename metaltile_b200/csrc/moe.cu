@@ -31,7 +31,7 @@ __global__ void __launch_bounds__(128) router_topk_kernel(const void *logits, ui
         if (r < per_lane) {
             const int j = r * 32 + lane;
             if (j < n_experts) {
-                z[r] = ld_as_f32(logits, base + j, dt);
+                z[r] = ld_written_as_f32(logits, base + j, dt);
                 if (z[r] > row_max) row_max = z[r];
             }
         }
@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(256) unpermute16_kernel(const uint4 *expert_ou
           for (int i = 0; i < 8; ++i) {
             if (j0 + i < k) {
                 const uint32_t pos = inv_perm[static_cast<size_t>(t) * k + j0 + i];
-                wts[i] = ld_as_f32(weights, static_cast<size_t>(t) * k + j0 + i, dt);
+                wts[i] = ld_written_as_f32(weights, static_cast<size_t>(t) * k + j0 + i, dt);
                 rows[i] = expert_out[static_cast<size_t>(pos) * hidden8 + h8];
             }
           }

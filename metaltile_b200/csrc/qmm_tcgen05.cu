@@ -775,8 +775,8 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
 #pragma unroll
                         for (int g = 0; g < 2; ++g) {
                             const int j = row_base + c0 + 8 * g + 2 * (lane & 3);
-                            ts[g].x = __ldg(tok_scale + min(j, tok_last));
-                            ts[g].y = __ldg(tok_scale + min(j + 1, tok_last));
+                            ts[g].x = tok_scale[min(j, tok_last)];
+                            ts[g].y = tok_scale[min(j + 1, tok_last)];
                         }
                     }
                     uint32_t v[2][8];
@@ -979,7 +979,7 @@ __global__ void __launch_bounds__(256) rows_to_f16_kernel(const __nv_bfloat16 *x
     uint4 *dst = reinterpret_cast<uint4 *>(y + static_cast<size_t>(on ? row : 0) * K);
     uint4 held[HELD];
 #pragma unroll
-    for (int q = 0; q < HELD; ++q) held[q] = i0 + q * STEP < nvec ? __ldg(src + i0 + q * STEP) : make_uint4(0u, 0u, 0u, 0u);
+    for (int q = 0; q < HELD; ++q) held[q] = i0 + q * STEP < nvec ? src[i0 + q * STEP] : make_uint4(0u, 0u, 0u, 0u);
     uint32_t amax = 0;                       // max of |x| as bf16 bit patterns (monotone for finite values)
     auto fold = [&](const uint4 &v) {
         const uint32_t u[4] = {v.x, v.y, v.z, v.w};
@@ -991,7 +991,7 @@ __global__ void __launch_bounds__(256) rows_to_f16_kernel(const __nv_bfloat16 *x
     };
 #pragma unroll
     for (int q = 0; q < HELD; ++q) fold(held[q]);
-    for (int i = i0 + HELD * STEP; i < nvec; i += STEP) fold(__ldg(src + i));
+    for (int i = i0 + HELD * STEP; i < nvec; i += STEP) fold(src[i]);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) amax = max(amax, __shfl_xor_sync(0xffffffffu, amax, o));
     if constexpr (W > 1) {
@@ -1018,7 +1018,7 @@ __global__ void __launch_bounds__(256) rows_to_f16_kernel(const __nv_bfloat16 *x
 #pragma unroll
     for (int q = 0; q < HELD; ++q)
         if (i0 + q * STEP < nvec) dst[i0 + q * STEP] = convert(held[q]);
-    for (int i = i0 + HELD * STEP; i < nvec; i += STEP) dst[i] = convert(__ldg(src + i));
+    for (int i = i0 + HELD * STEP; i < nvec; i += STEP) dst[i] = convert(src[i]);
 }
 cudaError_t launch_rows_to_f16(cudaStream_t st, const void *x, __half *y, float *row_scale, int rows, int K) {
     const __nv_bfloat16 *xb = static_cast<const __nv_bfloat16 *>(x);

@@ -97,21 +97,21 @@ __device__ __forceinline__ float comp(const float4 &v, int i) {
 //          ((jb * V + vv) * (CODES*MT/4) + (i*MT+m)/4) * 32 + ln, component (i*MT+m)%4,
 //          value x[m, k] * 2^(kPreExp - (i % CPW) * BITS);
 //   xsum : plain sum of the base chunk's x values, at ((jb*32 + ln) * V + vv) * MT + m.
-// CODES consecutive elements of a T array (f32, f16 or bf16; 16-byte aligned position) as f32.
+// CODES consecutive elements of a T array (f32, f16 or bf16; 16-byte aligned position) as f32.  Activations: plain loads (pdl_enter, common.cuh).
 template <int CODES>
 __device__ __forceinline__ void load_vals(const void *src, size_t base, int dt, float (&v)[CODES]) {
     if (dt == MTC_F32) {
         const float4 *p = reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(src) + base);
 #pragma unroll
         for (int q = 0; q < CODES / 4; ++q) {
-            float4 t = __ldg(p + q);
+            float4 t = p[q];
             v[4 * q] = t.x; v[4 * q + 1] = t.y; v[4 * q + 2] = t.z; v[4 * q + 3] = t.w;
         }
     } else {
         const uint4 *p = reinterpret_cast<const uint4 *>(reinterpret_cast<const uint16_t *>(src) + base);
 #pragma unroll
         for (int q = 0; q < CODES / 8; ++q) {
-            uint4 t = __ldg(p + q);
+            uint4 t = p[q];
             uint32_t u[4] = {t.x, t.y, t.z, t.w};
 #pragma unroll
             for (int h = 0; h < 4; ++h) {
@@ -367,7 +367,7 @@ __global__ void __launch_bounds__(256, (MT <= 2 ? 2 : 1)) qmv_pipe_kernel(const 
         // sum of squares of the (single) activation row over the CTA, then every thread holds inv_rms
         float ssq = 0.0f;
         for (int k = threadIdx.x; k < a.K; k += blockDim.x) {
-            const float v = ld_as_f32(a.x, static_cast<size_t>(k), a.dt);
+            const float v = ld_written_as_f32(a.x, static_cast<size_t>(k), a.dt);
             ssq = fmaf(v, v, ssq);
         }
 #pragma unroll

@@ -145,8 +145,8 @@ __device__ __forceinline__ void stage_x_mma(const MmaArgs &a, uint4 *xb, int seg
             if (i < total && m < a.M) {
                 const uint4 *p = reinterpret_cast<const uint4 *>(static_cast<const uint16_t *>(a.x) + static_cast<size_t>(m) * a.K +
                                                                  static_cast<size_t>(seg0 + s) * 64 + 16 * t);
-                v0[u] = __ldg(p);       // x[16t + 0..7]  as halves h0..h7:  word q holds (h[2q], h[2q+1])
-                v1[u] = __ldg(p + 1);   // x[16t + 8..15]
+                v0[u] = p[0];       // x[16t + 0..7]  as halves h0..h7:  word q holds (h[2q], h[2q+1])
+                v1[u] = p[1];   // x[16t + 8..15]
             }
         }
 #pragma unroll
@@ -347,8 +347,8 @@ __device__ __forceinline__ void stage_x_ring(const MmaArgs &a, uint4 *xb, float 
             v0[u] = v1[u] = make_uint4(0u, 0u, 0u, 0u);
             if (s < nseg && real) {
                 const uint4 *p = reinterpret_cast<const uint4 *>(xrow + static_cast<size_t>(s) * 64);
-                v0[u] = __ldg(p);
-                v1[u] = __ldg(p + 1);
+                v0[u] = p[0];
+                v1[u] = p[1];
             }
         }
 #pragma unroll

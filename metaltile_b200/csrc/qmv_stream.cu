@@ -197,8 +197,8 @@ __device__ __forceinline__ void stage_x(const void *x, int K, int M, unsigned ch
             if (on) {
                 const uint4 *p = reinterpret_cast<const uint4 *>(static_cast<const uint16_t *>(x) + static_cast<size_t>(m) * K +
                                                                  static_cast<size_t>(s) * 64 + 16 * t);
-                v0 = __ldg(p);        // x[16t + 0..7]
-                v1 = __ldg(p + 1);    // x[16t + 8..15]
+                v0 = p[0];            // x[16t + 0..7]
+                v1 = p[1];            // x[16t + 8..15]
             }
             uint4 f01, f23;
             float sum;
@@ -231,8 +231,8 @@ __device__ __forceinline__ void stage_x_warp(const void *x, int seg0, int seg1, 
             v0[i] = v1[i] = make_uint4(0u, 0u, 0u, 0u);
             if (it < nitems) {
                 const uint4 *p = reinterpret_cast<const uint4 *>(static_cast<const uint16_t *>(x) + static_cast<size_t>(seg0 + (it >> 2)) * 64 + 16 * t);
-                v0[i] = __ldg(p);
-                v1[i] = __ldg(p + 1);
+                v0[i] = p[0];
+                v1[i] = p[1];
             }
         }
 #pragma unroll

@@ -249,8 +249,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) qmv_tc_kernel(const __grid_cons
             uint4 v0 = make_uint4(0u, 0u, 0u, 0u), v1 = v0;
             if (on) {
                 const uint4 *src = reinterpret_cast<const uint4 *>(static_cast<const uint16_t *>(a.x) + static_cast<size_t>(m) * a.K + ur * 16);
-                v0 = __ldg(src);
-                v1 = __ldg(src + 1);
+                v0 = src[0];
+                v1 = src[1];
             }
             const uint32_t uw[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};   // word i: codes 2i, 2i+1
             uint32_t e[8], o[8];

@@ -49,18 +49,21 @@ struct QvCode {
 
 constexpr int kQvTickets = 4096;               // arrival counters at the head of the partial-sum block (one per column tile and x row)
 
-// NW consecutive 32-bit words from a 16-byte (NW % 4 == 0) or 8-byte (NW == 2) aligned address, read-only path
-template <int NW>
+// NW consecutive 32-bit words from a 16-byte (NW % 4 == 0) or 8-byte (NW == 2) aligned address: RO = the read-only path (scales and
+// biases), else plain loads (activations, which the previous kernel may be writing: pdl_enter)
+template <bool RO, int NW>
 __device__ __forceinline__ void qv_ld(const void *p, uint32_t (&o)[NW]) {
     static_assert(NW == 2 || NW % 4 == 0, "vector loads of 8 or 16 bytes");
     if (NW == 2) {
-        const uint2 v = __ldg(static_cast<const uint2 *>(p));
+        const uint2 *src = static_cast<const uint2 *>(p);
+        const uint2 v = RO ? __ldg(src) : *src;
         o[0] = v.x;
         o[1] = v.y;
     } else {
 #pragma unroll
         for (int i = 0; i < NW / 4; ++i) {
-            const uint4 v = __ldg(static_cast<const uint4 *>(p) + i);
+            const uint4 *src = static_cast<const uint4 *>(p) + i;
+            const uint4 v = RO ? __ldg(src) : *src;
             o[4 * i] = v.x; o[4 * i + 1] = v.y; o[4 * i + 2] = v.z; o[4 * i + 3] = v.w;
         }
     }
@@ -120,12 +123,12 @@ __global__ void __launch_bounds__(kQvWarps * 32, 2) qvm_kernel(const uint32_t *w
             for (int i = 0; i < S::WPT; ++i) sl.w[r][i] = __ldg(wp + i);
             wp += wpr;
         }
-        qv_ld<Slab::SW>(sc0 + static_cast<size_t>(g) * N * ESZ, sl.sc);
-        qv_ld<Slab::SW>(bi0 + static_cast<size_t>(g) * N * ESZ, sl.bi);
+        qv_ld<true, Slab::SW>(sc0 + static_cast<size_t>(g) * N * ESZ, sl.sc);
+        qv_ld<true, Slab::SW>(bi0 + static_cast<size_t>(g) * N * ESZ, sl.bi);
     };
     auto fetch_x = [&](int u, Slab &sl) {
         const int g = u / upg, d0 = g * gs + (u - g * upg) * R;
-        qv_ld<Slab::XW>(xrow + static_cast<size_t>(d0) * ESZ, sl.x);
+        qv_ld<false, Slab::XW>(xrow + static_cast<size_t>(d0) * ESZ, sl.x);
     };
     auto fetch = [&](int u, Slab &sl) {
         fetch_w(u, sl);

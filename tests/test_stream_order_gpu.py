@@ -58,3 +58,109 @@ def test_work_list_of_a_grouped_product(ctx, dt, by_rows):
 
     _same_without_waiting(step)
     assert ctx.status_word() == 0
+
+
+def _dense(n, k, bits, gs, dt, seed):
+    w, s, b, _ = dense_case(1, n, k, bits, gs, dt, seed=seed)
+    return to_dev(w), to_dev(s, dt), to_dev(b, dt)
+
+
+@pytest.mark.parametrize("m,bits,dt", [(1, 4, "bf16"), (1, 5, "f16"), (1, 4, "f32"), (4, 8, "f16"), (8, 4, "bf16"), (8, 8, "f32"), (16, 4, "f16"),
+                                       (64, 4, "bf16"), (300, 8, "bf16"), (300, 4, "f16")])
+def test_products_behind_swiglu_and_each_other(ctx, m, bits, dt):
+    """x of every product is what the launch before it stores: SwiGLU, a product, the row conversion of a prompt in bf16."""
+    import torch
+    from metaltile_b200 import ops
+    n, k = 2048, 1024
+    up, down = _dense(n, k, bits, 64, dt, 1), _dense(k, n, bits, 64, dt, 2)
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    xs = [(torch.randn(m, k, device="cuda", generator=gen) * 0.05).to(up[1].dtype) for _ in range(ROUNDS)]
+    act, mid, out = torch.empty_like(xs[0]), xs[0].new_empty(m, n), torch.empty_like(xs[0])
+
+    def step(i):
+        ops.swiglu(xs[i], xs[i], out=act, ctx=ctx)
+        ops.qmm(*up, act, bits, 64, out=mid, ctx=ctx)
+        ops.qmm(*down, mid, bits, 64, out=out, ctx=ctx)
+        return [mid, out]
+
+    _same_without_waiting(step)
+
+
+@pytest.mark.parametrize("kernel", ["stream", "mma", "tc", "cuda"])
+@pytest.mark.parametrize("m", [1, 4])
+def test_other_small_m_kernels_behind_swiglu(ctx, kernel, m):
+    import torch
+    from metaltile_b200 import ops
+    options = dict(stream=[("qmv_stream", 2)], mma=[("qmv_stream", 0), ("qmv_small_m_mma", 2)], tc=[("qmv_tc", 1)], cuda=[("qmv_stream", 0), ("qmv_small_m_mma", 0)])[kernel]
+    mat = _dense(2048, 1024, 4, 64, "bf16", 3)
+    xs = [torch.randn(m, 1024, device="cuda").to(torch.bfloat16) for _ in range(ROUNDS)]
+    act, out = torch.empty_like(xs[0]), xs[0].new_empty(m, 2048)
+    ctx.set_option("qmv_frag", 0)
+    for name, v in options:
+        ctx.set_option(name, v)
+    try:
+        def step(i):
+            ops.swiglu(xs[i], xs[i], out=act, ctx=ctx)
+            return [ops.qmv(*mat, act, 4, 64, out=out, ctx=ctx)]
+
+        _same_without_waiting(step)
+    finally:
+        for name, v in (("qmv_frag", 1), ("qmv_stream", 1), ("qmv_small_m_mma", 1), ("qmv_tc", 0)):
+            ctx.set_option(name, v)
+
+
+@pytest.mark.parametrize("m,bits,dt", [(1, 4, "bf16"), (1, 3, "f32"), (4, 4, "f16"), (2, 8, "bf16")])
+def test_qvm_behind_swiglu(ctx, m, bits, dt):
+    import torch
+    from metaltile_b200 import ops, synth
+    k, n = 2048, 4096
+    w = to_dev(synth.words(k * n * bits // 32, seed=4).reshape(k, -1))
+    s = (torch.rand(k // 64, n, device="cuda") * 0.01).to(getattr(torch, dict(f32="float32", f16="float16", bf16="bfloat16")[dt]))
+    xs = [torch.randn(m, k, device="cuda").to(s.dtype) for _ in range(ROUNDS)]
+    act, out = torch.empty_like(xs[0]), xs[0].new_empty(m, n)
+
+    def step(i):
+        ops.swiglu(xs[i], xs[i], out=act, ctx=ctx)
+        return [ops.qvm(w, s, s, act, bits, 64, out=out, ctx=ctx)]
+
+    _same_without_waiting(step)
+
+
+@pytest.mark.parametrize("tokens", [4, 200])
+def test_a_layer_of_experts(ctx, tokens):
+    """Router, sort, experts and unpermute over buffers of their own that every round rewrites; the logits are a SwiGLU's result."""
+    import torch
+    from metaltile_b200 import ops
+    e, h, i_dim = 16, 512, 256
+    mats = [tuple(t.view(e, -1, t.shape[-1]) for t in _dense(e * o, k, 4, 64, "bf16", 5 + j)) for j, (o, k) in enumerate(((i_dim, h), (i_dim, h), (h, i_dim)))]
+    xs = [torch.randn(tokens, h, device="cuda").to(torch.bfloat16) for _ in range(ROUNDS)]
+    raw = [torch.randn(tokens, e, device="cuda").to(torch.bfloat16) for _ in range(ROUNDS)]
+    logits, x, y, out = torch.empty_like(raw[0]), torch.empty_like(xs[0]), xs[0].new_empty(tokens * 4, h), torch.empty_like(xs[0])
+
+    def step(i):
+        ops.swiglu(xs[i], xs[i], out=x, ctx=ctx)
+        ops.swiglu(raw[i], raw[i], out=logits, ctx=ctx)
+        idx, wts = ops.moe_router_topk(logits, 4, ctx=ctx)
+        order, inverse, offsets, _ = ops.moe_sort(idx, e, ctx=ctx)
+        ops.moe_experts(x, *mats, 4, 64, offsets, sort_token_idx=order, out=y, ctx=ctx)
+        return [idx, wts, ops.moe_unpermute(y, inverse, wts, out=out, ctx=ctx)]
+
+    _same_without_waiting(step)
+
+
+@pytest.mark.parametrize("bits,dt", [(4, "bf16"), (3, "f16"), (8, "f32")])
+def test_codec_behind_swiglu_and_itself(ctx, bits, dt):
+    """Values just computed are quantized, read back and quantized again."""
+    import torch
+    from metaltile_b200 import ops
+    dtype = dict(f32=torch.float32, f16=torch.float16, bf16=torch.bfloat16)[dt]
+    xs = [torch.randn(512, 1024, device="cuda").to(dtype) for _ in range(ROUNDS)]
+    act = torch.empty_like(xs[0])
+
+    def step(i):
+        ops.swiglu(xs[i], xs[i], out=act, ctx=ctx)
+        q = ops.affine_quantize(act, bits, 64, ctx=ctx)
+        back = ops.affine_dequantize(*q, bits, 64, ctx=ctx)
+        return [*q, back, *ops.affine_quantize(back, bits, 64, ctx=ctx)]
+
+    _same_without_waiting(step)
