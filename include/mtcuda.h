@@ -249,8 +249,9 @@ int mtc_peer_barrier(mtc_ctx *ctx, void *stream, void *const *peer_flags, int n_
  *                      rounds of the grid (M > 256), 2 whenever M > 256
  *   "qmm_ksplit"       0: a dense launch of the tensor-core kernel never cuts K into slices (default 1: where whole tiles
  *                      would leave SMs idle in the last round, K is cut into up to 16 slices that run as work items of
- *                      their own, as the plan with the shortest estimated time says; f32 partial sums in a context scratch block are
- *                      added in slice order by a second kernel - deterministic, same products)
+ *                      their own, as the plan with the shortest estimated time says; f32 partial sums - 512 MiB at most - in a
+ *                      context scratch block are added in slice order by a second kernel - deterministic, same products.
+ *                      Where that block cannot grow, M > 16 runs without slices)
  *   "qmv_small_m_tc"   2 <= M <= 16 on shapes the warp-level kernels do not take (other widths than 4-bit, group 32):
  *                      1 (default) 9 <= M <= 16, and 5 <= M <= 8 on matrices of 32 Mi codes or more, run on the
  *                      tensor-core kernel (f16 / bf16, K % 64 == 0, power-of-two group >= 32) instead of one FFMA per
@@ -276,9 +277,12 @@ int mtc_peer_barrier(mtc_ctx *ctx, void *stream, void *const *peer_flags, int n_
  *                      copy of the shard) must set this to 0 or synchronise first.  x and every store always wait.
  *   "peer_poll_limit"  polls of a wait on another GPU (mtc_peer_barrier, mtc_qmv_batched_sync) before it gives up
  *                      and records 0x601 + rank in the status word (default 4194304)
- * Scratch blocks.  bf16 mtc_qmm, mtc_gather_qmm, mtc_moe_experts and the tensor-memory decode kernel keep work lists
- * and staged activations in grow-only blocks of the context.  A block moves only outside stream capture (a call that
- * would have to grow one during capture fails with MTC_ERR_BUFFER: run the shape once before capturing), and an outgrown
+ * Scratch blocks.  mtc_qmm and mtc_qmm_multi (bf16: staged activations; both types: the partial sums of a launch that cuts K into
+ * slices), mtc_qmv where it runs on the tensor-core kernel, mtc_qvm (partial sums and arrival counters), mtc_gather_qmm,
+ * mtc_moe_experts, the M = 1 MoE tail, mtc_rms_norm_qmv on shapes its fused kernel does not take and the tensor-memory decode
+ * kernel keep work lists, staged activations and partial sums in grow-only blocks of the context.  A block moves only outside
+ * stream capture (a call that would have to grow one during capture fails with MTC_ERR_BUFFER - run the shape once before
+ * capturing - except for the K slices of mtc_qmm and mtc_qmm_multi, which are left out then), and an outgrown
  * block stays allocated until mtc_destroy, so graphs captured earlier and work already enqueued never see freed memory.
  * The blocks are per context, not per stream: calls of these entries from two streams that may overlap on the GPU race
  * on them - keep them on one stream, or order the streams with events, or use one context per stream. */

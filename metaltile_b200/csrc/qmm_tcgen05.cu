@@ -1272,7 +1272,12 @@ struct DensePlan {
     int TN, items_m, ksplit, halves;      // halves: wide items of an incomplete last round that run as two single-chunk items each
     bool wide;
 };
-DensePlan plan_dense(const Ctx *ctx, int M, int N, int K, int bits) {
+//
+// Slices cost a block of the context: at most kSliceBytes of partial sums, so that a rising prompt length cannot pile up outgrown
+// blocks without bound (they are kept until the context goes), and so that the sum kernel's 32-bit index holds every output.
+// slices = false: the best plan without them, for a caller whose block cannot grow.
+constexpr size_t kSliceBytes = size_t{512} << 20;
+DensePlan plan_dense(const Ctx *ctx, int M, int N, int K, int bits, bool slices = true) {
     const int n_tiles = (N + BMW - 1) / BMW, nkb = K / BK, nsb = (nkb + SB_PER_RAW - 1) / SB_PER_RAW, sms = ctx->sm_count;
     const auto up16 = [](int v) { return (v + 15) / 16 * 16; };
     if (ctx->qmm_force_tn > 0) return DensePlan{ctx->qmm_force_tn, (M + ctx->qmm_force_tn - 1) / ctx->qmm_force_tn, 1, 0, false};
@@ -1294,7 +1299,8 @@ DensePlan plan_dense(const Ctx *ctx, int M, int N, int K, int bits) {
         const int left = static_cast<int>(units % sms), last_rows = M - (items_m - 1) * 2 * TN;
         const bool tail = form == 1 && units > sms && left > 0 && 2 * left <= sms && last_rows > TN;
         for (int S = 1; S <= 16; ++S) {
-            if (S > 1 && (!ctx->qmm_ksplit || S > nsb || (ctx->qmm_wide != 1 && M > TN_MAX))) break;
+            if (S > 1 && (!slices || !ctx->qmm_ksplit || S > nsb || (ctx->qmm_wide != 1 && M > TN_MAX))) break;
+            if (S > 1 && static_cast<size_t>(S) * M * N * sizeof(float) > kSliceBytes) break;
             const int kb = S == 1 ? nkb : (nsb + S - 1) / S * SB_PER_RAW;
             const long long full = units * S / sms, rest = units * S % sms;
             double us = full * (kb * kb_us + kItemUs);
@@ -1323,7 +1329,7 @@ __global__ void __launch_bounds__(256) ksplit_sum_kernel(const float *partial, c
     const size_t mn = static_cast<size_t>(M) * N;
     const uint32_t per_row = N / V;
     for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < mn / V; i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-        // 32-bit division: more outputs than that never take K slices (their partial sums would not fit the device)
+        // 32-bit division: the partial sums of a launch are at most kSliceBytes
         const uint32_t m = static_cast<uint32_t>(i) / per_row, n = (static_cast<uint32_t>(i) - m * per_row) * V;
         float v[V];
         if constexpr (V == 4) {
@@ -1378,7 +1384,17 @@ cudaError_t launch_qmm_tcgen05(Ctx *ctx, cudaStream_t st, const void *w, const v
                                const void *x, void *out, int M, int N, int K, int bits, int group_size, int dt,
                                std::string *why, void *const *outs, int n_outs, long long out_ld) {
     const int sms = ctx->sm_count;
-    const DensePlan plan = plan_dense(ctx, M, N, K, bits);
+    DensePlan plan = plan_dense(ctx, M, N, K, bits);
+    if (plan.ksplit > 1) {
+        cudaError_t ge = grow_block(ctx, st, &ctx->d_ksplit, &ctx->ksplit_bytes, static_cast<size_t>(plan.ksplit) * M * N * sizeof(float), why);
+        if (ge != cudaSuccess) {
+            if (M <= 16) return ge;         // the caller has a kernel without scratch for these
+            // during capture, or out of memory: the same product without slices needs no block
+            if (ge != cudaErrorStreamCaptureUnsupported) cudaGetLastError();
+            if (why) why->clear();
+            plan = plan_dense(ctx, M, N, K, bits, false);
+        }
+    }
     const int TN = plan.TN;
     const void *x_op = nullptr;
     const float *tok_scale = nullptr;
@@ -1408,8 +1424,6 @@ cudaError_t launch_qmm_tcgen05(Ctx *ctx, cudaStream_t st, const void *w, const v
     // Few weight-row tiles: they alone would leave most SMs idle, so K is cut into slices that run as items of their own (f32
     // partial sums, added in slice order by a second small kernel).
     if (plan.ksplit > 1) {
-        cudaError_t ge = grow_block(ctx, st, &ctx->d_ksplit, &ctx->ksplit_bytes, static_cast<size_t>(plan.ksplit) * M * N * sizeof(float), why);
-        if (ge != cudaSuccess) return ge;
         p.ksplit = plan.ksplit;
         p.partial = static_cast<float *>(ctx->d_ksplit);
         p.dense_items = p.n_tiles * p.m_chunks * plan.ksplit;

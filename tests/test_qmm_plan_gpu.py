@@ -59,3 +59,61 @@ def test_grouped_product_on_ragged_rows(ctx, bits, gs, counts):
             r = slice(off[i], off[i + 1])
             ref = oracle.qmm(w[i * n:(i + 1) * n], s[i * n:(i + 1) * n], b[i * n:(i + 1) * n], x[r], c, n, k, bits, gs)
             assert rel_err(got[r.start:r.stop].float().cpu().numpy(), ref) <= TOL[dt]
+
+
+@pytest.mark.parametrize("m,n,k,bits,gs,multi", [(300, 1024, 4096, 4, 64, False), (700, 576, 2880, 8, 32, False), (300, 1024, 4096, 4, 64, True)])
+def test_capture_without_a_first_run(m, n, k, bits, gs, multi):
+    """f16 prompts captured on a fresh context.  The plan for these sizes cuts K into slices, whose partial sums need a block that
+    cannot grow during capture: the launch runs without slices instead of failing, and the replay matches the oracle."""
+    import torch
+    from metaltile_b200 import Context
+    from metaltile_b200.ops import _TORCH_DT
+    fresh, dt = Context(0), "f16"
+    w, s, b, x = dense_case(m, n, k, bits, gs, dt, seed=33)
+    wd, sd, bd, xd = to_dev(w), to_dev(s, dt), to_dev(b, dt), to_dev(x, dt)
+    outs = [torch.zeros((m, n), dtype=torch.float16, device="cuda") for _ in range(2 if multi else 1)]
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            st = torch.cuda.current_stream().cuda_stream
+            if multi:
+                fresh.qmm_multi(wd.data_ptr(), sd.data_ptr(), bd.data_ptr(), xd.data_ptr(), [o.data_ptr() for o in outs], n, m, n, k, bits, gs,
+                                _TORCH_DT[xd.dtype], stream=st)
+            else:
+                fresh.qmm(wd.data_ptr(), sd.data_ptr(), bd.data_ptr(), xd.data_ptr(), outs[0].data_ptr(), m, n, k, bits, gs, _TORCH_DT[xd.dtype], stream=st)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert fresh.status_word() == 0
+    rows = np.unique(np.r_[0:8, m // 2 - 4:m // 2 + 4, m - 8:m])
+    ref = oracle.qmm(w, s, b, np.ascontiguousarray(x[rows]), len(rows), n, k, bits, gs)
+    for o in outs:
+        assert rel_err(o.float().cpu().numpy()[rows], ref) <= TOL[dt]
+    # the same call outside capture takes its slices: the same products, added in another order
+    eager = torch.zeros_like(outs[0])
+    fresh.qmm(wd.data_ptr(), sd.data_ptr(), bd.data_ptr(), xd.data_ptr(), eager.data_ptr(), m, n, k, bits, gs, _TORCH_DT[xd.dtype],
+              stream=torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert rel_err(eager.float().cpu().numpy()[rows], ref) <= TOL[dt]
+
+
+def test_slices_stay_within_their_bound(ctx):
+    """A prompt whose slices would take more than the bound on their partial sums, and lengths that rise: the products are right and
+    the block of partial sums (with what it outgrew) stays small beside the outputs."""
+    import torch
+    from metaltile_b200 import Context, ops
+    fresh = Context(0)
+    n, k, bits, gs, dt = 576, 4096, 4, 64, "f16"
+    w, s, b, x = dense_case(4096, n, k, bits, gs, dt, seed=34)
+    wd, sd, bd, xd = to_dev(w), to_dev(s, dt), to_dev(b, dt), to_dev(x, dt)
+    torch.cuda.synchronize()
+    free0 = torch.cuda.mem_get_info()[0]
+    for m in range(300, 4096, 211):
+        got = ops.qmm(wd, sd, bd, xd[:m], bits, gs, ctx=fresh)
+        rows = np.r_[0:4, m - 4:m]
+        ref = oracle.qmm(w, s, b, np.ascontiguousarray(x[rows]), len(rows), n, k, bits, gs)
+        assert rel_err(got.float().cpu().numpy()[rows], ref) <= TOL[dt]
+        del got
+    torch.cuda.empty_cache()
+    assert free0 - torch.cuda.mem_get_info()[0] < 3 * (512 << 20) * 1.5 + (64 << 20)
