@@ -331,8 +331,9 @@ __global__ void __launch_bounds__(256) affine_quantize8_kernel(const void *w, ui
         for (int o = 4; o < lpg; o <<= 1) m.merge_xor(o);
         if (gs_log2 >= 9) m.merge_xor(1);                          // 512 values: unit indexes 0 and 1, 2 and 3
         if (gs_log2 >= 10) m.merge_xor(2);                         // 1024: all four
-        const float my_mn = m.lo();
-        const float div = __fdiv_rn(__fsub_rn(m.hi(), my_mn), n_bins);
+        // the scalar formula starts from +inf and -inf, which is what a group of nothing but NaN keeps (scale 1, bias +inf)
+        const float my_mn = fminf(m.lo(), INFINITY);
+        const float div = __fdiv_rn(__fsub_rn(fmaxf(m.hi(), -INFINITY), my_mn), n_bins);
         const float scale = div < 1.0e-7f ? 1.0f : div;
         const float my_inv = __fdiv_rn(1.0f, scale);
         {   // the first lanes of a group hold its unit indexes: lane j of them stores the scale and bias of index j

@@ -33,3 +33,43 @@ def test_codec_is_exact(bits, gs, dt):
     assert np.array_equal(b_h, oracle.round_through(obi, ODT[dt]))
     ref = oracle.round_through(oracle.affine_dequantize(oq, s_h, b_h, n * gs, bits, gs), ODT[dt])
     assert np.array_equal(back.float().cpu().numpy().reshape(-1), ref)
+
+
+def _awkward_groups(gs, dt):
+    """Groups of values that are not ordinary numbers: all NaN, partly NaN, both infinities, one of them, nothing but one
+    infinity, a span past the largest f32 (or the type's largest values), and one whose 1 / scale is subnormal."""
+    big = {"f32": 3.4e38, "f16": 65504.0, "bf16": 3.38e38}[dt]
+    g = np.random.default_rng(gs).standard_normal((9, gs)).astype(np.float32)
+    g[0, :] = np.nan
+    g[1, ::3] = np.nan
+    g[2, 0], g[2, gs - 1] = np.inf, -np.inf
+    g[3, 5] = np.inf
+    g[4, 7] = -np.inf
+    g[5, :] = np.inf
+    g[6, 0], g[6, 1] = big, -big
+    g[7, :] = 0.0
+    g[7, 2] = big                                         # 2- and 3-bit f32: the scale is above 2^126
+    g[8, :gs - 1] = np.nan                                # one number among NaN: the scale is 1
+    return oracle.round_through(g, ODT[dt])
+
+
+@pytest.mark.parametrize("dt", ["f32", "f16", "bf16"])
+@pytest.mark.parametrize("bits", [2, 3, 4, 8])
+@pytest.mark.parametrize("gs,shift", [(32, 0), (64, 0), (256, 0), (512, 0), (1024, 0), (64, 1), (96, 0)])
+def test_values_that_are_not_numbers(gs, shift, bits, dt):
+    """The same codes, scales and biases as the scalar formula whatever kernel runs: the vector form (whole warps of units), the
+    warp-per-group form (``shift``: an input that is not 16-byte aligned; 96: no power of two)."""
+    import torch
+    from metaltile_b200 import ops
+    wf = _awkward_groups(gs, dt)
+    src = to_dev(wf, dt)
+    room = torch.empty(src.numel() + 8, dtype=src.dtype, device="cuda")
+    src = room[shift:shift + src.numel()].view(src.shape).copy_(src)
+    q, s, b = ops.affine_quantize(src, bits, gs)
+    torch.cuda.synchronize()
+    with np.errstate(all="ignore"):
+        oq, osc, obi = oracle.affine_quantize(wf, bits, gs)
+        osc, obi = oracle.round_through(osc, ODT[dt]), oracle.round_through(obi, ODT[dt])
+    assert np.array_equal(s.float().cpu().numpy().reshape(-1), osc, equal_nan=True)
+    assert np.array_equal(b.float().cpu().numpy().reshape(-1), obi, equal_nan=True)
+    assert np.array_equal(q.cpu().numpy().view(np.uint32).reshape(-1), oq)
