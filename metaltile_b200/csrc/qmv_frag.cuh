@@ -162,9 +162,14 @@ __device__ __forceinline__ void ldg4(const void *p, uint32_t *v, bool on) {
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p ld.global.nc.u32 %0, [%1];\n\t}"
                  : "+r"(v[0]) : "l"(p), "r"(static_cast<uint32_t>(on)));
 }
-__device__ __forceinline__ void ldg2(const void *p, uint32_t *v, bool on) {
-    asm volatile("{\n\t.reg .pred p;\n\t.reg .u16 h;\n\tsetp.ne.b32 p, %2, 0;\n\tcvt.u16.u32 h, %0;\n\t@p ld.global.nc.u16 h, [%1];\n\tcvt.u32.u16 %0, h;\n\t}"
-                 : "+r"(v[0]) : "l"(p), "r"(static_cast<uint32_t>(on)));
+// Scales and biases: zero outside the row.  What the run before left there need not be finite, and inf * 0 is not 0.
+__device__ __forceinline__ void ldg4_or_zero(const void *p, uint32_t *v, bool on) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\tmov.u32 %0, 0;\n\t@p ld.global.nc.u32 %0, [%1];\n\t}"
+                 : "=&r"(v[0]) : "l"(p), "r"(static_cast<uint32_t>(on)));
+}
+__device__ __forceinline__ void ldg2_or_zero(const void *p, uint32_t *v, bool on) {
+    asm volatile("{\n\t.reg .pred p;\n\t.reg .u16 h;\n\tsetp.ne.b32 p, %2, 0;\n\tmov.u16 h, 0;\n\t@p ld.global.nc.u16 h, [%1];\n\tcvt.u32.u16 %0, h;\n\t}"
+                 : "=r"(v[0]) : "l"(p), "r"(static_cast<uint32_t>(on)));
 }
 
 // ... and the plain ones, where the whole run lies inside the row
@@ -239,8 +244,8 @@ __device__ __forceinline__ float scale_f32(uint32_t raw) {
 }
 template <int XT>
 __device__ __forceinline__ void ld_scale(const char *p, uint32_t *v, bool on) {
-    if (XT == MTC_F32) ldg4(p, v, on);
-    else ldg2(p, v, on);
+    if (XT == MTC_F32) ldg4_or_zero(p, v, on);
+    else ldg2_or_zero(p, v, on);
 }
 template <int XT>
 __device__ __forceinline__ void ld_scale(const char *p, uint32_t *v) {

@@ -76,3 +76,29 @@ def test_projections_in_one_launch_equal_separate_ones(ctx, m, k, bits, gs):
     for g, t in zip(got, mats):
         assert rel_err(g.float().cpu().numpy().reshape(m, -1), t[3]) <= BOUND["bf16"]
         assert torch.equal(g.reshape(m, -1), ops.qmv(*t[:3], xd, bits, gs, ctx=ctx).reshape(m, -1))
+
+
+@pytest.mark.parametrize("bits,gs,dt,m", [(4, 64, "bf16", 1), (4, 32, "f16", 4), (8, 64, "f32", 5), (8, 64, "bf16", 7), (2, 64, "f16", 2)])
+def test_infinite_scales(ctx, bits, gs, dt, m):
+    """One group with an infinite scale in some rows, before a last run of K that is not full: lanes past the end of the row must
+    not multiply their zeros by what the run before left in their registers (inf * 0), and the other rows stay finite.  The
+    weights' codes are not zero, so the sum of the group is not, and the result is the infinity that the CUDA cores get."""
+    import torch
+    from metaltile_b200 import ops
+    n, k = 40000, 1088
+    w, s, b, x = dense_case(m, n, k, bits, gs, dt, seed=5)
+    w |= np.uint32({2: 0x55555555, 4: 0x11111111, 8: 0x01010101}[bits])
+    x = np.abs(x)
+    bad = np.arange(0, n, 97)
+    s[bad, 640 // gs] = np.inf                     # of the second run of 512 codes, in steps that the third one does not reach
+    s[bad[::2], 960 // gs] = np.inf
+    want = np.zeros(n, dtype=bool)
+    want[bad] = True
+    for frag in (0, 2):
+        ctx.set_option("qmv_frag", frag)
+        try:
+            got = ops.qmv(to_dev(w), to_dev(s, dt), to_dev(b, dt), to_dev(x, dt), bits, gs, ctx=ctx)
+        finally:
+            ctx.set_option("qmv_frag", 1)
+        got = got.float().cpu().numpy()
+        assert (np.isposinf(got) == want).all() and np.isfinite(got[:, ~want]).all(), frag
