@@ -289,6 +289,10 @@ __device__ __forceinline__ float stage_chunk(const FragArgs &a, int m, int k_lo,
                 o[p][r & 3] = b;
                 lo -= __uint_as_float(b << 16);
                 hi -= __uint_as_float(b & 0xFFFF0000u);
+                if (p == 0) {             // an infinity or a NaN is all in the first piece: inf - inf would make the others NaN
+                    if ((b & 0x7F80u) == 0x7F80u) lo = 0.0f;
+                    if ((b & 0x7F800000u) == 0x7F800000u) hi = 0.0f;
+                }
             }
             if ((r & 3) == 3) {
 #pragma unroll

@@ -102,3 +102,28 @@ def test_infinite_scales(ctx, bits, gs, dt, m):
             ctx.set_option("qmv_frag", 1)
         got = got.float().cpu().numpy()
         assert (np.isposinf(got) == want).all() and np.isfinite(got[:, ~want]).all(), frag
+
+
+@pytest.mark.parametrize("bits,dt,m", [(8, "f32", 5), (4, "f32", 16), (4, "bf16", 1), (8, "bf16", 4), (4, "f16", 2)])
+def test_infinite_activations(ctx, bits, dt, m):
+    """x = inf against weights that are all positive is inf (a CUDA-core product of the same inputs says so too), x = nan is nan, and
+    the other tokens know nothing of either."""
+    import torch
+    from metaltile_b200 import ops
+    n, k, gs = 64, 512, 64
+    w, s, b, x = dense_case(m, n, k, bits, gs, dt, seed=6)
+    w |= np.uint32(0x11111111 if bits == 4 else 0x01010101)             # no code is zero
+    b = np.abs(b)
+    x[0, 100] = np.inf
+    if m > 2:
+        x[2, 300] = np.nan
+    for frag in (2, 0):
+        ctx.set_option("qmv_frag", frag)
+        try:
+            got = ops.qmv(to_dev(w), to_dev(s, dt), to_dev(b, dt), to_dev(x, dt), bits, gs, ctx=ctx).float().cpu().numpy()
+        finally:
+            ctx.set_option("qmv_frag", 1)
+        assert (got[0] == np.inf).all(), frag
+        if m > 2:
+            assert np.isnan(got[2]).all()
+        assert np.isfinite(got[[i for i in range(m) if i not in (0, 2)]]).all()
