@@ -431,6 +431,14 @@ __device__ __noinline__ void store_row8(char *o, uint4 v, int n) {
         if (e < n) reinterpret_cast<unsigned short *>(o)[e] = static_cast<unsigned short>(w[e >> 1] >> (16 * (e & 1)));
 }
 
+// The epilogue warps' vote: true when all 128 threads say so (named barrier 1, which their blocks of rows use too)
+__device__ __forceinline__ bool epilogue_agrees(bool ok) {
+    uint32_t all;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.and.pred q, 1, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+                 : "=r"(all) : "r"(static_cast<uint32_t>(ok)) : "memory");
+    return all != 0;
+}
+
 struct Item {
     int n_tile, expert, row0, rows;
     int nc;                                 // token chunks of TN rows covered (1 or 2): one accumulator each
@@ -741,7 +749,11 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
             const int buf = both ? 0 : (tile_i & 1);
             const uint32_t acc_ph = (both ? tile_i : (tile_i >> 1)) & 1;
             const Item item = get_item<KSPLIT>(p, i);
-            if (!(ok = mbar_wait_warp(&ctl->acc_full[buf], acc_ph, ctl, p.status, 0x301, p.hint_ns))) break;
+            ok = mbar_wait_warp(&ctl->acc_full[buf], acc_ph, ctl, p.status, 0x301, p.hint_ns);
+            // The four warps share named barriers below, so they give up together: a warp that gave up while another saw the
+            // barrier complete would leave that one waiting for good.
+            if constexpr (!KSPLIT) ok = epilogue_agrees(ok);
+            if (!ok) break;
             tc_fence_after();
             const int n = item.n_tile * BMW + q * 32 + lane;     // output column owned by this thread
             const bool n_ok = n < p.N;
