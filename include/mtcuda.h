@@ -270,11 +270,13 @@ int mtc_peer_barrier(mtc_ctx *ctx, void *stream, void *const *peer_flags, int n_
  *   "qmv_tc"           1: those shapes run on the tensor-memory decode kernel instead (slower today; default 0)
  *   "gather_stream"    0: grouped products never take the weight-streaming kernel (default 1: the CSR form with
  *                      4-bit codes, f16 / bf16, k_in % 256 == 0, group 64 or 128 and m_total <= 64 n_experts does)
- *   "pdl_early_weights" 0: no decode kernel reads w, scales or biases before the previous kernel of its stream is
- *                      complete.  Default 1: the decode kernels are launched with programmatic dependent launch and
- *                      start copying WEIGHTS while the previous kernel drains - weights are constants of the model;
- *                      a caller whose previous kernel on the stream WRITES them (an on-stream repack, dequant or
- *                      copy of the shard) must set this to 0 or synchronise first.  x and every store always wait.
+ *   "pdl_early_weights" 0: no product reads w, scales or biases before the previous kernel of its stream is
+ *                      complete.  Default 1: the dense products (mtc_qmv*, mtc_qmm*, mtc_qvm, chains) are launched with
+ *                      programmatic dependent launch and start copying WEIGHTS while the previous kernel drains - weights are
+ *                      constants of the model.  mtc_affine_quantize in front of them is known to the context and always
+ *                      safe; a caller whose own previous kernel on the stream WRITES weights (an on-stream repack or copy of
+ *                      the shard) must set this to 0 or synchronise first.  x and every store always wait.  The grouped
+ *                      products, the codec and the M = 1 MoE tail wait for everything.
  *   "peer_poll_limit"  polls of a wait on another GPU (mtc_peer_barrier, mtc_qmv_batched_sync) before it gives up
  *                      and records 0x601 + rank in the status word (default 4194304)
  * Scratch blocks.  mtc_qmm and mtc_qmm_multi (bf16: staged activations; both types: the partial sums of a launch that cuts K into

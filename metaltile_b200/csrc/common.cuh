@@ -41,6 +41,8 @@ struct Ctx {
     std::vector<void *> retired;   // outgrown scratch blocks: freed by mtc_destroy, so that captured graphs never see freed memory
     int qmv_frag = 1;              // option "qmv_frag": 0 = never use the fragment kernel (qmv_frag.cuh), 2 = whenever it supports the shape
     int qmv_stream = 1;            // option "qmv_stream": 0 = never use the streaming decode kernel (qmv_stream.cu)
+    std::vector<cudaStream_t> fresh_weights;   // streams on which mtc_affine_quantize ran since their last product (early_weights below)
+    bool fresh_anywhere = false;   // more streams than that list holds: no product starts on its weights early any more
     int pdl_early_weights = 1;     // option "pdl_early_weights": 0 = no load of w / scales / biases before the previous kernel of the stream is complete
     void *d_worklist = nullptr;    // gather_qmm work list (grow-only, owned by the context)
     size_t worklist_bytes = 0;
@@ -84,6 +86,29 @@ inline cudaError_t grow_block(Ctx *ctx, cudaStream_t st, void **block, size_t *h
     *block = p;
     *have = want;
     return cudaSuccess;
+}
+
+// Products request their weights before the previous kernel of the stream is complete: weights are constants.  The one kernel of
+// this library that writes weights is the quantizer, so the first product behind it on its stream does not start early; by the
+// time that product lets the next one start, its own wait has made the quantizer's stores visible.  (That next one, and
+// everything on other streams that is ordered by an event, needs nothing more.)  A product that does not start early waits
+// before it signals its dependents.
+inline void weights_written(Ctx *ctx, cudaStream_t st) {
+    if (st == cudaStreamLegacy) st = nullptr;
+    for (cudaStream_t s : ctx->fresh_weights)
+        if (s == st) return;
+    if (ctx->fresh_weights.size() < 64) ctx->fresh_weights.push_back(st);
+    else ctx->fresh_anywhere = true;
+}
+// called once per product launch: may it start on its weights before the previous kernel of the stream is complete?
+inline int early_weights(Ctx *ctx, cudaStream_t st) {
+    if (st == cudaStreamLegacy) st = nullptr;
+    for (size_t i = 0; i < ctx->fresh_weights.size(); ++i)
+        if (ctx->fresh_weights[i] == st) {
+            ctx->fresh_weights.erase(ctx->fresh_weights.begin() + static_cast<std::ptrdiff_t>(i));
+            return 0;
+        }
+    return ctx->pdl_early_weights && !ctx->fresh_anywhere ? 1 : 0;
 }
 
 inline int fail(Ctx *ctx, int code, const std::string &msg) {

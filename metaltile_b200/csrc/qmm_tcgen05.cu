@@ -538,8 +538,8 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = ctl->tmem_base;
-    asm volatile("griddepcontrol.launch_dependents;");
     if (!p.pdl_roles) asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;");
     // a list of work items comes from an earlier kernel of the stream (pdl_roles is 0 then): its length after the wait
     const int num_items = p.items ? *p.item_count : p.dense_items;
 
@@ -1427,7 +1427,7 @@ cudaError_t launch_qmm_tcgen05(Ctx *ctx, cudaStream_t st, const void *w, const v
     p.M = M;
     p.m_chunks = (M + TN - 1) / TN;
     p.n_tiles = (N + BMW - 1) / BMW;
-    p.pdl_roles = ctx->pdl_early_weights ? 1 : 0;
+    p.pdl_roles = early_weights(ctx, st);
     p.wide = plan.wide ? 1 : 0;
     plan_smem(p, ctx, bits);
     p.m_chunks = plan.items_m;

@@ -581,7 +581,7 @@ cudaError_t launch_pipe(Ctx *ctx, cudaStream_t st, QmvArgs a, size_t per_jb, siz
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = early_weights(ctx, st);       // this kernel requests weights before it waits: an ordinary launch where it must not
     if constexpr (MT == 1) {
         if (tail) {        // multi-destination instantiation: same configuration, one more parameter
             auto mk = qmv_pipe_kernel<BITS, MT, kRows, V, PF, true>;

@@ -51,7 +51,7 @@ cudaError_t launch_qmv_frag(Ctx *ctx, cudaStream_t st, const mtc_qmv_desc *d, in
         a.gpr = K / d[0].group_size;
         a.steps = (K + 127) / 128;
         a.x = static_cast<const char *>(d[0].x) + static_cast<size_t>(m0) * K * esz;
-        a.early = ctx->pdl_early_weights;
+        a.early = early_weights(ctx, st);
         a.n_proj = n;
         bool aligned16 = true;
         for (int i = 0; i < n; ++i) {

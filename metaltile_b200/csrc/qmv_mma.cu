@@ -678,7 +678,7 @@ cudaError_t launch_ring(Ctx *ctx, cudaStream_t st, MmaArgs a) {
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = early_weights(ctx, st);       // this kernel requests weights before it waits: an ordinary launch where it must not
     if (a.M == NT * 8) return cudaLaunchKernelEx(&cfg, qmv_mma_ring_kernel<NT, BF16, true, GSH>, a);
     return cudaLaunchKernelEx(&cfg, qmv_mma_ring_kernel<NT, BF16, false, GSH>, a);
 }
@@ -720,7 +720,7 @@ cudaError_t launch_mma(Ctx *ctx, cudaStream_t st, MmaArgs a) {
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = early_weights(ctx, st);       // this kernel requests weights before it waits: an ordinary launch where it must not
     return cudaLaunchKernelEx(&cfg, kernel, a);
 }
 

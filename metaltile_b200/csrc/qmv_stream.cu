@@ -392,6 +392,7 @@ __global__ void __launch_bounds__(kThreads, 2) qmv_stream_kernel(const __grid_co
     const int g = lane >> 2, t = lane & 3;
     const bool chain = a.projs != nullptr;
 
+    if (!a.early_weights) asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;");
     if (threadIdx.x < kRedSlots) {
         ctl->cnt[threadIdx.x] = 0u;
@@ -471,7 +472,6 @@ __global__ void __launch_bounds__(kThreads, 2) qmv_stream_kernel(const __grid_co
         cp_commit();
     };
 
-    if (!a.early_weights) asm volatile("griddepcontrol.wait;" ::: "memory");
     copy_enter();
     // the whole ring is requested before anything waits: the copies run while the previous kernel of the stream drains
     // and while this CTA stages its activations
@@ -801,9 +801,9 @@ static cudaError_t launch_stream_kernel(cudaStream_t st, const SArgs &a, KernelF
     return cudaLaunchKernelEx(&cfg, fn, a);
 }
 
-static void fill_layout(SArgs &a, Ctx *ctx, const Plan &plan) {
+static void fill_layout(SArgs &a, Ctx *ctx, cudaStream_t st, const Plan &plan) {
     a.status = ctx->d_status;
-    a.early_weights = ctx->pdl_early_weights;
+    a.early_weights = early_weights(ctx, st);
     a.off_xsum = plan.off_xsum;
     a.off_red = plan.off_red;
     a.off_ring = plan.off_ring;
@@ -841,7 +841,7 @@ cudaError_t launch_qmv_stream(Ctx *ctx, cudaStream_t st, const mtc_qmv_desc *d, 
     const int M = d[0].M, K = d[0].K;
     const Plan plan = make_plan(M * K, K, M);
     if (plan.depth < 2) return cudaErrorInvalidValue;
-    fill_layout(a, ctx, plan);
+    fill_layout(a, ctx, st, plan);
     // one CTA per resident slot of the machine, at least 8 rows each
     long long grid = static_cast<long long>(ctx->sm_count) * plan.per_sm;
     if (grid > (rows + 7) / 8) grid = (rows + 7) / 8;
@@ -1002,7 +1002,7 @@ cudaError_t stream_chain_run(Ctx *ctx, cudaStream_t st, StreamChain *c) {
     a.max_pieces = c->max_pieces;
     a.sync = c->d_sync;
     a.n_phases = c->n_phases;
-    fill_layout(a, ctx, c->plan);
+    fill_layout(a, ctx, st, c->plan);
     if (c->n_phases > 1) {
         // CTAs wait for one another at phase boundaries: all of them must be resident, which a cooperative launch
         // guarantees (or refuses)

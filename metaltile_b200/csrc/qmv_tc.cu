@@ -203,6 +203,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) qmv_tc_kernel(const __grid_cons
     const int id1 = static_cast<int>(static_cast<long long>(a.items) * (blockIdx.x + 1) / gridDim.x);
     const int n_items = id1 - id0;
 
+    if (!a.early_weights) asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;");
     if (threadIdx.x == 0) {
         for (int s = 0; s < 2; ++s) {              // one pair of barriers per slice: its four stages are handed over together
@@ -315,7 +316,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) qmv_tc_kernel(const __grid_cons
                 cpa16(dst + r * 128 + ((cch ^ (r & 7)) << 4), src + static_cast<size_t>(grow) * a.rowbytes);
             }
         };
-        if (!a.early_weights) asm volatile("griddepcontrol.wait;" ::: "memory");
         int n_issue = sl;
 #pragma unroll 1
         for (int p = 0; p < ahead; ++p) {
@@ -630,7 +630,7 @@ cudaError_t launch_qmv_tc(Ctx *ctx, cudaStream_t st, const void *w, const void *
     a.status = ctx->d_status;
     const uint32_t fmt = dt == MTC_BF16 ? 1u : 0u;
     a.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | (static_cast<uint32_t>(16 >> 3) << 17) | (static_cast<uint32_t>(128 >> 4) << 24);
-    a.early_weights = ctx->pdl_early_weights;
+    a.early_weights = early_weights(ctx, st);
     a.bf16 = dt == MTC_BF16;
     size_t smem = 0;
     if (!tc_layout(M, K, a.off_p, a.off_ring, a.ahead, smem)) return cudaErrorInvalidValue;

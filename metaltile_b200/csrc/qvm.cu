@@ -134,6 +134,7 @@ __global__ void __launch_bounds__(kQvWarps * 32, 2) qvm_kernel(const uint32_t *w
         fetch_w(u, sl);
         fetch_x(u, sl);
     };
+    if (!early) asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;");
     // weights are constants of the model: the first slab may be requested while the previous kernel of the stream still runs
     const int u0 = kc * kQvWarps + warp;
@@ -390,9 +391,9 @@ __global__ void __launch_bounds__(kQmWarps * 32, 1) qvm_mma_kernel(const QmArgs 
 #pragma unroll
     for (int c = 0; c < S::CPL; ++c) acc[c] = 0.0f;
     At cur = batch_at(kc + a.KC * warp), ahead = next(cur);
+    if (!a.early) asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;");
     // weights are constants of the model: the first slabs may be requested while the previous kernel of the stream still runs
-    if (!a.early) asm volatile("griddepcontrol.wait;" ::: "memory");
     issue_w(cur, 0);
     issue_w(ahead, 1);
     issue_scales(cur);                                             // later batches: with the slab after their first one
@@ -665,7 +666,7 @@ cudaError_t launch_qvm(Ctx *ctx, cudaStream_t st, const void *w, const void *sca
     uint32_t *tickets = KC > 1 && n_tickets <= kQvTickets ? static_cast<uint32_t *>(scratch) : nullptr;   // else a second kernel adds the chunks
     float *partial = KC > 1 ? reinterpret_cast<float *>(static_cast<uint32_t *>(scratch) + kQvTickets) : nullptr;
     cudaError_t e;
-    const int early = ctx->pdl_early_weights;
+    const int early = early_weights(ctx, st);
     if (qvm_takes_mma(M, N, K, bits, group_size, dt)) {
         QmArgs a{static_cast<const uint32_t *>(w), scales, biases, x, partial, tickets, out, M, N, K, group_size, KC, 0, 1, K / 32, 0, early};
         qm_batches(ctx->sm_count, M, N, K, bits, group_size, &a.ch_log2, &a.bs);

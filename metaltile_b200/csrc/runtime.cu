@@ -841,6 +841,7 @@ int mtc_affine_quantize(mtc_ctx *ctx, void *stream, const void *w, void *out, vo
     if (!w || !out || !scales || !biases) return fail(ctx, MTC_ERR_INVALID, "affine_quantize: null pointer");
     MTC_CUDA(ctx, mtc::launch_affine_quantize(ctx, static_cast<cudaStream_t>(stream), w, out, scales, biases, n_elem / group_size, bits,
                                               group_size, dtype), MTC_ERR_DISPATCH);
+    mtc::weights_written(ctx, static_cast<cudaStream_t>(stream));
     return MTC_OK;
 }
 

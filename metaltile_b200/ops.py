@@ -142,7 +142,8 @@ def rms_norm_qmv(w, scales, biases, x, norm_weight, eps: float, bits: int, group
 def affine_quantize(w, bits: int, group_size: int, ctx: Context = None):
     """Float tensor ``w [..., K]`` (K a multiple of the group size) -> (packed int32 ``[..., K*bits/32]``, scales, biases
     ``[..., K/group_size]``) in the layout the quantized matmuls read (``mt_affine_quantize_int*``,
-    crates/metaltile-std/src/mlx/quantized.rs:3629-3667)."""
+    crates/metaltile-std/src/mlx/quantized.rs:3629-3667).  A product of them may follow on the same stream at once: the
+    context keeps it from requesting its weights before they are written (other writers: option ``pdl_early_weights``)."""
     return _native.affine_quantize(w, bits, group_size, ctx)
 
 
@@ -159,5 +160,6 @@ def dequant_gather(weight, scales, biases, indices, bits: int, group_size: int, 
 
 def qvm(w, scales, biases, x, bits: int, group_size: int, out=None, ctx: Context = None):
     """``x @ W`` with W stored transposed and quantized along K: w [K, N*bits/32], scales / biases [K/group_size, N],
-    x [M, K] -> out [M, N] (``mt_qvm_*``, crates/metaltile-std/src/mlx/quantized.rs:4397-4530)."""
+    x [M, K] -> out [M, N] (``mt_qvm_*``, crates/metaltile-std/src/mlx/quantized.rs:4397-4530).  Like the other dense products
+    it requests its first weights while the previous kernel of the stream drains (option ``pdl_early_weights``)."""
     return _native.qvm(w, scales, biases, x, bits, group_size, out, ctx)

@@ -164,3 +164,59 @@ def test_codec_behind_swiglu_and_itself(ctx, bits, dt):
         return [*q, back, *ops.affine_quantize(back, bits, 64, ctx=ctx)]
 
     _same_without_waiting(step)
+
+
+PRODUCTS = {
+    # kernel: (m, n, k, bits, dt, options)
+    "frag": (1, 1024, 2048, 4, "bf16", {}), "frag_8bit": (4, 1024, 2048, 8, "f16", {}), "frag_f32": (8, 1024, 2048, 4, "f32", {}),
+    "stream": (1, 4096, 2048, 4, "bf16", dict(qmv_frag=0)), "ring": (8, 1024, 2048, 4, "bf16", {}), "mma": (8, 1024, 2048 - 64, 4, "f16", dict(qmv_frag=0)),
+    "cuda": (1, 1024, 2048, 5, "bf16", dict(qmv_frag=0)), "tc": (2, 1024, 2048, 4, "bf16", dict(qmv_tc=1)),
+    "qmm": (200, 1024, 2048, 4, "f16", {}), "qmm_bf16": (200, 1024, 2048, 8, "bf16", {}), "grouped": (64, 2048, 1024, 4, "f16", {}),
+    "qvm": (1, 2048, 1024, 4, "bf16", {}), "qvm_mma": (4, 4096, 2048, 4, "f16", {}),
+}
+
+
+@pytest.mark.parametrize("early", [1, 0])
+@pytest.mark.parametrize("between", [False, True])
+@pytest.mark.parametrize("kind", sorted(PRODUCTS))
+def test_products_of_weights_just_quantized(ctx, kind, between, early):
+    """Packed words, scales and biases are rewritten in place by the quantizer and used at once: by the product behind it, by a second
+    one behind that, and with another kernel (which lets the product start while the quantizer may still run) in between."""
+    import torch
+    from metaltile_b200 import ops
+    from metaltile_b200.ops import _TORCH_DT
+    m, n, k, bits, dt, options = PRODUCTS[kind]
+    dtype = dict(f32=torch.float32, f16=torch.float16, bf16=torch.bfloat16)[dt]
+    rounds = 16
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    # qvm: groups along K of a transposed matrix; its words are those of [k, n] and its scales are made separately
+    qvm = kind.startswith("qvm")
+    shape = (k, n) if qvm else (n, k)
+    ws = [torch.randn(shape, device="cuda", generator=gen).to(dtype) for _ in range(rounds)]
+    q = [t.clone() for t in ops.affine_quantize(ws[0], bits, 64, ctx=ctx)]
+    t_s = torch.rand(k // 64, n, device="cuda", generator=gen).to(dtype)
+    x = torch.randn(m, k, device="cuda", generator=gen).to(dtype)
+    junk = torch.empty_like(x)
+    offsets = torch.tensor([0, m // 2, m // 2, m], dtype=torch.int32, device="cuda")
+
+    def product():
+        if qvm:
+            return ops.qvm(q[0], t_s, t_s, x, bits, 64, ctx=ctx)
+        if kind == "grouped":
+            return ops.gather_qmm(x, *(t[:n // 3 * 3].view(3, n // 3, -1) for t in q), bits, 64, expert_offsets=offsets, ctx=ctx)
+        return ops.qmm(*q, x, bits, 64, ctx=ctx)
+
+    def step(i):
+        ctx.affine_quantize(ws[i].data_ptr(), q[0].data_ptr(), q[1].data_ptr(), q[2].data_ptr(), ws[i].numel(), bits, 64, _TORCH_DT[dtype],
+                            stream=torch.cuda.current_stream().cuda_stream)
+        if between:
+            ops.swiglu(x, x, out=junk, ctx=ctx)
+        return [product(), product()]
+
+    for name, v in dict(options, pdl_early_weights=early).items():
+        ctx.set_option(name, v)
+    try:
+        _same_without_waiting(step, rounds)
+    finally:
+        for name, v in dict(qmv_frag=1, qmv_tc=0, pdl_early_weights=1).items():
+            ctx.set_option(name, v)
