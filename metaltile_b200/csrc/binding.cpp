@@ -78,6 +78,21 @@ void check_out(const at::Tensor &out, int64_t M, int64_t N, const at::Tensor &li
 
 void *stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
 
+// Without the interpreter lock: an allocation and an entry of the library may wait (a full launch queue, a block that grows, the
+// first load of a kernel) while other Python threads have work, on another GPU for instance.  Nothing of Python's inside; a C++
+// exception takes the lock again on its way out.
+struct Unlocked {
+    PyThreadState *state = PyEval_SaveThread();
+    Unlocked() = default;
+    Unlocked(const Unlocked &) = delete;
+    ~Unlocked() { PyEval_RestoreThread(state); }
+};
+template <typename F>
+int unlocked(F &&f) {
+    const Unlocked u;
+    return f();
+}
+
 // ---- the Context of a call ---------------------------------------------------------------------------
 // ops.context(device) makes a device's Context on first use; it is looked up here once per device.
 PyObject *g_context_fn = nullptr;               // ops.context
@@ -193,15 +208,17 @@ PyObject *dense(Args a, Py_ssize_t n) {
     nargs(n, 9);
     const long long which = integer(a[0]);
     Dense d(a[1], a[2], a[3], a[4], integer(a[5]), integer(a[6]));
-    at::Tensor made;
-    if (a[7] == Py_None) made = empty({d.rows.M, d.N}, d.x.scalar_type(), d.x);
-    else check_out(tensor(a[7], "out"), d.rows.M, d.N, d.x);
-    const at::Tensor &out = a[7] == Py_None ? made : THPVariable_Unpack(a[7]);
+    const bool given = a[7] != Py_None;
+    at::Tensor out = given ? tensor(a[7], "out") : at::Tensor();
+    if (given) check_out(out, d.rows.M, d.N, d.x);
     const Call c(a[8], d.x);
-    c.check((which ? mtc_qmm : mtc_qmv)(c.h, stream(), d.w.data_ptr(), d.scales.data_ptr(), d.biases.data_ptr(), d.rows.t->data_ptr(),
-                                        out.data_ptr(), static_cast<int>(d.rows.M), static_cast<int>(d.N), static_cast<int>(d.rows.K),
-                                        static_cast<int>(d.bits), static_cast<int>(d.group), d.dt));
-    return a[7] == Py_None ? wrap(std::move(made)) : same(a[7]);
+    c.check(unlocked([&] {
+        if (!given) out = empty({d.rows.M, d.N}, d.x.scalar_type(), d.x);
+        return (which ? mtc_qmm : mtc_qmv)(c.h, stream(), d.w.data_ptr(), d.scales.data_ptr(), d.biases.data_ptr(), d.rows.t->data_ptr(),
+                                           out.data_ptr(), static_cast<int>(d.rows.M), static_cast<int>(d.N), static_cast<int>(d.rows.K),
+                                           static_cast<int>(d.bits), static_cast<int>(d.group), d.dt);
+    }));
+    return given ? same(a[7]) : wrap(std::move(out));
 }
 
 // qmv_batched(mats, x, bits, group_size, out, ctx)
@@ -220,15 +237,23 @@ PyObject *qmv_batched(Args a, Py_ssize_t n) {
     int64_t total = 0, ns[4] = {};
     if (count < 1 || count > 4) {
         const Call c(a[5], x);
-        c.check(mtc_qmv_batched(c.h, stream(), descs, static_cast<int>(count)));
+        c.check(mtc_qmv_batched(c.h, stream(), descs, static_cast<int>(count)));         // (refused at once)
     }
-    PyObject *parts[4][3];
+    // held: another thread may change a list of the caller's while the lock is let go below
+    struct Parts {
+        PyObject *p[4][3] = {};
+        PyObject **operator[](Py_ssize_t i) { return p[i]; }
+        ~Parts() {
+            for (auto &m : p)
+                for (PyObject *o : m) Py_XDECREF(o);
+        }
+    } parts;
     for (Py_ssize_t i = 0; i < count; ++i) {
         PyObject *m = PySequence_Fast_GET_ITEM(mats, i);
         if (PyTuple_Check(m) && PyTuple_GET_SIZE(m) == 3) {
-            for (int j = 0; j < 3; ++j) parts[i][j] = PyTuple_GET_ITEM(m, j);
+            for (int j = 0; j < 3; ++j) parts[i][j] = same(PyTuple_GET_ITEM(m, j));
         } else if (PyList_Check(m) && PyList_GET_SIZE(m) == 3) {
-            for (int j = 0; j < 3; ++j) parts[i][j] = PyList_GET_ITEM(m, j);
+            for (int j = 0; j < 3; ++j) parts[i][j] = same(PyList_GET_ITEM(m, j));
         } else {
             raise(PyExc_ValueError, "mats must hold (w, scales, biases) triples");
         }
@@ -239,15 +264,22 @@ PyObject *qmv_batched(Args a, Py_ssize_t n) {
     if (!xrows) throw PyErr{};
     Hold hold_x{xrows};
     if (one) {
-        if (a[4] == Py_None) whole = empty({1, total}, x.scalar_type(), x);
-        else whole = tensor(a[4], "out");
+        if (a[4] == Py_None) {
+            const Unlocked u;
+            whole = empty({1, total}, x.scalar_type(), x);
+        } else {
+            whole = tensor(a[4], "out");
+        }
     }
     int64_t col = 0;
     for (Py_ssize_t i = 0; i < count; ++i) {
         Dense d(parts[i][0], parts[i][1], parts[i][2], xrows, bits, group);
         void *dst = nullptr;
         if (!one) {
-            outs[i] = empty({rows.M, ns[i]}, x.scalar_type(), x);
+            {
+                const Unlocked u;
+                outs[i] = empty({rows.M, ns[i]}, x.scalar_type(), x);
+            }
             dst = outs[i].data_ptr();
         } else if (a[4] == Py_None) {
             dst = static_cast<char *>(whole.data_ptr()) + col * static_cast<int64_t>(x.element_size());     // tiles of one row, side by side
@@ -272,7 +304,7 @@ PyObject *qmv_batched(Args a, Py_ssize_t n) {
         col += ns[i];
     }
     const Call c(a[5], x);
-    c.check(mtc_qmv_batched(c.h, stream(), descs, static_cast<int>(count)));
+    c.check(unlocked([&] { return mtc_qmv_batched(c.h, stream(), descs, static_cast<int>(count)); }));
     if (one) return a[4] == Py_None ? wrap(std::move(whole)) : same(a[4]);
     PyObject *list = PyList_New(count);
     if (!list) throw PyErr{};
@@ -298,14 +330,17 @@ PyObject *qvm(Args a, Py_ssize_t n) {
     const int64_t N = w.size(1) * 32 / bits;
     if (w.size(0) != rows.K || s.dim() != 2 || s.size(0) != rows.K / group || s.size(1) != N || b.sizes() != s.sizes())
         raise(PyExc_ValueError, "w must be [K, N*bits/32] and scales / biases [K/group_size, N]");
-    at::Tensor made;
-    if (a[6] == Py_None) made = empty({rows.M, N}, x.scalar_type(), x);
-    else check_out(tensor(a[6], "out"), rows.M, N, x);
-    const at::Tensor &out = a[6] == Py_None ? made : THPVariable_Unpack(a[6]);
+    const bool given = a[6] != Py_None;
+    at::Tensor out = given ? tensor(a[6], "out") : at::Tensor();
+    if (given) check_out(out, rows.M, N, x);
     const Call c(a[7], x);
-    c.check(mtc_qvm(c.h, stream(), w.data_ptr(), s.data_ptr(), b.data_ptr(), x.data_ptr(), out.data_ptr(), static_cast<int>(rows.M),
-                    static_cast<int>(N), static_cast<int>(rows.K), static_cast<int>(bits), static_cast<int>(group), need_dtype(x)));
-    return a[6] == Py_None ? wrap(std::move(made)) : same(a[6]);
+    const int dt = need_dtype(x);
+    c.check(unlocked([&] {
+        if (!given) out = empty({rows.M, N}, x.scalar_type(), x);
+        return mtc_qvm(c.h, stream(), w.data_ptr(), s.data_ptr(), b.data_ptr(), x.data_ptr(), out.data_ptr(), static_cast<int>(rows.M),
+                       static_cast<int>(N), static_cast<int>(rows.K), static_cast<int>(bits), static_cast<int>(group), dt);
+    }));
+    return given ? same(a[6]) : wrap(std::move(out));
 }
 
 // rms_norm_qmv(w, scales, biases, x, norm_weight, eps, bits, group_size, out, ctx)
@@ -319,27 +354,32 @@ PyObject *rms_norm_qmv(Args a, Py_ssize_t n) {
     const int64_t K = x.numel(), N = w.size(0);
     if (nw.numel() != K || w.size(1) * 32 != K * bits)
         raise(PyExc_ValueError, "x and norm_weight must have K elements and w must be [N, K*bits/32]");
-    at::Tensor made;
-    if (a[8] == Py_None) made = empty({1, N}, x.scalar_type(), x);
-    else check_out(tensor(a[8], "out"), 1, N, x);
-    const at::Tensor &out = a[8] == Py_None ? made : THPVariable_Unpack(a[8]);
+    const bool given = a[8] != Py_None;
+    at::Tensor out = given ? tensor(a[8], "out") : at::Tensor();
+    if (given) check_out(out, 1, N, x);
     const Call c(a[9], x);
-    c.check(mtc_rms_norm_qmv(c.h, stream(), x.data_ptr(), nw.data_ptr(), static_cast<float>(eps), w.data_ptr(), s.data_ptr(), b.data_ptr(),
-                             out.data_ptr(), static_cast<int>(N), static_cast<int>(K), static_cast<int>(bits), static_cast<int>(group),
-                             need_dtype(x)));
-    return a[8] == Py_None ? wrap(std::move(made)) : same(a[8]);
+    const int dt = need_dtype(x);
+    c.check(unlocked([&] {
+        if (!given) out = empty({1, N}, x.scalar_type(), x);
+        return mtc_rms_norm_qmv(c.h, stream(), x.data_ptr(), nw.data_ptr(), static_cast<float>(eps), w.data_ptr(), s.data_ptr(), b.data_ptr(),
+                                out.data_ptr(), static_cast<int>(N), static_cast<int>(K), static_cast<int>(bits), static_cast<int>(group), dt);
+    }));
+    return given ? same(a[8]) : wrap(std::move(out));
 }
 
 // swiglu(gate, up, out, ctx)
 PyObject *swiglu(Args a, Py_ssize_t n) {
     nargs(n, 4);
     const at::Tensor &g = tensor(a[0], "gate"), &u = tensor(a[1], "up");
-    at::Tensor made;
-    if (a[2] == Py_None) made = g.is_contiguous() ? empty(g.sizes(), g.scalar_type(), g) : at::empty_like(g);
-    const at::Tensor &out = a[2] == Py_None ? made : tensor(a[2], "out");
+    const bool given = a[2] != Py_None;
+    at::Tensor out = given ? tensor(a[2], "out") : at::Tensor();
     const Call c(a[3], g);
-    c.check(mtc_swiglu(c.h, stream(), g.data_ptr(), u.data_ptr(), out.data_ptr(), static_cast<size_t>(g.numel()), need_dtype(g)));
-    return a[2] == Py_None ? wrap(std::move(made)) : same(a[2]);
+    const int dt = need_dtype(g);
+    c.check(unlocked([&] {
+        if (!given) out = g.is_contiguous() ? empty(g.sizes(), g.scalar_type(), g) : at::empty_like(g);
+        return mtc_swiglu(c.h, stream(), g.data_ptr(), u.data_ptr(), out.data_ptr(), static_cast<size_t>(g.numel()), dt);
+    }));
+    return given ? same(a[2]) : wrap(std::move(out));
 }
 
 // moe_router_topk(logits, k, norm_topk_prob, ctx) -> (indices, weights)
@@ -348,10 +388,15 @@ PyObject *moe_router_topk(Args a, Py_ssize_t n) {
     const at::Tensor &l = tensor(a[0], "logits");
     if (l.dim() != 2) raise(PyExc_ValueError, "logits must be [rows, n_experts]");
     const int64_t k = integer(a[1]), norm = integer(a[2]);
-    at::Tensor idx = empty({l.size(0), k}, at::kInt, l), wts = empty({l.size(0), k}, l.scalar_type(), l);
+    at::Tensor idx, wts;
     const Call c(a[3], l);
-    c.check(mtc_moe_router_topk(c.h, stream(), l.data_ptr(), idx.data_ptr(), wts.data_ptr(), static_cast<int>(l.size(0)),
-                                static_cast<int>(l.size(1)), static_cast<int>(k), static_cast<int>(norm), need_dtype(l)));
+    const int dt = need_dtype(l);
+    c.check(unlocked([&] {
+        idx = empty({l.size(0), k}, at::kInt, l);
+        wts = empty({l.size(0), k}, l.scalar_type(), l);
+        return mtc_moe_router_topk(c.h, stream(), l.data_ptr(), idx.data_ptr(), wts.data_ptr(), static_cast<int>(l.size(0)),
+                                   static_cast<int>(l.size(1)), static_cast<int>(k), static_cast<int>(norm), dt);
+    }));
     PyObject *i = wrap(std::move(idx)), *w = THPVariable_Wrap(std::move(wts));
     PyObject *t = w ? PyTuple_Pack(2, i, w) : nullptr;
     Py_DECREF(i);
@@ -366,10 +411,16 @@ PyObject *moe_sort(Args a, Py_ssize_t n) {
     const at::Tensor &idx = tensor(a[0], "topk_idx");
     if (idx.dim() != 2) raise(PyExc_ValueError, "topk_idx must be [n_tokens, k]");
     const int64_t T = idx.size(0), k = idx.size(1), E = integer(a[1]);
-    at::Tensor r[4] = {empty({T * k}, at::kInt, idx), empty({T, k}, at::kInt, idx), empty({E + 1}, at::kInt, idx), empty({T * k}, at::kInt, idx)};
+    at::Tensor r[4];
     const Call c(a[2], idx);
-    c.check(mtc_moe_sort(c.h, stream(), idx.data_ptr(), static_cast<int>(T), static_cast<int>(k), static_cast<int>(E), r[0].data_ptr(),
-                         r[1].data_ptr(), r[2].data_ptr(), r[3].data_ptr()));
+    c.check(unlocked([&] {
+        r[0] = empty({T * k}, at::kInt, idx);
+        r[1] = empty({T, k}, at::kInt, idx);
+        r[2] = empty({E + 1}, at::kInt, idx);
+        r[3] = empty({T * k}, at::kInt, idx);
+        return mtc_moe_sort(c.h, stream(), idx.data_ptr(), static_cast<int>(T), static_cast<int>(k), static_cast<int>(E), r[0].data_ptr(),
+                            r[1].data_ptr(), r[2].data_ptr(), r[3].data_ptr());
+    }));
     PyObject *t = PyTuple_New(4);
     if (!t) throw PyErr{};
     for (int i = 0; i < 4; ++i) {
@@ -388,13 +439,15 @@ PyObject *moe_permute(Args a, Py_ssize_t n) {
     nargs(n, 4);
     const at::Tensor &tok = tensor(a[0], "tokens"), &idx = tensor(a[1], "sort_token_idx");
     const int64_t rows = idx.numel(), hidden = tok.size(1);
-    at::Tensor made;
-    if (a[2] == Py_None) made = empty({rows, hidden}, tok.scalar_type(), tok);
-    const at::Tensor &out = a[2] == Py_None ? made : tensor(a[2], "out");
+    const bool given = a[2] != Py_None;
+    at::Tensor out = given ? tensor(a[2], "out") : at::Tensor();
     const Call c(a[3], tok);
-    c.check(mtc_moe_permute(c.h, stream(), tok.data_ptr(), idx.data_ptr(), out.data_ptr(), static_cast<int>(rows), static_cast<int>(hidden),
-                            need_dtype(tok)));
-    return a[2] == Py_None ? wrap(std::move(made)) : same(a[2]);
+    const int dt = need_dtype(tok);
+    c.check(unlocked([&] {
+        if (!given) out = empty({rows, hidden}, tok.scalar_type(), tok);
+        return mtc_moe_permute(c.h, stream(), tok.data_ptr(), idx.data_ptr(), out.data_ptr(), static_cast<int>(rows), static_cast<int>(hidden), dt);
+    }));
+    return given ? same(a[2]) : wrap(std::move(out));
 }
 
 // moe_unpermute(expert_outputs, inv_perm, weights, out, ctx)
@@ -403,13 +456,16 @@ PyObject *moe_unpermute(Args a, Py_ssize_t n) {
     const at::Tensor &eo = tensor(a[0], "expert_outputs"), &inv = tensor(a[1], "inv_perm"), &wts = tensor(a[2], "weights");
     if (inv.dim() != 2) raise(PyExc_ValueError, "inv_perm must be [n_tokens, k]");
     const int64_t T = inv.size(0), k = inv.size(1), hidden = eo.size(1);
-    at::Tensor made;
-    if (a[3] == Py_None) made = empty({T, hidden}, eo.scalar_type(), eo);
-    const at::Tensor &out = a[3] == Py_None ? made : tensor(a[3], "out");
+    const bool given = a[3] != Py_None;
+    at::Tensor out = given ? tensor(a[3], "out") : at::Tensor();
     const Call c(a[4], eo);
-    c.check(mtc_moe_unpermute(c.h, stream(), eo.data_ptr(), inv.data_ptr(), wts.data_ptr(), out.data_ptr(), static_cast<int>(T),
-                              static_cast<int>(hidden), static_cast<int>(k), need_dtype(eo)));
-    return a[3] == Py_None ? wrap(std::move(made)) : same(a[3]);
+    const int dt = need_dtype(eo);
+    c.check(unlocked([&] {
+        if (!given) out = empty({T, hidden}, eo.scalar_type(), eo);
+        return mtc_moe_unpermute(c.h, stream(), eo.data_ptr(), inv.data_ptr(), wts.data_ptr(), out.data_ptr(), static_cast<int>(T),
+                                 static_cast<int>(hidden), static_cast<int>(k), dt);
+    }));
+    return given ? same(a[3]) : wrap(std::move(out));
 }
 
 // gather_qmm(x, w, scales, biases, bits, group_size, expert_offsets, indices, out, ctx)
@@ -426,17 +482,20 @@ PyObject *gather_qmm(Args a, Py_ssize_t n) {
     if (s.dim() != 3 || s.size(0) != E || s.size(1) != N || s.size(2) != K / group || b.sizes() != s.sizes())
         raise(PyExc_ValueError, "scales/biases must be [E, n_out, k_in/group_size]");
     need_contiguous({&x, &w, &s, &b});
-    at::Tensor made;
-    if (a[8] == Py_None) made = empty({M, N}, x.scalar_type(), x);
-    else check_out(tensor(a[8], "out"), M, N, x);
-    const at::Tensor &out = a[8] == Py_None ? made : THPVariable_Unpack(a[8]);
+    const bool given = a[8] != Py_None;
+    at::Tensor out = given ? tensor(a[8], "out") : at::Tensor();
+    if (given) check_out(out, M, N, x);
     const void *off = a[6] == Py_None ? nullptr : tensor(a[6], "expert_offsets").data_ptr();
     const void *ids = a[7] == Py_None ? nullptr : tensor(a[7], "indices").data_ptr();
     const Call c(a[9], x);
-    c.check(mtc_gather_qmm(c.h, stream(), x.data_ptr(), w.data_ptr(), s.data_ptr(), b.data_ptr(), off, ids, out.data_ptr(),
-                           static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), static_cast<int>(E), static_cast<int>(bits),
-                           static_cast<int>(group), need_dtype(x)));
-    return a[8] == Py_None ? wrap(std::move(made)) : same(a[8]);
+    const int dt = need_dtype(x);
+    c.check(unlocked([&] {
+        if (!given) out = empty({M, N}, x.scalar_type(), x);
+        return mtc_gather_qmm(c.h, stream(), x.data_ptr(), w.data_ptr(), s.data_ptr(), b.data_ptr(), off, ids, out.data_ptr(),
+                              static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), static_cast<int>(E), static_cast<int>(bits),
+                              static_cast<int>(group), dt);
+    }));
+    return given ? same(a[8]) : wrap(std::move(out));
 }
 
 // (w, scales, biases) of one stacked expert matrix
@@ -468,15 +527,18 @@ PyObject *moe_experts(Args a, Py_ssize_t n) {
     if (x.size(1) != hidden || g.t[0]->size(2) * 32 != hidden * bits || d.t[0]->size(2) * 32 != inter * bits)
         raise(PyExc_ValueError, "gate / up must be [E, inter, hidden*bits/32] and down [E, hidden, inter*bits/32] for x [rows, hidden]");
     need_contiguous({&x, g.t[0], g.t[1], g.t[2], u.t[0], u.t[1], u.t[2], d.t[0], d.t[1], d.t[2]});
-    at::Tensor made;
-    if (a[8] == Py_None) made = empty({M, hidden}, x.scalar_type(), x);
-    else check_out(tensor(a[8], "out"), M, hidden, x);
-    const at::Tensor &out = a[8] == Py_None ? made : THPVariable_Unpack(a[8]);
+    const bool given = a[8] != Py_None;
+    at::Tensor out = given ? tensor(a[8], "out") : at::Tensor();
+    if (given) check_out(out, M, hidden, x);
     const Call c(a[9], x);
-    c.check(mtc_moe_experts(c.h, stream(), x.data_ptr(), order ? order->data_ptr() : nullptr, static_cast<int>(x.size(0)), &g.m, &u.m, &d.m,
-                            off.data_ptr(), out.data_ptr(), static_cast<int>(M), static_cast<int>(hidden), static_cast<int>(inter),
-                            static_cast<int>(E), static_cast<int>(bits), static_cast<int>(group), need_dtype(x)));
-    return a[8] == Py_None ? wrap(std::move(made)) : same(a[8]);
+    const int dt = need_dtype(x);
+    c.check(unlocked([&] {
+        if (!given) out = empty({M, hidden}, x.scalar_type(), x);
+        return mtc_moe_experts(c.h, stream(), x.data_ptr(), order ? order->data_ptr() : nullptr, static_cast<int>(x.size(0)), &g.m, &u.m, &d.m,
+                               off.data_ptr(), out.data_ptr(), static_cast<int>(M), static_cast<int>(hidden), static_cast<int>(inter),
+                               static_cast<int>(E), static_cast<int>(bits), static_cast<int>(group), dt);
+    }));
+    return given ? same(a[8]) : wrap(std::move(out));
 }
 
 // affine_quantize(w, bits, group_size, ctx) -> (packed, scales, biases)
@@ -490,15 +552,19 @@ PyObject *affine_quantize(Args a, Py_ssize_t n) {
     const int64_t K = w.size(-1);
     if (K % group || (group * bits) % 32)
         raise(PyExc_ValueError, "the last dimension must hold whole groups and group_size * bits must be a multiple of 32");
-    std::vector<int64_t> shape(w.sizes().begin(), w.sizes().end());
-    shape.back() = K * bits / 32;
-    at::Tensor r[3] = {empty(shape, at::kInt, w), {}, {}};
-    shape.back() = K / group;
-    r[1] = empty(shape, w.scalar_type(), w);
-    r[2] = empty(shape, w.scalar_type(), w);
+    at::Tensor r[3];
     const Call c(a[3], w);
-    c.check(mtc_affine_quantize(c.h, stream(), w.data_ptr(), r[0].data_ptr(), r[1].data_ptr(), r[2].data_ptr(), static_cast<size_t>(w.numel()),
-                                static_cast<int>(bits), static_cast<int>(group), need_dtype(w)));
+    const int dt = need_dtype(w);
+    c.check(unlocked([&] {
+        std::vector<int64_t> shape(w.sizes().begin(), w.sizes().end());
+        shape.back() = K * bits / 32;
+        r[0] = empty(shape, at::kInt, w);
+        shape.back() = K / group;
+        r[1] = empty(shape, w.scalar_type(), w);
+        r[2] = empty(shape, w.scalar_type(), w);
+        return mtc_affine_quantize(c.h, stream(), w.data_ptr(), r[0].data_ptr(), r[1].data_ptr(), r[2].data_ptr(), static_cast<size_t>(w.numel()),
+                                   static_cast<int>(bits), static_cast<int>(group), dt);
+    }));
     PyObject *t = PyTuple_New(3);
     if (!t) throw PyErr{};
     for (int i = 0; i < 3; ++i) {
@@ -522,10 +588,14 @@ PyObject *affine_dequantize(Args a, Py_ssize_t n) {
     if (w.dim() == 0) raise(PyExc_IndexError, "w must have at least one dimension");
     std::vector<int64_t> shape(w.sizes().begin(), w.sizes().end());
     shape.back() = w.size(-1) * 32 / bits;
-    at::Tensor out = empty(shape, s.scalar_type(), w);
+    at::Tensor out;
     const Call c(a[5], w);
-    c.check(mtc_affine_dequantize(c.h, stream(), w.data_ptr(), s.data_ptr(), b.data_ptr(), out.data_ptr(), static_cast<size_t>(out.numel()),
-                                  static_cast<int>(bits), static_cast<int>(group), need_dtype(s)));
+    const int dt = need_dtype(s);
+    c.check(unlocked([&] {
+        out = empty(shape, s.scalar_type(), w);
+        return mtc_affine_dequantize(c.h, stream(), w.data_ptr(), s.data_ptr(), b.data_ptr(), out.data_ptr(), static_cast<size_t>(out.numel()),
+                                     static_cast<int>(bits), static_cast<int>(group), dt);
+    }));
     return wrap(std::move(out));
 }
 
@@ -537,10 +607,14 @@ PyObject *dequant_gather(Args a, Py_ssize_t n) {
     need_contiguous({&w, &s, &b, &idx});
     if (bits == 0) raise(PyExc_ZeroDivisionError, "bits must be positive");
     const int64_t vocab = w.size(0), hidden = w.size(1) * 32 / bits, T = idx.numel();
-    at::Tensor out = empty({T, hidden}, s.scalar_type(), w);
+    at::Tensor out;
     const Call c(a[6], w);
-    c.check(mtc_dequant_gather(c.h, stream(), w.data_ptr(), s.data_ptr(), b.data_ptr(), idx.data_ptr(), out.data_ptr(), static_cast<size_t>(T),
-                               static_cast<int>(hidden), static_cast<int>(vocab), static_cast<int>(bits), static_cast<int>(group), need_dtype(s)));
+    const int dt = need_dtype(s);
+    c.check(unlocked([&] {
+        out = empty({T, hidden}, s.scalar_type(), w);
+        return mtc_dequant_gather(c.h, stream(), w.data_ptr(), s.data_ptr(), b.data_ptr(), idx.data_ptr(), out.data_ptr(), static_cast<size_t>(T),
+                                  static_cast<int>(hidden), static_cast<int>(vocab), static_cast<int>(bits), static_cast<int>(group), dt);
+    }));
     return wrap(std::move(out));
 }
 
@@ -549,9 +623,12 @@ PyObject *unpack_codes(Args a, Py_ssize_t n) {
     nargs(n, 4);
     const at::Tensor &w = tensor(a[0], "w");
     const int64_t K = integer(a[1]), bits = integer(a[2]), N = w.size(0);
-    at::Tensor codes = empty({N, K}, at::kByte, w);
+    at::Tensor codes;
     const Call c(a[3], w);
-    c.check(mtc_unpack_codes(c.h, stream(), w.data_ptr(), codes.data_ptr(), static_cast<int>(N), static_cast<int>(K), static_cast<int>(bits)));
+    c.check(unlocked([&] {
+        codes = empty({N, K}, at::kByte, w);
+        return mtc_unpack_codes(c.h, stream(), w.data_ptr(), codes.data_ptr(), static_cast<int>(N), static_cast<int>(K), static_cast<int>(bits));
+    }));
     return wrap(std::move(codes));
 }
 
@@ -619,11 +696,7 @@ PyObject *dispatch(Args a, Py_ssize_t n) {
     }
     const Call c(a[0]);
     float us = 0.0f;
-    int rc;
-    Py_BEGIN_ALLOW_THREADS
-    rc = mtc_dispatch(c.h, kernel, dt, st.bufs.data(), static_cast<int>(st.bufs.size()), dims[0], dims[1], &us);
-    Py_END_ALLOW_THREADS
-    c.check(rc);
+    c.check(unlocked([&] { return mtc_dispatch(c.h, kernel, dt, st.bufs.data(), static_cast<int>(st.bufs.size()), dims[0], dims[1], &us); }));
     PyObject *r = Py_BuildValue("(Od)", st.outs, static_cast<double>(us));
     if (!r) throw PyErr{};
     return r;
