@@ -1,8 +1,9 @@
 """Build ``libmtcuda.so`` in-tree with nvcc for sm_100a (``python -m metaltile_b200.build``).
 
 Every ``csrc/*.cu`` is compiled to an object file (in parallel) and linked into
-``metaltile_b200/libmtcuda.so``.  The library depends on the CUDA runtime only.  ``csrc/binding.cpp`` becomes
-``metaltile_b200/_native.so``, the Python binding of the typed ops over that library (it alone knows about torch).
+``metaltile_b200/libmtcuda.so``.  The library depends on the CUDA runtime only.  ``csrc/dispatch_binding.cpp`` becomes
+``metaltile_b200/_dispatch.so``, the Python binding of the name-keyed call on host buffers, and ``csrc/binding.cpp``
+``metaltile_b200/_native.so``, that of the typed ops on tensors: it alone needs PyTorch, and is left out where there is none.
 """
 from __future__ import annotations
 
@@ -18,6 +19,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libmtcuda.so")
+DISPATCH = os.path.join(HERE, "_dispatch.so")    # the Python binding of the name-keyed call (csrc/dispatch_binding.cpp)
 NATIVE = os.path.join(HERE, "_native.so")        # the Python binding of the typed ops (csrc/binding.cpp)
 
 NVCC_FLAGS = [
@@ -60,35 +62,50 @@ def _compile(nvcc, src, obj, log, headers):
     return obj
 
 
-def _compile_native(log):
-    """csrc/binding.cpp -> _native.so with the host compiler, against the installed PyTorch's headers and libmtcuda.so."""
+def _torch():
+    """PyTorch, or None where it is not installed."""
+    try:
+        import torch
+        return torch
+    except ImportError:
+        return None
+
+
+def _extension(source, out, log, extra_flags=(), extra_libs=()):
+    """A CPython extension over libmtcuda.so with the host compiler."""
     import sysconfig
 
-    from torch.utils import cpp_extension
-
-    import torch
     cxx = shutil.which("g++") or "c++"
-    libs = os.path.join(os.path.dirname(torch.__file__), "lib")
-    cmd = [cxx, "-O2", "-std=c++17", "-fPIC", "-shared",
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-I", sysconfig.get_paths()["include"]]
-    for inc in cpp_extension.include_paths("cuda"):
-        cmd += ["-isystem", inc]
-    cmd += [os.path.join(CSRC, "binding.cpp"), "-o", NATIVE, "-L", HERE, "-l:libmtcuda.so", "-Wl,-rpath,$ORIGIN", "-L", libs,
-            "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda"]
+    cmd = [cxx, "-O2", "-std=c++17", "-fPIC", "-shared", "-I", sysconfig.get_paths()["include"], *extra_flags, os.path.join(CSRC, source),
+           "-o", out, "-L", HERE, "-l:libmtcuda.so", "-Wl,-rpath,$ORIGIN", *extra_libs]
     r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     with open(log, "w") as f:
         f.write(" ".join(cmd) + "\n" + r.stdout)
     if r.returncode != 0:
-        raise RuntimeError(f"{cxx} failed on binding.cpp:\n{r.stdout[-6000:]}")
+        raise RuntimeError(f"{cxx} failed on {source}:\n{r.stdout[-6000:]}")
+
+
+def _compile_native(torch, log):
+    """csrc/binding.cpp -> _native.so against the installed PyTorch's headers."""
+    from torch.utils import cpp_extension
+
+    flags = [f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    for inc in cpp_extension.include_paths("cuda"):
+        flags += ["-isystem", inc]
+    libs = os.path.join(os.path.dirname(torch.__file__), "lib")
+    _extension("binding.cpp", NATIVE, log, flags,
+               ["-L", libs, "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda"])
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
     srcs = sorted(glob.glob(os.path.join(CSRC, "*.cu")))
     headers = glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(HERE, "..", "include", "*.h"))
-    deps = srcs + [os.path.join(CSRC, "binding.cpp")] + headers
+    deps = srcs + [os.path.join(CSRC, "binding.cpp"), os.path.join(CSRC, "dispatch_binding.cpp")] + headers
     stamp = os.path.join(OBJ, "stamp")
     digest = _digest(deps)
-    if not force and os.path.exists(LIB) and os.path.exists(NATIVE) and os.path.exists(stamp) and open(stamp).read() == digest:
+    torch = _torch()
+    outputs = [LIB, DISPATCH] + ([NATIVE] if torch else [])
+    if not force and all(map(os.path.exists, outputs)) and os.path.exists(stamp) and open(stamp).read() == digest:
         return LIB
     if force:
         shutil.rmtree(OBJ, ignore_errors=True)
@@ -109,7 +126,11 @@ def build(force: bool = False, verbose: bool = False) -> str:
     r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True, env=env)
     if r.returncode != 0:
         raise RuntimeError("link failed:\n" + r.stdout)
-    _compile_native(os.path.join(OBJ, "binding.log"))
+    _extension("dispatch_binding.cpp", DISPATCH, os.path.join(OBJ, "dispatch_binding.log"))
+    if torch:
+        _compile_native(torch, os.path.join(OBJ, "binding.log"))
+    else:
+        print("PyTorch is not installed: _native.so (the typed ops on tensors) is not built")
     with open(stamp, "w") as f:
         f.write(digest)
     if verbose:

@@ -60,18 +60,16 @@ def _dt(dtype) -> int:
                   .replace("float32", "f32")]
 
 
-_native = None
+_dispatch = None
 
 
 def _binding():
-    """The native binding (it needs torch in the process, which nothing else of this module does: loaded on first use)."""
-    global _native
-    if _native is None:
-        import torch  # noqa: F401
-
-        from . import _native as mod
-        _native = mod
-    return _native
+    """The native binding of the name-keyed call (csrc/dispatch_binding.cpp), loaded on first use."""
+    global _dispatch
+    if _dispatch is None:
+        from . import _dispatch as mod
+        _dispatch = mod
+    return _dispatch
 
 
 class Context:

@@ -124,7 +124,6 @@ struct Call {
         }
         load();
     }
-    explicit Call(PyObject *given) : obj(given) { load(); }
     void load() {
         PyObject *v = PyObject_GetAttr(obj, s_handle);
         if (!v) throw PyErr{};
@@ -632,76 +631,6 @@ PyObject *unpack_codes(Args a, Py_ssize_t n) {
     return wrap(std::move(codes));
 }
 
-// dispatch(ctx, kernel, dtype, items, outputs, grid, tpg) -> ({name: bytes}, elapsed_us): mtc_dispatch on host buffers.
-// Inputs are read where they are (buffer protocol); every output is a bytes object of its own that starts as a copy of the
-// caller's buffer and that the library writes before anybody else can see it.
-PyObject *dispatch(Args a, Py_ssize_t n) {
-    nargs(n, 7);
-    const char *kernel = PyUnicode_AsUTF8(a[1]);
-    if (!kernel) throw PyErr{};
-    const int dt = static_cast<int>(integer(a[2]));
-    if (!PyDict_Check(a[3])) raise(PyExc_TypeError, "items must be a dict");
-    struct State {
-        std::vector<mtc_named_buf> bufs;
-        std::vector<Py_buffer> views;
-        std::vector<PyObject *> held;
-        PyObject *outs = PyDict_New();
-        ~State() {
-            for (Py_buffer &v : views) PyBuffer_Release(&v);
-            for (PyObject *o : held) Py_DECREF(o);
-            Py_XDECREF(outs);
-        }
-    } st;
-    if (!st.outs) throw PyErr{};
-    const Py_ssize_t count = PyDict_Size(a[3]);
-    st.bufs.reserve(count);
-    st.views.reserve(count);
-    PyObject *key, *val;
-    Py_ssize_t pos = 0;
-    while (PyDict_Next(a[3], &pos, &key, &val)) {
-        mtc_named_buf b{};
-        b.name = PyUnicode_AsUTF8(key);
-        if (!b.name) throw PyErr{};
-        const int is_out = PySequence_Contains(a[4], key);
-        if (is_out < 0) throw PyErr{};
-        Py_buffer view;
-        if (!PyObject_CheckBuffer(val)) {
-            val = PyBytes_FromObject(val);
-            if (!val) throw PyErr{};
-            st.held.push_back(val);
-        }
-        if (PyObject_GetBuffer(val, &view, PyBUF_C_CONTIGUOUS) != 0) throw PyErr{};
-        st.views.push_back(view);
-        b.data = view.buf;
-        b.bytes = static_cast<size_t>(view.len);
-        b.is_output = is_out;
-        if (is_out) {
-            PyObject *o = PyBytes_FromStringAndSize(static_cast<const char *>(view.buf), view.len);
-            if (!o) throw PyErr{};
-            b.data = PyBytes_AS_STRING(o);
-            const int rc = PyDict_SetItem(st.outs, key, o);
-            Py_DECREF(o);
-            if (rc != 0) throw PyErr{};
-        }
-        st.bufs.push_back(b);
-    }
-    uint32_t dims[2][3];
-    for (int i = 0; i < 2; ++i) {
-        PyObject *seq = PySequence_Fast(a[5 + i], "grid_groups and threads_per_group are sequences");
-        if (!seq) throw PyErr{};
-        for (int j = 0; j < 3; ++j)
-            dims[i][j] = j < PySequence_Fast_GET_SIZE(seq) ? static_cast<uint32_t>(PyLong_AsUnsignedLongMask(PySequence_Fast_GET_ITEM(seq, j))) : 1u;
-        Py_DECREF(seq);
-        if (PyErr_Occurred()) throw PyErr{};
-    }
-    const Call c(a[0]);
-    float us = 0.0f;
-    c.check(unlocked([&] { return mtc_dispatch(c.h, kernel, dt, st.bufs.data(), static_cast<int>(st.bufs.size()), dims[0], dims[1], &us); }));
-    PyObject *r = Py_BuildValue("(Od)", st.outs, static_cast<double>(us));
-    if (!r) throw PyErr{};
-    return r;
-}
-
 // ---- module ----------------------------------------------------------------------------------------
 PyObject *set_context(PyObject *, PyObject *fn) {
     Py_INCREF(fn);
@@ -724,7 +653,7 @@ PyObject *entry(PyObject *, PyObject *const *args, Py_ssize_t n) {
 #define OP(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&entry<name>)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {
     OP(dense), OP(qmv_batched), OP(qvm), OP(rms_norm_qmv), OP(swiglu), OP(moe_router_topk), OP(moe_sort), OP(moe_permute), OP(moe_unpermute),
-    OP(gather_qmm), OP(moe_experts), OP(affine_quantize), OP(affine_dequantize), OP(dequant_gather), OP(unpack_codes), OP(dispatch),
+    OP(gather_qmm), OP(moe_experts), OP(affine_quantize), OP(affine_dequantize), OP(dequant_gather), OP(unpack_codes),
     {"set_context", set_context, METH_O, nullptr},
     {nullptr, nullptr, 0, nullptr},
 };
