@@ -85,11 +85,20 @@ def _extension(source, out, log, extra_flags=(), extra_libs=()):
         raise RuntimeError(f"{cxx} failed on {source}:\n{r.stdout[-6000:]}")
 
 
+def native_digest(torch=None) -> str:
+    """What _native.so is tied to: its sources, the library's interface, and the PyTorch and the Python whose headers it is
+    compiled against (another PyTorch has another ABI: an extension left from the one before must not pass for current)."""
+    torch = torch or _torch()
+    tied = [torch.__version__, str(torch.version.git_version), str(torch._C._GLIBCXX_USE_CXX11_ABI), sys.version]
+    sources = [os.path.join(CSRC, "binding.cpp"), *glob.glob(os.path.join(HERE, "..", "include", "*.h"))]
+    return _digest(sources) + hashlib.sha256("\0".join(tied).encode()).hexdigest()
+
+
 def _compile_native(torch, log):
     """csrc/binding.cpp -> _native.so against the installed PyTorch's headers."""
     from torch.utils import cpp_extension
 
-    flags = [f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    flags = [f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f'-DMTC_TORCH_VERSION="{torch.__version__}"']
     for inc in cpp_extension.include_paths("cuda"):
         flags += ["-isystem", inc]
     libs = os.path.join(os.path.dirname(torch.__file__), "lib")
@@ -97,15 +106,27 @@ def _compile_native(torch, log):
                ["-L", libs, "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda"])
 
 
+def _stamp(path, digest):
+    with open(path, "w") as f:
+        f.write(digest)
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
     srcs = sorted(glob.glob(os.path.join(CSRC, "*.cu")))
     headers = glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(HERE, "..", "include", "*.h"))
-    deps = srcs + [os.path.join(CSRC, "binding.cpp"), os.path.join(CSRC, "dispatch_binding.cpp")] + headers
-    stamp = os.path.join(OBJ, "stamp")
-    digest = _digest(deps)
+    deps = srcs + [os.path.join(CSRC, "dispatch_binding.cpp")] + headers
     torch = _torch()
-    outputs = [LIB, DISPATCH] + ([NATIVE] if torch else [])
-    if not force and all(map(os.path.exists, outputs)) and os.path.exists(stamp) and open(stamp).read() == digest:
+    # the C library and the binding that needs it alone; the extension over PyTorch has a stamp of its own
+    stamps = [(os.path.join(OBJ, "stamp"), _digest(deps) + sys.version, (LIB, DISPATCH))]
+    if torch:
+        stamps.append((os.path.join(OBJ, "native.stamp"), native_digest(torch), (NATIVE,)))
+    stale = [force or not all(map(os.path.exists, outs)) or not os.path.exists(path) or open(path).read() != digest
+             for path, digest, outs in stamps]
+    if not any(stale):
+        return LIB
+    if not stale[0]:                                     # only the extension over PyTorch
+        _compile_native(torch, os.path.join(OBJ, "binding.log"))
+        _stamp(*stamps[1][:2])
         return LIB
     if force:
         shutil.rmtree(OBJ, ignore_errors=True)
@@ -131,8 +152,8 @@ def build(force: bool = False, verbose: bool = False) -> str:
         _compile_native(torch, os.path.join(OBJ, "binding.log"))
     else:
         print("PyTorch is not installed: _native.so (the typed ops on tensors) is not built")
-    with open(stamp, "w") as f:
-        f.write(digest)
+    for path, digest, _ in stamps:
+        _stamp(path, digest)
     if verbose:
         print("built", LIB)
     return LIB

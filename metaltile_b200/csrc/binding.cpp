@@ -665,5 +665,7 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", "typed ops on torch tens
 PyMODINIT_FUNC PyInit__native() {
     s_handle = PyUnicode_InternFromString("_handle");
     s_check = PyUnicode_InternFromString("_check");
-    return s_handle && s_check ? PyModule_Create(&module) : nullptr;
+    PyObject *m = s_handle && s_check ? PyModule_Create(&module) : nullptr;
+    if (m && PyModule_AddStringConstant(m, "torch_version", MTC_TORCH_VERSION) != 0) Py_CLEAR(m);       // ops.py compares it with the PyTorch in the process
+    return m;
 }

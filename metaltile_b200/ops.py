@@ -19,6 +19,10 @@ except ImportError as e:
     raise ImportError(f"the native binding of the typed ops is missing ({e}): build it with `python -m metaltile_b200.build` "
                       "(there is no CPU or PyTorch fallback for these ops)") from e
 
+if _native.torch_version != torch.__version__:
+    raise ImportError(f"the native binding of the typed ops was compiled against PyTorch {_native.torch_version}, this is {torch.__version__}: "
+                      "build it again with `python -m metaltile_b200.build`")
+
 _TORCH_DT = {torch.float32: F32, torch.float16: F16, torch.bfloat16: BF16}
 
 _ctx_cache = {}

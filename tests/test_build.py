@@ -1,7 +1,12 @@
-"""What the build and the name-keyed call need: no PyTorch for the C library and for calls on host buffers."""
+"""What the build and the name-keyed call need: no PyTorch for the C library and for calls on host buffers, and an extension that is
+built again when the PyTorch it was compiled against is another one."""
 import os
 import subprocess
 import sys
+
+import pytest
+
+from metaltile_b200 import build
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 # a Python in which PyTorch is not installed
@@ -40,3 +45,28 @@ def test_the_c_library_is_built_without_torch(tmp_path):
                   "made = [cmd[cmd.index('-o') + 1] for cmd in ran]\n"
                   "assert made == [build.LIB, build.DISPATCH], made\n")
     assert "PyTorch is not installed" in out
+
+
+def test_another_pytorch_or_python_means_another_extension(monkeypatch, tmp_path):
+    import torch
+    if not os.path.exists(os.path.join(build.OBJ, "native.stamp")):
+        pytest.skip("the build's stamps do not travel with the built files")
+    made = []
+    monkeypatch.setattr(build, "_compile_native", lambda torch, log: made.append("native"))
+    monkeypatch.setattr(build, "_stamp", lambda path, digest: made.append(os.path.basename(path)))
+    monkeypatch.setattr(build, "_compile", lambda *a: pytest.fail("the C library does not depend on PyTorch"))
+    build.build()
+    assert made == []
+    monkeypatch.setattr(torch, "__version__", torch.__version__ + ".other")
+    build.build()
+    assert made == ["native", "native.stamp"]
+    monkeypatch.undo()
+    here = build.native_digest()
+    monkeypatch.setattr(sys, "version", "other " + sys.version)
+    assert build.native_digest() != here
+
+
+def test_an_extension_of_another_pytorch_is_refused():
+    r = subprocess.run([sys.executable, "-c", "import torch\ntorch.__version__ += '.other'\nimport metaltile_b200.ops"], cwd=ROOT,
+                       stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    assert r.returncode != 0 and "compiled against PyTorch" in r.stdout
