@@ -77,13 +77,15 @@ PyObject *dispatch(Args a, Py_ssize_t n) {
         if (!b.name) throw PyErr{};
         const int is_out = PySequence_Contains(a[4], key);
         if (is_out < 0) throw PyErr{};
+        // whatever bytes() takes: a contiguous buffer where it is, anything else (a strided array, a list) as a bytes object
         Py_buffer view;
-        if (!PyObject_CheckBuffer(val)) {
+        if (!PyObject_CheckBuffer(val) || PyObject_GetBuffer(val, &view, PyBUF_C_CONTIGUOUS) != 0) {
+            PyErr_Clear();
             val = PyBytes_FromObject(val);
             if (!val) throw PyErr{};
             st.held.push_back(val);
+            if (PyObject_GetBuffer(val, &view, PyBUF_SIMPLE) != 0) throw PyErr{};
         }
-        if (PyObject_GetBuffer(val, &view, PyBUF_C_CONTIGUOUS) != 0) throw PyErr{};
         st.views.push_back(view);
         b.data = view.buf;
         b.bytes = static_cast<size_t>(view.len);
@@ -102,8 +104,14 @@ PyObject *dispatch(Args a, Py_ssize_t n) {
     for (int i = 0; i < 2; ++i) {
         PyObject *seq = PySequence_Fast(a[5 + i], "grid_groups and threads_per_group are sequences");
         if (!seq) throw PyErr{};
-        for (int j = 0; j < 3; ++j)
-            dims[i][j] = j < PySequence_Fast_GET_SIZE(seq) ? static_cast<uint32_t>(PyLong_AsUnsignedLongMask(PySequence_Fast_GET_ITEM(seq, j))) : 1u;
+        // three sizes that int() takes (fewer: the others are 0; they are ignored)
+        const Py_ssize_t given = PySequence_Fast_GET_SIZE(seq);
+        if (given > 3) PyErr_SetString(PyExc_IndexError, "invalid index");
+        for (int j = 0; j < 3 && !PyErr_Occurred(); ++j) {
+            PyObject *v = j < given ? PyNumber_Long(PySequence_Fast_GET_ITEM(seq, j)) : nullptr;
+            dims[i][j] = v ? static_cast<uint32_t>(PyLong_AsUnsignedLongMask(v)) : 0u;
+            Py_XDECREF(v);
+        }
         Py_DECREF(seq);
         if (PyErr_Occurred()) throw PyErr{};
     }

@@ -1597,7 +1597,7 @@ int dispatch_pass(mtc_ctx *ctx, const char *kernel_name, int dtype, mtc_named_bu
     for (Staged &sb : st_bufs) {
         sb.dev = static_cast<char *>(ctx->d_scratch) + base_off + sb.offset;
         if (!cc && sb.need && sb.need <= kSmallUpload && sb.offset + sb.need <= kHostStageBytes) {
-            // h_stage mirrors the scratch block's offsets; the previous call's copies out of it ended with that call
+            // h_stage mirrors the scratch block's offsets; the previous call's copies out of it ended with that call, if it failed as well
             if (run_end == 0) run_begin = sb.offset;
             std::memcpy(ctx->h_stage + sb.offset, sb.buf->data, sb.need);
             run_end = sb.offset + sb.need;
@@ -1755,6 +1755,8 @@ int dispatch_pass(mtc_ctx *ctx, const char *kernel_name, int dtype, mtc_named_bu
             std::memcpy(&word, ctx->h_stage, sizeof(word));
             rc = status_error(ctx, "dispatch", word);
         }
+    } else {
+        cudaStreamSynchronize(st);              // the uploads out of the page-locked block (and out of the caller's buffers) end here
     }
     if (elapsed_us) {
         float ms = 0.f;

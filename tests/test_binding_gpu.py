@@ -4,9 +4,10 @@ import _thread
 import sys
 import threading
 
+import numpy as np
 import pytest
 
-from helpers import dense_case, to_dev
+from helpers import bytes_to_f32, dense_case, dt_bytes, to_dev
 
 pytestmark = pytest.mark.gpu
 
@@ -102,3 +103,49 @@ def test_threads_with_contexts_of_their_own():
     for t in threads:
         t.join()
     assert not wrong
+
+
+def _qmv_call(ctx, n, k, dt="f32", form=bytes, grid=(1, 1, 1), extra=0):
+    w, s, b, x = dense_case(1, n, k, 4, 64, dt, seed=3)
+    esz = 4 if dt == "f32" else 2
+    bufs = dict(w=form(w.tobytes()), scales=form(dt_bytes(s, dt)), biases=form(dt_bytes(b, dt)), x=form(dt_bytes(x, dt)), out=form(bytes(n * esz + extra)))
+    return ctx.dispatch_with_grid("mt_qmv_b4", bufs, dict(k=k, n=n, group_size=64), grid, (64, 1, 1), dtype=dt)
+
+
+def _strided(raw):
+    a = np.zeros((len(raw), 2), dtype=np.uint8)
+    a[:, 0] = np.frombuffer(raw, dtype=np.uint8)
+    return a[:, 0]
+
+
+def test_forms_of_host_buffers_and_sizes():
+    """Whatever bytes() takes: bytes, bytearray, memoryview, an array, a strided array, a list; sizes that int() takes, three at most."""
+    from metaltile_b200 import ops
+    ctx = ops.context(0)
+    want = _qmv_call(ctx, 64, 512).outputs["out"]
+    for form in (bytearray, memoryview, lambda r: np.frombuffer(r, dtype=np.uint8), _strided, list):
+        assert _qmv_call(ctx, 64, 512, form=form).outputs["out"] == want
+    for grid in ((8.0, 1.0, 1.0), (np.int64(8), 1, True), (8,)):
+        assert _qmv_call(ctx, 64, 512, grid=grid).outputs["out"] == want
+    with pytest.raises(IndexError):
+        _qmv_call(ctx, 64, 512, grid=(8, 1, 1, 1))
+    with pytest.raises(TypeError):
+        _qmv_call(ctx, 64, 512, form=lambda r: "text")
+
+
+@pytest.mark.parametrize("k", [4096, 16384, 65536])
+def test_staging_at_its_limits(k):
+    """Inputs below, at and above the size up to which they travel together (64 KiB), outputs below and past the block they come back
+    through (1 MiB), outputs with bytes behind the result, and a call after one that failed with its uploads under way."""
+    from metaltile_b200 import MetalTileError, ops
+    ctx = ops.context(0)
+    for n in {4096: (8, 32, 4096, 300000), 16384: (8, 9, 64), 65536: (2, 3, 16)}[k]:
+        got = _qmv_call(ctx, n, k, extra=12)
+        assert len(got.outputs["out"]) == n * 4 + 12 and got.outputs["out"][-12:] == bytes(12)
+        w, s, b, x = dense_case(1, n, k, 4, 64, "f32", seed=3)
+        dev = ops.qmv(to_dev(w), to_dev(s, "f32"), to_dev(b, "f32"), to_dev(x, "f32"), 4, 64, ctx=ctx).cpu().numpy().reshape(-1)
+        assert np.array_equal(bytes_to_f32(got.outputs["out"][:n * 4], "f32"), dev)
+        with pytest.raises(MetalTileError):              # k > 32 experts a token: refused by the entry, after the uploads
+            ctx.dispatch_with_grid("mt_moe_router_topk", dict(router_logits=bytes(4 * 64 * 64), indices_out=bytes(64 * 160), weights_out=bytes(64 * 160)),
+                                   dict(n_experts=64, k=40), (1, 1, 1), (32, 1, 1), dtype="f32", outputs=("indices_out", "weights_out"))
+        assert _qmv_call(ctx, n, k, extra=12).outputs["out"] == got.outputs["out"]
