@@ -772,7 +772,7 @@ def extra_measurements(ctx, dev, hbm_peak, tf_peak, local_rank=0, layers=None):
         w, sc, bi = sets[0]
         us, clk = with_clocks(lambda: time_calls(lambda: ops.qmm(w, sc, bi, x, BITS, GROUP, out=o, ctx=ctx)))
         tf = 2.0 * m * n * k / us / 1e6
-        out[name] = {"us": us, "TFLOP/s": tf, "frac_of_bf16_peak": tf / tf_peak, "route": ctx.qmm_route(m, n, k, BITS, GROUP, "bf16"),
+        out[name] = {"us": us, "TFLOP/s": tf, "frac_of_bf16_peak": tf / tf_peak, "route": ctx.qmm_kernel(m, n, k, BITS, GROUP, "bf16"),
                      "clocks": clk}
         del sets
 
@@ -837,9 +837,8 @@ def extra_measurements(ctx, dev, hbm_peak, tf_peak, local_rank=0, layers=None):
         us, clk = with_clocks(lambda: time_rot([step8], 10))
         nbytes = step_bytes(m8, len(layers))
         out["c2_decode_set_m8"] = {"ms": us / 1e3, "GB/s": nbytes / us / 1e3, "frac_of_hbm_peak": nbytes / us / 1e3 / hbm_peak,
-                                   "launches": len(groups) if ctx.qmm_route(m8, 4096, 4096, BITS, GROUP, "bf16") == "qmv_stream"
-                                   else sum(len(g) for g in groups),
-                                   "route": ctx.qmm_route(m8, 4096, 4096, BITS, GROUP, "bf16"), "clocks": clk}
+                                   # every small-M kernel that takes these shapes takes the projections of a group in one launch
+                                   "launches": len(groups), "kernel": ctx.qmm_kernel(m8, 4096, 4096, BITS, GROUP, "bf16"), "clocks": clk}
     return out
 
 

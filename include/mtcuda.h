@@ -96,11 +96,14 @@ int mtc_qmv(mtc_ctx *ctx, void *stream, const void *w, const void *scales, const
  * Ragged M needs no padding (the reference pads to 32: quantized_mma_dynamic_m.rs:46-112). */
 int mtc_qmm(mtc_ctx *ctx, void *stream, const void *w, const void *scales, const void *biases,
             const void *x, void *out, int M, int N, int K, int bits, int group_size, int dtype);
-/* Name of the kernel family mtc_qmm's selector names for these arguments with aligned pointers and default options
- * ("qmv_stream", "qmv_cuda_core", "qmv_mma_sync", "qmm_tcgen05"; option "qmv_frag" lets the fragment kernel stand in for the
- * first three and, below 32 Mi codes, for the last at M <= 16); the analogue of asserting on
- * mt_qmm_for's routing (quantized.rs:5127-5199). */
+/* mtc_qmm_route: the kernel family of the selector without the fragment kernel, the analogue of asserting on mt_qmm_for's
+ * routing (quantized.rs:5127-5199): "qmv_stream", "qmv_cuda_core", "qmv_mma_sync" or "qmm_tcgen05" - what runs with option
+ * "qmv_frag" at 0 and the others at their defaults.
+ * mtc_qmm_kernel: the kernel that mtc_qmm launches for these arguments with aligned pointers under the options of `ctx` (NULL: the
+ * default options): one of those names, "qmv_frag" or "qmv_tcgen05_decode" (option "qmv_tc"); "" for arguments no kernel takes.
+ * The entry itself decides by the same function.  (M in 17..32 that runs as 16-row chunks: the kernel of a whole chunk.) */
 const char *mtc_qmm_route(int M, int N, int K, int bits, int group_size, int dtype);
+const char *mtc_qmm_kernel(const mtc_ctx *ctx, int M, int N, int K, int bits, int group_size, int dtype);
 
 /* ---- fused and chained decode projections ----
  * mtc_qmv_desc: one projection, the arguments of mtc_qmv plus up to 8 destinations of the [M, N] result (each gets

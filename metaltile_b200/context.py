@@ -333,7 +333,12 @@ class Context:
         self._check(self._lib.mtc_qmm(self._h, stream, w, scales, biases, x, out, M, N, K, bits, group_size,
                                       _dt(dtype)))
 
+    def qmm_kernel(self, M, N, K, bits, group_size, dtype) -> str:
+        """The kernel that ``qmm`` launches under this context's options (aligned pointers)."""
+        return self._lib.mtc_qmm_kernel(self._h, M, N, K, bits, group_size, _dt(dtype)).decode()
+
     def qmm_route(self, M, N, K, bits, group_size, dtype) -> str:
+        """The kernel family of the selector without the fragment kernel (option ``qmv_frag`` at 0)."""
         return self._lib.mtc_qmm_route(M, N, K, bits, group_size, _dt(dtype)).decode()
 
     def gather_qmm(self, x, w, scales, biases, out, m_total, n_out, k_in, n_experts, bits, group_size, dtype,

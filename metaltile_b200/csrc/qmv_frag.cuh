@@ -730,6 +730,8 @@ cudaError_t launch_one(cudaStream_t st, FragArgs a, int sms) {
     constexpr size_t kSmemMax = 226 * 1024, kSmemTwo = 112 * 1024;
     constexpr size_t kFrags = static_cast<size_t>(kCap<MODE>) * NT * 4 * kPitch<XT>, kSums = NT * (MODE == G8 ? 2 : 1) * 4 * (MODE == S1 ? 4 : 8);
     constexpr size_t step_bytes = kFrags + kSums;
+    // one run of activations for each of eight warps fits whatever the shape: there is always a plan
+    static_assert(RUN * step_bytes <= (kSmemMax - 8 * kCap<MODE> * NT * 64) / 8 / 128 * 128, "a run of activations fits a warp's part");
     const int total_runs = (a.steps + RUN - 1) / RUN;
     // Split of a CTA's eight warps: KS of them share a tile.  Cost of a split = tile rounds x (runs of a slice + the sum over
     // the warps, worth about half a run), plus the activations a warp stages: once when they fit, else with every tile.
@@ -779,7 +781,7 @@ cudaError_t launch_one(cudaStream_t st, FragArgs a, int sms) {
             }
         }
     }
-    if (best_grid == 0) return cudaErrorNotSupported;
+    if (best_grid == 0) return cudaErrorInvalidConfiguration;
     auto kern = qmv_frag_kernel<BITS, XT, MODE, NT, VEC>;
     static PerDeviceAttr attr;
     cudaError_t e = attr.set(kern, kSmemMax);
@@ -822,12 +824,14 @@ cudaError_t launch_type(cudaStream_t st, const FragArgs &a, const Shape &s, int 
         return launch_one<BITS, XT, S2, 4, 0>(st, a, sms);
     }
     if (s.mode == S4 && s.nt == 1) return launch_one<BITS, XT, S4, 1, 0>(st, a, sms);
+    // f32 activations: eight token rows a launch at most (rows_per_launch)
+    constexpr bool kMany = XT != MTC_F32;
     if constexpr (BITS == 4 || BITS == 8) {
-        if (s.nt == 1) return launch_one<BITS, XT, G8, 1, 0>(st, a, sms);
-        return launch_one<BITS, XT, G8, 2, 0>(st, a, sms);
+        if (!kMany || s.nt == 1) return launch_one<BITS, XT, G8, 1, 0>(st, a, sms);
+        if constexpr (kMany) return launch_one<BITS, XT, G8, 2, 0>(st, a, sms);
     } else {
-        if (s.nt == 2) return launch_one<BITS, XT, S4, 2, 0>(st, a, sms);
-        return launch_one<BITS, XT, S4, 4, 0>(st, a, sms);
+        if (!kMany || s.nt == 2) return launch_one<BITS, XT, S4, 2, 0>(st, a, sms);
+        if constexpr (kMany) return launch_one<BITS, XT, S4, 4, 0>(st, a, sms);
     }
 }
 

@@ -480,16 +480,38 @@ static bool small_m_tc_rule(int mode, int M, int N, int K) {
     return false;
 }
 
-static bool small_m_tc_preferred(mtc_ctx *ctx, int M, int N, int K, int bits, int group_size, int dtype, const void *w, const void *x,
+static bool small_m_tc_preferred(const Ctx *ctx, int M, int N, int K, int bits, int group_size, int dtype, const void *w, const void *x,
                                  const void *out) {
     return small_m_tc_rule(ctx->qmv_small_m_tc, M, N, K) && mtc::qmm_tcgen05_supported(M, N, K, bits, group_size, dtype, w, x, out);
+}
+
+// The kernel a product runs on: what mtc_qmv and mtc_qmm launch and what mtc_qmm_kernel names, so that the two cannot differ.
+enum ProductKernel { K_DECODE_TC, K_FRAG, K_STREAM, K_MMA, K_TCGEN05, K_CUDA };
+static const char *const kProductKernelNames[] = {"qmv_tcgen05_decode", "qmv_frag", "qmv_stream", "qmv_mma_sync", "qmm_tcgen05", "qmv_cuda_core"};
+
+static bool decode_tc_takes(const Ctx *ctx, int M, int N, int K, int bits, int group_size, int dtype, const void *w, const void *scales,
+                            const void *biases, const void *x) {
+    return ctx->qmv_tc && M >= 1 && N >= 1 && mtc::qmv_tc_supported(M, N, K, bits, group_size, dtype, w, scales, biases, x) &&
+           mtc::qmv_tc_counter_bytes(N) <= kTcCounterBytes;
+}
+
+static ProductKernel qmv_kernel_for(const Ctx *ctx, int M, int N, int K, int bits, int group_size, int dtype, const void *w, const void *scales,
+                                    const void *biases, const void *x, const void *out) {
+    if (decode_tc_takes(ctx, M, N, K, bits, group_size, dtype, w, scales, biases, x)) return K_DECODE_TC;
+    if (frag_takes(ctx, M, N, false, N, K, bits, group_size, dtype, w, scales, biases, x)) return K_FRAG;
+    if (stream_takes_single(ctx, M, N, K) && mtc::qmv_stream_supported(M, N, K, bits, group_size, dtype, w, scales, biases, x)) return K_STREAM;
+    if (ctx->qmv_small_m_mma && (M >= 2 || (M == 1 && ctx->qmv_small_m_mma == 2)) && mtc::qmv_mma_supported(M < 2 ? 2 : M, N, K, bits, group_size, dtype, w, x))
+        return K_MMA;
+    // a few token rows on a width or group the warp-level kernels do not take: one FFMA per (code, token) on CUDA cores against
+    // the tensor-memory kernel with K cut into slices
+    if (small_m_tc_preferred(ctx, M, N, K, bits, group_size, dtype, w, x, out)) return K_TCGEN05;
+    return K_CUDA;
 }
 
 // The tcgen05 decode kernel, when it takes the shape: 0 = launched, 1 = not its shape, < 0 = error.
 static int try_qmv_tc(mtc_ctx *ctx, void *stream, const void *w, const void *scales, const void *biases, const void *x,
                       void *const *outs, int n_outs, int M, int N, int K, int bits, int group_size, int dtype) {
-    if (!ctx->qmv_tc || M < 1 || N < 1 || !mtc::qmv_tc_supported(M, N, K, bits, group_size, dtype, w, scales, biases, x)) return 1;
-    if (mtc::qmv_tc_counter_bytes(N) > kTcCounterBytes) return 1;
+    if (!decode_tc_takes(ctx, M, N, K, bits, group_size, dtype, w, scales, biases, x)) return 1;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     int rc = ensure_tc_scratch(ctx, mtc::qmv_tc_scratch_bytes(M, N, K), st);
     if (rc != MTC_OK) return rc;
@@ -506,46 +528,35 @@ int mtc_qmv(mtc_ctx *ctx, void *stream, const void *w, const void *scales, const
     if (!dtype_ok(dtype)) return fail(ctx, MTC_ERR_UNSUPPORTED, "qmv: dtype must be f32, f16 or bf16");
     if (M > 0 && N > 0 && (!w || !scales || !biases || !x || !out)) return fail(ctx, MTC_ERR_INVALID, "qmv: null pointer");
     std::string why;
-    {
-        void *outs1[1] = {out};
-        const int t = try_qmv_tc(ctx, stream, w, scales, biases, x, outs1, 1, M, N, K, bits, group_size, dtype);
-        if (t <= 0) return t;
-    }
-    if (frag_takes(ctx, M, N, false, N, K, bits, group_size, dtype, w, scales, biases, x)) {
-        mtc_qmv_desc d{};
-        d.w = w; d.scales = scales; d.biases = biases; d.x = x;
-        d.outs[0] = out; d.n_outs = 1;
-        d.M = M; d.N = N; d.K = K; d.bits = bits; d.group_size = group_size; d.dtype = dtype;
-        cudaError_t e0 = mtc::launch_qmv_frag(ctx, static_cast<cudaStream_t>(stream), &d, 1);
-        if (e0 == cudaSuccess) return MTC_OK;
-        if (e0 != cudaErrorNotSupported) return fail(ctx, MTC_ERR_DISPATCH, std::string("qmv (fragments) launch: ") + cudaGetErrorString(e0));
-    }
-    if (stream_takes_single(ctx, M, N, K) && mtc::qmv_stream_supported(M, N, K, bits, group_size, dtype, w, scales, biases, x)) {
-        mtc_qmv_desc d{};
-        d.w = w; d.scales = scales; d.biases = biases; d.x = x;
-        d.outs[0] = out; d.n_outs = 1;
-        d.M = M; d.N = N; d.K = K; d.bits = bits; d.group_size = group_size; d.dtype = dtype;
-        cudaError_t e1 = mtc::launch_qmv_stream(ctx, static_cast<cudaStream_t>(stream), &d, 1);
-        if (e1 != cudaSuccess) return fail(ctx, MTC_ERR_DISPATCH, std::string("qmv (stream) launch: ") + cudaGetErrorString(e1));
-        return MTC_OK;
-    }
-    if (ctx->qmv_small_m_mma && (M >= 2 || ctx->qmv_small_m_mma == 2) &&
-        mtc::qmv_mma_supported(M < 2 ? 2 : M, N, K, bits, group_size, dtype, w, x)) {
-        cudaError_t e2 = mtc::launch_qmv_mma(ctx, static_cast<cudaStream_t>(stream), w, scales, biases, x, out, M, N, K,
-                                             group_size, dtype);
-        if (e2 != cudaSuccess) return fail(ctx, MTC_ERR_DISPATCH, std::string("qmv (mma) launch: ") + cudaGetErrorString(e2));
-        return MTC_OK;
-    }
-    if (small_m_tc_preferred(ctx, M, N, K, bits, group_size, dtype, w, x, out)) {
-        // a few token rows on a width or group the warp-level kernels do not take: one FFMA per (code, token) on CUDA
-        // cores against the tensor-memory kernel with K cut into slices
-        cudaError_t e3 = mtc::launch_qmm_tcgen05(ctx, static_cast<cudaStream_t>(stream), w, scales, biases, x, out, M, N, K, bits,
-                                                 group_size, dtype, &why);
-        if (e3 == cudaSuccess) return MTC_OK;
-        // a scratch block would have to grow during stream capture: the CUDA-core kernel needs none
-        if (e3 != cudaErrorStreamCaptureUnsupported)
-            return fail(ctx, MTC_ERR_DISPATCH, "qmv (tcgen05 qmm) launch: " + (why.empty() ? std::string(cudaGetErrorString(e3)) : why));
-        why.clear();
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    mtc_qmv_desc d{};
+    d.w = w; d.scales = scales; d.biases = biases; d.x = x;
+    d.outs[0] = out; d.n_outs = 1;
+    d.M = M; d.N = N; d.K = K; d.bits = bits; d.group_size = group_size; d.dtype = dtype;
+    cudaError_t ek = cudaSuccess;
+    switch (qmv_kernel_for(ctx, M, N, K, bits, group_size, dtype, w, scales, biases, x, out)) {
+        case K_DECODE_TC: return try_qmv_tc(ctx, stream, w, scales, biases, x, d.outs, 1, M, N, K, bits, group_size, dtype);
+        case K_FRAG:
+            ek = mtc::launch_qmv_frag(ctx, st, &d, 1);
+            if (ek != cudaSuccess) return fail(ctx, MTC_ERR_DISPATCH, std::string("qmv (fragments) launch: ") + cudaGetErrorString(ek));
+            return MTC_OK;
+        case K_STREAM:
+            ek = mtc::launch_qmv_stream(ctx, st, &d, 1);
+            if (ek != cudaSuccess) return fail(ctx, MTC_ERR_DISPATCH, std::string("qmv (stream) launch: ") + cudaGetErrorString(ek));
+            return MTC_OK;
+        case K_MMA:
+            ek = mtc::launch_qmv_mma(ctx, st, w, scales, biases, x, out, M, N, K, group_size, dtype);
+            if (ek != cudaSuccess) return fail(ctx, MTC_ERR_DISPATCH, std::string("qmv (mma) launch: ") + cudaGetErrorString(ek));
+            return MTC_OK;
+        case K_TCGEN05:
+            ek = mtc::launch_qmm_tcgen05(ctx, st, w, scales, biases, x, out, M, N, K, bits, group_size, dtype, &why);
+            if (ek == cudaSuccess) return MTC_OK;
+            // a scratch block would have to grow during stream capture: the CUDA-core kernel needs none
+            if (ek != cudaErrorStreamCaptureUnsupported)
+                return fail(ctx, MTC_ERR_DISPATCH, "qmv (tcgen05 qmm) launch: " + (why.empty() ? std::string(cudaGetErrorString(ek)) : why));
+            why.clear();
+            break;
+        case K_CUDA: break;
     }
     cudaError_t e = mtc::launch_qmv(ctx, static_cast<cudaStream_t>(stream), w, scales, biases, x, out, M, N, K, bits,
                                     group_size, dtype, &why);
@@ -618,8 +629,8 @@ int mtc_qmv_batched(mtc_ctx *ctx, void *stream, const mtc_qmv_desc *descs, int n
     }
     if (frag) {
         cudaError_t e = mtc::launch_qmv_frag(ctx, static_cast<cudaStream_t>(stream), descs, n);
-        if (e == cudaSuccess) return MTC_OK;
-        if (e != cudaErrorNotSupported) return fail(ctx, MTC_ERR_DISPATCH, std::string("qmv_batched (fragments) launch: ") + cudaGetErrorString(e));
+        if (e != cudaSuccess) return fail(ctx, MTC_ERR_DISPATCH, std::string("qmv_batched (fragments) launch: ") + cudaGetErrorString(e));
+        return MTC_OK;
     }
     if (fused) {
         cudaError_t e = mtc::launch_qmv_stream(ctx, static_cast<cudaStream_t>(stream), descs, n);
@@ -794,13 +805,32 @@ const char *mtc_qmm_route(int M, int N, int K, int bits, int group_size, int dty
     return "qmv_cuda_core";
 }
 
+// Whether mtc_qmm runs the shape as 16-row chunks of mtc_qmv
+static bool qmm_in_chunks(const Ctx *ctx, int M, int N, int K, int bits, int group_size, int dtype, const void *w, const void *x) {
+    return mma_chunks_preferred(ctx->qmm_mma_chunks && ctx->qmv_small_m_mma, ctx->qmm_ksplit, ctx->sm_count, M, N, K, bits, group_size, dtype, w, x);
+}
+
+const char *mtc_qmm_kernel(const mtc_ctx *ctx, int M, int N, int K, int bits, int group_size, int dtype) {
+    if (M < 1 || N < 1 || K < 1 || group_size < 1 || !dtype_ok(dtype)) return "";
+    Ctx defaults;
+    defaults.sm_count = mtc::kNumSMsB200;
+    const Ctx *c = ctx ? static_cast<const Ctx *>(ctx) : &defaults;
+    ProductKernel k;
+    if (qmm_in_chunks(c, M, N, K, bits, group_size, dtype, nullptr, nullptr))
+        k = qmv_kernel_for(c, 16, N, K, bits, group_size, dtype, nullptr, nullptr, nullptr, nullptr, nullptr);
+    else if (M > 16 && mtc::qmm_tcgen05_supported(M, N, K, bits, group_size, dtype, nullptr, nullptr, nullptr))
+        k = K_TCGEN05;
+    else
+        k = qmv_kernel_for(c, M, N, K, bits, group_size, dtype, nullptr, nullptr, nullptr, nullptr, nullptr);
+    return kProductKernelNames[k];
+}
+
 int mtc_qmm(mtc_ctx *ctx, void *stream, const void *w, const void *scales, const void *biases, const void *x,
             void *out, int M, int N, int K, int bits, int group_size, int dtype) {
     if (!ctx) return MTC_ERR_INVALID;
     MTC_ENTER(ctx);
     if (!dtype_ok(dtype)) return fail(ctx, MTC_ERR_UNSUPPORTED, "qmm: dtype must be f32, f16 or bf16");
-    if (w && scales && biases && x && out &&
-        mma_chunks_preferred(ctx->qmm_mma_chunks && ctx->qmv_small_m_mma, ctx->qmm_ksplit, ctx->sm_count, M, N, K, bits, group_size, dtype, w, x)) {
+    if (w && scales && biases && x && out && qmm_in_chunks(ctx, M, N, K, bits, group_size, dtype, w, x)) {
         const size_t esz = 2;      // f16 / bf16 only on this path
         for (int m0 = 0; m0 < M; m0 += 16) {
             const int mc = M - m0 < 16 ? M - m0 : 16;

@@ -318,6 +318,16 @@ def test_small_m_default_route_is_within_tolerance(ctx):
     torch.cuda.synchronize()
     ref = oracle.qmm(w, s, b, x, m, n, k, 8, 64, rows=(512, 576))[:, 512:576]
     assert rel_err(got.float().cpu().numpy()[:, 512:576], ref) <= TOL["bf16"] and ctx.status_word() == 0
+    # the same through the tensor-memory kernel, which the route names: the fragment kernel stands in for it on a matrix this small
+    assert ctx.qmm_kernel(m, n, k, 8, 64, "bf16") == "qmv_frag"
+    ctx.set_option("qmv_frag", 0)
+    try:
+        assert ctx.qmm_kernel(m, n, k, 8, 64, "bf16") == "qmm_tcgen05"
+        got = ops.qmv(to_dev(w), to_dev(s, "bf16"), to_dev(b, "bf16"), to_dev(x, "bf16"), 8, 64, ctx=ctx)
+    finally:
+        ctx.set_option("qmv_frag", 1)
+    torch.cuda.synchronize()
+    assert rel_err(got.float().cpu().numpy()[:, 512:576], ref) <= TOL["bf16"] and ctx.status_word() == 0
 
 
 def test_k_slices_replay_from_a_cuda_graph(ctx):
@@ -344,14 +354,17 @@ def test_k_slices_replay_from_a_cuda_graph(ctx):
     assert ctx.status_word() == 0
 
 
-def test_small_m_capture_without_a_first_run_falls_back_to_cuda_cores():
+@pytest.mark.parametrize("frag", [1, 0])        # 0: the tensor-memory route, whose scratch block the capture meets
+def test_small_m_capture_without_a_first_run_falls_back_to_cuda_cores(frag):
     """M = 16, 8-bit captured on a fresh context: the tensor-memory route would have to grow a scratch block during
     capture, so mtc_qmv takes the CUDA-core kernel for that call instead of failing; the replay matches the oracle."""
     import torch
     from metaltile_b200 import Context
     from metaltile_b200.ops import _TORCH_DT
     fresh = Context(0)
+    fresh.set_option("qmv_frag", frag)
     m, n, k, bits, gs, dt = 16, 1024, 2048, 8, 64, "bf16"
+    assert fresh.qmm_kernel(m, n, k, bits, gs, dt) == ("qmv_frag" if frag else "qmm_tcgen05")
     w, s, b, x = dense_case(m, n, k, bits, gs, dt, seed=13)
     wd, sd, bd, xd = to_dev(w), to_dev(s, dt), to_dev(b, dt), to_dev(x, dt)
     out = torch.zeros((m, n), dtype=torch.bfloat16, device="cuda")

@@ -370,8 +370,8 @@ def test_rms_norm_qmv_typed(ctx, n, k, gs, dt):
     assert rel_err(got.float().cpu().numpy(), ref) <= TOL[dt]
 
 
-@pytest.mark.parametrize("m", [2, 5, 16])
-def test_small_m_tensor_core_path_special_activations(ctx, m):
+@pytest.mark.parametrize("m,frag", [(2, 0), (2, 1), (5, 1), (16, 1)])      # 2 tokens: the ring kernel where the fragment kernel is off
+def test_small_m_tensor_core_path_special_activations(ctx, m, frag):
     """The ring kernel stages bf16 activations times 2^64 (and x / 16 for the nibbles at bits 4-7): zeros of both signs,
     bf16 subnormals, tiny and large magnitudes must come through exactly."""
     import torch
@@ -385,7 +385,12 @@ def test_small_m_tensor_core_path_special_activations(ctx, m):
     x[:, 5::11] = oracle.round_through(np.random.default_rng(15).standard_normal(x[:, 5::11].shape).astype(np.float32), oracle.BF16)
     ref = oracle.qmm(w, s, b, x, m, n, k, 4, 64)
     xd = torch.from_numpy((np.ascontiguousarray(x).view(np.uint32) >> 16).astype(np.int16)).cuda().view(torch.bfloat16)
-    got = ops.qmv(to_dev(w), to_dev(s, "bf16"), to_dev(b, "bf16"), xd, 4, 64, ctx=ctx)
+    ctx.set_option("qmv_frag", frag)
+    try:
+        assert ctx.qmm_kernel(m, n, k, 4, 64, "bf16") == ("qmv_frag" if m == 2 and frag else "qmv_mma_sync")
+        got = ops.qmv(to_dev(w), to_dev(s, "bf16"), to_dev(b, "bf16"), xd, 4, 64, ctx=ctx)
+    finally:
+        ctx.set_option("qmv_frag", 1)
     torch.cuda.synchronize()
     got = got.float().cpu().numpy()
     assert ctx.status_word() == 0 and np.all(np.isfinite(got))
