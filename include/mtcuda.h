@@ -114,7 +114,8 @@ const char *mtc_qmm_kernel(const mtc_ctx *ctx, int M, int N, int K, int bits, in
  * (crates/metaltile-std/src/ffai/batched_qkv_qgemv.rs:1-35: q, k, v in one dispatch, one concatenated result) and
  * ffai_batched_4_qgemv (crates/metaltile-std/src/ffai/batched_4_qgemv.rs:1-45).  The streaming kernel (M = 1), the ring
  * kernel (2 <= M <= 16) and the fragment kernel take several projections in one launch; what none of them takes runs as
- * separate mtc_qmv launches.
+ * separate mtc_qmv launches.  How K is split over the warps follows from the rows of the whole launch, so a fused projection may
+ * differ from mtc_qmv of it alone by the order of its f32 sums (the last bit of an output); the same call always gives the same bits.
  *
  * mtc_chain_*: a prepared list of projections walked by ONE persistent grid, the counterpart of
  * Context::dispatch_chain (crates/metaltile-runtime/src/context.rs:363-395: several passes, one commit, ordering

@@ -69,7 +69,7 @@ def _check_out(out, M, N, like):
 
 
 def qmv(w, scales, biases, x, bits: int, group_size: int, out=None, ctx: Context = None):
-    """out[M, N] = x[M, K] @ dequant(w)[N, K]^T on the CUDA-core path (decode, M <= 16 tuned)."""
+    """out[M, N] = x[M, K] @ dequant(w)[N, K]^T (decode, M <= 16 tuned); ``Context.qmm_kernel`` names the kernel."""
     return _native.dense(0, w, scales, biases, x, bits, group_size, out, ctx)
 
 
@@ -92,7 +92,9 @@ def qmv_batched(mats, x, bits: int, group_size: int, out=None, ctx: Context = No
 
     Returns ``out[M, sum(N_i)]`` with the results side by side - for M = 1 the concatenated vector of
     ``ffai_batched_qkv_qgemv`` (crates/metaltile-std/src/ffai/batched_qkv_qgemv.rs:1-35).  For M > 1 every
-    projection writes its own contiguous [M, N_i] tile and the tiles are returned as a list instead."""
+    projection writes its own contiguous [M, N_i] tile and the tiles are returned as a list instead.  The f32 sums of a fused
+    projection may be added in another order than ``qmv`` of it alone adds them (the last bit of an output may differ); the
+    same call always gives the same bits."""
     return _native.qmv_batched(mats, x, bits, group_size, out, ctx)
 
 

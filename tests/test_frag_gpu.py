@@ -60,8 +60,9 @@ def test_rounds_and_blocks(ctx, m, n, k, bits, gs, dt):
 
 @pytest.mark.parametrize("m,k,bits,gs", [(1, 1024, 4, 64), (3, 1024, 4, 64), (8, 1024, 4, 128), (16, 512, 4, 64), (4, 1088, 4, 64), (5, 640, 8, 32)])
 def test_projections_in_one_launch_equal_separate_ones(ctx, m, k, bits, gs):
-    """Rows that end inside a tile in the middle of the launch: every projection has its own tiles, so the results are the
-    separate launches' bit for bit on one kernel (M = 2 to 16 on the ring kernel, else the fragment kernel)."""
+    """Rows that end inside a tile in the middle of the launch: every projection has its own tiles.  With so few tiles the launch
+    splits K over its warps as each of the separate ones does, so the results are theirs bit for bit (M = 5 to 16 with 4-bit
+    codes on the ring kernel, else the fragment kernel); with more tiles the splits may differ, see the next test."""
     import torch
     from metaltile_b200 import ops
     mats = []
@@ -76,6 +77,37 @@ def test_projections_in_one_launch_equal_separate_ones(ctx, m, k, bits, gs):
     for g, t in zip(got, mats):
         assert rel_err(g.float().cpu().numpy().reshape(m, -1), t[3]) <= BOUND["bf16"]
         assert torch.equal(g.reshape(m, -1), ops.qmv(*t[:3], xd, bits, gs, ctx=ctx).reshape(m, -1))
+
+
+@pytest.mark.parametrize("m,k,bits,gs,dt", [(1, 4096, 4, 64, "bf16"), (8, 4096, 4, 64, "f16"), (16, 2048, 4, 128, "bf16"), (4, 2048, 8, 64, "f16")])
+def test_projections_in_one_launch_at_size(ctx, m, k, bits, gs, dt):
+    """Launches whose tiles fill the device, where the fused launch may split K otherwise than the separate ones: every product is
+    right, the call repeats itself bit for bit, and it differs from the separate launches by single roundings of the output."""
+    import torch
+    from metaltile_b200 import ops
+    ns, mats = (4096, 1024, 1040), []
+    for i, n in enumerate(ns):
+        w, s, b, _ = dense_case(m, n, k, bits, gs, dt, seed=22, salt=i)
+        mats.append((to_dev(w), to_dev(s, dt), to_dev(b, dt), w, s, b))
+    x = dense_case(m, 16, k, bits, gs, dt, seed=22)[3]
+    xd = to_dev(x, dt)
+    got, again = (ops.qmv_batched([t[:3] for t in mats], xd, bits, gs, ctx=ctx) for _ in range(2))
+    if m == 1:
+        got, again = torch.split(got, list(ns), dim=1), torch.split(again, list(ns), dim=1)
+    for n, t, g, a in zip(ns, mats, got, again):
+        assert torch.equal(g, a)
+        alone = ops.qmv(*t[:3], xd, bits, gs, ctx=ctx)
+        ref = oracle.qmm(t[3], t[4], t[5], x, m, n, k, bits, gs, rows=(0, 64))[:, :64]
+        assert rel_err(g[:, :64].float().cpu().numpy(), ref) <= BOUND[dt]
+        assert rel_err(g.float().cpu().numpy(), alone.float().cpu().numpy()) <= 2 * BOUND[dt]
+
+
+@pytest.mark.parametrize("m,gs,dt", [(1, 64, "bf16"), (1, 32, "f32"), (2, 64, "f16"), (4, 32, "bf16"), (7, 32, "f16"), (7, 64, "bf16")])
+@pytest.mark.parametrize("k", [8320, 8576, 14464])
+def test_long_lanes_past_a_staged_block(ctx, m, gs, dt, k):
+    """3-bit rows that start on 16 bytes (K a multiple of 128, so that lanes take consecutive chunks), a last run of K that is not full,
+    and - at several tokens - activations that are staged block by block."""
+    _check(ctx, m, 50, k, 3, gs, dt)
 
 
 @pytest.mark.parametrize("bits,gs,dt,m", [(4, 64, "bf16", 1), (4, 32, "f16", 4), (8, 64, "f32", 5), (8, 64, "bf16", 7), (2, 64, "f16", 2)])

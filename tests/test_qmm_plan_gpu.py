@@ -117,3 +117,34 @@ def test_slices_stay_within_their_bound(ctx):
         del got
     torch.cuda.empty_cache()
     assert free0 - torch.cuda.mem_get_info()[0] < 3 * (512 << 20) * 1.5 + (64 << 20)
+
+
+@pytest.mark.parametrize("m,n,k,bits,gs,dt,ld,shift", [
+    (70, 576, 2880, 8, 32, "f16", 600, 0), (300, 1024, 4096, 4, 64, "bf16", 4096, 8), (33, 130, 2048, 4, 64, "bf16", 131, 1),
+    (700, 192, 5120, 3, 64, "f16", 1000, 3)])
+def test_slices_with_several_destinations(ctx, m, n, k, bits, gs, dt, ld, shift):
+    """A product cut into K slices whose result is a column block of three wider matrices (rows and blocks that start anywhere): every
+    copy equals the plain product bit for bit, and nothing beside the block is written."""
+    import torch
+    from metaltile_b200 import ops
+    from metaltile_b200.ops import _TORCH_DT
+    w, s, b, x = dense_case(m, n, k, bits, gs, dt, seed=35)
+    wd, sd, bd, xd = to_dev(w), to_dev(s, dt), to_dev(b, dt), to_dev(x, dt)
+    ctx.set_option("qmm_mma_chunks", 0)                   # 33 rows: the tensor-core kernel, as for several destinations
+    try:
+        want = ops.qmm(wd, sd, bd, xd, bits, gs, ctx=ctx)
+    finally:
+        ctx.set_option("qmm_mma_chunks", 1)
+    rows = np.r_[0:4, m - 4:m]
+    ref = oracle.qmm(w, s, b, np.ascontiguousarray(x[rows]), len(rows), n, k, bits, gs)
+    assert rel_err(want.float().cpu().numpy()[rows], ref) <= TOL[dt]
+    outs = [torch.full((m * ld + 16,), 7.0, dtype=xd.dtype, device="cuda") for _ in range(3)]
+    ctx.qmm_multi(wd.data_ptr(), sd.data_ptr(), bd.data_ptr(), xd.data_ptr(), [o[shift:].data_ptr() for o in outs], ld, m, n, k, bits, gs,
+                  _TORCH_DT[xd.dtype], stream=torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert ctx.status_word() == 0
+    for o in outs:
+        block = o[shift:shift + m * ld].view(m, ld)
+        assert torch.equal(block[:, :n], want)
+        block[:, :n] = 7.0
+        assert bool((o == 7.0).all())
