@@ -82,9 +82,9 @@ int mtc_status_clear(mtc_ctx *ctx);
  * dequant_gemv_int2 family: out[m,n] = sum_k (q*scale + bias) * x[m,k], f32
  * accumulate (crates/metaltile-std/src/mlx/quantized.rs:7-308,343-1441,4273-4392;
  * crates/metaltile-std/src/ffai/dequant_gemv.rs:52-105).  Any M (tuned for M <= 16), bits in
- * {2,3,4,5,6,8}, K*bits % 32 == 0, group_size | K.  M = 1 and every general case run on CUDA cores;
- * 2 <= M <= 16 with 4-bit codes, f16/bf16 activations, K % 64 == 0 and a power-of-two group >= 64 use
- * warp-level tensor-core MMAs on the integer codes (f32 accumulate, affine part applied per group). */
+ * {2,3,4,5,6,8}, K*bits % 32 == 0, group_size | K.  M <= 16 runs on warp-level tensor-core MMAs on the integer codes
+ * (f32 accumulate, affine part applied per group) where a kernel for them takes the shape and is the faster one,
+ * else on CUDA cores, as does every general case; mtc_qmm_kernel names the choice. */
 int mtc_qmv(mtc_ctx *ctx, void *stream, const void *w, const void *scales, const void *biases,
             const void *x, void *out, int M, int N, int K, int bits, int group_size, int dtype);
 
@@ -261,14 +261,18 @@ int mtc_peer_barrier(mtc_ctx *ctx, void *stream, void *const *peer_flags, int n_
  *                      tensor-core kernel (f16 / bf16, K % 64 == 0, power-of-two group >= 32) instead of one FFMA per
  *                      (code, token) on CUDA cores; 0 never; 2 whenever that kernel takes the shape
  *   "qmv_stream"       the streaming decode kernel (4-bit, f16 / bf16, K % 512 == 0, group 64 or 128, 16-byte aligned
- *                      pointers): 1 (default) takes M = 1 where "qmv_frag" leaves it (0 there) - a single projection
- *                      from 8 Mi codes on, fused projections at any size; 2 takes every M <= 8 at any size
+ *                      pointers): 1 (default) takes M = 1 where the fragment kernel does not - which with "qmv_frag" at
+ *                      its default is no shape of this kernel below 4 GB of codes; with "qmv_frag" 0 a single projection
+ *                      from 8 Mi codes on and fused projections at any size.  mtc_qmv_multi, mtc_qmv_batched_sync and the
+ *                      chains run on it whatever "qmv_frag" says.  2 takes every M <= 8 at any size
  *                      (slower than the register-ring kernel at M >= 2); 0 never.  mtc_qmv_batched fuses its projections into one launch where this kernel,
  *                      the fragment kernel or the ring kernel takes them and launches them one by one otherwise
  *   "qmv_frag"         the fragment kernel (warp-level tensor cores, every width, weights straight from global memory): 1
- *                      (default) where it is faster than the other small-M kernels (widths other than 4-bit from M = 2 on, f32
- *                      activations from M = 5 on, 4-bit up to M = 4 and where the ring kernel does not go, M = 1 except
- *                      5-bit codes and large single 2 / 3 / 6-bit matrices) unless
+ *                      (default) where it is faster than the other small-M kernels: M = 1 except 5-bit codes and single 2 / 3 /
+ *                      6-bit matrices of more than 64 Mi codes; 4-bit codes on the ring kernel's shapes up to M = 4 (groups of 64
+ *                      and 128); everything else up to M = 4, up to M = 8 while K <= 8192 or below 32 Mi codes, and from
+ *                      M = 9 on groups that are multiples of 64 with K <= 5120 up to 20 Mi codes (fused: 128 Mi); f32
+ *                      activations from M = 5 on - unless
  *                      "qmv_stream", "qmv_small_m_mma" or "qmv_small_m_tc" selects another kernel; 2 whenever it supports
  *                      the shape (M <= 16, K % 32 == 0, power-of-two group >= 32, 16-byte aligned w and x); 0 never
  *   "qmv_tc"           1: those shapes run on the tensor-memory decode kernel instead (slower today; default 0)

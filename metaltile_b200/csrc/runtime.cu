@@ -169,10 +169,9 @@ bool read_const(mtc_named_buf *bufs, int n, const char *name, uint32_t *out) {
 
 constexpr size_t kTcCounterBytes = 1u << 20;       // (tile, quarter) counters of the tcgen05 decode kernel: N up to 8 Mi rows
 
-// Partial-sum planes of the tcgen05 decode kernel.  Grow-only; an outgrown block is kept until mtc_destroy, so a CUDA
-// graph captured earlier never reads freed memory.  Growing allocates: not during stream capture.
 // Option "qmv_stream": 1 (default) = the streaming decode kernel takes M = 1 where the fragment kernel (frag_rule below) does
-// not; 2 = every M <= 8 it supports (at 2 <= M <= 8 the register-ring kernel of qmv_mma.cu is faster: measured
+// not - with that kernel at its default, matrices of 4 GB of codes and more only; it is what option "qmv_frag" 0 falls back to, and
+// what mtc_qmv_multi, mtc_qmv_batched_sync and the chains run on; 2 = every M <= 8 it supports (at 2 <= M <= 8 the register-ring kernel of qmv_mma.cu is faster: measured
 // 13.3 against 21.7 us on 14336 x 4096 at M = 8); 0 = never.
 inline bool stream_takes(const Ctx *ctx, int M) { return ctx->qmv_stream == 2 ? M <= 8 : (ctx->qmv_stream == 1 && M == 1); }
 // A single projection on its own launch: below 8 Mi codes the CUDA-core kernel is the faster one (measured at M = 1:
@@ -215,6 +214,8 @@ inline bool frag_takes(const Ctx *ctx, int M, long long rows, bool fused, int N,
     return (ctx->qmv_frag == 2 || by_rule) && mtc::qmv_frag_supported(M, N, K, bits, group_size, dt, w, scales, biases, x);
 }
 
+// Partial-sum planes of the tcgen05 decode kernel.  Grow-only; an outgrown block is kept until mtc_destroy, so a CUDA
+// graph captured earlier never reads freed memory.  Growing allocates: not during stream capture.
 int ensure_tc_scratch(Ctx *ctx, size_t bytes, cudaStream_t st) {
     if (bytes <= ctx->tc_scratch_bytes) return MTC_OK;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
