@@ -6,6 +6,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -14,6 +16,15 @@
 namespace mtc {
 
 constexpr int kNumSMsB200 = 148;
+
+// Streams with weights that were just written.  Locked: two threads may quantize and multiply on streams of their own.
+struct FreshWeights {
+    static constexpr int kMost = 64;
+    std::mutex lock;
+    std::atomic<int> n{0};
+    std::atomic<bool> anywhere{false};     // more streams than the list holds: no product starts on its weights early any more
+    cudaStream_t streams[kMost] = {};
+};
 
 struct Ctx {
     int device = 0;
@@ -41,8 +52,7 @@ struct Ctx {
     std::vector<void *> retired;   // outgrown scratch blocks: freed by mtc_destroy, so that captured graphs never see freed memory
     int qmv_frag = 1;              // option "qmv_frag": 0 = never use the fragment kernel (qmv_frag.cuh), 2 = whenever it supports the shape
     int qmv_stream = 1;            // option "qmv_stream": 0 = never use the streaming decode kernel (qmv_stream.cu)
-    std::vector<cudaStream_t> fresh_weights;   // streams on which mtc_affine_quantize ran since their last product (early_weights below)
-    bool fresh_anywhere = false;   // more streams than that list holds: no product starts on its weights early any more
+    FreshWeights fresh;            // streams on which mtc_affine_quantize ran since their last product (early_weights below)
     int pdl_early_weights = 1;     // option "pdl_early_weights": 0 = no load of w / scales / biases before the previous kernel of the stream is complete
     void *d_worklist = nullptr;    // gather_qmm work list (grow-only, owned by the context)
     size_t worklist_bytes = 0;
@@ -95,20 +105,33 @@ inline cudaError_t grow_block(Ctx *ctx, cudaStream_t st, void **block, size_t *h
 // before it signals its dependents.
 inline void weights_written(Ctx *ctx, cudaStream_t st) {
     if (st == cudaStreamLegacy) st = nullptr;
-    for (cudaStream_t s : ctx->fresh_weights)
-        if (s == st) return;
-    if (ctx->fresh_weights.size() < 64) ctx->fresh_weights.push_back(st);
-    else ctx->fresh_anywhere = true;
+    FreshWeights &f = ctx->fresh;
+    const std::lock_guard<std::mutex> hold(f.lock);
+    const int n = f.n.load(std::memory_order_relaxed);
+    for (int i = 0; i < n; ++i)
+        if (f.streams[i] == st) return;
+    if (n < FreshWeights::kMost) {
+        f.streams[n] = st;
+        f.n.store(n + 1, std::memory_order_release);
+    } else {
+        f.anywhere.store(true);
+    }
 }
 // called once per product launch: may it start on its weights before the previous kernel of the stream is complete?
 inline int early_weights(Ctx *ctx, cudaStream_t st) {
-    if (st == cudaStreamLegacy) st = nullptr;
-    for (size_t i = 0; i < ctx->fresh_weights.size(); ++i)
-        if (ctx->fresh_weights[i] == st) {
-            ctx->fresh_weights.erase(ctx->fresh_weights.begin() + static_cast<std::ptrdiff_t>(i));
-            return 0;
-        }
-    return ctx->pdl_early_weights && !ctx->fresh_anywhere ? 1 : 0;
+    FreshWeights &f = ctx->fresh;
+    if (f.n.load(std::memory_order_acquire) != 0) {
+        if (st == cudaStreamLegacy) st = nullptr;
+        const std::lock_guard<std::mutex> hold(f.lock);
+        const int n = f.n.load(std::memory_order_relaxed);
+        for (int i = 0; i < n; ++i)
+            if (f.streams[i] == st) {
+                f.streams[i] = f.streams[n - 1];
+                f.n.store(n - 1, std::memory_order_release);
+                return 0;
+            }
+    }
+    return ctx->pdl_early_weights && !f.anywhere.load(std::memory_order_relaxed) ? 1 : 0;
 }
 
 inline int fail(Ctx *ctx, int code, const std::string &msg) {

@@ -105,6 +105,36 @@ def test_threads_with_contexts_of_their_own():
     assert not wrong
 
 
+def test_threads_that_quantize_and_multiply():
+    """Two threads on streams of their own and one Context: weights are packed and used at once in both (no shared scratch block)."""
+    import torch
+    from metaltile_b200 import ops
+    ctx = ops.context(0)
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    ws = [torch.randn(512, 1024, device="cuda", generator=gen).to(torch.bfloat16) for _ in range(8)]
+    x = torch.randn(4, 1024, device="cuda", generator=gen).to(torch.bfloat16)
+    want = []
+    for w in ws:
+        want.append(ops.qmv(*ops.affine_quantize(w, 8, 64, ctx=ctx), x, 8, 64, ctx=ctx))
+        torch.cuda.synchronize()
+    wrong = []
+
+    def work(seed):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for i in range(400):
+                k = (i * 3 + seed) % len(ws)
+                got = ops.qmv(*ops.affine_quantize(ws[k], 8, 64, ctx=ctx), x, 8, 64, ctx=ctx)
+                if not torch.equal(got, want[k]):
+                    wrong.append((seed, i))
+
+    threads = [threading.Thread(target=work, args=(t,)) for t in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
+
+
 def _qmv_call(ctx, n, k, dt="f32", form=bytes, grid=(1, 1, 1), extra=0):
     w, s, b, x = dense_case(1, n, k, 4, 64, dt, seed=3)
     esz = 4 if dt == "f32" else 2
