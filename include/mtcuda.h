@@ -112,7 +112,7 @@ const char *mtc_qmm_kernel(const mtc_ctx *ctx, int M, int N, int K, int bits, in
  * mtc_qmv_batched: 1 to 4 projections that read the SAME activations (same x, M, K, dtype) in one launch, each
  * writing its own output.  With the outputs laid out one after the other this is ffai_batched_qkv_qgemv(_fast)
  * (crates/metaltile-std/src/ffai/batched_qkv_qgemv.rs:1-35: q, k, v in one dispatch, one concatenated result) and
- * ffai_batched_4_qgemv (crates/metaltile-std/src/ffai/batched_4_qgemv.rs:1-45).  The streaming kernel (M = 1), the ring
+ * ffai_batched_4_qgemv (crates/metaltile-std/src/ffai/batched_4_qgemv.rs:1-45).  The streaming kernel (M = 1), the cluster
  * kernel (2 <= M <= 16) and the fragment kernel take several projections in one launch; what none of them takes runs as
  * separate mtc_qmv launches.  How K is split over the warps follows from the rows of the whole launch, so a fused projection may
  * differ from mtc_qmv of it alone by the order of its f32 sums (the last bit of an output); the same call always gives the same bits.
@@ -265,15 +265,16 @@ int mtc_peer_barrier(mtc_ctx *ctx, void *stream, void *const *peer_flags, int n_
  *                      its default is no shape of this kernel below 4 GB of codes; with "qmv_frag" 0 a single projection
  *                      from 8 Mi codes on and fused projections at any size.  mtc_qmv_multi, mtc_qmv_batched_sync and the
  *                      chains run on it whatever "qmv_frag" says.  2 takes every M <= 8 at any size
- *                      (slower than the register-ring kernel at M >= 2); 0 never.  mtc_qmv_batched fuses its projections into one launch where this kernel,
- *                      the fragment kernel or the ring kernel takes them and launches them one by one otherwise
+ *                      (slower than the cluster kernel at M >= 2); 0 never.  mtc_qmv_batched fuses its projections into one launch where this kernel,
+ *                      the fragment kernel or the cluster kernel takes them and launches them one by one otherwise
  *   "qmv_frag"         the fragment kernel (warp-level tensor cores, every width, weights straight from global memory): 1
  *                      (default) where it is faster than the other small-M kernels: M = 1 except 5-bit codes and single 2 / 3 /
- *                      6-bit matrices of more than 64 Mi codes; 4-bit codes on the ring kernel's shapes up to M = 4 (groups of 64
+ *                      6-bit matrices of more than 64 Mi codes; 4-bit codes with K % 512 == 0 up to M = 4 (groups of 64
  *                      and 128); everything else up to M = 4, up to M = 8 while K <= 8192 or below 32 Mi codes, and from
  *                      M = 9 on groups that are multiples of 64 with K <= 5120 up to 20 Mi codes (fused: 128 Mi); f32
  *                      activations from M = 5 on - unless
- *                      "qmv_stream", "qmv_small_m_mma" or "qmv_small_m_tc" selects another kernel; 2 whenever it supports
+ *                      "qmv_stream", "qmv_small_m_mma" or "qmv_small_m_tc" selects another kernel; from M = 5 on 4-bit codes, f32 activations and large 8-bit matrices run as
+ *                      clusters that split K (csrc/qmv_cluster.cuh) in its place; 2 itself whenever it supports
  *                      the shape (M <= 16, K % 32 == 0, power-of-two group >= 32, 16-byte aligned w and x); 0 never
  *   "qmv_tc"           1: those shapes run on the tensor-memory decode kernel instead (slower today; default 0)
  *   "gather_stream"    0: grouped products never take the weight-streaming kernel (default 1: the CSR form with

@@ -171,8 +171,8 @@ constexpr size_t kTcCounterBytes = 1u << 20;       // (tile, quarter) counters o
 
 // Option "qmv_stream": 1 (default) = the streaming decode kernel takes M = 1 where the fragment kernel (frag_rule below) does
 // not - with that kernel at its default, matrices of 4 GB of codes and more only; it is what option "qmv_frag" 0 falls back to, and
-// what mtc_qmv_multi, mtc_qmv_batched_sync and the chains run on; 2 = every M <= 8 it supports (at 2 <= M <= 8 the register-ring kernel of qmv_mma.cu is faster: measured
-// 13.3 against 21.7 us on 14336 x 4096 at M = 8); 0 = never.
+// what mtc_qmv_multi, mtc_qmv_batched_sync and the chains run on; 2 = every M <= 8 it supports (at 2 <= M <= 8 it is the slower one: 21.7 us on
+// 14336 x 4096 at M = 8, where the cluster kernel takes 9); 0 = never.
 inline bool stream_takes(const Ctx *ctx, int M) { return ctx->qmv_stream == 2 ? M <= 8 : (ctx->qmv_stream == 1 && M == 1); }
 // A single projection on its own launch: below 8 Mi codes the CUDA-core kernel is the faster one (measured at M = 1:
 // 1024 x 4096 3.4 against 3.9 us, 2048 x 2048 2.8 against 3.8, 4096 x 4096 5.5 = 5.4, 14336 x 4096 12.5 against 10.7).
@@ -191,11 +191,11 @@ inline bool stream_takes_single(const Ctx *ctx, int M, int N, int K) {
 //     kernel takes matrices of 32 Mi codes on.
 //   M >= 9: the tcgen05 kernel's time does not grow with M; this one keeps the small matrices (8-bit 4096 x 4096 14.4 -> 10.6) and,
 //     as one launch instead of three a projection, fused ones whose activations fit an SM (8-bit, 6 layers 823 -> 690).
-//   f32 activations: three pieces per value, so the FFMA kernel wins below M = 5 (M = 4: 14.0 against 16.8), not above (M = 16
-//     39.3 -> 25).
-//   4-bit, 2 <= M: up to M = 4 (4096 x 4096 / 28672 x 4096 / 4096 x 14336, ring kernel of qmv_mma.cu -> here, M = 2 5.0 / 20.0 /
-//     12.2 -> 4.0 / 14.5 / 10.2, M = 4 5.4 / 20.4 / 14.2 -> 5.0 / 16.2 / 12.3, M = 5 5.9 / 21.3 / 16.6 -> 6.0 / 27.9 / 20.4), and where the ring
-//     kernel does not go (K % 512 != 0 or group 32; 2880 x 2880 M = 4 7.7 -> 5.0).
+//   f32 activations: three pieces per value, so the FFMA kernel wins below M = 5 (M = 4: 14.0 against 16.8), not above.
+//   4-bit, 2 <= M: up to M = 4 (4096 x 4096 / 28672 x 4096 / 4096 x 14336, cluster kernel -> here, M = 2 5.3 / 16.9 / 13.0 -> 4.4 / 14.5 / 10.7,
+//     M = 4 5.5 / 17.2 / 13.6 -> 5.5 / 16.9 / 12.8, M = 5 5.6 / 16.6 / 13.5 -> 6.0 / 27.9 / 20.4), and where whole units of the cluster kernel do
+//     not fit (K % 512 != 0; 2880 x 2880 M = 4 7.7 -> 5.0).
+// From M = 5 on the launches of this family and of the K_MMA one go to the cluster kernel where that takes them (qmv_cluster_takes).
 inline bool frag_rule(int M, long long N, int K, int bits, int group_size, int dt, bool fused) {
     const long long codes = N * K;
     if (dt == MTC_F32) return M >= 5;
@@ -613,7 +613,7 @@ int mtc_qmv_batched(mtc_ctx *ctx, void *stream, const mtc_qmv_desc *descs, int n
     if (!descs || n < 1 || n > 4) return fail(ctx, MTC_ERR_INVALID, "qmv_batched: 1 to 4 projections");
     int rows = 0;                       // of all projections: they are one launch
     for (int i = 0; i < n; ++i) rows += descs[i].N > 0 && descs[i].N < (1 << 28) ? descs[i].N : 0;
-    bool fused = stream_takes(ctx, descs[0].M), frag = true, ring = ctx->qmv_small_m_mma != 0;
+    bool fused = stream_takes(ctx, descs[0].M), frag = true, cluster = ctx->qmv_small_m_mma != 0;
     for (int i = 0; i < n; ++i) {
         int rc = check_desc(ctx, descs[i], "qmv_batched");
         if (rc != MTC_OK) return rc;
@@ -623,8 +623,7 @@ int mtc_qmv_batched(mtc_ctx *ctx, void *stream, const mtc_qmv_desc *descs, int n
         fused = fused && d.group_size == descs[0].group_size;
         frag = frag && d.n_outs == 1 && d.bits == descs[0].bits && d.group_size == descs[0].group_size && d.M > 0 && d.N > 0 &&
                frag_takes(ctx, d.M, rows, n > 1, d.N, d.K, d.bits, d.group_size, d.dtype, d.w, d.scales, d.biases, d.x);
-        ring = ring && d.n_outs == 1 && d.group_size == descs[0].group_size &&
-               mtc::qmv_ring_supported(d.M, d.N, d.K, d.bits, d.group_size, d.dtype, d.w, d.scales, d.biases, d.x);
+        cluster = cluster && d.n_outs == 1 && d.M >= 2 && d.N > 0 && d.bits == 4 && d.dtype != MTC_F32;
         fused = fused && d.M > 0 && d.N > 0 &&
                 mtc::qmv_stream_supported(d.M, d.N, d.K, d.bits, d.group_size, d.dtype, d.w, d.scales, d.biases, d.x);
     }
@@ -638,9 +637,9 @@ int mtc_qmv_batched(mtc_ctx *ctx, void *stream, const mtc_qmv_desc *descs, int n
         if (e != cudaSuccess) return fail(ctx, MTC_ERR_DISPATCH, std::string("qmv_batched launch: ") + cudaGetErrorString(e));
         return MTC_OK;
     }
-    if (ring) {
-        cudaError_t e = mtc::launch_qmv_ring(ctx, static_cast<cudaStream_t>(stream), descs, n);
-        if (e != cudaSuccess) return fail(ctx, MTC_ERR_DISPATCH, std::string("qmv_batched (ring) launch: ") + cudaGetErrorString(e));
+    if (cluster && mtc::qmv_cluster_takes(descs, n, ctx->sm_count)) {
+        cudaError_t e = mtc::launch_qmv_cluster(ctx, static_cast<cudaStream_t>(stream), descs, n);
+        if (e != cudaSuccess) return fail(ctx, MTC_ERR_DISPATCH, std::string("qmv_batched (cluster) launch: ") + cudaGetErrorString(e));
         return MTC_OK;
     }
     for (int i = 0; i < n; ++i) {
