@@ -287,6 +287,10 @@ struct GatherMats {
 cudaError_t launch_gather_stream(Ctx *ctx, cudaStream_t st, const void *x, const void *x2, const uint32_t *row_src, int n_src_rows,
                                  const GatherMats *mats, int n_mats, const uint32_t *expert_offsets, int m_total, int n_out, int K,
                                  int n_experts, int group_size, int dtype, void *scratch);
+bool gather_frag_supported(int m_total, int n_out, int K, int n_experts, int bits, int group_size, int dt, const void *w, const void *scales,
+                           const void *biases, const void *x);
+cudaError_t launch_gather_frag(Ctx *ctx, cudaStream_t st, const void *x, const uint32_t *row_src, int n_src_rows, const GatherMats *mats, int n_mats,
+                               const uint32_t *expert_offsets, int m_total, int n_out, int K, int n_experts, int bits, int group_size, int dt);
 cudaError_t launch_affine_dequantize(Ctx *ctx, cudaStream_t st, const void *w, const void *scales, const void *biases, void *out,
                                      size_t n_elem, int bits, int group_size, int dt);
 size_t moe_decode_smem_bytes(int n_slots, int in_dim);

@@ -260,8 +260,8 @@ template <int XT>
 constexpr int kPitch = 64 * kPieces<XT> + 16;
 
 // Returns the sum of the 32 activations (not for G8, whose two halves have sums of their own).
-template <int BITS, int XT, int MODE>
-__device__ __forceinline__ float stage_chunk(const FragArgs &a, int m, int k_lo, int k_hi, char *dst) {
+template <int BITS, int XT, int MODE, typename A>              // A: x, K, M of the rows
+__device__ __forceinline__ float stage_chunk(const A &a, int m, int k_lo, int k_hi, char *dst) {
     // k_lo: first activation of registers 0-7, k_hi: of registers 8-15 (16 values each; both inside or outside the row)
     constexpr bool BF = XT != MTC_F16;
     if constexpr (XT == MTC_F32) {

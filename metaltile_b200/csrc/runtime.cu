@@ -6,6 +6,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <cstdlib>
 #include <map>
 #include <string>
 #include <thread>
@@ -204,6 +205,11 @@ inline bool frag_rule(int M, long long N, int K, int bits, int group_size, int d
     if (M <= 4) return true;
     if (M <= 8) return K <= 8192 || codes < (32ll << 20);
     return group_size % 64 == 0 && K <= 5120 && codes <= (fused ? 128ll << 20 : 20ll << 20);
+}
+// Grouped products by rows per expert in the mean: the grouped fragment kernel.
+inline bool gather_frag_rule(int m_total, int n_experts, int bits) {
+    const char *e = getenv("MTC_GF");
+    return e && atoi(e) * static_cast<long long>(n_experts) >= m_total && bits > 0;
 }
 // rows: weight rows of the launch (N, or those of all fused projections)
 inline bool frag_takes(const Ctx *ctx, int M, long long rows, bool fused, int N, int K, int bits, int group_size, int dt, const void *w, const void *scales,
@@ -1098,6 +1104,12 @@ int mtc_set_option(mtc_ctx *ctx, const char *name, int value) {
     return fail(ctx, MTC_ERR_UNSUPPORTED, std::string("unknown option: ") + name);
 }
 
+static bool gather_frag_takes(const Ctx *ctx, bool csr, int m_total, int n_out, int k_in, int n_experts, int bits, int group_size, int dtype,
+                              const void *w, const void *scales, const void *biases, const void *x) {
+    return csr && (!ctx || ctx->gather_stream) && gather_frag_rule(m_total, n_experts, bits) &&
+           mtc::gather_frag_supported(m_total, n_out, k_in, n_experts, bits, group_size, dtype, w, scales, biases, x);
+}
+
 int mtc_gather_qmm(mtc_ctx *ctx, void *stream, const void *x, const void *w, const void *scales, const void *biases,
                    const void *expert_offsets, const void *indices, void *out, int m_total, int n_out, int k_in,
                    int n_experts, int bits, int group_size, int dtype) {
@@ -1114,6 +1126,12 @@ int mtc_gather_qmm(mtc_ctx *ctx, void *stream, const void *x, const void *w, con
     if (m_total == 0 || n_out == 0) return MTC_OK;
     if (!x || !w || !scales || !biases || !out) return fail(ctx, MTC_ERR_INVALID, "gather_qmm: null pointer");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (gather_frag_takes(ctx, expert_offsets != nullptr, m_total, n_out, k_in, n_experts, bits, group_size, dtype, w, scales, biases, x)) {
+        const mtc::GatherMats one{w, scales, biases, out};
+        MTC_CUDA(ctx, mtc::launch_gather_frag(ctx, st, x, nullptr, 0, &one, 1, static_cast<const uint32_t *>(expert_offsets), m_total, n_out, k_in, n_experts,
+                                              bits, group_size, dtype), MTC_ERR_DISPATCH);
+        return MTC_OK;
+    }
     // few rows per expert: the layer is bound by reading every expert's matrix once - the streaming kernel
     if (ctx->gather_stream && expert_offsets && static_cast<long long>(m_total) <= 64ll * n_experts &&
         mtc::gather_stream_supported(m_total, n_out, k_in, n_experts, bits, group_size, dtype, w, scales, biases, x)) {
@@ -1164,10 +1182,27 @@ int mtc_moe_experts(mtc_ctx *ctx, void *stream, const void *x, const void *sort_
                           mtc::gather_stream_supported(m_total, inter, hidden, n_experts, bits, group_size, dtype, gate->w, gate->scales, gate->biases, x) &&
                           mtc::gather_stream_supported(m_total, inter, hidden, n_experts, bits, group_size, dtype, up->w, up->scales, up->biases, x) &&
                           mtc::gather_stream_supported(m_total, hidden, inter, n_experts, bits, group_size, dtype, down->w, down->scales, down->biases, nullptr);
+    const bool frag = gather_frag_takes(ctx, true, m_total, inter, hidden, n_experts, bits, group_size, dtype, gate->w, gate->scales, gate->biases, x) &&
+                      gather_frag_takes(ctx, true, m_total, inter, hidden, n_experts, bits, group_size, dtype, up->w, up->scales, up->biases, x) &&
+                      gather_frag_takes(ctx, true, m_total, hidden, inter, n_experts, bits, group_size, dtype, down->w, down->scales, down->biases, nullptr);
     std::string why;
-    cudaError_t e = mtc::grow_block(ctx, st, &ctx->d_moe, &ctx->moe_bytes, 2 * act_bytes + (streamed ? 0 : xp_bytes), &why);
+    cudaError_t e = mtc::grow_block(ctx, st, &ctx->d_moe, &ctx->moe_bytes, 2 * act_bytes + (streamed || frag ? 0 : xp_bytes), &why);
     if (e != cudaSuccess) return fail(ctx, MTC_ERR_BUFFER, "moe_experts intermediates: " + (why.empty() ? std::string(cudaGetErrorString(e)) : why));
     char *g = static_cast<char *>(ctx->d_moe), *u = g + act_bytes, *xp = u + act_bytes;
+    if (frag) {
+        // three launches: gate and up (the permutation folded in), SwiGLU, down
+        const uint32_t *offsets = static_cast<const uint32_t *>(expert_offsets);
+        const mtc::GatherMats gu[2] = {{gate->w, gate->scales, gate->biases, g}, {up->w, up->scales, up->biases, u}};
+        e = mtc::launch_gather_frag(ctx, st, x, static_cast<const uint32_t *>(sort_token_idx), n_tokens, gu, 2, offsets, m_total, inter, hidden, n_experts,
+                                    bits, group_size, dtype);
+        if (e != cudaSuccess) return fail(ctx, MTC_ERR_DISPATCH, std::string("moe_experts (gate, up) launch: ") + cudaGetErrorString(e));
+        const int rc = mtc_swiglu(ctx, stream, g, u, g, static_cast<size_t>(m_total) * inter, dtype);
+        if (rc != MTC_OK) return rc;
+        const mtc::GatherMats dn{down->w, down->scales, down->biases, y};
+        e = mtc::launch_gather_frag(ctx, st, g, nullptr, 0, &dn, 1, offsets, m_total, hidden, inter, n_experts, bits, group_size, dtype);
+        if (e != cudaSuccess) return fail(ctx, MTC_ERR_DISPATCH, std::string("moe_experts (down) launch: ") + cudaGetErrorString(e));
+        return MTC_OK;
+    }
     if (streamed) {
         // four launches: rows -> fragments (the permutation folded in), gate and up as one stream, SwiGLU -> fragments, down
         const size_t need = std::max(mtc::gather_stream_scratch_bytes(m_total, hidden), mtc::gather_stream_scratch_bytes(m_total, inter));
