@@ -6,7 +6,6 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
-#include <cstdlib>
 #include <map>
 #include <string>
 #include <thread>
@@ -206,10 +205,18 @@ inline bool frag_rule(int M, long long N, int K, int bits, int group_size, int d
     if (M <= 8) return K <= 8192 || codes < (32ll << 20);
     return group_size % 64 == 0 && K <= 5120 && codes <= (fused ? 128ll << 20 : 20ll << 20);
 }
-// Grouped products by rows per expert in the mean: the grouped fragment kernel.
-inline bool gather_frag_rule(int m_total, int n_experts, int bits) {
-    const char *e = getenv("MTC_GF");
-    return e && atoi(e) * static_cast<long long>(n_experts) >= m_total && bits > 0;
+// The grouped fragment kernel (gather_frag.cuh) against the tcgen05 kernel and, where that takes the shape (`streamed`), the streaming one, by
+// rows per expert and codes of a stacked matrix (us a layer, other kernel -> it).  Its passes hold eight rows and read the expert's matrices
+// once each; the others cost their launches whatever the rows.
+//   against tcgen05, 128 experts of 2048 x 768, 0.5 / 2 / 6 / 8 rows an expert: 8-bit 161 -> 85, 239 -> 176, 269 -> 259, 273 against 316; 2-bit 168 -> 68,
+//     258 -> 132, 295 -> 221, 296 -> 262; 3-bit, groups of 32 176 -> 82, 272 -> 181, 309 against 326.  32 experts of 1024 x 768 (24 Mi codes), 6 / 16
+//     rows: 2-bit 71 -> 42, 75 -> 71; 8-bit 72 -> 53, 74 against 84; 32 of 896 x 512, 9.5 rows, 6-bit 75 -> 56.
+//   against the streaming kernel, 128 experts of 2048 x 768, 0.06 / 0.25 / 0.5 / 0.75 rows: 38.7 -> 28.2, 52.4 -> 47.5, 67.8 -> 67.2, 79 against 89; 16 of
+//     1024 x 512 (8 Mi codes), 1 / 4 rows: 30 -> 22, 32 -> 26.
+inline bool gather_frag_rule(int m_total, int n_out, int k_in, int n_experts, bool streamed) {
+    const long long codes = static_cast<long long>(n_experts) * n_out * k_in, rows = m_total, experts = n_experts;
+    if (streamed) return 2 * rows <= experts || (rows <= 4 * experts && codes <= (16ll << 20));
+    return rows <= 4 * experts || (rows <= 10 * experts && codes <= (32ll << 20));
 }
 // rows: weight rows of the launch (N, or those of all fused projections)
 inline bool frag_takes(const Ctx *ctx, int M, long long rows, bool fused, int N, int K, int bits, int group_size, int dt, const void *w, const void *scales,
@@ -1104,9 +1111,16 @@ int mtc_set_option(mtc_ctx *ctx, const char *name, int value) {
     return fail(ctx, MTC_ERR_UNSUPPORTED, std::string("unknown option: ") + name);
 }
 
+static bool gather_stream_takes(const Ctx *ctx, bool csr, int m_total, int n_out, int k_in, int n_experts, int bits, int group_size, int dtype,
+                                const void *w, const void *scales, const void *biases, const void *x) {
+    return csr && (!ctx || ctx->gather_stream) && static_cast<long long>(m_total) <= 64ll * n_experts &&
+           mtc::gather_stream_supported(m_total, n_out, k_in, n_experts, bits, group_size, dtype, w, scales, biases, x);
+}
 static bool gather_frag_takes(const Ctx *ctx, bool csr, int m_total, int n_out, int k_in, int n_experts, int bits, int group_size, int dtype,
                               const void *w, const void *scales, const void *biases, const void *x) {
-    return csr && (!ctx || ctx->gather_stream) && gather_frag_rule(m_total, n_experts, bits) &&
+    return csr && (!ctx || ctx->gather_stream) &&
+           gather_frag_rule(m_total, n_out, k_in, n_experts,
+                            gather_stream_takes(ctx, csr, m_total, n_out, k_in, n_experts, bits, group_size, dtype, w, scales, biases, x)) &&
            mtc::gather_frag_supported(m_total, n_out, k_in, n_experts, bits, group_size, dtype, w, scales, biases, x);
 }
 
@@ -1133,8 +1147,7 @@ int mtc_gather_qmm(mtc_ctx *ctx, void *stream, const void *x, const void *w, con
         return MTC_OK;
     }
     // few rows per expert: the layer is bound by reading every expert's matrix once - the streaming kernel
-    if (ctx->gather_stream && expert_offsets && static_cast<long long>(m_total) <= 64ll * n_experts &&
-        mtc::gather_stream_supported(m_total, n_out, k_in, n_experts, bits, group_size, dtype, w, scales, biases, x)) {
+    if (gather_stream_takes(ctx, expert_offsets != nullptr, m_total, n_out, k_in, n_experts, bits, group_size, dtype, w, scales, biases, x)) {
         std::string why;
         cudaError_t e = mtc::grow_block(ctx, st, &ctx->d_gfrag, &ctx->gfrag_bytes, mtc::gather_stream_scratch_bytes(m_total, k_in), &why);
         if (e != cudaSuccess) return fail(ctx, MTC_ERR_BUFFER, "gather_qmm staging: " + (why.empty() ? std::string(cudaGetErrorString(e)) : why));
@@ -1178,13 +1191,16 @@ int mtc_moe_experts(mtc_ctx *ctx, void *stream, const void *x, const void *sort_
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const size_t esz = mtc::dtype_size(dtype);
     const size_t act_bytes = align_up(static_cast<size_t>(m_total) * inter * esz, 256), xp_bytes = align_up(static_cast<size_t>(m_total) * hidden * esz, 256);
-    const bool streamed = ctx->gather_stream && static_cast<long long>(m_total) <= 64ll * n_experts &&
-                          mtc::gather_stream_supported(m_total, inter, hidden, n_experts, bits, group_size, dtype, gate->w, gate->scales, gate->biases, x) &&
-                          mtc::gather_stream_supported(m_total, inter, hidden, n_experts, bits, group_size, dtype, up->w, up->scales, up->biases, x) &&
-                          mtc::gather_stream_supported(m_total, hidden, inter, n_experts, bits, group_size, dtype, down->w, down->scales, down->biases, nullptr);
-    const bool frag = gather_frag_takes(ctx, true, m_total, inter, hidden, n_experts, bits, group_size, dtype, gate->w, gate->scales, gate->biases, x) &&
-                      gather_frag_takes(ctx, true, m_total, inter, hidden, n_experts, bits, group_size, dtype, up->w, up->scales, up->biases, x) &&
-                      gather_frag_takes(ctx, true, m_total, hidden, inter, n_experts, bits, group_size, dtype, down->w, down->scales, down->biases, nullptr);
+    // the kernels that mtc_gather_qmm takes for the three products: fused where they agree, composed from the entries where they do not
+    const mtc_qmat *const mats[3] = {gate, up, down};
+    int n_frag = 0, n_stream = 0;
+    for (int i = 0; i < 3; ++i) {
+        const int n = i < 2 ? inter : hidden, k = i < 2 ? hidden : inter;
+        const void *const in = i < 2 ? x : nullptr;
+        n_frag += gather_frag_takes(ctx, true, m_total, n, k, n_experts, bits, group_size, dtype, mats[i]->w, mats[i]->scales, mats[i]->biases, in);
+        n_stream += gather_stream_takes(ctx, true, m_total, n, k, n_experts, bits, group_size, dtype, mats[i]->w, mats[i]->scales, mats[i]->biases, in);
+    }
+    const bool frag = n_frag == 3, streamed = n_frag == 0 && n_stream == 3;
     std::string why;
     cudaError_t e = mtc::grow_block(ctx, st, &ctx->d_moe, &ctx->moe_bytes, 2 * act_bytes + (streamed || frag ? 0 : xp_bytes), &why);
     if (e != cudaSuccess) return fail(ctx, MTC_ERR_BUFFER, "moe_experts intermediates: " + (why.empty() ? std::string(cudaGetErrorString(e)) : why));
@@ -1265,9 +1281,11 @@ int mtc_gather_qmm_static(mtc_ctx *ctx, void *stream, const void *x, const void 
 }
 
 const char *mtc_gather_qmm_route(int m_total, int n_out, int k_in, int n_experts, int bits, int group_size, int dtype) {
-    if (n_experts > 0 && static_cast<long long>(m_total) <= 64ll * n_experts &&
-        mtc::gather_stream_supported(m_total, n_out, k_in, n_experts, bits, group_size, dtype, nullptr, nullptr, nullptr, nullptr))
-        return "gather_qmm_stream";        // the CSR form with option "gather_stream" at its default
+    // the CSR form with option "gather_stream" at its default
+    if (n_experts > 0 && gather_frag_takes(nullptr, true, m_total, n_out, k_in, n_experts, bits, group_size, dtype, nullptr, nullptr, nullptr, nullptr))
+        return "gather_qmm_frag";
+    if (n_experts > 0 && gather_stream_takes(nullptr, true, m_total, n_out, k_in, n_experts, bits, group_size, dtype, nullptr, nullptr, nullptr, nullptr))
+        return "gather_qmm_stream";
     return mtc::qmm_tcgen05_supported(m_total, n_out, k_in, bits, group_size, dtype, nullptr, nullptr, nullptr)
                ? "gather_qmm_tcgen05" : "gather_qmm_cuda_core";
 }
