@@ -93,6 +93,7 @@ struct QmmParams {
     int n_tiles;                 // dense: weight-row tiles
     int ksplit;                  // dense: K slices per (weight-row tile, token rows) unit, each an item of its own; 1 = none
     float *partial;              // ksplit > 1: f32 partial sums [ksplit][M][N], added by ksplit_sum_kernel
+    int cluster;                 // 1: the slices of a unit are the CTAs of a cluster (an item each) and add up through distributed shared memory
     int pdl_roles;               // programmatic dependent launch: 1 = only the roles that touch what an earlier kernel of the
                                  //    stream may have written (producer: x; epilogue: token factors, out) wait for it, the
                                  //    dequant warps start on the weights at once; 0 = every thread waits first
@@ -111,6 +112,9 @@ struct __align__(8) SmemCtrl {
 };
 
 // ---- PTX wrappers -------------------------------------------------------------------------------
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
@@ -762,6 +766,18 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                 const int row_base = item.row0 + c * p.TN;
                 const int rows_h = item.nc == 2 ? min(p.TN, item.rows - c * p.TN) : item.rows;
                 if constexpr (KSPLIT) {
+                    if (p.cluster) {
+                        // the MMAs of the CTA's only item are complete: its ring becomes [token][128 outputs] of f32
+                        float *o = reinterpret_cast<float *>(smem) + c * p.TN * BMW + q * 32 + lane;
+                        for (int c0 = 0; c0 < rows_h; c0 += 32) {
+                            uint32_t v[32];
+                            tmem_ld32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + (buf + hh) * TN_MAX + c0, v);
+#pragma unroll
+                            for (int j = 0; j < 32; ++j)
+                                if (c0 + j < rows_h) o[(c0 + j) * BMW] = __uint_as_float(v[j]);
+                        }
+                        continue;
+                    }
                     // a K slice: f32 partial sums, 32 token rows at a time in 128-byte segments per warp and row
                     for (int c0 = 0; c0 < rows_h; c0 += 32) {
                         uint32_t v[32];
@@ -962,6 +978,49 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
         }
     }
 
+    if constexpr (KSPLIT) {
+        if (p.cluster) {
+            // The sum over the slices in slice order, the token factors, the stores: a CTA takes its share of the token rows, a warp a row, a
+            // lane four outputs.  Every role of every CTA comes here, also one that gave up.
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+            __syncwarp();
+            cluster_sync();
+            const Item item = get_item<KSPLIT>(p, blockIdx.x);
+            const int n = item.n_tile * BMW + lane * 4, left = p.N - n;
+            const uint32_t mine = smem_u32(smem) + lane * 16;
+            for (int j = item.rows * item.ks / p.ksplit + warp; j < item.rows * (item.ks + 1) / p.ksplit; j += NUM_THREADS / 32) {
+                float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                for (int r = 0; r < p.ksplit; ++r) {
+                    uint32_t a;
+                    float4 t;
+                    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(mine + j * (BMW * 4)), "r"(r));
+                    asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(t.x), "=f"(t.y), "=f"(t.z), "=f"(t.w) : "r"(a) : "memory");
+                    if (r == 0) v = t;
+                    else { v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w; }
+                }
+                if (left <= 0) continue;
+                const int m = item.row0 + j;
+                if (p.tok_scale) {
+                    const float f = p.tok_scale[m];
+                    v.x *= f; v.y *= f; v.z *= f; v.w *= f;
+                }
+                const uint32_t lo = pack_out(v.x, v.y, p.out_dt == MTC_F16), hi = pack_out(v.z, v.w, p.out_dt == MTC_F16);
+                for (int d = 0; d < p.n_outs; ++d) {
+                    unsigned short *const o = static_cast<unsigned short *>(p.outs[d]) + static_cast<size_t>(m) * p.out_ld + n;
+                    if (left >= 4 && p.out_ld % 4 == 0 && reinterpret_cast<uintptr_t>(p.outs[d]) % 8 == 0) {
+                        *reinterpret_cast<uint2 *>(o) = make_uint2(lo, hi);
+                    } else {
+                        const unsigned short e[4] = {static_cast<unsigned short>(lo), static_cast<unsigned short>(lo >> 16), static_cast<unsigned short>(hi),
+                                                     static_cast<unsigned short>(hi >> 16)};
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+                            if (k < left) o[k] = e[k];
+                    }
+                }
+            }
+            cluster_sync();                              // no CTA leaves while another reads its sums
+        }
+    }
     tc_fence_before();
     __syncthreads();
     if (warp == 2) {
@@ -1127,11 +1186,15 @@ cudaError_t launch_bits(cudaStream_t st, const CUtensorMap &tmap, const CUtensor
     cfg.blockDim = dim3(NUM_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute la[1];
+    cudaLaunchAttribute la[2];
     la[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     la[0].val.programmaticStreamSerializationAllowed = 1;
+    la[1].id = cudaLaunchAttributeClusterDimension;
+    la[1].val.clusterDim.x = p.cluster ? p.ksplit : 1;
+    la[1].val.clusterDim.y = 1;
+    la[1].val.clusterDim.z = 1;
     cfg.attrs = la;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = p.cluster ? 2 : 1;
     auto go = [&](auto kern, PerDeviceAttr &attr) {
         cudaError_t e = attr.set(kern, smem);
         return e != cudaSuccess ? e : cudaLaunchKernelEx(&cfg, kern, tmap, wmap, p);
@@ -1275,13 +1338,16 @@ cudaError_t stage_x(Ctx *ctx, cudaStream_t st, const void *x, int rows, int K, i
 constexpr double kKbBase = 0.47, kKbPerToken = 0.0006;
 constexpr double kWideBase = 0.45, kWidePerToken = 0.00075;      // an item of two chunks
 constexpr double kSliceUs = 2e-6;       // an f32 partial sum: written at ~3 TB/s, read at ~6
+// Clusters of one to eight CTAs, one CTA an SM, that are resident at once (cudaOccupancyMaxActiveClusters: the GPCs do not divide evenly)
+constexpr int kClusters[9] = {0, 148, 74, 45, 33, 26, 22, 15, 15};
+constexpr double kClusterUs = 5.5;      // their launch and barriers, and the sum: 128 x 2048 x 2048 took 12.4 us with them where two kernels take 10.5
 constexpr double kItemUs = 0.4;         // a further item on the same SM: its accumulators drain before the next pair starts
 
 // How a dense launch covers its M token rows: items of one chunk (TN rows, one accumulator) or of two (the dequantised W stage
 // is built once for both), chunks of equal width (333 rows are 2 x 176, not 256 + 77), and K slices where the items alone
 // would leave SMs idle.  Every form is priced by the rounds of the grid it takes.
 struct DensePlan {
-    int TN, items_m, ksplit, halves;      // halves: wide items of an incomplete last round that run as two single-chunk items each
+    int TN, items_m, ksplit, halves, cluster;      // halves: wide items of an incomplete last round that run as two single-chunk items each
     bool wide;
 };
 //
@@ -1289,10 +1355,14 @@ struct DensePlan {
 // blocks without bound (they are kept until the context goes), and so that the sum kernel's 32-bit index holds every output.
 // slices = false: the best plan without them, for a caller whose block cannot grow.
 constexpr size_t kSliceBytes = size_t{512} << 20;
+// options "qmm_ksplit" and "qmm_wide"; form 1: items of two chunks
+bool slices_allowed(const Ctx *ctx, int M, int form) {
+    return ctx->qmm_ksplit && (ctx->qmm_wide == 1 || M <= TN_MAX) && (form == 0 || (ctx->qmm_wide && M > TN_MAX));
+}
 DensePlan plan_dense(const Ctx *ctx, int M, int N, int K, int bits, bool slices = true) {
     const int n_tiles = (N + BMW - 1) / BMW, nkb = K / BK, nsb = (nkb + SB_PER_RAW - 1) / SB_PER_RAW, sms = ctx->sm_count;
     const auto up16 = [](int v) { return (v + 15) / 16 * 16; };
-    if (ctx->qmm_force_tn > 0) return DensePlan{ctx->qmm_force_tn, (M + ctx->qmm_force_tn - 1) / ctx->qmm_force_tn, 1, 0, false};
+    if (ctx->qmm_force_tn > 0) return DensePlan{ctx->qmm_force_tn, (M + ctx->qmm_force_tn - 1) / ctx->qmm_force_tn, 1, 0, 0, false};
     // two ring stages of one W and two X chunks beside two raw buffers
     const int raw_total = 2 * raw_bytes(bits);
     int tn_wide = ((RING_BYTES - raw_total) / 2 - A_BYTES) / (2 * BK * 2) / 16 * 16;
@@ -1320,7 +1390,27 @@ DensePlan plan_dense(const Ctx *ctx, int M, int N, int K, int bits, bool slices 
             if (S > 1) us += 2.0 + static_cast<double>(S) * M * N * kSliceUs;
             if (us < best_us - 1e-9) {
                 best_us = us;
-                best = DensePlan{TN, items_m, S, S == 1 && tail ? left : 0, form == 1};
+                best = DensePlan{TN, items_m, S, S == 1 && tail ? left : 0, 0, form == 1};
+            }
+        }
+    }
+    // ... or slices that are the CTAs of a cluster each and add up in shared memory: no block, no second kernel, but units of a round that the
+    // GPCs' odd sizes leave room for.  Taken where the price is a tenth lower: what the items cost differs by format (f16 4-bit 256 x 4096 x 4096
+    // 25.6 -> 23.2 us, 512 x 4096 x 4096 38.0 -> 35.7, 8-bit 333 x 7616 x 2880 37.2 -> 34.4, 2-bit 285 x 6400 x 3072 30.4 -> 28.0; without the tenth
+    // 8-bit 1000 x 1536 x 4352 29.4 -> 31.0), and of two chunks only as pairs (2-bit 285 x 3072 x 3072 as five 18.6 -> 19.6).
+    double cluster_us = 0.9 * best_us;
+    for (int form = 0; form < 2; ++form) {
+        if (!slices_allowed(ctx, M, form)) continue;
+        const int most = form == 1 ? 2 * tn_wide : TN_MAX, items_m = (M + most - 1) / most;
+        const int TN = form == 1 ? up16((M + 2 * items_m - 1) / (2 * items_m)) : up16((M + items_m - 1) / items_m);
+        const double kb_us = form == 1 ? kWideBase + kWidePerToken * 2 * TN : kKbBase + kKbPerToken * TN;
+        if ((form == 1 ? 2 : 1) * TN * BMW * 4 > RING_BYTES) continue;             // the sums take the ring's place
+        for (int S = 2; S <= (form == 1 ? 2 : 8) && S <= nsb; ++S) {
+            if (static_cast<long long>(n_tiles) * items_m > kClusters[S] * sms / kNumSMsB200) continue;            // one round: a second would start from nothing
+            const double us = (nsb + S - 1) / S * SB_PER_RAW * kb_us + kItemUs + kClusterUs;
+            if (us < cluster_us) {
+                cluster_us = us;
+                best = DensePlan{TN, items_m, S, 0, 1, form == 1};
             }
         }
     }
@@ -1397,7 +1487,7 @@ cudaError_t launch_qmm_tcgen05(Ctx *ctx, cudaStream_t st, const void *w, const v
                                std::string *why, void *const *outs, int n_outs, long long out_ld) {
     const int sms = ctx->sm_count;
     DensePlan plan = plan_dense(ctx, M, N, K, bits);
-    if (plan.ksplit > 1) {
+    if (plan.ksplit > 1 && !plan.cluster) {
         cudaError_t ge = grow_block(ctx, st, &ctx->d_ksplit, &ctx->ksplit_bytes, static_cast<size_t>(plan.ksplit) * M * N * sizeof(float), why);
         if (ge != cudaSuccess) {
             if (M <= 16) return ge;         // the caller has a kernel without scratch for these
@@ -1438,12 +1528,13 @@ cudaError_t launch_qmm_tcgen05(Ctx *ctx, cudaStream_t st, const void *w, const v
     if (plan.ksplit > 1) {
         p.ksplit = plan.ksplit;
         p.partial = static_cast<float *>(ctx->d_ksplit);
+        p.cluster = plan.cluster;
         p.dense_items = p.n_tiles * p.m_chunks * plan.ksplit;
     }
     set_out_vec(p);
-    const int grid = p.dense_items < sms ? p.dense_items : sms;
+    const int grid = p.dense_items < sms || p.cluster ? p.dense_items : sms;
     e = launch_any(bits, st, tmap, p, grid, N, why);
-    if (e != cudaSuccess || p.ksplit == 1) return e;
+    if (e != cudaSuccess || p.ksplit == 1 || p.cluster) return e;
     const bool vec = N % 4 == 0;
     size_t sgrid = (static_cast<size_t>(M) * N / (vec ? 4 : 1) + 255) / 256;
     if (sgrid > static_cast<size_t>(sms) * 8) sgrid = static_cast<size_t>(sms) * 8;
