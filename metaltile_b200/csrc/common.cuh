@@ -249,8 +249,7 @@ void stream_chain_destroy(StreamChain *c);
 bool qmv_frag_supported(int M, int N, int K, int bits, int group_size, int dt, const void *w, const void *scales, const void *biases,
                         const void *x);
 cudaError_t launch_qmv_frag(Ctx *ctx, cudaStream_t st, const mtc_qmv_desc *d, int n);
-bool qmv_cluster_takes(const mtc_qmv_desc *d, int n, int sms);
-cudaError_t launch_qmv_cluster(Ctx *ctx, cudaStream_t st, const mtc_qmv_desc *d, int n);
+bool try_qmv_cluster(Ctx *ctx, cudaStream_t st, const mtc_qmv_desc *d, int n, cudaError_t *e);
 bool qmv_mma_supported(int M, int N, int K, int bits, int group_size, int dt, const void *w, const void *x);
 cudaError_t launch_qmv_mma(Ctx *ctx, cudaStream_t st, const void *w, const void *scales, const void *biases, const void *x,
                            void *out, int M, int N, int K, int group_size, int dt);

@@ -53,7 +53,7 @@ bool supported(const mtc_qmv_desc &d) {
 //     21.5; groups of 32 4096 x 4096, 8 tokens 9.4 -> 6.9).
 //   8-bit, 16-bit activations: from 16 Mi codes on, from nine tokens on from 12 Mi (8192 x 8192, 8 tokens 23.6 -> 17.0, 14336 x 2048, 16 tokens 16.7
 //     -> 11.9; 2048 x 2048 3.8 = 3.9, 5120 x 3072 7.0 against 7.9), with groups of 32 always (2048 x 2048 4.8 -> 4.4).
-bool qmv_cluster_takes(const mtc_qmv_desc *d, int n, int sms) {
+static bool takes(const mtc_qmv_desc *d, int n, int sms, clu::Plan &plan) {
     long long codes = 0;
     int tiles = 0;
     for (int i = 0; i < n; ++i) {
@@ -62,12 +62,14 @@ bool qmv_cluster_takes(const mtc_qmv_desc *d, int n, int sms) {
         tiles += (d[i].N + 15) / 16;
     }
     if (d[0].bits == 8 && d[0].dtype != MTC_F32 && d[0].group_size != 32 && codes < ((d[0].M <= 8 ? 16ll : 12ll) << 20)) return false;
-    return clu::shape_plan(d[0], tiles, sms).shift >= 0;       // a part of K that shared memory cannot hold: no plan
+    plan = clu::shape_plan(d[0], tiles, sms);
+    return plan.shift >= 0;          // a part of K that shared memory cannot hold: no plan
 }
 
-// 1 to 4 projections that read the same activations, each writing its own output
-cudaError_t launch_qmv_cluster(Ctx *ctx, cudaStream_t st, const mtc_qmv_desc *d, int n) {
-    if (n < 1 || n > 4) return cudaErrorInvalidValue;
+// 1 to 4 projections that read the same activations, each writing its own output; false: not this kernel's shape, nothing is launched
+bool try_qmv_cluster(Ctx *ctx, cudaStream_t st, const mtc_qmv_desc *d, int n, cudaError_t *e) {
+    clu::Plan p;
+    if (n < 1 || n > 4 || !takes(d, n, ctx->sm_count, p)) return false;
     const int bits = d[0].bits, G = d[0].group_size;
     CluArgs a{};
     a.M = d[0].M;
@@ -88,10 +90,9 @@ cudaError_t launch_qmv_cluster(Ctx *ctx, cudaStream_t st, const mtc_qmv_desc *d,
         p.tile0 = a.tiles;
         a.tiles += (d[i].N + 15) / 16;
     }
-    const clu::Plan p = clu::shape_plan(d[0], a.tiles, ctx->sm_count);
-    if (p.shift < 0) return cudaErrorInvalidConfiguration;
     const clu::Shape s{a.M <= 8 ? 1 : 2, G, d[0].dtype};
-    return bits == 4 ? launch_cluster_b4(st, a, s, p) : launch_cluster_b8(st, a, s, p);
+    *e = bits == 4 ? launch_cluster_b4(st, a, s, p) : launch_cluster_b8(st, a, s, p);
+    return true;
 }
 
 }  // namespace mtc

@@ -195,7 +195,7 @@ inline bool stream_takes_single(const Ctx *ctx, int M, int N, int K) {
 //   4-bit, 2 <= M: up to M = 4 (4096 x 4096 / 28672 x 4096 / 4096 x 14336, cluster kernel -> here, M = 2 5.3 / 16.9 / 13.0 -> 4.4 / 14.5 / 10.7,
 //     M = 4 5.5 / 17.2 / 13.6 -> 5.5 / 16.9 / 12.8, M = 5 5.6 / 16.6 / 13.5 -> 6.0 / 27.9 / 20.4), and where whole units of the cluster kernel do
 //     not fit (K % 512 != 0; 2880 x 2880 M = 4 7.7 -> 5.0).
-// From M = 5 on the launches of this family and of the K_MMA one go to the cluster kernel where that takes them (qmv_cluster_takes).
+// From M = 5 on the launches of this family and of the K_MMA one go to the cluster kernel where that takes them (try_qmv_cluster).
 inline bool frag_rule(int M, long long N, int K, int bits, int group_size, int dt, bool fused) {
     const long long codes = N * K;
     if (dt == MTC_F32) return M >= 5;
@@ -650,8 +650,8 @@ int mtc_qmv_batched(mtc_ctx *ctx, void *stream, const mtc_qmv_desc *descs, int n
         if (e != cudaSuccess) return fail(ctx, MTC_ERR_DISPATCH, std::string("qmv_batched launch: ") + cudaGetErrorString(e));
         return MTC_OK;
     }
-    if (cluster && mtc::qmv_cluster_takes(descs, n, ctx->sm_count)) {
-        cudaError_t e = mtc::launch_qmv_cluster(ctx, static_cast<cudaStream_t>(stream), descs, n);
+    cudaError_t e = cudaSuccess;
+    if (cluster && mtc::try_qmv_cluster(ctx, static_cast<cudaStream_t>(stream), descs, n, &e)) {
         if (e != cudaSuccess) return fail(ctx, MTC_ERR_DISPATCH, std::string("qmv_batched (cluster) launch: ") + cudaGetErrorString(e));
         return MTC_OK;
     }
