@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(32 * kWarps, 1) qmv_cluster_kernel(const __gri
         const int i = i0 + j * W, s = NT == 1 ? i : i >> 1, tok = (NT == 1 ? 0 : (i & 1) * 8) + g;
         v[j].load(a.x, static_cast<size_t>(tok) * a.K + static_cast<size_t>(u0) * UC + s * SEG + t * LC, i < n_stage && tok < a.M);
       }
-      if (i0 == warp)
+      if (i0 == warp)                                         // the other units of the ring, once
 #pragma unroll
         for (int j = 1; j < kDepth; ++j) copy_next(j);
 #pragma unroll
@@ -327,6 +327,9 @@ __global__ void __launch_bounds__(32 * kWarps, 1) qmv_cluster_kernel(const __gri
         }
       }
     }
+    if (warp >= n_stage)                                      // a short row has fewer pieces than warps: these did not come by
+#pragma unroll
+        for (int j = 1; j < kDepth; ++j) copy_next(j);
     __syncthreads();
 
     // ---- products ----

@@ -66,6 +66,21 @@ def test_products(ns, k, m, bits, g, dt):
         _check(torch, o[:m * n].reshape(m, n), mat, x, bits, g, dt)
 
 
+# rows (or parts of rows) of fewer staged pieces than a CTA has warps, and so many tiles that the warps without a piece have two units and more:
+# the whole ring of every warp is requested all the same
+SHORT = [
+    ((16384,), 512, 8, 8, 64, "f32"), ((12288,), 768, 8, 8, 64, "f32"), ((16384,), 896, 5, 8, 64, "f32"), ((50257,), 768, 8, 4, 64, "f32"),
+    ((16384,), 384, 16, 8, 64, "f32"), ((50257,), 512, 5, 4, 64, "bf16"), ((40000,), 256, 16, 4, 64, "bf16"), ((40001,), 256, 6, 4, 32, "bf16"),
+    ((32000,), 768, 8, 8, 64, "bf16"), ((33000,), 512, 7, 8, 64, "f16"), ((30000, 9000, 1000), 512, 6, 4, 64, "f16"),
+    ((2576,), 3072, 8, 8, 64, "f32"), ((2000, 576), 3072, 6, 8, 128, "f32"),                                       # K split over four CTAs
+]
+
+
+@pytest.mark.parametrize("ns,k,m,bits,g,dt", SHORT)
+def test_short_rows_and_many_tiles(ns, k, m, bits, g, dt):
+    test_products(ns, k, m, bits, g, dt)
+
+
 @pytest.mark.parametrize("bits,dt", [(4, "bf16"), (4, "f16"), (4, "f32"), (8, "f32")])
 def test_infinity_and_nan_stay_in_their_token_and_row(bits, dt):
     import torch
