@@ -838,7 +838,7 @@ def extra_measurements(ctx, dev, hbm_peak, tf_peak, local_rank=0, layers=None):
         nbytes = step_bytes(m8, len(layers))
         out["c2_decode_set_m8"] = {"ms": us / 1e3, "GB/s": nbytes / us / 1e3, "frac_of_hbm_peak": nbytes / us / 1e3 / hbm_peak,
                                    # every small-M kernel that takes these shapes takes the projections of a group in one launch
-                                   "launches": len(groups), "kernel": ctx.qmm_kernel(m8, 4096, 4096, BITS, GROUP, "bf16"), "clocks": clk}
+                                   "launches": len(groups), "kernel": ctx.launch_of(m8, [4096], 4096, BITS, GROUP, "bf16")["kernel"], "clocks": clk}
     return out
 
 

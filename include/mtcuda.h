@@ -84,7 +84,7 @@ int mtc_status_clear(mtc_ctx *ctx);
  * crates/metaltile-std/src/ffai/dequant_gemv.rs:52-105).  Any M (tuned for M <= 16), bits in
  * {2,3,4,5,6,8}, K*bits % 32 == 0, group_size | K.  M <= 16 runs on warp-level tensor-core MMAs on the integer codes
  * (f32 accumulate, affine part applied per group) where a kernel for them takes the shape and is the faster one,
- * else on CUDA cores, as does every general case; mtc_qmm_kernel names the choice. */
+ * else on CUDA cores, as does every general case; mtc_launch_of names the choice. */
 int mtc_qmv(mtc_ctx *ctx, void *stream, const void *w, const void *scales, const void *biases,
             const void *x, void *out, int M, int N, int K, int bits, int group_size, int dtype);
 
@@ -99,11 +99,21 @@ int mtc_qmm(mtc_ctx *ctx, void *stream, const void *w, const void *scales, const
 /* mtc_qmm_route: the kernel family of the selector without the fragment kernel, the analogue of asserting on mt_qmm_for's
  * routing (quantized.rs:5127-5199): "qmv_stream", "qmv_cuda_core", "qmv_mma_sync" or "qmm_tcgen05" - what runs with option
  * "qmv_frag" at 0 and the others at their defaults.
- * mtc_qmm_kernel: the kernel that mtc_qmm launches for these arguments with aligned pointers under the options of `ctx` (NULL: the
+ * mtc_qmm_kernel: the kernel family that mtc_qmm takes for these arguments with aligned pointers under the options of `ctx` (NULL: the
  * default options): one of those names, "qmv_frag" or "qmv_tcgen05_decode" (option "qmv_tc"); "" for arguments no kernel takes.
- * The entry itself decides by the same function.  (M in 17..32 that runs as 16-row chunks: the kernel of a whole chunk.) */
+ * The entry itself decides by the same function.  (M in 17..32 that runs as 16-row chunks: the kernel of a whole chunk.)  Products of
+ * two families, "qmv_frag" (from M = 5 on) and "qmv_mma_sync", run on the cluster kernel where that takes the shape:
+ * mtc_launch_of: the launch itself, of mtc_qmm (n = 1; N[0] weight rows) or of mtc_qmv_batched (n = 2 to 4 projections that share x):
+ * `kernel` one of the names above or "qmv_cluster" (csrc/qmv_cluster.cuh), "" where no kernel takes the arguments or where the
+ * projections run one by one.  For "qmv_cluster" and "qmm_tcgen05" also its form, 0 for the others: CTAs, CTAs that are a cluster (1:
+ * none), slices of K, and ("qmv_cluster") the passes over a CTA's tiles. */
+typedef struct {
+    const char *kernel;
+    int ctas, cluster, k_slices, passes;
+} mtc_launch_info;
 const char *mtc_qmm_route(int M, int N, int K, int bits, int group_size, int dtype);
 const char *mtc_qmm_kernel(const mtc_ctx *ctx, int M, int N, int K, int bits, int group_size, int dtype);
+int mtc_launch_of(const mtc_ctx *ctx, int M, const int *N, int n, int K, int bits, int group_size, int dtype, mtc_launch_info *info);
 
 /* ---- fused and chained decode projections ----
  * mtc_qmv_desc: one projection, the arguments of mtc_qmv plus up to 8 destinations of the [M, N] result (each gets

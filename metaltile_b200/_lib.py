@@ -50,6 +50,11 @@ class QMat(ctypes.Structure):
     _fields_ = [("w", ctypes.c_void_p), ("scales", ctypes.c_void_p), ("biases", ctypes.c_void_p)]
 
 
+class LaunchInfo(ctypes.Structure):
+    """mtc_launch_info: what a product launches (``mtc_launch_of``)."""
+    _fields_ = [("kernel", ctypes.c_char_p)] + [(n, ctypes.c_int) for n in ("ctas", "cluster", "k_slices", "passes")]
+
+
 class NamedBuf(ctypes.Structure):
     _fields_ = [("name", ctypes.c_char_p), ("data", ctypes.c_void_p), ("bytes", ctypes.c_size_t),
                 ("is_output", ctypes.c_int)]
@@ -77,6 +82,7 @@ SIGNATURES = {
     "mtc_qmm": (_i, _DENSE),
     "mtc_qmm_route": (ctypes.c_char_p, [_i, _i, _i, _i, _i, _i]),
     "mtc_qmm_kernel": (ctypes.c_char_p, [_vp, _i, _i, _i, _i, _i, _i]),
+    "mtc_launch_of": (_i, [_vp, _i, ctypes.POINTER(_i), _i, _i, _i, _i, _i, ctypes.POINTER(LaunchInfo)]),
     "mtc_qmv_multi": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, ctypes.POINTER(_vp), _i, _i, _i, _i, _i, _i, _i]),
     "mtc_affine_quantize": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, ctypes.c_size_t, _i, _i, _i]),
     "mtc_affine_dequantize": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, ctypes.c_size_t, _i, _i, _i]),

@@ -17,7 +17,7 @@ from dataclasses import dataclass, field
 from typing import Dict, Mapping, Optional, Sequence
 
 from . import _lib
-from ._lib import BF16, F16, F32, BenchStatsC, DispatchSpec, NamedBuf, PeerSync, QMat, QmvDesc
+from ._lib import BF16, F16, F32, BenchStatsC, DispatchSpec, LaunchInfo, NamedBuf, PeerSync, QMat, QmvDesc
 
 DTYPES = {"f32": F32, "f16": F16, "bf16": BF16}
 
@@ -70,6 +70,15 @@ def _binding():
         from . import _dispatch as mod
         _dispatch = mod
     return _dispatch
+
+
+def launch_of(M, Ns, K, bits, group_size, dtype, ctx=None) -> dict:
+    """The kernel and the form of a launch (``mtc_launch_of``); without a context: under the default options, no GPU needed."""
+    info, ns = LaunchInfo(), (ctypes.c_int * len(Ns))(*Ns)
+    rc = _lib.load().mtc_launch_of(ctx._h if ctx else None, M, ns, len(Ns), K, bits, group_size, _dt(dtype), ctypes.byref(info))
+    if rc != 0:
+        raise MetalTileError(rc, "launch_of: one to four projections")
+    return dict(kernel=info.kernel.decode(), ctas=info.ctas, cluster=info.cluster, k_slices=info.k_slices, passes=info.passes)
 
 
 class Context:
@@ -334,8 +343,12 @@ class Context:
                                       _dt(dtype)))
 
     def qmm_kernel(self, M, N, K, bits, group_size, dtype) -> str:
-        """The kernel that ``qmm`` launches under this context's options (aligned pointers)."""
+        """The kernel family that ``qmm`` takes under this context's options (aligned pointers); ``launch_of`` names the launch."""
         return self._lib.mtc_qmm_kernel(self._h, M, N, K, bits, group_size, _dt(dtype)).decode()
+
+    def launch_of(self, M, Ns, K, bits, group_size, dtype) -> dict:
+        """What ``qmm`` (one N) or ``qmv_batched`` (two to four) launches under this context's options (``mtc_launch_of``)."""
+        return launch_of(M, Ns, K, bits, group_size, dtype, self)
 
     def qmm_route(self, M, N, K, bits, group_size, dtype) -> str:
         """The kernel family of the selector without the fragment kernel (option ``qmv_frag`` at 0)."""

@@ -1482,6 +1482,15 @@ bool qmm_tcgen05_supported(int M, int N, int K, int bits, int group_size, int dt
            al(x, 16) && al(out, 2);
 }
 
+// The form of a dense launch, for mtc_launch_of
+void qmm_tcgen05_form(const Ctx *ctx, int M, int N, int K, int bits, mtc_launch_info *info) {
+    const DensePlan plan = plan_dense(ctx, M, N, K, bits);
+    const int items = (N + BMW - 1) / BMW * plan.items_m * plan.ksplit + plan.halves;
+    info->ctas = items < ctx->sm_count || plan.cluster ? items : ctx->sm_count;
+    info->cluster = plan.cluster ? plan.ksplit : 1;
+    info->k_slices = plan.ksplit;
+}
+
 cudaError_t launch_qmm_tcgen05(Ctx *ctx, cudaStream_t st, const void *w, const void *scales, const void *biases,
                                const void *x, void *out, int M, int N, int K, int bits, int group_size, int dt,
                                std::string *why, void *const *outs, int n_outs, long long out_ld) {

@@ -66,6 +66,14 @@ static bool takes(const mtc_qmv_desc *d, int n, int sms, clu::Plan &plan) {
     return plan.shift >= 0;          // a part of K that shared memory cannot hold: no plan
 }
 
+// The form of that launch, for mtc_launch_of; false: not this kernel's shape
+bool qmv_cluster_form(const Ctx *ctx, const mtc_qmv_desc *d, int n, mtc_launch_info *info) {
+    clu::Plan p;
+    if (n < 1 || n > 4 || !takes(d, n, ctx->sm_count, p)) return false;
+    *info = mtc_launch_info{"qmv_cluster", p.clusters << p.shift, 1 << p.shift, 1 << p.shift, p.passes};
+    return true;
+}
+
 // 1 to 4 projections that read the same activations, each writing its own output; false: not this kernel's shape, nothing is launched
 bool try_qmv_cluster(Ctx *ctx, cudaStream_t st, const mtc_qmv_desc *d, int n, cudaError_t *e) {
     clu::Plan p;

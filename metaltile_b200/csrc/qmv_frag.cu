@@ -38,8 +38,6 @@ bool qmv_frag_supported(int M, int N, int K, int bits, int group_size, int dt, c
 // 1 to 4 projections that read the same activations, each writing its own output
 cudaError_t launch_qmv_frag(Ctx *ctx, cudaStream_t st, const mtc_qmv_desc *d, int n) {
     if (n < 1 || n > 4) return cudaErrorInvalidValue;
-    cudaError_t done;
-    if (ctx->qmv_frag != 2 && d[0].M >= 5 && try_qmv_cluster(ctx, st, d, n, &done)) return done;
     const int M = d[0].M, K = d[0].K, bits = d[0].bits, dt = d[0].dtype, esz = static_cast<int>(dtype_size(dt));
     int gs_shift = 0;
     while ((1 << gs_shift) < d[0].group_size) ++gs_shift;

@@ -352,8 +352,6 @@ cudaError_t launch_qmv_mma(Ctx *ctx, cudaStream_t st, const void *w, const void 
     d.w = w; d.scales = scales; d.biases = biases; d.x = x;
     d.outs[0] = out; d.n_outs = 1;
     d.M = M; d.N = N; d.K = K; d.bits = 4; d.group_size = group_size; d.dtype = dt;
-    cudaError_t done;
-    if (try_qmv_cluster(ctx, st, &d, 1, &done)) return done;
     const MmaArgs a = mma_args(d);
     if (dt == MTC_BF16) return M <= 8 ? launch_mma<1, true>(ctx, st, a) : launch_mma<2, true>(ctx, st, a);
     return M <= 8 ? launch_mma<1, false>(ctx, st, a) : launch_mma<2, false>(ctx, st, a);

@@ -195,7 +195,7 @@ inline bool stream_takes_single(const Ctx *ctx, int M, int N, int K) {
 //   4-bit, 2 <= M: up to M = 4 (4096 x 4096 / 28672 x 4096 / 4096 x 14336, cluster kernel -> here, M = 2 5.3 / 16.9 / 13.0 -> 4.4 / 14.5 / 10.7,
 //     M = 4 5.5 / 17.2 / 13.6 -> 5.5 / 16.9 / 12.8, M = 5 5.6 / 16.6 / 13.5 -> 6.0 / 27.9 / 20.4), and where whole units of the cluster kernel do
 //     not fit (K % 512 != 0; 2880 x 2880 M = 4 7.7 -> 5.0).
-// From M = 5 on the launches of this family and of the K_MMA one go to the cluster kernel where that takes them (try_qmv_cluster).
+// From M = 5 on the launches of this family and of the K_MMA one go to the cluster kernel where that takes them (cluster_first).
 inline bool frag_rule(int M, long long N, int K, int bits, int group_size, int dt, bool fused) {
     const long long codes = N * K;
     if (dt == MTC_F32) return M >= 5;
@@ -499,7 +499,7 @@ static bool small_m_tc_preferred(const Ctx *ctx, int M, int N, int K, int bits, 
     return small_m_tc_rule(ctx->qmv_small_m_tc, M, N, K) && mtc::qmm_tcgen05_supported(M, N, K, bits, group_size, dtype, w, x, out);
 }
 
-// The kernel a product runs on: what mtc_qmv and mtc_qmm launch and what mtc_qmm_kernel names, so that the two cannot differ.
+// The kernel family a product runs on: what mtc_qmv and mtc_qmm go by and what mtc_qmm_kernel names, so that the two cannot differ.
 enum ProductKernel { K_DECODE_TC, K_FRAG, K_STREAM, K_MMA, K_TCGEN05, K_CUDA };
 static const char *const kProductKernelNames[] = {"qmv_tcgen05_decode", "qmv_frag", "qmv_stream", "qmv_mma_sync", "qmm_tcgen05", "qmv_cuda_core"};
 
@@ -520,6 +520,25 @@ static ProductKernel qmv_kernel_for(const Ctx *ctx, int M, int N, int K, int bit
     // the tensor-memory kernel with K cut into slices
     if (small_m_tc_preferred(ctx, M, N, K, bits, group_size, dtype, w, x, out)) return K_TCGEN05;
     return K_CUDA;
+}
+
+// Families whose launches the cluster kernel takes over where it takes the shape (what mtc_launch_of names and the entries launch)
+static bool cluster_first(const Ctx *ctx, ProductKernel k, int M) { return k == K_MMA || (k == K_FRAG && ctx->qmv_frag != 2 && M >= 5); }
+
+// The same for projections that share x: K_FRAG, K_STREAM or K_MMA (which only the cluster kernel takes as one launch); K_CUDA: one by one.
+static ProductKernel batched_kernel_for(const Ctx *ctx, const mtc_qmv_desc *descs, int n) {
+    int rows = 0;                       // of all projections: they are one launch
+    for (int i = 0; i < n; ++i) rows += descs[i].N > 0 && descs[i].N < (1 << 28) ? descs[i].N : 0;
+    bool stream = stream_takes(ctx, descs[0].M), frag = true, mma = ctx->qmv_small_m_mma != 0;
+    for (int i = 0; i < n; ++i) {
+        const mtc_qmv_desc &d = descs[i];
+        frag = frag && d.n_outs == 1 && d.bits == descs[0].bits && d.group_size == descs[0].group_size && d.M > 0 && d.N > 0 &&
+               frag_takes(ctx, d.M, rows, n > 1, d.N, d.K, d.bits, d.group_size, d.dtype, d.w, d.scales, d.biases, d.x);
+        mma = mma && d.n_outs == 1 && d.M >= 2 && d.N > 0 && d.bits == 4 && d.dtype != MTC_F32;
+        stream = stream && d.group_size == descs[0].group_size && d.M > 0 && d.N > 0 &&
+                 mtc::qmv_stream_supported(d.M, d.N, d.K, d.bits, d.group_size, d.dtype, d.w, d.scales, d.biases, d.x);
+    }
+    return frag ? K_FRAG : stream ? K_STREAM : mma ? K_MMA : K_CUDA;
 }
 
 // The tcgen05 decode kernel, when it takes the shape: 0 = launched, 1 = not its shape, < 0 = error.
@@ -548,7 +567,12 @@ int mtc_qmv(mtc_ctx *ctx, void *stream, const void *w, const void *scales, const
     d.outs[0] = out; d.n_outs = 1;
     d.M = M; d.N = N; d.K = K; d.bits = bits; d.group_size = group_size; d.dtype = dtype;
     cudaError_t ek = cudaSuccess;
-    switch (qmv_kernel_for(ctx, M, N, K, bits, group_size, dtype, w, scales, biases, x, out)) {
+    const ProductKernel kernel = qmv_kernel_for(ctx, M, N, K, bits, group_size, dtype, w, scales, biases, x, out);
+    if (cluster_first(ctx, kernel, M) && mtc::try_qmv_cluster(ctx, st, &d, 1, &ek)) {
+        if (ek != cudaSuccess) return fail(ctx, MTC_ERR_DISPATCH, std::string("qmv (cluster) launch: ") + cudaGetErrorString(ek));
+        return MTC_OK;
+    }
+    switch (kernel) {
         case K_DECODE_TC: return try_qmv_tc(ctx, stream, w, scales, biases, x, d.outs, 1, M, N, K, bits, group_size, dtype);
         case K_FRAG:
             ek = mtc::launch_qmv_frag(ctx, st, &d, 1);
@@ -624,35 +648,27 @@ int mtc_qmv_batched(mtc_ctx *ctx, void *stream, const mtc_qmv_desc *descs, int n
     if (!ctx) return MTC_ERR_INVALID;
     MTC_ENTER(ctx);
     if (!descs || n < 1 || n > 4) return fail(ctx, MTC_ERR_INVALID, "qmv_batched: 1 to 4 projections");
-    int rows = 0;                       // of all projections: they are one launch
-    for (int i = 0; i < n; ++i) rows += descs[i].N > 0 && descs[i].N < (1 << 28) ? descs[i].N : 0;
-    bool fused = stream_takes(ctx, descs[0].M), frag = true, cluster = ctx->qmv_small_m_mma != 0;
     for (int i = 0; i < n; ++i) {
         int rc = check_desc(ctx, descs[i], "qmv_batched");
         if (rc != MTC_OK) return rc;
         const mtc_qmv_desc &d = descs[i];
         if (d.x != descs[0].x || d.M != descs[0].M || d.K != descs[0].K || d.dtype != descs[0].dtype)
             return fail(ctx, MTC_ERR_INVALID, "qmv_batched: the projections must share x, M, K and dtype");
-        fused = fused && d.group_size == descs[0].group_size;
-        frag = frag && d.n_outs == 1 && d.bits == descs[0].bits && d.group_size == descs[0].group_size && d.M > 0 && d.N > 0 &&
-               frag_takes(ctx, d.M, rows, n > 1, d.N, d.K, d.bits, d.group_size, d.dtype, d.w, d.scales, d.biases, d.x);
-        cluster = cluster && d.n_outs == 1 && d.M >= 2 && d.N > 0 && d.bits == 4 && d.dtype != MTC_F32;
-        fused = fused && d.M > 0 && d.N > 0 &&
-                mtc::qmv_stream_supported(d.M, d.N, d.K, d.bits, d.group_size, d.dtype, d.w, d.scales, d.biases, d.x);
     }
-    if (frag) {
-        cudaError_t e = mtc::launch_qmv_frag(ctx, static_cast<cudaStream_t>(stream), descs, n);
+    const ProductKernel kernel = batched_kernel_for(ctx, descs, n);
+    cudaError_t e = cudaSuccess;
+    if (cluster_first(ctx, kernel, descs[0].M) && mtc::try_qmv_cluster(ctx, static_cast<cudaStream_t>(stream), descs, n, &e)) {
+        if (e != cudaSuccess) return fail(ctx, MTC_ERR_DISPATCH, std::string("qmv_batched (cluster) launch: ") + cudaGetErrorString(e));
+        return MTC_OK;
+    }
+    if (kernel == K_FRAG) {
+        e = mtc::launch_qmv_frag(ctx, static_cast<cudaStream_t>(stream), descs, n);
         if (e != cudaSuccess) return fail(ctx, MTC_ERR_DISPATCH, std::string("qmv_batched (fragments) launch: ") + cudaGetErrorString(e));
         return MTC_OK;
     }
-    if (fused) {
-        cudaError_t e = mtc::launch_qmv_stream(ctx, static_cast<cudaStream_t>(stream), descs, n);
+    if (kernel == K_STREAM) {
+        e = mtc::launch_qmv_stream(ctx, static_cast<cudaStream_t>(stream), descs, n);
         if (e != cudaSuccess) return fail(ctx, MTC_ERR_DISPATCH, std::string("qmv_batched launch: ") + cudaGetErrorString(e));
-        return MTC_OK;
-    }
-    cudaError_t e = cudaSuccess;
-    if (cluster && mtc::try_qmv_cluster(ctx, static_cast<cudaStream_t>(stream), descs, n, &e)) {
-        if (e != cudaSuccess) return fail(ctx, MTC_ERR_DISPATCH, std::string("qmv_batched (cluster) launch: ") + cudaGetErrorString(e));
         return MTC_OK;
     }
     for (int i = 0; i < n; ++i) {
@@ -836,6 +852,38 @@ const char *mtc_qmm_kernel(const mtc_ctx *ctx, int M, int N, int K, int bits, in
     else
         k = qmv_kernel_for(c, M, N, K, bits, group_size, dtype, nullptr, nullptr, nullptr, nullptr, nullptr);
     return kProductKernelNames[k];
+}
+
+int mtc_launch_of(const mtc_ctx *ctx, int M, const int *N, int n, int K, int bits, int group_size, int dtype, mtc_launch_info *info) {
+    if (!N || !info || n < 1 || n > 4) return MTC_ERR_INVALID;
+    *info = mtc_launch_info{"", 0, 0, 0, 0};
+    for (int i = 0; i < n; ++i)
+        if (N[i] < 1) return MTC_OK;
+    if (M < 1 || K < 1 || group_size < 1 || !dtype_ok(dtype)) return MTC_OK;
+    Ctx defaults;
+    defaults.sm_count = mtc::kNumSMsB200;
+    const Ctx *c = ctx ? static_cast<const Ctx *>(ctx) : &defaults;
+    mtc_qmv_desc d[4] = {};
+    for (int i = 0; i < n; ++i) {
+        d[i].n_outs = 1;
+        d[i].M = M; d[i].N = N[i]; d[i].K = K; d[i].bits = bits; d[i].group_size = group_size; d[i].dtype = dtype;
+    }
+    ProductKernel k;
+    if (n > 1) {
+        k = batched_kernel_for(c, d, n);
+    } else if (qmm_in_chunks(c, M, N[0], K, bits, group_size, dtype, nullptr, nullptr)) {
+        M = d[0].M = 16;
+        k = qmv_kernel_for(c, M, N[0], K, bits, group_size, dtype, nullptr, nullptr, nullptr, nullptr, nullptr);
+    } else if (M > 16 && mtc::qmm_tcgen05_supported(M, N[0], K, bits, group_size, dtype, nullptr, nullptr, nullptr)) {
+        k = K_TCGEN05;
+    } else {
+        k = qmv_kernel_for(c, M, N[0], K, bits, group_size, dtype, nullptr, nullptr, nullptr, nullptr, nullptr);
+    }
+    if (cluster_first(c, k, M) && mtc::qmv_cluster_form(c, d, n, info)) return MTC_OK;
+    if (n > 1 && k != K_FRAG && k != K_STREAM) return MTC_OK;         // one by one
+    info->kernel = kProductKernelNames[k];
+    if (k == K_TCGEN05) mtc::qmm_tcgen05_form(c, M, N[0], K, bits, info);
+    return MTC_OK;
 }
 
 int mtc_qmm(mtc_ctx *ctx, void *stream, const void *w, const void *scales, const void *biases, const void *x,

@@ -69,7 +69,7 @@ def _check_out(out, M, N, like):
 
 
 def qmv(w, scales, biases, x, bits: int, group_size: int, out=None, ctx: Context = None):
-    """out[M, N] = x[M, K] @ dequant(w)[N, K]^T (decode, M <= 16 tuned); ``Context.qmm_kernel`` names the kernel."""
+    """out[M, N] = x[M, K] @ dequant(w)[N, K]^T (decode, M <= 16 tuned); ``Context.launch_of`` names the kernel."""
     return _native.dense(0, w, scales, biases, x, bits, group_size, out, ctx)
 
 

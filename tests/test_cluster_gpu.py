@@ -36,12 +36,12 @@ CASES = [
     ((1000, 520, 17), 1536, 7, 4, 64, "bf16"), ((96, 1, 300, 16), 2560, 13, 4, 128, "f16"), ((640, 128), 1536, 12, 4, 256, "bf16"),
     # long rows: the parts of K of two, four and eight CTAs
     ((200,), 8192, 8, 4, 64, "bf16"), ((600, 24), 14336, 8, 4, 64, "f16"), ((513,), 14336, 16, 4, 64, "bf16"), ((300,), 7168, 16, 4, 64, "f32"),
-    # passes over the tiles of a cluster
+    # many tiles a CTA
     ((28672,), 4096, 16, 4, 64, "bf16"), ((40000,), 1024, 8, 4, 64, "f16"), ((9000,), 4096, 8, 4, 32, "f32"),
     # scales of a unit shorter than a window, down to one of two bytes, at the end of the matrix
     ((31,), 512, 8, 4, 512, "bf16"), ((47,), 1024, 11, 4, 512, "bf16"), ((18,), 512, 6, 4, 256, "f16"), ((5,), 1024, 6, 4, 128, "f32"),
     # eight bits: from the size on where it takes over
-    ((4112,), 4096, 8, 8, 64, "bf16"), ((8200, 100), 2048, 16, 8, 128, "f16"), ((2049,), 8192, 9, 8, 256, "bf16"), ((100,), 1280, 5, 8, 64, "f32"),
+    ((4112,), 4096, 8, 8, 64, "bf16"), ((8200, 100), 2048, 16, 8, 128, "f16"), ((3400,), 4096, 9, 8, 256, "bf16"), ((100,), 1280, 5, 8, 64, "f32"),
     ((777,), 1024, 6, 8, 32, "bf16"), ((4100,), 4096, 5, 8, 512, "f16"),
 ]
 
@@ -56,6 +56,7 @@ def test_products(ns, k, m, bits, g, dt):
     mats = [_matrix(torch, n, k, bits, g, td, gen) for n in ns]
     x = torch.randn((m, k), device="cuda", generator=gen).to(td)
     ctx = ops.context()
+    assert ctx.launch_of(m, list(ns), k, bits, g, dt)["kernel"] == "qmv_cluster"
     outs = [torch.full((m * n + 64,), 7.0, dtype=td, device="cuda") for n in ns]
     ctx.qmv_batched([dict(w=w.data_ptr(), scales=s.data_ptr(), biases=b.data_ptr(), x=x.data_ptr(), outs=[o.data_ptr()], M=m, N=n, K=k, bits=bits,
                           group_size=g, dtype=dt) for (w, s, b), o, n in zip(mats, outs, ns)], torch.cuda.current_stream().cuda_stream)
@@ -76,8 +77,15 @@ SHORT = [
 ]
 
 
-@pytest.mark.parametrize("ns,k,m,bits,g,dt", SHORT)
-def test_short_rows_and_many_tiles(ns, k, m, bits, g, dt):
+# tiles of a cluster whose partial sums do not fit at once: two, three and four passes over them
+PASSES = [
+    ((988,), 13824, 11, 4, 256, "bf16"), ((1001, 24), 13568, 14, 4, 128, "f16"), ((262,), 9472, 12, 8, 256, "f32"), ((514,), 9472, 13, 8, 64, "f32"),
+    ((742,), 10240, 10, 8, 128, "f32"), ((16937,), 11520, 9, 4, 64, "bf16"),
+]
+
+
+@pytest.mark.parametrize("ns,k,m,bits,g,dt", SHORT + PASSES)
+def test_short_rows_and_passes(ns, k, m, bits, g, dt):
     test_products(ns, k, m, bits, g, dt)
 
 

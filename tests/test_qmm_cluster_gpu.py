@@ -24,10 +24,13 @@ def test_cluster_slices_equal_the_unsliced_product(m, n, k, bits, g, dt):
     b = (-(2.0 ** (bits - 1)) * s.float()).to(td)
     x = torch.randn((m, k), device="cuda", generator=gen).to(td)
     ctx = Context(0)
+    form = ctx.launch_of(m, [n], k, bits, g, dt)
+    assert form["kernel"] == "qmm_tcgen05" and form["cluster"] == form["k_slices"] >= 2
     got = torch.full((m + 1, n), 7.0, dtype=td, device="cuda")
     ops.qmm(w, s, b, x, bits, g, out=got[:m], ctx=ctx)
     again = ops.qmm(w, s, b, x, bits, g, ctx=ctx)
     ctx.set_option("qmm_ksplit", 0)
+    assert ctx.launch_of(m, [n], k, bits, g, dt)["k_slices"] == 1
     whole = ops.qmm(w, s, b, x, bits, g, ctx=ctx)
     torch.cuda.synchronize()
     assert ctx.status_word() == 0
@@ -38,4 +41,3 @@ def test_cluster_slices_equal_the_unsliced_product(m, n, k, bits, g, dt):
     mag = x.float().abs().sum(1, keepdim=True) * (2.0 ** (bits - 1)) * float(s.float().max())
     bound = unit * whole.float().abs() + 2.0 ** -23 * 16 * mag
     assert bool(((got[:m].float() - whole.float()).abs() <= bound).all())
-    assert not torch.equal(got[:m], whole) or dt == "bf16"            # the slices were taken: another order of the same sums
