@@ -84,7 +84,11 @@ int mtc_status_clear(mtc_ctx *ctx);
  * crates/metaltile-std/src/ffai/dequant_gemv.rs:52-105).  Any M (tuned for M <= 16), bits in
  * {2,3,4,5,6,8}, K*bits % 32 == 0, group_size | K.  M <= 16 runs on warp-level tensor-core MMAs on the integer codes
  * (f32 accumulate, affine part applied per group) where a kernel for them takes the shape and is the faster one,
- * else on CUDA cores, as does every general case; mtc_launch_of names the choice. */
+ * else on CUDA cores, as does every general case; mtc_launch_of names the choice.
+ * Range of bf16 and f32 activations: "qmv_cluster" (and the grouped "gather_qmm_frag") hold whatever the type does, infinities
+ * included, but a token whose values all lie below 2^-112 comes out as zeros; one with a value from 2^31 on, or all of them below 2^-64, makes
+ * its launch some 20 times as long.  "qmv_frag", "qmv_stream" and "gather_qmm_stream" make an infinity of a value from 2^63 on, and
+ * lose bits where all values of a token lie below 2^-57. */
 int mtc_qmv(mtc_ctx *ctx, void *stream, const void *w, const void *scales, const void *biases,
             const void *x, void *out, int M, int N, int K, int bits, int group_size, int dtype);
 

@@ -17,6 +17,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "far_tokens.cuh"
 #include "qmv_frag.cuh"
 
 namespace mtc {
@@ -47,6 +48,72 @@ struct RowX {                        // one row of activations, as stage_chunk r
     int K, M;
 };
 
+struct Tile {
+    int pass, expert, tok0, ntok, second, row0;
+};
+// The rows of expert e: how many, from `lo` on
+__device__ __forceinline__ int rows_of(const GfArgs &a, int e, int &lo) {
+    const uint32_t p = a.offsets[e], q = a.offsets[e + 1], m = static_cast<uint32_t>(a.m_total);
+    lo = static_cast<int>(min(p, m));
+    if (p > m || q > m || q < p) atomicCAS(a.status, 0u, 0x901u);                      // clamped and reported
+    return max(static_cast<int>(min(q, m)) - lo, 0);
+}
+// start[e]: passes of MP rows before expert e
+template <int MP>
+__device__ __forceinline__ void locate(const GfArgs &a, const int *start, int tile, Tile &q) {
+    q.pass = tile / a.tpe;
+    const int r = tile - q.pass * a.tpe;
+    int lo = 0, hi = a.n_experts;                                      // the last expert with start[e] <= pass: it has rows
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (start[mid] <= q.pass) lo = mid; else hi = mid;
+    }
+    q.expert = lo;
+    int first;
+    const int rows = rows_of(a, lo, first), done = (q.pass - start[lo]) * MP;
+    q.tok0 = first + done;
+    q.ntok = min(MP, rows - done);
+    q.second = r >= a.tpm ? 1 : 0;
+    q.row0 = (r - (q.second ? a.tpm : 0)) * 16;
+}
+// The row of x that row r of the product is
+__device__ __forceinline__ const char *row_of(const GfArgs &a, int r) {
+    size_t row = static_cast<size_t>(r);
+    if (a.row_src) {
+        const uint32_t s = a.row_src[row];
+        if (s >= static_cast<uint32_t>(a.n_src_rows)) atomicCAS(a.status, 0u, 0x903u);     // not a row of x: row 0 is read instead
+        row = s < static_cast<uint32_t>(a.n_src_rows) ? s : 0;
+    }
+    return static_cast<const char *>(a.x) + row * (static_cast<size_t>(a.K) * 2);
+}
+
+// The outputs of rows that are out of range (far_tokens.cuh), once more, by the warp that has stored them: of tiles t_lo to t_hi, two rows of x a
+// turn.
+template <int BITS, int XT, int MP>
+__device__ __noinline__ void far_rows(const GfArgs &a, const int *start, int t_lo, int t_hi) {
+    const int lane = threadIdx.x & 31, slice = (threadIdx.x >> 5) % a.ks;
+    uint32_t far = 0;
+    __syncwarp();
+    for (int tile = t_lo, pass = -1; tile < t_hi; ++tile) {
+        Tile q;
+        locate<MP>(a, start, tile, q);
+        if (q.pass != pass) far = 0;
+        for (int e = slice * 32; e < q.ntok * 16; e += 32 * a.ks)
+            for (int tok = e >> 4; tok < min((e >> 4) + 2, q.ntok); ++tok) {
+                const char *const x = row_of(a, q.tok0 + tok);
+                if (q.pass != pass && far_tokens::out_of_range<XT>(x, a.K)) far |= 1u << tok;
+                if (!(far >> tok & 1u)) continue;
+                for (int n = q.row0; n < min(q.row0 + 16, a.n_out); ++n) {
+                    const size_t row = static_cast<size_t>(q.expert) * a.n_out + n, groups = row * a.gpr * 2;
+                    const float v = far_tokens::sum<BITS, XT>(a.w[q.second] + row * a.wpr, static_cast<const char *>(a.scales[q.second]) + groups,
+                                                              static_cast<const char *>(a.biases[q.second]) + groups, x, a.K, a.gs_shift);
+                    if (lane == 0) st_from_f32(a.out[q.second], static_cast<size_t>(q.tok0 + tok) * a.n_out + n, v, XT);
+                }
+            }
+        pass = q.pass;
+    }
+}
+
 template <int BITS, int XT, int MODE, int NT>
 __global__ void __launch_bounds__(32 * kGfWarps, 2) gather_frag_kernel(const __grid_constant__ GfArgs a) {
     constexpr int RUN = MODE == G8 ? 2 : kRun<BITS>, H = MODE == G8 ? 2 : 1, CAP = kCap<MODE>, MP = CAP * NT, ESZ = 2;
@@ -58,15 +125,9 @@ __global__ void __launch_bounds__(32 * kGfWarps, 2) gather_frag_kernel(const __g
     pdl_enter();                     // the offsets, the rows
     // ---- passes: start[e] = passes before expert e ----
     int *start = reinterpret_cast<int *>(smem);
-    const auto rows_of = [&](int e, int &lo) {
-        const uint32_t p = a.offsets[e], q = a.offsets[e + 1], m = static_cast<uint32_t>(a.m_total);
-        lo = static_cast<int>(min(p, m));
-        if (p > m || q > m || q < p) atomicCAS(a.status, 0u, 0x901u);                  // clamped and reported
-        return max(static_cast<int>(min(q, m)) - lo, 0);
-    };
     for (int e = threadIdx.x; e < a.n_experts; e += 32 * kGfWarps) {
         int lo;
-        start[e + 1] = (rows_of(e, lo) + MP - 1) / MP;
+        start[e + 1] = (rows_of(a, e, lo) + MP - 1) / MP;
     }
     if (threadIdx.x == 0) start[0] = 0;
     __syncthreads();
@@ -89,26 +150,6 @@ __global__ void __launch_bounds__(32 * kGfWarps, 2) gather_frag_kernel(const __g
     const int t_lo = static_cast<int>(total * id / n_slots), t_hi = static_cast<int>(total * (id + 1) / n_slots);
     if (t_lo >= t_hi) return;        // whole slots leave: the barriers below are their own
 
-    struct Tile {
-        int pass, expert, tok0, ntok, second, row0;
-    };
-    auto locate = [&](int tile, Tile &q) {
-        q.pass = tile / a.tpe;
-        const int r = tile - q.pass * a.tpe;
-        int lo = 0, hi = a.n_experts;                                  // the last expert with start[e] <= pass: it has rows
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (start[mid] <= q.pass) lo = mid; else hi = mid;
-        }
-        q.expert = lo;
-        int first;
-        const int rows = rows_of(lo, first), done = (q.pass - start[lo]) * MP;
-        q.tok0 = first + done;
-        q.ntok = min(MP, rows - done);
-        q.second = r >= a.tpm ? 1 : 0;
-        q.row0 = (r - (q.second ? a.tpm : 0)) * 16;
-    };
-
     // ---- requests: one run of steps in registers, one run ahead of the products (see qmv_frag_kernel) ----
     const int total_runs = (a.steps + RUN - 1) / RUN, r0 = slice * total_runs / a.ks, r1 = (slice + 1) * total_runs / a.ks;
     const int n_units = MODE == G8 ? a.K >> 6 : a.K >> 5;                          // halves (G8) or chunks of a row
@@ -125,7 +166,7 @@ __global__ void __launch_bounds__(32 * kGfWarps, 2) gather_frag_kernel(const __g
     bool whole = true;
     Tile lt;
     auto open_tile = [&]() {
-        locate(l_tile, lt);
+        locate<MP>(a, start, l_tile, lt);
         const size_t row0 = static_cast<size_t>(lt.expert) * a.n_out;
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
@@ -192,24 +233,16 @@ __global__ void __launch_bounds__(32 * kGfWarps, 2) gather_frag_kernel(const __g
         static_assert(32 % (4 * MP) == 0, "a lane stages one token");
         const int em = (lane >> 2) % MP, et = lane & 3, n = (r1 - r0) * RUN * 4 * MP;
         RowX rx{a.x, a.K, em < q.ntok ? 1 : 0};
-        if (rx.M) {
-            size_t row = static_cast<size_t>(q.tok0 + em);
-            if (a.row_src) {
-                const uint32_t r = a.row_src[row];
-                if (r >= static_cast<uint32_t>(a.n_src_rows)) atomicCAS(a.status, 0u, 0x903u);     // not a row of x: row 0 is read instead
-                row = r < static_cast<uint32_t>(a.n_src_rows) ? r : 0;
-            }
-            rx.x = static_cast<const char *>(a.x) + row * (static_cast<size_t>(a.K) * ESZ);
-        }
+        if (rx.M) rx.x = row_of(a, q.tok0 + em);
         for (int e0 = 0; e0 < n; e0 += 32) {
             const int e = e0 + lane, es = (e >> 2) / MP, k = (r0 * RUN + es) * 128;
             float sum = 0.0f;
             if (e < n)
-                sum = stage_chunk<BITS, XT, MODE>(rx, 0, MODE == G8 ? k + 16 * et : k + 32 * et, MODE == G8 ? k + 64 + 16 * et : k + 32 * et + 16,
+                sum = stage_chunk<BITS, XT, MODE, far_tokens::kUp>(rx, 0, MODE == G8 ? k + 16 * et : k + 32 * et, MODE == G8 ? k + 64 + 16 * et : k + 32 * et + 16,
                                                   part + static_cast<size_t>(e) * kPitch<XT>);
             if (MODE != G8) {
-                // in the units of the products: x times 2^64 against codes times 2^-133, f16: codes times 2^-24
-                constexpr uint32_t unit = (XT == MTC_F16 ? 127u - 24u : 127u - 69u) << 23;
+                // in the units of the products: x times 2^kUp against codes times 2^-133, f16: codes times 2^-24
+                constexpr uint32_t unit = (XT == MTC_F16 ? 127u - 24u : 127u - far_tokens::kUnit) << 23;
                 if (MODE == S4) sum += __shfl_xor_sync(0xffffffffu, sum, 1);                       // chunks 0 and 1, 2 and 3
                 const uint32_t at = (em / CAP) * 32 + (MODE == S2 ? et * 8 : (et >> 1) * 16) + (em % CAP) * 4;
                 if (e < n && (MODE != S4 || !(et & 1))) *reinterpret_cast<float *>(sums + es * SUM + at) = sum * __uint_as_float(unit);
@@ -231,12 +264,13 @@ __global__ void __launch_bounds__(32 * kGfWarps, 2) gather_frag_kernel(const __g
     };
 
     // ---- tiles ----
-    const float post = XT == MTC_F16 ? __uint_as_float((127u + 24u) << 23) : __uint_as_float((127u + 69u) << 23);
+    const float post = XT == MTC_F16 ? __uint_as_float((127u + 24u) << 23) : __uint_as_float((127u + far_tokens::kUnit) << 23);
     float *const red = reinterpret_cast<float *>(smem + a.off_red) + slot * a.ks * (2 * MP * 16);     // [buffer][warp of the slot][token][row]
     int staged = -1, buf = 0;
+    bool odd = false;                // a sum that this lane has stored may be of a row out of range (far_tokens.cuh)
     for (int tile = t_lo; tile < t_hi; ++tile) {
         Tile q;
-        locate(tile, q);
+        locate<MP>(a, start, tile, q);
         if (q.pass != staged) {
             stage(q);
             staged = q.pass;
@@ -305,10 +339,14 @@ __global__ void __launch_bounds__(32 * kGfWarps, 2) gather_frag_kernel(const __g
             const float *base = red + buf * a.ks * (MP * 16) + e;
             float v = base[0];
             for (int s = 1; s < a.ks; ++s) v += base[s * (MP * 16)];
-            if (q.row0 + row < a.n_out) st_from_f32(a.out[q.second], static_cast<size_t>(q.tok0 + tok) * a.n_out + q.row0 + row, v * post, XT);
+            if (q.row0 + row < a.n_out) {
+                st_from_f32(a.out[q.second], static_cast<size_t>(q.tok0 + tok) * a.n_out + q.row0 + row, v * post, XT);
+                odd = odd || far_tokens::odd<XT>(v);
+            }
         }
         buf ^= 1;
     }
+    if (__any_sync(0xffffffffu, odd)) far_rows<BITS, XT, MP>(a, start, t_lo, t_hi);
 }
 
 // ---- host side -----------------------------------------------------------------------------------------------------

@@ -27,6 +27,7 @@
 #include <cuda.h>
 
 #include "common.cuh"
+#include "far_tokens.cuh"
 #include "qmv_frag.cuh"
 
 namespace mtc {
@@ -153,7 +154,7 @@ __device__ __forceinline__ float stage_unit(const XUnit<XT, LC> &v, uint32_t dst
         uint32_t o[3][4];
 #pragma unroll
         for (int r = 0; r < LC / 2; ++r) {
-            const float sc = __uint_as_float(static_cast<uint32_t>(127 + 64 - frag::field_pos<BITS, true>(r)) << 23);
+            const float sc = __uint_as_float(static_cast<uint32_t>(127 + far_tokens::kUp - frag::field_pos<BITS, true>(r)) << 23);
             float lo = __uint_as_float(v.r[frag::code_lo<BITS>(r)]) * sc, hi = __uint_as_float(v.r[frag::code_hi<BITS>(r)]) * sc;
 #pragma unroll
             for (int p = 0; p < 3; ++p) {
@@ -178,14 +179,48 @@ __device__ __forceinline__ float stage_unit(const XUnit<XT, LC> &v, uint32_t dst
         for (int r = 0; r < LC / 2; ++r) {
             const int lo = frag::code_lo<BITS>(r), hi = frag::code_hi<BITS>(r);
             uint32_t b = __byte_perm(v.r[lo >> 1], v.r[hi >> 1], ((lo & 1) ? 0x32 : 0x10) | ((hi & 1) ? 0x7600 : 0x5400));
-            if (XT == MTC_BF16) {         // times 2^(64 - pos): exact, subnormals included (inf beyond 2^63)
-                const uint32_t e = static_cast<uint32_t>(127 + 64 - frag::field_pos<BITS, true>(r)) << 7;
+            if (XT == MTC_BF16) {         // times 2^(kUp - pos): exact, subnormals included
+                const uint32_t e = static_cast<uint32_t>(127 + far_tokens::kUp - frag::field_pos<BITS, true>(r)) << 7;
                 asm("mul.rn.bf16x2 %0, %0, %1;" : "+r"(b) : "r"(e * 0x10001u));
             }
             o[r & 3] = b;
             if ((r & 3) == 3) sts16((dst + ((r >> 2) << 4)) ^ flip, o[0], o[1], o[2], o[3]);
         }
         return 0.0f;
+    }
+}
+
+// The outputs of tokens that are out of range, once more: by the warps that have stored them (the tiles of every pass as in the kernel).
+// far: shared memory that nothing uses any more.
+template <int BITS, int XT>
+__device__ __noinline__ void far_outputs(const CluArgs &a, uint32_t *far) {
+    constexpr int ESZ = XT == MTC_F32 ? 4 : 2;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, cs = 1 << a.cs_shift, cr = blockIdx.x & (cs - 1), cid = static_cast<int>(blockIdx.x) >> a.cs_shift;
+    const int t_lo = cid * a.per + min(cid, a.per_more), t_n = a.per + (cid < a.per_more);
+    const auto token = [&](int t) { return static_cast<const char *>(a.x) + static_cast<size_t>(t) * a.K * ESZ; };
+    if (warp < a.M) {                                                              // as many warps as tokens
+        const uint32_t is = far_tokens::out_of_range<XT>(token(warp), a.K);
+        if (lane == 0) far[warp] = is;
+    }
+    __syncthreads();
+    for (int t = 0; t < a.M; ++t) {
+        if (far[t] == 0) continue;
+        for (int pass = 0; pass < a.passes; ++pass) {
+            const int ta = t_lo + t_n * pass / a.passes, tb = t_lo + t_n * (pass + 1) / a.passes;
+            for (int tile = ta + cr * kWarps + warp; tile < tb; tile += cs * kWarps) {
+                int pi = 0;
+                for (int j = 1; j < a.n_proj; ++j)
+                    if (tile >= a.p[j].tile0) pi = j;
+                const FragProj &pr = a.p[pi];
+                const int n0 = (tile - pr.tile0) * 16;
+                for (int n = n0; n < min(n0 + 16, pr.N); ++n) {
+                    const size_t row = static_cast<size_t>(n), groups = row * a.s_pitch;
+                    const float o = far_tokens::sum<BITS, XT>(pr.w + row * (a.K / 32 * BITS), static_cast<const char *>(pr.scales) + groups,
+                                                              static_cast<const char *>(pr.biases) + groups, token(t), a.K, a.gs_shift);
+                    if (lane == 0) st_from_f32(pr.out, static_cast<size_t>(t) * pr.N + n, o, XT);
+                }
+            }
+        }
     }
 }
 
@@ -311,7 +346,7 @@ __global__ void __launch_bounds__(32 * kWarps, 1) qmv_cluster_kernel(const __gri
         if constexpr (XT == MTC_F32) {
             sum += __shfl_xor_sync(0xffffffffu, sum, 1);
             sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-            if (t == 0) *reinterpret_cast<float *>(sums_p + (s * MP + tok) * 4) = sum * __uint_as_float((127u - 69u) << 23);      // in the units of the products
+            if (t == 0) *reinterpret_cast<float *>(sums_p + (s * MP + tok) * 4) = sum * __uint_as_float((127u - far_tokens::kUnit) << 23);      // in the units of the products
         } else {                              // the sums in the units of the products: against codes that are all one
             __syncwarp();
             float d[4];
@@ -333,7 +368,9 @@ __global__ void __launch_bounds__(32 * kWarps, 1) qmv_cluster_kernel(const __gri
     __syncthreads();
 
     // ---- products ----
-    const float post = XT == MTC_F16 ? __uint_as_float((127u + 24u) << 23) : __uint_as_float((127u + 69u) << 23);
+    uint32_t *const odd = reinterpret_cast<uint32_t *>(smem + a.off_bar + W * kDepth * 8);         // a result may be of a token out of range
+    if (threadIdx.x == 0) *odd = 0;                                                // (far_tokens.cuh); set behind the barrier of a pass
+    const float post = XT == MTC_F16 ? __uint_as_float((127u + 24u) << 23) : __uint_as_float((127u + far_tokens::kUnit) << 23);
     // Row r of a unit is UB lines of 128 bytes; TMA stores 16-byte chunk c of line l at c ^ (l & 7): the rows a load phase reads (two
     // of 64 bytes, four of 32, eight of 16) fall on different banks.
     uint32_t w_lane[UB];
@@ -486,13 +523,17 @@ __global__ void __launch_bounds__(32 * kWarps, 1) qmv_cluster_kernel(const __gri
                 const float o[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
-                    if (nn < pr.N && tok + j < a.M) st_from_f32(pr.out, static_cast<size_t>(tok + j) * pr.N + nn, o[j] * post, XT);
+                    if (nn < pr.N && tok + j < a.M) {
+                        st_from_f32(pr.out, static_cast<size_t>(tok + j) * pr.N + nn, o[j] * post, XT);
+                        if (XT != MTC_F16 && far_tokens::odd<XT>(o[j])) *odd = 1;
+                    }
             }
         }
         // no partial tile is rewritten, and no CTA leaves, while another reads it
         if (cs > 1) cluster_sync();
-        else if (pass + 1 < a.passes) __syncthreads();
+        else if (pass + 1 < a.passes || XT != MTC_F16) __syncthreads();
     }
+    if (XT != MTC_F16 && *odd != 0) far_outputs<BITS, XT>(a, reinterpret_cast<uint32_t *>(smem));
 }
 
 // ---- host side -----------------------------------------------------------------------------------------------------
@@ -524,7 +565,7 @@ inline Plan make_plan(int tiles, int units, int pieces, int us, uint32_t xseg, i
         p.off_sum = W * kDepth * slot + p.plane * pieces;
         p.off_scale = (p.off_sum + static_cast<uint32_t>(nu) * us * mp * 4 + 15) / 16 * 16;
         p.off_bar = p.off_scale + W * kDepth * sslot;
-        p.off_red = (p.off_bar + W * kDepth * 8 + 127) / 128 * 128;
+        p.off_red = (p.off_bar + W * kDepth * 8 + 4 + 127) / 128 * 128;           // barriers, a word on the results
         if (p.off_red > kSmemMax) continue;
         p.clusters = cs <= 2 ? sms / cs : cs == 4 ? sms * 33 / 148 : sms * 15 / 148;       // what fits the GPCs at once
         if (p.clusters > tiles) p.clusters = tiles;

@@ -260,7 +260,7 @@ template <int XT>
 constexpr int kPitch = 64 * kPieces<XT> + 16;
 
 // Returns the sum of the 32 activations (not for G8, whose two halves have sums of their own).
-template <int BITS, int XT, int MODE, typename A>              // A: x, K, M of the rows
+template <int BITS, int XT, int MODE, int UP = 64, typename A>              // bf16: x times 2^UP; A: x, K, M of the rows
 __device__ __forceinline__ float stage_chunk(const A &a, int m, int k_lo, int k_hi, char *dst) {
     // k_lo: first activation of registers 0-7, k_hi: of registers 8-15 (16 values each; both inside or outside the row)
     constexpr bool BF = XT != MTC_F16;
@@ -281,7 +281,7 @@ __device__ __forceinline__ float stage_chunk(const A &a, int m, int k_lo, int k_
         uint32_t o[3][4];
 #pragma unroll
         for (int r = 0; r < 16; ++r) {
-            const float sc = __uint_as_float(static_cast<uint32_t>(127 + 64 - field_pos<BITS, true>(r)) << 23);
+            const float sc = __uint_as_float(static_cast<uint32_t>(127 + UP - field_pos<BITS, true>(r)) << 23);
             float lo = v[code_lo<BITS>(r)] * sc, hi = v[code_hi<BITS>(r)] * sc;
 #pragma unroll
             for (int p = 0; p < 3; ++p) {
@@ -325,8 +325,8 @@ __device__ __forceinline__ float stage_chunk(const A &a, int m, int k_lo, int k_
         for (int r = 0; r < 16; ++r) {
             const int lo = code_lo<BITS>(r), hi = code_hi<BITS>(r);
             uint32_t b = __byte_perm(u[lo >> 1], u[hi >> 1], ((lo & 1) ? 0x32 : 0x10) | ((hi & 1) ? 0x7600 : 0x5400));
-            if (BF) {                     // times 2^(64 - pos): exact, subnormals included (inf beyond 2^63)
-                const uint32_t e = static_cast<uint32_t>(127 + 64 - field_pos<BITS, true>(r)) << 7;
+            if (BF) {                     // times 2^(UP - pos): exact, subnormals included (inf beyond 2^(127 - UP))
+                const uint32_t e = static_cast<uint32_t>(127 + UP - field_pos<BITS, true>(r)) << 7;
                 asm("mul.rn.bf16x2 %0, %0, %1;" : "+r"(b) : "r"(e * 0x10001u));
             }
             o[r & 3] = b;
