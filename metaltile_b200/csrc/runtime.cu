@@ -213,10 +213,16 @@ inline bool frag_rule(int M, long long N, int K, int bits, int group_size, int d
 //     rows: 2-bit 71 -> 42, 75 -> 71; 8-bit 72 -> 53, 74 against 84; 32 of 896 x 512, 9.5 rows, 6-bit 75 -> 56.
 //   against the streaming kernel, 128 experts of 2048 x 768, 0.06 / 0.25 / 0.5 / 0.75 rows: 38.7 -> 28.2, 52.4 -> 47.5, 67.8 -> 67.2, 79 against 89; 16 of
 //     1024 x 512 (8 Mi codes), 1 / 4 rows: 30 -> 22, 32 -> 26.
-inline bool gather_frag_rule(int m_total, int n_out, int k_in, int n_experts, bool streamed) {
+// The mean says nothing of how the rows fall: where a few experts get most of them, the tcgen05 kernel converts a few matrices and the passes
+// stay (router logits N(0, 1), plus a bias of the expert of N(0, 1), of N(0, 4); 128 experts of 2048 x 768): groups of 64, 8-bit, 2 rows 1.31 / 1.15 / 1.04
+// times as fast, 4 rows 1.15 / 0.97 / 0.90; 5- and 6-bit, 4 rows 1.3 / 1.06 / 0.96; the streaming kernel's, 0.5 rows 1.02 / 0.94 / 0.87.  With groups of 32,
+// where a pass costs more, 8-bit, 2 rows 1.19 / 1.05 / 0.95, 2.5 rows 0.96 / 0.95 / 0.94, 4 rows 0.97 / 0.82 / 0.76; 4-bit, 3 rows 1.14 / 1.04 / 1.00, 4
+// rows 1.16 / 0.96 / 0.88; 3-bit 1.07 / 0.96 / 0.91 and 1.08 / 0.88 / 0.81.
+inline bool gather_frag_rule(int m_total, int n_out, int k_in, int n_experts, int bits, int group_size, bool streamed) {
     const long long codes = static_cast<long long>(n_experts) * n_out * k_in, rows = m_total, experts = n_experts;
     if (streamed) return 2 * rows <= experts || (rows <= 4 * experts && codes <= (16ll << 20));
-    return rows <= 4 * experts || (rows <= 10 * experts && codes <= (32ll << 20));
+    if (codes <= (32ll << 20)) return rows <= 10 * experts;
+    return rows <= (group_size % 64 == 0 ? 4 : bits == 8 ? 2 : 3) * experts;
 }
 // rows: weight rows of the launch (N, or those of all fused projections)
 inline bool frag_takes(const Ctx *ctx, int M, long long rows, bool fused, int N, int K, int bits, int group_size, int dt, const void *w, const void *scales,
@@ -1167,7 +1173,7 @@ static bool gather_stream_takes(const Ctx *ctx, bool csr, int m_total, int n_out
 static bool gather_frag_takes(const Ctx *ctx, bool csr, int m_total, int n_out, int k_in, int n_experts, int bits, int group_size, int dtype,
                               const void *w, const void *scales, const void *biases, const void *x) {
     return csr && (!ctx || ctx->gather_stream) &&
-           gather_frag_rule(m_total, n_out, k_in, n_experts,
+           gather_frag_rule(m_total, n_out, k_in, n_experts, bits, group_size,
                             gather_stream_takes(ctx, csr, m_total, n_out, k_in, n_experts, bits, group_size, dtype, w, scales, biases, x)) &&
            mtc::gather_frag_supported(m_total, n_out, k_in, n_experts, bits, group_size, dtype, w, scales, biases, x);
 }

@@ -4,8 +4,8 @@ import random
 
 import pytest
 
-from metaltile_b200 import MetalTileError
-from metaltile_b200.context import launch_of
+from metaltile_b200 import MetalTileError, _lib
+from metaltile_b200.context import _dt, launch_of
 from test_cluster_gpu import CASES, PASSES, SHORT
 from test_qmm_cluster_gpu import CASES as SLICED
 
@@ -36,6 +36,13 @@ def test_forms():
         assert form["kernel"] == "qmm_tcgen05" and form["cluster"] == form["k_slices"] >= 2 and form["ctas"] % form["cluster"] == 0
     with pytest.raises(MetalTileError):
         launch_of(1, [64] * 5, 64, 4, 64, "bf16")
+
+
+@pytest.mark.parametrize("bits,group,most", [(8, 64, 512), (6, 128, 512), (8, 32, 256), (4, 32, 384), (3, 32, 384)])
+def test_rows_an_expert_of_the_grouped_fragment_kernel(bits, group, most):
+    route = lambda m, n, k, e: _lib.load().mtc_gather_qmm_route(m, n, k, e, bits, group, _dt("bf16")).decode()  # noqa: E731
+    assert [route(m, 768, 2048, 128) for m in (most, most + 1)] == ["gather_qmm_frag", "gather_qmm_tcgen05"]
+    assert [route(m, 768, 1024, 32) for m in (320, 321)] == ["gather_qmm_frag", "gather_qmm_tcgen05"]      # up to 32 Mi codes
 
 
 def _walk(ns, k, m, bits, g, dt):
