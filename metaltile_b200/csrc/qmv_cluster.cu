@@ -53,6 +53,9 @@ bool supported(const mtc_qmv_desc &d) {
 //     21.5; groups of 32 4096 x 4096, 8 tokens 9.4 -> 6.9).
 //   8-bit, 16-bit activations: from 16 Mi codes on, from nine tokens on from 12 Mi (8192 x 8192, 8 tokens 23.6 -> 17.0, 14336 x 2048, 16 tokens 16.7
 //     -> 11.9; 2048 x 2048 3.8 = 3.9, 5120 x 3072 7.0 against 7.9), with groups of 32 always (2048 x 2048 4.8 -> 4.4).
+//   4-bit from nine tokens on where K is an odd multiple of 256 (the fragment kernel had these) and no CTA has more than a tile: neither for
+//     K = 1792 to 3840, where its few warps walk all of K (477 x 3840 5.3 against 6.3, 865 x 2816 4.5 against 5.1, 2048 x 2304 4.8 against 5.0; 865 x
+//     1280 and 4352 and 4096 x 2816 are faster here).
 static bool takes(const mtc_qmv_desc *d, int n, int sms, clu::Plan &plan) {
     long long codes = 0;
     int tiles = 0;
@@ -62,6 +65,7 @@ static bool takes(const mtc_qmv_desc *d, int n, int sms, clu::Plan &plan) {
         tiles += (d[i].N + 15) / 16;
     }
     if (d[0].bits == 8 && d[0].dtype != MTC_F32 && d[0].group_size != 32 && codes < ((d[0].M <= 8 ? 16ll : 12ll) << 20)) return false;
+    if (d[0].bits == 4 && d[0].dtype != MTC_F32 && d[0].M > 8 && d[0].K % 512 != 0 && d[0].K > 1536 && d[0].K < 4096 && tiles <= sms) return false;
     plan = clu::shape_plan(d[0], tiles, sms);
     return plan.shift >= 0;          // a part of K that shared memory cannot hold: no plan
 }

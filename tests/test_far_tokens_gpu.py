@@ -34,7 +34,7 @@ def _check(torch, got, x, q, b, groups, dt):
 
 
 @pytest.mark.parametrize("n,k,m,bits,g,dt", [
-    (100, 2048, 8, 4, 64, "bf16"), (601, 14336, 7, 4, 64, "bf16"), (333, 2816, 12, 4, 256, "bf16"), (9000, 4096, 16, 4, 128, "bf16"), (777, 1024, 6, 8, 32, "bf16"),
+    (100, 2048, 8, 4, 64, "bf16"), (601, 14336, 7, 4, 64, "bf16"), (3999, 2816, 12, 4, 256, "bf16"), (9000, 4096, 16, 4, 128, "bf16"), (777, 1024, 6, 8, 32, "bf16"),
     (300, 7168, 16, 4, 64, "f32"), (100, 1280, 7, 8, 64, "f32"), (2100, 5888, 16, 4, 64, "bf16"), (100, 1024, 6, 4, 512, "bf16")])
 def test_cluster_kernel(n, k, m, bits, g, dt):
     import torch
