@@ -269,7 +269,8 @@ int mtc_peer_barrier(mtc_ctx *ctx, void *stream, void *const *peer_flags, int n_
  *                      would leave SMs idle in the last round, K is cut into up to 16 slices that run as work items of
  *                      their own, as the plan with the shortest estimated time says; f32 partial sums - 512 MiB at most - in a
  *                      context scratch block are added in slice order by a second kernel - deterministic, same products.
- *                      Where that block cannot grow, M > 16 runs without slices)
+ *                      Where that block cannot grow, M > 16 runs without slices.  Slices of one round may instead be the CTAs of a
+ *                      cluster each and add up in shared memory, without block or second kernel)
  *   "qmv_small_m_tc"   2 <= M <= 16 on shapes the warp-level kernels do not take (other widths than 4-bit, group 32):
  *                      1 (default) 9 <= M <= 16, and 5 <= M <= 8 on matrices of 32 Mi codes or more, run on the
  *                      tensor-core kernel (f16 / bf16, K % 64 == 0, power-of-two group >= 32) instead of one FFMA per
@@ -287,8 +288,8 @@ int mtc_peer_barrier(mtc_ctx *ctx, void *stream, void *const *peer_flags, int n_
  *                      and 128); everything else up to M = 4, up to M = 8 while K <= 8192 or below 32 Mi codes, and from
  *                      M = 9 on groups that are multiples of 64 with K <= 5120 up to 20 Mi codes (fused: 128 Mi); f32
  *                      activations from M = 5 on - unless
- *                      "qmv_stream", "qmv_small_m_mma" or "qmv_small_m_tc" selects another kernel; from M = 5 on 4-bit codes, f32 activations and large 8-bit matrices run as
- *                      clusters that split K (csrc/qmv_cluster.cuh) in its place; 2 itself whenever it supports
+ *                      "qmv_stream", "qmv_small_m_mma" or "qmv_small_m_tc" selects another kernel; from M = 5 on 4-bit codes, f32 activations and large 8-bit matrices run on
+ *                      the cluster kernel (csrc/qmv_cluster.cuh) in its place; 2 itself whenever it supports
  *                      the shape (M <= 16, K % 32 == 0, power-of-two group >= 32, 16-byte aligned w and x); 0 never
  *   "qmv_tc"           1: those shapes run on the tensor-memory decode kernel instead (slower today; default 0)
  *   "gather_stream"    0: grouped products never take the weight-streaming kernel (default 1: the CSR form with

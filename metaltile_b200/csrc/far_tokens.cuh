@@ -5,8 +5,8 @@
 // other sign (with f16 operands, which have none of the other limits, too).  Every result says which it may be: an infinity or a NaN comes out
 // as one, and what has lost bits is tiny (sums err by 2^-139 units at most; a result of 2^-110 and more has its 24 bits all the same).  So
 // the kernels that took over from ones that scale every row by itself look at the sums that they store.  Where one is odd, they look for
-// tokens that are out of range and add those up from the definition, a warp an output (28672 x 4096, 8 tokens: 15 us, one of them out of range
-// 320, a NaN 18).  With x times 2^96 that is a token with a value from 2^31 on, or all of them below 2^-64; one whose results all come out as zero, where
+// tokens that are out of range and add those up from the definition, a warp an output (28672 x 4096 from L2, 8 tokens: 15 us, one of them out
+// of range 320, a NaN 18).  With x times 2^96 that is a token with a value from 2^31 on, or all of them below 2^-64; one whose results all come out as zero, where
 // its values lie below 2^-112, is left as it is.  (Noting the largest value of every token while it is staged costs 0.2 us a launch of 15, and
 // looking for tokens behind every result of zero 2 to 4, with each token of zeros that fills up a batch.)
 #pragma once

@@ -47,15 +47,20 @@ bool supported(const mtc_qmv_desc &d) {
 
 }  // namespace
 
-// Whether one launch of this kernel takes the projections (M >= 2), and is the faster one (us, the kernel it took over from -> this one):
+// Whether one launch of this kernel takes the projections (M >= 2), and is the faster one (us, the kernel it took over from -> this one), among
+// those that the entries offer it (cluster_first and frag_rule, runtime.cu): from nine tokens on they keep groups of 32, single 8-bit matrices
+// above 20 Mi codes or of K > 5120, and at five to eight 8-bit ones of K > 8192 from 32 Mi codes on for the tcgen05 kernel, unmeasured against this one.
 //   f32 activations: always (8-bit 4096 x 4096, 8 / 16 tokens 15.0 -> 10.7 / 28.1 -> 15.2; 8192 x 8192 4-bit 60 -> 21 / 118 -> 35).
 //   4-bit: always (4096 x 4096, 8 / 16 tokens 6.3 -> 5.9 / 10.2 -> 9.0, 28672 x 4096 21.8 -> 16.6 / 28.8 -> 25.1, 4096 x 14336 17.4 -> 13.7 / 29.2 ->
 //     21.5; groups of 32 4096 x 4096, 8 tokens 9.4 -> 6.9).
-//   8-bit, 16-bit activations: from 16 Mi codes on, from nine tokens on from 12 Mi (8192 x 8192, 8 tokens 23.6 -> 17.0, 14336 x 2048, 16 tokens 16.7
-//     -> 11.9; 2048 x 2048 3.8 = 3.9, 5120 x 3072 7.0 against 7.9), with groups of 32 always (2048 x 2048 4.8 -> 4.4).
-//   4-bit from nine tokens on where K is an odd multiple of 256 (the fragment kernel had these) and no CTA has more than a tile: neither for
+//   8-bit, 16-bit activations: from 16 Mi codes on, from nine tokens on from 12 Mi (8192 x 8192, 8 tokens 23.6 -> 17.0, 14336 x 2048 as part of a
+//     fused launch, 16 tokens 16.7 -> 11.9; 2048 x 2048 3.8 = 3.9, 5120 x 3072 7.0 against 7.9), with groups of 32 always (2048 x 2048, 8 tokens
+//     4.8 -> 4.4).
+//   4-bit from nine tokens on where K is an odd multiple of 256 (the fragment kernel had these) and no CTA has more than a tile: not for
 //     K = 1792 to 3840, where its few warps walk all of K (477 x 3840 5.3 against 6.3, 865 x 2816 4.5 against 5.1, 2048 x 2304 4.8 against 5.0; 865 x
 //     1280 and 4352 and 4096 x 2816 are faster here).
+// A call costs the host 0.2 us more than the ring kernel before it did (a tensor map a projection): products too small to hide it, 4-bit of 1 Mi
+// codes, go from 4.4 to 4.6 us a call, though not in a graph (1247 x 512, 12 tokens 3.37 -> 2.95; 602 x 2560, 5 tokens 3.70 -> 3.43).
 static bool takes(const mtc_qmv_desc *d, int n, int sms, clu::Plan &plan) {
     long long codes = 0;
     int tiles = 0;

@@ -1,4 +1,5 @@
-// qmv_cluster — quantized products of 5 to 16 token rows: 4- and 8-bit codes, K split over a cluster of CTAs where it is long.
+// qmv_cluster — quantized products of 5 to 16 token rows: 4- and 8-bit codes, the activations staged once an SM; K split over a cluster of CTAs
+// where their rows are too long for that (one CTA by itself is the usual launch).
 //
 //   out[m, n] = sum_k (q(n,k) * scale[n, k/G] + bias[n, k/G]) * x[m, k]      1 <= M <= 16, f32 accumulation
 //
@@ -17,7 +18,7 @@
 //     one, and no barrier stands between tiles.  A warp leaves one partial tile for every tile that its share touches; they are added at the
 //     end in the order of K (deterministic).
 //
-// What bounds it (28672 x 4096, 8 tokens: 16.6 us, 66 MB): the ring alone streams at 5.6 TB/s (11.8 us with its launch); the products take 4 us
+// What bounds it (28672 x 4096, 8 tokens: 16.6 us, 66 MB; 17.6 where every fourth launch drains, as in the profile of its counters): the ring alone streams at 5.6 TB/s (11.8 us with its launch); the products take 4 us
 // that the stream does not hide (43 instructions a 64-code segment of 16 rows where the stream leaves 100 issue slots, at 16 warps'
 // latency), staging the activations 1.5, the last sum and the stores 1.  Taken back: rings of 3 and 4 units (the partial tiles lose their room
 // and a launch takes two passes: 25 -> 30 us at 16 tokens), every 16th unit to a warp instead of a run of them (partial tiles: five passes,

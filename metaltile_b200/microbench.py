@@ -69,7 +69,7 @@ def main(argv=None):
     if a.family == "sweep":
         # the sweep grid of the qmv family: every cell cycles enough weight copies to exceed L2 twice over
         hbm = 6552.3
-        print("bits group M KN us GB/s frac_of_6552", flush=True)
+        print("bits group M KN us GB/s frac_of_6552 kernel", flush=True)
         for kn in (2048, 4096, 8192):
             for bits in (2, 3, 4, 6, 8):
                 for group in (32, 64, 128):
@@ -104,7 +104,8 @@ def main(argv=None):
                         torch.cuda.synchronize()
                         us = e0.elapsed_time(e1) * 1e3 / (a.reps * copies)
                         tot = nbytes + 2 * m * kn * dt.itemsize
-                        print(f"{bits} {group} {m} {kn} {us:.2f} {tot / us / 1e3:.0f} {tot / us / 1e3 / hbm:.3f}", flush=True)
+                        kernel = ctx.launch_of(m, [kn], kn, bits, group, a.dtype)["kernel"]
+                        print(f"{bits} {group} {m} {kn} {us:.2f} {tot / us / 1e3:.0f} {tot / us / 1e3 / hbm:.3f} {kernel}", flush=True)
                         del graph
                     del sets
                     torch.cuda.empty_cache()

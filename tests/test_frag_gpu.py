@@ -62,7 +62,7 @@ def test_rounds_and_blocks(ctx, m, n, k, bits, gs, dt):
 def test_projections_in_one_launch_equal_separate_ones(ctx, m, k, bits, gs):
     """Rows that end inside a tile in the middle of the launch: every projection has its own tiles.  With so few tiles the launch
     splits K over its warps as each of the separate ones does, so the results are theirs bit for bit (M = 5 to 16 with 4-bit
-    codes on the ring kernel, else the fragment kernel); with more tiles the splits may differ, see the next test."""
+    codes on the cluster kernel, else the fragment kernel); with more tiles the splits may differ, see the next test."""
     import torch
     from metaltile_b200 import ops
     mats = []

@@ -179,7 +179,7 @@ def test_shapes_and_edges(m, n, k, bits, gs, dt):
     (12, 8, 128, 64, "bf16"),                                   # fewer rows than one 16-row tile
 ])
 def test_small_m_tensor_core_path(ctx, m, n, k, gs, dt):
-    """2 <= M <= 16 with 4-bit codes runs on warp-level MMAs (the register / cp.async ring kernels of qmv_mma.cu once
+    """2 <= M <= 16 with 4-bit codes runs on warp-level MMAs (the cluster kernel or qmv_mma.cu once
     the streaming kernel is switched off); same oracle, and within round-off of the CUDA-core kernel for the same call."""
     assert ctx.qmm_route(m, n, k, 4, gs, dt) in ("qmv_mma_sync", "qmv_stream")
     w, s, b, x = dense_case(m, n, k, 4, gs, dt, seed=6, salt=m * 31 + n)
@@ -370,9 +370,9 @@ def test_rms_norm_qmv_typed(ctx, n, k, gs, dt):
     assert rel_err(got.float().cpu().numpy(), ref) <= TOL[dt]
 
 
-@pytest.mark.parametrize("m,frag", [(2, 0), (2, 1), (5, 1), (16, 1)])      # 2 tokens: the ring kernel where the fragment kernel is off
+@pytest.mark.parametrize("m,frag", [(2, 0), (2, 1), (5, 1), (16, 1)])      # 2 tokens: the cluster kernel where the fragment kernel is off
 def test_small_m_tensor_core_path_special_activations(ctx, m, frag):
-    """The ring kernel stages bf16 activations times 2^64 (and x / 16 for the nibbles at bits 4-7): zeros of both signs,
+    """The kernels stage bf16 activations times a power of two (less for the nibbles at bits 4-7): zeros of both signs,
     bf16 subnormals, tiny and large magnitudes must come through exactly."""
     import torch
     from metaltile_b200 import ops

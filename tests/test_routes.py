@@ -17,7 +17,7 @@ def kernel(m, n, k, bits, group, dt):
     ((1, 4096, 4096, 4, 64, "bf16"), FRAG), ((1, 16384, 16384, 4, 64, "f16"), FRAG), ((1, 64, 512, 8, 32, "bf16"), FRAG),
     ((1, 8192, 8192, 3, 64, "bf16"), FRAG), ((1, 8224, 8192, 3, 64, "bf16"), CUDA), ((1, 16384, 16384, 2, 64, "f16"), CUDA),
     ((1, 4096, 4096, 6, 128, "f16"), FRAG), ((1, 4096, 4096, 5, 64, "bf16"), CUDA), ((1, 4096, 4096, 4, 64, "f32"), CUDA),
-    # 4 bits, the ring kernel's shapes: up to four tokens, groups of 64 and 128
+    # 4 bits, K % 512 == 0: up to four tokens, groups of 64 and 128
     ((2, 4096, 4096, 4, 64, "bf16"), FRAG), ((4, 4096, 4096, 4, 128, "bf16"), FRAG), ((5, 4096, 4096, 4, 64, "bf16"), RING),
     ((16, 4096, 4096, 4, 64, "bf16"), RING), ((2, 4096, 4096, 4, 256, "bf16"), RING),
     # ... and where that kernel does not go: K % 512, groups of 32
