@@ -1339,8 +1339,12 @@ constexpr double kKbBase = 0.47, kKbPerToken = 0.0006;
 constexpr double kWideBase = 0.45, kWidePerToken = 0.00075;      // an item of two chunks
 constexpr double kSliceUs = 2e-6;       // an f32 partial sum: written at ~3 TB/s, read at ~6
 // Clusters of one to eight CTAs, one CTA an SM, that are resident at once (cudaOccupancyMaxActiveClusters: the GPCs do not divide evenly)
-constexpr int kClusters[9] = {0, 148, 74, 45, 33, 26, 22, 15, 15};
-constexpr double kClusterUs = 5.5;      // their launch and barriers, and the sum: 128 x 2048 x 2048 took 12.4 us with them where two kernels take 10.5
+// (45 of three are, but with all of them at once products of x in bf16 took 1.1 to 1.2 times as long as with 44)
+constexpr int kClusters[9] = {0, 148, 74, 44, 33, 26, 22, 15, 15};
+constexpr double kClusterUs = 5.5;      // what a cluster's launch, barriers and sum cost at least
+// What launches take beyond the prices above, us over the leanest (means of 520 shapes of 17 to 1300 tokens, every format, sliced in memory and in
+// clusters in turn): the clusters of S CTAs, the pairs of two-chunk items, and the plans of 1, 2, 3, 4 and more slices without clusters
+constexpr double kClusterMore[9] = {0, 0, 4.5, 4.0, 2.0, 3.5, 4.0, 4.0, 3.0}, kWidePairMore = 7.5, kSlicedMore[6] = {0, 2, 4, 2, 1, 0};
 constexpr double kItemUs = 0.4;         // a further item on the same SM: its accumulators drain before the next pair starts
 
 // How a dense launch covers its M token rows: items of one chunk (TN rows, one accumulator) or of two (the dequantised W stage
@@ -1395,10 +1399,15 @@ DensePlan plan_dense(const Ctx *ctx, int M, int N, int K, int bits, bool slices 
         }
     }
     // ... or slices that are the CTAs of a cluster each and add up in shared memory: no block, no second kernel, but units of a round that the
-    // GPCs' odd sizes leave room for.  Taken where the price is a tenth lower: what the items cost differs by format (f16 4-bit 256 x 4096 x 4096
-    // 25.6 -> 23.2 us, 512 x 4096 x 4096 38.0 -> 35.7, 8-bit 333 x 7616 x 2880 37.2 -> 34.4, 2-bit 285 x 6400 x 3072 30.4 -> 28.0; without the tenth
-    // 8-bit 1000 x 1536 x 4352 29.4 -> 31.0), and of two chunks only as pairs (2-bit 285 x 3072 x 3072 as five 18.6 -> 19.6).
+    // GPCs' odd sizes leave room for (f16 4-bit 256 x 4096 x 4096 25.6 -> 23.2 us, 512 x 4096 x 4096 38.0 -> 35.7, 8-bit 333 x 7616 x 2880 37.2 -> 34.4,
+    // 2-bit 285 x 6400 x 3072 30.4 -> 28.0).  The candidate has to be a tenth cheaper (8-bit 1000 x 1536 x 4352 29.4 -> 31.0), of two chunks only as
+    // pairs (2-bit 285 x 3072 x 3072 as five 18.6 -> 19.6), and then cheaper with what either kind of launch was measured to take besides.
+    // Whole items without slices stay where K is whole super-blocks: there pairs lost every time (8-bit 364 x 6144 x 2560 27.1 -> 34.4, 810 x 4608 x 2560
+    // 25.3 -> 31.9); where it is not, whole items take longer than their price (800 x 4352 x 3904 47.3 -> 41.2, 2-bit 313 x 7680 x 3712 50.3 -> 38.5).
+    // Of those 520 shapes, all of them a tenth cheaper, clusters lost more than 2 % on 130 (by up to 21) and gained 3.4 in the mean; the 352 that are
+    // left lose on 16, and the mean is 5.2.
     double cluster_us = 0.9 * best_us;
+    DensePlan cluster{};
     for (int form = 0; form < 2; ++form) {
         if (!slices_allowed(ctx, M, form)) continue;
         const int most = form == 1 ? 2 * tn_wide : TN_MAX, items_m = (M + most - 1) / most;
@@ -1410,11 +1419,15 @@ DensePlan plan_dense(const Ctx *ctx, int M, int N, int K, int bits, bool slices 
             const double us = (nsb + S - 1) / S * SB_PER_RAW * kb_us + kItemUs + kClusterUs;
             if (us < cluster_us) {
                 cluster_us = us;
-                best = DensePlan{TN, items_m, S, 0, 1, form == 1};
+                cluster = DensePlan{TN, items_m, S, 0, 1, form == 1};
             }
         }
     }
-    return best;
+    if (!cluster.cluster) return best;
+    if (best.ksplit == 1 && K % (SB_PER_RAW * BK) != 0) return cluster;
+    if (best.ksplit == 1 && cluster.wide) return best;
+    const double more = cluster.wide ? kWidePairMore : kClusterMore[cluster.ksplit];
+    return cluster_us + more < best_us + kSlicedMore[best.ksplit < 5 ? best.ksplit : 5] ? cluster : best;
 }
 
 // out[m, n] = sum over the K slices of partial[s][m, n], in slice order, times the factor of token row m; V outputs of a row per

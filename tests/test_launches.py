@@ -38,6 +38,11 @@ def test_forms():
     for m, n, k, bits, g, dt in SLICED:
         form = launch_of(m, [n], k, bits, g, dt)
         assert form["kernel"] == "qmm_tcgen05" and form["cluster"] == form["k_slices"] >= 2 and form["ctas"] % form["cluster"] == 0
+    # K slices: in clusters where that was measured to be faster than whole items, or than slices that add up through memory
+    for args, slices, cluster in (((364, [6144], 2560, 8, 128, "bf16"), 1, 1), ((800, [4352], 3904, 4, 32, "f16"), 2, 2), ((202, [5760], 6208, 8, 32, "bf16"), 3, 1),
+                                  ((212, [5376], 5120, 4, 64, "f16"), 3, 3), ((699, [832], 3072, 4, 128, "bf16"), 6, 1), ((186, [4096], 1024, 4, 64, "bf16"), 4, 4)):
+        form = launch_of(*args)
+        assert (form["k_slices"], form["cluster"]) == (slices, cluster), args
     with pytest.raises(MetalTileError):
         launch_of(1, [64] * 5, 64, 4, 64, "bf16")
 
