@@ -57,8 +57,9 @@ bool supported(const mtc_qmv_desc &d) {
 //     fused launch, 16 tokens 16.7 -> 11.9; 2048 x 2048 3.8 = 3.9, 5120 x 3072 7.0 against 7.9), with groups of 32 always (2048 x 2048, 8 tokens
 //     4.8 -> 4.4).
 //   4-bit from nine tokens on where K is an odd multiple of 256 (the fragment kernel had these) and no CTA has more than a tile: not for
-//     K = 1792 to 3840, where its few warps walk all of K (477 x 3840 5.3 against 6.3, 865 x 2816 4.5 against 5.1, 2048 x 2304 4.8 against 5.0; 865 x
-//     1280 and 4352 and 4096 x 2816 are faster here).
+//     K = 2304 to 3840, where its few warps walk all of K (477 x 3840 5.3 against 6.3, 865 x 2816 4.5 against 5.1, 2048 x 2304 4.8 against 5.0; 865 x
+//     1280 and 4352 and 4096 x 2816 are faster here; K = 1792 is slower by itself, 281 rows 3.7 against 4.0, but faster between the other launches of a
+//     decode step: six layers of 1792 / 256 / 1792, 15 tokens 142 -> 131).
 // A call costs the host 0.2 us more than the ring kernel before it did (a tensor map a projection): products too small to hide it, 4-bit of 1 Mi
 // codes, go from 4.4 to 4.6 us a call, though not in a graph (1247 x 512, 12 tokens 3.37 -> 2.95; 602 x 2560, 5 tokens 3.70 -> 3.43).
 static bool takes(const mtc_qmv_desc *d, int n, int sms, clu::Plan &plan) {
@@ -70,7 +71,7 @@ static bool takes(const mtc_qmv_desc *d, int n, int sms, clu::Plan &plan) {
         tiles += (d[i].N + 15) / 16;
     }
     if (d[0].bits == 8 && d[0].dtype != MTC_F32 && d[0].group_size != 32 && codes < ((d[0].M <= 8 ? 16ll : 12ll) << 20)) return false;
-    if (d[0].bits == 4 && d[0].dtype != MTC_F32 && d[0].M > 8 && d[0].K % 512 != 0 && d[0].K > 1536 && d[0].K < 4096 && tiles <= sms) return false;
+    if (d[0].bits == 4 && d[0].dtype != MTC_F32 && d[0].M > 8 && d[0].K % 512 != 0 && d[0].K > 2048 && d[0].K < 4096 && tiles <= sms) return false;
     plan = clu::shape_plan(d[0], tiles, sms);
     return plan.shift >= 0;          // a part of K that shared memory cannot hold: no plan
 }

@@ -369,8 +369,8 @@ __global__ void __launch_bounds__(32 * kWarps, 1) qmv_cluster_kernel(const __gri
     __syncthreads();
 
     // ---- products ----
-    uint32_t *const odd = reinterpret_cast<uint32_t *>(smem + a.off_bar + W * kDepth * 8);         // a result may be of a token out of range
-    if (threadIdx.x == 0) *odd = 0;                                                // (far_tokens.cuh); set behind the barrier of a pass
+    uint32_t *const odd = reinterpret_cast<uint32_t *>(smem + a.off_bar + W * kDepth * 8);         // a result may be of a token out of range (far_tokens.cuh);
+    if (XT != MTC_F16 && threadIdx.x == 0) *odd = 0;                               // set behind the barrier of a pass
     const float post = XT == MTC_F16 ? __uint_as_float((127u + 24u) << 23) : __uint_as_float((127u + far_tokens::kUnit) << 23);
     // Row r of a unit is UB lines of 128 bytes; TMA stores 16-byte chunk c of line l at c ^ (l & 7): the rows a load phase reads (two
     // of 64 bytes, four of 32, eight of 16) fall on different banks.

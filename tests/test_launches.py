@@ -20,7 +20,7 @@ WARPS = 16
     ((9, [3072], 4096, 8, 64, "bf16"), "qmv_cluster"), ((9, [3071], 4096, 8, 64, "bf16"), "qmv_frag"), ((16, [8192], 8192, 8, 64, "bf16"), "qmm_tcgen05"),
     ((16, [4096], 4096, 4, 32, "bf16"), "qmm_tcgen05"), ((20, [4096], 4096, 4, 64, "bf16"), "qmv_cluster"), ((2048, [4096], 4096, 4, 64, "bf16"), "qmm_tcgen05"),
     # from nine tokens on, K an odd multiple of 256, a tile a CTA
-    ((9, [2368], 2304, 4, 64, "bf16"), "qmv_frag"), ((9, [2369], 2304, 4, 64, "bf16"), "qmv_cluster"), ((16, [865], 1792, 4, 256, "f16"), "qmv_frag"),
+    ((9, [2368], 2304, 4, 64, "bf16"), "qmv_frag"), ((9, [2369], 2304, 4, 64, "bf16"), "qmv_cluster"), ((16, [865], 1792, 4, 256, "f16"), "qmv_cluster"),
     ((16, [865], 1280, 4, 64, "f16"), "qmv_cluster"), ((16, [865], 3840, 4, 64, "bf16"), "qmv_frag"), ((16, [865], 4352, 4, 64, "bf16"), "qmv_cluster"),
     ((8, [865], 2816, 4, 64, "bf16"), "qmv_frag"), ((16, [865], 2816, 4, 64, "f32"), "qmv_cluster"), ((9, [1000, 400], 2304, 4, 64, "bf16"), "qmv_frag"),
     # projections that share x: one launch, or "" where they run one by one
