@@ -43,6 +43,7 @@ def test_cluster_kernel(n, k, m, bits, g, dt):
     gen = torch.Generator(device="cuda").manual_seed(n)
     td = getattr(torch, TYPES[dt])
     w, s, b = _matrix(torch, n, k, bits, g, td, gen)
+    assert ops.context().launch_of(m, [n], k, bits, g, dt)["kernel"] == "qmv_cluster"
     x = torch.randn((m, k), device="cuda", generator=gen).to(td)
     clean = ops.qmv(w, s, b, x, bits, g)
     usual = _far(torch, x, dt)
