@@ -292,10 +292,12 @@ int mtc_peer_barrier(mtc_ctx *ctx, void *stream, void *const *peer_flags, int n_
  *                      the cluster kernel (csrc/qmv_cluster.cuh) in its place; 2 itself whenever it supports
  *                      the shape (M <= 16, K % 32 == 0, power-of-two group >= 32, 16-byte aligned w and x); 0 never
  *   "qmv_tc"           1: those shapes run on the tensor-memory decode kernel instead (slower today; default 0)
- *   "gather_stream"    0: grouped products never take the weight-streaming kernel (default 1: the CSR form with
- *                      4-bit codes, f16 / bf16, k_in % 256 == 0, group 64 or 128 and m_total <= 64 n_experts does), nor the
- *                      grouped fragment kernel (every width, f16 / bf16, k_in % 32 == 0, power-of-two group >= 32, few rows per
- *                      expert: mtc_gather_qmm_route names "gather_qmm_frag")
+ *   "gather_stream"    0: grouped products never take the weight-streaming kernels nor the grouped fragment kernel (default 1: the CSR
+ *                      form does.  Few rows per expert, every width, f16 / bf16, k_in % 32 == 0, power-of-two group >= 32: the fragment
+ *                      kernel, mtc_gather_qmm_route names "gather_qmm_frag".  4-bit codes, group 64 or 128, "gather_qmm_stream": with bf16 up
+ *                      to 512 rows per expert the tcgen05 kernel on exact operands (csrc/gather_exact.cu: k_in a multiple of the group, a row of
+ *                      scales of at most some 100 groups, n_out * groups a multiple of 8, 16-byte aligned arrays), else, with
+ *                      k_in % 256 == 0 and m_total <= 64 n_experts, the one on warp-level tensor cores); 2: as 1 without the exact kernel
  *   "pdl_early_weights" 0: no product reads w, scales or biases before the previous kernel of its stream is
  *                      complete.  Default 1: the dense products (mtc_qmv*, mtc_qmm*, mtc_qvm, chains) are launched with
  *                      programmatic dependent launch and start copying WEIGHTS while the previous kernel drains - weights are

@@ -288,6 +288,12 @@ struct GatherMats {
 cudaError_t launch_gather_stream(Ctx *ctx, cudaStream_t st, const void *x, const void *x2, const uint32_t *row_src, int n_src_rows,
                                  const GatherMats *mats, int n_mats, const uint32_t *expert_offsets, int m_total, int n_out, int K,
                                  int n_experts, int group_size, int dtype, void *scratch);
+bool gather_exact_supported(int m_total, int n_out, int K, int n_experts, int bits, int group_size, int dtype, const void *w,
+                            const void *scales, const void *biases, const void *x);
+size_t gather_exact_scratch_bytes(int m_total, int K);
+cudaError_t launch_gather_exact(Ctx *ctx, cudaStream_t st, const void *x, const uint32_t *row_src, int n_src_rows, const GatherMats *mats, int n_mats,
+                                void *act, const uint32_t *expert_offsets, int m_total, int n_out, int K, int n_experts, int group_size,
+                                void *scratch, std::string *why);
 bool gather_frag_supported(int m_total, int n_out, int K, int n_experts, int bits, int group_size, int dt, const void *w, const void *scales,
                            const void *biases, const void *x);
 cudaError_t launch_gather_frag(Ctx *ctx, cudaStream_t st, const void *x, const uint32_t *row_src, int n_src_rows, const GatherMats *mats, int n_mats,

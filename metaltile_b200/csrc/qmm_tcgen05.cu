@@ -32,9 +32,7 @@
 // Work items (weight-row tile, expert, first token row, token count) are enumerated arithmetically
 // for the dense case and read from a list in scratch memory for the gather case; that list is built
 // on the device from expert_offsets by build_items_kernel.
-#include <cuda.h>
-
-#include "common.cuh"
+#include "tcgen05.cuh"
 
 namespace mtc {
 namespace {
@@ -56,7 +54,6 @@ constexpr int NUM_THREADS = 512;
 constexpr int DEQ_WARP0 = 8, DEQ_THREADS = 256;
 constexpr int EPI_WARP0 = 4;
 constexpr int COPY_WARP0 = 2, COPY_THREADS = 64;
-constexpr uint32_t kSpinLimit = 1u << 22;   // bounded waits: ~seconds, then give up
 struct QmmParams {
     const uint32_t *w;
     const void *scales, *biases;
@@ -115,101 +112,6 @@ struct __align__(8) SmemCtrl {
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
-
-__device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_try(uint64_t *bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-    return ok != 0;
-}
-// try_wait with a suspend-time hint: the thread may sleep in hardware for up to `ns` before it reports failure
-__device__ __forceinline__ bool mbar_try_hint(uint64_t *bar, uint32_t parity, uint32_t ns) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity), "r"(ns) : "memory");
-    return ok != 0;
-}
-// Bounded wait.  Returns false (and raises the CTA's abort flag + the global status word) when the
-// barrier did not complete within kSpinLimit polls or another role already aborted.  `sleep_ns` > 0 lets
-// the hardware suspend the thread between polls: without it the fourteen waiting threads of a CTA issue
-// more poll instructions than the dequant warps issue useful ones (ncu: SYNCS + BRA + BREAK were 60 % of all
-// instructions executed).
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, SmemCtrl *ctl, uint32_t *status, uint32_t code,
-                                          uint32_t sleep_ns = 0) {
-    for (uint32_t i = 0; i < kSpinLimit; ++i) {
-        if (sleep_ns ? mbar_try_hint(bar, parity, sleep_ns) : mbar_try(bar, parity)) return true;
-        if ((i & 63u) == 63u && ctl->abort) return false;
-    }
-    ctl->abort = 1;
-    atomicCAS(status, 0u, code);
-    return false;
-}
-// Whole-warp wait.  All lanes poll together, one instruction for the warp: with lane 0 polling and broadcasting, the other
-// lanes' yields and the reconvergence after every poll were on the path of every hand-off.
-__device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t parity, SmemCtrl *ctl, uint32_t *status, uint32_t code,
-                                               uint32_t sleep_ns) {
-    const bool ok = mbar_wait(bar, parity, ctl, status, code, sleep_ns);
-    __syncwarp();
-    return ok;
-}
-
-__device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, int c0, int c1, uint64_t *bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-        ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(smem_u32(bar)) : "memory");
-}
-
-__device__ __forceinline__ void tma_load_2d_at(uint32_t dst, const CUtensorMap *map, int c0, int c1, uint64_t *bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-        ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(smem_u32(bar)) : "memory");
-}
-
-// Shared-memory matrix descriptor: K-major operand, 128-byte swizzle, 8-row atoms 1024 B apart.
-__device__ __forceinline__ uint64_t make_desc_sw128(uint32_t saddr) {
-    uint64_t d = 0;
-    d |= static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4);   // start address  [0,14)
-    d |= static_cast<uint64_t>(1) << 16;                   // leading byte offset (unused with 128B swizzle)
-    d |= static_cast<uint64_t>(1024 >> 4) << 32;           // stride byte offset [32,46)
-    d |= static_cast<uint64_t>(1) << 46;                   // descriptor version (sm_100)
-    d |= static_cast<uint64_t>(2) << 61;                   // SWIZZLE_128B
-    return d;
-}
-
-__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ bool elect_one() {
-    uint32_t pred;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(pred));
-    return pred != 0;
-}
-__device__ __forceinline__ void umma_commit(uint64_t *bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-
 // 32 TMEM lanes x 16 columns in the layout of an MMA accumulator: thread t holds, for the 8 lanes of block k (0..3) and the 8
 // columns of half g, lane t / 4 and columns 2 (t % 4), 2 (t % 4) + 1: v[k >> 1][4 g + 2 (k & 1)], + 1.
 __device__ __forceinline__ void tmem_ld_frag(uint32_t taddr, uint32_t (&v)[2][8]) {
@@ -229,19 +131,6 @@ __device__ __forceinline__ uint32_t pack_out(float lo, float hi, bool f16) {
 // four 8 x 8 blocks, each stored transposed: lane i gives the address of row i % 8 of block i / 8
 __device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
     asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
-}
-
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
-          "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
-          "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-        : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
 __device__ __forceinline__ uint32_t pack_f16x2(float lo, float hi) {
@@ -535,8 +424,7 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 2) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&ctl->tmem_base)), "r"(512));
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+        tmem_alloc_all(&ctl->tmem_base);
     }
     tc_fence_before();
     __syncthreads();
@@ -557,15 +445,15 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
             for (int i = blockIdx.x; i < num_items && ok; i += gridDim.x) {
                 const Item item = get_item<KSPLIT>(p, i);
                 for (int kb = 0; kb < item.nkb; kb += KPS) {
-                    if (!(ok = mbar_wait(&ctl->empty[s], ph ^ 1, ctl, p.status, 0x101, p.hint_ns))) break;
+                    if (!(ok = mbar_wait(&ctl->empty[s], ph ^ 1, &ctl->abort, p.status, 0x101, p.hint_ns))) break;
                     const int k0 = ((KSPLIT ? item.kb0 : 0) + kb) * BK;
                     if constexpr (KPS == 2) {
                         const int nb = min(2, item.nkb - kb);                 // k blocks of this stage
                         mbar_expect_tx(&ctl->full[s], x_bytes * nb);
-                        for (int c = 0; c < nb; ++c) tma_load_2d(sX + s * x_slot + c * x_stage, &tmap_x, k0 + c * BK, item.row0, &ctl->full[s]);
+                        for (int c = 0; c < nb; ++c) tma_load_2d(smem_u32(sX) + s * x_slot + c * x_stage, &tmap_x, k0 + c * BK, item.row0, &ctl->full[s]);
                     } else {
                         mbar_expect_tx(&ctl->full[s], x_bytes * item.nc);
-                        for (int c = 0; c < item.nc; ++c) tma_load_2d(sX + s * x_slot + c * x_stage, &tmap_x, k0, item.row0 + c * p.TN, &ctl->full[s]);
+                        for (int c = 0; c < item.nc; ++c) tma_load_2d(smem_u32(sX) + s * x_slot + c * x_stage, &tmap_x, k0, item.row0 + c * p.TN, &ctl->full[s]);
                     }
                     if (++s == nst) {
                         s = 0;
@@ -600,11 +488,11 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                 const bool both = p.wide != 0;
                 const int buf = both ? 0 : (tile_i & 1);
                 const uint32_t acc_ph = (both ? tile_i : (tile_i >> 1)) & 1;
-                if (!(ok = mbar_wait_warp(&ctl->acc_empty[buf], acc_ph ^ 1, ctl, p.status, 0x201, 0))) break;
+                if (!(ok = mbar_wait_warp(&ctl->acc_empty[buf], acc_ph ^ 1, &ctl->abort, p.status, 0x201, 0))) break;
                 tc_fence_after();
                 const uint32_t tmem_d = tmem_base + buf * TN_MAX;
                 for (int kb = 0; kb < item.nkb; kb += KPS) {
-                    if (!(ok = mbar_wait_warp(&ctl->full[s], ph, ctl, p.status, 0x202, 0))) break;
+                    if (!(ok = mbar_wait_warp(&ctl->full[s], ph, &ctl->abort, p.status, 0x202, 0))) break;
                     tc_fence_after();
                     if (leader) {
                         const uint64_t bdesc = bdesc0 + static_cast<uint64_t>(s * b_step);
@@ -657,7 +545,7 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                 const size_t erow = static_cast<size_t>(im.expert) * p.N;
                 const int sb0 = (KSPLIT ? im.kb0 : 0) / SB_PER_RAW, sb1 = sb0 + (im.nkb + SB_PER_RAW - 1) / SB_PER_RAW;
                 for (int sbk = sb0; sbk < sb1; ++sbk) {
-                    if (!(ok = mbar_wait_warp(&ctl->raw_empty[buf], ph ^ 1, ctl, p.status, 0x501, p.hint_ns))) break;
+                    if (!(ok = mbar_wait_warp(&ctl->raw_empty[buf], ph ^ 1, &ctl->abort, p.status, 0x501, p.hint_ns))) break;
                     const uint32_t dstt = raw0 + buf * p.raw_tile;
                     if constexpr (R::TMA) {
                         if (t == 0) {
@@ -665,7 +553,7 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                             // rows past the array and words past the row arrive as zeros; rows past N are never stored
 #pragma unroll
                             for (int q = 0; q < BITS / 4; ++q)
-                                tma_load_2d_at(dstt + q * (BMW * 128), &tmap_w, sbk * (8 * BITS) + q * 32, static_cast<int>(erow) + n0, &ctl->raw_full[buf]);
+                                tma_load_2d(dstt + q * (BMW * 128), &tmap_w, sbk * (8 * BITS) + q * 32, static_cast<int>(erow) + n0, &ctl->raw_full[buf]);
                         }
                     } else {
                         if (t == 0) mbar_arrive(&ctl->raw_full[buf]);
@@ -753,7 +641,7 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
             const int buf = both ? 0 : (tile_i & 1);
             const uint32_t acc_ph = (both ? tile_i : (tile_i >> 1)) & 1;
             const Item item = get_item<KSPLIT>(p, i);
-            ok = mbar_wait_warp(&ctl->acc_full[buf], acc_ph, ctl, p.status, 0x301, p.hint_ns);
+            ok = mbar_wait_warp(&ctl->acc_full[buf], acc_ph, &ctl->abort, p.status, 0x301, p.hint_ns);
             // The four warps share named barriers below, so they give up together: a warp that gave up while another saw the
             // barrier complete would leave that one waiting for good.
             if constexpr (!KSPLIT) ok = epilogue_agrees(ok);
@@ -771,7 +659,8 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                         float *o = reinterpret_cast<float *>(smem) + c * p.TN * BMW + q * 32 + lane;
                         for (int c0 = 0; c0 < rows_h; c0 += 32) {
                             uint32_t v[32];
-                            tmem_ld32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + (buf + hh) * TN_MAX + c0, v);
+                            tmem_ld<32>(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + (buf + hh) * TN_MAX + c0, v);
+                            tmem_wait_ld();
 #pragma unroll
                             for (int j = 0; j < 32; ++j)
                                 if (c0 + j < rows_h) o[(c0 + j) * BMW] = __uint_as_float(v[j]);
@@ -781,7 +670,8 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                     // a K slice: f32 partial sums, 32 token rows at a time in 128-byte segments per warp and row
                     for (int c0 = 0; c0 < rows_h; c0 += 32) {
                         uint32_t v[32];
-                        tmem_ld32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + (buf + hh) * TN_MAX + c0, v);
+                        tmem_ld<32>(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + (buf + hh) * TN_MAX + c0, v);
+                        tmem_wait_ld();
                         if (!n_ok) continue;
                         float *o = p.partial + (static_cast<size_t>(item.ks) * p.M + row_base + c0) * p.N + n;
 #pragma unroll
@@ -866,7 +756,7 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
             for (int i = blockIdx.x; i < num_items && ok; i += gridDim.x) {
                 const Item item = get_item<KSPLIT>(p, i);
                 for (int kb0 = 0; kb0 < item.nkb && ok; kb0 += SB_PER_RAW) {
-                    if (!(ok = mbar_wait_warp(&ctl->raw_full[buf], buf_ph, ctl, p.status, 0x402, 0))) break;
+                    if (!(ok = mbar_wait_warp(&ctl->raw_full[buf], buf_ph, &ctl->abort, p.status, 0x402, 0))) break;
                     const uint32_t base = raw0 + buf * p.raw_tile;
                     // the row's scales and biases of the whole super-block (4, 8 or 16 bytes are in use)
                     uint4 sline, bline;
@@ -898,7 +788,7 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                         uint32_t wv[BITS];                   // read before the wait for the stage
                         R::read(base, r, j, h, wv);
                         const uint32_t sub = KPS == 2 ? j & 1 : 0;              // k block of the stage
-                        if (sub == 0 && !(ok = mbar_wait_warp(&ctl->empty[s], ph ^ 1, ctl, p.status, 0x401, 0))) break;
+                        if (sub == 0 && !(ok = mbar_wait_warp(&ctl->empty[s], ph ^ 1, &ctl->abort, p.status, 0x401, 0))) break;
                         {
                             const unsigned short sr = static_cast<unsigned short>(sb_half(sline, j, h, p.gs_shift));
                             const unsigned short br = static_cast<unsigned short>(sb_half(bline, j, h, p.gs_shift));
@@ -957,7 +847,7 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                 const uint32_t sr = sn, br = bn;
                 if (kb + 1 < item.nkb) request(kb0 + kb + 1);      // the next k block is requested before this one is converted
                 // the stage is free once empty[s] has completed (the producer waits on the same barrier)
-                if (!(ok = mbar_wait_warp(&ctl->empty[s], ph ^ 1, ctl, p.status, 0x401, 0))) break;
+                if (!(ok = mbar_wait_warp(&ctl->empty[s], ph ^ 1, &ctl->abort, p.status, 0x401, 0))) break;
                 float sc, bi;
                 if (p.sb_dt == MTC_F16) {
                     sc = __half2float(__ushort_as_half(static_cast<unsigned short>(sr)));
@@ -1025,7 +915,7 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
     __syncthreads();
     if (warp == 2) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512));
+        tmem_free_all(tmem_base);
     }
 }
 
@@ -1204,48 +1094,16 @@ cudaError_t launch_bits(cudaStream_t st, const CUtensorMap &tmap, const CUtensor
     return p.ksplit > 1 ? go(qmm_tcgen05_kernel<BITS, true, 1>, attr[2]) : go(qmm_tcgen05_kernel<BITS, false, 1>, attr[3]);
 }
 
-// X as a 2-D tensor [rows, K] of 16-bit elements, box 64 x TN, 128-byte swizzle; rows past the end read as zero.
+// X as a 2-D tensor [rows, K] of 16-bit elements, box 64 x TN
 cudaError_t make_x_map(CUtensorMap *tmap, const void *x, int rows, int K, int TN, int op_f16, std::string *why) {
-    EncodeTiledFn encode = get_encode_fn();
-    if (!encode) {
-        if (why) *why = "cuTensorMapEncodeTiled is not available from the driver";
-        return cudaErrorNotSupported;
-    }
-    const cuuint64_t dims[2] = {static_cast<cuuint64_t>(K), static_cast<cuuint64_t>(rows)};
-    const cuuint64_t strides[1] = {static_cast<cuuint64_t>(K) * 2};
-    const cuuint32_t box[2] = {BK, static_cast<cuuint32_t>(TN)};
-    const cuuint32_t estr[2] = {1, 1};
-    CUresult r = encode(tmap, op_f16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
-                        const_cast<void *>(x), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                        CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) {
-        if (why) *why = "cuTensorMapEncodeTiled failed with code " + std::to_string(static_cast<int>(r));
-        return cudaErrorInvalidValue;
-    }
-    return cudaSuccess;
-}
-
-// Packed words as a 2-D tensor [rows, words], box 128 bytes x 128 rows, 128-byte swizzle
-cudaError_t make_w_map(CUtensorMap *tmap, const QmmParams &p, long long rows, std::string *why) {
-    EncodeTiledFn encode = get_encode_fn();
-    if (!encode) return cudaErrorNotSupported;          // make_x_map has said why
-    const cuuint64_t dims[2] = {static_cast<cuuint64_t>(p.wpr), static_cast<cuuint64_t>(rows)};
-    const cuuint64_t strides[1] = {static_cast<cuuint64_t>(p.wpr) * 4};
-    const cuuint32_t box[2] = {32, BMW};
-    const cuuint32_t estr[2] = {1, 1};
-    CUresult r = encode(tmap, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<uint32_t *>(p.w), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                        CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) {
-        if (why) *why = "cuTensorMapEncodeTiled failed with code " + std::to_string(static_cast<int>(r));
-        return cudaErrorInvalidValue;
-    }
-    return cudaSuccess;
+    return make_map_2d(tmap, op_f16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, x, rows, K, TN, BK, why);
 }
 
 cudaError_t launch_any(int bits, cudaStream_t st, const CUtensorMap &tmap, const QmmParams &p, int grid, long long w_rows, std::string *why) {
     CUtensorMap wmap = tmap;                            // not read where the words do not travel by TMA
     if (p.raw && (bits == 4 || bits == 8)) {
-        cudaError_t e = make_w_map(&wmap, p, w_rows, why);
+        // packed words [rows, words], box 128 bytes x 128 rows
+        cudaError_t e = make_map_2d(&wmap, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, p.w, w_rows, p.wpr, BMW, 32, why);
         if (e != cudaSuccess) return e;
     }
     switch (bits) {
@@ -1485,6 +1343,40 @@ __global__ void __launch_bounds__(256) ksplit_sum_kernel(const float *partial, c
 }
 
 }  // namespace
+
+namespace {
+cudaError_t encode_map(CUtensorMap *map, CUtensorMapDataType type, int rank, const void *base, const cuuint64_t *dims, const cuuint64_t *strides,
+                       const cuuint32_t *box, std::string *why) {
+    EncodeTiledFn encode = get_encode_fn();
+    if (!encode) {
+        if (why) *why = "cuTensorMapEncodeTiled is not available from the driver";
+        return cudaErrorNotSupported;
+    }
+    const cuuint32_t estr[3] = {1, 1, 1};
+    const CUresult r = encode(map, type, rank, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) {
+        if (why) *why = "cuTensorMapEncodeTiled failed with code " + std::to_string(static_cast<int>(r));
+        return cudaErrorInvalidValue;
+    }
+    return cudaSuccess;
+}
+}  // namespace
+
+cudaError_t make_map_2d(CUtensorMap *map, CUtensorMapDataType type, int elem_bytes, const void *base, long long rows, long long cols,
+                        int box_rows, int box_cols, std::string *why) {
+    const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
+    const cuuint64_t strides[1] = {static_cast<cuuint64_t>(cols) * elem_bytes};
+    const cuuint32_t box[2] = {static_cast<cuuint32_t>(box_cols), static_cast<cuuint32_t>(box_rows)};
+    return encode_map(map, type, 2, base, dims, strides, box, why);
+}
+
+cudaError_t make_map_blocks(CUtensorMap *map, const void *base, long long rows, long long cols, int box_rows, int box_blocks, std::string *why) {
+    const cuuint64_t dims[3] = {64, static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(cols / 64)};
+    const cuuint64_t strides[2] = {static_cast<cuuint64_t>(cols) * 2, 128};
+    const cuuint32_t box[3] = {64, static_cast<cuuint32_t>(box_rows), static_cast<cuuint32_t>(box_blocks)};
+    return encode_map(map, CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, base, dims, strides, box, why);
+}
 
 bool qmm_tcgen05_supported(int M, int N, int K, int bits, int group_size, int dt, const void *w, const void *x,
                            const void *out) {

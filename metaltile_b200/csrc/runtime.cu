@@ -224,6 +224,24 @@ inline bool gather_frag_rule(int m_total, int n_out, int k_in, int n_experts, in
     if (codes <= (32ll << 20)) return rows <= 10 * experts;
     return rows <= (group_size % 64 == 0 ? 4 : bits == 8 ? 2 : 3) * experts;
 }
+// The exact tcgen05 kernel (gather_exact.cu) against those, 4-bit bf16 layers, by the same measures (us a layer, other kernel -> it).  It reads an expert's
+// matrices once for up to 64 rows, but its launches and an item's start cost more.
+//   up to 16 Mi codes, against the fragment kernel: 16 of 1024 x 512, 4 rows 28.1 against 28.4; 6 rows 37.8 -> 29.1, 16 rows 44 -> 30; 64 of 512 x 256, 4
+//     rows 26.6 against 29.8, 6 rows 35.2 -> 30.5; 8 of 1600 x 1088 4 rows 35.1 against 35.3, 8 rows 40.7 -> 36.6.
+//   up to 64 Mi: where the streaming kernel takes the shape, 32 of 1024 x 768, half a row 26.4 against 29.4, one row 37.5 -> 34.7, 8 rows 46.6 -> 41, 32
+//     rows 70 -> 49; 64 of 1024 x 768, one to four rows as fast.  Where it does not: 32 of 1088 x 832, one row 39.1 against 39.8, two 46.0 and 45.9, three 55.6 ->
+//     46.3, 37 rows 114 -> 56.
+//   more: 128 of 1024 x 768 (96 Mi), streamed, 1 / 2 / 4 rows 62 / 72 / 76 against 64 / 75 / 79; 128 of 2048 x 768, 2 / 4 / 8 / 32 rows 105 against 115, 127
+//     and 127, 139 -> 130, 258 -> 156, 64 rows 356 -> 238; not streamed, 128 of 2112 x 832, 1/8 / 1/4 / 1/2 / 4 rows 41 against 47, 62 and 61, 92 -> 81, 287 -> 157.
+//   the most: against the tcgen05 kernel, which converts a matrix once for up to 256 rows: 8 of 2048 x 1536, 256 / 512 / 1024 rows 135 -> 98, 196 -> 161, 280
+//     against 282; 32 of 1024 x 768 168 -> 136, 267 -> 241, 433 against 462.
+inline bool gather_exact_rule(int m_total, int n_out, int k_in, int n_experts, bool streamed) {
+    const long long codes = static_cast<long long>(n_experts) * n_out * k_in, rows = m_total, experts = n_experts;
+    if (rows > 512 * experts) return false;
+    if (codes <= (16ll << 20)) return rows > 4 * experts;
+    if (codes <= (64ll << 20)) return 2 * rows > (streamed ? 1 : 3) * experts;
+    return streamed ? rows > 4 * experts : 4 * rows > experts;
+}
 // rows: weight rows of the launch (N, or those of all fused projections)
 inline bool frag_takes(const Ctx *ctx, int M, long long rows, bool fused, int N, int K, int bits, int group_size, int dt, const void *w, const void *scales,
                        const void *biases, const void *x) {
@@ -1147,7 +1165,7 @@ int mtc_set_option(mtc_ctx *ctx, const char *name, int value) {
         return MTC_OK;
     }
     if (std::strcmp(name, "gather_stream") == 0) {
-        ctx->gather_stream = value ? 1 : 0;
+        ctx->gather_stream = value < 0 ? 0 : (value > 2 ? 2 : value);
         return MTC_OK;
     }
     if (std::strcmp(name, "qmm_wide") == 0) {
@@ -1170,9 +1188,17 @@ static bool gather_stream_takes(const Ctx *ctx, bool csr, int m_total, int n_out
     return csr && (!ctx || ctx->gather_stream) && static_cast<long long>(m_total) <= 64ll * n_experts &&
            mtc::gather_stream_supported(m_total, n_out, k_in, n_experts, bits, group_size, dtype, w, scales, biases, x);
 }
+static bool gather_exact_takes(const Ctx *ctx, bool csr, int m_total, int n_out, int k_in, int n_experts, int bits, int group_size, int dtype,
+                               const void *w, const void *scales, const void *biases, const void *x) {
+    return csr && (!ctx || ctx->gather_stream == 1) &&
+           gather_exact_rule(m_total, n_out, k_in, n_experts,
+                             gather_stream_takes(ctx, csr, m_total, n_out, k_in, n_experts, bits, group_size, dtype, w, scales, biases, x)) &&
+           mtc::gather_exact_supported(m_total, n_out, k_in, n_experts, bits, group_size, dtype, w, scales, biases, x);
+}
 static bool gather_frag_takes(const Ctx *ctx, bool csr, int m_total, int n_out, int k_in, int n_experts, int bits, int group_size, int dtype,
                               const void *w, const void *scales, const void *biases, const void *x) {
     return csr && (!ctx || ctx->gather_stream) &&
+           !gather_exact_takes(ctx, csr, m_total, n_out, k_in, n_experts, bits, group_size, dtype, w, scales, biases, x) &&
            gather_frag_rule(m_total, n_out, k_in, n_experts, bits, group_size,
                             gather_stream_takes(ctx, csr, m_total, n_out, k_in, n_experts, bits, group_size, dtype, w, scales, biases, x)) &&
            mtc::gather_frag_supported(m_total, n_out, k_in, n_experts, bits, group_size, dtype, w, scales, biases, x);
@@ -1198,6 +1224,17 @@ int mtc_gather_qmm(mtc_ctx *ctx, void *stream, const void *x, const void *w, con
         const mtc::GatherMats one{w, scales, biases, out};
         MTC_CUDA(ctx, mtc::launch_gather_frag(ctx, st, x, nullptr, 0, &one, 1, static_cast<const uint32_t *>(expert_offsets), m_total, n_out, k_in, n_experts,
                                               bits, group_size, dtype), MTC_ERR_DISPATCH);
+        return MTC_OK;
+    }
+    // 4-bit bf16 layers: nothing rounded, on tcgen05
+    if (gather_exact_takes(ctx, expert_offsets != nullptr, m_total, n_out, k_in, n_experts, bits, group_size, dtype, w, scales, biases, x)) {
+        std::string why;
+        cudaError_t e = mtc::grow_block(ctx, st, &ctx->d_gfrag, &ctx->gfrag_bytes, mtc::gather_exact_scratch_bytes(m_total, k_in), &why);
+        if (e != cudaSuccess) return fail(ctx, MTC_ERR_BUFFER, "gather_qmm staging: " + (why.empty() ? std::string(cudaGetErrorString(e)) : why));
+        const mtc::GatherMats one{w, scales, biases, out};
+        e = mtc::launch_gather_exact(ctx, st, x, nullptr, 0, &one, 1, nullptr, static_cast<const uint32_t *>(expert_offsets), m_total, n_out, k_in, n_experts,
+                                     group_size, ctx->d_gfrag, &why);
+        if (e != cudaSuccess) return fail(ctx, MTC_ERR_DISPATCH, "gather_qmm (exact) launch: " + (why.empty() ? std::string(cudaGetErrorString(e)) : why));
         return MTC_OK;
     }
     // few rows per expert: the layer is bound by reading every expert's matrix once - the streaming kernel
@@ -1247,16 +1284,17 @@ int mtc_moe_experts(mtc_ctx *ctx, void *stream, const void *x, const void *sort_
     const size_t act_bytes = align_up(static_cast<size_t>(m_total) * inter * esz, 256), xp_bytes = align_up(static_cast<size_t>(m_total) * hidden * esz, 256);
     // the kernels that mtc_gather_qmm takes for the three products: fused where they agree, composed from the entries where they do not
     const mtc_qmat *const mats[3] = {gate, up, down};
-    int n_frag = 0, n_stream = 0;
+    int n_frag = 0, n_stream = 0, n_exact = 0;
     for (int i = 0; i < 3; ++i) {
         const int n = i < 2 ? inter : hidden, k = i < 2 ? hidden : inter;
         const void *const in = i < 2 ? x : nullptr;
         n_frag += gather_frag_takes(ctx, true, m_total, n, k, n_experts, bits, group_size, dtype, mats[i]->w, mats[i]->scales, mats[i]->biases, in);
+        n_exact += gather_exact_takes(ctx, true, m_total, n, k, n_experts, bits, group_size, dtype, mats[i]->w, mats[i]->scales, mats[i]->biases, in);
         n_stream += gather_stream_takes(ctx, true, m_total, n, k, n_experts, bits, group_size, dtype, mats[i]->w, mats[i]->scales, mats[i]->biases, in);
     }
-    const bool frag = n_frag == 3, streamed = n_frag == 0 && n_stream == 3;
+    const bool frag = n_frag == 3, exact = n_frag == 0 && n_exact == 3, streamed = n_frag == 0 && n_exact == 0 && n_stream == 3;
     std::string why;
-    cudaError_t e = mtc::grow_block(ctx, st, &ctx->d_moe, &ctx->moe_bytes, 2 * act_bytes + (streamed || frag ? 0 : xp_bytes), &why);
+    cudaError_t e = mtc::grow_block(ctx, st, &ctx->d_moe, &ctx->moe_bytes, 2 * act_bytes + (streamed || exact || frag ? 0 : xp_bytes), &why);
     if (e != cudaSuccess) return fail(ctx, MTC_ERR_BUFFER, "moe_experts intermediates: " + (why.empty() ? std::string(cudaGetErrorString(e)) : why));
     char *g = static_cast<char *>(ctx->d_moe), *u = g + act_bytes, *xp = u + act_bytes;
     if (frag) {
@@ -1270,6 +1308,21 @@ int mtc_moe_experts(mtc_ctx *ctx, void *stream, const void *x, const void *sort_
         if (rc != MTC_OK) return rc;
         const mtc::GatherMats dn{down->w, down->scales, down->biases, y};
         e = mtc::launch_gather_frag(ctx, st, g, nullptr, 0, &dn, 1, offsets, m_total, hidden, inter, n_experts, bits, group_size, dtype);
+        if (e != cudaSuccess) return fail(ctx, MTC_ERR_DISPATCH, std::string("moe_experts (down) launch: ") + cudaGetErrorString(e));
+        return MTC_OK;
+    }
+    if (exact) {
+        // four launches: rows -> operands (the permutation folded in), gate and up with SwiGLU, rows -> operands, down
+        const size_t need = std::max(mtc::gather_exact_scratch_bytes(m_total, hidden), mtc::gather_exact_scratch_bytes(m_total, inter));
+        e = mtc::grow_block(ctx, st, &ctx->d_gfrag, &ctx->gfrag_bytes, need, &why);
+        if (e != cudaSuccess) return fail(ctx, MTC_ERR_BUFFER, "moe_experts staging: " + (why.empty() ? std::string(cudaGetErrorString(e)) : why));
+        const mtc::GatherMats gu[2] = {{gate->w, gate->scales, gate->biases, nullptr}, {up->w, up->scales, up->biases, nullptr}};
+        e = mtc::launch_gather_exact(ctx, st, x, static_cast<const uint32_t *>(sort_token_idx), n_tokens, gu, 2, g, static_cast<const uint32_t *>(expert_offsets),
+                                     m_total, inter, hidden, n_experts, group_size, ctx->d_gfrag, &why);
+        if (e != cudaSuccess) return fail(ctx, MTC_ERR_DISPATCH, std::string("moe_experts (gate, up) launch: ") + cudaGetErrorString(e));
+        const mtc::GatherMats dn{down->w, down->scales, down->biases, y};
+        e = mtc::launch_gather_exact(ctx, st, g, nullptr, 0, &dn, 1, nullptr, static_cast<const uint32_t *>(expert_offsets), m_total, hidden, inter,
+                                     n_experts, group_size, ctx->d_gfrag, &why);
         if (e != cudaSuccess) return fail(ctx, MTC_ERR_DISPATCH, std::string("moe_experts (down) launch: ") + cudaGetErrorString(e));
         return MTC_OK;
     }
@@ -1338,6 +1391,8 @@ const char *mtc_gather_qmm_route(int m_total, int n_out, int k_in, int n_experts
     // the CSR form with option "gather_stream" at its default
     if (n_experts > 0 && gather_frag_takes(nullptr, true, m_total, n_out, k_in, n_experts, bits, group_size, dtype, nullptr, nullptr, nullptr, nullptr))
         return "gather_qmm_frag";
+    if (n_experts > 0 && gather_exact_takes(nullptr, true, m_total, n_out, k_in, n_experts, bits, group_size, dtype, nullptr, nullptr, nullptr, nullptr))
+        return "gather_qmm_stream";
     if (n_experts > 0 && gather_stream_takes(nullptr, true, m_total, n_out, k_in, n_experts, bits, group_size, dtype, nullptr, nullptr, nullptr, nullptr))
         return "gather_qmm_stream";
     return mtc::qmm_tcgen05_supported(m_total, n_out, k_in, bits, group_size, dtype, nullptr, nullptr, nullptr)

@@ -1,0 +1,136 @@
+"""The exact grouped 4-bit bf16 kernel (csrc/gather_exact.cu): edges of its columns, k blocks, stages, halves and rows of scales against 64-bit sums,
+powers of two of rows and tokens at the ends of their ranges, what stays inside its token, what it reports, and the fused layer against the separate
+entries."""
+import pytest
+
+from test_gather_frag_gpu import _codes, _offsets, _stack
+
+pytestmark = pytest.mark.gpu
+
+
+def _product(torch, ops, ctx, counts, n, k, g, change=None, x_change=None, seed=0):
+    """(got, ref, bound) of one product; mags: what the bound is in terms of."""
+    gen = torch.Generator(device="cuda").manual_seed(seed + 31 * n + k)
+    e, m = len(counts), sum(counts)
+    w, s, b = _stack(torch, e, n, k, 4, g, torch.bfloat16, gen)
+    x = torch.randn((m, k), device="cuda", generator=gen).to(torch.bfloat16)
+    if change:
+        s, b = change(s, b)
+    if x_change:
+        x = x_change(x)
+    out = torch.full((m + 1, n), 7.0, dtype=torch.bfloat16, device="cuda")
+    ops.gather_qmm(x, w, s, b, 4, g, expert_offsets=_offsets(torch, counts), out=out[:m], ctx=ctx)
+    again = ops.gather_qmm(x, w, s, b, 4, g, expert_offsets=_offsets(torch, counts), ctx=ctx)
+    torch.cuda.synchronize()
+    assert ctx.status_word() == 0 and bool((out[m] == 7.0).all())
+    assert torch.equal(out[:m].nan_to_num(3.0), again.nan_to_num(3.0))
+    refs, bounds, row = [], [], 0
+    steps = k // 16 + 4 * ((k // 64 + 7) // 8)
+    for i, c in enumerate(counts):
+        sd, bd = (t[i].double().repeat_interleave(g, 1) for t in (s, b))
+        xs = x[row:row + c].double()
+        wd = _codes(torch, w[i], 4, k).double() * sd + bd
+        mag = xs.abs() @ (16 * sd.abs() + bd.abs()).T
+        # rounded to bf16 once; a chain of steps, each truncated to 24 bits; scales far below their row's largest are rounded
+        small = 2.0 ** -19 * (8 * sd.abs() + bd.abs()).amax(1) * xs.abs().sum(1, keepdim=True)
+        far = (s[i].abs().amax(1) > 2.0 ** 8 * s[i].abs().amin(1)) | (b[i].abs().amax(1) > 2.0 ** 11 * s[i].abs().amin(1))
+        refs.append(xs @ wd.T)
+        bounds.append(2.0 ** -8 * refs[-1].abs() + 2.0 ** -23 * steps * mag + far.double() * small + 2.0 ** -133)
+        row += c
+    return out[:m], torch.cat(refs), torch.cat(bounds)
+
+
+CASES = [([1, 15, 16, 17], 64, 64, 64), ([31, 0, 32, 33], 72, 128, 64), ([47, 48, 49], 200, 192, 64), ([63, 64, 65, 0, 130], 128, 320, 64),
+         ([9, 300], 136, 256, 128), ([40, 7, 25], 64, 640, 128), ([20, 21], 264, 1088, 64), ([5, 36], 320, 2048, 64), ([30], 8, 448, 64),
+         ([12, 6, 44], 96, 4096, 64), ([18] * 40, 64, 128, 128)]
+
+
+@pytest.mark.parametrize("counts,n,k,g", CASES)
+def test_products(counts, n, k, g):
+    import torch
+    from metaltile_b200 import ops
+
+    ctx = ops.context()
+    assert ctx.gather_qmm_route(sum(counts), n, k, len(counts), 4, g, "bf16") == "gather_qmm_stream"
+    got, ref, bound = _product(torch, ops, ctx, counts, n, k, g)
+    assert bool(((got.double() - ref).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("what", ["rows", "groups", "zeros", "biases", "negative"])
+def test_scales_of_every_size(what):
+    import torch
+    from metaltile_b200 import ops
+
+    def change(s, b):
+        e, n, g = s.shape
+        if what == "rows":                                   # a power of two a row, from 2^-40 to 2^40
+            p = torch.exp2(torch.linspace(-40, 40, n, device="cuda").round())[None, :, None]
+        elif what == "groups":                               # within a row up to 2^14 apart
+            p = torch.exp2((torch.arange(g, device="cuda") * 7 % 15).float())[None, None, :]
+        else:
+            p = torch.ones((), device="cuda")
+        s, b = s.float() * p, b.float() * p
+        if what == "zeros":
+            s[:, ::3] = 0
+            b[:, ::6] = 0
+            s[:, 1::4, 1] = 0
+        if what == "biases":
+            b = b * 4096
+        if what == "negative":
+            s = -s
+        return s.to(torch.bfloat16), b.to(torch.bfloat16)
+
+    got, ref, bound = _product(torch, ops, ops.context(), [20, 0, 37], 192, 512, 64, change)
+    assert bool(torch.isfinite(got).all()) and bool(((got.double() - ref).abs() <= bound).all())
+
+
+def test_tokens_of_every_size():
+    """Rows of x from 2^-100 to 2^100; an infinity and a NaN stay in their tokens."""
+    import torch
+    from metaltile_b200 import ops
+
+    m = 45
+    p = torch.exp2(torch.linspace(-100, 100, m, device="cuda").round())[:, None]
+    got, ref, bound = _product(torch, ops, ops.context(), [m], 64, 256, 64, x_change=lambda x: (x.float() * p).to(torch.bfloat16))
+    assert bool(((got.double() - ref).abs() <= bound).all())
+
+    def odd(x):
+        x = x.clone()
+        x[3, 17], x[20, 200] = float("inf"), float("nan")
+        x[30] = 0
+        return x
+
+    got, ref, bound = _product(torch, ops, ops.context(), [30, 15], 64, 256, 64, x_change=odd)
+    keep = [i for i in range(m) if i not in (3, 20)]
+    assert not bool(torch.isfinite(got[3]).any()) and bool(got[20].isnan().all()) and bool((got[30] == 0).all())
+    assert bool(((got.double() - ref).abs() <= bound)[keep].all())
+
+
+@pytest.mark.parametrize("tokens,e,top,hidden,inter,g", [(40, 8, 2, 512, 320, 64), (90, 16, 8, 384, 256, 128), (100, 8, 4, 448, 200 * 8, 64)])
+def test_layer_equals_the_separate_entries(tokens, e, top, hidden, inter, g):
+    import torch
+    from metaltile_b200 import ops
+
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    gate, up, down = (_stack(torch, e, n, k, 4, g, torch.bfloat16, gen) for n, k in ((inter, hidden), (inter, hidden), (hidden, inter)))
+    x = torch.randn((tokens, hidden), device="cuda", generator=gen).to(torch.bfloat16)
+    idx, _ = ops.moe_router_topk(torch.randn((tokens, e), device="cuda", generator=gen).to(torch.bfloat16), top)
+    order, _, off, _ = ops.moe_sort(idx, e)
+    fused = ops.moe_experts(x, gate, up, down, 4, g, off, sort_token_idx=order)
+    rows = ops.moe_permute(x, order)
+    act = ops.swiglu(ops.gather_qmm(rows, *gate, 4, g, expert_offsets=off), ops.gather_qmm(rows, *up, 4, g, expert_offsets=off))
+    assert torch.equal(fused, ops.gather_qmm(act, *down, 4, g, expert_offsets=off))
+    assert ops.context().status_word() == 0
+
+
+def test_rule():
+    from metaltile_b200 import _lib
+    from metaltile_b200.context import _dt
+
+    def route(m, n, k, e, bits=4, g=64, dt="bf16"):
+        return _lib.load().mtc_gather_qmm_route(m, n, k, e, bits, g, _dt(dt)).decode()
+
+    frag, stream, tc = "gather_qmm_frag", "gather_qmm_stream", "gather_qmm_tcgen05"
+    assert [route(m, 768, 1088, 32) for m in (48, 49, 512 * 32, 512 * 32 + 1)] == [frag, stream, stream, tc]
+    assert [route(m, 832, 2112, 128) for m in (32, 33)] == [frag, stream]
+    assert [route(m, 832, 2112, 128, dt="f16") for m in (33, 1300)] == [frag, tc]
