@@ -457,8 +457,10 @@ __global__ void __launch_bounds__(kThreads, 1) gather_exact_kernel(const __grid_
                 for (int c = 0; c < nch; ++c) {
                     if (turn == team) {
                         if (c == 0) ctl->row_factor[e][r] = __uint_as_float(static_cast<uint32_t>(254 - up) << 23);
-                        if (!wait(full + s * 8, ph, 0xa08)) return;
+                        // in this order: with the MMAs of this team's stage before complete, the pass of the ring before this one is, and
+                        // its phase cannot be taken for this one's
                         if (!wait(a_empty + team * 8, aph ^ 1, 0xa09)) return;
+                        if (!wait(full + s * 8, ph, 0xa08)) return;
                         __syncwarp();
                         tc_fence_after();
                         aph ^= 1;
