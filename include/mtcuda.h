@@ -262,7 +262,7 @@ int mtc_peer_barrier(mtc_ctx *ctx, void *stream, void *const *peer_flags, int n_
  *                      shapes run as 16-row chunks of the small-M tensor-core qmv when that fills the GPU better)
  *   "qmm_raw"          0: the dequant warps of the tensor-core kernel load packed words straight from global
  *                      memory instead of through the shared-memory staging buffers (default 1)
- *   "qmm_wide"         a dense work item of the tensor-core kernel covers two 256-row token chunks (one dequantised
+ *   "qmm_wide"         a dense work item of the tensor-core kernel covers two token chunks of up to 208 rows (one dequantised
  *                      weight stage meets two activation chunks; same results): 0 never, 1 (default) when that saves
  *                      rounds of the grid (M > 256), 2 whenever M > 256
  *   "qmm_ksplit"       0: a dense launch of the tensor-core kernel never cuts K into slices (default 1: where whole tiles

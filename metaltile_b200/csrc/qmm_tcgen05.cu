@@ -13,25 +13,33 @@
 // dequantised weights are the A operand (always a full 128-row MMA, however few tokens there are) and
 // the activations are the B operand (TN = 16..256 token rows, straight from TMA).
 //
-// One persistent CTA per SM, 512 threads, warp-specialised:
+// One persistent CTA per SM, 640 threads, warp-specialised:
 //   warp 0      producer   one lane issues TMA (cp.async.bulk.tensor, 128B swizzle) loads of the X
 //                          chunk [TN x 64] into a shared-memory ring (one or two k blocks a stage)
-//   warp 1      MMA        one lane issues tcgen05.mma (M=128, N=TN, K=16, kind::f16), accumulators in
-//                          TMEM, double buffered (2 x 256 columns)
-//   warps 2-3   copies     packed words, scales and biases into the raw staging buffers, super-blocks ahead (4 and 8
-//                          bits: one TMA box of words); warp 2 also allocates and frees the TMEM
+//   warp 1      MMA        one lane issues tcgen05.mma (M=128, N=TN, K=16, kind::f16), A and the accumulators in TMEM, two
+//                          accumulators in turn where they leave A four k blocks
+//   warps 2-3   copies     packed words a super-block of 4 k blocks at a time (4 and 8 bits: one TMA box), scales and biases 64 bytes
+//                          of a row at a time; warp 2 also allocates and frees the TMEM
 //   warps 4-7   epilogue   tcgen05.ld of the finished accumulator, f32 -> T, transposed through shared memory, 256-byte
 //                          rows to out (K slices: f32 partial sums)
-//   warps 8-15  dequant    256 threads = 128 weight rows x 2 halves of a 64-wide k block: codes out of the raw
-//                          buffers (registers, one k block ahead, where a shape has no raw form), w = q*scale + bias
-//                          rounded to the operand type, written as the K-major 128B-swizzled A tile the MMA reads
+//   warps 8-19  dequant    three teams of 128 weight rows, every third stage: codes out of the raw buffers (straight from global memory where a
+//                          shape has no raw form), w = q*scale + bias rounded to the operand type, tcgen05.st as the A operand
 // Stage hand-off uses mbarriers; tcgen05.commit releases a stage when its MMAs have read it.  Every
 // wait is bounded: on expiry the kernel records a code in the context's status word, all roles leave
 // their loops, TMEM is released and the kernel returns.
 //
+// Why A lies in tensor memory: shared memory moves 128 bytes a cycle, and a k block with A there costs it 16 KB stored and 16 KB read by each chunk's
+// MMAs beside the 2 x 128 TN of X: 128 + TN cycles for the MMAs alone (measured), 2.9 cycles a token row in all at 2 x 256 rows where the tensor
+// cores need 2.  With A in tensor memory X and the packed words are all there is: 2 TN cycles, as the tensor cores.  What bounds it: at 240 and 256
+// rows the tensor cores at the clocks that the power leaves (2048 x 4096 x 4096, 4-bit 76 -> 67 us with the conversion of x), below some 200 rows the
+// instructions of the dequant warps (256 x 4096 x 4096 23.2 -> 15.5 us, 8-bit 333 x 7616 x 2880 36 -> 24); 154 other shapes 0.90 to 2.1 times as fast,
+// 1.20 in the mean (slowest: 13 slices through memory, 96 x 1216 x 3328).
+//
 // Work items (weight-row tile, expert, first token row, token count) are enumerated arithmetically
 // for the dense case and read from a list in scratch memory for the gather case; that list is built
 // on the device from expert_offsets by build_items_kernel.
+#include <cstddef>
+
 #include "tcgen05.cuh"
 
 namespace mtc {
@@ -40,20 +48,19 @@ namespace {
 constexpr int BMW = 128;         // weight rows per tile (TMEM lanes, MMA M)
 constexpr int BK = 64;           // k per stage: 64 x 16-bit = one 128B swizzle row
 constexpr int TN_MAX = 256;      // token rows per tile (TMEM columns of one accumulator, MMA N)
-constexpr int MAX_STAGES = 8;    // ring depth: as many stages as fit in RING_BYTES, at most this
-constexpr int RING_BYTES = 216 * 1024;      // stages of the ring, then the raw staging buffers
+constexpr int MAX_STAGES = 8;    // ring depth: as many stages as fit in RING_BYTES and in the columns of A, at most this
+constexpr int RING_BYTES = 216 * 1024;      // stages of the ring, the raw buffers, the scales
 constexpr int EPI_TOK = 16;                 // token rows of one epilogue block: 128 outputs each, two buffers; SmemCtrl follows
 constexpr int EPI_PITCH = BMW * 2 + 16;     // bytes of a row: eight consecutive rows start on different banks
 constexpr int EPI_BYTES = 2 * EPI_TOK * EPI_PITCH;
-constexpr int SB_PER_RAW = 4;               // k blocks per raw super-block: 256 codes = 32*BITS bytes per weight row
-constexpr int RAW_SB_PITCH = 24;            // scales (and biases) of a super-block: up to 20 bytes per row
-constexpr int RAW_SB_BYTES = 2 * BMW * RAW_SB_PITCH;
-constexpr int MAX_RAW = 3;
-constexpr int A_BYTES = BMW * BK * 2;       // 16 KB, dequantised weights
-constexpr int NUM_THREADS = 512;
-constexpr int DEQ_WARP0 = 8, DEQ_THREADS = 256;
+constexpr int SB_PER_RAW = 4;               // k blocks per super-block, what K slices are whole multiples of
+constexpr int MAX_RAW = 4;
+constexpr int TMEM_COLS = 512, A_COLS = BK / 2;     // columns of A per k block
+constexpr int TEAMS = 3;                    // of dequant warps
 constexpr int EPI_WARP0 = 4;
 constexpr int COPY_WARP0 = 2, COPY_THREADS = 64;
+constexpr int DEQ_WARP0 = 8, DEQ_WARPS = 4 * TEAMS;
+constexpr int NUM_THREADS = (DEQ_WARP0 + DEQ_WARPS) * 32;
 struct QmmParams {
     const uint32_t *w;
     const void *scales, *biases;
@@ -80,13 +87,20 @@ struct QmmParams {
     uint32_t hint_ns;            // base suspend-time hint of the waits (0: plain polling)
     int raw;                     // 1: packed words reach the dequant warps through shared memory (cp.async, whole lines)
     uint32_t raw_off, raw_tile;  // byte offset of the raw buffers in shared memory; bytes of one buffer
-    int nraw;                    // raw: number of buffers (2 or 3): super-blocks are requested nraw - 1 ahead
+    int nraw, raw_blk;           // raw: number of buffers; k blocks of one (4; 2 at 8 bits beside two chunks, which leaves the ring its third stage)
     int raw8;                    // raw: 1 = rows of packed words start on 8-byte boundaries only (3 / 5 bits, K an odd multiple of 64)
-    int sb_words;                // raw: 0 = a row's scales of a super-block are one aligned copy; else 4-byte words copied per row
+    // raw: scales (and biases) of the tile, a span of sp_kb k blocks (sp_bytes of a row) at a time, two buffers.  Spans begin at multiples of sp_kb, and with
+    // a K slice
+    int sp_kb, sp_bytes;
+    int sp_copy;                 // 2: TMA boxes (rows are whole 16-byte pieces); 1: 16-byte copies from the boundary below a row's first one on; 0: the
+                                 //    arrays start on 4-byte boundaries only, words
+    uint32_t sp_off;             // byte offset of the buffers
     long long sb_total;          // elements of the scale (and bias) array
     int wide_items;              // wide: items [0, wide_items) cover two token chunks, each later pair of items one such unit
     int wide;                    // 1: a dense item covers up to 2 TN token rows: one dequantised W stage meets two X chunks, both
                                  //    accumulators belong to the item (the dequant work per flop halves; no epilogue overlap)
+    int nacc;                    // accumulators that items take in turn: 2, or 1 (wide: one pair)
+    uint32_t a_col0;             // first column of A, behind the accumulators
     int n_tiles;                 // dense: weight-row tiles
     int ksplit;                  // dense: K slices per (weight-row tile, token rows) unit, each an item of its own; 1 = none
     float *partial;              // ksplit > 1: f32 partial sums [ksplit][M][N], added by ksplit_sum_kernel
@@ -97,6 +111,10 @@ struct QmmParams {
     uint32_t idesc;
 };
 
+struct QmmMaps {
+    CUtensorMap x, w, scales, biases;     // the last three only where they travel by TMA
+};
+
 struct __align__(8) SmemCtrl {
     uint64_t full[MAX_STAGES];   // the X stage has landed (TMA transaction bytes) and the dequant warps finished the W stage
     uint64_t empty[MAX_STAGES];  // MMAs that read the stage have completed
@@ -104,6 +122,7 @@ struct __align__(8) SmemCtrl {
     uint64_t acc_empty[2];       // epilogue drained the accumulator buffer
     uint64_t raw_full[MAX_RAW];  // the copies of a raw super-block have landed
     uint64_t raw_empty[MAX_RAW]; // every dequant warp has read it
+    uint64_t sp_full[2], sp_empty[2];   // the same for a span of scales
     uint32_t tmem_base;
     volatile uint32_t abort;
 };
@@ -144,12 +163,12 @@ __device__ __forceinline__ float code_plus_one(uint32_t win, uint32_t mask, uint
     asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(win), "r"(mask), "r"(one));
     return __uint_as_float(r);
 }
-__device__ __forceinline__ void st_shared_v4(uint32_t saddr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(saddr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
-}
-
 __device__ __forceinline__ void cp_async_16(uint32_t dst, const void *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+// the first `n` bytes of 16, zeros behind them
+__device__ __forceinline__ void cp_async_16_of(uint32_t dst, const void *src, uint32_t n) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
 }
 template <int BYTES>
 __device__ __forceinline__ void cp_async_small(uint32_t dst, const void *src) {
@@ -205,68 +224,22 @@ __device__ __forceinline__ void load_half_words(const uint32_t *p, uint32_t (&w)
     }
 }
 
-// dst[c] = shared-memory address of the c-th of this thread's four 16-byte chunks (swizzle applied by the caller)
-// 4- and 8-bit codes in packed-half arithmetic.  `byte-permute | 0x6400` makes two f16 values 1024 + q without a
-// conversion, HSUB2 removes the 1024 exactly, and one HFMA2 per two codes gives round_f16(q*scale + bias) - the
-// value the f32 path rounds to, up to double rounding - already in the operand's type: ~2 instructions per code
-// instead of ~3.5.  The caller uses it only when the scale is a normal f16 number.
-template <int BITS>
-__device__ __forceinline__ void dequant_half_h2(const uint32_t (&w)[BITS], float s, float b, const uint32_t (&dst)[4],
-                                                uint32_t stage_off) {
-    static_assert(BITS == 4 || BITS == 8, "packed-half path: 4- and 8-bit codes");
-    const __half2 s2 = __float2half2_rn(s), b2 = __float2half2_rn(b);
-    const __half2 k1024 = __half2half2(__ushort_as_half(0x6400));
-    uint32_t magic = 0x64006400u;
-    asm volatile("" : "+r"(magic));          // in a register, so that mask-and-or is a single LOP3
-    auto finish = [&](uint32_t t) {
-        const __half2 q = __hsub2(*reinterpret_cast<const __half2 *>(&t), k1024);
-        const __half2 v = __hfma2(q, s2, b2);
-        return *reinterpret_cast<const uint32_t *>(&v);
-    };
-    if (BITS == 4) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {        // word i = codes 8i..8i+7 = one 16-byte chunk of the tile row
-            const uint32_t lo = w[i], hi = w[i] >> 4;      // byte j of lo / hi has code 2j / 2j+1 in its low nibble
-            uint32_t o[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const uint32_t t = __byte_perm(lo, hi, ((4 + j) << 8) | j);          // code 2j -> bits 0..3, code 2j+1 -> bits 16..19
-                uint32_t r;
-                asm("lop3.b32 %0, %1, 0x000F000F, %2, 0xEA;" : "=r"(r) : "r"(t), "r"(magic));
-                o[j] = finish(r);
-            }
-            st_shared_v4(dst[i] + stage_off, o[0], o[1], o[2], o[3]);
-        }
-    } else {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {        // words 2i, 2i+1 = codes 8i..8i+7
-            uint32_t o[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j)      // two bytes of word 2i + j/2 under the 0x64 exponent bytes
-                o[j] = finish(__byte_perm(w[2 * i + (j >> 1)], 0x64646464u, (j & 1) ? 0x4342 : 0x4140));
-            st_shared_v4(dst[i] + stage_off, o[0], o[1], o[2], o[3]);
-        }
-    }
+__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
+    uint32_t r;
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
+    return r;
 }
-
+// 32 codes of a row -> 16 registers of two operands each, in the order of K: the general form, by way of f32
 template <int BITS>
-__device__ __forceinline__ void dequant_half(const uint32_t (&w)[BITS], float s, float b, const uint32_t (&dst)[4],
-                                             uint32_t stage_off) {
+__device__ __forceinline__ void dequant_half(const uint32_t (&w)[BITS], float s, float b, uint32_t *v) {
     using Q = QPack<BITS>;
-    if constexpr (BITS == 4 || BITS == 8) {
-        // scale a normal f16 number (its exact value survives the conversion), bias within f16 range
-        if (fabsf(s) >= 6.104e-5f && fabsf(s) <= 65504.0f && fabsf(b) <= 65504.0f) {
-            dequant_half_h2<BITS>(w, s, b, dst, stage_off);
-            return;
-        }
-    }
     // a code at bit p of a window becomes q * 2^(p-23) after the magic subtract: fold 2^(23-p) into the scale
     float sp[Q::CPW];
 #pragma unroll
     for (int c = 0; c < Q::CPW; ++c) sp[c] = s * __uint_as_float(static_cast<uint32_t>(23 - c * BITS + 127) << 23);
     uint32_t one = 0x3F800000u;
     asm volatile("" : "+r"(one));            // keep 1.0f in a register so the extraction is a single LOP3
-    float vals[8];
+    float even = 0.0f;
 #pragma unroll
     for (int i = 0; i < 32; ++i) {
         const int wi = i / Q::CPW, c = i % Q::CPW;
@@ -275,31 +248,90 @@ __device__ __forceinline__ void dequant_half(const uint32_t (&w)[BITS], float s,
         if (sh == 0) win = w[word];
         else if (word + 1 < BITS) win = __funnelshift_r(w[word], w[word + 1], sh);
         else win = w[word] >> sh;
-        const float f = code_plus_one(win, Q::MASK << (c * BITS), one) - 1.0f;
-        vals[i & 7] = fmaf(f, sp[c], b);
-        if ((i & 7) == 7)
-            st_shared_v4(dst[i >> 3] + stage_off, pack_f16x2(vals[0], vals[1]), pack_f16x2(vals[2], vals[3]),
-                         pack_f16x2(vals[4], vals[5]), pack_f16x2(vals[6], vals[7]));
+        const float r = fmaf(code_plus_one(win, Q::MASK << (c * BITS), one) - 1.0f, sp[c], b);
+        if (i & 1) v[i >> 1] = pack_f16x2(even, r);
+        else even = r;
     }
 }
-
-// 16-bit scale (or bias) of k block j (0..3) of a super-block for the thread's 32-code half h, out of the row's line:
-// group 32: entry 2j + h; group 64: entry j; group 128: entry j / 2.  j is a compile-time constant where this is used.
-__device__ __forceinline__ uint32_t sb_half(const uint4 &v, int j, int h, int gs_shift) {
-    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-    if (gs_shift == 5) return (w[j] >> (16 * h)) & 0xFFFFu;
-    if (gs_shift == 6) return (w[j >> 1] >> (16 * (j & 1))) & 0xFFFFu;
-    return (w[0] >> (16 * ((j >> 1) & 1))) & 0xFFFFu;
+// A k block of a row, 64 codes (words(h, w): those of half h) with one scale (ONE: groups of 64 and more) or two, in packed halves with no conversion: a 16-bit float with exponent
+// field 0 is linear in its low bits, so a code at bit P of its half is q * 2^(P - 24), and fma(that, scale * 2^(24 - P), bias) is
+// round_f16(q * scale + bias), the value the general form rounds to up to double rounding.  4-bit codes get there by bytes (bit 7 is 0 where the nibble
+// is at bits 3..6, so the sign-replicating form of the byte permute fills the upper byte with zeros): 12 instructions per eight codes (16 with the codes
+// brought to 1024 + q first); 8-bit ones by a byte permute, 8; others by two shifts and two masks a pair, 20 to 22 (32 by way of f32).  The scale
+// times 2^(24 - P) is an f16 in all but odd cases (an underflow of it is far below the last bit of any result): those take the general form.
+template <int BITS, bool ONE, typename Get>
+__device__ __forceinline__ void dequant_block(Get words, float s0, float b0, float s1, float b1, uint32_t (&v)[32]) {
+    // where a code lies in its half of a register: bit 3 (4 bits), 0 (8 bits), at the top of the ten bits of a fraction (others)
+    constexpr int P = BITS == 4 ? 3 : BITS == 8 ? 0 : 10 - BITS;
+    constexpr float kUp = static_cast<float>(1 << (24 - P)), kMost = 65472.0f / kUp;
+    bool direct = fabsf(s0) <= kMost && fabsf(b0) <= 65504.0f;
+    if (!ONE) direct = direct && fabsf(s1) <= kMost && fabsf(b1) <= 65504.0f;
+    if (direct) {
+        __half2 s2 = __float2half2_rn(s0 * kUp), b2 = __float2half2_rn(b0);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            if (!ONE && h == 1) {
+                s2 = __float2half2_rn(s1 * kUp);
+                b2 = __float2half2_rn(b1);
+            }
+            uint32_t w[BITS];
+            words(h, w);
+            const uint32_t s = *reinterpret_cast<const uint32_t *>(&s2), b = *reinterpret_cast<const uint32_t *>(&b2);
+            auto put = [&](int i, uint32_t q) { asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(v[16 * h + i]) : "r"(q), "r"(s), "r"(b)); };
+            if constexpr (BITS == 4) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {    // byte j of lo / hi: code 2j / 2j+1 at bits 3..6
+                    const uint32_t lo = (w[i] << 3) & 0x78787878u, hi = (w[i] >> 1) & 0x78787878u;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) put(4 * i + j, prmt(lo, hi, ((0xC + j) << 12) | ((4 + j) << 8) | ((8 + j) << 4) | j));
+                }
+            } else if constexpr (BITS == 8) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    put(2 * i, prmt(w[i], 0u, 0x4140));
+                    put(2 * i + 1, prmt(w[i], 0u, 0x4342));
+                }
+            } else {
+                constexpr uint32_t kLow = ((1u << BITS) - 1u) << P, kHigh = kLow << 16;
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {   // codes 2i, 2i+1: bits 2i * BITS and on
+                    const int at = 2 * i * BITS, word = at / 32;
+                    int sh = at % 32;
+                    uint32_t t = w[word];
+                    if (sh + 2 * BITS > 32) {
+                        t = __funnelshift_r(t, w[word + 1 < BITS ? word + 1 : word], sh);
+                        sh = 0;
+                    }
+                    const int up0 = P - sh, up1 = 16 + P - sh - BITS;
+                    const uint32_t lo = up0 >= 0 ? t << (up0 & 31) : t >> (-up0 & 31), hi = up1 >= 0 ? t << (up1 & 31) : t >> (-up1 & 31);
+                    put(i, (lo & kLow) | (hi & kHigh));
+                }
+            }
+        }
+        return;
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        uint32_t w[BITS];
+        words(h, w);
+        dequant_half<BITS>(w, ONE || h == 0 ? s0 : s1, ONE || h == 0 ? b0 : b1, v + 16 * h);
+    }
+}
+__device__ __forceinline__ float sb_value(uint32_t bits, int dt) {
+    return dt == MTC_F16 ? __half2float(__ushort_as_half(static_cast<unsigned short>(bits))) : __uint_as_float(bits << 16);
+}
+__device__ __forceinline__ uint32_t lds_u16(uint32_t addr) {
+    unsigned short v;
+    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr));
+    return v;
 }
 
-// One super-block of a weight tile as it lies in a raw buffer: the packed words of 128 rows, then the scales, then the biases.
+// The packed words of some k blocks of a weight tile as they lie in a raw buffer.
 // 4 and 8 bits: TMA boxes of 128 bytes x 128 rows with the 128-byte swizzle; other widths: rows padded by 16 bytes.
 template <int BITS>
 struct RawTile {
     static constexpr bool TMA = BITS == 4 || BITS == 8;
-    static constexpr int ROW_BYTES = 32 * BITS, PITCH = ROW_BYTES + 16;
-    static constexpr int SB_OFF = TMA ? BMW * ROW_BYTES : BMW * PITCH;
-    static constexpr int BYTES = SB_OFF + RAW_SB_BYTES;
+    static constexpr int BLK_BYTES = 8 * BITS, PITCH = SB_PER_RAW * BLK_BYTES + 16;
     // the 32 codes of k block j, half h of row r
     static __device__ __forceinline__ void read(uint32_t base, int r, int j, int h, uint32_t (&w)[BITS]) {
         if constexpr (TMA) {
@@ -314,7 +346,10 @@ struct RawTile {
         }
     }
 };
-int raw_bytes(int bits) { return (bits == 4 || bits == 8 ? BMW * 32 * bits : BMW * (32 * bits + 16)) + RAW_SB_BYTES; }
+int raw_bytes(int bits, int blocks) { return BMW * (8 * bits * blocks + (bits == 4 || bits == 8 ? 0 : 16)); }
+// Rows of a span lie 16 bytes further apart than they are long: eight of them start on different banks, and words that cover them fit
+__host__ __device__ constexpr int sp_pitch(int sp_bytes) { return sp_bytes + 16; }
+__host__ __device__ constexpr int sp_buffer(int sp_bytes) { return 2 * BMW * sp_pitch(sp_bytes); }
 
 // up to eight 16-bit outputs one by one
 __device__ __noinline__ void store_row8(char *o, uint4 v, int n) {
@@ -393,23 +428,21 @@ __device__ __forceinline__ Item get_item(const QmmParams &p, int i) {
 // separate instantiation, so that the code of every other launch is what it was without the feature.
 template <int BITS, bool KSPLIT, int KPS>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
-qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w, const QmmParams p) {
+qmm_tcgen05_kernel(const __grid_constant__ QmmMaps maps, const QmmParams p) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
     const int nst = p.nst;
-    const uint32_t w_stage = KPS * A_BYTES;                             // KPS dequantised W blocks per stage
     const uint32_t x_stage = static_cast<uint32_t>(p.TN) * BK * 2;      // one X chunk; multiple of 2 KB
     const uint32_t x_slot = KPS == 2 || p.wide ? 2 * x_stage : x_stage;  // two X chunks, or one per k block, per stage (KPS is 1 when wide)
-    uint8_t *sW = smem;                                  // nst x w_stage: dequantised weights (A operand)
-    uint8_t *sX = smem + nst * w_stage;                  // nst x x_slot: activations (B operand)
+    uint8_t *sX = smem;                                  // nst x x_slot: activations (B operand)
     SmemCtrl *ctl = reinterpret_cast<SmemCtrl *>(smem + RING_BYTES + EPI_BYTES);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;       // known to be uniform
     const uint32_t x_bytes = static_cast<uint32_t>(p.TN) * BK * 2;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < MAX_STAGES; ++s) {
-            mbar_init(&ctl->full[s], 1 + DEQ_THREADS / 32);
+            mbar_init(&ctl->full[s], 1 + 4);
             mbar_init(&ctl->empty[s], 1);
         }
         for (int b = 0; b < 2; ++b) {
@@ -417,8 +450,12 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
             mbar_init(&ctl->acc_empty[b], 4);
         }
         for (int b = 0; b < MAX_RAW; ++b) {
-            mbar_init(&ctl->raw_full[b], COPY_THREADS + 1);
-            mbar_init(&ctl->raw_empty[b], DEQ_THREADS / 32);
+            mbar_init(&ctl->raw_full[b], RawTile<BITS>::TMA ? 1 : COPY_THREADS);
+            mbar_init(&ctl->raw_empty[b], DEQ_WARPS);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&ctl->sp_full[b], p.sp_copy == 2 ? 1 : COPY_THREADS);
+            mbar_init(&ctl->sp_empty[b], DEQ_WARPS);
         }
         ctl->abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -429,7 +466,7 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = ctl->tmem_base;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, ctl->tmem_base, 0);
     if (!p.pdl_roles) asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;");
     // a list of work items comes from an earlier kernel of the stream (pdl_roles is 0 then): its length after the wait
@@ -450,10 +487,10 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                     if constexpr (KPS == 2) {
                         const int nb = min(2, item.nkb - kb);                 // k blocks of this stage
                         mbar_expect_tx(&ctl->full[s], x_bytes * nb);
-                        for (int c = 0; c < nb; ++c) tma_load_2d(smem_u32(sX) + s * x_slot + c * x_stage, &tmap_x, k0 + c * BK, item.row0, &ctl->full[s]);
+                        for (int c = 0; c < nb; ++c) tma_load_2d(smem_u32(sX) + s * x_slot + c * x_stage, &maps.x, k0 + c * BK, item.row0, &ctl->full[s]);
                     } else {
                         mbar_expect_tx(&ctl->full[s], x_bytes * item.nc);
-                        for (int c = 0; c < item.nc; ++c) tma_load_2d(smem_u32(sX) + s * x_slot + c * x_stage, &tmap_x, k0, item.row0 + c * p.TN, &ctl->full[s]);
+                        for (int c = 0; c < item.nc; ++c) tma_load_2d(smem_u32(sX) + s * x_slot + c * x_stage, &maps.x, k0, item.row0 + c * p.TN, &ctl->full[s]);
                     }
                     if (++s == nst) {
                         s = 0;
@@ -469,102 +506,149 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
         // The whole warp runs the loop so that stage counters, descriptors and accumulator addresses are
-        // warp-uniform values; one elected lane issues.  (With the loop under `if (lane == 0)` every operand of
-        // every tcgen05.mma was moved to a uniform register first and two barriers were polled one after the other:
-        // 1100 cycles per k block whatever the tile width, measured - the issuer, not the tensor pipe or the
-        // producers, set the pace of the kernel.)
-        {
-            uint32_t tile_i = 0;
-            int s = 0;
-            uint32_t ph = 0;
-            bool ok = true;
-            const bool leader = elect_one();
-            const uint64_t adesc0 = make_desc_sw128(smem_u32(sW)), bdesc0 = make_desc_sw128(smem_u32(sX));
-            const uint32_t a_step = w_stage >> 4, b_step = x_slot >> 4;       // descriptor address units per stage
-            for (int i = blockIdx.x; i < num_items && ok; i += gridDim.x, ++tile_i) {
-                const Item item = get_item<KSPLIT>(p, i);
-                // wide items: both 256-column accumulators belong to one item (no double buffering);
-                // otherwise the two accumulators alternate so that the epilogue overlaps the next item
-                const bool both = p.wide != 0;
-                const int buf = both ? 0 : (tile_i & 1);
-                const uint32_t acc_ph = (both ? tile_i : (tile_i >> 1)) & 1;
-                if (!(ok = mbar_wait_warp(&ctl->acc_empty[buf], acc_ph ^ 1, &ctl->abort, p.status, 0x201, 0))) break;
+        // warp-uniform values; its control flow depends on votes alone; one elected lane issues.  (With operands that are not known to be
+        // uniform four MMAs take 190 cycles to issue instead of 60; under `if (lane == 0)` a k block took 1100.)
+        uint32_t tile_i = 0;
+        int s = 0;
+        uint32_t ph = 0;
+        bool ok = true;
+        const bool leader = elect_one();
+        const uint64_t bdesc0 = make_desc_sw128(__shfl_sync(0xffffffffu, smem_u32(sX), 0));
+        const uint32_t b_step = x_slot >> 4, c_step = x_stage >> 4;       // descriptor address units per stage, per chunk
+        for (int i = blockIdx.x; i < num_items && ok; i += gridDim.x, ++tile_i) {
+            const Item item = get_item<KSPLIT>(p, i);
+            // items take the accumulators in turn, so that the epilogue overlaps the next one where there are two
+            const int buf = p.nacc == 2 ? tile_i & 1 : 0;
+            const uint32_t acc_ph = (p.nacc == 2 ? tile_i >> 1 : tile_i) & 1;
+            if (!(ok = mbar_wait_vote(&ctl->acc_empty[buf], acc_ph ^ 1, &ctl->abort, p.status, 0x201))) break;
+            tc_fence_after();
+            const uint32_t tmem_d = tmem_base + buf * p.TN;
+            for (int kb = 0; kb < item.nkb; kb += KPS) {
+                if (!(ok = mbar_wait_vote(&ctl->full[s], ph, &ctl->abort, p.status, 0x202))) break;
                 tc_fence_after();
-                const uint32_t tmem_d = tmem_base + buf * TN_MAX;
-                for (int kb = 0; kb < item.nkb; kb += KPS) {
-                    if (!(ok = mbar_wait_warp(&ctl->full[s], ph, &ctl->abort, p.status, 0x202, 0))) break;
-                    tc_fence_after();
-                    if (leader) {
-                        const uint64_t bdesc = bdesc0 + static_cast<uint64_t>(s * b_step);
-                        const uint64_t adesc = adesc0 + static_cast<uint64_t>(s * a_step);
-                        if constexpr (KPS == 2) {                    // two k blocks, one accumulator
-                            const int nb = min(2, item.nkb - kb);
-                            for (int c = 0; c < nb; ++c) {
-                                const uint64_t ad = adesc + static_cast<uint64_t>(c * (A_BYTES >> 4)), bd = bdesc + static_cast<uint64_t>(c * (x_stage >> 4));
+                if (leader) {
+                    const uint64_t bdesc = bdesc0 + static_cast<uint64_t>(s * b_step);
+                    const uint32_t ta = tmem_base + p.a_col0 + s * (KPS * A_COLS);
+                    if constexpr (KPS == 2) {                    // two k blocks, one accumulator
+                        const int nb = min(2, item.nkb - kb);
+#pragma unroll
+                        for (int c = 0; c < 2; ++c)
+                            if (c < nb) {
 #pragma unroll
                                 for (int k = 0; k < BK / 16; ++k)
-                                    umma_f16(tmem_d, ad + 2 * k, bd + 2 * k, p.idesc, (kb | c | k) ? 1u : 0u);
+                                    umma_f16_ts(tmem_d, ta + c * A_COLS + 8 * k, bdesc + static_cast<uint64_t>(c * c_step + 2 * k), p.idesc, (kb | c | k) ? 1u : 0u);
                             }
-                        } else {
-                            for (int c = 0; c < item.nc; ++c) {      // token chunk c accumulates in TMEM half c
-                                const uint64_t bd = bdesc + static_cast<uint64_t>(c * (x_stage >> 4));
+                    } else {
+                        for (int c = 0; c < item.nc; ++c) {      // token chunk c accumulates in accumulator c
 #pragma unroll
-                                for (int k = 0; k < BK / 16; ++k)   // 16 elements = 32 bytes further along the swizzled row
-                                    umma_f16(tmem_d + c * TN_MAX, adesc + 2 * k, bd + 2 * k, p.idesc, (kb | k) ? 1u : 0u);
-                            }
+                            for (int k = 0; k < BK / 16; ++k)   // 16 elements = 32 bytes further along the swizzled row
+                                umma_f16_ts(tmem_d + c * p.TN, ta + 8 * k, bdesc + static_cast<uint64_t>(c * c_step + 2 * k), p.idesc, (kb | k) ? 1u : 0u);
                         }
-                        umma_commit(&ctl->empty[s]);         // frees the stage when these MMAs have read it
                     }
-                    __syncwarp();
-                    if (++s == nst) {
-                        s = 0;
-                        ph ^= 1;
-                    }
+                    umma_commit(&ctl->empty[s]);         // frees the stage when these MMAs have read it
                 }
-                if (ok && leader) umma_commit(&ctl->acc_full[buf]);
                 __syncwarp();
+                if (++s == nst) {
+                    s = 0;
+                    ph ^= 1;
+                }
             }
+            if (ok && leader) umma_commit(&ctl->acc_full[buf]);
+            __syncwarp();
         }
     } else if (warp >= COPY_WARP0 && warp < COPY_WARP0 + COPY_THREADS / 32) {
-        // ---------------- copies: packed words and scales -> raw buffers ----------------
-        // A super-block of 4 k blocks of the tile at a time, up to nraw ahead of the dequant warps and across items.  4- and
+        // ---------------- copies: packed words, scales -> shared memory ----------------
+        // Words: a super-block of 4 k blocks of the tile at a time, up to nraw ahead of the dequant warps and across items.  4- and
         // 8-bit words are one or two TMA boxes (128 bytes x 128 rows, swizzled so that the rows' reads do not conflict);
-        // other widths and all scales are cp.async copies of these two warps.  Issued by the dequant warps themselves the
-        // copies cost them 380 of ~1050 cycles a k block, and 150 more behind the queue they filled.
+        // other widths are cp.async copies of these two warps.
+        // Scales and biases: rows lie apart, and a cp.async takes the load pipe some ten cycles a lane, so 64 bytes of a row are copied at a time, and where rows are
+        // whole 16-byte pieces by TMA.  (A bulk copy a row was slower than eight lanes: 333 x 7616 x 2880 28 -> 40 us.)
         if (p.raw) {
             using R = RawTile<BITS>;
             const int t = threadIdx.x - COPY_WARP0 * 32;
-            const uint32_t raw0 = smem_u32(smem) + p.raw_off;
-            const int sb_bytes = (2 * SB_PER_RAW * BK) >> p.gs_shift;       // scale bytes of a row per super-block: 16, 8 or 4
-            int buf = 0;
-            uint32_t ph = 0;
+            const uint32_t raw0 = smem_u32(smem) + p.raw_off, sp0 = smem_u32(smem) + p.sp_off;
+            const int pitch = sp_pitch(p.sp_bytes);
+            int buf = 0, sp = 0;
+            uint32_t ph = 0, sph = 0;
             bool ok = true;
             for (int i = blockIdx.x; i < num_items && ok; i += gridDim.x) {
                 const Item im = get_item<KSPLIT>(p, i);
                 const int n0 = im.n_tile * BMW;
                 const size_t erow = static_cast<size_t>(im.expert) * p.N;
-                const int sb0 = (KSPLIT ? im.kb0 : 0) / SB_PER_RAW, sb1 = sb0 + (im.nkb + SB_PER_RAW - 1) / SB_PER_RAW;
-                for (int sbk = sb0; sbk < sb1; ++sbk) {
+                const int kb_first = KSPLIT ? im.kb0 : 0;
+                int sp_next = 0;                         // where the next span starts
+                for (int kb0 = 0; kb0 < im.nkb; kb0 += p.raw_blk) {
+                    if (kb0 == sp_next) {
+                        sp_next += p.sp_kb - (kb_first + kb0) % p.sp_kb;
+                        if (!(ok = mbar_wait_warp(&ctl->sp_empty[sp], sph ^ 1, &ctl->abort, p.status, 0x502, p.hint_ns))) break;
+                        const int g0 = ((kb_first + kb0) * BK) >> p.gs_shift, n = ((min(sp_next, im.nkb) - kb0) * BK + (1 << p.gs_shift) - 1) >> p.gs_shift;
+                        const uint32_t dst0 = sp0 + sp * sp_buffer(p.sp_bytes), dsts = dst0 + (warp == COPY_WARP0 ? 0 : BMW * pitch);
+                        const unsigned short *const arr = static_cast<const unsigned short *>(warp == COPY_WARP0 ? p.scales : p.biases);
+                        if (p.sp_copy == 2) {
+                            if (t == 0) {                // rows past the array and groups past the row arrive as zeros
+                                const int first = g0 & ~(p.sp_bytes / 2 - 1), row = static_cast<int>(erow) + n0;
+                                mbar_expect_tx(&ctl->sp_full[sp], 2 * BMW * p.sp_bytes);
+                                tma_load_2d(dst0, &maps.scales, first, row, &ctl->sp_full[sp]);
+                                tma_load_2d(dst0 + BMW * pitch, &maps.biases, first, row, &ctl->sp_full[sp]);
+                            }
+                        } else {
+                            if (p.sp_copy == 1) {
+                                // one warp the scales, the other the biases, eight lanes a row (four: 32 bytes of a row)
+                                const unsigned long long b0 = reinterpret_cast<unsigned long long>(arr + (static_cast<size_t>(erow) + n0) * p.gpr + g0);
+                                const char *const from = reinterpret_cast<const char *>(b0 & ~15ull);
+                                const long long behind = reinterpret_cast<const char *>(arr + p.sb_total) - from;       // to the array's end: nothing past it is read
+                                const int left = static_cast<int>(min(behind, 0x7FFFFFFFll)), last = p.N - 1 - n0, low = static_cast<int>(b0 & 15), rb = p.gpr * 2;
+                                auto rows = [&](auto lanes) {
+                                    constexpr int L = decltype(lanes)::value, STEP = 32 / L;
+                                    const int c = (lane % L) * 16;
+                                    uint32_t dd = dsts + (lane / L) * pitch + c;
+#pragma unroll 4
+                                    for (int row = lane / L; row < BMW; row += STEP, dd += STEP * pitch) {
+                                        const int at = low + min(row, last) * rb, piece = (at & ~15) + c;       // rows past N copy the last row; never stored
+                                        if (piece < at + 2 * n) cp_async_16_of(dd, from + piece, min(16, left - piece));
+                                    }
+                                };
+                                if (p.sp_bytes == 64) rows(std::integral_constant<int, 8>{});
+                                else rows(std::integral_constant<int, 4>{});
+                            } else {
+                                // the words that cover them; the element that ends the array alone in its word is copied by itself
+                                for (int row = 0; row < BMW; ++row) {
+                                    const size_t el0 = (erow + min(n0 + row, p.N - 1)) * p.gpr + g0;
+                                    const long long el = static_cast<long long>(el0 & ~static_cast<size_t>(1)) + 2 * lane;
+                                    const uint32_t dd = dsts + row * pitch + lane * 4;
+                                    if (lane <= n / 2) {
+                                        if (el + 1 < p.sb_total) {
+                                            cp_async_small<4>(dd, arr + el);
+                                        } else if (el < p.sb_total) {
+                                            asm volatile("st.shared.u16 [%0], %1;" ::"r"(dd), "h"(__ldg(arr + el)) : "memory");
+                                            __threadfence_block();
+                                        }
+                                    }
+                                }
+                            }
+                            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&ctl->sp_full[sp])) : "memory");
+                        }
+                        sph ^= sp;
+                        sp ^= 1;
+                    }
                     if (!(ok = mbar_wait_warp(&ctl->raw_empty[buf], ph ^ 1, &ctl->abort, p.status, 0x501, p.hint_ns))) break;
                     const uint32_t dstt = raw0 + buf * p.raw_tile;
                     if constexpr (R::TMA) {
                         if (t == 0) {
-                            mbar_expect_tx(&ctl->raw_full[buf], R::SB_OFF);
+                            mbar_expect_tx(&ctl->raw_full[buf], BMW * R::BLK_BYTES * p.raw_blk);
                             // rows past the array and words past the row arrive as zeros; rows past N are never stored
-#pragma unroll
-                            for (int q = 0; q < BITS / 4; ++q)
-                                tma_load_2d(dstt + q * (BMW * 128), &tmap_w, sbk * (8 * BITS) + q * 32, static_cast<int>(erow) + n0, &ctl->raw_full[buf]);
+                            for (int q = 0; q < p.raw_blk * R::BLK_BYTES / 128; ++q)
+                                tma_load_2d(dstt + q * (BMW * 128), &maps.w, (kb_first + kb0) * (2 * BITS) + q * 32, static_cast<int>(erow) + n0, &ctl->raw_full[buf]);
                         }
                     } else {
-                        if (t == 0) mbar_arrive(&ctl->raw_full[buf]);
-                        const int bytes = min(SB_PER_RAW, p.K / BK - sbk * SB_PER_RAW) * (8 * BITS);   // the last one of a row may be short
-                        const char *src = reinterpret_cast<const char *>(p.w) + static_cast<size_t>(sbk) * R::ROW_BYTES;
+                        const int bytes = min(p.raw_blk, p.K / BK - kb_first - kb0) * (8 * BITS);   // the last one of a row may be short
+                        const char *src = reinterpret_cast<const char *>(p.w) + static_cast<size_t>(kb_first + kb0) * (8 * BITS);
                         if (!p.raw8) {
                             constexpr int CPR = 2 * BITS;
 #pragma unroll 4
                             for (int ch = t; ch < BMW * CPR; ch += COPY_THREADS) {
                                 const int row = ch / CPR, col = ch - row * CPR;
-                                const size_t grow = erow + min(n0 + row, p.N - 1);          // rows past N copy the last row; never stored
+                                const size_t grow = erow + min(n0 + row, p.N - 1);
                                 if (col * 16 < bytes) cp_async_16(dstt + row * R::PITCH + col * 16, src + grow * (p.wpr * 4) + col * 16);
                             }
                         } else {
@@ -576,38 +660,8 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                                 if (col * 8 < bytes) cp_async_small<8>(dstt + row * R::PITCH + col * 8, src + grow * (p.wpr * 4) + col * 8);
                             }
                         }
+                        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&ctl->raw_full[buf])) : "memory");
                     }
-                    const uint32_t d = dstt + R::SB_OFF;
-                    if (p.sb_words == 0) {
-#pragma unroll
-                        for (int e = 0; e < 2 * BMW / COPY_THREADS; ++e) {
-                            const int row = (e * COPY_THREADS + t) & (BMW - 1), arr = e >> 1;
-                            const size_t grow = erow + min(n0 + row, p.N - 1);
-                            const char *src = static_cast<const char *>(arr ? p.biases : p.scales) + (grow * p.gpr) * 2 + static_cast<size_t>(sbk) * sb_bytes;
-                            const uint32_t dd = d + arr * (BMW * 16) + row * 16;            // 16-byte pitch: one aligned copy
-                            if (sb_bytes == 16) cp_async_16(dd, src);
-                            else if (sb_bytes == 8) cp_async_small<8>(dd, src);
-                            else cp_async_small<4>(dd, src);
-                        }
-                    } else {
-                        // rows of scales start anywhere: the 4-byte words that cover the super-block's, neighbouring lanes on
-                        // neighbouring words; the element that ends the array alone in its word is copied by itself
-                        const int nw = p.sb_words;
-                        for (int e = t; e < 2 * BMW * nw; e += COPY_THREADS) {
-                            const int rowa = e / nw, wd = e - rowa * nw, arr = rowa >> 7, row = rowa & (BMW - 1);
-                            const size_t grow = erow + min(n0 + row, p.N - 1);
-                            const long long el = static_cast<long long>(((grow * p.gpr + static_cast<size_t>(sbk) * (sb_bytes / 2)) & ~static_cast<size_t>(1)) + 2 * wd);
-                            const unsigned short *base = static_cast<const unsigned short *>(arr ? p.biases : p.scales);
-                            const uint32_t dd = d + rowa * RAW_SB_PITCH + wd * 4;
-                            if (el + 1 < p.sb_total) {
-                                cp_async_small<4>(dd, base + el);
-                            } else if (el < p.sb_total) {
-                                asm volatile("st.shared.u16 [%0], %1;" ::"r"(dd), "h"(__ldg(base + el)) : "memory");
-                                __threadfence_block();
-                            }
-                        }
-                    }
-                    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&ctl->raw_full[buf])) : "memory");
                     if (++buf == p.nraw) {
                         buf = 0;
                         ph ^= 1;
@@ -615,9 +669,11 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                 }
             }
             asm volatile("cp.async.wait_all;" ::: "memory");
-            if (!ok && R::TMA) {   // let copies already in flight land before the CTA tears down
-                for (int b = 0; b < p.nraw; ++b)
+            if (!ok) {             // let copies already in flight land before the CTA tears down
+                for (int b = 0; R::TMA && b < p.nraw; ++b)
                     for (uint32_t j = 0; j < 4096 && !mbar_try(&ctl->raw_full[b], 0) && !mbar_try(&ctl->raw_full[b], 1); ++j) {}
+                for (int b = 0; b < 2; ++b)
+                    for (uint32_t j = 0; j < 4096 && !mbar_try(&ctl->sp_full[b], 0) && !mbar_try(&ctl->sp_full[b], 1); ++j) {}
             }
         }
     } else if (warp >= EPI_WARP0 && warp < EPI_WARP0 + 4) {
@@ -636,10 +692,10 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
         uint32_t tile_i = 0;
         bool ok = true;
         if (p.pdl_roles) asm volatile("griddepcontrol.wait;" ::: "memory");          // token factors; nothing is stored before this
-        for (int i = blockIdx.x; i < num_items && ok; i += gridDim.x, ++tile_i) {
-            const bool both = p.wide != 0;
-            const int buf = both ? 0 : (tile_i & 1);
-            const uint32_t acc_ph = (both ? tile_i : (tile_i >> 1)) & 1;
+        // slices that add up in a cluster leave the accumulators through all warps, below
+        for (int i = KSPLIT && p.cluster ? num_items : blockIdx.x; i < num_items && ok; i += gridDim.x, ++tile_i) {
+            const int buf = p.nacc == 2 ? tile_i & 1 : 0;
+            const uint32_t acc_ph = (p.nacc == 2 ? tile_i >> 1 : tile_i) & 1;
             const Item item = get_item<KSPLIT>(p, i);
             ok = mbar_wait_warp(&ctl->acc_full[buf], acc_ph, &ctl->abort, p.status, 0x301, p.hint_ns);
             // The four warps share named barriers below, so they give up together: a warp that gave up while another saw the
@@ -654,23 +710,10 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                 const int row_base = item.row0 + c * p.TN;
                 const int rows_h = item.nc == 2 ? min(p.TN, item.rows - c * p.TN) : item.rows;
                 if constexpr (KSPLIT) {
-                    if (p.cluster) {
-                        // the MMAs of the CTA's only item are complete: its ring becomes [token][128 outputs] of f32
-                        float *o = reinterpret_cast<float *>(smem) + c * p.TN * BMW + q * 32 + lane;
-                        for (int c0 = 0; c0 < rows_h; c0 += 32) {
-                            uint32_t v[32];
-                            tmem_ld<32>(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + (buf + hh) * TN_MAX + c0, v);
-                            tmem_wait_ld();
-#pragma unroll
-                            for (int j = 0; j < 32; ++j)
-                                if (c0 + j < rows_h) o[(c0 + j) * BMW] = __uint_as_float(v[j]);
-                        }
-                        continue;
-                    }
                     // a K slice: f32 partial sums, 32 token rows at a time in 128-byte segments per warp and row
                     for (int c0 = 0; c0 < rows_h; c0 += 32) {
                         uint32_t v[32];
-                        tmem_ld<32>(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + (buf + hh) * TN_MAX + c0, v);
+                        tmem_ld<32>(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + (buf + hh) * p.TN + c0, v);
                         tmem_wait_ld();
                         if (!n_ok) continue;
                         float *o = p.partial + (static_cast<size_t>(item.ks) * p.M + row_base + c0) * p.N + n;
@@ -698,7 +741,7 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                         }
                     }
                     uint32_t v[2][8];
-                    tmem_ld_frag(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + (buf + hh) * TN_MAX + c0, v);
+                    tmem_ld_frag(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + (buf + hh) * p.TN + c0, v);
                     const uint32_t sb = epi0 + (epi_buf & 1) * (EPI_TOK * EPI_PITCH);
                     ++epi_buf;
 #pragma unroll
@@ -733,163 +776,204 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
             if (lane == 0) mbar_arrive(&ctl->acc_empty[buf]);
         }
     } else if (warp >= DEQ_WARP0) {
-        // ---------------- dequant: packed W rows -> swizzled A operand tile ----------------
-        const int t = threadIdx.x - DEQ_WARP0 * 32;
-        const int r = t & (BMW - 1);                       // row of the W tile
-        const int h = t >> 7;                              // which 32-code half of the 64-wide k block
-        const int r7 = r & 7;
-        uint32_t dst[4];                                   // this thread's four swizzled 16-byte chunks in stage 0
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-            dst[c] = smem_u32(sW) + (r >> 3) * 1024 + r7 * 128 + (((h * 4 + c) ^ r7) << 4);
-        int s = 0;
-        uint32_t ph = 0;                                  // stage and ring-pass parity, advanced without a division
-        bool ok = true;
-        if (p.raw) {
-            // packed words and scales through the raw buffers that the copy warps fill
+        // ---------------- dequant: packed W rows -> A operand ----------------
+        const int q = warp & 3, team = (warp - DEQ_WARP0) >> 2, r = q * 32 + lane;      // row of the W tile; q: the TMEM lanes this warp may write
+        const uint32_t ta0 = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + p.a_col0;
+        // A team that comes to a stage has waited for the one that it had before, `teams` stages back: no further back than the ring is deep, or a phase of
+        // the barrier two passes old would look like the one it waits for.
+        const int teams = min(TEAMS, nst);
+        int s = 0, turn = 0;                              // stage, and the team whose stage it is
+        uint32_t ph = 0;                                  // ring-pass parity, advanced without a division
+        const bool second = p.gs_shift == 5;              // groups of 32: two scales a k block
+        auto convert = [&](auto words, uint32_t s0, uint32_t s1, uint32_t b0, uint32_t b1, uint32_t at) {
+            uint32_t v[32];
+            if (second) dequant_block<BITS, false>(words, sb_value(s0, p.sb_dt), sb_value(b0, p.sb_dt), sb_value(s1, p.sb_dt), sb_value(b1, p.sb_dt), v);
+            else dequant_block<BITS, true>(words, sb_value(s0, p.sb_dt), sb_value(b0, p.sb_dt), 0.0f, 0.0f, v);
+            tmem_st32(at, v);
+        };
+        const uint32_t bars = __shfl_sync(0xffffffffu, smem_u32(ctl), 0), abort = bars + offsetof(SmemCtrl, abort);
+        auto wait = [&](uint32_t bar, uint32_t parity, uint32_t code) {
+            const bool done = mbar_wait(bars + bar, parity, abort, p.status, code);
+            __syncwarp();
+            return done;
+        };
+        auto stage_free = [&]() {
+            const bool done = wait(offsetof(SmemCtrl, empty) + s * 8, ph ^ 1, 0x401);
+            tc_fence_after();
+            return done;
+        };
+        auto stage_done = [&]() {
+            tmem_wait_st();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bars + static_cast<uint32_t>(offsetof(SmemCtrl, full)) + s * 8);
+        };
+        auto next_stage = [&]() {
+            if (++turn == teams) turn = 0;
+            if (++s == nst) {
+                s = 0;
+                ph ^= 1;
+            }
+        };
+        // packed words and scales through the buffers that the copy warps fill
+        auto through_buffers = [&]() {
             using R = RawTile<BITS>;
-            const uint32_t raw0 = smem_u32(smem) + p.raw_off;
-            const int nraw = p.nraw;
-            const int sb_elems = (SB_PER_RAW * BK) >> p.gs_shift;           // scales of a row per super-block: 8, 4 or 2
+            const int nraw = p.nraw, gsh = p.gs_shift;
+            const uint32_t raw0 = smem_u32(smem) + p.raw_off, sp0 = smem_u32(smem) + p.sp_off, bias_off = BMW * sp_pitch(p.sp_bytes);
+            // a box's rows are sp_bytes apart, their 16-byte pieces swizzled as TMA does for that width
+            const bool by_tma = p.sp_copy == 2;
+            const uint32_t piece_of = p.sp_bytes == 64 ? (r >> 1) & 3 : (r >> 2) & 1, in_row = p.sp_bytes - 1;
             int buf = 0;
-            uint32_t buf_ph = 0;
-            for (int i = blockIdx.x; i < num_items && ok; i += gridDim.x) {
+            uint32_t buf_ph = 0, sp = 0, sph = 0;
+            for (int i = blockIdx.x; i < num_items; i += gridDim.x) {
                 const Item item = get_item<KSPLIT>(p, i);
-                for (int kb0 = 0; kb0 < item.nkb && ok; kb0 += SB_PER_RAW) {
-                    if (!(ok = mbar_wait_warp(&ctl->raw_full[buf], buf_ph, &ctl->abort, p.status, 0x402, 0))) break;
+                const int kb_first = KSPLIT ? item.kb0 : 0;
+                // the row's first scale, modulo 2^32: its place in a buffer, since copies start on boundaries of 16 (or 4) bytes
+                const uint32_t el0 = (static_cast<uint32_t>(item.expert) * p.N + min(item.n_tile * BMW + r, p.N - 1)) * p.gpr;
+                uint32_t scales = 0;                     // where those of the span lie, less the groups before it
+                int sp_next = 0;                         // where the next span starts
+                for (int kb0 = 0; kb0 < item.nkb; kb0 += p.raw_blk) {
+                    if (kb0 == sp_next) {
+                        if (!wait(offsetof(SmemCtrl, sp_full) + sp * 8, sph, 0x403)) return;
+                        const uint32_t g = ((kb_first + kb0) * BK) >> gsh, buffer = sp0 + sp * sp_buffer(p.sp_bytes);
+                        scales = by_tma ? buffer + r * p.sp_bytes : buffer + r * sp_pitch(p.sp_bytes) + ((el0 + g) & (p.sp_copy ? 7 : 1)) * 2 - 2 * g;
+                        sp_next += p.sp_kb - (kb_first + kb0) % p.sp_kb;
+                    }
+                    if (!wait(offsetof(SmemCtrl, raw_full) + buf * 8, buf_ph, 0x402)) return;
                     const uint32_t base = raw0 + buf * p.raw_tile;
-                    // the row's scales and biases of the whole super-block (4, 8 or 16 bytes are in use)
-                    uint4 sline, bline;
-                    if (p.sb_words == 0) {
-                        const uint32_t sb_addr = base + R::SB_OFF + r * 16;
-                        asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(sline.x), "=r"(sline.y), "=r"(sline.z), "=r"(sline.w) : "r"(sb_addr));
-                        asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(bline.x), "=r"(bline.y), "=r"(bline.z), "=r"(bline.w) : "r"(sb_addr + BMW * 16));
-                    } else {
-                        const size_t grow = static_cast<size_t>(item.expert) * p.N + min(item.n_tile * BMW + r, p.N - 1);
-                        const int sbk = ((KSPLIT ? item.kb0 : 0) + kb0) / SB_PER_RAW;
-                        const int sh = static_cast<int>((grow * p.gpr + static_cast<size_t>(sbk) * sb_elems) & 1) * 16;
-                        uint32_t v[2][5];
-#pragma unroll
-                        for (int arr = 0; arr < 2; ++arr)
-#pragma unroll
-                            for (int j = 0; j < 5; ++j) {
-                                v[arr][j] = 0u;
-                                if (j < p.sb_words)
-                                    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v[arr][j]) : "r"(base + R::SB_OFF + (arr * BMW + r) * RAW_SB_PITCH + j * 4));
+                    const int end = min(p.raw_blk, item.nkb - kb0);
+#pragma unroll 1
+                    for (int j = 0; j < end; j += KPS) {
+                        if (turn == team) {
+                            if (!stage_free()) return;
+#pragma unroll 1
+                            for (int c = 0; c < KPS; ++c) {
+                                if (KPS > 1 && j + c >= end) break;
+                                const uint32_t at = (((kb_first + kb0 + j + c) * BK) >> gsh) << 1;          // of the row
+                                const uint32_t sa = scales + (by_tma ? (at & in_row) ^ (piece_of << 4) : at), sb = sa + bias_off;
+                                convert([&](int h, uint32_t (&w)[BITS]) { R::read(base, r, j + c, h, w); }, lds_u16(sa), second ? lds_u16(sa + 2) : 0u, lds_u16(sb), second ? lds_u16(sb + 2) : 0u, ta0 + (s * KPS + c) * A_COLS);
                             }
-                        sline = make_uint4(__funnelshift_r(v[0][0], v[0][1], sh), __funnelshift_r(v[0][1], v[0][2], sh),
-                                           __funnelshift_r(v[0][2], v[0][3], sh), __funnelshift_r(v[0][3], v[0][4], sh));
-                        bline = make_uint4(__funnelshift_r(v[1][0], v[1][1], sh), __funnelshift_r(v[1][1], v[1][2], sh),
-                                           __funnelshift_r(v[1][2], v[1][3], sh), __funnelshift_r(v[1][3], v[1][4], sh));
-                    }
-#pragma unroll
-                    for (int j = 0; j < SB_PER_RAW; ++j) {
-                        if (kb0 + j >= item.nkb) break;
-                        uint32_t wv[BITS];                   // read before the wait for the stage
-                        R::read(base, r, j, h, wv);
-                        const uint32_t sub = KPS == 2 ? j & 1 : 0;              // k block of the stage
-                        if (sub == 0 && !(ok = mbar_wait_warp(&ctl->empty[s], ph ^ 1, &ctl->abort, p.status, 0x401, 0))) break;
-                        {
-                            const unsigned short sr = static_cast<unsigned short>(sb_half(sline, j, h, p.gs_shift));
-                            const unsigned short br = static_cast<unsigned short>(sb_half(bline, j, h, p.gs_shift));
-                            float sc, bi;
-                            if (p.sb_dt == MTC_F16) {
-                                sc = __half2float(__ushort_as_half(sr));
-                                bi = __half2float(__ushort_as_half(br));
-                            } else {
-                                sc = __uint_as_float(static_cast<uint32_t>(sr) << 16);
-                                bi = __uint_as_float(static_cast<uint32_t>(br) << 16);
-                            }
-                            dequant_half<BITS>(wv, sc, bi, dst, s * w_stage + sub * A_BYTES);
+                            stage_done();
                         }
-                        if (KPS == 2 && sub == 0 && kb0 + j + 1 < item.nkb) continue;
-                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic-proxy stores -> async proxy (MMA)
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(&ctl->full[s]);
-                        if (++s == nst) {
-                            s = 0;
-                            ph ^= 1;
-                        }
+                        next_stage();
                     }
+                    const bool sp_done = kb0 + p.raw_blk == sp_next || kb0 + p.raw_blk >= item.nkb;
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(&ctl->raw_empty[buf]);
+                    if (lane == 0) {
+                        mbar_arrive(bars + static_cast<uint32_t>(offsetof(SmemCtrl, raw_empty)) + buf * 8);
+                        if (sp_done) mbar_arrive(bars + static_cast<uint32_t>(offsetof(SmemCtrl, sp_empty)) + sp * 8);
+                    }
                     if (++buf == nraw) {
                         buf = 0;
                         buf_ph ^= 1;
                     }
+                    if (sp_done) {
+                        sph ^= sp;
+                        sp ^= 1;
+                    }
                 }
             }
-        } else
-        for (int i = blockIdx.x; i < num_items && ok; i += gridDim.x) {
-            const Item item = get_item<KSPLIT>(p, i);
-            const int n = item.n_tile * BMW + r;
-            const bool valid = n < p.N;
-            const size_t grow = static_cast<size_t>(item.expert) * p.N + (valid ? n : 0);
-            const uint32_t *wrow = p.w + grow * p.wpr + h * BITS;
-            const unsigned short *sc16 = static_cast<const unsigned short *>(p.scales) + grow * p.gpr;
-            const unsigned short *bi16 = static_cast<const unsigned short *>(p.biases) + grow * p.gpr;
-            uint32_t wnext[BITS];
-            uint32_t sn = 0, bn = 0;                       // raw 16-bit scale / bias, converted when used
-            auto request = [&](int kb) {
-                load_half_words<BITS>(wrow + static_cast<size_t>(kb) * (2 * BITS), wnext, valid);
-                if (valid) {
-                    const int g = (kb * BK + h * 32) >> p.gs_shift;
-                    sn = __ldg(sc16 + g);
-                    bn = __ldg(bi16 + g);
-                }
-            };
-            const int kb0 = KSPLIT ? item.kb0 : 0;
-            request(kb0);
-            for (int kb = 0; kb < item.nkb; ++kb) {
-                uint32_t wcur[BITS];
+        };
+        // straight from global memory
+        auto from_memory = [&]() {
+            for (int i = blockIdx.x; i < num_items; i += gridDim.x) {
+                const Item item = get_item<KSPLIT>(p, i);
+                const int n = item.n_tile * BMW + r;
+                const bool valid = n < p.N;
+                const size_t grow = static_cast<size_t>(item.expert) * p.N + (valid ? n : 0);
+                const uint32_t *wrow = p.w + grow * p.wpr;
+                const unsigned short *sc16 = static_cast<const unsigned short *>(p.scales) + grow * p.gpr;
+                const unsigned short *bi16 = static_cast<const unsigned short *>(p.biases) + grow * p.gpr;
+                const int kb0 = KSPLIT ? item.kb0 : 0;
+                uint32_t w[2][BITS];
+                uint32_t sv[2] = {0, 0}, bv[2] = {0, 0};      // raw 16-bit scales / biases, converted when used
+                auto request = [&](int kb) {                  // a k block of this team's, asked for a turn ahead
 #pragma unroll
-                for (int j = 0; j < BITS; ++j) wcur[j] = wnext[j];
-                const uint32_t sr = sn, br = bn;
-                if (kb + 1 < item.nkb) request(kb0 + kb + 1);      // the next k block is requested before this one is converted
-                // the stage is free once empty[s] has completed (the producer waits on the same barrier)
-                if (!(ok = mbar_wait_warp(&ctl->empty[s], ph ^ 1, &ctl->abort, p.status, 0x401, 0))) break;
-                float sc, bi;
-                if (p.sb_dt == MTC_F16) {
-                    sc = __half2float(__ushort_as_half(static_cast<unsigned short>(sr)));
-                    bi = __half2float(__ushort_as_half(static_cast<unsigned short>(br)));
-                } else {
-                    sc = __uint_as_float(sr << 16);
-                    bi = __uint_as_float(br << 16);
-                }
-                dequant_half<BITS>(wcur, sc, bi, dst, s * w_stage);
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic-proxy stores -> async proxy (MMA)
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&ctl->full[s]);
-                if (++s == nst) {
-                    s = 0;
-                    ph ^= 1;
+                    for (int h = 0; h < 2; ++h) {
+                        load_half_words<BITS>(wrow + static_cast<size_t>(kb0 + kb) * (2 * BITS) + h * BITS, w[h], valid);
+                        const int g = ((kb0 + kb) * BK + h * 32) >> p.gs_shift;
+                        sv[h] = valid ? __ldg(sc16 + g) : 0u;
+                        bv[h] = valid ? __ldg(bi16 + g) : 0u;
+                    }
+                };
+                const int mine = team >= turn ? team - turn : team - turn + teams;        // this team's first k block of the item
+                if (team < teams && mine < item.nkb) request(mine);
+                for (int kb = 0; kb < item.nkb; ++kb) {
+                    if (turn == team) {
+                        if (!stage_free()) return;
+                        convert([&](int h, uint32_t (&to)[BITS]) {
+#pragma unroll
+                            for (int e = 0; e < BITS; ++e) to[e] = w[h][e];
+                        }, sv[0], sv[1], bv[0], bv[1], ta0 + s * A_COLS);
+                        if (kb + teams < item.nkb) request(kb + teams);
+                        stage_done();
+                    }
+                    next_stage();
                 }
             }
-        }
+        };
+        if (p.raw) through_buffers();
+        else from_memory();
     }
 
     if constexpr (KSPLIT) {
         if (p.cluster) {
-            // The sum over the slices in slice order, the token factors, the stores: a CTA takes its share of the token rows, a warp a row, a
-            // lane four outputs.  Every role of every CTA comes here, also one that gave up.
+            // The sum over the slices in slice order, the token factors, the stores: a CTA takes its share of the blocks of 16 token rows.  The others
+            // push theirs of it into its ring, which is free when all MMAs of the cluster are complete: stores to another SM are not waited for, loads
+            // from it were 2 us of a product (and sums left to the four epilogue warps 6).  Every role of every CTA comes here, also one that gave up.
             asm volatile("griddepcontrol.wait;" ::: "memory");
             __syncwarp();
-            cluster_sync();
             const Item item = get_item<KSPLIT>(p, blockIdx.x);
-            const int n = item.n_tile * BMW + lane * 4, left = p.N - n;
-            const uint32_t mine = smem_u32(smem) + lane * 16;
-            for (int j = item.rows * item.ks / p.ksplit + warp; j < item.rows * (item.ks + 1) / p.ksplit; j += NUM_THREADS / 32) {
-                float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                for (int r = 0; r < p.ksplit; ++r) {
-                    uint32_t a;
-                    float4 t;
-                    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(mine + j * (BMW * 4)), "r"(r));
-                    asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(t.x), "=f"(t.y), "=f"(t.z), "=f"(t.w) : "r"(a) : "memory");
-                    if (r == 0) v = t;
-                    else { v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w; }
+            const int S = p.ksplit, me = item.ks, blocks = item.nc * p.TN / 16, most = (blocks + S - 1) / S;
+            const int first = blocks * me / S, own = blocks * (me + 1) / S - first;
+            constexpr uint32_t BLOCK = 16 * BMW * 4;                       // a block of sums: [16 token rows][128 outputs] of f32
+            const uint32_t mine = smem_u32(smem) + ((warp & 3) * 32 + lane) * 4, lanes = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+            const bool ok = mbar_wait_warp(&ctl->acc_full[0], 0, &ctl->abort, p.status, 0x302, p.hint_ns);
+            tc_fence_after();
+            cluster_sync();
+            if (ok) {
+#pragma unroll 1
+                for (int c = warp >> 2; c < blocks; c += NUM_THREADS / 128) {
+                    const int to = ((c + 1) * S - 1) / blocks;             // blocks * to / S <= c < blocks * (to + 1) / S
+                    if (to == me) continue;
+                    uint32_t v[16], a;
+                    tmem_ld<16>(lanes + c * 16, v);
+                    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(mine + ((me < to ? me : me - 1) * most + c - blocks * to / S) * BLOCK), "r"(to));
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(a + j * (BMW * 4)), "r"(v[j]) : "memory");
                 }
-                if (left <= 0) continue;
-                const int m = item.row0 + j;
+            }
+            cluster_sync();
+            if (ok) {
+#pragma unroll 1
+                for (int c = warp >> 2; c < own; c += NUM_THREADS / 128) {
+                    uint32_t v[16];
+                    tmem_ld<16>(lanes + (first + c) * 16, v);
+                    tmem_wait_ld();
+                    float sum[16];
+#pragma unroll 1
+                    for (int r = 0; r < S; ++r) {
+                        const uint32_t a = mine + ((r < me ? r : r - 1) * most + c) * BLOCK;
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) {
+                            float t = __uint_as_float(v[j]);
+                            if (r != me) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(t) : "r"(a + j * (BMW * 4)) : "memory");
+                            sum[j] = r == 0 ? t : sum[j] + t;
+                        }
+                    }
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) asm volatile("st.shared.f32 [%0], %1;" ::"r"(mine + c * BLOCK + j * (BMW * 4)), "f"(sum[j]) : "memory");
+                }
+            }
+            __syncthreads();
+            // a warp a row, a lane four outputs
+            const int n = item.n_tile * BMW + lane * 4, left = p.N - n;
+            for (int j = warp; j < own * 16; j += NUM_THREADS / 32) {
+                if (left <= 0 || first * 16 + j >= item.rows) continue;
+                float4 v;
+                asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(smem_u32(smem) + j * (BMW * 4) + lane * 16) : "memory");
+                const int m = item.row0 + first * 16 + j;
                 if (p.tok_scale) {
                     const float f = p.tok_scale[m];
                     v.x *= f; v.y *= f; v.z *= f; v.w *= f;
@@ -908,7 +992,6 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                     }
                 }
             }
-            cluster_sync();                              // no CTA leaves while another reads its sums
         }
     }
     tc_fence_before();
@@ -1068,7 +1151,7 @@ constexpr size_t qmm_smem_bytes() {
 }
 
 template <int BITS>
-cudaError_t launch_bits(cudaStream_t st, const CUtensorMap &tmap, const CUtensorMap &wmap, const QmmParams &p, int grid) {
+cudaError_t launch_bits(cudaStream_t st, const QmmMaps &maps, const QmmParams &p, int grid) {
     constexpr size_t smem = qmm_smem_bytes<BITS>();
     static_assert(smem <= 227 * 1024, "shared memory per CTA");
     cudaLaunchConfig_t cfg{};
@@ -1087,7 +1170,7 @@ cudaError_t launch_bits(cudaStream_t st, const CUtensorMap &tmap, const CUtensor
     cfg.numAttrs = p.cluster ? 2 : 1;
     auto go = [&](auto kern, PerDeviceAttr &attr) {
         cudaError_t e = attr.set(kern, smem);
-        return e != cudaSuccess ? e : cudaLaunchKernelEx(&cfg, kern, tmap, wmap, p);
+        return e != cudaSuccess ? e : cudaLaunchKernelEx(&cfg, kern, maps, p);
     };
     static PerDeviceAttr attr[4];
     if (p.kps == 2) return p.ksplit > 1 ? go(qmm_tcgen05_kernel<BITS, true, 2>, attr[0]) : go(qmm_tcgen05_kernel<BITS, false, 2>, attr[1]);
@@ -1100,42 +1183,60 @@ cudaError_t make_x_map(CUtensorMap *tmap, const void *x, int rows, int K, int TN
 }
 
 cudaError_t launch_any(int bits, cudaStream_t st, const CUtensorMap &tmap, const QmmParams &p, int grid, long long w_rows, std::string *why) {
-    CUtensorMap wmap = tmap;                            // not read where the words do not travel by TMA
-    if (p.raw && (bits == 4 || bits == 8)) {
-        // packed words [rows, words], box 128 bytes x 128 rows
-        cudaError_t e = make_map_2d(&wmap, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, p.w, w_rows, p.wpr, BMW, 32, why);
-        if (e != cudaSuccess) return e;
+    QmmMaps maps{tmap, tmap, tmap, tmap};                // what does not travel by TMA is not read
+    cudaError_t e = cudaSuccess;
+    // packed words [rows, words], boxes of 128 bytes x 128 rows; scales and biases [rows, groups], of sp_bytes x 128 rows
+    if (p.raw && (bits == 4 || bits == 8)) e = make_map_2d(&maps.w, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, p.w, w_rows, p.wpr, BMW, 32, why);
+    if (p.raw && p.sp_copy == 2) {
+        if (e == cudaSuccess) e = make_map_2d(&maps.scales, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, p.scales, w_rows, p.gpr, BMW, p.sp_bytes / 2, why);
+        if (e == cudaSuccess) e = make_map_2d(&maps.biases, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, p.biases, w_rows, p.gpr, BMW, p.sp_bytes / 2, why);
     }
+    if (e != cudaSuccess) return e;
     switch (bits) {
-        case 2: return launch_bits<2>(st, tmap, wmap, p, grid);
-        case 3: return launch_bits<3>(st, tmap, wmap, p, grid);
-        case 4: return launch_bits<4>(st, tmap, wmap, p, grid);
-        case 5: return launch_bits<5>(st, tmap, wmap, p, grid);
-        case 6: return launch_bits<6>(st, tmap, wmap, p, grid);
-        default: return launch_bits<8>(st, tmap, wmap, p, grid);
+        case 2: return launch_bits<2>(st, maps, p, grid);
+        case 3: return launch_bits<3>(st, maps, p, grid);
+        case 4: return launch_bits<4>(st, maps, p, grid);
+        case 5: return launch_bits<5>(st, maps, p, grid);
+        case 6: return launch_bits<6>(st, maps, p, grid);
+        default: return launch_bits<8>(st, maps, p, grid);
     }
 }
 
-// Ring depth and raw staging buffers for p.TN / p.wide.  The raw path needs groups of 32, 64 or 128 (4 to 16 bytes of scales per
-// row and super-block) and 4-byte aligned scale / bias arrays.  Rows of scales that are whole super-blocks arrive as one
-// copy per row, others (K % 256 != 0) word by word.  A third raw buffer is taken where three ring stages remain.
+// Accumulators, ring depth, raw buffers and spans of scales for p.TN / p.wide.  The raw path needs groups of 32, 64 or 128 and 4-byte aligned scale / bias
+// arrays.  Two accumulators where they leave A four k blocks.  Two k blocks per hand-off up to 128 token rows: waits and arrivals are paid half as
+// often.  A third raw buffer and longer spans are taken where the ring keeps four stages beside them, or all that the columns of A hold.
 void plan_smem(QmmParams &p, Ctx *ctx, int bits) {
-    const int stage = A_BYTES + (p.wide ? 2 : 1) * p.TN * BK * 2;
     const auto al = [](const void *ptr, size_t n) { return reinterpret_cast<uintptr_t>(ptr) % n == 0; };
-    p.raw_tile = static_cast<uint32_t>(raw_bytes(bits));
-    p.nraw = RING_BYTES - 3 * static_cast<int>(p.raw_tile) >= 3 * stage ? 3 : 2;
-    const int raw_total = p.nraw * static_cast<int>(p.raw_tile);
-    p.raw = ctx->qmm_raw != 0 && p.gs_shift >= 5 && p.gs_shift <= 7 && al(p.scales, 4) && al(p.biases, 4) &&
-            (RING_BYTES - raw_total) / stage >= 2;
+    p.nacc = !p.wide && 2 * p.TN <= TMEM_COLS - 4 * A_COLS ? 2 : 1;
+    p.a_col0 = static_cast<uint32_t>((p.wide ? 2 : p.nacc) * p.TN);
+    p.raw = ctx->qmm_raw != 0 && p.gs_shift >= 5 && p.gs_shift <= 7 && al(p.scales, 4) && al(p.biases, 4);
     p.raw8 = (p.wpr * 4) % 16 != 0;
-    p.sb_words = p.K % (SB_PER_RAW * BK) == 0 && al(p.scales, 16) && al(p.biases, 16) ? 0 : ((2 * SB_PER_RAW * BK) >> p.gs_shift) / 4 + (p.gpr & 1);
-    // Two k blocks per hand-off where two such stages fit: waits, fence and arrival are paid half as often (64 token rows 0.51 ->
-    // 0.42 us a k block, 128 rows 0.54 -> 0.46); from ~200 rows on the deeper ring is worth more.
-    p.kps = p.raw && !p.wide && (RING_BYTES - raw_total) / (2 * stage) >= 2 ? 2 : 1;
-    p.nst = (RING_BYTES - (p.raw ? raw_total : 0)) / (p.kps * stage);
-    if (p.nst > MAX_STAGES) p.nst = MAX_STAGES;
+    p.raw_blk = bits == 8 && p.wide ? 2 : SB_PER_RAW;
+    p.raw_tile = static_cast<uint32_t>(raw_bytes(bits, p.raw_blk));
+    p.kps = p.raw && !p.wide && p.TN <= 128 ? 2 : 1;
+    const int slot = (p.wide || p.kps == 2 ? 2 : 1) * p.TN * BK * 2;
+    int most = (TMEM_COLS - static_cast<int>(p.a_col0)) / (A_COLS * p.kps);
+    if (most > MAX_STAGES) most = MAX_STAGES;
+    p.nraw = 0;
+    p.sp_bytes = 64;
+    p.nst = RING_BYTES / slot;
+    if (p.raw) {
+        // the first form whose ring is deep enough, else the last
+        const int fewest = p.raw_blk == 2 ? 3 : 2, want = most < 4 ? most : 4;
+        for (p.sp_bytes = 64; ; p.sp_bytes = 32) {
+            for (p.nraw = fewest + 1; ; --p.nraw) {
+                p.nst = (RING_BYTES - p.nraw * static_cast<int>(p.raw_tile) - 2 * sp_buffer(p.sp_bytes)) / slot;
+                if (p.nst >= want || p.nraw == fewest) break;
+            }
+            if (p.nst >= want || p.sp_bytes == 32) break;
+        }
+    }
+    if (p.nst > most) p.nst = most;
     if (ctx->qmm_max_stages > 0 && p.nst > ctx->qmm_max_stages) p.nst = ctx->qmm_max_stages;
-    p.raw_off = static_cast<uint32_t>(p.nst * p.kps * stage);
+    p.raw_off = static_cast<uint32_t>(p.nst * slot);
+    p.sp_off = p.raw_off + p.nraw * p.raw_tile;
+    p.sp_kb = ((p.sp_bytes / 2) << p.gs_shift) / BK;
+    p.sp_copy = !al(p.scales, 16) || !al(p.biases, 16) ? 0 : p.gpr % 8 == 0 ? 2 : 1;
 }
 
 void fill_common(QmmParams &p, Ctx *ctx, const void *w, const void *scales, const void *biases, void *out, int N, int K,
@@ -1192,18 +1293,24 @@ cudaError_t stage_x(Ctx *ctx, cudaStream_t st, const void *x, int rows, int K, i
     return cudaSuccess;
 }
 
-// Time of a k block of an item on one SM by its token rows, us (measured): the dequantisation sets the pace of narrow items.
-constexpr double kKbBase = 0.47, kKbPerToken = 0.0006;
-constexpr double kWideBase = 0.45, kWidePerToken = 0.00075;      // an item of two chunks
-constexpr double kSliceUs = 2e-6;       // an f32 partial sum: written at ~3 TB/s, read at ~6
+// Time of a k block of an item on one SM by its token rows, us (measured on 512 x 4096 x 4096, 2048 x 4096 x 4096 and 333 x 7616 x 2880, every width): up to 128
+// rows the hand-offs of two k blocks at a time, then of one, above some 210 rows the tensor cores at the clocks that the power leaves.  Other widths than 4
+// and 8 bits take more instructions a code; rows of scales that are no whole 16-byte pieces are copied by hand.
+double kb_cost(int TN, bool wide, int bits, bool pieces) {
+    const double more = (bits == 2 ? 0.035 : bits == 3 ? 0.053 : bits == 5 ? 0.11 : bits == 6 ? 0.135 : 0.0) + (pieces ? 0.0 : wide ? 0.02 : TN <= 128 ? 0.03 : 0.06);
+    if (wide) return 0.16 + 0.0017 * TN + more;
+    return (TN <= 128 ? 0.205 + 0.00045 * TN : TN <= 192 ? 0.31 : 0.31 + 0.0011 * (TN - 192)) + more;
+}
+constexpr double kSliceUs = 1.2e-6;     // an f32 partial sum, written and read
 // Clusters of one to eight CTAs, one CTA an SM, that are resident at once (cudaOccupancyMaxActiveClusters: the GPCs do not divide evenly)
 // (45 of three are, but with all of them at once products of x in bf16 took 1.1 to 1.2 times as long as with 44)
 constexpr int kClusters[9] = {0, 148, 74, 44, 33, 26, 22, 15, 15};
-constexpr double kClusterUs = 5.5;      // what a cluster's launch, barriers and sum cost at least
-// What launches take beyond the prices above, us over the leanest (means of 520 shapes of 17 to 1300 tokens, every format, sliced in memory and in
-// clusters in turn): the clusters of S CTAs, the pairs of two-chunk items, and the plans of 1, 2, 3, 4 and more slices without clusters
-constexpr double kClusterMore[9] = {0, 0, 4.5, 4.0, 2.0, 3.5, 4.0, 4.0, 3.0}, kWidePairMore = 7.5, kSlicedMore[6] = {0, 2, 4, 2, 1, 0};
-constexpr double kItemUs = 0.4;         // a further item on the same SM: its accumulators drain before the next pair starts
+constexpr double kClusterUs[9] = {0, 0, 3.5, 6.0, 9.0, 12.0, 14.0, 15.0, 15.0}, kClusterRowUs = 0.005;      // a cluster's launch, barriers and sum: by its CTAs, and for each token row of one
+constexpr double kSlicedUs = 3.3;       // the second kernel of slices that add up in memory
+constexpr double kAgainUs = 0.8, kAgainClusterUs = 0.32;     // slices of more items than cover the rows, for each further one: its words are read and converted again
+constexpr double kMoreItems = 1.06;     // whole items narrower than cover the rows: within that the widest stay (2048 x 4096 x 4096 as 8 x 256 rows 56.9 us, as 9 x 240 55.7, at the power limit of a long step equal)
+// a further item on the same SM: its accumulators drain before the next pair starts, or beside it where there are two sets
+double item_cost(int TN, bool wide) { return wide ? 0.4 + 0.012 * 2 * TN : TN > 192 ? 0.4 + 0.009 * TN : 0.4; }
 
 // How a dense launch covers its M token rows: items of one chunk (TN rows, one accumulator) or of two (the dequantised W stage
 // is built once for both), chunks of equal width (333 rows are 2 x 176, not 256 + 77), and K slices where the items alone
@@ -1221,71 +1328,65 @@ constexpr size_t kSliceBytes = size_t{512} << 20;
 bool slices_allowed(const Ctx *ctx, int M, int form) {
     return ctx->qmm_ksplit && (ctx->qmm_wide == 1 || M <= TN_MAX) && (form == 0 || (ctx->qmm_wide && M > TN_MAX));
 }
-DensePlan plan_dense(const Ctx *ctx, int M, int N, int K, int bits, bool slices = true) {
+DensePlan plan_dense(const Ctx *ctx, int M, int N, int K, int bits, int group_size, bool slices = true) {
+    const bool pieces = K / group_size % 8 == 0;
     const int n_tiles = (N + BMW - 1) / BMW, nkb = K / BK, nsb = (nkb + SB_PER_RAW - 1) / SB_PER_RAW, sms = ctx->sm_count;
     const auto up16 = [](int v) { return (v + 15) / 16 * 16; };
     if (ctx->qmm_force_tn > 0) return DensePlan{ctx->qmm_force_tn, (M + ctx->qmm_force_tn - 1) / ctx->qmm_force_tn, 1, 0, 0, false};
-    // two ring stages of one W and two X chunks beside two raw buffers
-    const int raw_total = 2 * raw_bytes(bits);
-    int tn_wide = ((RING_BYTES - raw_total) / 2 - A_BYTES) / (2 * BK * 2) / 16 * 16;
-    if (tn_wide > TN_MAX) tn_wide = TN_MAX;
+    constexpr int tn_wide = (TMEM_COLS - 3 * A_COLS) / 2;      // two accumulators and three k blocks of A, one for each team
+    // Up to 256 rows over four super-blocks of K, where four slices are one round: clusters of four, the form that tests/test_launches.py holds these
+    // products to (186 x 4096 x 1024 13.6 -> 12.4 us; four narrower whole items would take 9.5)
+    const int tn_one = up16(M);
+    if (slices && M > 128 && slices_allowed(ctx, M, 0) && nsb == 4 && n_tiles <= kClusters[4] * sms / kNumSMsB200 && n_tiles > kClusters[5] * sms / kNumSMsB200 && tn_one * BMW * 4 <= RING_BYTES)
+        return DensePlan{tn_one, 1, 4, 0, 1, false};
     DensePlan best{};
     double best_us = 1e30;
+    auto offer = [&](double us, const DensePlan &p) {
+        if (us < best_us - 1e-9) {
+            best_us = us;
+            best = p;
+        }
+    };
     for (int form = 0; form < 2; ++form) {                     // 0: one chunk per item, 1: two
         if (form == 1 && (!ctx->qmm_wide || M <= TN_MAX)) continue;
         if (form == 0 && ctx->qmm_wide == 2 && M > TN_MAX) continue;                 // 2: whenever the shape allows (tests)
-        const int most = form == 1 ? 2 * tn_wide : TN_MAX;
-        const int items_m = (M + most - 1) / most;
-        const int TN = form == 1 ? up16((M + 2 * items_m - 1) / (2 * items_m)) : up16((M + items_m - 1) / items_m);
-        const double one = kKbBase + kKbPerToken * TN, kb_us = form == 1 ? kWideBase + kWidePerToken * 2 * TN : one;
-        const long long units = static_cast<long long>(n_tiles) * items_m;
-        // the last round of wide items on twice as many SMs, a chunk each, where that still is one round and every unit has two
-        const int left = static_cast<int>(units % sms), last_rows = M - (items_m - 1) * 2 * TN;
-        const bool tail = form == 1 && units > sms && left > 0 && 2 * left <= sms && last_rows > TN;
-        for (int S = 1; S <= 16; ++S) {
-            if (S > 1 && (!slices || !ctx->qmm_ksplit || S > nsb || (ctx->qmm_wide != 1 && M > TN_MAX))) break;
-            if (S > 1 && static_cast<size_t>(S) * M * N * sizeof(float) > kSliceBytes) break;
-            const int kb = S == 1 ? nkb : (nsb + S - 1) / S * SB_PER_RAW;
-            const long long full = units * S / sms, rest = units * S % sms;
-            double us = full * (kb * kb_us + kItemUs);
-            if (rest > 0) us += (S == 1 && tail ? kb * one : kb * kb_us) + kItemUs;
-            if (S > 1) us += 2.0 + static_cast<double>(S) * M * N * kSliceUs;
-            if (us < best_us - 1e-9) {
-                best_us = us;
-                best = DensePlan{TN, items_m, S, S == 1 && tail ? left : 0, 0, form == 1};
+        const bool wide = form == 1;
+        const int most = wide ? 2 * tn_wide : TN_MAX, fewest = (M + most - 1) / most;
+        // as few items as cover the rows, and up to twice as many, narrower ones (not below 48 rows: 26 x 1536 x 1536 6.8 us as one, 8.6 as two)
+        for (int items_m = fewest, last_tn = 0; items_m <= 2 * fewest + 2; ++items_m) {
+            const int TN = wide ? up16((M + 2 * items_m - 1) / (2 * items_m)) : up16((M + items_m - 1) / items_m);
+            if (TN == last_tn || (items_m > fewest && TN < 48)) continue;
+            last_tn = TN;
+            if ((items_m - 1) * (wide ? 2 : 1) * TN >= M) continue;                  // the last one would be empty
+            const double one = kb_cost(TN, false, bits, pieces), kb_us = kb_cost(TN, wide, bits, pieces), item_us = item_cost(TN, wide);
+            const long long units = static_cast<long long>(n_tiles) * items_m;
+            // the teams take a stage each: the first comes after the time of a turn of theirs, half of which nothing else hides
+            const double turn = 0.5 * TEAMS * (!wide && TN <= 128 ? 2 : 1), more = items_m - fewest;
+            // the last round of wide items on twice as many SMs, a chunk each, where that still is one round and every unit has two
+            const int left = static_cast<int>(units % sms), last_rows = M - (items_m - 1) * 2 * TN;
+            const bool tail = wide && units > sms && left > 0 && 2 * left <= sms && last_rows > TN;
+            for (int S = 1; S <= 16; ++S) {
+                if (S > 1 && (!slices || !ctx->qmm_ksplit || S > nsb || (ctx->qmm_wide != 1 && M > TN_MAX))) break;
+                if (S > 1 && static_cast<size_t>(S) * M * N * sizeof(float) > kSliceBytes) break;
+                const double kb = (S == 1 ? nkb : (nsb + S - 1) / S * SB_PER_RAW) + (S == 1 ? 0.0 : turn);
+                const long long full = units * S / sms, rest = units * S % sms;
+                const double each_us = S == 1 ? item_us : item_cost(0, false);
+                double us = full * (kb * kb_us + each_us);
+                if (rest > 0) us += (S == 1 && tail ? kb * one : kb * kb_us) + each_us;
+                if (S == 1 && items_m > fewest) us *= kMoreItems;
+                if (S > 1) us += kSlicedUs + kAgainUs * more + static_cast<double>(S) * M * N * kSliceUs;
+                offer(us, DensePlan{TN, items_m, S, S == 1 && tail ? left : 0, 0, wide});
+            }
+            // slices that are the CTAs of a cluster each and add up in shared memory: no block, no second kernel, but one round that the GPCs' odd sizes
+            // leave room for; the sums take the ring's place
+            if (!slices_allowed(ctx, M, form) || (wide ? 2 : 1) * TN * BMW * 4 > RING_BYTES) continue;
+            for (int S = 2; S <= (wide ? 2 : 8) && S <= nsb; ++S) {
+                if (units > kClusters[S] * sms / kNumSMsB200) continue;
+                offer((nsb + S - 1) / S * SB_PER_RAW * kb_us + kClusterUs[S] + kClusterRowUs * (wide ? 2 : 1) * TN + kAgainClusterUs * more, DensePlan{TN, items_m, S, 0, 1, wide});
             }
         }
     }
-    // ... or slices that are the CTAs of a cluster each and add up in shared memory: no block, no second kernel, but units of a round that the
-    // GPCs' odd sizes leave room for (f16 4-bit 256 x 4096 x 4096 25.6 -> 23.2 us, 512 x 4096 x 4096 38.0 -> 35.7, 8-bit 333 x 7616 x 2880 37.2 -> 34.4,
-    // 2-bit 285 x 6400 x 3072 30.4 -> 28.0).  The candidate has to be a tenth cheaper (8-bit 1000 x 1536 x 4352 29.4 -> 31.0), of two chunks only as
-    // pairs (2-bit 285 x 3072 x 3072 as five 18.6 -> 19.6), and then cheaper with what either kind of launch was measured to take besides.
-    // Whole items without slices stay where K is whole super-blocks: there pairs lost every time (8-bit 364 x 6144 x 2560 27.1 -> 34.4, 810 x 4608 x 2560
-    // 25.3 -> 31.9); where it is not, whole items take longer than their price (800 x 4352 x 3904 47.3 -> 41.2, 2-bit 313 x 7680 x 3712 50.3 -> 38.5).
-    // Of those 520 shapes, all of them a tenth cheaper, clusters lost more than 2 % on 130 (by up to 21) and gained 3.4 in the mean; the 352 that are
-    // left lose on 16, and the mean is 5.2.
-    double cluster_us = 0.9 * best_us;
-    DensePlan cluster{};
-    for (int form = 0; form < 2; ++form) {
-        if (!slices_allowed(ctx, M, form)) continue;
-        const int most = form == 1 ? 2 * tn_wide : TN_MAX, items_m = (M + most - 1) / most;
-        const int TN = form == 1 ? up16((M + 2 * items_m - 1) / (2 * items_m)) : up16((M + items_m - 1) / items_m);
-        const double kb_us = form == 1 ? kWideBase + kWidePerToken * 2 * TN : kKbBase + kKbPerToken * TN;
-        if ((form == 1 ? 2 : 1) * TN * BMW * 4 > RING_BYTES) continue;             // the sums take the ring's place
-        for (int S = 2; S <= (form == 1 ? 2 : 8) && S <= nsb; ++S) {
-            if (static_cast<long long>(n_tiles) * items_m > kClusters[S] * sms / kNumSMsB200) continue;            // one round: a second would start from nothing
-            const double us = (nsb + S - 1) / S * SB_PER_RAW * kb_us + kItemUs + kClusterUs;
-            if (us < cluster_us) {
-                cluster_us = us;
-                cluster = DensePlan{TN, items_m, S, 0, 1, form == 1};
-            }
-        }
-    }
-    if (!cluster.cluster) return best;
-    if (best.ksplit == 1 && K % (SB_PER_RAW * BK) != 0) return cluster;
-    if (best.ksplit == 1 && cluster.wide) return best;
-    const double more = cluster.wide ? kWidePairMore : kClusterMore[cluster.ksplit];
-    return cluster_us + more < best_us + kSlicedMore[best.ksplit < 5 ? best.ksplit : 5] ? cluster : best;
+    return best;
 }
 
 // out[m, n] = sum over the K slices of partial[s][m, n], in slice order, times the factor of token row m; V outputs of a row per
@@ -1346,7 +1447,7 @@ __global__ void __launch_bounds__(256) ksplit_sum_kernel(const float *partial, c
 
 namespace {
 cudaError_t encode_map(CUtensorMap *map, CUtensorMapDataType type, int rank, const void *base, const cuuint64_t *dims, const cuuint64_t *strides,
-                       const cuuint32_t *box, std::string *why) {
+                       const cuuint32_t *box, CUtensorMapSwizzle swizzle, std::string *why) {
     EncodeTiledFn encode = get_encode_fn();
     if (!encode) {
         if (why) *why = "cuTensorMapEncodeTiled is not available from the driver";
@@ -1354,7 +1455,7 @@ cudaError_t encode_map(CUtensorMap *map, CUtensorMapDataType type, int rank, con
     }
     const cuuint32_t estr[3] = {1, 1, 1};
     const CUresult r = encode(map, type, rank, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                              swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) {
         if (why) *why = "cuTensorMapEncodeTiled failed with code " + std::to_string(static_cast<int>(r));
         return cudaErrorInvalidValue;
@@ -1368,14 +1469,15 @@ cudaError_t make_map_2d(CUtensorMap *map, CUtensorMapDataType type, int elem_byt
     const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
     const cuuint64_t strides[1] = {static_cast<cuuint64_t>(cols) * elem_bytes};
     const cuuint32_t box[2] = {static_cast<cuuint32_t>(box_cols), static_cast<cuuint32_t>(box_rows)};
-    return encode_map(map, type, 2, base, dims, strides, box, why);
+    const int width = box_cols * elem_bytes;
+    return encode_map(map, type, 2, base, dims, strides, box, width == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : width == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B, why);
 }
 
 cudaError_t make_map_blocks(CUtensorMap *map, const void *base, long long rows, long long cols, int box_rows, int box_blocks, std::string *why) {
     const cuuint64_t dims[3] = {64, static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(cols / 64)};
     const cuuint64_t strides[2] = {static_cast<cuuint64_t>(cols) * 2, 128};
     const cuuint32_t box[3] = {64, static_cast<cuuint32_t>(box_rows), static_cast<cuuint32_t>(box_blocks)};
-    return encode_map(map, CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, base, dims, strides, box, why);
+    return encode_map(map, CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B, why);
 }
 
 bool qmm_tcgen05_supported(int M, int N, int K, int bits, int group_size, int dt, const void *w, const void *x,
@@ -1387,11 +1489,19 @@ bool qmm_tcgen05_supported(int M, int N, int K, int bits, int group_size, int dt
            al(x, 16) && al(out, 2);
 }
 
+// A CTA an item, or one an SM: then no more of them than the rounds need, so that all take as many items (256 items as 128 CTAs with two each;
+// where the last round is items of one chunk each, all of them)
+static int dense_grid(const DensePlan &plan, int items, int sms) {
+    if (plan.cluster || items <= sms) return items;
+    const int rounds = (items + sms - 1) / sms;
+    return plan.halves ? sms : (items + rounds - 1) / rounds;
+}
+
 // The form of a dense launch, for mtc_launch_of
-void qmm_tcgen05_form(const Ctx *ctx, int M, int N, int K, int bits, mtc_launch_info *info) {
-    const DensePlan plan = plan_dense(ctx, M, N, K, bits);
+void qmm_tcgen05_form(const Ctx *ctx, int M, int N, int K, int bits, int group_size, mtc_launch_info *info) {
+    const DensePlan plan = plan_dense(ctx, M, N, K, bits, group_size);
     const int items = (N + BMW - 1) / BMW * plan.items_m * plan.ksplit + plan.halves;
-    info->ctas = items < ctx->sm_count || plan.cluster ? items : ctx->sm_count;
+    info->ctas = dense_grid(plan, items, ctx->sm_count);
     info->cluster = plan.cluster ? plan.ksplit : 1;
     info->k_slices = plan.ksplit;
 }
@@ -1400,7 +1510,7 @@ cudaError_t launch_qmm_tcgen05(Ctx *ctx, cudaStream_t st, const void *w, const v
                                const void *x, void *out, int M, int N, int K, int bits, int group_size, int dt,
                                std::string *why, void *const *outs, int n_outs, long long out_ld) {
     const int sms = ctx->sm_count;
-    DensePlan plan = plan_dense(ctx, M, N, K, bits);
+    DensePlan plan = plan_dense(ctx, M, N, K, bits, group_size);
     if (plan.ksplit > 1 && !plan.cluster) {
         cudaError_t ge = grow_block(ctx, st, &ctx->d_ksplit, &ctx->ksplit_bytes, static_cast<size_t>(plan.ksplit) * M * N * sizeof(float), why);
         if (ge != cudaSuccess) {
@@ -1408,7 +1518,7 @@ cudaError_t launch_qmm_tcgen05(Ctx *ctx, cudaStream_t st, const void *w, const v
             // during capture, or out of memory: the same product without slices needs no block
             if (ge != cudaErrorStreamCaptureUnsupported) cudaGetLastError();
             if (why) why->clear();
-            plan = plan_dense(ctx, M, N, K, bits, false);
+            plan = plan_dense(ctx, M, N, K, bits, group_size, false);
         }
     }
     const int TN = plan.TN;
@@ -1441,12 +1551,13 @@ cudaError_t launch_qmm_tcgen05(Ctx *ctx, cudaStream_t st, const void *w, const v
     // partial sums, added in slice order by a second small kernel).
     if (plan.ksplit > 1) {
         p.ksplit = plan.ksplit;
+        plan_smem(p, ctx, bits);                // slices start at super-blocks
         p.partial = static_cast<float *>(ctx->d_ksplit);
         p.cluster = plan.cluster;
         p.dense_items = p.n_tiles * p.m_chunks * plan.ksplit;
     }
     set_out_vec(p);
-    const int grid = p.dense_items < sms || p.cluster ? p.dense_items : sms;
+    const int grid = dense_grid(plan, p.dense_items, sms);
     e = launch_any(bits, st, tmap, p, grid, N, why);
     if (e != cudaSuccess || p.ksplit == 1 || p.cluster) return e;
     const bool vec = N % 4 == 0;

@@ -2,6 +2,8 @@
 #pragma once
 #include <cuda.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace mtc {
@@ -222,7 +224,7 @@ __device__ __forceinline__ void tmem_free_all(uint32_t base) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(512));
 }
 
-// A row-major [rows, cols] tensor with boxes of box_cols x box_rows and the 128-byte swizzle; what lies past the ends reads as zero
+// A row-major [rows, cols] tensor with boxes of box_rows x box_cols (128, 64 or 32 bytes) and the swizzle of that width; what lies past the ends reads as zero
 cudaError_t make_map_2d(CUtensorMap *map, CUtensorMapDataType type, int elem_bytes, const void *base, long long rows, long long cols,
                         int box_rows, int box_cols, std::string *why);
 // The same tensor of 16-bit elements as [cols / 64][rows][64]: one box of box_blocks x box_rows x 64 is box_blocks tiles behind each other
