@@ -6,7 +6,8 @@
 // w u32[K, N*bits/32] (row d = LSB-first bit-stream of N codes), scales / biases T[K/G, N], x T[M, K], out T[M, N].
 // Stands in for mt_qvm_b{3,4,5,6,8} and mt_qvm_int4_fast (crates/metaltile-std/src/mlx/quantized.rs:4397-4530,4582-4700).
 //
-// Two kernels: the one described here, and one on the warp-level tensor cores for several tokens (below).  Both are launched
+// Three kernels: the one described here, one that streams 4- and 8-bit codes through shared memory for one token, and one on the warp-level tensor
+// cores for several tokens (below).  All are launched
 // while the previous kernel of the stream drains and request their first weights before it is complete (4096 x 14336 4-bit, one
 // token, back to back: 16.4 -> 14.5 us).  Every packed word is read once per row of x.  A lane owns the columns of one packed word (2 / 4 / 8-bit:
 // 16 / 8 / 4 columns) or of one 32-column period of the bit-stream (3 / 5 / 6-bit: b words), so a warp reads whole
@@ -89,6 +90,50 @@ struct QvSlab {
     uint32_t w[R][S::WPT];
     uint32_t x[XW], sc[SW], bi[SW];
 };
+
+// The end of a CTA: its warps' sums red[warp][column j of lane l at j * 32 + l] added in warp order, then the chunks of K.
+template <int CPT, int DT, int WARPS>
+__device__ __forceinline__ void qv_finish(const float *red, int pitch, uint32_t *s_last, float *partial, uint32_t *tickets, void *out, int M, int N, int KC) {
+    const int tile = blockIdx.x, kc = blockIdx.y, m = blockIdx.z;
+    // column (tile * 32 + l) * CPT + j of the tile: summed over the warps in warp order
+    for (int idx = threadIdx.x; idx < 32 * CPT; idx += WARPS * 32) {
+        const int j = idx >> 5, l = idx & 31;
+        const int c = (tile * 32 + l) * CPT + j;
+        if (c >= N) continue;
+        float v = 0.0f;
+#pragma unroll
+        for (int q = 0; q < WARPS; ++q) v += red[q * pitch + idx];
+        if (KC == 1) st_from_f32(out, static_cast<size_t>(m) * N + c, v, DT);
+        else partial[(static_cast<size_t>(kc) * M + m) * N + c] = v;
+    }
+    if (KC == 1 || tickets == nullptr) return;
+    // K chunks: the CTA that arrives last for (column tile, x row) adds the chunks in chunk order (deterministic) and
+    // leaves the counter at zero for the next launch.  Nothing waits for anything.
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const uint32_t old = atomicAdd(tickets + static_cast<size_t>(m) * gridDim.x + tile, 1u);
+        *s_last = old == static_cast<uint32_t>(KC - 1) ? 1u : 0u;
+    }
+    __syncthreads();
+    if (!*s_last) return;
+    __threadfence();
+    for (int idx = threadIdx.x; idx < 32 * CPT; idx += WARPS * 32) {
+        const int j = idx >> 5, l = idx & 31;
+        const int c = (tile * 32 + l) * CPT + j;
+        if (c >= N) continue;
+        float v = 0.0f;
+        const float *src = partial + static_cast<size_t>(m) * N + c;
+        const size_t stride = static_cast<size_t>(M) * N;
+        float pv[32];                                              // KC <= 32: every load in flight, added in chunk order
+#pragma unroll
+        for (int i = 0; i < 32; ++i) pv[i] = i < KC ? __ldcg(src + i * stride) : 0.0f;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v += pv[i];
+        st_from_f32(out, static_cast<size_t>(m) * N + c, v, DT);
+    }
+    if (threadIdx.x == 0) tickets[static_cast<size_t>(m) * gridDim.x + tile] = 0u;
+}
 
 template <int BITS, int DT>
 __global__ void __launch_bounds__(kQvWarps * 32, 2) qvm_kernel(const uint32_t *w, const void *scales, const void *biases, const void *x,
@@ -193,44 +238,136 @@ __global__ void __launch_bounds__(kQvWarps * 32, 2) qvm_kernel(const uint32_t *w
 #pragma unroll
     for (int j = 0; j < S::CPT; ++j) red[warp][j * 32 + lane] = acc[j];
     __syncthreads();
-    // column (tile * 32 + l) * CPT + j of the tile: summed over the warps in warp order
-    for (int idx = threadIdx.x; idx < 32 * S::CPT; idx += kQvWarps * 32) {
-        const int j = idx >> 5, l = idx & 31;
-        const int c = (tile * 32 + l) * S::CPT + j;
-        if (c >= N) continue;
-        float v = 0.0f;
+    qv_finish<S::CPT, DT, kQvWarps>(&red[0][0], 32 * S::CPT + 1, &s_last, partial, tickets, out, M, N, KC);
+}
+
+// ---- one token, 4- and 8-bit codes ----------------------------------------------------------------------------------------------
+// The same arithmetic with the packed words on their way through shared memory.  Above, a warp has one or two slabs in flight and waits between
+// them, with 3 instructions a code beside.  Here a warp owns a contiguous range of units (16 rows of 128 bytes) of its CTA's chunk of K and keeps four of
+// them in flight with 16-byte asynchronous copies; x waits as f32 times 2^64 beside the sum of every unit, so a code costs one LOP3, one FFMA and a
+// quarter of an instruction more, and scales are applied once a group (f32: once a unit), from registers that were loaded when the group began.  One CTA of 16 warps
+// an SM, which has the SM's shared memory to itself: with room for two, CTAs land in pairs and leave SMs idle (17.9 us for the first shape below), and
+// two or three CTAs of 8 warps in twice or three times as many chunks of K pay more for start and sum (13.5, 14.4).  Six units in flight: 14.0; 24 warps:
+// 13.8.  bf16, 4-bit groups of 64, K x N 14336 x 4096 14.8 -> 13.2 us, 4096 x 4096 7.5 -> 7.0, 4096 x 14336 14.7 -> 13.0, 16384 x 16384 52.4 -> 36.3 (4.2
+// TB/s), 8-bit 8192 x 8192 22.8 -> 15.4 (4.6 TB/s), 2048 x 16384 13.8 -> 9.0.  Bound by the ALU pipe and the start and end of the launch.
+constexpr int kQrDepth = 4, kQrRows = 16, kQrWarps = 16;      // units in flight a warp, rows of a unit
+constexpr int kQrRing = kQrWarps * kQrDepth * kQrRows * 128;
+constexpr int kQrMaxUnits = (226 * 1024 - kQrRing) / ((kQrRows + 1) * 4);                            // of a CTA: their x fit beside the ring
+constexpr int qr_smem(int units) { return kQrRing + units * (kQrRows + 1) * 4; }
+
+template <int BITS, int DT>
+__global__ void __launch_bounds__(kQrWarps * 32, 1) qvm_ring_kernel(const uint32_t *w, const void *scales, const void *biases, const void *x,
+                                                                     float *partial, uint32_t *tickets, void *out, int M, int N, int K, int gs, int KC, int early) {
+    constexpr int CPT = 32 / BITS, ESZ = DT == MTC_F32 ? 4 : 2, SW = CPT * ESZ / 4, D = kQrDepth, R = kQrRows;
+    extern __shared__ __align__(16) unsigned char qr_raw[];
+    __shared__ uint32_t s_last;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int tile = blockIdx.x, kc = blockIdx.y, m = blockIdx.z;
+    const int col0 = (tile * 32 + lane) * CPT;
+    const bool on = col0 < N;                                      // N % CPT == 0: a lane is in or out as a whole
+    const int wpr = N * BITS / 32, units = K / R, upg = gs / R;    // gs % 16 == 0, wpr % 4 == 0 (host)
+    const int c0 = static_cast<int>(static_cast<long long>(units) * kc / KC), nu = static_cast<int>(static_cast<long long>(units) * (kc + 1) / KC) - c0;
+    const int u0 = c0 + nu * warp / kQrWarps, u1 = c0 + nu * (warp + 1) / kQrWarps;
+    float *sx = reinterpret_cast<float *>(qr_raw + kQrRing), *ssum = sx + nu * R;
+    const uint32_t *ring = reinterpret_cast<const uint32_t *>(qr_raw) + warp * (D * R * 32) + lane;
+    const uint32_t dst0 = static_cast<uint32_t>(__cvta_generic_to_shared(qr_raw)) + warp * (D * R * 128) + lane * 16;
+    const int piece = tile * 32 + (lane & 7) * 4;
+    const uint32_t bytes = piece < wpr ? 16u : 0u;
+    const char *src = reinterpret_cast<const char *>(w + static_cast<size_t>(u0 * R + (lane >> 3)) * wpr + (bytes ? piece : 0));
+    const size_t step = static_cast<size_t>(wpr) * 16;             // bytes of four rows
+    int slot_in = 0, next = u0;
+    auto fetch = [&]() {                                           // a group per call, so that waits count units
+        if (next < u1) {
+            const uint32_t dst = dst0 + slot_in * (R * 128);
 #pragma unroll
-        for (int q = 0; q < kQvWarps; ++q) v += red[q][idx];
-        if (KC == 1) st_from_f32(out, static_cast<size_t>(m) * N + c, v, DT);
-        else partial[(static_cast<size_t>(kc) * M + m) * N + c] = v;
+            for (int i = 0; i < R / 4; ++i)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + i * 512), "l"(src + i * step), "r"(bytes) : "memory");
+            src += (R / 4) * step;
+            ++next;
+            if (++slot_in == D) slot_in = 0;
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    if (!early) asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;");
+    // weights are constants of the model: requested while the previous kernel of the stream still runs
+#pragma unroll
+    for (int i = 0; i < D; ++i) fetch();
+    const char *sc = static_cast<const char *>(scales) + static_cast<size_t>(on ? col0 : 0) * ESZ, *bi = static_cast<const char *>(biases) + static_cast<size_t>(on ? col0 : 0) * ESZ;
+    const size_t srow = static_cast<size_t>(N) * ESZ;
+    int g = u0 / upg, left = upg - (u0 - g * upg);                 // group, units to its end
+    uint32_t sv[SW], bv[SW];
+    if (u0 < u1) {
+        qv_ld<true, SW>(sc + g * srow, sv);
+        qv_ld<true, SW>(bi + g * srow, bv);
     }
-    if (KC == 1 || tickets == nullptr) return;
-    // K chunks: the CTA that arrives last for (column tile, x row) adds the chunks in chunk order (deterministic) and
-    // leaves the counter at zero for the next launch.  Nothing waits for anything.
-    __threadfence();
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    for (int i = threadIdx.x; i < nu * (R / 4); i += kQrWarps * 32) {      // four values a thread, whole units by four lanes
+        const unsigned who = __activemask();
+        constexpr int XW = ESZ;
+        uint32_t xw[XW];
+        qv_ld<false, XW>(static_cast<const char *>(x) + (static_cast<size_t>(m) * K + static_cast<size_t>(c0) * R + 4 * i) * ESZ, xw);
+        const float v0 = qv_elem<DT>(xw, 0), v1 = qv_elem<DT>(xw, 1), v2 = qv_elem<DT>(xw, 2), v3 = qv_elem<DT>(xw, 3), up = 18446744073709551616.0f;       // 2^64: see multiply above
+        *reinterpret_cast<float4 *>(sx + 4 * i) = make_float4(v0 * up, v1 * up, v2 * up, v3 * up);
+        float t = (v0 + v1) + (v2 + v3);
+        t += __shfl_xor_sync(who, t, 1);
+        t += __shfl_xor_sync(who, t, 2);
+        if ((i & 3) == 0) ssum[i / 4] = t;
+    }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        const uint32_t old = atomicAdd(tickets + static_cast<size_t>(m) * gridDim.x + tile, 1u);
-        s_last = old == static_cast<uint32_t>(KC - 1) ? 1u : 0u;
+    float acc[CPT], raw[CPT], xs = 0.0f;
+#pragma unroll
+    for (int j = 0; j < CPT; ++j) acc[j] = raw[j] = 0.0f;
+    int slot = 0;
+    for (int u = u0; u < u1; ++u) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(D - 1) : "memory");
+        __syncwarp();
+        const uint32_t *wp = ring + slot * (R * 32);
+        const float *xp = sx + (u - c0) * R;
+        uint32_t wd[R][1];
+#pragma unroll
+        for (int r = 0; r < R; ++r) wd[r][0] = wp[r * 32];
+        __syncwarp();
+        fetch();                                                   // the slot is in registers
+#pragma unroll
+        for (int r4 = 0; r4 < R; r4 += 4) {
+            const float4 xv = *reinterpret_cast<const float4 *>(xp + r4);
+            const float xr[4] = {xv.x, xv.y, xv.z, xv.w};
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int j = 0; j < CPT; ++j) raw[j] = fmaf(xr[r], __uint_as_float(QvCode<BITS>::field(wd[r4 + r], j)), raw[j]);
+        }
+        xs += ssum[u - c0];
+        if (++slot == D) slot = 0;
+        const bool end = --left == 0 || u + 1 == u1;
+        // f32: sums no longer than above (with a whole group of them the error against 64 bits was 1.1 to 2 times as large; 16-bit results are the same)
+        if (DT == MTC_F32 || end) {
+#pragma unroll
+            for (int j = 0; j < CPT; ++j) {
+                const float post = __uint_as_float(static_cast<uint32_t>(127 + 85 - QvCode<BITS>::pos(j)) << 23);     // 2^(85 - p)
+                acc[j] = fmaf(qv_elem<DT>(sv, j) * post, raw[j], fmaf(qv_elem<DT>(bv, j), xs, acc[j]));
+                raw[j] = 0.0f;
+            }
+            xs = 0.0f;
+        }
+        if (end) {
+            left = upg;
+            if (u + 1 < u1) {
+                ++g;
+                qv_ld<true, SW>(sc + g * srow, sv);
+                qv_ld<true, SW>(bi + g * srow, bv);
+            }
+        }
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();                                               // the ring's place holds the warps' sums
+    float *red = reinterpret_cast<float *>(qr_raw);
+    constexpr int PITCH = 32 * CPT;
+#pragma unroll
+    for (int j = 0; j < CPT; ++j) red[warp * PITCH + j * 32 + lane] = acc[j];
     __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    for (int idx = threadIdx.x; idx < 32 * S::CPT; idx += kQvWarps * 32) {
-        const int j = idx >> 5, l = idx & 31;
-        const int c = (tile * 32 + l) * S::CPT + j;
-        if (c >= N) continue;
-        float v = 0.0f;
-        const float *src = partial + static_cast<size_t>(m) * N + c;
-        const size_t stride = static_cast<size_t>(M) * N;
-        float pv[32];                                              // KC <= 32: every load in flight, added in chunk order
-#pragma unroll
-        for (int i = 0; i < 32; ++i) pv[i] = i < KC ? __ldcg(src + i * stride) : 0.0f;
-#pragma unroll
-        for (int i = 0; i < 32; ++i) v += pv[i];
-        st_from_f32(out, static_cast<size_t>(m) * N + c, v, DT);
-    }
-    if (threadIdx.x == 0) tickets[static_cast<size_t>(m) * gridDim.x + tile] = 0u;
+    qv_finish<CPT, DT, kQrWarps>(red, PITCH, &s_last, partial, tickets, out, M, N, KC);
 }
 
 __global__ void __launch_bounds__(256) qvm_sum_kernel(const float *partial, void *out, size_t mn, int KC, int dt) {
@@ -573,6 +710,26 @@ cudaError_t qm_launch(cudaStream_t st, const QmArgs &a, int dt) {
     return a.M == 1 ? qm_go<BITS, MTC_BF16, 1>(st, a) : a.M == 2 ? qm_go<BITS, MTC_BF16, 2>(st, a) : qm_go<BITS, MTC_BF16, 4>(st, a);
 }
 
+template <int BITS, int DT>
+cudaError_t qr_go(cudaStream_t st, dim3 grid, const uint32_t *w, const void *scales, const void *biases, const void *x, float *partial, uint32_t *tickets,
+                  void *out, int M, int N, int K, int gs, int KC, int early) {
+    static PerDeviceAttr attr;
+    cudaError_t e = attr.set(qvm_ring_kernel<BITS, DT>, qr_smem(kQrMaxUnits));
+    if (e != cudaSuccess) return e;
+    const int units = (K / kQrRows + KC - 1) / KC;
+    return launch_pdl(qvm_ring_kernel<BITS, DT>, grid, kQrWarps * 32, qr_smem(units), st, w, scales, biases, x, partial, tickets, out, M, N, K, gs, KC, early);
+}
+template <int BITS>
+cudaError_t qr_launch(cudaStream_t st, const void *w, const void *scales, const void *biases, const void *x, float *partial,
+                      uint32_t *tickets, void *out, int M, int N, int K, int gs, int KC, int dt, int early) {
+    constexpr int COLS = 32 * (32 / BITS);
+    const dim3 grid((N + COLS - 1) / COLS, KC, M);
+    const uint32_t *wp = static_cast<const uint32_t *>(w);
+    if (dt == MTC_F32) return qr_go<BITS, MTC_F32>(st, grid, wp, scales, biases, x, partial, tickets, out, M, N, K, gs, KC, early);
+    if (dt == MTC_F16) return qr_go<BITS, MTC_F16>(st, grid, wp, scales, biases, x, partial, tickets, out, M, N, K, gs, KC, early);
+    return qr_go<BITS, MTC_BF16>(st, grid, wp, scales, biases, x, partial, tickets, out, M, N, K, gs, KC, early);
+}
+
 template <int BITS>
 cudaError_t qvm_launch(cudaStream_t st, const void *w, const void *scales, const void *biases, const void *x, float *partial,
                        uint32_t *tickets, void *out, int M, int N, int K, int gs, int KC, int dt, int early) {
@@ -600,6 +757,23 @@ static bool qvm_takes_mma(int M, int N, int K, int bits, int group_size, int dt)
     return M >= 2 && N >= 1024 && codes >= (bits == 4 ? 8 << 20 : 4 << 20);
 }
 
+static int qvm_ring_chunks(int sms, int N, int K, int bits) {
+    const int tiles = (N + 1024 / bits - 1) / (1024 / bits), units = K / kQrRows;
+    int kc = sms / tiles;                     // one CTA an SM
+    if (kc > units / kQrWarps) kc = units / kQrWarps;
+    if (kc > 32) kc = 32;
+    return kc < 1 ? 1 : kc;
+}
+// One token through the ring: rows of whole 16-byte pieces, x of a CTA's chunk beside the ring, and enough codes to pay for a CTA of 16 warps (4-bit
+// 2048 x 1024 4.9 against 5.7 us here, 4096 x 1024 6.9 against 5.9; 8-bit 4096 x 2048 5.5
+// against 5.7, 4096 x 4096 7.5 against 7.2, 2048 x 16384 13.8 against 9.0).
+// Further tokens would read the words again for each: f32, 2 tokens of 4096 x 4096 11.8 above, 13.3 here.
+static bool qvm_takes_ring(int sms, int M, int N, int K, int bits) {
+    if (M != 1 || (bits != 4 && bits != 8) || N * bits / 32 % 4 != 0 || static_cast<long long>(N) * K < (bits == 4 ? 4 << 20 : 12 << 20)) return false;
+    const int kc = qvm_ring_chunks(sms, N, K, bits);
+    return (K / kQrRows + kc - 1) / kc <= kQrMaxUnits;
+}
+
 // slabs of 32 rows that share a range: as many as a group and a batch of 128 rows allow (fewer scales to read and apply where
 // several tokens leave fewer ranges); ranges of a batch: no more than give every warp of the device a batch
 static void qm_batches(int sms, int M, int N, int K, int bits, int group_size, int *ch_log2, int *bs) {
@@ -625,6 +799,7 @@ int qvm_k_chunks(int sms, int M, int N, int K, int bits, int group_size, int dt)
         if (kc > 32) kc = 32;
         return kc < 1 ? 1 : kc;
     }
+    if (qvm_takes_ring(sms, M, N, K, bits)) return qvm_ring_chunks(sms, N, K, bits);
     const int cpt = (bits == 3 || bits == 5 || bits == 6) ? 32 : 32 / bits;
     const int tiles = (N + 32 * cpt - 1) / (32 * cpt);
     const int units = K / ((bits == 3 || bits == 5 || bits == 6) ? 8 : 16);      // slabs of R rows
@@ -672,6 +847,9 @@ cudaError_t launch_qvm(Ctx *ctx, cudaStream_t st, const void *w, const void *sca
         qm_batches(ctx->sm_count, M, N, K, bits, group_size, &a.ch_log2, &a.bs);
         a.batches = (a.slabs + a.bs - 1) / a.bs;
         e = bits == 2 ? qm_launch<2>(st, a, dt) : bits == 4 ? qm_launch<4>(st, a, dt) : qm_launch<8>(st, a, dt);
+    } else if (qvm_takes_ring(ctx->sm_count, M, N, K, bits)) {
+        e = bits == 4 ? qr_launch<4>(st, w, scales, biases, x, partial, tickets, out, M, N, K, group_size, KC, dt, early)
+                      : qr_launch<8>(st, w, scales, biases, x, partial, tickets, out, M, N, K, group_size, KC, dt, early);
     } else switch (bits) {
         case 2: e = qvm_launch<2>(st, w, scales, biases, x, partial, tickets, out, M, N, K, group_size, KC, dt, early); break;
         case 3: e = qvm_launch<3>(st, w, scales, biases, x, partial, tickets, out, M, N, K, group_size, KC, dt, early); break;
