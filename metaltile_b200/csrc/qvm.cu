@@ -91,50 +91,6 @@ struct QvSlab {
     uint32_t x[XW], sc[SW], bi[SW];
 };
 
-// The end of a CTA: its warps' sums red[warp][column j of lane l at j * 32 + l] added in warp order, then the chunks of K.
-template <int CPT, int DT, int WARPS>
-__device__ __forceinline__ void qv_finish(const float *red, int pitch, uint32_t *s_last, float *partial, uint32_t *tickets, void *out, int M, int N, int KC) {
-    const int tile = blockIdx.x, kc = blockIdx.y, m = blockIdx.z;
-    // column (tile * 32 + l) * CPT + j of the tile: summed over the warps in warp order
-    for (int idx = threadIdx.x; idx < 32 * CPT; idx += WARPS * 32) {
-        const int j = idx >> 5, l = idx & 31;
-        const int c = (tile * 32 + l) * CPT + j;
-        if (c >= N) continue;
-        float v = 0.0f;
-#pragma unroll
-        for (int q = 0; q < WARPS; ++q) v += red[q * pitch + idx];
-        if (KC == 1) st_from_f32(out, static_cast<size_t>(m) * N + c, v, DT);
-        else partial[(static_cast<size_t>(kc) * M + m) * N + c] = v;
-    }
-    if (KC == 1 || tickets == nullptr) return;
-    // K chunks: the CTA that arrives last for (column tile, x row) adds the chunks in chunk order (deterministic) and
-    // leaves the counter at zero for the next launch.  Nothing waits for anything.
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const uint32_t old = atomicAdd(tickets + static_cast<size_t>(m) * gridDim.x + tile, 1u);
-        *s_last = old == static_cast<uint32_t>(KC - 1) ? 1u : 0u;
-    }
-    __syncthreads();
-    if (!*s_last) return;
-    __threadfence();
-    for (int idx = threadIdx.x; idx < 32 * CPT; idx += WARPS * 32) {
-        const int j = idx >> 5, l = idx & 31;
-        const int c = (tile * 32 + l) * CPT + j;
-        if (c >= N) continue;
-        float v = 0.0f;
-        const float *src = partial + static_cast<size_t>(m) * N + c;
-        const size_t stride = static_cast<size_t>(M) * N;
-        float pv[32];                                              // KC <= 32: every load in flight, added in chunk order
-#pragma unroll
-        for (int i = 0; i < 32; ++i) pv[i] = i < KC ? __ldcg(src + i * stride) : 0.0f;
-#pragma unroll
-        for (int i = 0; i < 32; ++i) v += pv[i];
-        st_from_f32(out, static_cast<size_t>(m) * N + c, v, DT);
-    }
-    if (threadIdx.x == 0) tickets[static_cast<size_t>(m) * gridDim.x + tile] = 0u;
-}
-
 template <int BITS, int DT>
 __global__ void __launch_bounds__(kQvWarps * 32, 2) qvm_kernel(const uint32_t *w, const void *scales, const void *biases, const void *x,
                                                                float *partial, uint32_t *tickets, void *out, int M, int N, int K, int gs, int KC, int early) {
@@ -238,7 +194,44 @@ __global__ void __launch_bounds__(kQvWarps * 32, 2) qvm_kernel(const uint32_t *w
 #pragma unroll
     for (int j = 0; j < S::CPT; ++j) red[warp][j * 32 + lane] = acc[j];
     __syncthreads();
-    qv_finish<S::CPT, DT, kQvWarps>(&red[0][0], 32 * S::CPT + 1, &s_last, partial, tickets, out, M, N, KC);
+    // column (tile * 32 + l) * CPT + j of the tile: summed over the warps in warp order
+    for (int idx = threadIdx.x; idx < 32 * S::CPT; idx += kQvWarps * 32) {
+        const int j = idx >> 5, l = idx & 31;
+        const int c = (tile * 32 + l) * S::CPT + j;
+        if (c >= N) continue;
+        float v = 0.0f;
+#pragma unroll
+        for (int q = 0; q < kQvWarps; ++q) v += red[q][idx];
+        if (KC == 1) st_from_f32(out, static_cast<size_t>(m) * N + c, v, DT);
+        else partial[(static_cast<size_t>(kc) * M + m) * N + c] = v;
+    }
+    if (KC == 1 || tickets == nullptr) return;
+    // K chunks: the CTA that arrives last for (column tile, x row) adds the chunks in chunk order (deterministic) and
+    // leaves the counter at zero for the next launch.  Nothing waits for anything.
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const uint32_t old = atomicAdd(tickets + static_cast<size_t>(m) * gridDim.x + tile, 1u);
+        s_last = old == static_cast<uint32_t>(KC - 1) ? 1u : 0u;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    for (int idx = threadIdx.x; idx < 32 * S::CPT; idx += kQvWarps * 32) {
+        const int j = idx >> 5, l = idx & 31;
+        const int c = (tile * 32 + l) * S::CPT + j;
+        if (c >= N) continue;
+        float v = 0.0f;
+        const float *src = partial + static_cast<size_t>(m) * N + c;
+        const size_t stride = static_cast<size_t>(M) * N;
+        float pv[32];                                              // KC <= 32: every load in flight, added in chunk order
+#pragma unroll
+        for (int i = 0; i < 32; ++i) pv[i] = i < KC ? __ldcg(src + i * stride) : 0.0f;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v += pv[i];
+        st_from_f32(out, static_cast<size_t>(m) * N + c, v, DT);
+    }
+    if (threadIdx.x == 0) tickets[static_cast<size_t>(m) * gridDim.x + tile] = 0u;
 }
 
 // ---- one token, 4- and 8-bit codes ----------------------------------------------------------------------------------------------
@@ -254,6 +247,50 @@ constexpr int kQrDepth = 4, kQrRows = 16, kQrWarps = 16;      // units in flight
 constexpr int kQrRing = kQrWarps * kQrDepth * kQrRows * 128;
 constexpr int kQrMaxUnits = (226 * 1024 - kQrRing) / ((kQrRows + 1) * 4);                            // of a CTA: their x fit beside the ring
 constexpr int qr_smem(int units) { return kQrRing + units * (kQrRows + 1) * 4; }
+
+// The end of a CTA as in the kernel above (which keeps its own: with a shared one its 2-bit f32 form took 1.14 times as long): its warps' sums red[warp][column j of lane l at j * 32 + l] added in warp order, then the chunks of K.
+template <int CPT, int DT, int WARPS>
+__device__ __forceinline__ void qv_finish(const float *red, int pitch, uint32_t *s_last, float *partial, uint32_t *tickets, void *out, int M, int N, int KC) {
+    const int tile = blockIdx.x, kc = blockIdx.y, m = blockIdx.z;
+    // column (tile * 32 + l) * CPT + j of the tile: summed over the warps in warp order
+    for (int idx = threadIdx.x; idx < 32 * CPT; idx += WARPS * 32) {
+        const int j = idx >> 5, l = idx & 31;
+        const int c = (tile * 32 + l) * CPT + j;
+        if (c >= N) continue;
+        float v = 0.0f;
+#pragma unroll
+        for (int q = 0; q < WARPS; ++q) v += red[q * pitch + idx];
+        if (KC == 1) st_from_f32(out, static_cast<size_t>(m) * N + c, v, DT);
+        else partial[(static_cast<size_t>(kc) * M + m) * N + c] = v;
+    }
+    if (KC == 1 || tickets == nullptr) return;
+    // K chunks: the CTA that arrives last for (column tile, x row) adds the chunks in chunk order (deterministic) and
+    // leaves the counter at zero for the next launch.  Nothing waits for anything.
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const uint32_t old = atomicAdd(tickets + static_cast<size_t>(m) * gridDim.x + tile, 1u);
+        *s_last = old == static_cast<uint32_t>(KC - 1) ? 1u : 0u;
+    }
+    __syncthreads();
+    if (!*s_last) return;
+    __threadfence();
+    for (int idx = threadIdx.x; idx < 32 * CPT; idx += WARPS * 32) {
+        const int j = idx >> 5, l = idx & 31;
+        const int c = (tile * 32 + l) * CPT + j;
+        if (c >= N) continue;
+        float v = 0.0f;
+        const float *src = partial + static_cast<size_t>(m) * N + c;
+        const size_t stride = static_cast<size_t>(M) * N;
+        float pv[32];                                              // KC <= 32: every load in flight, added in chunk order
+#pragma unroll
+        for (int i = 0; i < 32; ++i) pv[i] = i < KC ? __ldcg(src + i * stride) : 0.0f;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v += pv[i];
+        st_from_f32(out, static_cast<size_t>(m) * N + c, v, DT);
+    }
+    if (threadIdx.x == 0) tickets[static_cast<size_t>(m) * gridDim.x + tile] = 0u;
+}
 
 template <int BITS, int DT>
 __global__ void __launch_bounds__(kQrWarps * 32, 1) qvm_ring_kernel(const uint32_t *w, const void *scales, const void *biases, const void *x,

@@ -6,7 +6,7 @@ pytestmark = pytest.mark.gpu
 
 CASES = [
     # m, n, k, bits, group, type, factor of the scales, elements that the scale arrays are off a 16-byte boundary, options
-    (64, 130, 1088, 4, 64, "bf16", 1.0, 0, {}), (65, 256, 2048, 4, 128, "f16", 16.0, 0, {}), (200, 100, 2048, 3, 32, "bf16", 1.0, 2, {}),
+    (64, 130, 1088, 4, 64, "bf16", 1.0, 0, {}), (65, 256, 2048, 4, 128, "f16", 16.0, 0, {}), (200, 100, 2048, 3, 32, "bf16", 1.0, 2, {}), (200, 136, 1024, 4, 64, "f16", 1.0, 1, {}),
     (257, 128, 1024, 8, 64, "f16", 1.0, 0, {}), (129, 640, 960, 5, 32, "f16", 1.0, 8, {}), (300, 72, 1472, 6, 64, "bf16", 64.0, 2, {}),
     (192, 384, 4096, 2, 64, "bf16", 2.0 ** -12, 0, {}), (333, 200, 2880, 8, 32, "f16", 8.0, 0, {}), (100, 96, 1024, 4, 256, "bf16", 1.0, 0, {}),
     (300, 260, 1536, 4, 64, "f16", 1.0, 0, {"qmm_max_stages": 1}), (300, 260, 1536, 8, 32, "bf16", 1.0, 0, {"qmm_max_stages": 2}),
