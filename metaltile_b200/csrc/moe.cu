@@ -83,12 +83,17 @@ __global__ void __launch_bounds__(128) router_topk_kernel(const void *logits, ui
 // The reference leaves the sort to its caller (moe.rs:253-271 states the contract only).  Definition
 // used here: stable sort of the flat slots f = token*k + slot by (expert[f], f).  One CTA of 1024
 // threads; warp w owns the contiguous slots [w * per, (w + 1) * per) and walks them 32 at a time:
-// (1) per-warp, per-expert counts (lanes of a sub-chunk are grouped per expert with __match_any_sync; no
+// (1) per-warp, per-expert counts (lanes of a sub-chunk are grouped per expert; no
 // atomics: a warp only writes its own row), (2) per expert a prefix over the 32 warps and the expert
 // totals, scanned into expert_offsets, (3) the same walk again, now placing: position = first row of the
 // expert + slots of earlier warps + slots of earlier sub-chunks of this warp + rank inside the sub-chunk.
 constexpr int kSortThreads = 1024, kSortHeld = 4;
+// Slots between which rows go through shared memory to be stored in order.  A warp's stores of scattered rows are a sector each, all of them on one SM:
+// with the lanes of each expert kept from the first walk 4096 slots of 128 experts take 9.0 us instead of 12.3; up to 256 slots it makes no
+// difference, and a kernel of its own is a quarter of a microsecond less.
+constexpr int kSortDirect = 256, kSortStaged = 12288, kSortMatched = 16;      // kSortMatched: experts up to which matches are used
 
+template <bool MANY>
 __global__ void __launch_bounds__(kSortThreads) moe_sort_kernel(const uint32_t *topk_idx, int total, int k, int n_experts,
                                                                 uint32_t *sort_token_idx, uint32_t *inv_perm,
                                                                 uint32_t *expert_offsets, uint32_t *row_expert,
@@ -99,28 +104,44 @@ __global__ void __launch_bounds__(kSortThreads) moe_sort_kernel(const uint32_t *
     uint32_t *wcnt = sm + n_experts + 1;           // [32][n_experts] per-warp counts, then running positions
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int per = ((total + 32 * 32 - 1) / (32 * 32)) * 32;          // slots per warp, whole sub-chunks
+    const bool staged = MANY && total <= kSortStaged;
+    uint32_t *rows = wcnt + 32 * n_experts;        // staged: [total] expert << 16 | token of every row
     const int f0 = warp * per, f1 = min(f0 + per, total);
-    // the first sub-chunks' ids are read once, all of them in flight, and kept for the second walk
-    uint32_t held[kSortHeld];
+    // the first sub-chunks' ids are read once, all of them in flight, and kept for the second walk, with the lanes that share each
+    uint32_t held[kSortHeld], shared_by[kSortHeld];
 #pragma unroll
     for (int q = 0; q < kSortHeld; ++q) held[q] = f0 + 32 * q + lane < f1 ? topk_idx[f0 + 32 * q + lane] : 0xFFFFFFFFu;
     const int used = min(32, (total + per - 1) / max(per, 1));          // warps that have slots
     for (int i = tid; i < used * n_experts; i += kSortThreads) wcnt[i] = 0;
     __syncthreads();
     uint32_t *mine = wcnt + warp * n_experts;
+    // lanes of the warp with the same expert, by a vote a bit: a match instruction takes a pass for each expert in the warp (4096 slots of 128 experts
+    // 9.0 us by matches, 7.4 by votes; 8192 of 8 experts 10.0 and 11.3, 64 of 128 experts 2.8 and 3.1)
+    const int bits = 32 - __clz(n_experts - 1);
+    auto same_expert = [&](uint32_t e, bool ok) {
+        if (!MANY) return __match_any_sync(0xffffffffu, ok ? e : 0xFFFFFFFFu);
+        uint32_t peers = __ballot_sync(0xffffffffu, ok);
+        for (int b = 0; b < bits; ++b) {
+            const bool set = (e >> b) & 1u;
+            const uint32_t with = __ballot_sync(0xffffffffu, set);
+            peers &= set ? with : ~with;
+        }
+        return peers;
+    };
     auto count = [&](int c, uint32_t id) {
         const int f = c + lane;
         const bool have = f < f1;
         const uint32_t e = have ? id : 0xFFFFFFFFu;
         const bool ok = have && e < static_cast<uint32_t>(n_experts);
         if (have && !ok) atomicCAS(status, 0u, 0x501u);        // expert id out of range: recorded, slot skipped
-        const uint32_t peers = __match_any_sync(0xffffffffu, ok ? e : 0xFFFFFFFFu);
+        const uint32_t peers = same_expert(e, ok);
         if (ok && __popc(peers & ((1u << lane) - 1u)) == 0) mine[e] += __popc(peers);
         __syncwarp();
+        return peers;
     };
 #pragma unroll
     for (int q = 0; q < kSortHeld; ++q)
-        if (f0 + 32 * q < f1) count(f0 + 32 * q, held[q]);
+        if (f0 + 32 * q < f1) shared_by[q] = count(f0 + 32 * q, held[q]);
     for (int c = f0 + 32 * kSortHeld; c < f1; c += 32) count(c, c + lane < f1 ? topk_idx[c + lane] : 0xFFFFFFFFu);
     __syncthreads();
     for (int ee = tid; ee < n_experts; ee += kSortThreads) {   // per expert: exclusive prefix over the warps, total
@@ -151,12 +172,10 @@ __global__ void __launch_bounds__(kSortThreads) moe_sort_kernel(const uint32_t *
     }
     __syncthreads();
     for (int e = tid; e <= n_experts; e += kSortThreads) expert_offsets[e] = cursor[e];
-    auto place = [&](int c, uint32_t id) {
+    auto in_range = [&](int c, uint32_t id) { return c + lane < f1 && id < static_cast<uint32_t>(n_experts); };
+    auto place = [&](int c, uint32_t e, uint32_t peers) {
         const int f = c + lane;
-        const bool have = f < f1;
-        const uint32_t e = have ? id : 0xFFFFFFFFu;
-        const bool ok = have && e < static_cast<uint32_t>(n_experts);
-        const uint32_t peers = __match_any_sync(0xffffffffu, ok ? e : 0xFFFFFFFFu);
+        const bool ok = in_range(c, e);
         const uint32_t rank = __popc(peers & ((1u << lane) - 1u));
         uint32_t before = 0;
         if (ok) before = mine[e];                  // slots of this expert in earlier warps and earlier sub-chunks
@@ -164,16 +183,31 @@ __global__ void __launch_bounds__(kSortThreads) moe_sort_kernel(const uint32_t *
         if (ok && rank == 0) mine[e] = before + __popc(peers);
         __syncwarp();
         if (ok) {
-            const uint32_t pos = cursor[e] + before + rank;
-            sort_token_idx[pos] = static_cast<uint32_t>(f / k);
+            const uint32_t pos = cursor[e] + before + rank, token = static_cast<uint32_t>(f / k);
             inv_perm[f] = pos;
-            if (row_expert) row_expert[pos] = e;
+            if (staged) {
+                rows[pos] = e << 16 | token;
+            } else {
+                sort_token_idx[pos] = token;
+                if (row_expert) row_expert[pos] = e;
+            }
         }
     };
 #pragma unroll
     for (int q = 0; q < kSortHeld; ++q)
-        if (f0 + 32 * q < f1) place(f0 + 32 * q, held[q]);
-    for (int c = f0 + 32 * kSortHeld; c < f1; c += 32) place(c, c + lane < f1 ? topk_idx[c + lane] : 0xFFFFFFFFu);
+        if (f0 + 32 * q < f1) place(f0 + 32 * q, held[q], shared_by[q]);
+    for (int c = f0 + 32 * kSortHeld; c < f1; c += 32) {
+        const uint32_t id = c + lane < f1 ? topk_idx[c + lane] : 0xFFFFFFFFu;
+        place(c, id, same_expert(id, in_range(c, id)));
+    }
+    if (!staged) return;
+    __syncthreads();
+    const uint32_t n_rows = cursor[n_experts];     // slots without an expert have no row
+    for (uint32_t i = tid; i < n_rows; i += kSortThreads) {
+        const uint32_t v = rows[i];
+        sort_token_idx[i] = v & 0xFFFFu;
+        if (row_expert) row_expert[i] = v >> 16;
+    }
 }
 
 // ---- mt_moe_permute (moe.rs:283-302): permuted[p, :] = tokens[sort_token_idx[p], :] ----------------
@@ -354,11 +388,14 @@ cudaError_t launch_router_topk(cudaStream_t st, const void *logits, uint32_t *id
 
 cudaError_t launch_moe_sort(cudaStream_t st, const uint32_t *topk_idx, int n_tokens, int k, int n_experts, uint32_t *sti,
                             uint32_t *inv, uint32_t *offsets, uint32_t *row_expert, uint32_t *status) {
-    const size_t smem = (static_cast<size_t>(n_experts) + 1 + 32 * static_cast<size_t>(n_experts)) * sizeof(uint32_t);
+    const int total = n_tokens * k;
+    const bool many = total > kSortDirect && n_experts > kSortMatched;
+    const size_t smem = (static_cast<size_t>(n_experts) + 1 + 32 * static_cast<size_t>(n_experts) + (many && total <= kSortStaged ? total : 0)) * sizeof(uint32_t);
     static PerDeviceAttr attr;
-    cudaError_t e = attr.set(moe_sort_kernel, 200 * 1024);
+    static PerDeviceAttr attr_many;
+    cudaError_t e = many ? attr_many.set(moe_sort_kernel<true>, 200 * 1024) : attr.set(moe_sort_kernel<false>, 200 * 1024);
     if (e != cudaSuccess) return e;
-    return launch_pdl(moe_sort_kernel, 1, kSortThreads, smem, st, topk_idx, n_tokens * k, k, n_experts, sti, inv, offsets, row_expert, status);
+    return launch_pdl(many ? moe_sort_kernel<true> : moe_sort_kernel<false>, 1, kSortThreads, smem, st, topk_idx, total, k, n_experts, sti, inv, offsets, row_expert, status);
 }
 
 cudaError_t launch_permute(cudaStream_t st, const void *tokens, const uint32_t *sti, void *permuted, int n_rows, int hidden,
