@@ -40,6 +40,7 @@
 // on the device from expert_offsets by build_items_kernel.
 #include <cstddef>
 
+#include "ring.h"
 #include "tcgen05.cuh"
 
 namespace mtc {
@@ -58,7 +59,7 @@ constexpr int MAX_RAW = 4;
 constexpr int TMEM_COLS = 512, A_COLS = BK / 2;     // columns of A per k block
 constexpr int TEAMS = 3;                    // of dequant warps
 constexpr int EPI_WARP0 = 4;
-constexpr int COPY_WARP0 = 2, COPY_THREADS = 64;
+constexpr int COPY_WARP0 = 2, COPY_THREADS = ring::kCopyWarps * 32;
 constexpr int DEQ_WARP0 = 8, DEQ_WARPS = 4 * TEAMS;
 constexpr int NUM_THREADS = (DEQ_WARP0 + DEQ_WARPS) * 32;
 struct QmmParams {
@@ -450,11 +451,11 @@ qmm_tcgen05_kernel(const __grid_constant__ QmmMaps maps, const QmmParams p) {
             mbar_init(&ctl->acc_empty[b], 4);
         }
         for (int b = 0; b < MAX_RAW; ++b) {
-            mbar_init(&ctl->raw_full[b], RawTile<BITS>::TMA ? 1 : COPY_THREADS);
+            mbar_init(&ctl->raw_full[b], ring::fill_arrivals(RawTile<BITS>::TMA));
             mbar_init(&ctl->raw_empty[b], DEQ_WARPS);
         }
         for (int b = 0; b < 2; ++b) {
-            mbar_init(&ctl->sp_full[b], p.sp_copy == 2 ? 1 : COPY_THREADS);
+            mbar_init(&ctl->sp_full[b], ring::fill_arrivals(p.sp_copy == 2));
             mbar_init(&ctl->sp_empty[b], DEQ_WARPS);
         }
         ctl->abort = 0;
@@ -563,8 +564,10 @@ qmm_tcgen05_kernel(const __grid_constant__ QmmMaps maps, const QmmParams p) {
         // other widths are cp.async copies of these two warps.
         // Scales and biases: rows lie apart, and a cp.async takes the load pipe some ten cycles a lane, so 64 bytes of a row are copied at a time, and where rows are
         // whole 16-byte pieces by TMA.  (A bulk copy a row was slower than eight lanes: 333 x 7616 x 2880 28 -> 40 us.)
-        if (p.raw) {
-            using R = RawTile<BITS>;
+        // A warp waits only for buffers that it helps to fill (ring.h): what TMA copies is the first warp's alone.
+        using R = RawTile<BITS>;
+        const bool words_here = ring::fills(R::TMA, warp - COPY_WARP0), scales_here = ring::fills(p.sp_copy == 2, warp - COPY_WARP0);
+        if (p.raw && (words_here || scales_here)) {
             const int t = threadIdx.x - COPY_WARP0 * 32;
             const uint32_t raw0 = smem_u32(smem) + p.raw_off, sp0 = smem_u32(smem) + p.sp_off;
             const int pitch = sp_pitch(p.sp_bytes);
@@ -578,8 +581,9 @@ qmm_tcgen05_kernel(const __grid_constant__ QmmMaps maps, const QmmParams p) {
                 const int kb_first = KSPLIT ? im.kb0 : 0;
                 int sp_next = 0;                         // where the next span starts
                 for (int kb0 = 0; kb0 < im.nkb; kb0 += p.raw_blk) {
-                    if (kb0 == sp_next) {
-                        sp_next += p.sp_kb - (kb_first + kb0) % p.sp_kb;
+                    const bool start = kb0 == sp_next;
+                    if (start) sp_next += p.sp_kb - (kb_first + kb0) % p.sp_kb;
+                    if (start && scales_here) {
                         if (!(ok = mbar_wait_warp(&ctl->sp_empty[sp], sph ^ 1, &ctl->abort, p.status, 0x502, p.hint_ns))) break;
                         const int g0 = ((kb_first + kb0) * BK) >> p.gs_shift, n = ((min(sp_next, im.nkb) - kb0) * BK + (1 << p.gs_shift) - 1) >> p.gs_shift;
                         const uint32_t dst0 = sp0 + sp * sp_buffer(p.sp_bytes), dsts = dst0 + (warp == COPY_WARP0 ? 0 : BMW * pitch);
@@ -631,6 +635,7 @@ qmm_tcgen05_kernel(const __grid_constant__ QmmMaps maps, const QmmParams p) {
                         sph ^= sp;
                         sp ^= 1;
                     }
+                    if (!words_here) continue;
                     if (!(ok = mbar_wait_warp(&ctl->raw_empty[buf], ph ^ 1, &ctl->abort, p.status, 0x501, p.hint_ns))) break;
                     const uint32_t dstt = raw0 + buf * p.raw_tile;
                     if constexpr (R::TMA) {
