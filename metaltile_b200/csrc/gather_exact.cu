@@ -21,7 +21,7 @@
 //   warp 16      producer  a stage at a time: 16 KB of packed words (128 bytes of each row) and the activations of the same codes; an item at a
 //                          time: its scales and biases, which lie in one piece.  It also allocates and frees the tensor memory.
 //   warp 17      MMA       four K = 16 steps a k block of 64 codes, A from tensor memory; two accumulators, items in turn
-// Every wait is bounded: on expiry the kernel records a code in the status word, all roles leave, copies in flight are awaited (bounded
+// Every wait is bounded: on expiry the kernel records a code in the status word, all roles leave, copies and MMAs in flight are awaited (bounded
 // too) and the tensor memory is freed.
 //
 // What was measured on the way to this form (a layer of 512 tokens, 128 experts of 2048 x 768, top-8, us; the mma.sync kernel 257): the integer codes as
@@ -88,6 +88,8 @@ struct __align__(16) ECtrl {
     int4 head[2];                                      // the item's pass: expert, first row, rows
     uint32_t tmem_base;
     volatile uint32_t abort;
+    uint64_t drained;                                  // giving up: the MMAs are complete
+    uint32_t stages_issued, items_issued;              // what the producer started
     alignas(16) float row_factor[2][kRows];
     alignas(16) float tok_factor[kEpiWarps][kMaxTB];
 };
@@ -278,6 +280,19 @@ __device__ __forceinline__ uint32_t max4(const uint4 &v) {          // of |bf16|
     return __vmaxu2(__vmaxu2(v.x & 0x7FFF7FFFu, v.y & 0x7FFF7FFFu), __vmaxu2(v.z & 0x7FFF7FFFu, v.w & 0x7FFF7FFFu));
 }
 
+// A launch that gave up, once every role has ended: lets what is on its way arrive before the CTA tears down.
+__device__ __noinline__ void rest(ECtrl *ctl, int nst) {
+    const int warp = threadIdx.x >> 5;
+    if (warp == kMmaWarp && elect_one()) {
+        umma_commit(&ctl->drained);
+        drain_ring(&ctl->drained, 1, 1);
+    } else if (warp == kLoadWarp && (threadIdx.x & 31) == 0) {
+        drain_ring(ctl->full, ctl->stages_issued, nst);
+        drain_ring(ctl->item_full, ctl->items_issued, 2);
+    }
+    __syncthreads();
+}
+
 __global__ void __launch_bounds__(kThreads, 1) gather_exact_kernel(const __grid_constant__ EMaps maps, const __grid_constant__ EArgs a) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -301,6 +316,7 @@ __global__ void __launch_bounds__(kThreads, 1) gather_exact_kernel(const __grid_
             mbar_init(&ctl->d_full[s], 1);
             mbar_init(&ctl->d_empty[s], kEpiWarps);
         }
+        mbar_init(&ctl->drained, 1);
         ctl->abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -323,7 +339,7 @@ __global__ void __launch_bounds__(kThreads, 1) gather_exact_kernel(const __grid_
         if (lane == 0) {
             auto pass_of = [&](int i) { return i < n_items ? *reinterpret_cast<const int4 *>(&a.table->pass[i / a.tiles]) : make_int4(0, 0, 0, 0); };
             int s = 0;
-            uint32_t ph = 0, e = 0, eph = 0;
+            uint32_t ph = 0, e = 0, eph = 0, laps = 0, started = 0;
             bool ok = true;
             int4 next = pass_of(blockIdx.x);
             for (int i = blockIdx.x; i < n_items && ok; i += gridDim.x) {
@@ -346,6 +362,7 @@ __global__ void __launch_bounds__(kThreads, 1) gather_exact_kernel(const __grid_
                     }
                     eph ^= e;
                     e ^= 1;
+                    ++started;
                 }
                 const CUtensorMap *const map_x = &maps.x[(cols >> 4) - 1];
                 const int row0 = pass.x * a.n_out + n0, row1 = a.two ? row0 : row0 + 64;
@@ -360,15 +377,11 @@ __global__ void __launch_bounds__(kThreads, 1) gather_exact_kernel(const __grid_
                         tma_load_2d(dst + kWordBytes / 2, &maps.w[a.two], c * (kChunk * 8), row1, bar);
                     }
                     tma_load_3d(dst + kWordBytes, map_x, 0, pass.y, codes ? c * kChunk : a.nkb + (c - ncc) * kChunk, bar);       // blocks past the row too
-                    if (++s == nst) { s = 0; ph ^= 1; }
+                    if (++s == nst) { s = 0; ph ^= 1; ++laps; }
                 }
             }
-            if (!ok) {   // let copies already in flight land before the CTA tears down
-                for (int b = 0; b < nst; ++b)
-                    for (uint32_t j = 0; j < 4096 && !mbar_try(&ctl->full[b], 0) && !mbar_try(&ctl->full[b], 1); ++j) {}
-                for (int b = 0; b < 2; ++b)
-                    for (uint32_t j = 0; j < 4096 && !mbar_try(&ctl->item_full[b], 0) && !mbar_try(&ctl->item_full[b], 1); ++j) {}
-            }
+            ctl->stages_issued = laps * nst + s;
+            ctl->items_issued = started;
         }
     } else if (warp == kMmaWarp) {
         // ---------------- MMA ----------------
@@ -634,6 +647,7 @@ __global__ void __launch_bounds__(kThreads, 1) gather_exact_kernel(const __grid_
     }
     tc_fence_before();
     __syncthreads();
+    if (ctl->abort) rest(ctl, nst);
     if (warp == kLoadWarp) {
         tc_fence_after();
         tmem_free_all(tmem);

@@ -26,7 +26,7 @@
 //                          shape has no raw form), w = q*scale + bias rounded to the operand type, tcgen05.st as the A operand
 // Stage hand-off uses mbarriers; tcgen05.commit releases a stage when its MMAs have read it.  Every
 // wait is bounded: on expiry the kernel records a code in the context's status word, all roles leave
-// their loops, TMEM is released and the kernel returns.
+// their loops, copies and MMAs in flight are awaited (bounded too), TMEM is released and the kernel returns.
 //
 // Why A lies in tensor memory: shared memory moves 128 bytes a cycle, and a k block with A there costs it 16 KB stored and 16 KB read by each chunk's
 // MMAs beside the 2 x 128 TN of X: 128 + TN cycles for the MMAs alone (measured), 2.9 cycles a token row in all at 2 x 256 rows where the tensor
@@ -40,7 +40,7 @@
 // on the device from expert_offsets by build_items_kernel.
 #include <cstddef>
 
-#include "ring.h"
+#include "ring.cuh"
 #include "tcgen05.cuh"
 
 namespace mtc {
@@ -126,6 +126,8 @@ struct __align__(8) SmemCtrl {
     uint64_t sp_full[2], sp_empty[2];   // the same for a span of scales
     uint32_t tmem_base;
     volatile uint32_t abort;
+    uint64_t drained;                   // giving up: the MMAs are complete
+    uint32_t stages_issued, raw_issued, sp_issued, converted[DEQ_WARPS];      // what was started; stages that a dequant warp which gave up has converted
 };
 
 // ---- PTX wrappers -------------------------------------------------------------------------------
@@ -425,6 +427,25 @@ __device__ __forceinline__ Item get_item(const QmmParams &p, int i) {
     return it;
 }
 
+// A launch that gave up, once every role has ended: lets what is on its way arrive before the CTA tears down.
+__device__ __noinline__ void rest(SmemCtrl *ctl, int nst, int nraw) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (warp >= DEQ_WARP0 && lane == 0) {            // the phases that an X copy completes take these arrivals too
+        for (uint32_t u = ctl->converted[warp - DEQ_WARP0]; u < ctl->stages_issued; ++u)
+            if (ring::owed(u, min(TEAMS, nst), (warp - DEQ_WARP0) >> 2)) mbar_arrive(&ctl->full[u % nst]);
+    } else if (warp == 1 && elect_one()) {
+        umma_commit(&ctl->drained);
+        drain_ring(&ctl->drained, 1, 1);
+    } else if (warp == 0 && lane == 0) {
+        drain_ring(ctl->full, ctl->stages_issued, nst);
+        if (nraw) {
+            drain_ring(ctl->raw_full, ctl->raw_issued, nraw);
+            drain_ring(ctl->sp_full, ctl->sp_issued, 2);
+        }
+    }
+    __syncthreads();
+}
+
 // KSPLIT: the launch cuts K into slices (items carry a first k block, the epilogue writes f32 partial sums); a
 // separate instantiation, so that the code of every other launch is what it was without the feature.
 template <int BITS, bool KSPLIT, int KPS>
@@ -458,6 +479,7 @@ qmm_tcgen05_kernel(const __grid_constant__ QmmMaps maps, const QmmParams p) {
             mbar_init(&ctl->sp_full[b], ring::fill_arrivals(p.sp_copy == 2));
             mbar_init(&ctl->sp_empty[b], DEQ_WARPS);
         }
+        mbar_init(&ctl->drained, 1);
         ctl->abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -477,7 +499,7 @@ qmm_tcgen05_kernel(const __grid_constant__ QmmMaps maps, const QmmParams p) {
         // ---------------- producer: TMA loads of the X chunk ----------------
         if (lane == 0) {
             int s = 0;
-            uint32_t ph = 0;                              // stage and ring-pass parity, advanced without a division
+            uint32_t ph = 0, laps = 0;                    // stage and ring-pass parity, advanced without a division
             bool ok = true;
             if (p.pdl_roles) asm volatile("griddepcontrol.wait;" ::: "memory");      // x may come from the previous kernel
             for (int i = blockIdx.x; i < num_items && ok; i += gridDim.x) {
@@ -496,13 +518,11 @@ qmm_tcgen05_kernel(const __grid_constant__ QmmMaps maps, const QmmParams p) {
                     if (++s == nst) {
                         s = 0;
                         ph ^= 1;
+                        ++laps;
                     }
                 }
             }
-            if (!ok) {   // let copies already in flight land before the CTA tears down
-                for (int s = 0; s < nst; ++s)
-                    for (uint32_t j = 0; j < 4096 && !mbar_try(&ctl->full[s], 0) && !mbar_try(&ctl->full[s], 1); ++j) {}
-            }
+            ctl->stages_issued = laps * nst + s;
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
@@ -564,7 +584,7 @@ qmm_tcgen05_kernel(const __grid_constant__ QmmMaps maps, const QmmParams p) {
         // other widths are cp.async copies of these two warps.
         // Scales and biases: rows lie apart, and a cp.async takes the load pipe some ten cycles a lane, so 64 bytes of a row are copied at a time, and where rows are
         // whole 16-byte pieces by TMA.  (A bulk copy a row was slower than eight lanes: 333 x 7616 x 2880 28 -> 40 us.)
-        // A warp waits only for buffers that it helps to fill (ring.h): what TMA copies is the first warp's alone.
+        // A warp waits only for buffers that it helps to fill (ring.cuh): what TMA copies is the first warp's alone.
         using R = RawTile<BITS>;
         const bool words_here = ring::fills(R::TMA, warp - COPY_WARP0), scales_here = ring::fills(p.sp_copy == 2, warp - COPY_WARP0);
         if (p.raw && (words_here || scales_here)) {
@@ -572,7 +592,7 @@ qmm_tcgen05_kernel(const __grid_constant__ QmmMaps maps, const QmmParams p) {
             const uint32_t raw0 = smem_u32(smem) + p.raw_off, sp0 = smem_u32(smem) + p.sp_off;
             const int pitch = sp_pitch(p.sp_bytes);
             int buf = 0, sp = 0;
-            uint32_t ph = 0, sph = 0;
+            uint32_t ph = 0, sph = 0, laps = 0, spans = 0;
             bool ok = true;
             for (int i = blockIdx.x; i < num_items && ok; i += gridDim.x) {
                 const Item im = get_item<KSPLIT>(p, i);
@@ -634,6 +654,7 @@ qmm_tcgen05_kernel(const __grid_constant__ QmmMaps maps, const QmmParams p) {
                         }
                         sph ^= sp;
                         sp ^= 1;
+                        ++spans;
                     }
                     if (!words_here) continue;
                     if (!(ok = mbar_wait_warp(&ctl->raw_empty[buf], ph ^ 1, &ctl->abort, p.status, 0x501, p.hint_ns))) break;
@@ -670,15 +691,14 @@ qmm_tcgen05_kernel(const __grid_constant__ QmmMaps maps, const QmmParams p) {
                     if (++buf == p.nraw) {
                         buf = 0;
                         ph ^= 1;
+                        ++laps;
                     }
                 }
             }
             asm volatile("cp.async.wait_all;" ::: "memory");
-            if (!ok) {             // let copies already in flight land before the CTA tears down
-                for (int b = 0; R::TMA && b < p.nraw; ++b)
-                    for (uint32_t j = 0; j < 4096 && !mbar_try(&ctl->raw_full[b], 0) && !mbar_try(&ctl->raw_full[b], 1); ++j) {}
-                for (int b = 0; b < 2; ++b)
-                    for (uint32_t j = 0; j < 4096 && !mbar_try(&ctl->sp_full[b], 0) && !mbar_try(&ctl->sp_full[b], 1); ++j) {}
+            if (t == 0) {          // what TMA copies: the others' copies have landed
+                ctl->raw_issued = R::TMA ? laps * p.nraw + buf : 0;
+                ctl->sp_issued = p.sp_copy == 2 ? spans : 0;
             }
         }
     } else if (warp >= EPI_WARP0 && warp < EPI_WARP0 + 4) {
@@ -789,6 +809,7 @@ qmm_tcgen05_kernel(const __grid_constant__ QmmMaps maps, const QmmParams p) {
         const int teams = min(TEAMS, nst);
         int s = 0, turn = 0;                              // stage, and the team whose stage it is
         uint32_t ph = 0;                                  // ring-pass parity, advanced without a division
+        int gave_up = num_items, gave_up_kb = 0;          // item and k block where a wait ran out
         const bool second = p.gs_shift == 5;              // groups of 32: two scales a k block
         auto convert = [&](auto words, uint32_t s0, uint32_t s1, uint32_t b0, uint32_t b1, uint32_t at) {
             uint32_t v[32];
@@ -839,18 +860,27 @@ qmm_tcgen05_kernel(const __grid_constant__ QmmMaps maps, const QmmParams p) {
                 int sp_next = 0;                         // where the next span starts
                 for (int kb0 = 0; kb0 < item.nkb; kb0 += p.raw_blk) {
                     if (kb0 == sp_next) {
-                        if (!wait(offsetof(SmemCtrl, sp_full) + sp * 8, sph, 0x403)) return;
+                        if (!wait(offsetof(SmemCtrl, sp_full) + sp * 8, sph, 0x403)) {
+                            gave_up = i, gave_up_kb = kb0;
+                            return;
+                        }
                         const uint32_t g = ((kb_first + kb0) * BK) >> gsh, buffer = sp0 + sp * sp_buffer(p.sp_bytes);
                         scales = by_tma ? buffer + r * p.sp_bytes : buffer + r * sp_pitch(p.sp_bytes) + ((el0 + g) & (p.sp_copy ? 7 : 1)) * 2 - 2 * g;
                         sp_next += p.sp_kb - (kb_first + kb0) % p.sp_kb;
                     }
-                    if (!wait(offsetof(SmemCtrl, raw_full) + buf * 8, buf_ph, 0x402)) return;
+                    if (!wait(offsetof(SmemCtrl, raw_full) + buf * 8, buf_ph, 0x402)) {
+                        gave_up = i, gave_up_kb = kb0;
+                        return;
+                    }
                     const uint32_t base = raw0 + buf * p.raw_tile;
                     const int end = min(p.raw_blk, item.nkb - kb0);
 #pragma unroll 1
                     for (int j = 0; j < end; j += KPS) {
                         if (turn == team) {
-                            if (!stage_free()) return;
+                            if (!stage_free()) {
+                                gave_up = i, gave_up_kb = kb0 + j;
+                                return;
+                            }
 #pragma unroll 1
                             for (int c = 0; c < KPS; ++c) {
                                 if (KPS > 1 && j + c >= end) break;
@@ -905,7 +935,10 @@ qmm_tcgen05_kernel(const __grid_constant__ QmmMaps maps, const QmmParams p) {
                 if (team < teams && mine < item.nkb) request(mine);
                 for (int kb = 0; kb < item.nkb; ++kb) {
                     if (turn == team) {
-                        if (!stage_free()) return;
+                        if (!stage_free()) {
+                            gave_up = i, gave_up_kb = kb;
+                            return;
+                        }
                         convert([&](int h, uint32_t (&to)[BITS]) {
 #pragma unroll
                             for (int e = 0; e < BITS; ++e) to[e] = w[h][e];
@@ -919,6 +952,12 @@ qmm_tcgen05_kernel(const __grid_constant__ QmmMaps maps, const QmmParams p) {
         };
         if (p.raw) through_buffers();
         else from_memory();
+        uint32_t stages = 0xFFFFFFFFu;
+        if (gave_up < num_items) {                       // those before that
+            stages = gave_up_kb / KPS;
+            for (int i = blockIdx.x; i < gave_up; i += gridDim.x) stages += (get_item<KSPLIT>(p, i).nkb + KPS - 1) / KPS;
+        }
+        if (lane == 0) ctl->converted[warp - DEQ_WARP0] = stages;
     }
 
     if constexpr (KSPLIT) {
@@ -1001,6 +1040,7 @@ qmm_tcgen05_kernel(const __grid_constant__ QmmMaps maps, const QmmParams p) {
     }
     tc_fence_before();
     __syncthreads();
+    if (ctl->abort) rest(ctl, nst, p.raw ? p.nraw : 0);
     if (warp == 2) {
         tc_fence_after();
         tmem_free_all(tmem_base);

@@ -20,5 +20,13 @@ MTC_HD constexpr bool fills(bool by_tma, int warp) { return !by_tma || warp == 0
 // arrivals that fill a buffer: one thread's, or those of all threads of both warps
 MTC_HD constexpr int fill_arrivals(bool by_tma) { return by_tma ? 1 : kCopyWarps * 32; }
 
+// Giving up.  A CTA whose waits ran out leaves only when what it set in motion has come to rest: use u of a ring takes slot u % slots, so of `issued` uses
+// the last one of a slot completes the phase of this parity (-1: none took it).  Where a phase also takes arrivals of warps that convert (use u is that
+// of team u % teams), those that have left owe theirs for the uses from `done` on that were issued: `owed`.
+MTC_HD constexpr int last_parity(unsigned issued, int slots, int slot) {
+    return issued <= static_cast<unsigned>(slot) ? -1 : static_cast<int>((issued - 1 - slot) / slots & 1);
+}
+MTC_HD constexpr bool owed(unsigned use, int teams, int team) { return static_cast<int>(use % teams) == team; }
+
 }  // namespace ring
 }  // namespace mtc

@@ -5,6 +5,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "ring.cuh"
 
 namespace mtc {
 
@@ -104,6 +105,14 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t parity, v
 // The same for a loop whose counters and addresses have to stay warp-uniform (the issue of MMAs): the outcome is a vote.
 __device__ __forceinline__ bool mbar_wait_vote(uint64_t *bar, uint32_t parity, volatile uint32_t *abort, uint32_t *status, uint32_t code) {
     return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort, status, code));
+}
+
+// On the way out of a launch that gave up, by one thread once every role has ended: bounded waits for the copies (or MMAs) that are still on their way.
+static __device__ __noinline__ void drain_ring(uint64_t *bars, uint32_t issued, int slots) {
+    for (int b = 0; b < slots; ++b) {
+        const int parity = ring::last_parity(issued, slots, b);
+        for (uint32_t i = 0; parity >= 0 && i < 1u << 16 && !mbar_try(&bars[b], parity); ++i) {}
+    }
 }
 
 // Waits and arrivals of loops that keep the barriers' shared-memory addresses: `abort` is the address of the CTA's abort flag.

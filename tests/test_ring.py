@@ -1,4 +1,4 @@
-"""The barrier protocol of the tcgen05 kernels' rings, played on the CPU: the rules of csrc/ring.h, compiled by the host compiler, against a model of
+"""The barrier protocol of the tcgen05 kernels' rings, played on the CPU: the rules of csrc/ring.cuh, compiled by the host compiler, against a model of
 mbarriers in which every role may be held back for as long as another can go on."""
 import ctypes
 import os
@@ -14,9 +14,11 @@ CSRC = os.path.join(os.path.dirname(__file__), os.pardir, "metaltile_b200", "csr
 def ring(tmp_path_factory):
     d = tmp_path_factory.mktemp("ring")
     src = d / "ring.cpp"
-    src.write_text('#include "ring.h"\nusing namespace mtc::ring;\nextern "C" {\n'
+    src.write_text('#include "ring.cuh"\nusing namespace mtc::ring;\nextern "C" {\n'
                    "int fills_(int tma, int w) { return fills(tma, w); }\n"
                    "int fill_arrivals_(int tma) { return fill_arrivals(tma); }\n"
+                   "int last_parity_(unsigned n, int slots, int slot) { return last_parity(n, slots, slot); }\n"
+                   "int owed_(unsigned use, int teams, int team) { return owed(use, teams, team); }\n"
                    "}\n")
     subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I", CSRC, str(src), "-o", str(d / "ring.so")], check=True)
     return ctypes.CDLL(str(d / "ring.so"))
@@ -95,3 +97,62 @@ def test_a_warp_that_nobody_waits_for_is():
         fill_arrivals_ = staticmethod(lambda tma: 1)
 
     assert not play(_copies(Both, 2, 2, 1, False), 1, random.Random(0))
+
+
+def _gives_up(ring, slots, teams, uses, steps, rng):
+    """Copies, teams that convert and MMAs over one ring; after ``steps`` steps every wait fails.  Returns what leaving has to put right: the barriers, the
+    copies still on their way, the uses that were issued, how far each warp came."""
+    per = 4                                                  # warps of a team; MMAs as in the kernel: full takes the copy's arrival and theirs
+    full = [Barrier(1 + per) for _ in range(slots)]
+    empty = [Barrier(1) for _ in range(slots)]
+    landing, state = [], dict(issued=0, converted=[0] * (per * teams))
+
+    def producer():
+        for u in range(uses):
+            yield lambda b=u % slots, par=u // slots % 2: empty[b].passed(par ^ 1)
+            landing.append(u % slots)                        # the copy's bytes hold the phase open as an arrival does
+            state["issued"] = u + 1
+
+    def convert(w):
+        for u in range(uses):
+            if u % teams == w // per:
+                yield lambda b=u % slots, par=u // slots % 2: empty[b].passed(par ^ 1)
+                full[u % slots].arrive()
+            state["converted"][w] = u + 1
+
+    def mma():
+        for u in range(uses):
+            yield lambda b=u % slots, par=u // slots % 2: full[b].passed(par)
+            empty[u % slots].arrive()
+
+    roles = [producer(), mma()] + [convert(w) for w in range(per * teams)]
+    waiting = [next(r, None) for r in roles]
+    for _ in range(steps):
+        ready = [i for i, w in enumerate(waiting) if w is not None and w()]
+        if landing and (not ready or rng.random() < 0.3):
+            full[landing.pop(rng.randrange(len(landing)))].arrive()
+        elif ready:
+            i = rng.choice(ready)
+            waiting[i] = next(roles[i], None)
+    return full, landing, state
+
+
+@pytest.mark.parametrize("slots,teams", [(1, 1), (2, 2), (3, 3), (4, 3), (8, 3)])
+def test_leaving_waits_for_every_copy(ring, slots, teams):
+    """Wherever the roles stop: with the arrivals that are owed every issued copy's phase completes when the copy lands, not before, and takes no other."""
+    rng = random.Random(slots)
+    for trial in range(300):
+        full, landing, state = _gives_up(ring, slots, teams, 20, rng.randrange(400), rng)
+        issued = state["issued"]
+        for w, done in enumerate(state["converted"]):
+            for u in range(done, issued):
+                if ring.owed_(u, teams, w // 4):
+                    full[u % slots].arrive()
+        parity = [ring.last_parity_(issued, slots, b) for b in range(slots)]
+        for b in range(slots):
+            if parity[b] >= 0:
+                assert full[b].passed(parity[b]) == (b not in landing)
+        for b in landing:
+            full[b].arrive()
+        assert all(full[b].passed(p) for b, p in enumerate(parity) if p >= 0)
+        assert [p for p in parity if p < 0] == [-1] * max(0, slots - issued)
