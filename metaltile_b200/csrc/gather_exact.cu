@@ -12,7 +12,10 @@
 // groups of (bias + 8 * scale) * sum(x), is a short product of its own at the end of K: biases and 8 * scales against the sums of x, the sums cut
 // into three bf16 pieces that hold their 24 bits.  Everything adds up in one f32 accumulator.  Powers of two keep the factors in f16's range: one for
 // each weight row (its largest scale, or bias / 8, comes to [2^-9, 2^-8)), one for each row of x (its largest value to [2^14, 2^15)); the
-// epilogue takes them out.  Scales below 2^-8 of their row's largest, and elements of x below 2^-38 of theirs, are rounded, by 2^-19 of the largest weight.
+// epilogue takes them out.  That holds every scale down to 2^-8 of its row's largest.  Where a row of the 32 of a warp has smaller ones, they come to
+// [2^12, 2^13) instead and the operand is (1024 + q - 1032) * scale, 13 instructions, which holds them down to 2^-29 (the layer below 151 us
+// before there was this form, 154 with it, 174 where every row takes it).  Rows with smaller ones yet, or with infinities, are added up from the definition.  Elements of x below 2^-31 of their
+// row's largest are rounded, by 2^-40 of it at most, as every tcgen05 product of bf16 rows does.
 //
 // Work.  A PASS is (expert, up to TB of its rows); an item is a pass x 128 weight rows (64 of gate and 64 of up where one launch covers
 // both), all of K.  One persistent CTA per SM walks the items; its roles meet at mbarriers and run ahead of each other across items:
@@ -31,6 +34,7 @@
 // is waited for together with the loads of tensor memory: 4 such loads a stage took 1000 cycles, hence the bulk copies.
 #include <cstddef>
 
+#include "far_tokens.cuh"
 #include "tcgen05.cuh"
 
 namespace mtc {
@@ -66,6 +70,10 @@ struct EArgs {
     void *act;                       // not null: silu(rows 0..63) * rows 64..127 goes here, outs are not written
     const ETable *table;
     const float *tok_scale;          // powers of two that the rows of x were divided by
+    const uint32_t *w[2];            // for rows that are added up from the definition
+    const __nv_bfloat16 *x;
+    const uint32_t *row_src;
+    int n_src_rows;
     uint32_t *status;
     int two;                         // 1: an item is 64 rows of each matrix; 0: 128 rows of the first
     int n_out, gpr, gs_shift;
@@ -88,9 +96,11 @@ struct __align__(16) ECtrl {
     int4 head[2];                                      // the item's pass: expert, first row, rows
     uint32_t tmem_base;
     volatile uint32_t abort;
+    volatile int again;                                // 1 + the last item with such results, for the epilogue
+    uint32_t marked[kEpiWarps];                        // its weight rows that are added up from the definition
     uint64_t drained;                                  // giving up: the MMAs are complete
     uint32_t stages_issued, items_issued;              // what the producer started
-    alignas(16) float row_factor[2][kRows];
+    alignas(16) float row_factor[2][kRows];            // negative: a row whose scales the operands do not hold
     alignas(16) float tok_factor[kEpiWarps][kMaxTB];
 };
 constexpr int kCtlBytes = (sizeof(ECtrl) + 1023) / 1024 * 1024;
@@ -251,6 +261,16 @@ __device__ __forceinline__ uint32_t hfma2(uint32_t a, uint32_t b, uint32_t c) {
     return r;
 }
 
+// q - 8 of the codes at bits 0..3 / 4..7 of either half: 1024 + q (1024 + 16 q) by an OR
+__device__ __forceinline__ uint32_t low_code(uint32_t w) {
+    uint32_t r;
+    asm("add.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"((w & 0x000F000Fu) | 0x64006400u), "r"(0xE408E408u /* -1032 */));
+    return r;
+}
+__device__ __forceinline__ uint32_t high_code(uint32_t w) {
+    return hfma2((w & 0x00F000F0u) | 0x64006400u, 0x2C002C00u /* 2^-4 */, 0xD480D480u /* -72 */);
+}
+
 // Two 16-bit values from shared memory; WIDE: the address is a multiple of 4
 template <bool WIDE>
 __device__ __forceinline__ uint32_t lds4(uint32_t addr) {
@@ -278,6 +298,68 @@ __device__ __forceinline__ uint4 lds16(uint32_t addr) {
 }
 __device__ __forceinline__ uint32_t max4(const uint4 &v) {          // of |bf16| pairs
     return __vmaxu2(__vmaxu2(v.x & 0x7FFF7FFFu, v.y & 0x7FFF7FFFu), __vmaxu2(v.z & 0x7FFF7FFFu, v.w & 0x7FFF7FFFu));
+}
+__device__ __forceinline__ uint32_t min4(const uint4 &v) {
+    return __vminu2(__vminu2(v.x & 0x7FFF7FFFu, v.y & 0x7FFF7FFFu), __vminu2(v.z & 0x7FFF7FFFu, v.w & 0x7FFF7FFFu));
+}
+// the least |bf16| of a row of `rb` bytes that is not zero; 0x7FFF without one
+__device__ __noinline__ uint32_t least_nonzero(uint32_t row, uint32_t rb) {
+    uint32_t low = 0x7FFFu;
+    for (uint32_t g = 0; g < rb; g += 2) {
+        unsigned short v;
+        asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(row + g));
+        if (v & 0x7FFF) low = min(low, v & 0x7FFFu);
+    }
+    return low;
+}
+
+// A stage's k blocks in the form for scales far apart: pair, later: the scales of its groups.  Not inlined, so that the other form's loop stays in one piece.
+__device__ __noinline__ void wide_blocks(uint32_t words, int r, uint32_t dst, int blocks, uint32_t pair, uint32_t later, bool groups64, float f) {
+#pragma unroll 1
+    for (int j = 0; j < blocks; ++j) {
+        uint32_t v[32];
+        const __half2 s2 = __float2half2_rn(__uint_as_float(pair << 16) * f);
+        const uint32_t s = *reinterpret_cast<const uint32_t *>(&s2);
+        if (groups64 || (j & 1)) pair = (j & 1) && groups64 ? later : pair >> 16;
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+            const uint4 q = lds16<16>(words + (((2 * j + p) ^ (r & 7)) << 4));
+            const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const uint32_t u = w[k] >> 8;
+                v[16 * p + 4 * k] = hmul2(low_code(w[k]), s);
+                v[16 * p + 4 * k + 1] = hmul2(high_code(w[k]), s);
+                v[16 * p + 4 * k + 2] = hmul2(low_code(u), s);
+                v[16 * p + 4 * k + 3] = hmul2(high_code(u), s);
+            }
+        }
+        tmem_st32(dst + j * 32, v);
+    }
+}
+
+// Results of an item that its operands do not hold, in the buffer of results, by the definition, a warp an output: those of the marked weight rows (`row`:
+// that of the calling thread of the epilogue is).
+__device__ __noinline__ void from_definition(const EArgs &a, ECtrl *ctl, const int4 pass, const int n0, const bool row) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, K = a.gpr << a.gs_shift;
+    const uint32_t rows = __ballot_sync(0xffffffffu, row && n0 + (a.two ? threadIdx.x & 63 : threadIdx.x) < static_cast<uint32_t>(a.n_out));
+    if (lane == 0) ctl->marked[warp] = rows;
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+    unsigned short *const staged = reinterpret_cast<unsigned short *>(reinterpret_cast<uint8_t *>(ctl) + kCtlBytes);
+    for (int t = warp; t < pass.z; t += kEpiWarps) {         // the tokens that this warp stores
+        size_t src = pass.y + t;
+        if (a.row_src) src = a.row_src[src] < static_cast<uint32_t>(a.n_src_rows) ? a.row_src[src] : 0;
+        const __nv_bfloat16 *const x = a.x + src * K;
+        for (int q = 0; q < kRows / 32; ++q)
+            for (uint32_t todo = ctl->marked[q]; todo != 0; todo &= todo - 1) {
+                const int at = q * 32 + __ffs(todo) - 1, m = a.two ? at >> 6 : 0;
+                const size_t n = static_cast<size_t>(pass.x) * a.n_out + n0 + (a.two ? at & 63 : at);
+                const float v = far_tokens::sum<4, MTC_BF16>(a.w[m] + n * (K / 8), static_cast<const __nv_bfloat16 *>(a.scales[m]) + n * a.gpr,
+                                                             static_cast<const __nv_bfloat16 *>(a.biases[m]) + n * a.gpr, x, K, a.gs_shift);
+                if (lane == 0) staged[t * kRows + at] = static_cast<unsigned short>(pack_bf16(v, 0.0f));
+            }
+        __syncwarp();
+    }
 }
 
 // A launch that gave up, once every role has ended: lets what is on its way arrive before the CTA tears down.
@@ -318,6 +400,7 @@ __global__ void __launch_bounds__(kThreads, 1) gather_exact_kernel(const __grid_
         }
         mbar_init(&ctl->drained, 1);
         ctl->abort = 0;
+        ctl->again = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == kLoadWarp) tmem_alloc_all(&ctl->tmem_base);
@@ -442,18 +525,22 @@ __global__ void __launch_bounds__(kThreads, 1) gather_exact_kernel(const __grid_
                 if (!wait(item_full + e * 8, eph, 0xa07)) return;
                 __syncwarp();
                 const uint32_t row = items + e * a.item_bytes + r * rb, brow = row + kRows * rb;
-                // the power of two of the row: its largest scale, or bias / 8, to [2^-9, 2^-8)
-                uint32_t top = 0, btop = 0;
+                // the power of two of the row, by its largest scale or bias / 8, and its least scale
+                uint32_t top = 0, btop = 0, low = 0x7FFF7FFFu;
                 if (align == 16) {                      // lanes start at different pieces: rows lie 64 bytes apart, or some such number
                     uint32_t at = (lane >> 1) * 16 % rb;
                     for (uint32_t g = 0; g < rb; g += 16) {
-                        top = __vmaxu2(top, max4(lds16<16>(row + at)));
+                        const uint4 sv = lds16<16>(row + at);
+                        top = __vmaxu2(top, max4(sv));
+                        low = __vminu2(low, min4(sv));
                         btop = __vmaxu2(btop, max4(lds16<16>(brow + at)));
                         at = at + 16 == rb ? 0 : at + 16;
                     }
                 } else if (align == 4) {
                     for (uint32_t g = 0; g < rb; g += 4) {
-                        top = __vmaxu2(top, lds4<true>(row + g) & 0x7FFF7FFFu);
+                        const uint32_t sv = lds4<true>(row + g) & 0x7FFF7FFFu;
+                        top = __vmaxu2(top, sv);
+                        low = __vminu2(low, sv);
                         btop = __vmaxu2(btop, lds4<true>(brow + g) & 0x7FFF7FFFu);
                     }
                 } else {                                // an odd number: the last one with the one before it
@@ -461,15 +548,23 @@ __global__ void __launch_bounds__(kThreads, 1) gather_exact_kernel(const __grid_
                         const uint32_t at = min(g, rb - min(rb, 4u));
                         const uint32_t sv = lds4<false>(row + at), bv = lds4<false>(brow + at), keep = rb == 2 ? 0x7FFFu : 0x7FFF7FFFu;
                         top = __vmaxu2(top, sv & keep);
+                        low = __vminu2(low, (sv & keep) | (0x7FFF7FFFu & ~keep));
                         btop = __vmaxu2(btop, bv & keep);
                     }
                 }
                 const int es = static_cast<int>(max(top & 0xFFFFu, top >> 16) >> 7), eb = static_cast<int>(max(btop & 0xFFFFu, btop >> 16) >> 7);
-                const int ex = max(es, eb - 3), up = min(max(245 - ex, 1), 253);           // biased exponent of the factor, 2^(118 - ex)
+                const int ex = max(es, eb - 3);
+                uint32_t least = min(low & 0xFFFFu, low >> 16);
+                if (least == 0) least = least_nonzero(row, rb);
+                // the biased exponent of the factor: 2^(118 - ex), or 2^(139 - ex) where that leaves a scale of these rows less than 2^-17, whose last bit f16 does
+                // not hold.  Rows that this leaves one, too, are marked.
+                int up = max(245 - ex, 1);
+                const bool wide = __any_sync(0xffffffffu, static_cast<int>(least >> 7) + up < 237);
+                if (wide) up = min(max(266 - ex, 1), 253);
                 const float f = __uint_as_float(static_cast<uint32_t>(up) << 23);
                 for (int c = 0; c < nch; ++c) {
                     if (turn == team) {
-                        if (c == 0) ctl->row_factor[e][r] = __uint_as_float(static_cast<uint32_t>(254 - up) << 23);
+                        if (c == 0) ctl->row_factor[e][r] = __uint_as_float(static_cast<uint32_t>(254 - up) << 23 | (static_cast<int>(least >> 7) + up < 237 ? 0x80000000u : 0u));
                         // in this order: with the MMAs of this team's stage before complete, the pass of the ring before this one is, and
                         // its phase cannot be taken for this one's
                         if (!wait(a_empty + team * 8, aph ^ 1, 0xa09)) return;
@@ -488,8 +583,9 @@ __global__ void __launch_bounds__(kThreads, 1) gather_exact_kernel(const __grid_
                                 pair = align == 2 ? lds4<false>(at) : lds4<true>(at);
                                 if (a.gs_shift == 6) later = align == 2 ? lds4<false>(at + 4) : lds4<true>(at + 4);
                             }
+                            if (wide) wide_blocks(words, r, dst, blocks, pair, later, a.gs_shift == 6, f);
 #pragma unroll 1
-                            for (int j = 0; j < blocks; ++j) {
+                            for (int j = wide ? blocks : 0; j < blocks; ++j) {
                                 uint32_t w[8], v[32];
 #pragma unroll
                                 for (int p = 0; p < 2; ++p)
@@ -581,6 +677,7 @@ __global__ void __launch_bounds__(kThreads, 1) gather_exact_kernel(const __grid_
             if (!epilogue_votes(ok)) break;
             tc_fence_after();
             const float rf = ctl->row_factor[e][r];
+            if (rf < 0.0f) ctl->again = i + 1;
             unsigned short *const to = reinterpret_cast<unsigned short *>(staged) + r;
 #pragma unroll 1
             for (int t0 = 0; t0 < pass.z; t0 += 16) {
@@ -607,8 +704,9 @@ __global__ void __launch_bounds__(kThreads, 1) gather_exact_kernel(const __grid_
             eph ^= e;
             e ^= 1;
             asm volatile("bar.sync 1, 128;" ::: "memory");
-            // out of shared memory, a token a warp
             const int n0 = i % a.tiles * tile_rows;
+            if (ctl->again == i + 1) from_definition(a, ctl, pass, n0, rf < 0.0f);
+            // out of shared memory, a token a warp
             if (a.act) {
                 const int n = n0 + 2 * lane;
                 const bool pairs = (a.n_out & 1) == 0 && (reinterpret_cast<uintptr_t>(a.act) & 3) == 0;
@@ -715,6 +813,10 @@ cudaError_t launch_gather_exact(Ctx *ctx, cudaStream_t st, const void *x, const 
         a.biases[i] = m.biases;
         a.outs[i] = m.out;
     }
+    for (int i = 0; i < 2; ++i) a.w[i] = static_cast<const uint32_t *>(mats[n_mats == 2 ? i : 0].w);
+    a.x = static_cast<const __nv_bfloat16 *>(x);
+    a.row_src = row_src;
+    a.n_src_rows = n_src_rows;
     a.act = act;
     a.table = table;
     a.tok_scale = tok_scale;

@@ -31,11 +31,9 @@ def _product(torch, ops, ctx, counts, n, k, g, change=None, x_change=None, seed=
         xs = x[row:row + c].double()
         wd = _codes(torch, w[i], 4, k).double() * sd + bd
         mag = xs.abs() @ (16 * sd.abs() + bd.abs()).T
-        # rounded to bf16 once; a chain of steps, each truncated to 24 bits; scales far below their row's largest are rounded
-        small = 2.0 ** -19 * (8 * sd.abs() + bd.abs()).amax(1) * xs.abs().sum(1, keepdim=True)
-        far = (s[i].abs().amax(1) > 2.0 ** 8 * s[i].abs().amin(1)) | (b[i].abs().amax(1) > 2.0 ** 11 * s[i].abs().amin(1))
+        # rounded to bf16 once; a chain of steps, each truncated to 24 bits
         refs.append(xs @ wd.T)
-        bounds.append(2.0 ** -8 * refs[-1].abs() + 2.0 ** -23 * steps * mag + far.double() * small + 2.0 ** -133)
+        bounds.append(2.0 ** -8 * refs[-1].abs() + 2.0 ** -23 * steps * mag + 2.0 ** -133)
         row += c
     return out[:m], torch.cat(refs), torch.cat(bounds)
 
@@ -56,8 +54,10 @@ def test_products(counts, n, k, g):
     assert bool(((got.double() - ref).abs() <= bound).all())
 
 
-@pytest.mark.parametrize("what", ["rows", "groups", "zeros", "biases", "negative"])
-def test_scales_of_every_size(what):
+@pytest.mark.parametrize("g,k", [(64, 512), (64, 320), (128, 640)])            # rows of scales on boundaries of 16 bytes, of 2, of 2
+@pytest.mark.parametrize("what", ["rows", "groups", "zeros", "biases", "negative", "most", "outlier 9", "outlier 14", "outlier 29", "outlier 30", "outlier 60"])
+def test_scales_of_every_size(what, g, k):
+    """Also of one row: as far apart as either form of the operands holds, and farther."""
     import torch
     from metaltile_b200 import ops
 
@@ -78,9 +78,21 @@ def test_scales_of_every_size(what):
             b = b * 4096
         if what == "negative":
             s = -s
+        if what == "most":                                   # biases of rows without scales, and with scales far below them
+            s[:, 1::2] *= 2.0 ** -20
+            s[:, ::4] = 0
+        if what.startswith("outlier"):                       # a group of some rows, where the tokens are zero: what is left is the others'
+            s[:, ::5, 1] *= 2.0 ** int(what[8:])
+            b[:, ::7, 1] *= 2.0 ** int(what[8:])
         return s.to(torch.bfloat16), b.to(torch.bfloat16)
 
-    got, ref, bound = _product(torch, ops, ops.context(), [20, 0, 37], 192, 512, 64, change)
+    def no_outlier(x):
+        x = x.clone()
+        if what.startswith("outlier"):
+            x[::2, g:2 * g] = 0
+        return x
+
+    got, ref, bound = _product(torch, ops, ops.context(), [20, 0, 37], 192, k, g, change, no_outlier)
     assert bool(torch.isfinite(got).all()) and bool(((got.double() - ref).abs() <= bound).all())
 
 
