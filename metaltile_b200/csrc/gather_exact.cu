@@ -14,8 +14,8 @@
 // each weight row (its largest scale, or bias / 8, comes to [2^-9, 2^-8)), one for each row of x (its largest value to [2^14, 2^15)); the
 // epilogue takes them out.  That holds every scale down to 2^-8 of its row's largest.  Where a row of the 32 of a warp has smaller ones, they come to
 // [2^12, 2^13) instead and the operand is (1024 + q - 1032) * scale, 13 instructions, which holds them down to 2^-29 (the layer below 151 us
-// before there was this form, 154 with it, 174 where every row takes it).  Rows with smaller ones yet, or with infinities, are added up from the definition.  Elements of x below 2^-31 of their
-// row's largest are rounded, by 2^-40 of it at most, as every tcgen05 product of bf16 rows does.
+// before there was this form, 154 with it, 174 where every row takes it).  Rows with smaller ones yet or with
+// an infinity, and infinite tokens, are added up from the definition.  Elements of x below 2^-31 of their row's largest are rounded, by 2^-40 of it at most, as every tcgen05 product of bf16 rows does.
 //
 // Work.  A PASS is (expert, up to TB of its rows); an item is a pass x 128 weight rows (64 of gate and 64 of up where one launch covers
 // both), all of K.  One persistent CTA per SM walks the items; its roles meet at mbarriers and run ahead of each other across items:
@@ -69,7 +69,7 @@ struct EArgs {
     void *outs[2];
     void *act;                       // not null: silu(rows 0..63) * rows 64..127 goes here, outs are not written
     const ETable *table;
-    const float *tok_scale;          // powers of two that the rows of x were divided by
+    const float *tok_scale;          // powers of two that the rows of x were divided by; negative: an infinite row
     const uint32_t *w[2];            // for rows that are added up from the definition
     const __nv_bfloat16 *x;
     const uint32_t *row_src;
@@ -96,8 +96,8 @@ struct __align__(16) ECtrl {
     int4 head[2];                                      // the item's pass: expert, first row, rows
     uint32_t tmem_base;
     volatile uint32_t abort;
-    volatile int again;                                // 1 + the last item with such results, for the epilogue
-    uint32_t marked[kEpiWarps];                        // its weight rows that are added up from the definition
+    volatile int again;                                // 1 + the last item with results that are added up from the definition
+    uint32_t again_rows[2][kEpiWarps];                 // of the item's rows those that are for every token, and all that there are
     uint64_t drained;                                  // giving up: the MMAs are complete
     uint32_t stages_issued, items_issued;              // what the producer started
     alignas(16) float row_factor[2][kRows];            // negative: a row whose scales the operands do not hold
@@ -192,7 +192,8 @@ __global__ void __launch_bounds__(256) exact_prep_kernel(const __nv_bfloat16 *x,
     const int ex = static_cast<int>(max(amax & 0xFFFFu, amax >> 16) >> 7);      // biased exponent of the row maximum
     const int e = ex == 0 || ex == 0xFF ? 0 : max(ex - 127 - 14, -126);        // zero rows and inf / nan rows stay unscaled; 2^-e and 2^e both normal
     const float down = __uint_as_float(static_cast<uint32_t>(127 - e) << 23);
-    if (on && i0 == 0) tok_scale[m] = __uint_as_float(static_cast<uint32_t>(127 + e) << 23);
+    // negative: an infinity and no NaN.  The products with such a token are added up from the definition.
+    if (on && i0 == 0) tok_scale[m] = __uint_as_float(static_cast<uint32_t>(127 + e) << 23 | (max(amax & 0xFFFFu, amax >> 16) == 0x7F80u ? 0x80000000u : 0u));
     auto convert = [&](int i, const uint4 &v) {
         const bool here = i < nvec;
         const uint32_t u[4] = {v.x, v.y, v.z, v.w};
@@ -339,19 +340,25 @@ __device__ __noinline__ void wide_blocks(uint32_t words, int r, uint32_t dst, in
 }
 
 // Results of an item that its operands do not hold, in the buffer of results, by the definition, a warp an output: those of the marked weight rows (`row`:
-// that of the calling thread of the epilogue is).
+// that of the calling thread of the epilogue is), and those of infinite tokens, where the infinity has met zeros and values of the other sign on
+// the way.
 __device__ __noinline__ void from_definition(const EArgs &a, ECtrl *ctl, const int4 pass, const int n0, const bool row) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, K = a.gpr << a.gs_shift;
-    const uint32_t rows = __ballot_sync(0xffffffffu, row && n0 + (a.two ? threadIdx.x & 63 : threadIdx.x) < static_cast<uint32_t>(a.n_out));
-    if (lane == 0) ctl->marked[warp] = rows;
+    const bool exists = n0 + (a.two ? threadIdx.x & 63 : threadIdx.x) < static_cast<uint32_t>(a.n_out);
+    const uint32_t marked = __ballot_sync(0xffffffffu, row && exists), all = __ballot_sync(0xffffffffu, exists);
+    if (lane == 0) {
+        ctl->again_rows[0][warp] = marked;
+        ctl->again_rows[1][warp] = all;
+    }
     asm volatile("bar.sync 1, 128;" ::: "memory");
     unsigned short *const staged = reinterpret_cast<unsigned short *>(reinterpret_cast<uint8_t *>(ctl) + kCtlBytes);
     for (int t = warp; t < pass.z; t += kEpiWarps) {         // the tokens that this warp stores
         size_t src = pass.y + t;
         if (a.row_src) src = a.row_src[src] < static_cast<uint32_t>(a.n_src_rows) ? a.row_src[src] : 0;
         const __nv_bfloat16 *const x = a.x + src * K;
+        const int which = ctl->tok_factor[warp][t] < 0.0f;
         for (int q = 0; q < kRows / 32; ++q)
-            for (uint32_t todo = ctl->marked[q]; todo != 0; todo &= todo - 1) {
+            for (uint32_t todo = ctl->again_rows[which][q]; todo != 0; todo &= todo - 1) {
                 const int at = q * 32 + __ffs(todo) - 1, m = a.two ? at >> 6 : 0;
                 const size_t n = static_cast<size_t>(pass.x) * a.n_out + n0 + (a.two ? at & 63 : at);
                 const float v = far_tokens::sum<4, MTC_BF16>(a.w[m] + n * (K / 8), static_cast<const __nv_bfloat16 *>(a.scales[m]) + n * a.gpr,
@@ -557,14 +564,15 @@ __global__ void __launch_bounds__(kThreads, 1) gather_exact_kernel(const __grid_
                 uint32_t least = min(low & 0xFFFFu, low >> 16);
                 if (least == 0) least = least_nonzero(row, rb);
                 // the biased exponent of the factor: 2^(118 - ex), or 2^(139 - ex) where that leaves a scale of these rows less than 2^-17, whose last bit f16 does
-                // not hold.  Rows that this leaves one, too, are marked.
+                // not hold.  Rows that this leaves one, too, are marked, and those with an infinity.
                 int up = max(245 - ex, 1);
                 const bool wide = __any_sync(0xffffffffu, static_cast<int>(least >> 7) + up < 237);
                 if (wide) up = min(max(266 - ex, 1), 253);
+                const bool mark = static_cast<int>(least >> 7) + up < 237 || ex >= 252;
                 const float f = __uint_as_float(static_cast<uint32_t>(up) << 23);
                 for (int c = 0; c < nch; ++c) {
                     if (turn == team) {
-                        if (c == 0) ctl->row_factor[e][r] = __uint_as_float(static_cast<uint32_t>(254 - up) << 23 | (static_cast<int>(least >> 7) + up < 237 ? 0x80000000u : 0u));
+                        if (c == 0) ctl->row_factor[e][r] = __uint_as_float(static_cast<uint32_t>(254 - up) << 23 | (mark ? 0x80000000u : 0u));
                         // in this order: with the MMAs of this team's stage before complete, the pass of the ring before this one is, and
                         // its phase cannot be taken for this one's
                         if (!wait(a_empty + team * 8, aph ^ 1, 0xa09)) return;
@@ -667,9 +675,14 @@ __global__ void __launch_bounds__(kThreads, 1) gather_exact_kernel(const __grid_
             bool ok = wait(item_full + e * 8, eph, 0xa0a);
             __syncwarp();
             const int4 pass = ctl->head[e];
+            bool infinite = false;                  // a token is
             if (ok) {
 #pragma unroll
-                for (int p = 0; p < kMaxTB; p += 32) tf[p + lane] = p + lane < pass.z ? a.tok_scale[pass.y + p + lane] : 0.0f;
+                for (int p = 0; p < kMaxTB; p += 32) {
+                    const float f = p + lane < pass.z ? a.tok_scale[pass.y + p + lane] : 0.0f;
+                    infinite = infinite || f < 0.0f;
+                    tf[p + lane] = f;
+                }
                 ok = wait(d_full + e * 8, eph, 0xa0b);
             }
             __syncwarp();
@@ -677,7 +690,7 @@ __global__ void __launch_bounds__(kThreads, 1) gather_exact_kernel(const __grid_
             if (!epilogue_votes(ok)) break;
             tc_fence_after();
             const float rf = ctl->row_factor[e][r];
-            if (rf < 0.0f) ctl->again = i + 1;
+            if (rf < 0.0f || infinite) ctl->again = i + 1;
             unsigned short *const to = reinterpret_cast<unsigned short *>(staged) + r;
 #pragma unroll 1
             for (int t0 = 0; t0 < pass.z; t0 += 16) {

@@ -118,6 +118,32 @@ def test_tokens_of_every_size():
     assert bool(((got.double() - ref).abs() <= bound)[keep].all())
 
 
+@pytest.mark.parametrize("g,k", [(64, 256), (128, 640)])
+def test_infinities_are_what_the_definition_gives(g, k):
+    """An infinite activation, bias or scale: infinities of the products' signs, NaN where two signs meet (or a weight of zero); others are as without it."""
+    import torch
+    from metaltile_b200 import ops
+
+    inf = float("inf")
+
+    def odd(x):
+        x = x.clone()
+        x[3, 17], x[7, 130], x[20, 200], x[20, 3] = inf, -inf, float("nan"), inf
+        x[33, 5], x[33, k - 1] = inf, -inf
+        return x
+
+    def change(s, b):
+        s, b = s.clone(), b.clone()
+        b[0, 9, 1], b[1, 70, 0], s[1, 71, 2] = inf, -inf, inf
+        return s, b
+
+    got, ref, bound = _product(torch, ops, ops.context(), [30, 15], 136, k, g, change, odd)
+    finite = torch.isfinite(ref)
+    assert bool(((got.double() - ref).abs() <= bound)[finite].all())
+    assert torch.equal(got[~finite].double().nan_to_num(7.0, 1.0, -1.0), ref[~finite].nan_to_num(7.0, 1.0, -1.0))
+    assert bool(finite[8].any()) and bool((ref[3] == inf).any()) and bool((ref[3] == -inf).any()) and not bool(finite[[3, 7, 20, 33]].any())
+
+
 @pytest.mark.parametrize("tokens,e,top,hidden,inter,g", [(40, 8, 2, 512, 320, 64), (90, 16, 8, 384, 256, 128), (100, 8, 4, 448, 200 * 8, 64)])
 def test_layer_equals_the_separate_entries(tokens, e, top, hidden, inter, g):
     import torch
