@@ -258,7 +258,7 @@ __device__ __forceinline__ void dequant_half(const uint32_t (&w)[BITS], float s,
 }
 // A k block of a row, 64 codes (words(h, w): those of half h) with one scale (ONE: groups of 64 and more) or two, in packed halves with no conversion: a 16-bit float with exponent
 // field 0 is linear in its low bits, so a code at bit P of its half is q * 2^(P - 24), and fma(that, scale * 2^(24 - P), bias) is
-// round_f16(q * scale + bias), the value the general form rounds to up to double rounding.  4-bit codes get there by bytes (bit 7 is 0 where the nibble
+// round_f16(q * scale + bias), the value the general form rounds to (4 and 8 bits: with the bias an f16 of its own first).  4-bit codes get there by bytes (bit 7 is 0 where the nibble
 // is at bits 3..6, so the sign-replicating form of the byte permute fills the upper byte with zeros): 12 instructions per eight codes (16 with the codes
 // brought to 1024 + q first); 8-bit ones by a byte permute, 8; others by two shifts and two masks a pair, 20 to 22 (32 by way of f32).  The scale
 // times 2^(24 - P) is an f16 in all but odd cases (an underflow of it is far below the last bit of any result): those take the general form.
@@ -267,8 +267,10 @@ __device__ __forceinline__ void dequant_block(Get words, float s0, float b0, flo
     // where a code lies in its half of a register: bit 3 (4 bits), 0 (8 bits), at the top of the ten bits of a fraction (others)
     constexpr int P = BITS == 4 ? 3 : BITS == 8 ? 0 : 10 - BITS;
     constexpr float kUp = static_cast<float>(1 << (24 - P)), kMost = 65472.0f / kUp;
-    bool direct = fabsf(s0) <= kMost && fabsf(b0) <= 65504.0f;
-    if (!ONE) direct = direct && fabsf(s1) <= kMost && fabsf(b1) <= 65504.0f;
+    // a bias that is no f16 (a bf16 below 2^-17) would be rounded by itself first
+    auto fits = [](float b) { return BITS == 4 || BITS == 8 ? fabsf(b) <= 65504.0f : __half2float(__float2half_rn(b)) == b; };
+    bool direct = fabsf(s0) <= kMost && fits(b0);
+    if (!ONE) direct = direct && fabsf(s1) <= kMost && fits(b1);
     if (direct) {
         __half2 s2 = __float2half2_rn(s0 * kUp), b2 = __float2half2_rn(b0);
 #pragma unroll

@@ -48,3 +48,22 @@ def test_product_against_float64(m, n, k, bits, g, dt, factor, off, options):
     mag = x.double().abs() @ weights.abs().T
     bound = x.double().abs() @ per_weight.T + (k / 16 + 16) * 2.0 ** -24 * mag + (2.0 ** -8 if dt == "bf16" else 2.0 ** -11) * want.abs() + 2.0 ** -25
     assert bool(((got.double() - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("g", [32, 64])
+@pytest.mark.parametrize("bits", [2, 3, 5, 6])
+def test_a_weight_is_rounded_once(bits, g):
+    """Scale and bias just below half of the least f16, codes of one: their sum is that f16, and each alone would be rounded to nothing."""
+    import torch
+    from metaltile_b200 import ops
+
+    m, n, k = 40, 136, 512
+    row = 0
+    for i in range(k):
+        row |= 1 << (i * bits)
+    words = [(row >> (32 * i)) & 0xFFFFFFFF for i in range(k * bits // 32)]
+    w = torch.tensor(words, dtype=torch.int64, device="cuda").to(torch.int32).expand(n, -1).contiguous()
+    s = torch.full((n, k // g), 255 * 2.0 ** -33, dtype=torch.bfloat16, device="cuda")
+    x = torch.full((m, k), 1024.0, dtype=torch.bfloat16, device="cuda")
+    assert ops.context().launch_of(m, [n], k, bits, g, "bf16")["kernel"] == "qmm_tcgen05"
+    assert bool((ops.qmm(w, s, s, x, bits, g).double() == k * 1024 * 2.0 ** -24).all())
