@@ -259,42 +259,49 @@ __device__ __forceinline__ void dequant_half(const uint32_t (&w)[BITS], float s,
 // A k block of a row, 64 codes (words(h, w): those of half h) with one scale (ONE: groups of 64 and more) or two, in packed halves with no conversion: a 16-bit float with exponent
 // field 0 is linear in its low bits, so a code at bit P of its half is q * 2^(P - 24), and fma(that, scale * 2^(24 - P), bias) is
 // round_f16(q * scale + bias), the value the general form rounds to (4 and 8 bits: with the bias an f16 of its own first).  4-bit codes get there by bytes (bit 7 is 0 where the nibble
-// is at bits 3..6, so the sign-replicating form of the byte permute fills the upper byte with zeros): 12 instructions per eight codes (16 with the codes
-// brought to 1024 + q first); 8-bit ones by a byte permute, 8; others by two shifts and two masks a pair, 20 to 22 (32 by way of f32).  The scale
-// times 2^(24 - P) is an f16 in all but odd cases (an underflow of it is far below the last bit of any result): those take the general form.
+// is at bits 3..6, so the sign-replicating form of the byte permute fills the upper byte with zeros): 12 instructions per eight codes; 8-bit ones by a
+// byte permute, 8; others by two shifts and two masks a pair, 20 to 22 (32 by way of f32).
+// That takes scales up to 65472 / 2^(24 - P): 0.031 (4 bits), 0.0039 (8 bits).  Where a row of the warp has larger ones, its codes become 1024 + q * 2^P by
+// an OR of the exponent, an exact subtraction takes the 1024 away, and the factor is scale * 2^-P, one instruction a pair more; a warp whose scales are too far apart for
+// either form takes the general one.  The choice is the warp's: lanes that go different ways take the time of both.
 template <int BITS, bool ONE, typename Get>
 __device__ __forceinline__ void dequant_block(Get words, float s0, float b0, float s1, float b1, uint32_t (&v)[32]) {
     // where a code lies in its half of a register: bit 3 (4 bits), 0 (8 bits), at the top of the ten bits of a fraction (others)
     constexpr int P = BITS == 4 ? 3 : BITS == 8 ? 0 : 10 - BITS;
-    constexpr float kUp = static_cast<float>(1 << (24 - P)), kMost = 65472.0f / kUp;
+    constexpr float kUp = static_cast<float>(1 << (24 - P)), kMost = 65472.0f / kUp, kDown = 1.0f / (1 << P);
+    auto f16_holds = [](float f) { return __half2float(__float2half_rn(f)) == f; };
     // a bias that is no f16 (a bf16 below 2^-17) would be rounded by itself first
-    auto fits = [](float b) { return BITS == 4 || BITS == 8 ? fabsf(b) <= 65504.0f : __half2float(__float2half_rn(b)) == b; };
-    bool direct = fabsf(s0) <= kMost && fits(b0);
-    if (!ONE) direct = direct && fabsf(s1) <= kMost && fits(b1);
-    if (direct) {
-        __half2 s2 = __float2half2_rn(s0 * kUp), b2 = __float2half2_rn(b0);
+    auto fits = [&](float b) { return BITS == 4 || BITS == 8 ? fabsf(b) <= 65504.0f : f16_holds(b); };
+    auto packed = [&](auto form) {
+        constexpr bool LARGE = decltype(form)::value;
+        constexpr float kFactor = LARGE ? kDown : kUp;
+        __half2 s2 = __float2half2_rn(s0 * kFactor), b2 = __float2half2_rn(b0);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             if (!ONE && h == 1) {
-                s2 = __float2half2_rn(s1 * kUp);
+                s2 = __float2half2_rn(s1 * kFactor);
                 b2 = __float2half2_rn(b1);
             }
             uint32_t w[BITS];
             words(h, w);
             const uint32_t s = *reinterpret_cast<const uint32_t *>(&s2), b = *reinterpret_cast<const uint32_t *>(&b2);
-            auto put = [&](int i, uint32_t q) { asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(v[16 * h + i]) : "r"(q), "r"(s), "r"(b)); };
+            auto put = [&](int i, uint32_t q) {          // LARGE: 1024 + q * 2^P
+                if (LARGE) asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(q) : "r"(q), "r"(0x64006400u));
+                asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(v[16 * h + i]) : "r"(q), "r"(s), "r"(b));
+            };
+            constexpr uint32_t kOne = LARGE ? 0x64006400u : 0u, kTop = LARGE ? 0x64646464u : 0u;
             if constexpr (BITS == 4) {
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {    // byte j of lo / hi: code 2j / 2j+1 at bits 3..6
                     const uint32_t lo = (w[i] << 3) & 0x78787878u, hi = (w[i] >> 1) & 0x78787878u;
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) put(4 * i + j, prmt(lo, hi, ((0xC + j) << 12) | ((4 + j) << 8) | ((8 + j) << 4) | j));
+                    for (int j = 0; j < 4; ++j) put(4 * i + j, prmt(lo, hi, ((0xC + j) << 12) | ((4 + j) << 8) | ((8 + j) << 4) | j) | kOne);
                 }
             } else if constexpr (BITS == 8) {
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
-                    put(2 * i, prmt(w[i], 0u, 0x4140));
-                    put(2 * i + 1, prmt(w[i], 0u, 0x4342));
+                    put(2 * i, prmt(w[i], kTop, 0x4140));
+                    put(2 * i + 1, prmt(w[i], kTop, 0x4342));
                 }
             } else {
                 constexpr uint32_t kLow = ((1u << BITS) - 1u) << P, kHigh = kLow << 16;
@@ -309,17 +316,23 @@ __device__ __forceinline__ void dequant_block(Get words, float s0, float b0, flo
                     }
                     const int up0 = P - sh, up1 = 16 + P - sh - BITS;
                     const uint32_t lo = up0 >= 0 ? t << (up0 & 31) : t >> (-up0 & 31), hi = up1 >= 0 ? t << (up1 & 31) : t >> (-up1 & 31);
-                    put(i, (lo & kLow) | (hi & kHigh));
+                    put(i, ((lo & kLow) | kOne) | (hi & kHigh));
                 }
             }
         }
-        return;
-    }
+    };
+    const bool small = fabsf(s0) <= kMost && fits(b0) && (ONE || (fabsf(s1) <= kMost && fits(b1)));
+    if (__all_sync(0xffffffffu, small)) {
+        packed(std::false_type{});
+    } else if (__all_sync(0xffffffffu, f16_holds(s0 * kDown) && fits(b0) && (ONE || (f16_holds(s1 * kDown) && fits(b1))))) {
+        packed(std::true_type{});
+    } else {
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        uint32_t w[BITS];
-        words(h, w);
-        dequant_half<BITS>(w, ONE || h == 0 ? s0 : s1, ONE || h == 0 ? b0 : b1, v + 16 * h);
+        for (int h = 0; h < 2; ++h) {
+            uint32_t w[BITS];
+            words(h, w);
+            dequant_half<BITS>(w, ONE || h == 0 ? s0 : s1, ONE || h == 0 ? b0 : b1, v + 16 * h);
+        }
     }
 }
 __device__ __forceinline__ float sb_value(uint32_t bits, int dt) {
