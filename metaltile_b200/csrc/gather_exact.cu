@@ -771,10 +771,16 @@ int row_elems(int K) { return K + (K / 64 + kSegs - 1) / kSegs * kBlk; }
 // Scales and biases of an item as they lie in memory: 128 rows; the ring starts behind two of them.
 int item_bytes(int gpr) { return 2 * kRows * gpr * 2; }
 int ring_offset(int gpr) { return (kCtlBytes + kOutBytes + 2 * item_bytes(gpr) + 1023) / 1024 * 1024; }
-// Rows of a pass at most: 32, 48 or 64 columns are stages of 32, 40 or 48 KB.  Room for nearly all of the experts of an even router.
-int pass_rows(int m_total, int n_experts) {
+// Three stages have to fit beside the rows of scales.
+bool passes_fit(int TB, int gpr) { return ring_offset(gpr) + 3 * (kWordBytes + kChunk * TB * 128) <= kSmemBytes; }
+// Rows of a pass at most: 32, 48 or 64 columns are stages of 32, 40 or 48 KB.  Room for nearly all of the experts of an even router, or fewer where
+// rows of scales are long: 64 columns fit beside 63 groups, 48 beside 87, 32 beside 111.  0: none do.  (8 experts of 4096 x 1536, groups of 64, where 64
+// columns do not fit, 40 / 60 / 300 rows an expert: 74 / 89 / 203 us; the other kernels 130 / 159 / 285 at that time.)
+int pass_rows(int m_total, int n_experts, int gpr) {
     const long long rows = m_total, e = n_experts;
-    return rows <= 16 * e ? 32 : rows <= 34 * e ? 48 : 64;
+    int TB = rows <= 16 * e ? 32 : rows <= 34 * e ? 48 : 64;
+    while (TB > 0 && !passes_fit(TB, gpr)) TB = TB > 32 ? TB - 16 : 0;
+    return TB;
 }
 
 }  // namespace
@@ -786,9 +792,8 @@ bool gather_exact_supported(int m_total, int n_out, int K, int n_experts, int bi
     if (static_cast<long long>(n_experts) + m_total / 32 > kMaxPasses) return false;
     if (static_cast<long long>(n_experts) * n_out > 0x7FFF0000ll || static_cast<long long>(m_total) * K > (1ll << 40)) return false;
     const int gpr = K / group_size;
-    // scales and biases of an item are copied in one piece; three stages have to fit beside them
-    if (static_cast<long long>(n_out) * gpr % 8 != 0 || gpr > 1024 ||
-        ring_offset(gpr) + 3 * (kWordBytes + kChunk * pass_rows(m_total, n_experts) * 128) > kSmemBytes) return false;
+    // scales and biases of an item are copied in one piece
+    if (static_cast<long long>(n_out) * gpr % 8 != 0 || gpr > kSmemBytes / (2 * kRows * 4) || pass_rows(m_total, n_experts, gpr) == 0) return false;
     const auto al = [](const void *q, uintptr_t n) { return q == nullptr || reinterpret_cast<uintptr_t>(q) % n == 0; };
     return al(w, 16) && al(x, 16) && al(scales, 16) && al(biases, 16);
 }
@@ -804,7 +809,7 @@ cudaError_t launch_gather_exact(Ctx *ctx, cudaStream_t st, const void *x, const 
                                 void *act, const uint32_t *expert_offsets, int m_total, int n_out, int K, int n_experts, int group_size, void *scratch,
                                 std::string *why) {
     if (n_mats < 1 || n_mats > 2 || (act && n_mats != 2)) return cudaErrorInvalidValue;
-    const int elems = row_elems(K), TB = pass_rows(m_total, n_experts);
+    const int elems = row_elems(K), TB = pass_rows(m_total, n_experts, K / group_size);
     unsigned short *xprep = static_cast<unsigned short *>(scratch);
     float *tok_scale = reinterpret_cast<float *>(static_cast<char *>(scratch) + up256(static_cast<size_t>(m_total) * elems * 2));
     ETable *table = reinterpret_cast<ETable *>(reinterpret_cast<char *>(tok_scale) + up256(static_cast<size_t>(m_total) * sizeof(float)));

@@ -289,7 +289,7 @@ __device__ __forceinline__ void dequant_block(Get words, float s0, float b0, flo
                 if (LARGE) asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(q) : "r"(q), "r"(0x64006400u));
                 asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(v[16 * h + i]) : "r"(q), "r"(s), "r"(b));
             };
-            constexpr uint32_t kOne = LARGE ? 0x64006400u : 0u, kTop = LARGE ? 0x64646464u : 0u;
+            [[maybe_unused]] constexpr uint32_t kOne = LARGE ? 0x64006400u : 0u, kTop = LARGE ? 0x64646464u : 0u;
             if constexpr (BITS == 4) {
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {    // byte j of lo / hi: code 2j / 2j+1 at bits 3..6

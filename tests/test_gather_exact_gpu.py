@@ -40,7 +40,9 @@ def _product(torch, ops, ctx, counts, n, k, g, change=None, x_change=None, seed=
 
 CASES = [([1, 15, 16, 17], 64, 64, 64), ([31, 0, 32, 33], 72, 128, 64), ([47, 48, 49], 200, 192, 64), ([63, 64, 65, 0, 130], 128, 320, 64),
          ([9, 300], 136, 256, 128), ([40, 7, 25], 64, 640, 128), ([20, 21], 264, 1088, 64), ([5, 36], 320, 2048, 64), ([30], 8, 448, 64),
-         ([12, 6, 44], 96, 4096, 64), ([18] * 40, 64, 128, 128)]
+         ([12, 6, 44], 96, 4096, 64), ([18] * 40, 64, 128, 128),
+         # long rows of scales: the most for 64 columns, one more, the most for 48, one more, the most for 32
+         ([64, 41], 64, 4032, 64), ([64, 41], 64, 4096, 64), ([48, 49], 64, 5568, 64), ([48, 49], 64, 5632, 64), ([33, 64], 64, 7104, 64)]
 
 
 @pytest.mark.parametrize("counts,n,k,g", CASES)
@@ -144,7 +146,9 @@ def test_infinities_are_what_the_definition_gives(g, k):
     assert bool(finite[8].any()) and bool((ref[3] == inf).any()) and bool((ref[3] == -inf).any()) and not bool(finite[[3, 7, 20, 33]].any())
 
 
-@pytest.mark.parametrize("tokens,e,top,hidden,inter,g", [(40, 8, 2, 512, 320, 64), (90, 16, 8, 384, 256, 128), (100, 8, 4, 448, 200 * 8, 64)])
+@pytest.mark.parametrize("tokens,e,top,hidden,inter,g", [(40, 8, 2, 512, 320, 64), (90, 16, 8, 384, 256, 128), (100, 8, 4, 448, 200 * 8, 64),
+                                                               (40, 4, 4, 4096, 320, 64),       # passes of 48 rows, then of 64
+                                                               (6, 4, 2, 8192, 256, 64), (40, 4, 2, 8192, 256, 64), (30, 4, 2, 7168, 320, 64)])      # down alone
 def test_layer_equals_the_separate_entries(tokens, e, top, hidden, inter, g):
     import torch
     from metaltile_b200 import ops
@@ -159,6 +163,15 @@ def test_layer_equals_the_separate_entries(tokens, e, top, hidden, inter, g):
     act = ops.swiglu(ops.gather_qmm(rows, *gate, 4, g, expert_offsets=off), ops.gather_qmm(rows, *up, 4, g, expert_offsets=off))
     assert torch.equal(fused, ops.gather_qmm(act, *down, 4, g, expert_offsets=off))
     assert ops.context().status_word() == 0
+
+
+def test_long_rows_of_scales_take_narrower_passes():
+    from metaltile_b200 import _lib
+    from metaltile_b200.context import _dt
+
+    route = lambda k, rows, dt="bf16": _lib.load().mtc_gather_qmm_route(8 * rows, 1536, k, 8, 4, 64, _dt(dt)).decode()  # noqa: E731
+    assert {route(64 * g, 300) for g in (63, 64, 87, 88, 111)} == {route(2048, 300)}
+    assert route(64 * 112, 300) == route(64 * 112, 300, "f16") != route(2048, 300)
 
 
 def test_rule():
