@@ -1282,80 +1282,56 @@ int mtc_moe_experts(mtc_ctx *ctx, void *stream, const void *x, const void *sort_
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const size_t esz = mtc::dtype_size(dtype);
     const size_t act_bytes = align_up(static_cast<size_t>(m_total) * inter * esz, 256), xp_bytes = align_up(static_cast<size_t>(m_total) * hidden * esz, 256);
-    // the kernels that mtc_gather_qmm takes for the three products: fused where they agree, composed from the entries where they do not
-    const mtc_qmat *const mats[3] = {gate, up, down};
-    int n_frag = 0, n_stream = 0, n_exact = 0;
-    for (int i = 0; i < 3; ++i) {
-        const int n = i < 2 ? inter : hidden, k = i < 2 ? hidden : inter;
-        const void *const in = i < 2 ? x : nullptr;
-        n_frag += gather_frag_takes(ctx, true, m_total, n, k, n_experts, bits, group_size, dtype, mats[i]->w, mats[i]->scales, mats[i]->biases, in);
-        n_exact += gather_exact_takes(ctx, true, m_total, n, k, n_experts, bits, group_size, dtype, mats[i]->w, mats[i]->scales, mats[i]->biases, in);
-        n_stream += gather_stream_takes(ctx, true, m_total, n, k, n_experts, bits, group_size, dtype, mats[i]->w, mats[i]->scales, mats[i]->biases, in);
-    }
-    const bool frag = n_frag == 3, exact = n_frag == 0 && n_exact == 3, streamed = n_frag == 0 && n_exact == 0 && n_stream == 3;
+    // The kernels that mtc_gather_qmm takes for the three products.  Gate and up are one launch where they agree (they may not where their arrays are aligned
+    // differently), whatever runs down: with 8 experts of 8192 x 1024 in groups of 64 the exact kernel takes down alone, and a layer composed from the entries
+    // took 138 us for 10 tokens, 86 so (40 tokens 154, 121).
+    enum { OTHER, FRAG, EXACT, STREAM };
+    auto kernel_of = [&](const mtc_qmat *m, int n, int k, const void *in) {
+        if (gather_frag_takes(ctx, true, m_total, n, k, n_experts, bits, group_size, dtype, m->w, m->scales, m->biases, in)) return FRAG;
+        if (gather_exact_takes(ctx, true, m_total, n, k, n_experts, bits, group_size, dtype, m->w, m->scales, m->biases, in)) return EXACT;
+        return gather_stream_takes(ctx, true, m_total, n, k, n_experts, bits, group_size, dtype, m->w, m->scales, m->biases, in) ? STREAM : OTHER;
+    };
+    const auto for_gate = kernel_of(gate, inter, hidden, x), for_up = kernel_of(up, inter, hidden, x), pair = for_gate == for_up ? for_gate : OTHER,
+               last = kernel_of(down, hidden, inter, nullptr);
     std::string why;
-    cudaError_t e = mtc::grow_block(ctx, st, &ctx->d_moe, &ctx->moe_bytes, 2 * act_bytes + (streamed || exact || frag ? 0 : xp_bytes), &why);
+    cudaError_t e = mtc::grow_block(ctx, st, &ctx->d_moe, &ctx->moe_bytes, 2 * act_bytes + (pair == OTHER ? xp_bytes : 0), &why);
     if (e != cudaSuccess) return fail(ctx, MTC_ERR_BUFFER, "moe_experts intermediates: " + (why.empty() ? std::string(cudaGetErrorString(e)) : why));
     char *g = static_cast<char *>(ctx->d_moe), *u = g + act_bytes, *xp = u + act_bytes;
-    if (frag) {
-        // three launches: gate and up (the permutation folded in), SwiGLU, down
-        const uint32_t *offsets = static_cast<const uint32_t *>(expert_offsets);
-        const mtc::GatherMats gu[2] = {{gate->w, gate->scales, gate->biases, g}, {up->w, up->scales, up->biases, u}};
-        e = mtc::launch_gather_frag(ctx, st, x, static_cast<const uint32_t *>(sort_token_idx), n_tokens, gu, 2, offsets, m_total, inter, hidden, n_experts,
-                                    bits, group_size, dtype);
-        if (e != cudaSuccess) return fail(ctx, MTC_ERR_DISPATCH, std::string("moe_experts (gate, up) launch: ") + cudaGetErrorString(e));
-        const int rc = mtc_swiglu(ctx, stream, g, u, g, static_cast<size_t>(m_total) * inter, dtype);
-        if (rc != MTC_OK) return rc;
-        const mtc::GatherMats dn{down->w, down->scales, down->biases, y};
-        e = mtc::launch_gather_frag(ctx, st, g, nullptr, 0, &dn, 1, offsets, m_total, hidden, inter, n_experts, bits, group_size, dtype);
-        if (e != cudaSuccess) return fail(ctx, MTC_ERR_DISPATCH, std::string("moe_experts (down) launch: ") + cudaGetErrorString(e));
-        return MTC_OK;
-    }
-    if (exact) {
-        // four launches: rows -> operands (the permutation folded in), gate and up with SwiGLU, rows -> operands, down
-        const size_t need = std::max(mtc::gather_exact_scratch_bytes(m_total, hidden), mtc::gather_exact_scratch_bytes(m_total, inter));
+    auto staged_bytes = [&](int kernel, int k) {
+        return kernel == EXACT ? mtc::gather_exact_scratch_bytes(m_total, k) : kernel == STREAM ? mtc::gather_stream_scratch_bytes(m_total, k) : 0;
+    };
+    if (const size_t need = std::max(staged_bytes(pair, hidden), staged_bytes(last, inter))) {
         e = mtc::grow_block(ctx, st, &ctx->d_gfrag, &ctx->gfrag_bytes, need, &why);
         if (e != cudaSuccess) return fail(ctx, MTC_ERR_BUFFER, "moe_experts staging: " + (why.empty() ? std::string(cudaGetErrorString(e)) : why));
-        const mtc::GatherMats gu[2] = {{gate->w, gate->scales, gate->biases, nullptr}, {up->w, up->scales, up->biases, nullptr}};
-        e = mtc::launch_gather_exact(ctx, st, x, static_cast<const uint32_t *>(sort_token_idx), n_tokens, gu, 2, g, static_cast<const uint32_t *>(expert_offsets),
-                                     m_total, inter, hidden, n_experts, group_size, ctx->d_gfrag, &why);
-        if (e != cudaSuccess) return fail(ctx, MTC_ERR_DISPATCH, std::string("moe_experts (gate, up) launch: ") + cudaGetErrorString(e));
-        const mtc::GatherMats dn{down->w, down->scales, down->biases, y};
-        e = mtc::launch_gather_exact(ctx, st, g, nullptr, 0, &dn, 1, nullptr, static_cast<const uint32_t *>(expert_offsets), m_total, hidden, inter,
-                                     n_experts, group_size, ctx->d_gfrag, &why);
-        if (e != cudaSuccess) return fail(ctx, MTC_ERR_DISPATCH, std::string("moe_experts (down) launch: ") + cudaGetErrorString(e));
-        return MTC_OK;
     }
-    if (streamed) {
-        // four launches: rows -> fragments (the permutation folded in), gate and up as one stream, SwiGLU -> fragments, down
-        const size_t need = std::max(mtc::gather_stream_scratch_bytes(m_total, hidden), mtc::gather_stream_scratch_bytes(m_total, inter));
-        e = mtc::grow_block(ctx, st, &ctx->d_gfrag, &ctx->gfrag_bytes, need, &why);
-        if (e != cudaSuccess) return fail(ctx, MTC_ERR_BUFFER, "moe_experts staging: " + (why.empty() ? std::string(cudaGetErrorString(e)) : why));
-        const mtc::GatherMats gu[2] = {{gate->w, gate->scales, gate->biases, g}, {up->w, up->scales, up->biases, u}};
-        e = mtc::launch_gather_stream(ctx, st, x, nullptr, static_cast<const uint32_t *>(sort_token_idx), n_tokens, gu, 2,
-                                      static_cast<const uint32_t *>(expert_offsets), m_total, inter, hidden, n_experts, group_size, dtype,
-                                      ctx->d_gfrag);
-        if (e != cudaSuccess) return fail(ctx, MTC_ERR_DISPATCH, std::string("moe_experts (gate, up) launch: ") + cudaGetErrorString(e));
-        const mtc::GatherMats dn{down->w, down->scales, down->biases, y};
-        e = mtc::launch_gather_stream(ctx, st, g, u, nullptr, 0, &dn, 1, static_cast<const uint32_t *>(expert_offsets), m_total, hidden, inter,
-                                      n_experts, group_size, dtype, ctx->d_gfrag);
-        if (e != cudaSuccess) return fail(ctx, MTC_ERR_DISPATCH, std::string("moe_experts (down) launch: ") + cudaGetErrorString(e));
-        return MTC_OK;
-    }
-    // composed from the separate entries, same results
-    const void *rows = x;
+    const uint32_t *const offsets = static_cast<const uint32_t *>(expert_offsets), *const order = static_cast<const uint32_t *>(sort_token_idx);
+    const mtc::GatherMats gu[2] = {{gate->w, gate->scales, gate->biases, g}, {up->w, up->scales, up->biases, u}};
     int rc = MTC_OK;
-    if (sort_token_idx) {
-        rc = mtc_moe_permute(ctx, stream, x, sort_token_idx, xp, m_total, hidden, dtype);
-        if (rc != MTC_OK) return rc;
-        rows = xp;
+    if (pair == OTHER) {
+        const void *rows = x;
+        if (order) {
+            rc = mtc_moe_permute(ctx, stream, x, sort_token_idx, xp, m_total, hidden, dtype);
+            if (rc != MTC_OK) return rc;
+            rows = xp;
+        }
+        for (const mtc::GatherMats &m : gu) {
+            rc = mtc_gather_qmm(ctx, stream, rows, m.w, m.scales, m.biases, expert_offsets, nullptr, m.out, m_total, inter, hidden, n_experts, bits, group_size, dtype);
+            if (rc != MTC_OK) return rc;
+        }
+    } else {
+        // the permutation folded in: fragment kernel; rows -> operands, the exact kernel with SwiGLU; rows -> fragments, both matrices as one stream
+        e = pair == FRAG ? mtc::launch_gather_frag(ctx, st, x, order, n_tokens, gu, 2, offsets, m_total, inter, hidden, n_experts, bits, group_size, dtype)
+            : pair == EXACT ? mtc::launch_gather_exact(ctx, st, x, order, n_tokens, gu, 2, g, offsets, m_total, inter, hidden, n_experts, group_size, ctx->d_gfrag, &why)
+                            : mtc::launch_gather_stream(ctx, st, x, nullptr, order, n_tokens, gu, 2, offsets, m_total, inter, hidden, n_experts, group_size, dtype, ctx->d_gfrag);
+        if (e != cudaSuccess) return fail(ctx, MTC_ERR_DISPATCH, "moe_experts (gate, up) launch: " + (why.empty() ? std::string(cudaGetErrorString(e)) : why));
     }
-    rc = mtc_gather_qmm(ctx, stream, rows, gate->w, gate->scales, gate->biases, expert_offsets, nullptr, g, m_total, inter, hidden, n_experts, bits, group_size, dtype);
-    if (rc != MTC_OK) return rc;
-    rc = mtc_gather_qmm(ctx, stream, rows, up->w, up->scales, up->biases, expert_offsets, nullptr, u, m_total, inter, hidden, n_experts, bits, group_size, dtype);
-    if (rc != MTC_OK) return rc;
-    rc = mtc_swiglu(ctx, stream, g, u, g, static_cast<size_t>(m_total) * inter, dtype);
-    if (rc != MTC_OK) return rc;
+    if (pair == STREAM && last == STREAM) {          // SwiGLU -> fragments, down
+        const mtc::GatherMats dn{down->w, down->scales, down->biases, y};
+        e = mtc::launch_gather_stream(ctx, st, g, u, nullptr, 0, &dn, 1, offsets, m_total, hidden, inter, n_experts, group_size, dtype, ctx->d_gfrag);
+        if (e != cudaSuccess) return fail(ctx, MTC_ERR_DISPATCH, std::string("moe_experts (down) launch: ") + cudaGetErrorString(e));
+        return MTC_OK;
+    }
+    if (pair != EXACT && (rc = mtc_swiglu(ctx, stream, g, u, g, static_cast<size_t>(m_total) * inter, dtype)) != MTC_OK) return rc;
     return mtc_gather_qmm(ctx, stream, g, down->w, down->scales, down->biases, expert_offsets, nullptr, y, m_total, hidden, inter, n_experts, bits, group_size, dtype);
 }
 
