@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(kQvWarps * 32, 2) qvm_kernel(const uint32_t *w
 // The same arithmetic with the packed words on their way through shared memory.  Above, a warp has one or two slabs in flight and waits between
 // them, with 3 instructions a code beside.  Here a warp owns a contiguous range of units (16 rows of 128 bytes) of its CTA's chunk of K and keeps four of
 // them in flight with 16-byte asynchronous copies; x waits as f32 times 2^64 beside the sum of every unit, so a code costs one LOP3, one FFMA and a
-// quarter of an instruction more, and scales are applied once a group (f32: once a unit), from registers that were loaded when the group began.  One CTA of 16 warps
+// quarter of an instruction more, and scales are applied once a group (f32: once a unit) to the sum of its units' sums, from registers that were loaded when the group began.  One CTA of 16 warps
 // an SM, which has the SM's shared memory to itself: with room for two, CTAs land in pairs and leave SMs idle (17.9 us for the first shape below), and
 // two or three CTAs of 8 warps in twice or three times as many chunks of K pay more for start and sum (13.5, 14.4).  Six units in flight: 14.0; 24 warps:
 // 13.8.  bf16, 4-bit groups of 64, K x N 14336 x 4096 14.8 -> 13.2 us, 4096 x 4096 7.5 -> 7.0, 4096 x 14336 14.7 -> 13.0, 16384 x 16384 52.4 -> 36.3 (4.2
@@ -352,9 +352,9 @@ __global__ void __launch_bounds__(kQrWarps * 32, 1) qvm_ring_kernel(const uint32
         if ((i & 3) == 0) ssum[i / 4] = t;
     }
     __syncthreads();
-    float acc[CPT], raw[CPT], xs = 0.0f;
+    float acc[CPT], of_group[CPT], xs = 0.0f;
 #pragma unroll
-    for (int j = 0; j < CPT; ++j) acc[j] = raw[j] = 0.0f;
+    for (int j = 0; j < CPT; ++j) acc[j] = of_group[j] = 0.0f;
     int slot = 0;
     for (int u = u0; u < u1; ++u) {
         asm volatile("cp.async.wait_group %0;" ::"n"(D - 1) : "memory");
@@ -366,6 +366,9 @@ __global__ void __launch_bounds__(kQrWarps * 32, 1) qvm_ring_kernel(const uint32
         for (int r = 0; r < R; ++r) wd[r][0] = wp[r * 32];
         __syncwarp();
         fetch();                                                   // the slot is in registers
+        float raw[CPT];
+#pragma unroll
+        for (int j = 0; j < CPT; ++j) raw[j] = 0.0f;
 #pragma unroll
         for (int r4 = 0; r4 < R; r4 += 4) {
             const float4 xv = *reinterpret_cast<const float4 *>(xp + r4);
@@ -378,13 +381,15 @@ __global__ void __launch_bounds__(kQrWarps * 32, 1) qvm_ring_kernel(const uint32
         xs += ssum[u - c0];
         if (++slot == D) slot = 0;
         const bool end = --left == 0 || u + 1 == u1;
-        // f32: sums no longer than above (with a whole group of them the error against 64 bits was 1.1 to 2 times as large; 16-bit results are the same)
+        // sums of codes are those of a unit, as above (f32 with a whole group of them: the error against 64 bits was 1.1 to 2 times as large)
+#pragma unroll
+        for (int j = 0; j < CPT; ++j) of_group[j] = DT == MTC_F32 ? raw[j] : of_group[j] + raw[j];
         if (DT == MTC_F32 || end) {
 #pragma unroll
             for (int j = 0; j < CPT; ++j) {
                 const float post = __uint_as_float(static_cast<uint32_t>(127 + 85 - QvCode<BITS>::pos(j)) << 23);     // 2^(85 - p)
-                acc[j] = fmaf(qv_elem<DT>(sv, j) * post, raw[j], fmaf(qv_elem<DT>(bv, j), xs, acc[j]));
-                raw[j] = 0.0f;
+                acc[j] = fmaf(qv_elem<DT>(sv, j) * post, of_group[j], fmaf(qv_elem<DT>(bv, j), xs, acc[j]));
+                of_group[j] = 0.0f;
             }
             xs = 0.0f;
         }
