@@ -1397,7 +1397,7 @@ DensePlan plan_dense(const Ctx *ctx, int M, int N, int K, int bits, int group_si
     // Up to 256 rows over four super-blocks of K, where four slices are one round: clusters of four, the form that tests/test_launches.py holds these
     // products to (186 x 4096 x 1024 13.6 -> 12.4 us; four narrower whole items would take 9.5)
     const int tn_one = up16(M);
-    if (slices && M > 128 && slices_allowed(ctx, M, 0) && nsb == 4 && n_tiles <= kClusters[4] * sms / kNumSMsB200 && n_tiles > kClusters[5] * sms / kNumSMsB200 && tn_one * BMW * 4 <= RING_BYTES)
+    if (slices && M > 128 && M <= TN_MAX && slices_allowed(ctx, M, 0) && nsb == 4 && n_tiles <= kClusters[4] * sms / kNumSMsB200 && n_tiles > kClusters[5] * sms / kNumSMsB200 && tn_one * BMW * 4 <= RING_BYTES)
         return DensePlan{tn_one, 1, 4, 0, 1, false};
     DensePlan best{};
     double best_us = 1e30;

@@ -148,3 +148,18 @@ def test_slices_with_several_destinations(ctx, m, n, k, bits, gs, dt, ld, shift)
         assert torch.equal(block[:, :n], want)
         block[:, :n] = 7.0
         assert bool((o == 7.0).all())
+
+
+@pytest.mark.parametrize("m", [256, 257, 300, 432, 433])
+@pytest.mark.parametrize("n,k", [(4096, 1024), (3520, 896)])
+def test_a_chunk_has_at_most_256_rows(ctx, m, n, k):
+    """27 to 33 weight tiles and four super-blocks of K: the rows that one chunk holds, and those that take two."""
+    import torch
+    from metaltile_b200 import ops
+    w, s, b, x = dense_case(m, n, k, 4, 64, "f16", seed=33)
+    got = ops.qmm(to_dev(w), to_dev(s, "f16"), to_dev(b, "f16"), to_dev(x, "f16"), 4, 64, ctx=ctx)
+    torch.cuda.synchronize()
+    assert ctx.status_word() == 0
+    rows = np.unique(np.r_[0:2, 255:m][:12])
+    ref = oracle.qmm(w, s, b, np.ascontiguousarray(x[rows]), len(rows), n, k, 4, 64)
+    assert rel_err(got.float().cpu().numpy()[rows], ref) <= TOL["f16"]
