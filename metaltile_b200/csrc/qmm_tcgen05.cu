@@ -32,8 +32,8 @@
 // MMAs beside the 2 x 128 TN of X: 128 + TN cycles for the MMAs alone (measured), 2.9 cycles a token row in all at 2 x 256 rows where the tensor
 // cores need 2.  With A in tensor memory X and the packed words are all there is: 2 TN cycles, as the tensor cores.  What bounds it: at 240 and 256
 // rows the tensor cores at the clocks that the power leaves (2048 x 4096 x 4096, 4-bit 76 -> 67 us with the conversion of x), below some 200 rows the
-// instructions of the dequant warps (256 x 4096 x 4096 23.2 -> 15.5 us, 8-bit 333 x 7616 x 2880 36 -> 24); 154 other shapes 0.90 to 2.1 times as fast,
-// 1.20 in the mean (slowest: 13 slices through memory, 96 x 1216 x 3328).
+// instructions of the dequant warps (256 x 4096 x 4096 23.2 -> 15.5 us, 8-bit 333 x 7616 x 2880 36 -> 22); 2900 other products 0.85
+// to 2.3 times as fast, 1.25 in the mean (slowest: 5-bit rows that start on 8-byte boundaries only).
 //
 // Work items (weight-row tile, expert, first token row, token count) are enumerated arithmetically
 // for the dense case and read from a list in scratch memory for the gather case; that list is built
@@ -1353,24 +1353,34 @@ cudaError_t stage_x(Ctx *ctx, cudaStream_t st, const void *x, int rows, int K, i
     return cudaSuccess;
 }
 
-// Time of a k block of an item on one SM by its token rows, us (measured on 512 x 4096 x 4096, 2048 x 4096 x 4096 and 333 x 7616 x 2880, every width): up to 128
-// rows the hand-offs of two k blocks at a time, then of one, above some 210 rows the tensor cores at the clocks that the power leaves.  Other widths than 4
-// and 8 bits take more instructions a code; rows of scales that are no whole 16-byte pieces are copied by hand.
-double kb_cost(int TN, bool wide, int bits, bool pieces) {
-    const double more = (bits == 2 ? 0.035 : bits == 3 ? 0.053 : bits == 5 ? 0.11 : bits == 6 ? 0.135 : 0.0) + (pieces ? 0.0 : wide ? 0.02 : TN <= 128 ? 0.03 : 0.06);
-    if (wide) return 0.16 + 0.0017 * TN + more;
-    return (TN <= 128 ? 0.205 + 0.00045 * TN : TN <= 192 ? 0.31 : 0.31 + 0.0011 * (TN - 192)) + more;
+// Prices of a dense launch's forms, us, fitted together to 62000 launches in the forms that 2900 products of 17 to 2048 rows can take, every width (the one
+// taken is 1.025 times as long as the fastest in the mean; with prices fitted to a dozen products it was 1.07, since slices went through memory where clusters
+// are faster: 66 x 4224 x 1664 12.0 us, 8.1 in clusters of two; 453 x 384 x 3840 12.8, 9.4 in clusters of three.  One product in fifty became more than 5 %
+// slower by the new ones, up to 24 %: 1332 x 320 x 1408 at 5 bits 10.1 us as 14 items, 12.5 in 14 pairs.)
+// A k block of an item on one SM by its token rows: up to 128 the hand-offs of two k blocks at a time, then of one, above 192 and with two chunks the tensor
+// cores, behind which other widths than 4 and 8 bits hide what more they take a code.  Rows of scales that are no whole 16-byte pieces are copied
+// by hand; rows of words that start on 8-byte boundaries only set a pace of their own.
+double kb_cost(int TN, bool wide, int K, int bits, bool pieces) {
+    const double more = wide || TN > 192 ? 0.0 : bits == 2 ? 0.034 : bits == 3 ? 0.049 : bits == 5 ? 0.095 : bits == 6 ? 0.046 : 0.0;
+    const double by_hand = pieces ? 0.0 : wide ? 0.021 : TN <= 128 ? 0.033 : 0.038;
+    const double us = wide ? 0.24 + 0.00201 * TN : TN <= 128 ? 0.226 + 0.0007 * TN : TN <= 192 ? 0.349 : 0.349 + 0.00195 * (TN - 192);
+    return std::max(us + more + by_hand, K * bits / 8 % 16 != 0 ? 0.116 * bits : 0.0);
 }
-constexpr double kSliceUs = 1.2e-6;     // an f32 partial sum, written and read
+// a further item on the same SM: its accumulators drain before the next pair starts, or beside it where there are two sets
+double item_cost(int TN, bool wide) { return wide ? 0.4 + 0.012 * 2 * TN : TN > 192 ? 0.13 + 0.0106 * TN : 0.13; }
+constexpr double kMoreItems = 1.06;     // whole items narrower than cover the rows have to be that much cheaper (1.0: forms 1.0265 times the fastest in the mean, 1.06: 1.0245, 1.1: 1.0258)
+// K slices that add up in memory, beside the k blocks of one: the second kernel, for each slice, for each f32 partial sum that is written and read.
+constexpr double kSlicedUs = 7.2, kEachSliceUs = 0.054, kSliceUs = 1.52e-6;
 // Clusters of one to eight CTAs, one CTA an SM, that are resident at once (cudaOccupancyMaxActiveClusters: the GPCs do not divide evenly)
 // (45 of three are, but with all of them at once products of x in bf16 took 1.1 to 1.2 times as long as with 44)
 constexpr int kClusters[9] = {0, 148, 74, 44, 33, 26, 22, 15, 15};
-constexpr double kClusterUs[9] = {0, 0, 3.5, 6.0, 9.0, 12.0, 14.0, 15.0, 15.0}, kClusterRowUs = 0.005;      // a cluster's launch, barriers and sum: by its CTAs, and for each token row of one
-constexpr double kSlicedUs = 3.3;       // the second kernel of slices that add up in memory
-constexpr double kAgainUs = 0.8, kAgainClusterUs = 0.32;     // slices of more items than cover the rows, for each further one: its words are read and converted again
-constexpr double kMoreItems = 1.06;     // whole items narrower than cover the rows: within that the widest stay (2048 x 4096 x 4096 as 8 x 256 rows 56.9 us, as 9 x 240 55.7, at the power limit of a long step equal)
-// a further item on the same SM: its accumulators drain before the next pair starts, or beside it where there are two sets
-double item_cost(int TN, bool wide) { return wide ? 0.4 + 0.012 * 2 * TN : TN > 192 ? 0.4 + 0.009 * TN : 0.4; }
+// Slices that are the CTAs of a cluster: launch, barriers and sum; for each token row; for the share of such clusters that run, which wait for each other's SMs
+// (f16 products follow one another without a conversion of x between them), and steeply for the last tenth of the pairs (414 x 1536 x 1536 in 72 of them 16.1
+// us, 13.1 in 48).
+double cluster_cost(int S, int rows, long long units, bool f16) {
+    const double share = static_cast<double>(units) / kClusters[S];
+    return (S <= 4 ? 2.03 : 4.22) + 0.0106 * rows + ((S == 2 ? 0.77 : 2.95) + (f16 ? 1.21 : 0.0)) * share + (S == 2 ? 11.9 * std::max(0.0, share - 0.9) : 0.0);
+}
 
 // How a dense launch covers its M token rows: items of one chunk (TN rows, one accumulator) or of two (the dequantised W stage
 // is built once for both), chunks of equal width (333 rows are 2 x 176, not 256 + 77), and K slices where the items alone
@@ -1388,17 +1398,12 @@ constexpr size_t kSliceBytes = size_t{512} << 20;
 bool slices_allowed(const Ctx *ctx, int M, int form) {
     return ctx->qmm_ksplit && (ctx->qmm_wide == 1 || M <= TN_MAX) && (form == 0 || (ctx->qmm_wide && M > TN_MAX));
 }
-DensePlan plan_dense(const Ctx *ctx, int M, int N, int K, int bits, int group_size, bool slices = true) {
+DensePlan plan_dense(const Ctx *ctx, int M, int N, int K, int bits, int group_size, bool f16, bool slices = true) {
     const bool pieces = K / group_size % 8 == 0;
     const int n_tiles = (N + BMW - 1) / BMW, nkb = K / BK, nsb = (nkb + SB_PER_RAW - 1) / SB_PER_RAW, sms = ctx->sm_count;
     const auto up16 = [](int v) { return (v + 15) / 16 * 16; };
     if (ctx->qmm_force_tn > 0) return DensePlan{ctx->qmm_force_tn, (M + ctx->qmm_force_tn - 1) / ctx->qmm_force_tn, 1, 0, 0, false};
     constexpr int tn_wide = (TMEM_COLS - 3 * A_COLS) / 2;      // two accumulators and three k blocks of A, one for each team
-    // Up to 256 rows over four super-blocks of K, where four slices are one round: clusters of four, the form that tests/test_launches.py holds these
-    // products to (186 x 4096 x 1024 13.6 -> 12.4 us; four narrower whole items would take 9.5)
-    const int tn_one = up16(M);
-    if (slices && M > 128 && M <= TN_MAX && slices_allowed(ctx, M, 0) && nsb == 4 && n_tiles <= kClusters[4] * sms / kNumSMsB200 && n_tiles > kClusters[5] * sms / kNumSMsB200 && tn_one * BMW * 4 <= RING_BYTES)
-        return DensePlan{tn_one, 1, 4, 0, 1, false};
     DensePlan best{};
     double best_us = 1e30;
     auto offer = [&](double us, const DensePlan &p) {
@@ -1418,23 +1423,21 @@ DensePlan plan_dense(const Ctx *ctx, int M, int N, int K, int bits, int group_si
             if (TN == last_tn || (items_m > fewest && TN < 48)) continue;
             last_tn = TN;
             if ((items_m - 1) * (wide ? 2 : 1) * TN >= M) continue;                  // the last one would be empty
-            const double one = kb_cost(TN, false, bits, pieces), kb_us = kb_cost(TN, wide, bits, pieces), item_us = item_cost(TN, wide);
+            const double one = kb_cost(TN, false, K, bits, pieces), kb_us = kb_cost(TN, wide, K, bits, pieces), item_us = item_cost(TN, wide);
             const long long units = static_cast<long long>(n_tiles) * items_m;
-            // the teams take a stage each: the first comes after the time of a turn of theirs, half of which nothing else hides
-            const double turn = 0.5 * TEAMS * (!wide && TN <= 128 ? 2 : 1), more = items_m - fewest;
             // the last round of wide items on twice as many SMs, a chunk each, where that still is one round and every unit has two
             const int left = static_cast<int>(units % sms), last_rows = M - (items_m - 1) * 2 * TN;
             const bool tail = wide && units > sms && left > 0 && 2 * left <= sms && last_rows > TN;
             for (int S = 1; S <= 16; ++S) {
                 if (S > 1 && (!slices || !ctx->qmm_ksplit || S > nsb || (ctx->qmm_wide != 1 && M > TN_MAX))) break;
                 if (S > 1 && static_cast<size_t>(S) * M * N * sizeof(float) > kSliceBytes) break;
-                const double kb = (S == 1 ? nkb : (nsb + S - 1) / S * SB_PER_RAW) + (S == 1 ? 0.0 : turn);
+                const double kb = S == 1 ? nkb : (nsb + S - 1) / S * SB_PER_RAW;
                 const long long full = units * S / sms, rest = units * S % sms;
                 const double each_us = S == 1 ? item_us : item_cost(0, false);
                 double us = full * (kb * kb_us + each_us);
                 if (rest > 0) us += (S == 1 && tail ? kb * one : kb * kb_us) + each_us;
                 if (S == 1 && items_m > fewest) us *= kMoreItems;
-                if (S > 1) us += kSlicedUs + kAgainUs * more + static_cast<double>(S) * M * N * kSliceUs;
+                if (S > 1) us += kSlicedUs + kEachSliceUs * S + static_cast<double>(S) * M * N * kSliceUs;
                 offer(us, DensePlan{TN, items_m, S, S == 1 && tail ? left : 0, 0, wide});
             }
             // slices that are the CTAs of a cluster each and add up in shared memory: no block, no second kernel, but one round that the GPCs' odd sizes
@@ -1442,7 +1445,7 @@ DensePlan plan_dense(const Ctx *ctx, int M, int N, int K, int bits, int group_si
             if (!slices_allowed(ctx, M, form) || (wide ? 2 : 1) * TN * BMW * 4 > RING_BYTES) continue;
             for (int S = 2; S <= (wide ? 2 : 8) && S <= nsb; ++S) {
                 if (units > kClusters[S] * sms / kNumSMsB200) continue;
-                offer((nsb + S - 1) / S * SB_PER_RAW * kb_us + kClusterUs[S] + kClusterRowUs * (wide ? 2 : 1) * TN + kAgainClusterUs * more, DensePlan{TN, items_m, S, 0, 1, wide});
+                offer((nsb + S - 1) / S * SB_PER_RAW * kb_us + cluster_cost(S, (wide ? 2 : 1) * TN, units, f16), DensePlan{TN, items_m, S, 0, 1, wide});
             }
         }
     }
@@ -1558,8 +1561,8 @@ static int dense_grid(const DensePlan &plan, int items, int sms) {
 }
 
 // The form of a dense launch, for mtc_launch_of
-void qmm_tcgen05_form(const Ctx *ctx, int M, int N, int K, int bits, int group_size, mtc_launch_info *info) {
-    const DensePlan plan = plan_dense(ctx, M, N, K, bits, group_size);
+void qmm_tcgen05_form(const Ctx *ctx, int M, int N, int K, int bits, int group_size, int dt, mtc_launch_info *info) {
+    const DensePlan plan = plan_dense(ctx, M, N, K, bits, group_size, dt == MTC_F16);
     const int items = (N + BMW - 1) / BMW * plan.items_m * plan.ksplit + plan.halves;
     info->ctas = dense_grid(plan, items, ctx->sm_count);
     info->cluster = plan.cluster ? plan.ksplit : 1;
@@ -1570,7 +1573,7 @@ cudaError_t launch_qmm_tcgen05(Ctx *ctx, cudaStream_t st, const void *w, const v
                                const void *x, void *out, int M, int N, int K, int bits, int group_size, int dt,
                                std::string *why, void *const *outs, int n_outs, long long out_ld) {
     const int sms = ctx->sm_count;
-    DensePlan plan = plan_dense(ctx, M, N, K, bits, group_size);
+    DensePlan plan = plan_dense(ctx, M, N, K, bits, group_size, dt == MTC_F16);
     if (plan.ksplit > 1 && !plan.cluster) {
         cudaError_t ge = grow_block(ctx, st, &ctx->d_ksplit, &ctx->ksplit_bytes, static_cast<size_t>(plan.ksplit) * M * N * sizeof(float), why);
         if (ge != cudaSuccess) {
@@ -1578,7 +1581,7 @@ cudaError_t launch_qmm_tcgen05(Ctx *ctx, cudaStream_t st, const void *w, const v
             // during capture, or out of memory: the same product without slices needs no block
             if (ge != cudaErrorStreamCaptureUnsupported) cudaGetLastError();
             if (why) why->clear();
-            plan = plan_dense(ctx, M, N, K, bits, group_size, false);
+            plan = plan_dense(ctx, M, N, K, bits, group_size, dt == MTC_F16, false);
         }
     }
     const int TN = plan.TN;

@@ -906,7 +906,7 @@ int mtc_launch_of(const mtc_ctx *ctx, int M, const int *N, int n, int K, int bit
     if (cluster_first(c, k, M) && mtc::qmv_cluster_form(c, d, n, info)) return MTC_OK;
     if (n > 1 && k != K_FRAG && k != K_STREAM) return MTC_OK;         // one by one
     info->kernel = kProductKernelNames[k];
-    if (k == K_TCGEN05) mtc::qmm_tcgen05_form(c, M, N[0], K, bits, group_size, info);
+    if (k == K_TCGEN05) mtc::qmm_tcgen05_form(c, M, N[0], K, bits, group_size, dtype, info);
     return MTC_OK;
 }
 
