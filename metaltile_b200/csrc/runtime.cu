@@ -1368,7 +1368,7 @@ const char *mtc_gather_qmm_route(int m_total, int n_out, int k_in, int n_experts
     if (n_experts > 0 && gather_frag_takes(nullptr, true, m_total, n_out, k_in, n_experts, bits, group_size, dtype, nullptr, nullptr, nullptr, nullptr))
         return "gather_qmm_frag";
     if (n_experts > 0 && gather_exact_takes(nullptr, true, m_total, n_out, k_in, n_experts, bits, group_size, dtype, nullptr, nullptr, nullptr, nullptr))
-        return "gather_qmm_stream";
+        return "gather_qmm_exact";
     if (n_experts > 0 && gather_stream_takes(nullptr, true, m_total, n_out, k_in, n_experts, bits, group_size, dtype, nullptr, nullptr, nullptr, nullptr))
         return "gather_qmm_stream";
     return mtc::qmm_tcgen05_supported(m_total, n_out, k_in, bits, group_size, dtype, nullptr, nullptr, nullptr)

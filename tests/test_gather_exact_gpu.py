@@ -1,6 +1,6 @@
 """The exact grouped 4-bit bf16 kernel (csrc/gather_exact.cu): edges of its columns, k blocks, stages, halves and rows of scales against 64-bit sums,
-powers of two of rows and tokens at the ends of their ranges, what stays inside its token, what it reports, and the fused layer against the separate
-entries."""
+powers of two of rows and tokens at the ends of their ranges, infinities, what stays inside its token, what it reports, and the fused layer against the
+separate entries."""
 import pytest
 
 from test_gather_frag_gpu import _codes, _offsets, _stack
@@ -51,7 +51,7 @@ def test_products(counts, n, k, g):
     from metaltile_b200 import ops
 
     ctx = ops.context()
-    assert ctx.gather_qmm_route(sum(counts), n, k, len(counts), 4, g, "bf16") == "gather_qmm_stream"
+    assert ctx.gather_qmm_route(sum(counts), n, k, len(counts), 4, g, "bf16") == "gather_qmm_exact"
     got, ref, bound = _product(torch, ops, ctx, counts, n, k, g)
     assert bool(((got.double() - ref).abs() <= bound).all())
 
@@ -165,13 +165,47 @@ def test_layer_equals_the_separate_entries(tokens, e, top, hidden, inter, g):
     assert ops.context().status_word() == 0
 
 
+def test_reports_what_does_not_exist():
+    """Offsets past the rows or backwards: clamped, 0x901.  A row index past x: row 0 is read instead, 0x903."""
+    import torch
+    from metaltile_b200 import Context, MetalTileError, ops
+
+    ctx = Context(0)
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    e, n, k, g, m = 3, 200, 320, 64, 60
+    assert ctx.gather_qmm_route(m, n, k, e, 4, g, "bf16") == ctx.gather_qmm_route(m, k, n * 8, e, 4, g, "bf16") == "gather_qmm_exact"
+    w, s, b = _stack(torch, e, n, k, 4, g, torch.bfloat16, gen)
+    x = torch.randn((m, k), device="cuda", generator=gen).to(torch.bfloat16)
+
+    def reported(code):
+        with pytest.raises(MetalTileError):
+            ctx.sync(torch.cuda.current_stream().cuda_stream)
+        assert ctx.status_word() == code
+        ctx.status_clear()
+
+    for off, same in (([0, 20, 1000, 1001], [0, 20, 60, 60]), ([0, 40, 10, 60], None)):
+        out = torch.full((m + 1, n), 7.0, dtype=torch.bfloat16, device="cuda")
+        ops.gather_qmm(x, w, s, b, 4, g, expert_offsets=torch.tensor(off, dtype=torch.int32, device="cuda"), out=out[:m], ctx=ctx)
+        reported(0x901)
+        assert bool((out[m] == 7.0).all())
+        if same:
+            assert torch.equal(out[:m], ops.gather_qmm(x, w, s, b, 4, g, expert_offsets=torch.tensor(same, dtype=torch.int32, device="cuda"), ctx=ctx))
+    gate, up, down = (_stack(torch, e, a, c, 4, g, torch.bfloat16, gen) for a, c in ((192, k), (192, k), (k, 192)))
+    order, off = torch.arange(m, dtype=torch.int32, device="cuda") % 50, _offsets(torch, [25, 20, 15])
+    order[7], order[33] = 50, -1                             # not rows of the first 50
+    got = ops.moe_experts(x[:50], gate, up, down, 4, g, off, sort_token_idx=order, ctx=ctx)
+    reported(0x903)
+    order[7] = order[33] = 0
+    assert torch.equal(got, ops.moe_experts(x[:50], gate, up, down, 4, g, off, sort_token_idx=order, ctx=ctx)) and ctx.status_word() == 0
+
+
 def test_long_rows_of_scales_take_narrower_passes():
     from metaltile_b200 import _lib
     from metaltile_b200.context import _dt
 
     route = lambda k, rows, dt="bf16": _lib.load().mtc_gather_qmm_route(8 * rows, 1536, k, 8, 4, 64, _dt(dt)).decode()  # noqa: E731
-    assert {route(64 * g, 300) for g in (63, 64, 87, 88, 111)} == {route(2048, 300)}
-    assert route(64 * 112, 300) == route(64 * 112, 300, "f16") != route(2048, 300)
+    assert {route(64 * g, 300) for g in (63, 64, 87, 88, 111)} == {"gather_qmm_exact"}
+    assert route(64 * 112, 300) == route(64 * 112, 300, "f16") == "gather_qmm_tcgen05"
 
 
 def test_rule():
@@ -181,7 +215,7 @@ def test_rule():
     def route(m, n, k, e, bits=4, g=64, dt="bf16"):
         return _lib.load().mtc_gather_qmm_route(m, n, k, e, bits, g, _dt(dt)).decode()
 
-    frag, stream, tc = "gather_qmm_frag", "gather_qmm_stream", "gather_qmm_tcgen05"
-    assert [route(m, 768, 1088, 32) for m in (48, 49, 512 * 32, 512 * 32 + 1)] == [frag, stream, stream, tc]
-    assert [route(m, 832, 2112, 128) for m in (32, 33)] == [frag, stream]
+    frag, exact, tc = "gather_qmm_frag", "gather_qmm_exact", "gather_qmm_tcgen05"
+    assert [route(m, 768, 1088, 32) for m in (48, 49, 512 * 32, 512 * 32 + 1)] == [frag, exact, exact, tc]
+    assert [route(m, 832, 2112, 128) for m in (32, 33)] == [frag, exact]
     assert [route(m, 832, 2112, 128, dt="f16") for m in (33, 1300)] == [frag, tc]

@@ -101,7 +101,7 @@ def test_rule():
 
     frag, stream, tc = "gather_qmm_frag", "gather_qmm_stream", "gather_qmm_tcgen05"
     assert [route(m, 768, 2048, 128, 4, 64) for m in (64, 65)] == [frag, stream]
-    assert [route(m, 512, 1024, 16, 4, 64) for m in (64, 65)] == [frag, stream]
+    assert [route(m, 512, 1024, 16, 4, 64) for m in (64, 65)] == [frag, "gather_qmm_exact"]
     assert [route(m, 768, 2048, 128, 8, 64) for m in (512, 513)] == [frag, tc]
     assert [route(m, 768, 1024, 32, 6, 32) for m in (320, 321)] == [frag, tc]
     assert route(8, 768, 2048, 128, 8, 64, "f32") == "gather_qmm_cuda_core"

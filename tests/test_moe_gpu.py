@@ -174,6 +174,13 @@ def test_gather_qmm_matches_oracle(ctx, n_experts, n_out, k_in, bits, gs, dt, co
     assert ctx.status_word() == 0
 
 
+@pytest.fixture
+def without_the_exact_kernel(request, ctx):
+    ctx.set_option("gather_stream", 2 if request.param else 1)
+    yield
+    ctx.set_option("gather_stream", 1)
+
+
 @pytest.mark.parametrize("n_experts,n_out,k_in,gs,dt,counts", [
     (6, 768, 2048, 64, "bf16", [31, 32, 33, 0, 1, 65]),                 # one, two and three passes per expert; an empty one
     (5, 2048, 768, 64, "bf16", [8, 9, 40, 17, 24]),                     # K = 1.5 x 512: runs of 256 codes
@@ -182,10 +189,13 @@ def test_gather_qmm_matches_oracle(ctx, n_experts, n_out, k_in, bits, gs, dt, co
     (2, 48, 8192, 128, "f16", [9, 2]),                                  # K = 8192: 8 rows per pass
     (40, 64, 256, 64, "bf16", [(7 * i) % 11 for i in range(40)]),       # many small experts, more experts than a scan round
     (1, 16, 256, 64, "f16", [1]),
+    (4, 33, 256, 64, "bf16", [10, 70, 0, 21]),                          # rows of scales that the exact kernel does not take
+    (3, 64, 8192, 64, "bf16", [6, 17, 5]),                              # nor ones as long
 ])
-def test_gather_stream_matches_oracle(ctx, n_experts, n_out, k_in, gs, dt, counts):
-    """The weight-streaming grouped product (few rows per expert) against the oracle, and - where the tensor-memory kernel
-    takes the shape too - against that kernel within rounding."""
+@pytest.mark.parametrize("without_the_exact_kernel", [False, True], indirect=True)
+def test_gather_stream_matches_oracle(ctx, without_the_exact_kernel, n_experts, n_out, k_in, gs, dt, counts):
+    """The weight-streaming grouped products (few rows per expert) against the oracle, and - where the tensor-memory kernel
+    takes the shape too - against that kernel within rounding.  Also without the exact kernel, which else takes most of the bf16 shapes."""
     import torch
     from metaltile_b200 import ops
     w, s, b, x, off, _ = _gather_case(n_experts, n_out, k_in, 4, gs, dt, counts, seed=2)
@@ -208,7 +218,7 @@ def test_gather_stream_matches_oracle(ctx, n_experts, n_out, k_in, gs, dt, count
     assert rel_err(out.float().cpu().numpy(), other.float().cpu().numpy()) <= 2 * TOL[dt]
 
 
-@pytest.mark.parametrize("stream_kernel", [1, 0])
+@pytest.mark.parametrize("stream_kernel", [1, 2, 0])
 def test_gather_reports_bad_offsets(ctx, stream_kernel):
     """expert_offsets that run past m_total are clamped to it on both tensor-core paths (nothing outside x or out is
     touched: the rows that exist get their expert's product, the others do not exist) and reported: 0x901."""
@@ -282,13 +292,14 @@ def test_moe_layer_config4(ctx):
     assert ctx.status_word() == 0
 
 
+@pytest.mark.parametrize("without_the_exact_kernel", [False, True], indirect=True)
 @pytest.mark.parametrize("dt,hidden,inter,gs,bits,counts", [
-    ("bf16", 512, 256, 64, 4, [9, 0, 33, 20, 2]),          # the streamed form (four launches)
+    ("bf16", 512, 256, 64, 4, [9, 0, 33, 20, 2]),          # the exact form; without it the streamed one (four launches)
     ("f16", 256, 512, 128, 4, [5, 17, 1]),
     ("bf16", 128, 64, 32, 4, [4, 6]),                      # outside the streaming kernel's contract: composed from the entries
     ("f32", 128, 64, 32, 8, [3, 0, 5]),
 ])
-def test_moe_experts_equals_the_separate_entries(ctx, dt, hidden, inter, gs, bits, counts):
+def test_moe_experts_equals_the_separate_entries(ctx, without_the_exact_kernel, dt, hidden, inter, gs, bits, counts):
     """mtc_moe_experts == permute -> gather_qmm(gate), gather_qmm(up) -> swiglu -> gather_qmm(down), bit for bit, with and
     without the permutation folded in; and against the oracle for one expert."""
     import torch
