@@ -71,8 +71,11 @@ int mtc_memset(mtc_ctx *ctx, void *stream, void *d_ptr, int value, size_t bytes)
 int mtc_sync(mtc_ctx *ctx, void *stream);
 int mtc_sync_deadline(mtc_ctx *ctx, void *stream, int timeout_ms);
 /* 0 when no kernel has reported a bounded-wait expiry or a rejected index since the context was created or the
- * word was cleared; otherwise the code of the first report: 0x101-0x402 roles of the tensor-core kernel, 0x601 + r
- * rank r never arrived at a peer barrier, 0x701 / 0x702 phase counter / partial-sum slot of a chained launch. */
+ * word was cleared; otherwise the code of the first report: 0x101-0x403, 0x501, 0x502 waits of the tensor-core kernel's roles (0x501 also
+ * an expert id out of range in mtc_moe_sort), 0x601 + r rank r never arrived at a peer barrier, 0x701 / 0x702 phase counter /
+ * partial-sum slot of a chained launch, 0x801-0x831 the tensor-memory decode kernel, 0x901 expert_offsets that run backwards or past the rows,
+ * 0x902 more passes than a grouped product's table holds, 0x903 / 0x904 a row index that does not exist, 0xa01-0xa0b waits of the exact
+ * grouped kernel's roles. */
 int mtc_status_word(mtc_ctx *ctx, uint32_t *word);
 int mtc_status_clear(mtc_ctx *ctx);
 
@@ -88,7 +91,9 @@ int mtc_status_clear(mtc_ctx *ctx);
  * Range of bf16 and f32 activations: "qmv_cluster" (and the grouped "gather_qmm_frag") hold whatever the type does, infinities
  * included, but a token whose values all lie below 2^-112 comes out as zeros; one with a value from 2^31 on, or all of them below 2^-64, makes
  * its launch some 20 times as long.  "qmv_frag", "qmv_stream" and "gather_qmm_stream" make an infinity of a value from 2^63 on, and
- * lose bits where all values of a token lie below 2^-57. */
+ * lose bits where all values of a token lie below 2^-57.  "gather_qmm_exact" and the tensor-core kernel ("qmm_tcgen05", "gather_qmm_tcgen05") scale
+ * every bf16 token by its largest value and round what lies below 2^-31 of it, by 2^-40 of it at most; the exact one gives infinities as the
+ * sum from the definition does, the other as f16 operands do (an infinite token makes an infinity of its values from 65520 on, too). */
 int mtc_qmv(mtc_ctx *ctx, void *stream, const void *w, const void *scales, const void *biases,
             const void *x, void *out, int M, int N, int K, int bits, int group_size, int dtype);
 
@@ -294,10 +299,10 @@ int mtc_peer_barrier(mtc_ctx *ctx, void *stream, void *const *peer_flags, int n_
  *   "qmv_tc"           1: those shapes run on the tensor-memory decode kernel instead (slower today; default 0)
  *   "gather_stream"    0: grouped products never take the weight-streaming kernels nor the grouped fragment kernel (default 1: the CSR
  *                      form does.  Few rows per expert, every width, f16 / bf16, k_in % 32 == 0, power-of-two group >= 32: the fragment
- *                      kernel, mtc_gather_qmm_route names "gather_qmm_frag".  4-bit codes, group 64 or 128, "gather_qmm_stream": with bf16 up
- *                      to 512 rows per expert the tcgen05 kernel on exact operands (csrc/gather_exact.cu: k_in a multiple of the group, a row of
- *                      scales of at most some 100 groups, n_out * groups a multiple of 8, 16-byte aligned arrays), else, with
- *                      k_in % 256 == 0 and m_total <= 64 n_experts, the one on warp-level tensor cores); 2: as 1 without the exact kernel
+ *                      kernel, mtc_gather_qmm_route names "gather_qmm_frag".  4-bit codes, group 64 or 128: with bf16 up
+ *                      to 512 rows per expert the tcgen05 kernel on exact operands (csrc/gather_exact.cu, "gather_qmm_exact": k_in a multiple of the
+ *                      group, a row of scales of at most 111 groups, n_out * groups a multiple of 8, 16-byte aligned arrays), else, with
+ *                      k_in % 256 == 0 and m_total <= 64 n_experts, the one on warp-level tensor cores, "gather_qmm_stream"); 2: as 1 without the exact kernel
  *   "pdl_early_weights" 0: no product reads w, scales or biases before the previous kernel of its stream is
  *                      complete.  Default 1: the dense products (mtc_qmv*, mtc_qmm*, mtc_qvm, chains) are launched with
  *                      programmatic dependent launch and start copying WEIGHTS while the previous kernel drains - weights are
@@ -324,7 +329,7 @@ int mtc_set_option(mtc_ctx *ctx, const char *name, int value);
  * x rows are sorted by expert; w is stacked u32[E, n_out, k_in*bits/32], scales/biases T[E, n_out, k_in/group].
  * Exactly one of expert_offsets / indices is non-NULL.  f16/bf16 activations with k_in % 64 == 0 and a
  * power-of-two group >= 32 run on the tensor cores (few rows per expert - see "gather_stream" - on the
- * weight-streaming kernel, else on the tensor-memory kernel), everything else on CUDA cores.  Offsets that reach
+ * weight-streaming kernels, else on the tensor-memory kernel), everything else on CUDA cores.  Offsets that reach
  * past m_total or run backwards are clamped (rows that do not exist are neither read nor written) and reported
  * through the status word (0x901). */
 int mtc_gather_qmm(mtc_ctx *ctx, void *stream, const void *x, const void *w, const void *scales,
@@ -353,9 +358,9 @@ int mtc_gather_qmm_static(mtc_ctx *ctx, void *stream, const void *x, const void 
  * gate, up: [n_experts, inter, hidden*bits/32]; down: [n_experts, hidden, inter*bits/32]; y: [m_total, hidden].
  * The gate and up products and the SwiGLU are rounded to the activation type exactly as the separate entries
  * (mtc_moe_permute, mtc_gather_qmm twice, mtc_swiglu, mtc_gather_qmm) round them: same results bit for bit.
- * Few rows per expert (m_total <= 64 n_experts; 4-bit, f16 / bf16, group 64 / 128, hidden and inter multiples of 256):
- * four launches on the weight-streaming kernel - rows to MMA fragments with the permutation folded in, gate and up as
- * one stream over both matrices, SwiGLU to fragments, down.  Other shapes: composed from the separate entries.
+ * Each product runs on the kernel that mtc_gather_qmm takes for it.  Gate and up are one launch, with the permutation folded in, on the fragment
+ * kernel, on the exact one (which applies the SwiGLU, behind a launch that prepares the rows) and on the streaming one (whose down product stages
+ * silu(gate) * up itself, four launches in all); on the tensor-memory and CUDA-core kernels the layer is composed from the separate entries.
  * The intermediates live in grow-only blocks of the context (they move only outside stream capture). */
 typedef struct {
     const void *w, *scales, *biases;

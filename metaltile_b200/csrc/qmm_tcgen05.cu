@@ -32,8 +32,8 @@
 // MMAs beside the 2 x 128 TN of X: 128 + TN cycles for the MMAs alone (measured), 2.9 cycles a token row in all at 2 x 256 rows where the tensor
 // cores need 2.  With A in tensor memory X and the packed words are all there is: 2 TN cycles, as the tensor cores.  What bounds it: at 240 and 256
 // rows the tensor cores at the clocks that the power leaves (2048 x 4096 x 4096, 4-bit 76 -> 67 us with the conversion of x), below some 200 rows the
-// instructions of the dequant warps (256 x 4096 x 4096 23.2 -> 15.5 us, 8-bit 333 x 7616 x 2880 36 -> 22); 2900 other products 0.85
-// to 2.3 times as fast, 1.25 in the mean (slowest: 5-bit rows that start on 8-byte boundaries only).
+// instructions of the dequant warps (256 x 4096 x 4096 23.2 -> 15.5 us, 8-bit 333 x 7616 x 2880 36 -> 22); 3200 other products 0.87
+// to 2.1 times as fast, 1.25 in the mean, eleven of them below 0.97.
 //
 // Work items (weight-row tile, expert, first token row, token count) are enumerated arithmetically
 // for the dense case and read from a list in scratch memory for the gather case; that list is built
@@ -88,7 +88,7 @@ struct QmmParams {
     uint32_t hint_ns;            // base suspend-time hint of the waits (0: plain polling)
     int raw;                     // 1: packed words reach the dequant warps through shared memory (cp.async, whole lines)
     uint32_t raw_off, raw_tile;  // byte offset of the raw buffers in shared memory; bytes of one buffer
-    int nraw, raw_blk;           // raw: number of buffers; k blocks of one (4; 2 at 8 bits beside two chunks, which leaves the ring its third stage)
+    int nraw, raw_blk;           // raw: number of buffers; k blocks of one (4; 2 at 8 bits beside two chunks, so that the ring keeps two stages)
     int raw8;                    // raw: 1 = rows of packed words start on 8-byte boundaries only (3 / 5 bits, K an odd multiple of 64)
     // raw: scales (and biases) of the tile, a span of sp_kb k blocks (sp_bytes of a row) at a time, two buffers.  Spans begin at multiples of sp_kb, and with
     // a K slice
@@ -194,7 +194,7 @@ __device__ __forceinline__ void lds_words(uint32_t addr, uint32_t (&w)[BITS]) {
     }
 }
 
-// ---- dequantisation of half a W row segment (32 codes = BITS words) into 4 swizzled 16-byte chunks --
+// ---- dequantisation: windows of codes that a f32 fraction holds, for the general form ----------------
 template <int BITS>
 struct QPack {
     static constexpr int CPW = 23 / BITS;       // codes per window: a window must fit the 23 mantissa bits
@@ -1064,7 +1064,7 @@ qmm_tcgen05_kernel(const __grid_constant__ QmmMaps maps, const QmmParams p) {
 
 // bf16 activations -> f16 with one power-of-two factor per row.  bf16 keeps 8 significant bits, so
 // x * 2^-e is exact in f16 (11 bits) once the row maximum is brought to [2^14, 2^15); elements more than
-// 2^38 below the row maximum lose bits, which changes nothing measurable.  The MMA then runs on f16
+// 2^31 below the row maximum lose bits (2^-40 of it at most), which changes nothing measurable.  The MMA then runs on f16
 // operands, whose 3 extra mantissa bits keep the dequantised weights 8x closer to the f32 oracle than
 // bf16 weights would be; the epilogue multiplies the accumulator by 2^e again.
 // W warps share a row and hold it in registers between the maximum and the conversion (one read of x instead of two), eight
@@ -1403,7 +1403,7 @@ DensePlan plan_dense(const Ctx *ctx, int M, int N, int K, int bits, int group_si
     const int n_tiles = (N + BMW - 1) / BMW, nkb = K / BK, nsb = (nkb + SB_PER_RAW - 1) / SB_PER_RAW, sms = ctx->sm_count;
     const auto up16 = [](int v) { return (v + 15) / 16 * 16; };
     if (ctx->qmm_force_tn > 0) return DensePlan{ctx->qmm_force_tn, (M + ctx->qmm_force_tn - 1) / ctx->qmm_force_tn, 1, 0, 0, false};
-    constexpr int tn_wide = (TMEM_COLS - 3 * A_COLS) / 2;      // two accumulators and three k blocks of A, one for each team
+    constexpr int tn_wide = (TMEM_COLS - 3 * A_COLS) / 2;      // two accumulators and three k blocks of A (5-, 6- and 8-bit rings have two stages there)
     DensePlan best{};
     double best_us = 1e30;
     auto offer = [&](double us, const DensePlan &p) {

@@ -224,7 +224,8 @@ inline bool gather_frag_rule(int m_total, int n_out, int k_in, int n_experts, in
     if (codes <= (32ll << 20)) return rows <= 10 * experts;
     return rows <= (group_size % 64 == 0 ? 4 : bits == 8 ? 2 : 3) * experts;
 }
-// The exact tcgen05 kernel (gather_exact.cu) against those, 4-bit bf16 layers, by the same measures (us a layer, other kernel -> it).  It reads an expert's
+// The exact tcgen05 kernel (gather_exact.cu) against those, 4-bit bf16 layers, by the same measures (us a layer, other kernel -> it; the figures of the tcgen05
+// kernel that dequantises, here and above, are from before its operand lay in tensor memory, which made it 1.1 to 1.4 times as fast).  It reads an expert's
 // matrices once for up to 64 rows, but its launches and an item's start cost more.
 //   up to 16 Mi codes, against the fragment kernel: 16 of 1024 x 512, 4 rows 28.1 against 28.4; 6 rows 37.8 -> 29.1, 16 rows 44 -> 30; 64 of 512 x 256, 4
 //     rows 26.6 against 29.8, 6 rows 35.2 -> 30.5; 8 of 1600 x 1088 4 rows 35.1 against 35.3, 8 rows 40.7 -> 36.6.
