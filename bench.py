@@ -569,7 +569,7 @@ def main():
                 "note": "per-GPU; launch-averaged over the 4 matrix shapes of the step (graph replay, events)"}
     line = {"metric": METRIC, "value": value, "unit": "GB/s", "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True, "scaling": "strong",
-            "vs_baseline": None, "dtype": "f32", "data": "synthetic", "config": config, "run": run_info, "verified": verified,
+            "vs_baseline": None, "dtype": "bf16", "data": "synthetic", "config": config, "run": run_info, "verified": verified,
             "clocks": clocks,
             "e2e": {"value": e2e_value, "unit": "GB/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                     "ms_per_step": e2e_ms},
