@@ -566,9 +566,14 @@ __global__ void __launch_bounds__(kThreads, 1) gather_exact_kernel(const __grid_
                 // the biased exponent of the factor: 2^(118 - ex), or 2^(139 - ex) where that leaves a scale of these rows less than 2^-17, whose last bit f16 does
                 // not hold.  Rows that this leaves one, too, are marked, and those with an infinity.
                 int up = max(245 - ex, 1);
-                const bool wide = __any_sync(0xffffffffu, static_cast<int>(least >> 7) + up < 237);
-                if (wide) up = min(max(266 - ex, 1), 253);
-                const bool mark = static_cast<int>(least >> 7) + up < 237 || ex >= 252;
+                const bool far = static_cast<int>(least >> 7) + up < 237 || ex >= 252;
+                bool wide = __any_sync(0xffffffffu, far), mark = false;
+                if (wide) {                             // rows past n_out hold what an item before left in the buffer, or nothing yet
+                    const bool exists = i % a.tiles * tile_rows + (a.two ? r & 63 : r) < a.n_out;
+                    wide = __any_sync(0xffffffffu, far && exists);
+                    if (wide) up = min(max(266 - ex, 1), 253);
+                    mark = exists && (static_cast<int>(least >> 7) + up < 237 || ex >= 252);
+                }
                 const float f = __uint_as_float(static_cast<uint32_t>(up) << 23);
                 for (int c = 0; c < nch; ++c) {
                     if (turn == team) {
