@@ -232,16 +232,21 @@ inline bool gather_frag_rule(int m_total, int n_out, int k_in, int n_experts, in
 //   up to 64 Mi: where the streaming kernel takes the shape, 32 of 1024 x 768, half a row 26.4 against 29.4, one row 37.5 -> 34.7, 8 rows 46.6 -> 41, 32
 //     rows 70 -> 49; 64 of 1024 x 768, one to four rows as fast.  Where it does not: 32 of 1088 x 832, one row 39.1 against 39.8, two 46.0 and 45.9, three 55.6 ->
 //     46.3, 37 rows 114 -> 56.
-//   more: 128 of 1024 x 768 (96 Mi), streamed, 1 / 2 / 4 rows 62 / 72 / 76 against 64 / 75 / 79; 128 of 2048 x 768, 2 / 4 / 8 / 32 rows 105 against 115, 127
-//     and 127, 139 -> 130, 258 -> 156, 64 rows 356 -> 238; not streamed, 128 of 2112 x 832, 1/8 / 1/4 / 1/2 / 4 rows 41 against 47, 62 and 61, 92 -> 81, 287 -> 157.
+//     Many small experts in whole runs of the streaming kernel: 128 of 512 x 1024, 1 / 4 / 7 / 12 rows 52 / 65 / 69 / 80 against 56 / 73 / 75 / 79; 128 of 512 x 512 42 /
+//     50 / 53 / 60 against 42 / 52 / 53 / 55; 64 of 512 x 1024, 4 / 7 / 12 rows 47 / 52 / 59 against 48 / 51 / 53; but 64 of 768 x 512, 1 / 4 rows 36 / 44 -> 35 / 43.
+//   more, streamed (whose time steps up behind eight rows): the smaller an expert's matrix, the more an item's start weighs.  128 of 512 x 1536, 4 / 6 / 8 / 10 rows 82 /
+//     85 / 89 / 105 against 94 / 96 / 98 / 99; 128 of 1024 x 1024 88 / 94 / 99 / 110 against 97 / 99 / 101 / 100; 128 of 2048 x 768 128 / 133 / 138 / 157 against 133 /
+//     134 / 136 / 137; 64 of 1536 x 1024 78 / 82 / 86 / 97 against 82 / 82 / 83 / 83; 64 of 2048 x 1536, 4 / 5 / 6 rows 127 / 129 / 131 against 128 / 128 / 127; 128 of
+//     2048 x 768, 32 / 64 rows 258 -> 156, 356 -> 238; not streamed, 128 of 2112 x 832, 1/8 / 1/4 / 1/2 / 4 rows 41 against 47, 62 and 61, 92 -> 81, 287 -> 157.
 //   the most: against the tcgen05 kernel, which converts a matrix once for up to 256 rows: 8 of 2048 x 1536, 256 / 512 / 1024 rows 135 -> 98, 196 -> 161, 280
 //     against 282; 32 of 1024 x 768 168 -> 136, 267 -> 241, 433 against 462.
 inline bool gather_exact_rule(int m_total, int n_out, int k_in, int n_experts, bool streamed) {
     const long long codes = static_cast<long long>(n_experts) * n_out * k_in, rows = m_total, experts = n_experts;
     if (rows > 512 * experts) return false;
     if (codes <= (16ll << 20)) return rows > 4 * experts;
-    if (codes <= (64ll << 20)) return 2 * rows > (streamed ? 1 : 3) * experts;
-    return streamed ? rows > 4 * experts : 4 * rows > experts;
+    if (codes <= (64ll << 20)) return 2 * rows > (!streamed ? 3 : experts >= 64 && k_in % 512 == 0 ? 16 : 1) * experts;
+    const long long each = codes / experts;
+    return streamed ? rows > (each >= 2 << 20 ? 5 : each >= 3 << 19 ? 6 : 8) * experts : 4 * rows > experts;
 }
 // rows: weight rows of the launch (N, or those of all fused projections)
 inline bool frag_takes(const Ctx *ctx, int M, long long rows, bool fused, int N, int K, int bits, int group_size, int dt, const void *w, const void *scales,
