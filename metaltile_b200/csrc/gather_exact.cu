@@ -14,7 +14,7 @@
 // each weight row (its largest scale, or bias / 8, comes to [2^-9, 2^-8)), one for each row of x (its largest value to [2^14, 2^15)); the
 // epilogue takes them out.  That holds every scale down to 2^-8 of its row's largest.  Where a row of the 32 of a warp has smaller ones, they come to
 // [2^12, 2^13) instead and the operand is (1024 + q - 1032) * scale, 13 instructions, which holds them down to 2^-29 (the layer below 151 us
-// before there was this form, 154 with it, 174 where every row takes it).  Rows with smaller ones yet or with
+// before there was this form, 152.5 with it, 173 where every row takes it).  Rows with smaller ones yet or with
 // an infinity, and infinite tokens, are added up from the definition.  Elements of x below 2^-31 of their row's largest are rounded, by 2^-40 of it at most, as every tcgen05 product of bf16 rows does.
 //
 // Work.  A PASS is (expert, up to TB of its rows); an item is a pass x 128 weight rows (64 of gate and 64 of up where one launch covers
@@ -96,8 +96,7 @@ struct __align__(16) ECtrl {
     int4 head[2];                                      // the item's pass: expert, first row, rows
     uint32_t tmem_base;
     volatile uint32_t abort;
-    volatile int again;                                // 1 + the last item with results that are added up from the definition
-    uint32_t again_rows[2][kEpiWarps];                 // of the item's rows those that are for every token, and all that there are
+    uint32_t again_rows[2][kEpiWarps];                 // of an item's rows those that are added up from the definition for every token, and all that there are
     uint64_t drained;                                  // giving up: the MMAs are complete
     uint32_t stages_issued, items_issued;              // what the producer started
     alignas(16) float row_factor[2][kRows];            // negative: a row whose scales the operands do not hold
@@ -407,7 +406,6 @@ __global__ void __launch_bounds__(kThreads, 1) gather_exact_kernel(const __grid_
         }
         mbar_init(&ctl->drained, 1);
         ctl->abort = 0;
-        ctl->again = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == kLoadWarp) tmem_alloc_all(&ctl->tmem_base);
@@ -532,10 +530,12 @@ __global__ void __launch_bounds__(kThreads, 1) gather_exact_kernel(const __grid_
                 if (!wait(item_full + e * 8, eph, 0xa07)) return;
                 __syncwarp();
                 const uint32_t row = items + e * a.item_bytes + r * rb, brow = row + kRows * rb;
-                // the power of two of the row, by its largest scale or bias / 8, and its least scale
+                // the power of two of the row, by its largest scale or bias / 8, and its least scale.  (Loops that run once an item are not unrolled, here and in the
+                // epilogue: straight-line code is fetched anew, a line of it some 250 cycles.  512 tokens of 128 experts 154.7 -> 152.0 us.)
                 uint32_t top = 0, btop = 0, low = 0x7FFF7FFFu;
                 if (align == 16) {                      // lanes start at different pieces: rows lie 64 bytes apart, or some such number
                     uint32_t at = (lane >> 1) * 16 % rb;
+#pragma unroll 1
                     for (uint32_t g = 0; g < rb; g += 16) {
                         const uint4 sv = lds16<16>(row + at);
                         top = __vmaxu2(top, max4(sv));
@@ -544,6 +544,7 @@ __global__ void __launch_bounds__(kThreads, 1) gather_exact_kernel(const __grid_
                         at = at + 16 == rb ? 0 : at + 16;
                     }
                 } else if (align == 4) {
+#pragma unroll 1
                     for (uint32_t g = 0; g < rb; g += 4) {
                         const uint32_t sv = lds4<true>(row + g) & 0x7FFF7FFFu;
                         top = __vmaxu2(top, sv);
@@ -551,6 +552,7 @@ __global__ void __launch_bounds__(kThreads, 1) gather_exact_kernel(const __grid_
                         btop = __vmaxu2(btop, lds4<true>(brow + g) & 0x7FFF7FFFu);
                     }
                 } else {                                // an odd number: the last one with the one before it
+#pragma unroll 1
                     for (uint32_t g = 0; g < rb; g += 4) {
                         const uint32_t at = min(g, rb - min(rb, 4u));
                         const uint32_t sv = lds4<false>(row + at), bv = lds4<false>(brow + at), keep = rb == 2 ? 0x7FFFu : 0x7FFF7FFFu;
@@ -692,10 +694,14 @@ __global__ void __launch_bounds__(kThreads, 1) gather_exact_kernel(const __grid_
             }
             __syncwarp();
             // The warps share the buffer and named barriers, so they give up together; by this vote the item before has left the buffer.
-            if (!epilogue_votes(ok)) break;
+            // Items with results that the operands do not hold are found by the same vote.
+            const float rf = ok ? ctl->row_factor[e][r] : 0.0f;
+            bool again = false;
+            if (!epilogue_votes(ok && rf >= 0.0f && !infinite)) {
+                if (!epilogue_votes(ok)) break;
+                again = true;
+            }
             tc_fence_after();
-            const float rf = ctl->row_factor[e][r];
-            if (rf < 0.0f || infinite) ctl->again = i + 1;
             unsigned short *const to = reinterpret_cast<unsigned short *>(staged) + r;
 #pragma unroll 1
             for (int t0 = 0; t0 < pass.z; t0 += 16) {
@@ -723,13 +729,13 @@ __global__ void __launch_bounds__(kThreads, 1) gather_exact_kernel(const __grid_
             e ^= 1;
             asm volatile("bar.sync 1, 128;" ::: "memory");
             const int n0 = i % a.tiles * tile_rows;
-            if (ctl->again == i + 1) from_definition(a, ctl, pass, n0, rf < 0.0f);
+            if (again) from_definition(a, ctl, pass, n0, rf < 0.0f);
             // out of shared memory, a token a warp
             if (a.act) {
                 const int n = n0 + 2 * lane;
                 const bool pairs = (a.n_out & 1) == 0 && (reinterpret_cast<uintptr_t>(a.act) & 3) == 0;
                 unsigned short *const o = static_cast<unsigned short *>(a.act) + static_cast<size_t>(pass.y) * a.n_out + n;
-#pragma unroll 2
+#pragma unroll 1
                 for (int t = warp; t < pass.z; t += kEpiWarps) {
                     const uint32_t *const from = reinterpret_cast<const uint32_t *>(staged + t * (kRows * 2)) + lane;
                     const uint32_t v = silu_mul(from[0], from[32]);
@@ -745,7 +751,7 @@ __global__ void __launch_bounds__(kThreads, 1) gather_exact_kernel(const __grid_
                 const int m = a.two ? lane >> 4 : 0, n = n0 + (a.two ? lane & 15 : lane) * 4;
                 const bool vec = (a.n_out & 3) == 0 && (reinterpret_cast<uintptr_t>(a.outs[m]) & 7) == 0;
                 unsigned short *const o = static_cast<unsigned short *>(a.outs[m]) + static_cast<size_t>(pass.y) * a.n_out + n;
-#pragma unroll 2
+#pragma unroll 1
                 for (int t = warp; t < pass.z; t += kEpiWarps) {
                     const uint2 v = *reinterpret_cast<const uint2 *>(staged + t * (kRows * 2) + lane * 8);
                     unsigned short *const p = o + static_cast<size_t>(t) * a.n_out;
