@@ -227,4 +227,7 @@ def test_rule():
     frag, exact, tc = "gather_qmm_frag", "gather_qmm_exact", "gather_qmm_tcgen05"
     assert [route(m, 768, 1088, 32) for m in (48, 49, 512 * 32, 512 * 32 + 1)] == [frag, exact, exact, tc]
     assert [route(m, 832, 2112, 128) for m in (32, 33)] == [frag, exact]
+    # where the streaming kernel takes the shape, rows an expert by the size of an expert's matrix
+    for n, k, e, rows in ((1024, 512, 128, 8), (512, 768, 64, 0.5), (1536, 512, 128, 8), (768, 2048, 128, 6), (1536, 2048, 64, 5)):
+        assert [route(m, n, k, e) for m in (int(rows * e), int(rows * e) + 1)] == [frag if rows < 1 else "gather_qmm_stream", exact], (n, k, e)
     assert [route(m, 832, 2112, 128, dt="f16") for m in (33, 1300)] == [frag, tc]
